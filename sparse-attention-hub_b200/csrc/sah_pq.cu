@@ -118,23 +118,34 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
   SAH_REQUIRE((xs_s * 2) % 16 == 0 && (xs_h * 2) % 16 == 0 && (xs_b * 2) % 16 == 0 && ((uintptr_t)x % 16) == 0,
               "pq_assign_tc: key rows must be 16-byte aligned");
   if (key_begin == key_end) return SAH_OK;
-  static bool allowed = false;
-  if (!allowed) {
-    cudaError_t e = cudaFuncSetAttribute(pq_assign_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PtcCfg::SMEM);
-    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_assign_tc attr: %s", cudaGetErrorString(e));
-    allowed = true;
-  }
   if (sm_count <= 0) sm_count = 148;
-  const int64_t groups = (int64_t)B * Hkv * n_sub;
-  const int64_t n_tiles = sah_ceil_div(key_end - key_begin, (int64_t)PTC_TILE);
-  int64_t slices = sah_ceil_div((int64_t)4 * sm_count, groups);  // about two waves of two CTAs per SM
-  if (slices > n_tiles) slices = n_tiles;
-  if (slices < 1) slices = 1;
-  SAH_REQUIRE(groups <= 65535, "pq_assign_tc: too many groups per launch");
-  dim3 grid((unsigned)slices, (unsigned)groups);
-  pq_assign_tc_kernel<<<grid, PTC_THREADS, PtcCfg::SMEM, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), xs_b, xs_h, xs_s, Hkv, key_begin, key_end, init_offset, n_sub,
-      n_cent, centroids, codes, cap, errflag);
+  // four neighbouring sub-vectors per CTA (a key's 64 bytes, one 4-byte store of codes) when the
+  // layout allows it, else one; n_cent padded to a power-of-two number of 32-column blocks
+  const int ns = (n_sub % 4 == 0 && (reinterpret_cast<uintptr_t>(codes) & 3) == 0) ? 4 : 1;
+  const int64_t n_blocks = (int64_t)B * Hkv * (n_sub / ns);
+  const int64_t items = n_blocks * sah_ceil_div(key_end - key_begin, (int64_t)PTC_TILE);
+  const unsigned grid = (unsigned)(items < 2 * (int64_t)sm_count ? (items + 1) / 2 : sm_count);
+  const cudaStream_t st = (cudaStream_t)stream;
+#define PTC_LAUNCH(NS, NB)                                                                                       \
+  do {                                                                                                           \
+    static const cudaError_t allowed = cudaFuncSetAttribute(                                                     \
+        pq_assign_tc_kernel<NS, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, PtcCfg<NS>::SMEM);             \
+    if (allowed != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_assign_tc attr: %s", cudaGetErrorString(allowed)); \
+    pq_assign_tc_kernel<NS, NB><<<grid, PTC_THREADS, PtcCfg<NS>::SMEM, st>>>(                                    \
+        reinterpret_cast<const __nv_bfloat16*>(x), xs_b, xs_h, xs_s, Hkv, key_begin, key_end, init_offset,       \
+        n_sub, n_cent, n_blocks, centroids, codes, cap, errflag);                                                \
+  } while (0)
+#define PTC_LAUNCH_NS(NS)                   \
+  do {                                      \
+    if (n_cent <= 32) PTC_LAUNCH(NS, 1);    \
+    else if (n_cent <= 64) PTC_LAUNCH(NS, 2);  \
+    else if (n_cent <= 128) PTC_LAUNCH(NS, 4); \
+    else PTC_LAUNCH(NS, 8);                 \
+  } while (0)
+  if (ns == 4) PTC_LAUNCH_NS(4);
+  else PTC_LAUNCH_NS(1);
+#undef PTC_LAUNCH_NS
+#undef PTC_LAUNCH
   SAH_LAUNCH_CHECK("pq_assign_tc");
   return SAH_OK;
 }

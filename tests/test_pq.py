@@ -245,3 +245,31 @@ def test_gpu_ip_metric_build_decode_and_append_equal_the_reference():
     np.testing.assert_array_equal(idx, g["append_idx"])
     np.testing.assert_array_equal(ptr, g["append_ptr"])
     np.testing.assert_allclose(out, g["append_out"], atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_sub,n_cent,n_keys", [(16, 256, 1), (16, 64, 129), (4, 128, 300), (6, 256, 255), (3, 32, 128)])
+def test_gpu_assignment_tile_edges_and_layouts(n_sub, n_cent, n_keys):
+    """`sah_pq_assign_tc` at the edges of its tiles (one key, a tile, a tile and one), for every
+    padded centroid count and with one or four sub-vectors per CTA, on integer-valued keys and
+    centroids (many exact ties): the codes of `sah_pq_assign`."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, off = 1, 2, 3
+    gen = torch.Generator(device=dev).manual_seed(n_cent + n_keys)
+    keys = torch.randint(-3, 4, (B, Hkv, n_keys + off, n_sub * 8), generator=gen, device=dev).to(torch.bfloat16)
+    cent = torch.randint(-3, 4, (B * Hkv * n_sub, n_cent, 8), generator=gen, device=dev).float()
+    cap, st = n_keys + 2, _native.stream_of(torch.device(dev))
+    want = torch.full((B, Hkv, cap, n_sub), 255, dtype=torch.uint8, device=dev)
+    got = want.clone()
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    strides = (keys.stride(0), keys.stride(1), keys.stride(2))
+    _native.check(lib.sah_pq_assign(keys.data_ptr(), _native.SAH_BF16, *strides, B, Hkv, off, n_keys + off, off, n_sub, 8,
+                                    n_cent, cent.data_ptr(), want.data_ptr(), cap, 0, st), "sah_pq_assign")
+    _native.check(lib.sah_pq_assign_tc(keys.data_ptr(), *strides, B, Hkv, off, n_keys + off, off, n_sub, 8, n_cent,
+                                       cent.data_ptr(), got.data_ptr(), cap, err.data_ptr(), 148, st), "sah_pq_assign_tc")
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and torch.equal(got, want)
