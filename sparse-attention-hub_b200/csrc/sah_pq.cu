@@ -150,39 +150,107 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
   return SAH_OK;
 }
 
-// Cluster sums in fp64 (so that the summation order does not reach the fp32
-// result) and counts; shared-memory accumulation per CTA, then global atomics.
+// Cluster sums in fp64 (so that the summation order does not reach the fp32 result) and counts.
+// A CTA takes strips of PQA_STRIP keys of one group: it sorts the strip's keys by code (a
+// counting sort with integer atomics in shared memory), then two threads per centroid walk the
+// centroid's keys, each adding half of the channels into fp64 registers that live across the
+// strips; the registers go to global memory with one atomic per (centroid, channel) and CTA.
+// Bound: shared-memory integer atomics and L2 (every 32-byte sector of a key is fetched by the
+// CTAs of two sub-vectors).  8 KV heads x 65472 keys x 16 sub-vectors: 134 us; with one fp64
+// shared-memory atomic per key and channel -- a compare-and-swap loop -- it took 812 us.
+#define PQA_THREADS 512
+#define PQA_STRIP 4096
+
 template <typename T>
-__global__ void __launch_bounds__(PQ_TILE)
+__global__ void __launch_bounds__(PQA_THREADS, 3)
 pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
-                     int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent,
+                     int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int vec8,
                      const uint8_t* __restrict__ codes, int64_t cap, double* __restrict__ sums,
                      int* __restrict__ counts) {
-  extern __shared__ double pq_sum_sm[];  // [n_cent][sub_d] then int [n_cent]
-  int* cnt_sm = reinterpret_cast<int*>(pq_sum_sm + n_cent * sub_d);
+  __shared__ int pos_sm[256];              // histogram, then the next free slot of every centroid
+  __shared__ int start_sm[257];
+  __shared__ int scan_sm[33];
+  __shared__ uint16_t order_sm[PQA_STRIP]; // key numbers of the strip, sorted by code
+  constexpr int HALF = (PQ_MAX_SUBD + 1) / 2;
+  constexpr int PER = PQA_STRIP / PQA_THREADS;
+  const int tid = threadIdx.x;
   const int sub = blockIdx.y;
   const int64_t bk = blockIdx.z;
   const int kvh = (int)(bk % Hkv);
   const int64_t b = bk / Hkv;
   const int64_t grp = bk * n_sub + sub;
-  for (int i = threadIdx.x; i < n_cent * sub_d; i += PQ_TILE) pq_sum_sm[i] = 0.0;
-  for (int i = threadIdx.x; i < n_cent; i += PQ_TILE) cnt_sm[i] = 0;
-  __syncthreads();
-  // each CTA walks a strip of keys so that the global atomics stay few
-  const int64_t strip = (n_keys + gridDim.x - 1) / gridDim.x;
-  const int64_t j0 = (int64_t)blockIdx.x * strip;
-  const int64_t j1 = j0 + strip < n_keys ? j0 + strip : n_keys;
-  for (int64_t j = j0 + threadIdx.x; j < j1; j += PQ_TILE) {
-    const int c = codes[(bk * cap + j) * n_sub + sub];
-    const T* xr = x + b * xs_b + kvh * xs_h + (j + init_offset) * xs_s + sub * sub_d;
-    for (int d = 0; d < sub_d; ++d) atomicAdd(&pq_sum_sm[c * sub_d + d], (double)sah_to_float<T>(xr[d]));
-    atomicAdd(&cnt_sm[c], 1);
+  const int cent = tid >> 1;
+  const int half = (sub_d + 1) / 2;        // channels of the even threads
+  const int d0 = (tid & 1) ? half : 0, nd = (tid & 1) ? sub_d - half : half;
+  const T* xg = x + b * xs_b + kvh * xs_h + init_offset * xs_s + sub * sub_d + d0;
+  const uint8_t* cg = codes + bk * cap * n_sub + sub;
+  double acc[HALF];
+  int count = 0;
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) acc[i] = 0.0;
+  for (int64_t j0 = (int64_t)blockIdx.x * PQA_STRIP; j0 < n_keys; j0 += (int64_t)gridDim.x * PQA_STRIP) {
+    if (tid < 256) pos_sm[tid] = 0;
+    int code[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int64_t j = j0 + i * PQA_THREADS + tid;
+      code[i] = j < n_keys ? cg[j * n_sub] : -1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (code[i] >= 0) atomicAdd(&pos_sm[code[i]], 1);
+    __syncthreads();
+    int total;
+    const int before = sah_block_excl_scan<int>(tid < 256 ? pos_sm[tid] : 0, scan_sm, &total);
+    if (tid < 256) { start_sm[tid] = before; pos_sm[tid] = before; }
+    if (tid == 0) start_sm[256] = total;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (code[i] >= 0) order_sm[atomicAdd(&pos_sm[code[i]], 1)] = (uint16_t)(i * PQA_THREADS + tid);
+    __syncthreads();
+    const int e1 = start_sm[cent + 1];
+    int e = start_sm[cent];
+    count += e1 - e;
+    const T* xs = xg + j0 * xs_s;
+    if (sizeof(T) == 2 && vec8) {  // four channels in 8 aligned bytes; four keys in flight
+      for (; e + 4 <= e1; e += 4) {
+        uint2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u] * xs_s);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          acc[0] += (double)__uint_as_float(v[u].x << 16);
+          acc[1] += (double)__uint_as_float(v[u].x & 0xffff0000u);
+          acc[2] += (double)__uint_as_float(v[u].y << 16);
+          acc[3] += (double)__uint_as_float(v[u].y & 0xffff0000u);
+        }
+      }
+      for (; e < e1; ++e) {
+        const uint2 v = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e] * xs_s);
+        acc[0] += (double)__uint_as_float(v.x << 16);
+        acc[1] += (double)__uint_as_float(v.x & 0xffff0000u);
+        acc[2] += (double)__uint_as_float(v.y << 16);
+        acc[3] += (double)__uint_as_float(v.y & 0xffff0000u);
+      }
+    } else {
+      for (; e < e1; ++e) {
+        const T* xr = xs + (int64_t)order_sm[e] * xs_s;
+#pragma unroll
+        for (int i = 0; i < HALF; ++i)
+          if (i < nd) acc[i] += (double)sah_to_float<T>(xr[i]);
+      }
+    }
+    __syncthreads();  // the sorted list and the starts are done with
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_cent * sub_d; i += PQ_TILE)
-    if (pq_sum_sm[i] != 0.0) atomicAdd(&sums[grp * n_cent * sub_d + i], pq_sum_sm[i]);
-  for (int i = threadIdx.x; i < n_cent; i += PQ_TILE)
-    if (cnt_sm[i]) atomicAdd(&counts[grp * n_cent + i], cnt_sm[i]);
+  if (cent < n_cent && count > 0) {
+    double* out = sums + (grp * n_cent + cent) * sub_d + d0;
+#pragma unroll
+    for (int i = 0; i < HALF; ++i)
+      if (i < nd) atomicAdd(out + i, acc[i]);
+    if ((tid & 1) == 0) atomicAdd(&counts[grp * n_cent + cent], count);
+  }
 }
 
 extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
@@ -193,13 +261,21 @@ extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t
   SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_cent > 0 && n_keys >= 0,
               "pq_accumulate: bad extents");
   if (n_keys == 0) return SAH_OK;
-  int strips = (int)sah_ceil_div(n_keys, 4096);
-  if (strips > 64) strips = 64;
-  dim3 grid((unsigned)strips, (unsigned)n_sub, (unsigned)((int64_t)B * Hkv));
-  const size_t smem = (size_t)n_cent * sub_d * sizeof(double) + (size_t)n_cent * sizeof(int);
+  if (sub_d > PQ_MAX_SUBD || n_cent > 256)
+    return sah_fail(SAH_ERR_UNSUPPORTED, "pq_accumulate: sub-vector dim %d (<= %d) / %d centroids (<= 256)",
+                    sub_d, PQ_MAX_SUBD, n_cent);
+  // one wave of three CTAs per SM; the strips of a slice share the CTA's registers
+  const int64_t groups = (int64_t)B * Hkv * n_sub;
+  int64_t slices = (int64_t)3 * 148 / groups;
+  if (slices < 1) slices = 1;
+  const int64_t strips = sah_ceil_div(n_keys, (int64_t)PQA_STRIP);
+  if (slices > strips) slices = strips;
+  dim3 grid((unsigned)slices, (unsigned)n_sub, (unsigned)((int64_t)B * Hkv));
+  const int vec8 = sub_d == 8 && (reinterpret_cast<uintptr_t>(x) & 7) == 0 && xs_s % 4 == 0 && xs_h % 4 == 0 &&
+                   xs_b % 4 == 0;
   SAH_DISPATCH_DTYPE(dtype, T, {
-    pq_accumulate_kernel<T><<<grid, PQ_TILE, smem, (cudaStream_t)stream>>>(
-        (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, codes, cap,
+    pq_accumulate_kernel<T><<<grid, PQA_THREADS, 0, (cudaStream_t)stream>>>(
+        (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, vec8, codes, cap,
         sums, counts);
   });
   SAH_LAUNCH_CHECK("pq_accumulate");

@@ -273,3 +273,40 @@ def test_gpu_assignment_tile_edges_and_layouts(n_sub, n_cent, n_keys):
                                        cent.data_ptr(), got.data_ptr(), cap, err.data_ptr(), 148, st), "sah_pq_assign_tc")
     torch.cuda.synchronize()
     assert int(err.item()) == 0 and torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,n_sub,sub_d,n_keys", [("bf16", 16, 8, 1), ("bf16", 16, 8, 4097), ("bf16", 4, 9, 5000),
+                                                      ("f32", 3, 16, 4096), ("f32", 2, 5, 9000)])
+def test_gpu_cluster_sums_equal_float64_sums(dtype, n_sub, sub_d, n_keys):
+    """`sah_pq_accumulate`: counts exact, and float64 sums that round to the float32 sums of numpy's
+    float64 additions (values are multiples of 2^-8 below 8, so float64 sums are exact in any
+    order); one cluster holds half of the keys and one none."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, off, n_cent = 2, 1, 2, 32
+    gen = torch.Generator(device=dev).manual_seed(n_keys)
+    keys = (torch.randint(-2047, 2048, (B, Hkv, n_keys + off, n_sub * sub_d), generator=gen, device=dev) / 256.0)
+    keys = keys.to(workloads.torch_dtype(dtype))
+    cap = n_keys + 3
+    codes = torch.randint(0, n_cent - 1, (B, Hkv, cap, n_sub), generator=gen, device=dev)
+    codes[:, :, ::2] = 7
+    codes = codes.to(torch.uint8)
+    groups = B * Hkv * n_sub
+    sums = torch.zeros((groups, n_cent, sub_d), dtype=torch.float64, device=dev)
+    counts = torch.zeros((groups, n_cent), dtype=torch.int32, device=dev)
+    _native.check(lib.sah_pq_accumulate(keys.data_ptr(), _native.dtype_code(keys.dtype), keys.stride(0), keys.stride(1),
+                                        keys.stride(2), B, Hkv, n_keys, off, n_sub, sub_d, n_cent, codes.data_ptr(), cap,
+                                        sums.data_ptr(), counts.data_ptr(), _native.stream_of(torch.device(dev))),
+                  "sah_pq_accumulate")
+    x = keys.double().cpu().numpy()[:, :, off:].reshape(B * Hkv, n_keys, n_sub, sub_d)
+    c = codes.cpu().numpy()[:, :, :n_keys].reshape(B * Hkv, n_keys, n_sub)
+    want, cnt = np.zeros((groups, n_cent, sub_d)), np.zeros((groups, n_cent), np.int64)
+    for g in range(groups):
+        np.add.at(want[g], c[g // n_sub, :, g % n_sub], x[g // n_sub, :, g % n_sub])
+        cnt[g] = np.bincount(c[g // n_sub, :, g % n_sub], minlength=n_cent)
+    np.testing.assert_array_equal(counts.cpu().numpy(), cnt)
+    np.testing.assert_array_equal(sums.cpu().numpy(), want)
