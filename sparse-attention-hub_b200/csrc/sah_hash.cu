@@ -5,15 +5,26 @@
 #include "sah_select.cuh"
 
 // ---------------------------------------------------------------------------
-// Encode.  One CTA hashes a tile of TK vectors of one (batch, output head).
-// Activations live in shared memory as fp32 [channel][vector]; one layer is a
-// register-tiled product where each thread owns KT vectors x 4 outputs and
-// walks the input channels in ascending order with a single fp32 accumulator
-// per output, which fixes the summation order the CPU restatement follows.
+// Encode.  A persistent CTA hashes tiles of HE_TK vectors; its tiles are a contiguous range of
+// the (batch, output head, tile) list, so that a head's weights (fp32, every layer) are staged
+// once and stay in shared memory while the head lasts, and every SM gets the same share of the
+// list.  Activations are fp32 [channel][vector] and overwritten layer by layer.
+//
+// One layer is a register-tiled product in which every output has a single fp32 accumulator
+// that walks the input channels in ascending order, fma by fma; that fixes the summation order
+// that the CPU restatement follows, and it is why the tensor cores are no help.  What bounds it
+// is the fp32 pipe (two vectors per instruction, fma.rn.f32x2, each half rounding as the scalar
+// fma does) against the shared-memory reads that feed it: a thread owns 16 vectors x 4 outputs,
+// whose 64 multiply-adds need four broadcast reads of activations and one of weights.
+// 32 heads x 16384 keys through 128-128-128-32: 1963 us with tiles of 64 vectors, 8 x 4 outputs
+// per thread, scalar fma and the weights staged per tile; 981 us now (19.3 G
+// multiply-adds; 540 us at 128 per clock and SM).
 // ---------------------------------------------------------------------------
-#define HE_TK 64        // vectors per CTA
+#define HE_TK 128       // vectors per tile
 #define HE_THREADS 256
 #define HE_MAXD 128     // widest layer
+#define HE_PITCH 132    // floats per activation channel: lanes that write neighbouring channels
+                        // four vectors at a time hit different banks
 
 struct HashEncodeArgs {
   const void* x;
@@ -27,6 +38,8 @@ struct HashEncodeArgs {
   int act;
   const uint16_t* act_table;
   uint32_t* codes;
+  int64_t tiles_per_head, tiles;  // the tiled kernel's list
+  int resident;                   // every layer's weights fit beside the activations
 };
 
 template <typename T>
@@ -52,114 +65,182 @@ __device__ __forceinline__ float he_activate<float>(float v, int act, const uint
 
 #include "sah_hash_tc.cuh"
 
-template <typename T, int KT>
-__device__ __forceinline__ void he_layer(const float* __restrict__ a_in, float* __restrict__ a_out,
-                                         const float* __restrict__ w_sm,
-                                         const T* __restrict__ bias_h, int din, int dout,
-                                         bool last, int act, const uint16_t* act_table,
-                                         unsigned int* codes_sm) {
-  const int nkg = HE_TK / KT;  // vector groups
-  const int tk = threadIdx.x % nkg, to = threadIdx.x / nkg;
-  float acc[KT][4];
-#pragma unroll
-  for (int i = 0; i < KT; ++i)
-#pragma unroll
-    for (int o = 0; o < 4; ++o) acc[i][o] = 0.f;
+__device__ __forceinline__ unsigned long long he_pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
 
+// One layer over the tile: thread (kg, og) owns vectors kg * KP + i and outputs o * NOG + og.
+// KP x OP is 16 x 4 for 128 outputs, 16 x 2 for 64, 8 x 2 for 32, 8 x 1 for 16, so that 256
+// threads always cover the tile.  w_sm is [channel][og][o]: a thread's weights adjoin.
+template <typename T, int KP, int OP>
+__device__ __forceinline__ void he_layer(float* __restrict__ act, const float* __restrict__ w_sm,
+                                         const T* __restrict__ bias_h, int din, bool last, int act_kind,
+                                         const uint16_t* act_table, uint32_t* codes, int nvalid) {
+  constexpr int NOG = HE_THREADS / (HE_TK / KP);
+  const int og = threadIdx.x % NOG, kg = threadIdx.x / NOG;
+  unsigned long long acc[KP / 2][OP];
+#pragma unroll
+  for (int i = 0; i < KP / 2; ++i)
+#pragma unroll
+    for (int o = 0; o < OP; ++o) acc[i][o] = 0ull;
+  float b[OP];
+#pragma unroll
+  for (int o = 0; o < OP; ++o) b[o] = sah_to_float<T>(bias_h[o * NOG + og]);
+
+  const float* ap = act + kg * KP;
+  const float* wp = w_sm + og * OP;
+#pragma unroll 4
   for (int d = 0; d < din; ++d) {
-    float a[KT];
-    const float* ap = a_in + d * HE_TK + tk * KT;
+    unsigned long long a[KP / 2], w[OP];
 #pragma unroll
-    for (int i = 0; i < KT; ++i) a[i] = ap[i];
-    const float4 w = *reinterpret_cast<const float4*>(w_sm + d * dout + to * 4);
-#pragma unroll
-    for (int i = 0; i < KT; ++i) {
-      acc[i][0] = fmaf(a[i], w.x, acc[i][0]);
-      acc[i][1] = fmaf(a[i], w.y, acc[i][1]);
-      acc[i][2] = fmaf(a[i], w.z, acc[i][2]);
-      acc[i][3] = fmaf(a[i], w.w, acc[i][3]);
+    for (int i = 0; i < KP / 4; ++i) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(ap + d * HE_PITCH + i * 4);
+      a[2 * i] = v.x;
+      a[2 * i + 1] = v.y;
     }
+    if (OP == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(wp + d * (NOG * OP));
+      w[0] = he_pack2(v.x, v.x); w[1 % OP] = he_pack2(v.y, v.y);
+      w[2 % OP] = he_pack2(v.z, v.z); w[3 % OP] = he_pack2(v.w, v.w);
+    } else if (OP == 2) {
+      const float2 v = *reinterpret_cast<const float2*>(wp + d * (NOG * OP));
+      w[0] = he_pack2(v.x, v.x); w[1 % OP] = he_pack2(v.y, v.y);
+    } else {
+      const float v = wp[d * (NOG * OP)];
+      w[0] = he_pack2(v, v);
+    }
+#pragma unroll
+    for (int o = 0; o < OP; ++o)
+#pragma unroll
+      for (int i = 0; i < KP / 2; ++i)
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][o]) : "l"(a[i]), "l"(w[o]));
   }
+  __syncthreads();  // everybody has read the input activations
 
-  float b[4];
+  unsigned int word = 0u;
 #pragma unroll
-  for (int o = 0; o < 4; ++o) b[o] = sah_to_float<T>(bias_h[to * 4 + o]);
-
+  for (int o = 0; o < OP; ++o) {
+    float v[KP];
 #pragma unroll
-  for (int i = 0; i < KT; ++i) {
-    unsigned int nib = 0u;
+    for (int i = 0; i < KP / 2; ++i)
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * i]), "=f"(v[2 * i + 1]) : "l"(acc[i][o]));
 #pragma unroll
-    for (int o = 0; o < 4; ++o) {
-      float v = sah_round_to<T>(acc[i][o]);        // einsum output in dtype
-      v = sah_round_to<T>(__fadd_rn(v, b[o]));     // + bias, rounded
-      if (!last) {
-        v = he_activate<T>(v, act, act_table);
-        a_out[(to * 4 + o) * HE_TK + tk * KT + i] = v;
-      } else {
-        nib |= (v > 0.f ? 1u : 0u) << o;
+    for (int i = 0; i < KP; ++i) {
+      v[i] = sah_round_to<T>(v[i]);                   // einsum output in dtype
+      v[i] = sah_round_to<T>(__fadd_rn(v[i], b[o]));  // + bias, rounded
+      if (!last) v[i] = he_activate<T>(v[i], act_kind, act_table);
+    }
+    if (!last) {
+      float* dst = act + (o * NOG + og) * HE_PITCH + kg * KP;
+#pragma unroll
+      for (int i = 0; i < KP / 4; ++i)
+        *reinterpret_cast<float4*>(dst + i * 4) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    } else if (NOG == 16) {
+      // signatures have at most 32 bits: OP <= 2, the halves of a warp are two vector groups
+#pragma unroll
+      for (int i = 0; i < KP; ++i) {
+        const unsigned int bits = __ballot_sync(0xffffffffu, v[i] > 0.f);
+        const unsigned int mine = (threadIdx.x & 16) ? bits >> 16 : bits & 0xffffu;
+        if (og == i) word |= mine << (16 * o);
       }
     }
-    if (last && nib) atomicOr(&codes_sm[tk * KT + i], nib << (to * 4));
   }
+  if (last && NOG == 16 && og < KP && kg * KP + og < nvalid) codes[kg * KP + og] = word;
+}
+
+// where output `out` of a layer of width dout goes: he_layer's [og][o]
+__device__ __forceinline__ int he_weight_slot(int dout, int out) {
+  const int nog = dout >= 64 ? 32 : 16;
+  return (out % nog) * (dout / nog) + out / nog;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(HE_THREADS)
+__global__ void __launch_bounds__(HE_THREADS, 1)
 hash_encode_kernel(HashEncodeArgs p) {
   extern __shared__ __align__(16) unsigned char he_smem[];
-  float* act0 = reinterpret_cast<float*>(he_smem);
-  float* act1 = act0 + HE_MAXD * HE_TK;
-  float* w_sm = act1 + HE_MAXD * HE_TK;
-  __shared__ unsigned int codes_sm[HE_TK];
+  float* act = reinterpret_cast<float*>(he_smem);  // [HE_MAXD][HE_PITCH]
+  float* w_sm = act + HE_MAXD * HE_PITCH;
+  const int D = p.dims[0], cpr = D / 8;
+  const int64_t t_first = p.tiles * blockIdx.x / gridDim.x, t_last = p.tiles * (blockIdx.x + 1) / gridDim.x;
+  int staged = -1;  // the head whose weights are in w_sm
 
-  const int64_t tile = blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int h_in = h / (p.H_out / p.H_in);
-  const int64_t n0 = p.n_begin + tile * HE_TK;
-  const int D = p.dims[0];
-  const T* xb = reinterpret_cast<const T*>(p.x) + b * p.xs_b + h_in * p.xs_h;
-
-  // Stage the input tile transposed: act0[d][i].
-  const int chunks = D / 8;
-  for (int idx = threadIdx.x; idx < HE_TK * chunks; idx += HE_THREADS) {
-    int i = idx % HE_TK, c = idx / HE_TK;
-    int64_t n = n0 + i;
-    float f[8];
-    if (n < p.n_end) {
-      sah_load8<T>(xb + n * p.xs_n + c * 8, f);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = 0.f;
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) act0[(c * 8 + e) * HE_TK + i] = f[e];
-  }
-  if (threadIdx.x < HE_TK) codes_sm[threadIdx.x] = 0u;
-
-  float* a_in = act0;
-  float* a_out = act1;
-  for (int l = 0; l < p.n_layers; ++l) {
+  auto stage_weights = [&](int l, int h, float* dst) {
     const int din = p.dims[l], dout = p.dims[l + 1];
-    __syncthreads();  // previous layer done with w_sm / a_out complete
     const T* wl = reinterpret_cast<const T*>(p.weights[l]) + (int64_t)h * din * dout;
-    for (int idx = threadIdx.x; idx < din * dout; idx += HE_THREADS)
-      w_sm[idx] = sah_to_float<T>(wl[idx]);
-    __syncthreads();
-    const T* bl = reinterpret_cast<const T*>(p.bias[l]) + (int64_t)h * dout;
-    const bool last = (l == p.n_layers - 1);
-    switch (dout) {
-      case 128: he_layer<T, 8>(a_in, a_out, w_sm, bl, din, dout, last, p.act, p.act_table, codes_sm); break;
-      case 64:  he_layer<T, 4>(a_in, a_out, w_sm, bl, din, dout, last, p.act, p.act_table, codes_sm); break;
-      case 32:  he_layer<T, 2>(a_in, a_out, w_sm, bl, din, dout, last, p.act, p.act_table, codes_sm); break;
-      default:  he_layer<T, 1>(a_in, a_out, w_sm, bl, din, dout, last, p.act, p.act_table, codes_sm); break;
+    const int out = threadIdx.x % dout, slot = he_weight_slot(dout, out), step = HE_THREADS / dout;
+#pragma unroll 8
+    for (int d = threadIdx.x / dout; d < din; d += step) dst[d * dout + slot] = sah_to_float<T>(wl[d * dout + out]);
+  };
+  // A tile's input, transposed on its way into shared memory.  bfloat16 rows are fetched into
+  // registers while the last layer of the tile before is computed.
+  constexpr int FETCH = HE_TK * HE_MAXD / 8 / HE_THREADS;
+  uint4 raw[FETCH];
+  auto row_of = [&](int64_t t, int i) -> const T* {
+    const int64_t bh = t / p.tiles_per_head;
+    const int64_t n = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK + i;
+    if (n >= p.n_end) return nullptr;
+    const int h = (int)(bh % p.H_out);
+    return reinterpret_cast<const T*>(p.x) + bh / p.H_out * p.xs_b + h / (p.H_out / p.H_in) * p.xs_h + n * p.xs_n;
+  };
+  auto fetch = [&](int64_t t) {
+    const T* row = row_of(t, threadIdx.x % HE_TK);
+#pragma unroll
+    for (int f = 0; f < FETCH; ++f) {
+      const int c = threadIdx.x / HE_TK + f * (HE_THREADS / HE_TK);
+      raw[f] = make_uint4(0u, 0u, 0u, 0u);
+      if (c < cpr && row != nullptr) raw[f] = *reinterpret_cast<const uint4*>(row + c * 8);
     }
-    float* t = a_in; a_in = a_out; a_out = t;
-  }
-  __syncthreads();
-  if (threadIdx.x < HE_TK) {
-    int64_t n = n0 + threadIdx.x;
-    if (n < p.n_end)
-      p.codes[((int64_t)b * p.H_out + h) * p.n_total + n] = codes_sm[threadIdx.x];
+  };
+  if (sizeof(T) == 2 && t_first < t_last) fetch(t_first);
+
+  for (int64_t t = t_first; t < t_last; ++t) {
+    const int64_t bh = t / p.tiles_per_head;
+    const int h = (int)(bh % p.H_out);
+    const int64_t n0 = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK;
+    // (the last layer's barrier stands between the reads of the tile before and these writes)
+    {
+      const int i = threadIdx.x % HE_TK;
+      const T* row = sizeof(T) == 2 ? nullptr : row_of(t, i);
+#pragma unroll
+      for (int f = 0; f < FETCH; ++f) {
+        const int c = threadIdx.x / HE_TK + f * (HE_THREADS / HE_TK);
+        if (c < cpr) {
+          float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          if (sizeof(T) == 2) sah_unpack8(raw[f], v);
+          else if (row != nullptr) sah_load8<T>(row + c * 8, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) act[(c * 8 + e) * HE_PITCH + i] = v[e];
+        }
+      }
+    }
+    if (p.resident && staged != h) {
+      float* dst = w_sm;
+      for (int l = 0; l < p.n_layers; ++l) {
+        stage_weights(l, h, dst);
+        dst += p.dims[l] * p.dims[l + 1];
+      }
+      staged = h;
+    }
+    const float* w_l = w_sm;
+    uint32_t* codes = p.codes + bh * p.n_total + n0;
+    const int nvalid = (int)(p.n_end - n0 < HE_TK ? p.n_end - n0 : HE_TK);
+    for (int l = 0; l < p.n_layers; ++l) {
+      const int din = p.dims[l], dout = p.dims[l + 1];
+      const bool last = l == p.n_layers - 1;
+      if (!p.resident) stage_weights(l, h, w_sm);  // the layer before ended its reads at a barrier
+      __syncthreads();
+      if (sizeof(T) == 2 && last && t + 1 < t_last) fetch(t + 1);
+      const T* bl = reinterpret_cast<const T*>(p.bias[l]) + (int64_t)h * dout;
+      switch (dout) {
+        case 128: he_layer<T, 16, 4>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+        case 64:  he_layer<T, 16, 2>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+        case 32:  he_layer<T, 8, 2>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+        default:  he_layer<T, 8, 1>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+      }
+      if (p.resident) w_l += din * dout;
+    }
   }
 }
 
@@ -312,8 +393,9 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
   // SAH_HASH_TC=1 in the environment sends bfloat16 index builds through the tensor-core kernel
   // (same bits, see sah_hash_tc.cuh).  It is not the default: each layer rounds its products to
   // bfloat16, about 31 % of the accumulators lie within the error band of a rounding midpoint, so
-  // nearly every warp repeats nearly every output in the fixed order and the build takes 2.6x to
-  // 4.6x as long as hash_encode_kernel (134 ms against 52 ms for 8 x 32768 keys x 32 heads).
+  // nearly every warp repeats nearly every output in the fixed order and the build took 2.6x to
+  // 4.6x as long as hash_encode_kernel did at 52 ms for 8 x 32768 keys x 32 heads (134 ms), which
+  // has halved since.
   const char* tc_e = getenv("SAH_HASH_TC");
   const int tc_env = (tc_e != nullptr && tc_e[0] == '1') ? 1 : 0;
   bool tc = tc_env == 1 && dtype == SAH_BF16 && n_layers <= HTC_MAX_LAYERS && n_end - n_begin >= 1024 &&
@@ -360,8 +442,20 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
     sah_prof_end(SAH_PROF_HASH_ENCODE, st);
     return SAH_OK;
   }
-  const size_t smem = (size_t)(2 * HE_MAXD * HE_TK + HE_MAXD * HE_MAXD) * sizeof(float);
-  dim3 grid((unsigned)sah_ceil_div(n_end - n_begin, HE_TK), (unsigned)H_out, (unsigned)B);
+  // Weights beside the 66 KB of activations: all layers while they fit (128-128-128-32 does),
+  // else one region of the widest layer, staged layer by layer for every tile.
+  size_t w_all = 0, w_max = 0;
+  for (int l = 0; l < n_layers; ++l) {
+    const size_t w = (size_t)dims[l] * dims[l + 1] * sizeof(float);
+    w_all += w;
+    w_max = w > w_max ? w : w_max;
+  }
+  const size_t act_bytes = (size_t)HE_MAXD * HE_PITCH * sizeof(float);
+  p.resident = act_bytes + w_all <= 227 * 1024 ? 1 : 0;
+  const size_t smem = act_bytes + (p.resident ? w_all : w_max);
+  p.tiles_per_head = sah_ceil_div(n_end - n_begin, (int64_t)HE_TK);
+  p.tiles = p.tiles_per_head * H_out * B;
+  const unsigned grid = (unsigned)(p.tiles < 148 ? p.tiles : 148);
   sah_prof_begin(SAH_PROF_HASH_ENCODE, (cudaStream_t)stream);
   SAH_DISPATCH_DTYPE(dtype, T, {
     cudaError_t e = cudaFuncSetAttribute(hash_encode_kernel<T>,

@@ -457,3 +457,28 @@ def test_hash_signatures_from_tensor_cores_equal_the_fixed_order_kernel(hidden, 
     bias = [workloads.to_dtype(a, "bf16") for a in w["key_bias"]]
     ref = o_hash.signatures(o_attention.repeat_kv(k[:, :, :n], Hq // Hkv), mats, bias, act, "bf16")
     np.testing.assert_array_equal(whole[:, :, :n].cpu().numpy().view(np.uint32), ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,widths,n0,n,act", [
+    ("bf16", (128, 128, 128, 32), 0, 17, "silu"), ("bf16", (128, 128, 128, 32), 5, 128, "silu"),
+    ("bf16", (64, 32, 16), 3, 129, "relu"), ("bf16", (72, 16, 64, 128, 32), 0, 300, "tanh"),
+    ("bf16", (128, 128, 128, 128, 32), 0, 257, "gelu"), ("bf16", (128, 128, 128, 32), 0, 12000, "silu"),
+    ("f32", (128, 128, 128, 32), 1, 255, "silu"), ("f32", (8, 16), 0, 130, "relu")])
+def test_hash_signatures_of_tiles_equal_those_of_single_vectors(dtype, widths, n0, n, act):
+    """Ranges of more than 16 vectors go through tiles of 128 (weights of all layers resident in
+    shared memory, or layer by layer where they do not fit; several heads per CTA), shorter ones
+    one vector per CTA.  Both walk the channels in the same order: the same words, and words
+    outside the range untouched."""
+    torch.manual_seed(sum(widths) + n)
+    B, Hkv, Hq, S = 2, 2, 4, n0 + n + 3
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    k = torch.randn((B, S, Hkv, widths[0]), device=DEV).to(dt).transpose(1, 2)
+    weights = [(torch.randn((Hq, a, b), device=DEV) / a ** 0.5).to(dt) for a, b in zip(widths, widths[1:])]
+    biases = [(torch.randn((Hq, b), device=DEV) * 0.1).to(dt) for b in widths[1:]]
+    whole = torch.full((B, Hq, S + 5), -7, dtype=torch.int32, device=DEV)
+    single = whole.clone()
+    _native_ops.hash_encode(k, Hq, weights, biases, act, whole, n0, n0 + n)
+    for s0 in range(n0, n0 + n, 16):
+        _native_ops.hash_encode(k, Hq, weights, biases, act, single, s0, min(n0 + n, s0 + 16))
+    assert torch.equal(whole, single)
