@@ -363,10 +363,15 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
   if (!allowed) {
     e = cudaFuncSetAttribute(lsh_key_sign_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LtcCfg::SMEM);
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign_tc attr: %s", cudaGetErrorString(e));
+    e = cudaFuncSetAttribute(lsh_sign_recheck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LTC_RC_SMEM);
+    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_sign_recheck attr: %s", cudaGetErrorString(e));
     allowed = true;
   }
   if (sm_count <= 0) sm_count = 148;
-  const int chunks = (L * 8 + LTC_NCHUNK - 1) / LTC_NCHUNK;
+  // chunks of equal width: every CTA transforms as many keys and reads as many columns
+  int chunks = (L * 8 + LTC_NCHUNK - 1) / LTC_NCHUNK;
+  const int chunk_cols = ((L * 8 + chunks - 1) / chunks + 31) / 32 * 32;
+  chunks = (L * 8 + chunk_cols - 1) / chunk_cols;
   const int64_t BH = (int64_t)B * Hkv;
   const int64_t tiles = BH * ((s1 - s0 + LTC_TILE - 1) / LTC_TILE);
   int64_t workers = sm_count / chunks;
@@ -376,9 +381,9 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
   lsh_key_sign_tc_kernel<<<grid, LTC_THREADS, LtcCfg::SMEM, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(keys), ks_b, ks_h, ks_s, Hkv, BH, s0, s1,
       reinterpret_cast<const __nv_bfloat16*>(mean), norms, max_norm_bits, reinterpret_cast<const __nv_bfloat16*>(proj),
-      L, cap, reinterpret_cast<uint8_t*>(codes), list, list_cap, status, status + 1);
+      L, chunk_cols, cap, reinterpret_cast<uint8_t*>(codes), list, list_cap, status, status + 1);
   SAH_LAUNCH_CHECK("lsh_key_sign_tc");
-  lsh_sign_recheck_kernel<<<(unsigned)(sm_count * 4), 256, 0, st>>>(
+  lsh_sign_recheck_kernel<<<(unsigned)(sm_count * 3), LTC_RC_WARPS * 32, LTC_RC_SMEM, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(keys), ks_b, ks_h, ks_s, Hkv, reinterpret_cast<const __nv_bfloat16*>(mean),
       norms, max_norm_bits, reinterpret_cast<const __nv_bfloat16*>(proj), L, cap, reinterpret_cast<uint8_t*>(codes),
       list, list_cap, status);

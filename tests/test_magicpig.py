@@ -332,3 +332,50 @@ def test_gpu_signatures_from_tensor_cores_equal_the_fixed_order_kernel(L, S, cen
         k_np, None if m_np is None else m_np[:, :, None, :], "bf16"), "bf16"))
     codes = magicpig.key_codes(k_np, m_np, nk, M, proj.float().cpu().numpy(), L, K, "bf16")
     np.testing.assert_array_equal(got[:, :, :n, :L].cpu().numpy().astype(np.int64), codes)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,S,scale,centred,dup", [
+    (1, 1, 1.0, True, False), (2, 127, 1.0, False, False), (75, 129, 1.0, True, True), (300, 640, 1.0, True, False),
+    (33, 257, 5e-20, True, False), (75, 300, 3e17, False, False), (10, 500, 1.0, False, True)])
+def test_gpu_tensor_core_signatures_at_the_edges(L, S, scale, centred, dup):
+    """Ends of key tiles and column chunks; maximum norms for which the transform divides instead
+    of multiplying by the reciprocal; zero channels and hyperplanes orthogonal to every key (all
+    projections of a column redone, queues that overflow): the bytes of the fixed-order kernel."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, D, K, cap = 1, 3, 128, 8, S + 5
+    gen = torch.Generator(device=dev).manual_seed(S)
+    keys = (torch.randn((B, Hkv, cap, D), generator=gen, device=dev) * scale)
+    keys[..., 5:40:7] = 0.0
+    keys[:, :, ::3, 64] *= 2.0 ** -70
+    keys = keys.to(torch.bfloat16)[:, :, :S]
+    proj = torch.randn((D + 1, L * K), generator=gen, device=dev).to(torch.bfloat16)
+    if dup:  # columns whose projection is 0 for every key: all of them are redone
+        proj[:, 3] = 0.0
+    mean = keys.float().mean(dim=2).to(torch.bfloat16).contiguous() if centred else None
+    norms = torch.zeros((B, Hkv, cap), dtype=torch.float32, device=dev)
+    max_norm = torch.zeros(1, dtype=torch.int32, device=dev)
+    st = _native.stream_of(torch.device(dev))
+    kargs = (keys.data_ptr(), _native.SAH_BF16, keys.stride(0), keys.stride(1), keys.stride(2), B, Hkv)
+    _native.check(lib.sah_lsh_key_stats(*kargs, 0, S, D, _native.ptr(mean), cap, norms.data_ptr(),
+                                        max_norm.data_ptr(), 148, st), "sah_lsh_key_stats")
+    pitch = (L + 15) // 16 * 16
+    want = torch.full((B, Hkv, cap, pitch), 0xAA, dtype=torch.uint8, device=dev)
+    got = torch.full_like(want, 0x55)
+    _native.check(lib.sah_lsh_key_sign(*kargs, 0, S, D, _native.ptr(mean), norms.data_ptr(), max_norm.data_ptr(),
+                                       proj.data_ptr(), L, K, cap, want.data_ptr(), st), "sah_lsh_key_sign")
+    nbytes = int(lib.sah_lsh_key_sign_tc_ws_bytes(B, Hkv, S))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _native.check(lib.sah_lsh_key_sign_tc(keys.data_ptr(), keys.stride(0), keys.stride(1), keys.stride(2), B, Hkv,
+                                          0, S, D, _native.ptr(mean), norms.data_ptr(), max_norm.data_ptr(),
+                                          proj.data_ptr(), L, K, cap, got.data_ptr(), ws.data_ptr(), nbytes, 148,
+                                          st), "sah_lsh_key_sign_tc")
+    redone, err = ws[:8].view(torch.int32).tolist()
+    assert err == 0 and redone <= (nbytes - 16) // 16
+    assert not dup or redone >= B * Hkv * S
+    assert torch.equal(got[:, :, :S], want[:, :, :S])
+    assert bool((got[:, :, S:] == 0x55).all())
