@@ -5,18 +5,34 @@
 // The reference sorts the exp weights of a row (bf16 values), takes a running sum in sorted
 // order -- torch's CPU cumsum: one float32 accumulator, every prefix rounded to bf16 --
 // normalises by the last prefix and searches for top_p.  The threshold is a value of the
-// sorted list, so only sums at the ends of runs of equal values matter, and a bf16 weight in
-// (0, 1] is one of 16256 bit patterns: a histogram over bit patterns replaces the sort, and
-// one thread replays the accumulator over the non-empty bins from the largest value down.
-// Inside a run the accumulator moves by a constant amount while it stays in one binade (two
-// steps in after entering it, which also settles round-to-even ties), so the replay jumps to
-// the end of the binade instead of adding one by one; once an add no longer changes the
-// accumulator nothing smaller will, and the replay stops.
+// sorted list, so only sums at the ends of runs of equal values matter, and the weight is a
+// function of d = logit - maximum, a non-positive bf16 number: exp rounds to 1 for |d| < 2^-10
+// and to 0 from |d| = 128 on, which leaves 17 * 128 values of d.  A histogram over those replaces
+// the sort (and a comparison of d replaces the second look-up of the weight), and the accumulator
+// is replayed over the bins from the largest weight down.
+//
+// The replay runs in parallel, binade by binade of the accumulator.  Inside a binade of spacing u
+// the accumulator is an integer A times u, and an add of v = (k + f) u moves it by k or k + 1
+// whatever A is, unless f is exactly one half; then the sum goes to the even neighbour, so the
+// move depends on A's parity and every later add of the same v moves by the even one of k, k + 1.
+// A bin is therefore a function of A's parity (two moves), such functions compose, and a scan
+// over the bins gives every prefix up to the first one that reaches the next binade; that bin is
+// added by one thread, run by run, and the scan starts again behind it (about a dozen times).
+//
+// A row is shared by a cluster of up to eight CTAs where there are few rows.  What bounds the
+// kernel is the instruction issue of the three passes over the row (maximum, histogram, emit;
+// the row stays in L1/L2).  128 rows x 65536 keys: 186 us with scalar loads, two gathers of the
+// weight per key from global memory and the accumulator replayed by one thread; 62 us now.
+// ---------------------------------------------------------------------------
 #include "sah_common.cuh"
+#include <cooperative_groups.h>
 
 #define TP_THREADS 1024
-#define TP_BINS 16257            // bf16 bit patterns 0 .. 0x3F80 (0.0 .. 1.0)
-#define TP_WORDS ((TP_BINS + 31) / 32)
+#define TP_D0 0xBA80                 // bf16 bits of -2^-10: smaller magnitudes have weight 1
+#define TP_D1 0xC300                 // -128: weight 0 from here on
+#define TP_BINS (TP_D1 - TP_D0 + 2)  // bin 0: weight 1; bins 1 .. : d = TP_D0 ..; last bin: weight 0
+#define TP_PER 3                     // bins per thread
+#define TP_MAX_CLUSTER 8
 
 struct ToppArgs {
   const void* scores;      // [rows][S] unscaled q.k in bf16
@@ -71,17 +87,82 @@ __device__ __forceinline__ bool tp_add_run(float& acc, float v, unsigned int cou
   return true;
 }
 
+// bin of d = logit - maximum: ascending bins have descending weights.  A NaN (an infinite or NaN
+// logit) counts as weight 1.
+__device__ __forceinline__ int tp_bin(float d) {
+  const uint32_t b = __float_as_uint(d) >> 16;
+  if (b > 0xFF80u) return 0;
+  return min(max((int)b - (TP_D0 - 1), 0), TP_BINS - 1);
+}
+
+// 8 columns from column c0 of a row (zeros past the end); `vec`: rows are 16-byte aligned
+__device__ __forceinline__ void tp_load8(const __nv_bfloat16* __restrict__ s, int64_t c0, int64_t S, bool vec,
+                                         float* f) {
+  if (vec && c0 + 8 <= S) {
+    sah_unpack8(*reinterpret_cast<const uint4*>(s + c0), f);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = c0 + i < S ? __bfloat162float(s[c0 + i]) : 0.f;
+  }
+}
+
+// moves of A for the bin's adds by A's parity at entry, clamped to TP_FAR (past any binade)
+#define TP_FAR (1u << 25)
+struct TpMove {
+  unsigned int d0, d1;
+};
+__device__ __forceinline__ TpMove tp_then(const TpMove& f, const TpMove& g) {
+  TpMove r;
+  r.d0 = min(f.d0 + ((f.d0 & 1u) ? g.d1 : g.d0), TP_FAR);
+  r.d1 = min(f.d1 + ((f.d1 & 1u) ? g.d0 : g.d1), TP_FAR);
+  return r;
+}
+// `count` adds of the positive bf16 value with bits `vb` to an accumulator whose binade has
+// exponent field `ea` (spacing 2^(ea - 150))
+__device__ __forceinline__ TpMove tp_move(unsigned int vb, unsigned int count, int ea) {
+  int ev = (int)(vb >> 7);
+  unsigned int m = vb & 127u;
+  if (ev) m |= 128u; else ev = 1;   // v = m * 2^(ev - 134)
+  const int sh = ea - 16 - ev;      // v / u = m * 2^-sh
+  unsigned int k, first1, step;
+  if (sh <= 0) {
+    k = m << -sh;                   // v is not above the accumulator, so at most 2^24
+    first1 = step = k;
+  } else if (sh > 8) {
+    k = first1 = step = 0u;         // below half a spacing
+  } else {
+    k = m >> sh;
+    const unsigned int rem = m & ((1u << sh) - 1u), half = 1u << (sh - 1);
+    if (rem == half) {
+      step = k + (k & 1u);          // from an even A to an even A
+      first1 = k + 1u - (k & 1u);   // from an odd A to an even A
+    } else {
+      if (rem > half) ++k;
+      first1 = step = k;
+    }
+  }
+  const unsigned long long rest = (unsigned long long)(count - 1u) * step;
+  TpMove r;
+  r.d0 = (unsigned int)min(rest + step, (unsigned long long)TP_FAR);
+  r.d1 = (unsigned int)min(rest + first1, (unsigned long long)TP_FAR);
+  return r;
+}
+
 __global__ void __launch_bounds__(TP_THREADS)
 topp_select_kernel(ToppArgs a) {
   sah_pdl_entry();
-  extern __shared__ unsigned int tp_hist[];   // [TP_BINS] counts, then the run-end sums
-  __shared__ unsigned int nz[TP_WORDS];       // non-empty bins
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ unsigned int hist[TP_PER * TP_THREADS];  // this CTA's counts; in rank 0 the row's
+  __shared__ uint16_t weight[TP_PER * TP_THREADS];    // bf16 bits of exp(d) by bin
   __shared__ float scratch[32];
-  __shared__ float total_sm;
-  __shared__ int stop_sm;                     // bins below it were not replayed: sum = total
-  __shared__ int pick_sm, low_sm;
-  const int tid = threadIdx.x;
-  const int64_t row = blockIdx.x;
+  __shared__ uint2 warp_move[32];
+  __shared__ float max_sm;                            // this CTA's maximum
+  __shared__ float acc_sm;
+  __shared__ int cross_sm, pick_sm, last_sm, thr_sm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int64_t row = blockIdx.x / ranks;
   const int qi = (int)(row % a.Sq);
   const int64_t bh = row / a.Sq;
   const int h = (int)(bh % a.Hq);
@@ -91,87 +172,222 @@ topp_select_kernel(ToppArgs a) {
   const T* bias = a.bias ? reinterpret_cast<const T*>(a.bias) + b * a.bias_s_b + h * a.bias_s_h +
                                qi * a.bias_s_q
                          : nullptr;
-  const uint32_t* pb = a.prev_bits + row * a.W;
+  const bool vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
+  const bool bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
+  const unsigned char* pb = reinterpret_cast<const unsigned char*>(a.prev_bits + row * a.W);
   const float lowest = __uint_as_float(0xFF7F0000u);   // the most negative finite bf16
 
-  // scaled logit, previously active positions pushed to the lowest value (:96-104)
-  auto logit = [&](int64_t j) {
-    if ((pb[j >> 5] >> (j & 31)) & 1u) return lowest;
-    float t = sah_round_to<T>(__fmul_rn(sah_to_float<T>(s[j]), a.scaling));
-    if (bias) t = sah_round_to<T>(__fadd_rn(t, sah_to_float<T>(bias[j])));
-    return t;
+  // the row in bytes of the bitmap, 8 columns each, cut into one range per CTA of the cluster
+  const int64_t nb = a.W * 4;
+  const int64_t b_lo = nb * rank / ranks, b_hi = nb * (rank + 1) / ranks;
+
+  // scaled logits of a byte's columns, previously active positions pushed to the lowest value
+  // (:96-104)
+  auto logits = [&](int64_t byte, float* f) {
+    const int64_t c0 = byte * 8;
+    tp_load8(s, c0, a.S, vec, f);
+    const unsigned int act = pb[byte];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = sah_round_to<T>(__fmul_rn(f[i], a.scaling));
+    if (bias) {
+      float bv[8];
+      tp_load8(bias, c0, a.S, bias_vec, bv);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = sah_round_to<T>(__fadd_rn(f[i], bv[i]));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = (act >> i) & 1u ? lowest : f[i];
   };
-  for (int i = tid; i < TP_BINS; i += TP_THREADS) tp_hist[i] = 0u;
-  for (int i = tid; i < TP_WORDS; i += TP_THREADS) nz[i] = 0u;
-  if (tid == 0) { pick_sm = -1; low_sm = TP_BINS; stop_sm = 0; }
+
+  for (int i = tid; i < TP_PER * TP_THREADS; i += TP_THREADS) {
+    hist[i] = 0u;
+    // bin 0 has weight 1, the last bin 0 (and everything past it)
+    const unsigned int e = i == 0 ? 0x3F80u : i >= TP_BINS - 1 ? 0u : a.exp_table[TP_D0 - 1 + i];
+    weight[i] = (uint16_t)min(e, 0x3F80u);
+  }
 
   float mx = -INFINITY;
-  for (int64_t j = tid; j < a.S; j += TP_THREADS) mx = fmaxf(mx, logit(j));
+  for (int64_t y = b_lo + tid; y < b_hi; y += TP_THREADS) {
+    if (y * 8 >= a.S) break;
+    float f[8];
+    logits(y, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (y * 8 + i < a.S) mx = fmaxf(mx, f[i]);
+  }
   mx = tp_block_max(mx, scratch);
-  auto weight_bits = [&](int64_t j) {   // bf16 bits of exp(logit - max), 0 .. 0x3F80
-    const float d = sah_round_to<T>(__fsub_rn(logit(j), mx));
-    unsigned int e = a.exp_table[__float_as_uint(d) >> 16];
-    return e > 0x3F80u ? 0x3F80u : e;   // not reached for finite logits
-  };
+  if (ranks > 1) {
+    if (tid == 0) max_sm = mx;
+    cluster.sync();
+    for (int r = 0; r < ranks; ++r) mx = fmaxf(mx, *cluster.map_shared_rank(&max_sm, r));
+  }
 
-  // histogram over bit patterns
-  for (int64_t j = tid; j < a.S; j += TP_THREADS) atomicAdd(&tp_hist[weight_bits(j)], 1u);
+  // histogram over d
+  for (int64_t y = b_lo + tid; y < b_hi; y += TP_THREADS) {
+    if (y * 8 >= a.S) break;
+    float f[8];
+    logits(y, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (y * 8 + i < a.S) atomicAdd(&hist[tp_bin(sah_round_to<T>(__fsub_rn(f[i], mx)))], 1u);
+  }
   __syncthreads();
-  for (int i = tid; i < TP_BINS; i += TP_THREADS)
-    if (i > 0 && tp_hist[i] != 0u) atomicOr(&nz[i >> 5], 1u << (i & 31));
-  __syncthreads();
+  if (ranks > 1) {
+    cluster.sync();
+    if (rank != 0) {
+      unsigned int* h0 = cluster.map_shared_rank(hist, 0);
+      for (int i = tid; i < TP_BINS; i += TP_THREADS)
+        if (hist[i] != 0u) atomicAdd(&h0[i], hist[i]);
+    }
+    cluster.sync();
+  }
 
-  // replay of the accumulator, largest value first
-  if (tid == 0) {
-    float acc = 0.f;
-    bool alive = true;
-    int stop = 0;
-    for (int wi = TP_WORDS - 1; wi >= 0 && alive; --wi) {
-      unsigned int m = nz[wi];
-      while (m) {
-        const int bit = 31 - __clz(m);
-        m &= ~(1u << bit);
-        const int bin = wi * 32 + bit;
-        alive = tp_add_run(acc, __uint_as_float((unsigned int)bin << 16), tp_hist[bin]);
-        tp_hist[bin] = __float_as_uint(acc);
-        if (!alive) { stop = bin; break; }
+  if (rank == 0) {
+    // replay of the accumulator, largest weight first; thread t holds bins 3 t .. 3 t + 2
+    unsigned int cnt[TP_PER], val[TP_PER];
+    float sum[TP_PER];
+    int last = -1;
+#pragma unroll
+    for (int i = 0; i < TP_PER; ++i) {
+      const int bin = tid * TP_PER + i;
+      val[i] = weight[bin];
+      cnt[i] = val[i] ? hist[bin] : 0u;
+      sum[i] = 0.f;
+      if (cnt[i]) last = bin;
+    }
+    if (tid == 0) { acc_sm = 0.f; pick_sm = -1; last_sm = -1; thr_sm = -1; }
+    int pos = 0;   // bins before it are done
+    for (;;) {
+      if (tid == 0) cross_sm = TP_BINS;
+      __syncthreads();
+      const float acc = acc_sm;
+      const int ea = (int)(__float_as_uint(acc) >> 23);
+      unsigned int A = (__float_as_uint(acc) & 0x7FFFFFu) | 0x800000u;
+      TpMove mv[TP_PER], all;
+      all.d0 = all.d1 = 0u;
+      if (acc > 0.f) {
+#pragma unroll
+        for (int i = 0; i < TP_PER; ++i) {
+          mv[i].d0 = mv[i].d1 = 0u;
+          if (cnt[i] && tid * TP_PER + i >= pos) mv[i] = tp_move(val[i], cnt[i], ea);
+          all = tp_then(all, mv[i]);
+        }
+        // exclusive scan over the threads
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          TpMove left;
+          left.d0 = __shfl_up_sync(0xffffffffu, all.d0, o);
+          left.d1 = __shfl_up_sync(0xffffffffu, all.d1, o);
+          if (lane >= o) all = tp_then(left, all);
+        }
+        if (lane == 31) warp_move[warp] = make_uint2(all.d0, all.d1);
+        TpMove ex;
+        ex.d0 = __shfl_up_sync(0xffffffffu, all.d0, 1);
+        ex.d1 = __shfl_up_sync(0xffffffffu, all.d1, 1);
+        if (lane == 0) ex.d0 = ex.d1 = 0u;
+        __syncthreads();
+        TpMove w;
+        w.d0 = warp_move[lane].x;
+        w.d1 = warp_move[lane].y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          TpMove left;
+          left.d0 = __shfl_up_sync(0xffffffffu, w.d0, o);
+          left.d1 = __shfl_up_sync(0xffffffffu, w.d1, o);
+          if (lane >= o) w = tp_then(left, w);
+        }
+        TpMove before;
+        before.d0 = __shfl_sync(0xffffffffu, w.d0, (warp + 31) & 31);
+        before.d1 = __shfl_sync(0xffffffffu, w.d1, (warp + 31) & 31);
+        if (warp == 0) before.d0 = before.d1 = 0u;
+        before = tp_then(before, ex);
+        A += (A & 1u) ? before.d1 : before.d0;
       }
+      // own bins: a prefix below the next binade is final, the first that reaches it is added
+      // run by run below
+      float entry = acc;
+      int mine = TP_BINS;
+#pragma unroll
+      for (int i = 0; i < TP_PER; ++i) {
+        const int bin = tid * TP_PER + i;
+        if (mine == TP_BINS && cnt[i] && bin >= pos) {
+          const unsigned int next = acc > 0.f ? A + ((A & 1u) ? mv[i].d1 : mv[i].d0) : TP_FAR;
+          if (A < (1u << 24)) entry = acc > 0.f ? __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu)) : 0.f;
+          if (next < (1u << 24)) {
+            A = next;
+            sum[i] = __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu));
+          } else {
+            mine = bin;
+          }
+        }
+      }
+      if (mine < TP_BINS) atomicMin(&cross_sm, mine);
+      if (tid == TP_THREADS - 1 && mine == TP_BINS && acc > 0.f && A < (1u << 24))
+        acc_sm = __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu));  // no crossing at all: the total
+      __syncthreads();
+      const int cross = cross_sm;
+      if (cross == TP_BINS) break;
+      if (mine == cross) {
+#pragma unroll
+        for (int i = 0; i < TP_PER; ++i)
+          if (tid * TP_PER + i == cross) {
+            tp_add_run(entry, __uint_as_float(val[i] << 16), cnt[i]);
+            sum[i] = entry;
+          }
+        acc_sm = entry;
+      }
+      pos = cross + 1;
+      __syncthreads();
     }
-    total_sm = sah_round_to<T>(acc);
-    stop_sm = stop;
-  }
-  __syncthreads();
 
-  // first run (largest value) whose normalised prefix exceeds top_p (:118-131)
-  const float total = total_sm;
-  const float p = sah_round_to<T>(a.top_p);
-  const int stop = stop_sm;
-  int best = -1, low = TP_BINS;
-  for (int i = tid; i < TP_BINS; i += TP_THREADS) {
-    if (i == 0 || !((nz[i >> 5] >> (i & 31)) & 1u)) continue;
-    low = min(low, i);
-    const float sum = (i < stop) ? total : sah_round_to<T>(__uint_as_float(tp_hist[i]));
-    const float ratio = sah_round_to<T>(__fdiv_rn(sum, total));
-    if (ratio > p) best = max(best, i);
+    // first run (largest value) whose normalised prefix exceeds top_p (:118-131)
+    const float total = sah_round_to<T>(acc_sm);
+    const float p = sah_round_to<T>(a.top_p);
+    int best = TP_BINS;
+#pragma unroll
+    for (int i = TP_PER - 1; i >= 0; --i)
+      if (cnt[i] && sah_round_to<T>(__fdiv_rn(sah_round_to<T>(sum[i]), total)) > p) best = tid * TP_PER + i;
+    if (tid == 0) cross_sm = TP_BINS;
+    __syncthreads();
+    if (best < TP_BINS) atomicMin(&cross_sm, best);
+    if (last >= 0) atomicMax(&last_sm, last);
+    // weight 0 among the keys: bins whose weight is 0
+#pragma unroll
+    for (int i = 0; i < TP_PER; ++i)
+      if (val[i] == 0u && hist[tid * TP_PER + i] != 0u) pick_sm = 1;
+    __syncthreads();
+    // nothing exceeds top_p: the search position is clamped to the last sorted element (:127-130)
+    unsigned int thr;
+    if (cross_sm < TP_BINS) thr = weight[cross_sm];
+    else thr = (pick_sm > 0 || last_sm < 0) ? 0u : weight[last_sm];
+    // the last bin that is selected (weight >= threshold, :158-160)
+    int keep = -1;
+#pragma unroll
+    for (int i = 0; i < TP_PER; ++i)
+      if (tid * TP_PER + i < TP_BINS && val[i] >= thr) keep = tid * TP_PER + i;
+    if (keep >= 0) atomicMax(&thr_sm, keep);
+    __syncthreads();
   }
-  atomicMax(&pick_sm, best);
-  atomicMin(&low_sm, low);
-  __syncthreads();
-  // nothing exceeds top_p: the search position is clamped to the last sorted element (:127-130)
-  unsigned int thr;
-  if (pick_sm >= 0) thr = (unsigned int)pick_sm;
-  else thr = (tp_hist[0] != 0u || low_sm >= TP_BINS) ? 0u : (unsigned int)low_sm;
+  int last_bin;
+  if (ranks > 1) {
+    cluster.sync();
+    last_bin = *cluster.map_shared_rank(&thr_sm, 0);
+    cluster.sync();  // rank 0 may not leave while its threshold is being read
+  } else {
+    last_bin = thr_sm;
+  }
 
-  // emit: weight >= threshold (:158-160)
-  uint32_t* out = a.out_bits + row * a.W;
-  for (int64_t w = tid; w < a.W; w += TP_THREADS) {
-    uint32_t bits = 0u;
-    const int64_t c0 = w * 32;
-    for (int i = 0; i < 32; ++i) {
-      const int64_t j = c0 + i;
-      if (j < a.S && weight_bits(j) >= thr) bits |= 1u << i;
+  unsigned char* out = reinterpret_cast<unsigned char*>(a.out_bits + row * a.W);
+  for (int64_t y = b_lo + tid; y < b_hi; y += TP_THREADS) {
+    unsigned int bits = 0u;
+    if (y * 8 < a.S) {
+      float f[8];
+      logits(y, f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (y * 8 + i < a.S && tp_bin(sah_round_to<T>(__fsub_rn(f[i], mx))) <= last_bin) bits |= 1u << i;
     }
-    out[w] = a.or_prev ? (bits | pb[w]) : bits;
+    out[y] = (unsigned char)(a.or_prev ? (bits | pb[y]) : bits);
   }
 }
 
@@ -194,11 +410,23 @@ extern "C" int sah_topp_select(const void* scores, int dtype, float scaling, con
   a.or_prev = or_prev; a.exp_table = exp_table; a.out_bits = out_bits;
   const int64_t rows = (int64_t)B * Hq * Sq;
   SAH_REQUIRE(rows <= 2147483647, "topp_select: too many rows");
-  const int smem = TP_BINS * (int)sizeof(unsigned int);
-  cudaError_t e = cudaFuncSetAttribute(topp_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "topp_select attr: %s", cudaGetErrorString(e));
+  // Few rows: several CTAs per row (a power of two, so that the bitmap bytes split evenly), as
+  // long as one wave of 148 holds them all and each still has a pass of 8 columns per thread.
+  int ranks = 1;
+  while (ranks < TP_MAX_CLUSTER && rows * ranks * 2 <= 148 && S >= (int64_t)ranks * 2 * 8 * TP_THREADS) ranks *= 2;
   sah_prof_begin(SAH_PROF_TOPP, (cudaStream_t)stream);
-  sah_launch_chain(topp_select_kernel, (unsigned)rows, TP_THREADS, smem, (cudaStream_t)stream, a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(rows * ranks));
+  cfg.blockDim = dim3(TP_THREADS);
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, topp_select_kernel, a);  // the error stays for SAH_LAUNCH_CHECK
   SAH_LAUNCH_CHECK("topp_select");
   sah_prof_end(SAH_PROF_TOPP, (cudaStream_t)stream);
   return SAH_OK;

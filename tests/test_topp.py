@@ -196,3 +196,26 @@ def test_restatement_three_query_positions_under_a_causal_mask():
     np.testing.assert_array_equal(ptr, g["ptr"])
     np.testing.assert_array_equal(data, g["data"])
     np.testing.assert_allclose(out, g["out"], atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,S,spread,top_p,masked", [
+    (1, 131072, 25.0, 0.9, False), (2, 70001, 60.0, 0.999, True), (20, 16384, 4.0, 0.7, False),
+    (75, 2040, 300.0, 0.5, True), (150, 1031, 25.0, 0.95, True), (3, 40, 900.0, 0.9, False)])
+def test_gpu_rows_shared_by_clusters_and_ragged_rows(rows, S, spread, top_p, masked):
+    """Rows cut between 8, 4, 2 and 1 CTAs; lengths that end inside a bitmap byte (no 16-byte
+    loads); flat rows (every add near a tie of the accumulator) and steep ones (weights down to
+    the denormals and 0); additive masks with the lowest value and -inf."""
+    from oracle.bf16 import round_bf16
+
+    rng = np.random.default_rng(S)
+    sc = round_bf16(rng.normal(0.0, spread, (1, rows, 1, S)).astype(np.float32)).astype(np.float32)
+    prev = rng.random(sc.shape) < 0.01
+    am = None
+    if masked:
+        am = np.zeros((1, 1, 1, S), np.float32)
+        am[..., S // 2:S // 2 + 37] = round_bf16(np.float32(-3.3895e38))
+        am[..., 3] = -np.inf
+    scaling = 0.08838834764831845
+    want = topp.select(sc, scaling, am, prev, top_p) | prev
+    np.testing.assert_array_equal(_native_select(sc, am, scaling, prev, top_p), want)
