@@ -48,7 +48,15 @@ __global__ void lsh_key_sums_kernel(const T* __restrict__ k, int64_t ks_b, int64
   const T* base = k + b * ks_b + h * ks_h;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     double acc = 0.0;
-    for (int64_t s = lo; s < hi; ++s) acc += (double)sah_to_float<T>(base[s * ks_s + d]);
+    int64_t s = lo;
+    for (; s + 16 <= hi; s += 16) {  // sixteen rows in flight; one at a time took 111 us for 8 x 65500 keys
+      T x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x[i] = base[(s + i) * ks_s + d];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) acc += (double)sah_to_float<T>(x[i]);
+    }
+    for (; s < hi; ++s) acc += (double)sah_to_float<T>(base[s * ks_s + d]);
     atomicAdd(&sums[bh * D + d], acc);
   }
 }
@@ -166,6 +174,83 @@ __device__ __forceinline__ float lsh_augment(float nk, float M) {
 // ---------------------------------------------------------------------------------------
 #define LSH_KT 64  // keys per CTA tile
 
+// Hyperplane columns [c0, c0 + nc) of all Dp channels into shared memory [Dp][LSH_COLS], every
+// copy requested before the first is waited for (no wait in here).
+#define LSH_COLS 64
+#define LSH_COLS_THREADS 128
+template <typename T>
+__device__ __forceinline__ void lsh_stage_columns(const T* __restrict__ proj, int nbits, int Dp, int c0, int nc,
+                                                  T* __restrict__ sm) {
+  constexpr int PER = 16 / (int)sizeof(T);
+  if ((reinterpret_cast<uintptr_t>(proj) & 15) == 0 && nbits % PER == 0 && c0 % PER == 0 && nc % PER == 0) {
+    const int cpr = nc / PER;
+    for (int i = threadIdx.x; i < Dp * cpr; i += LSH_COLS_THREADS) {
+      const int ch = i / cpr, c = (i - ch * cpr) * PER;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(sm + ch * LSH_COLS + c)),
+                   "l"(proj + (int64_t)ch * nbits + c0 + c)
+                   : "memory");
+    }
+  } else {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < Dp * nc; i += LSH_COLS_THREADS) {
+      const int ch = i / nc, c = i - ch * nc;
+      sm[ch * LSH_COLS + c] = proj[(int64_t)ch * nbits + c0 + c];
+    }
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// The keys that a decode step appends: a CTA takes one key and LSH_COLS / K tables, so that the
+// hyperplanes (155 KB for 75 tables of 8 bits) are fetched by many SMs at once and every value is
+// on its way before the first is used; then one thread per column adds up the channels in order.
+// Latency is all there is: 8 heads x 1 key took 25 us with one CTA per head, 4.5 us now.
+#define LSH_FEW_KEYS 4
+template <typename T, typename CodeT>
+__global__ void __launch_bounds__(LSH_COLS_THREADS)
+lsh_key_sign_few_kernel(const T* __restrict__ k, int64_t ks_b, int64_t ks_h, int64_t ks_s, int Hkv,
+                        int64_t s0, int D, const T* __restrict__ mean, const float* __restrict__ norms,
+                        const unsigned int* __restrict__ max_bits, const T* __restrict__ proj, int L, int K,
+                        int64_t cap, CodeT* __restrict__ codes) {
+  sah_pdl_entry_early();
+  extern __shared__ __align__(16) unsigned char lsh_smem[];
+  const int nbits = L * K, Dp = D + 1;
+  T* pr = reinterpret_cast<T*>(lsh_smem);                                         // [Dp][LSH_COLS]
+  float* xt = reinterpret_cast<float*>(lsh_smem + (size_t)Dp * LSH_COLS * sizeof(T));  // [Dp]
+  unsigned char* sb = reinterpret_cast<unsigned char*>(xt + Dp);                  // [LSH_COLS]
+  const int tables = LSH_COLS / K, l0 = blockIdx.x * tables;
+  const int lt = L - l0 < tables ? L - l0 : tables;
+  lsh_stage_columns<T>(proj, nbits, Dp, l0 * K, lt * K, pr);
+  const int64_t bh = blockIdx.y, s = s0 + blockIdx.z;
+  const T* kr = k + bh / Hkv * ks_b + bh % Hkv * ks_h + s * ks_s;
+  const float M = __uint_as_float(*max_bits);
+  for (int c = threadIdx.x; c < D; c += LSH_COLS_THREADS) {
+    const float x = sah_to_float<T>(kr[c]);
+    const float cx = mean ? sah_round_to<T>(__fsub_rn(x, sah_to_float<T>(mean[bh * D + c]))) : x;
+    xt[c] = sah_round_to<T>(__fdiv_rn(cx, M));
+  }
+  if (threadIdx.x == 0) xt[D] = lsh_augment<T>(norms[bh * cap + s], M);
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < lt * K) {
+    float acc = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < Dp; ++c)
+      acc = __fadd_rn(acc, __fmul_rn(xt[c], sah_to_float<T>(pr[c * LSH_COLS + threadIdx.x])));
+    sb[threadIdx.x] = acc > 0.f ? 1 : 0;
+  }
+  __syncthreads();
+  // bit j of table l is column l * K + j; the last CTA also writes the zero padding of the row
+  const int LP = lsh_row_pitch<CodeT>(L);
+  const int end = blockIdx.x == gridDim.x - 1 ? LP : l0 + lt;
+  for (int l = l0 + threadIdx.x; l < end; l += LSH_COLS_THREADS) {
+    unsigned int code = 0;
+    if (l < L)
+      for (int j = 0; j < K; ++j) code |= (unsigned int)sb[(l - l0) * K + j] << j;
+    codes[(bh * cap + s) * LP + l] = (CodeT)code;
+  }
+}
+
 template <typename T, typename CodeT>
 __global__ void __launch_bounds__(256)
 lsh_key_sign_kernel(const T* __restrict__ k, int64_t ks_b, int64_t ks_h, int64_t ks_s, int Hkv,
@@ -208,71 +293,28 @@ lsh_key_sign_kernel(const T* __restrict__ k, int64_t ks_b, int64_t ks_h, int64_t
 
   // one output column per thread, 8 keys at a time; single accumulator per (key, column),
   // channels ascending (products of dtype values, added in float)
-  // keys of this tile that exist (a decode step appends one key: one pass of eight, not eight)
+  // keys of this tile that exist
   const int kt_used = (int)((s1 - t0 < LSH_KT ? s1 - t0 : LSH_KT) + 7) & ~7;
-  if (s1 - t0 == 1) {
-    // The key that a decode step appends: up to three columns per thread and the hyperplane
-    // values of 8 channels x 3 columns requested before the first is used, so that a thread
-    // waits for memory 17 times instead of 129 x 3 (that chain made this launch 66 us, all of
-    // it load latency).  Same order of additions per column.  The body is kept small on
-    // purpose: a decode step runs with cold caches, the instruction cache included, and a
-    // fully unrolled 16-channel body measured slower (106 us) than the plain loop.
-    constexpr int CB = 8, OC = 3;
-    for (int o0 = threadIdx.x; o0 < nbits; o0 += 256 * OC) {
-      const bool has1 = o0 + 256 < nbits, has2 = o0 + 512 < nbits;
-      float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f;
-      const T* pp = proj + o0;
-#pragma unroll 1
-      for (int c0 = 0; c0 + CB <= Dp; c0 += CB) {
-        float p0[CB], p1[CB], p2[CB];
+  for (int o = threadIdx.x; o < nbits; o += 256) {
+    for (int k8 = 0; k8 < kt_used; k8 += 8) {
+      float acc[8];
 #pragma unroll
-        for (int i = 0; i < CB; ++i) {
-          const T* q = pp + (int64_t)(c0 + i) * nbits;
-          p0[i] = sah_to_float<T>(q[0]);
-          p1[i] = has1 ? sah_to_float<T>(q[256]) : 0.f;
-          p2[i] = has2 ? sah_to_float<T>(q[512]) : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < CB; ++i) {
-          const float a = xt[(c0 + i) * LSH_KT];
-          acc0 = __fadd_rn(acc0, __fmul_rn(a, p0[i]));
-          acc1 = __fadd_rn(acc1, __fmul_rn(a, p1[i]));
-          acc2 = __fadd_rn(acc2, __fmul_rn(a, p2[i]));
-        }
+      for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+      for (int c = 0; c < Dp; ++c) {
+        const float p = sah_to_float<T>(proj[(int64_t)c * nbits + o]);
+        const float4 a = *reinterpret_cast<const float4*>(xt + c * LSH_KT + k8);
+        const float4 bq = *reinterpret_cast<const float4*>(xt + c * LSH_KT + k8 + 4);
+        acc[0] = __fadd_rn(acc[0], __fmul_rn(a.x, p));
+        acc[1] = __fadd_rn(acc[1], __fmul_rn(a.y, p));
+        acc[2] = __fadd_rn(acc[2], __fmul_rn(a.z, p));
+        acc[3] = __fadd_rn(acc[3], __fmul_rn(a.w, p));
+        acc[4] = __fadd_rn(acc[4], __fmul_rn(bq.x, p));
+        acc[5] = __fadd_rn(acc[5], __fmul_rn(bq.y, p));
+        acc[6] = __fadd_rn(acc[6], __fmul_rn(bq.z, p));
+        acc[7] = __fadd_rn(acc[7], __fmul_rn(bq.w, p));
       }
-      for (int c = Dp / CB * CB; c < Dp; ++c) {  // the channels left over (the augmented one)
-        const T* q = pp + (int64_t)c * nbits;
-        const float a = xt[c * LSH_KT];
-        acc0 = __fadd_rn(acc0, __fmul_rn(a, sah_to_float<T>(q[0])));
-        if (has1) acc1 = __fadd_rn(acc1, __fmul_rn(a, sah_to_float<T>(q[256])));
-        if (has2) acc2 = __fadd_rn(acc2, __fmul_rn(a, sah_to_float<T>(q[512])));
-      }
-      sb[o0] = acc0 > 0.f ? 1 : 0;
-      if (has1) sb[o0 + 256] = acc1 > 0.f ? 1 : 0;
-      if (has2) sb[o0 + 512] = acc2 > 0.f ? 1 : 0;
-    }
-  } else {
-    for (int o = threadIdx.x; o < nbits; o += 256) {
-      for (int k8 = 0; k8 < kt_used; k8 += 8) {
-        float acc[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-        for (int c = 0; c < Dp; ++c) {
-          const float p = sah_to_float<T>(proj[(int64_t)c * nbits + o]);
-          const float4 a = *reinterpret_cast<const float4*>(xt + c * LSH_KT + k8);
-          const float4 bq = *reinterpret_cast<const float4*>(xt + c * LSH_KT + k8 + 4);
-          acc[0] = __fadd_rn(acc[0], __fmul_rn(a.x, p));
-          acc[1] = __fadd_rn(acc[1], __fmul_rn(a.y, p));
-          acc[2] = __fadd_rn(acc[2], __fmul_rn(a.z, p));
-          acc[3] = __fadd_rn(acc[3], __fmul_rn(a.w, p));
-          acc[4] = __fadd_rn(acc[4], __fmul_rn(bq.x, p));
-          acc[5] = __fadd_rn(acc[5], __fmul_rn(bq.y, p));
-          acc[6] = __fadd_rn(acc[6], __fmul_rn(bq.z, p));
-          acc[7] = __fadd_rn(acc[7], __fmul_rn(bq.w, p));
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sb[(k8 + j) * nbits + o] = acc[j] > 0.f ? 1 : 0;
-      }
+      for (int j = 0; j < 8; ++j) sb[(k8 + j) * nbits + o] = acc[j] > 0.f ? 1 : 0;
     }
   }
   __syncthreads();
@@ -306,6 +348,29 @@ extern "C" int sah_lsh_key_sign(const void* keys, int dtype, int64_t ks_b, int64
     return sah_fail(SAH_ERR_UNSUPPORTED, "lsh_key_sign: %d x %d signature bits exceed shared memory", L, K);
   dim3 grid((unsigned)((s1 - s0 + LSH_KT - 1) / LSH_KT), (unsigned)(B * Hkv));
   cudaStream_t st = (cudaStream_t)stream;
+  if (s1 - s0 <= LSH_FEW_KEYS) {
+    const int tables = LSH_COLS / K;
+    dim3 fgrid((unsigned)((L + tables - 1) / tables), (unsigned)(B * Hkv), (unsigned)(s1 - s0));
+#define LSH_FEW_LAUNCH(T, CodeT)                                                                   \
+  do {                                                                                             \
+    const int bytes = (D + 1) * (LSH_COLS * (int)sizeof(T) + 4) + LSH_COLS;                        \
+    if (bytes > 48 * 1024) {                                                                       \
+      cudaError_t e = cudaFuncSetAttribute(lsh_key_sign_few_kernel<T, CodeT>,                      \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);    \
+      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign attr: %s", cudaGetErrorString(e)); \
+    }                                                                                              \
+    sah_launch_chain(lsh_key_sign_few_kernel<T, CodeT>, fgrid, LSH_COLS_THREADS, bytes, st, \
+        reinterpret_cast<const T*>(keys), ks_b, ks_h, ks_s, Hkv, s0, D,                            \
+        reinterpret_cast<const T*>(mean), norms, max_norm_bits, reinterpret_cast<const T*>(proj),  \
+        L, K, cap, reinterpret_cast<CodeT*>(codes));                                               \
+  } while (0)
+    SAH_DISPATCH_DTYPE(dtype, T, {
+      if (K <= 8) LSH_FEW_LAUNCH(T, uint8_t); else LSH_FEW_LAUNCH(T, uint16_t);
+    });
+#undef LSH_FEW_LAUNCH
+    SAH_LAUNCH_CHECK("lsh_key_sign_few");
+    return SAH_OK;
+  }
 #define LSH_SIGN_LAUNCH(T, CodeT)                                                                  \
   do {                                                                                             \
     cudaError_t e = cudaFuncSetAttribute(lsh_key_sign_kernel<T, CodeT>,                            \
@@ -394,17 +459,27 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
 // ---------------------------------------------------------------------------------------
 // query: centre, normalise, signatures, unit vector
 // ---------------------------------------------------------------------------------------
+// A CTA takes one query row and LSH_COLS / K tables: the hyperplanes are requested at once, the
+// first warp normalises the query meanwhile (every CTA of the row does; the first one writes it
+// out), then one thread per column adds up the channels in order.  This kernel sits on the
+// critical path of every decode step and is all latency: 32 rows took 12.5 us with one CTA per
+// row, 7.7 us now.
 template <typename T, typename CodeT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(LSH_COLS_THREADS)
 lsh_query_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs_q, int Hq, int Sq,
                  int G, int D, const T* __restrict__ mean, const T* __restrict__ proj, int L, int K,
                  CodeT* __restrict__ qcodes, float* __restrict__ qunit, T* __restrict__ qhat,
                  float* __restrict__ qmu) {
   sah_pdl_entry_early();
   extern __shared__ __align__(16) unsigned char lsh_smem[];
-  float* qn = reinterpret_cast<float*>(lsh_smem);                 // [D] normalised query
-  unsigned char* sb = lsh_smem + (size_t)D * sizeof(float);       // [L*K]
-  const int nbits = L * K;
+  const int nbits = L * K, Dp = D + 1;
+  T* pr = reinterpret_cast<T*>(lsh_smem);                                         // [Dp][LSH_COLS]
+  float* qn = reinterpret_cast<float*>(lsh_smem + (size_t)Dp * LSH_COLS * sizeof(T));  // [D] normalised query
+  unsigned char* sb = reinterpret_cast<unsigned char*>(qn + D);                   // [LSH_COLS]
+  const int tables = LSH_COLS / K, l0 = blockIdx.y * tables;
+  const int lt = L - l0 < tables ? L - l0 : tables;
+  lsh_stage_columns<T>(proj, nbits, Dp, l0 * K, lt * K, pr);
+  const bool writer = blockIdx.y == 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t row = blockIdx.x;
   const int qi = (int)(row % Sq);
@@ -442,48 +517,29 @@ lsh_query_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs
     for (int t = 0; t < LSH_MAX_PER_LANE; ++t)
       if (t < per) {
         const float u = sah_round_to<T>(__fdiv_rn(c[t], den2));
-        qunit[row * D + lane * per + t] = u;
-        if (qhat != nullptr) qhat[row * D + lane * per + t] = sah_from_float<T>(u);  // exact
+        if (writer) qunit[row * D + lane * per + t] = u;
+        if (writer && qhat != nullptr) qhat[row * D + lane * per + t] = sah_from_float<T>(u);  // exact
         if (mean) mu = __fmaf_rn(u, m[t], mu);
       }
     // unit query . key mean, the query-side constant of the centred cosine
     mu = lsh_warp_sum(mu);
-    if (qmu != nullptr && lane == 0) qmu[row] = mu;
+    if (writer && qmu != nullptr && lane == 0) qmu[row] = mu;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < lt * K) {  // one accumulator per column, channels ascending, as everywhere
+    float acc = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < D; ++c)
+      acc = __fadd_rn(acc, __fmul_rn(qn[c], sah_to_float<T>(pr[c * LSH_COLS + threadIdx.x])));
+    acc = __fadd_rn(acc, __fmul_rn(0.f, sah_to_float<T>(pr[D * LSH_COLS + threadIdx.x])));
+    sb[threadIdx.x] = acc > 0.f ? 1 : 0;
   }
   __syncthreads();
-  // A thread owns the columns o, o + 256, ... (four at a time); per column one accumulator and
-  // channels ascending, as everywhere.  The hyperplane values of 16 channels x 4 columns are
-  // requested before the first is used: this kernel sits on the critical path of every decode
-  // step and would otherwise be a chain of 129 dependent (cold) loads per column.
-  for (int o0 = threadIdx.x; o0 < nbits; o0 += 4 * 256) {
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int c0 = 0; c0 < D; c0 += 16) {
-      T pv[4][16];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          pv[j][i] = (o0 + j * 256 < nbits) ? proj[(int64_t)(c0 + i) * nbits + o0 + j * 256] : sah_from_float<T>(0.f);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          acc[j] = __fadd_rn(acc[j], __fmul_rn(qn[c0 + i], sah_to_float<T>(pv[j][i])));
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int o = o0 + j * 256;
-      if (o < nbits) {
-        const float a = __fadd_rn(acc[j], __fmul_rn(0.f, sah_to_float<T>(proj[(int64_t)D * nbits + o])));
-        sb[o] = a > 0.f ? 1 : 0;
-      }
-    }
-  }
-  __syncthreads();
-  for (int l = threadIdx.x; l < L; l += 256) {
+  for (int l = threadIdx.x; l < lt; l += LSH_COLS_THREADS) {
     unsigned int code = 0;
     for (int j = 0; j < K; ++j) code |= (unsigned int)sb[l * K + j] << j;
-    qcodes[row * L + l] = (CodeT)code;
+    qcodes[row * L + l0 + l] = (CodeT)code;
   }
 }
 
@@ -500,18 +556,25 @@ extern "C" int sah_lsh_query(const void* q, int dtype, int64_t qs_b, int64_t qs_
     return sah_fail(SAH_ERR_UNSUPPORTED, "lsh_query: %d x %d signature bits exceed shared memory", L, K);
   const int64_t rows = (int64_t)B * Hq * Sq;
   cudaStream_t st = (cudaStream_t)stream;
+  const int tables = LSH_COLS / K;
+  const dim3 grid((unsigned)rows, (unsigned)((L + tables - 1) / tables));
+#define LSH_QUERY_LAUNCH(T, CodeT)                                                                 \
+  do {                                                                                             \
+    const int bytes = (D + 1) * LSH_COLS * (int)sizeof(T) + D * 4 + LSH_COLS;                      \
+    if (bytes > 48 * 1024) {                                                                       \
+      cudaError_t e = cudaFuncSetAttribute(lsh_query_kernel<T, CodeT>,                             \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);    \
+      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_query attr: %s", cudaGetErrorString(e)); \
+    }                                                                                              \
+    sah_launch_chain(lsh_query_kernel<T, CodeT>, grid, LSH_COLS_THREADS, bytes, st, \
+        reinterpret_cast<const T*>(q), qs_b, qs_h, qs_q, Hq, Sq, G, D,                             \
+        reinterpret_cast<const T*>(mean), reinterpret_cast<const T*>(proj), L, K,                  \
+        reinterpret_cast<CodeT*>(qcodes), qunit, reinterpret_cast<T*>(qhat), qmu);                 \
+  } while (0)
   SAH_DISPATCH_DTYPE(dtype, T, {
-    if (K <= 8)
-      sah_launch_chain(lsh_query_kernel<T, uint8_t>, (unsigned)rows, 256, smem, st,
-          reinterpret_cast<const T*>(q), qs_b, qs_h, qs_q, Hq, Sq, G, D,
-          reinterpret_cast<const T*>(mean), reinterpret_cast<const T*>(proj), L, K,
-          reinterpret_cast<uint8_t*>(qcodes), qunit, reinterpret_cast<T*>(qhat), qmu);
-    else
-      sah_launch_chain(lsh_query_kernel<T, uint16_t>, (unsigned)rows, 256, smem, st,
-          reinterpret_cast<const T*>(q), qs_b, qs_h, qs_q, Hq, Sq, G, D,
-          reinterpret_cast<const T*>(mean), reinterpret_cast<const T*>(proj), L, K,
-          reinterpret_cast<uint16_t*>(qcodes), qunit, reinterpret_cast<T*>(qhat), qmu);
+    if (K <= 8) LSH_QUERY_LAUNCH(T, uint8_t); else LSH_QUERY_LAUNCH(T, uint16_t);
   });
+#undef LSH_QUERY_LAUNCH
   SAH_LAUNCH_CHECK("lsh_query");
   return SAH_OK;
 }

@@ -71,6 +71,58 @@ pq_assign_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs
   codes[(bk * cap + (j - init_offset)) * n_sub + sub] = (uint8_t)arg;
 }
 
+// The same for the keys that a decode step appends: a warp takes one sub-vector of one key and
+// deals the centroids to its lanes, straight from global memory (8 heads x 16 sub-vectors x 1 key
+// took 56 us with one thread walking all 256 centroids of a CTA's table, 7.8 us now, all latency).
+#define PQ_FEW_KEYS 16
+template <typename T, bool DTYPE_MATH>
+__global__ void __launch_bounds__(256)
+pq_assign_few_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
+                     int64_t key_begin, int n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent,
+                     int64_t items, const float* __restrict__ centroids, uint8_t* __restrict__ codes,
+                     int64_t cap) {
+  const int lane = threadIdx.x & 31;
+  const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // (group, key)
+  if (item >= items) return;
+  const int64_t grp = item / n_keys, j = key_begin + item % n_keys;
+  const int sub = (int)(grp % n_sub);
+  const int64_t bk = grp / n_sub;
+  const T* xr = x + bk / Hkv * xs_b + bk % Hkv * xs_h + j * xs_s + sub * sub_d;
+  float xv[PQ_MAX_SUBD];
+#pragma unroll
+  for (int d = 0; d < PQ_MAX_SUBD; ++d) xv[d] = d < sub_d ? sah_to_float<T>(xr[d]) : 0.f;
+  float best = INFINITY;
+  int arg = 256;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = i * 32 + lane;
+    if (c < n_cent) {
+      const float* cp = centroids + (grp * n_cent + c) * sub_d;
+      float dist = 0.f;  // pq_dist / pq_dist_dtype with the sub-vector in registers
+#pragma unroll
+      for (int d = 0; d < PQ_MAX_SUBD; ++d)
+        if (d < sub_d) {
+          const float t = __fsub_rn(xv[d], cp[d]);
+          if (DTYPE_MATH) {
+            const float r = sah_round_to<T>(t);
+            dist = __fadd_rn(dist, sah_round_to<T>(__fmul_rn(r, r)));
+          } else {
+            dist = __fadd_rn(dist, __fmul_rn(t, t));
+          }
+        }
+      if (DTYPE_MATH) dist = sah_round_to<T>(dist);
+      if (dist < best) { best = dist; arg = c; }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+    if (ob < best || (ob == best && oa < arg)) { best = ob; arg = oa; }  // first minimum wins
+  }
+  if (lane == 0) codes[(bk * cap + (j - init_offset)) * n_sub + sub] = (uint8_t)(arg < 256 ? arg : 0);
+}
+
 extern "C" int sah_pq_assign(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
                              int B, int Hkv, int64_t key_begin, int64_t key_end,
                              int64_t init_offset, int n_sub, int sub_d, int n_cent,
@@ -84,6 +136,23 @@ extern "C" int sah_pq_assign(const void* x, int dtype, int64_t xs_b, int64_t xs_
     return sah_fail(SAH_ERR_UNSUPPORTED, "pq_assign: sub-vector dim %d (<= %d) / %d centroids (<= 256)",
                     sub_d, PQ_MAX_SUBD, n_cent);
   if (key_begin == key_end) return SAH_OK;
+  if (key_end - key_begin <= PQ_FEW_KEYS) {
+    const int n_keys = (int)(key_end - key_begin);
+    const int64_t items = (int64_t)B * Hkv * n_sub * n_keys;
+    const unsigned few = (unsigned)sah_ceil_div(items, (int64_t)8);
+    SAH_DISPATCH_DTYPE(dtype, T, {
+      if (dtype_math)
+        pq_assign_few_kernel<T, true><<<few, 256, 0, (cudaStream_t)stream>>>(
+            (const T*)x, xs_b, xs_h, xs_s, Hkv, key_begin, n_keys, init_offset, n_sub, sub_d, n_cent, items,
+            centroids, codes, cap);
+      else
+        pq_assign_few_kernel<T, false><<<few, 256, 0, (cudaStream_t)stream>>>(
+            (const T*)x, xs_b, xs_h, xs_s, Hkv, key_begin, n_keys, init_offset, n_sub, sub_d, n_cent, items,
+            centroids, codes, cap);
+    });
+    SAH_LAUNCH_CHECK("pq_assign_few");
+    return SAH_OK;
+  }
   dim3 grid((unsigned)sah_ceil_div(key_end - key_begin, PQ_TILE), (unsigned)n_sub,
             (unsigned)((int64_t)B * Hkv));
   const size_t smem = (size_t)n_cent * sub_d * sizeof(float);

@@ -379,3 +379,44 @@ def test_gpu_tensor_core_signatures_at_the_edges(L, S, scale, centred, dup):
     assert not dup or redone >= B * Hkv * S
     assert torch.equal(got[:, :, :S], want[:, :, :S])
     assert bool((got[:, :, S:] == 0x55).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,L,K,D,centred", [("bf16", 75, 8, 128, True), ("bf16", 7, 3, 64, True),
+                                                 ("f32", 9, 11, 128, False), ("f32", 75, 8, 256, True),
+                                                 ("bf16", 5, 16, 32, False), ("bf16", 130, 1, 128, True)])
+def test_gpu_signatures_of_single_keys_equal_those_of_a_tile(dtype, L, K, D, centred):
+    """Up to four keys are hashed by CTAs that share a key's tables, longer ranges tile by tile:
+    the same rows, padding included, whatever the table width and the alignment of the
+    hyperplanes' rows."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    B, Hkv, S = 2, 2, 9
+    torch.manual_seed(L + D)
+    keys = torch.randn((B, Hkv, S, D), device=dev).to(dt)
+    proj = torch.randn((D + 1, L * K), device=dev).to(dt)
+    mean = keys.float().mean(dim=2).to(dt).contiguous() if centred else None
+    norms = torch.zeros((B, Hkv, S), dtype=torch.float32, device=dev)
+    max_norm = torch.zeros(1, dtype=torch.int32, device=dev)
+    st = _native.stream_of(torch.device(dev))
+    kargs = (keys.data_ptr(), _native.dtype_code(dt), keys.stride(0), keys.stride(1), keys.stride(2), B, Hkv)
+    _native.check(lib.sah_lsh_key_stats(*kargs, 0, S, D, _native.ptr(mean), S, norms.data_ptr(),
+                                        max_norm.data_ptr(), 148, st), "sah_lsh_key_stats")
+    width = 1 if K <= 8 else 2
+    pitch = (L * width + 15) // 16 * 16
+    whole = torch.full((B, Hkv, S, pitch), 0xAA, dtype=torch.uint8, device=dev)
+    parts = torch.full_like(whole, 0x55)
+
+    def sign(codes, s0, s1):
+        _native.check(lib.sah_lsh_key_sign(*kargs, s0, s1, D, _native.ptr(mean), norms.data_ptr(),
+                                           max_norm.data_ptr(), proj.data_ptr(), L, K, S, codes.data_ptr(), st),
+                      "sah_lsh_key_sign")
+
+    sign(whole, 0, S)
+    for s0, s1 in ((0, 1), (1, 5), (5, 7), (7, 8), (8, 9)):
+        sign(parts, s0, s1)
+    assert torch.equal(whole, parts)

@@ -310,3 +310,36 @@ def test_gpu_cluster_sums_equal_float64_sums(dtype, n_sub, sub_d, n_keys):
         cnt[g] = np.bincount(c[g // n_sub, :, g % n_sub], minlength=n_cent)
     np.testing.assert_array_equal(counts.cpu().numpy(), cnt)
     np.testing.assert_array_equal(sums.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("n_sub,sub_d,n_cent,math", [(16, 8, 256, 1), (3, 5, 33, 0), (1, 16, 1, 1), (4, 9, 31, 0)])
+def test_gpu_few_appended_keys_equal_the_tile_kernel(dtype, n_sub, sub_d, n_cent, math):
+    """Up to 16 keys are quantised by a warp per sub-vector, longer ranges by a thread per key: the
+    same codes, equal distances (duplicated centroids) and not-a-number keys included."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    B, Hkv, S, off = 2, 3, 40, 2
+    torch.manual_seed(n_cent)
+    x = torch.randn((B, Hkv, S, n_sub * sub_d), device=dev).to(dt)
+    x[:, :, 11, :] = float("nan")
+    cent = torch.randn((B * Hkv * n_sub, n_cent, sub_d), device=dev).to(dt).float()
+    cent[:, n_cent // 2:] = cent[:, :n_cent - n_cent // 2].clone()
+    st = _native.stream_of(torch.device(dev))
+
+    def assign(codes, s0, s1):
+        _native.check(lib.sah_pq_assign(x.data_ptr(), _native.dtype_code(dt), x.stride(0), x.stride(1), x.stride(2),
+                                        B, Hkv, s0, s1, off, n_sub, sub_d, n_cent, cent.data_ptr(), codes.data_ptr(),
+                                        S, math, st), "sah_pq_assign")
+
+    whole = torch.full((B, Hkv, S, n_sub), 77, dtype=torch.uint8, device=dev)
+    parts = whole.clone()
+    assign(whole, off, S)
+    for s0, s1 in ((off, off + 1), (off + 1, off + 17), (off + 17, off + 20), (off + 20, off + 36), (off + 36, S)):
+        assign(parts, s0, s1)
+    assert torch.equal(whole, parts)
