@@ -8,7 +8,9 @@
 // Encode.  A persistent CTA hashes tiles of HE_TK vectors; its tiles are a contiguous range of
 // the (batch, output head, tile) list, so that a head's weights (fp32, every layer) are staged
 // once and stay in shared memory while the head lasts, and every SM gets the same share of the
-// list.  Activations are fp32 [channel][vector] and overwritten layer by layer.
+// list.  Four groups of two warps each take a tile at a time, with barriers of their own, so that
+// one group's rounding, activation look-ups and stores run under another's multiply-adds.
+// Activations are fp32 [channel][vector] and overwritten layer by layer.
 //
 // One layer is a register-tiled product in which every output has a single fp32 accumulator
 // that walks the input channels in ascending order, fma by fma; that fixes the summation order
@@ -17,13 +19,15 @@
 // fma does) against the shared-memory reads that feed it: a thread owns 16 vectors x 4 outputs,
 // whose 64 multiply-adds need four broadcast reads of activations and one of weights.
 // 32 heads x 16384 keys through 128-128-128-32: 1963 us with tiles of 64 vectors, 8 x 4 outputs
-// per thread, scalar fma and the weights staged per tile; 981 us now (19.3 G
-// multiply-adds; 540 us at 128 per clock and SM).
+// per thread, scalar fma and the weights staged per tile; 981 us with one tile of 128 vectors per
+// CTA; 907 us now (19.3 G multiply-adds; 540 us at 128 per clock and SM).
 // ---------------------------------------------------------------------------
-#define HE_TK 128       // vectors per tile
-#define HE_THREADS 256
+#define HE_TK 32        // vectors per tile
+#define HE_GT 64        // threads per group
+#define HE_GROUPS 4
+#define HE_THREADS (HE_GT * HE_GROUPS)
 #define HE_MAXD 128     // widest layer
-#define HE_PITCH 132    // floats per activation channel: lanes that write neighbouring channels
+#define HE_PITCH 36     // floats per activation channel: lanes that write neighbouring channels
                         // four vectors at a time hit different banks
 
 struct HashEncodeArgs {
@@ -71,15 +75,19 @@ __device__ __forceinline__ unsigned long long he_pack2(float lo, float hi) {
   return r;
 }
 
+__device__ __forceinline__ void he_group_sync() {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(1 + (int)threadIdx.x / HE_GT), "n"(HE_GT) : "memory");
+}
+
 // One layer over the tile: thread (kg, og) owns vectors kg * KP + i and outputs o * NOG + og.
-// KP x OP is 16 x 4 for 128 outputs, 16 x 2 for 64, 8 x 2 for 32, 8 x 1 for 16, so that 256
-// threads always cover the tile.  w_sm is [channel][og][o]: a thread's weights adjoin.
+// KP x OP is 16 x 4 for 128 outputs, 16 x 2 for 64, 8 x 2 for 32, 8 x 1 for 16, so that the
+// group's threads always cover the tile.  w_sm is [channel][og][o]: a thread's weights adjoin.
 template <typename T, int KP, int OP>
 __device__ __forceinline__ void he_layer(float* __restrict__ act, const float* __restrict__ w_sm,
                                          const T* __restrict__ bias_h, int din, bool last, int act_kind,
                                          const uint16_t* act_table, uint32_t* codes, int nvalid) {
-  constexpr int NOG = HE_THREADS / (HE_TK / KP);
-  const int og = threadIdx.x % NOG, kg = threadIdx.x / NOG;
+  constexpr int NOG = HE_GT / (HE_TK / KP);
+  const int gt = threadIdx.x % HE_GT, og = gt % NOG, kg = gt / NOG;
   unsigned long long acc[KP / 2][OP];
 #pragma unroll
   for (int i = 0; i < KP / 2; ++i)
@@ -117,7 +125,7 @@ __device__ __forceinline__ void he_layer(float* __restrict__ act, const float* _
       for (int i = 0; i < KP / 2; ++i)
         asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][o]) : "l"(a[i]), "l"(w[o]));
   }
-  __syncthreads();  // everybody has read the input activations
+  he_group_sync();  // everybody has read the input activations
 
   unsigned int word = 0u;
 #pragma unroll
@@ -160,11 +168,11 @@ template <typename T>
 __global__ void __launch_bounds__(HE_THREADS, 1)
 hash_encode_kernel(HashEncodeArgs p) {
   extern __shared__ __align__(16) unsigned char he_smem[];
-  float* act = reinterpret_cast<float*>(he_smem);  // [HE_MAXD][HE_PITCH]
-  float* w_sm = act + HE_MAXD * HE_PITCH;
+  const int grp = threadIdx.x / HE_GT, gt = threadIdx.x % HE_GT;
+  float* act = reinterpret_cast<float*>(he_smem) + grp * HE_MAXD * HE_PITCH;  // [HE_MAXD][HE_PITCH] per group
+  float* w_sm = reinterpret_cast<float*>(he_smem) + HE_GROUPS * HE_MAXD * HE_PITCH;
   const int D = p.dims[0], cpr = D / 8;
   const int64_t t_first = p.tiles * blockIdx.x / gridDim.x, t_last = p.tiles * (blockIdx.x + 1) / gridDim.x;
-  int staged = -1;  // the head whose weights are in w_sm
 
   auto stage_weights = [&](int l, int h, float* dst) {
     const int din = p.dims[l], dout = p.dims[l + 1];
@@ -173,74 +181,90 @@ hash_encode_kernel(HashEncodeArgs p) {
 #pragma unroll 8
     for (int d = threadIdx.x / dout; d < din; d += step) dst[d * dout + slot] = sah_to_float<T>(wl[d * dout + out]);
   };
-  // A tile's input, transposed on its way into shared memory.  bfloat16 rows are fetched into
-  // registers while the last layer of the tile before is computed.
-  constexpr int FETCH = HE_TK * HE_MAXD / 8 / HE_THREADS;
+  // A tile's input, transposed on its way into shared memory: a thread holds every other chunk of
+  // eight channels of one vector.  bfloat16 rows are fetched into registers while the last layer
+  // of the tile before is computed.
+  constexpr int FETCH = HE_TK * HE_MAXD / 8 / HE_GT;
   uint4 raw[FETCH];
-  auto row_of = [&](int64_t t, int i) -> const T* {
+  auto row_of = [&](int64_t t) -> const T* {
     const int64_t bh = t / p.tiles_per_head;
-    const int64_t n = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK + i;
-    if (n >= p.n_end) return nullptr;
+    const int64_t n = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK + gt % HE_TK;
+    if (t >= t_last || n >= p.n_end) return nullptr;
     const int h = (int)(bh % p.H_out);
     return reinterpret_cast<const T*>(p.x) + bh / p.H_out * p.xs_b + h / (p.H_out / p.H_in) * p.xs_h + n * p.xs_n;
   };
   auto fetch = [&](int64_t t) {
-    const T* row = row_of(t, threadIdx.x % HE_TK);
+    const T* row = row_of(t);
 #pragma unroll
     for (int f = 0; f < FETCH; ++f) {
-      const int c = threadIdx.x / HE_TK + f * (HE_THREADS / HE_TK);
+      const int c = gt / HE_TK + f * (HE_GT / HE_TK);
       raw[f] = make_uint4(0u, 0u, 0u, 0u);
       if (c < cpr && row != nullptr) raw[f] = *reinterpret_cast<const uint4*>(row + c * 8);
     }
   };
-  if (sizeof(T) == 2 && t_first < t_last) fetch(t_first);
 
-  for (int64_t t = t_first; t < t_last; ++t) {
-    const int64_t bh = t / p.tiles_per_head;
+  // the range head by head; within a head group g takes the tiles g, g + HE_GROUPS, ...
+  for (int64_t t0 = t_first; t0 < t_last;) {
+    const int64_t bh = t0 / p.tiles_per_head;
     const int h = (int)(bh % p.H_out);
-    const int64_t n0 = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK;
-    // (the last layer's barrier stands between the reads of the tile before and these writes)
-    {
-      const int i = threadIdx.x % HE_TK;
-      const T* row = sizeof(T) == 2 ? nullptr : row_of(t, i);
-#pragma unroll
-      for (int f = 0; f < FETCH; ++f) {
-        const int c = threadIdx.x / HE_TK + f * (HE_THREADS / HE_TK);
-        if (c < cpr) {
-          float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          if (sizeof(T) == 2) sah_unpack8(raw[f], v);
-          else if (row != nullptr) sah_load8<T>(row + c * 8, v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) act[(c * 8 + e) * HE_PITCH + i] = v[e];
-        }
-      }
-    }
-    if (p.resident && staged != h) {
+    int64_t t1 = (bh + 1) * p.tiles_per_head;
+    if (t1 > t_last) t1 = t_last;
+    int64_t t = t0 + grp;
+    if (sizeof(T) == 2) fetch(t < t1 ? t : t_last);  // zeros where the group has no tile
+    if (p.resident) {
+      __syncthreads();  // the weights of the head before are done with
       float* dst = w_sm;
       for (int l = 0; l < p.n_layers; ++l) {
         stage_weights(l, h, dst);
         dst += p.dims[l] * p.dims[l + 1];
       }
-      staged = h;
-    }
-    const float* w_l = w_sm;
-    uint32_t* codes = p.codes + bh * p.n_total + n0;
-    const int nvalid = (int)(p.n_end - n0 < HE_TK ? p.n_end - n0 : HE_TK);
-    for (int l = 0; l < p.n_layers; ++l) {
-      const int din = p.dims[l], dout = p.dims[l + 1];
-      const bool last = l == p.n_layers - 1;
-      if (!p.resident) stage_weights(l, h, w_sm);  // the layer before ended its reads at a barrier
       __syncthreads();
-      if (sizeof(T) == 2 && last && t + 1 < t_last) fetch(t + 1);
-      const T* bl = reinterpret_cast<const T*>(p.bias[l]) + (int64_t)h * dout;
-      switch (dout) {
-        case 128: he_layer<T, 16, 4>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
-        case 64:  he_layer<T, 16, 2>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
-        case 32:  he_layer<T, 8, 2>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
-        default:  he_layer<T, 8, 1>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
-      }
-      if (p.resident) w_l += din * dout;
     }
+    // weights that are staged layer by layer keep the groups together: all of them go round
+    // equally often, with nothing to write where a group has no tile left
+    const int64_t rounds = p.resident ? (t < t1 ? (t1 - t + HE_GROUPS - 1) / HE_GROUPS : 0)
+                                      : (t1 - t0 + HE_GROUPS - 1) / HE_GROUPS;
+    for (int64_t round = 0; round < rounds; ++round, t += HE_GROUPS) {
+      {  // (the last layer's barrier stands between the reads of the tile before and these writes)
+        const T* row = sizeof(T) == 2 ? nullptr : (t < t1 ? row_of(t) : nullptr);
+#pragma unroll
+        for (int f = 0; f < FETCH; ++f) {
+          const int c = gt / HE_TK + f * (HE_GT / HE_TK);
+          if (c < cpr) {
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (sizeof(T) == 2) sah_unpack8(raw[f], v);
+            else if (row != nullptr) sah_load8<T>(row + c * 8, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) act[(c * 8 + e) * HE_PITCH + gt % HE_TK] = v[e];
+          }
+        }
+      }
+      const float* w_l = w_sm;
+      const int64_t n0 = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK;
+      uint32_t* codes = p.codes + bh * p.n_total + n0;
+      const int nvalid = t >= t1 ? 0 : (int)(p.n_end - n0 < HE_TK ? p.n_end - n0 : HE_TK);
+      for (int l = 0; l < p.n_layers; ++l) {
+        const int din = p.dims[l], dout = p.dims[l + 1];
+        const bool last = l == p.n_layers - 1;
+        if (p.resident) {
+          he_group_sync();
+        } else {
+          __syncthreads();  // the layer before is done with the region
+          stage_weights(l, h, w_sm);
+          __syncthreads();
+        }
+        if (sizeof(T) == 2 && last && t + HE_GROUPS < t1) fetch(t + HE_GROUPS);
+        const T* bl = reinterpret_cast<const T*>(p.bias[l]) + (int64_t)h * dout;
+        switch (dout) {
+          case 128: he_layer<T, 16, 4>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+          case 64:  he_layer<T, 16, 2>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+          case 32:  he_layer<T, 8, 2>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+          default:  he_layer<T, 8, 1>(act, w_l, bl, din, last, p.act, p.act_table, codes, nvalid); break;
+        }
+        if (p.resident) w_l += din * dout;
+      }
+    }
+    t0 = t1;
   }
 }
 
@@ -442,7 +466,7 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
     sah_prof_end(SAH_PROF_HASH_ENCODE, st);
     return SAH_OK;
   }
-  // Weights beside the 66 KB of activations: all layers while they fit (128-128-128-32 does),
+  // Weights beside the 72 KB of activations: all layers while they fit (128-128-128-32 does),
   // else one region of the widest layer, staged layer by layer for every tile.
   size_t w_all = 0, w_max = 0;
   for (int l = 0; l < n_layers; ++l) {
@@ -450,12 +474,13 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
     w_all += w;
     w_max = w > w_max ? w : w_max;
   }
-  const size_t act_bytes = (size_t)HE_MAXD * HE_PITCH * sizeof(float);
+  const size_t act_bytes = (size_t)HE_GROUPS * HE_MAXD * HE_PITCH * sizeof(float);
   p.resident = act_bytes + w_all <= 227 * 1024 ? 1 : 0;
   const size_t smem = act_bytes + (p.resident ? w_all : w_max);
   p.tiles_per_head = sah_ceil_div(n_end - n_begin, (int64_t)HE_TK);
   p.tiles = p.tiles_per_head * H_out * B;
-  const unsigned grid = (unsigned)(p.tiles < 148 ? p.tiles : 148);
+  const int64_t ctas = sah_ceil_div(p.tiles, (int64_t)HE_GROUPS);
+  const unsigned grid = (unsigned)(ctas < 148 ? ctas : 148);
   sah_prof_begin(SAH_PROF_HASH_ENCODE, (cudaStream_t)stream);
   SAH_DISPATCH_DTYPE(dtype, T, {
     cudaError_t e = cudaFuncSetAttribute(hash_encode_kernel<T>,
