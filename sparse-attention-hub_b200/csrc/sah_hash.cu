@@ -496,53 +496,59 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
 // ---------------------------------------------------------------------------
 // Top-k over Hamming scores.
 // ---------------------------------------------------------------------------
-struct HashKeyPlain {
-  const uint32_t* kc;
-  uint32_t qc;
-  int nbits;
-  __device__ __forceinline__ unsigned int operator()(int64_t j) const {
-    return (unsigned int)(nbits - __popc(kc[j] ^ qc));  // matching bits: monotone in the score
-  }
-};
-
+// with an additive mask: the rounded sum of score and mask, eight columns at a time
 template <typename T, int KEYBITS>
-struct HashKeyBiased {
-  const uint32_t* kc;
-  uint32_t qc;
+struct HashBiasedKeys {
+  const uint32_t* kcodes;
+  int64_t kc_stride;
+  const uint32_t* qcodes;
   int nbits;
   const T* bias;
-  __device__ __forceinline__ unsigned int operator()(int64_t j) const {
-    float s = (float)(nbits - 2 * __popc(kc[j] ^ qc));
-    float f = sah_round_to<T>(__fadd_rn(s, sah_to_float<T>(bias[j]))) + 0.0f;
-    unsigned int key = sah_float_key(f);
-    return KEYBITS == 16 ? (key >> 16) : key;
+  int64_t bias_s_b, bias_s_h, bias_s_q;
+  int Hq, Sq;
+  int64_t S;
+  const uint32_t* kc;
+  uint32_t qc;
+  const T* br;
+  bool vec, bias_vec;
+  __device__ __forceinline__ void open(int64_t row) {
+    const int q = (int)(row % Sq);
+    const int64_t bh = row / Sq;
+    kc = kcodes + bh * kc_stride;
+    qc = qcodes[row];
+    br = bias + bh / Hq * bias_s_b + bh % Hq * bias_s_h + q * bias_s_q;
+    vec = (reinterpret_cast<uintptr_t>(kc) & 15) == 0;
+    bias_vec = (reinterpret_cast<uintptr_t>(br) & 15) == 0;
+  }
+  __device__ __forceinline__ void load(int64_t c0, uint32_t* w) const {
+    uint32_t c[8], key[8];
+    float bv[8];
+    if (vec && c0 + 8 <= S) {
+      const uint4 a = *reinterpret_cast<const uint4*>(kc + c0), b = *reinterpret_cast<const uint4*>(kc + c0 + 4);
+      c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
+      c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[i] = c0 + i < S ? kc[c0 + i] : 0u;
+    }
+    if (bias_vec && c0 + 8 <= S) {
+      sah_load8<T>(br + c0, bv);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) bv[i] = c0 + i < S ? sah_to_float<T>(br[c0 + i]) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float s = (float)(nbits - 2 * __popc(c[i] ^ qc));
+      key[i] = sah_float_key(sah_round_to<T>(__fadd_rn(s, bv[i])) + 0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (KEYBITS == 32) w[i] = key[i];
+      else if (i & 1) w[i >> 1] = __byte_perm(key[i - 1], key[i], 0x7632);  // the upper halves
+    }
   }
 };
-
-template <typename T, int KEYBITS, bool BIASED>
-__global__ void __launch_bounds__(SAH_SELECT_THREADS)
-hash_topk_kernel(const uint32_t* __restrict__ kcodes, int64_t kc_stride,
-                 const uint32_t* __restrict__ qcodes, int nbits, const T* __restrict__ bias, int64_t bias_s_b, int64_t bias_s_h,
-                 int64_t bias_s_q, int Hq, int Sq, int64_t S, int64_t W,
-                 const uint32_t* __restrict__ prev_bits, int64_t k,
-                 uint32_t* __restrict__ out_bits) {
-  sah_pdl_entry();
-  __shared__ SahSelectSmem sm;
-  const int64_t row = blockIdx.x;
-  const int q = (int)(row % Sq);
-  const int64_t bh = row / Sq;
-  const int h = (int)(bh % Hq);
-  const int64_t b = bh / Hq;
-  const uint32_t* kc = kcodes + bh * kc_stride;
-  const uint32_t qc = qcodes[row];
-  if (BIASED) {
-    HashKeyBiased<T, KEYBITS> kf{kc, qc, nbits, bias + b * bias_s_b + h * bias_s_h + q * bias_s_q};
-    sah_select_row<KEYBITS>(kf, prev_bits + row * W, out_bits + row * W, S, W, 0, S, k, sm);
-  } else {
-    HashKeyPlain kf{kc, qc, nbits};
-    sah_select_row<8>(kf, prev_bits + row * W, out_bits + row * W, S, W, 0, S, k, sm);
-  }
-}
 
 // Counting select for the unbiased case: a score takes at most nbits + 1
 // values, so the k-th best score and the number of ties to take at it follow
@@ -990,13 +996,15 @@ extern "C" int sah_hash_topk(const uint32_t* kcodes, int64_t kc_stride, const ui
       sah_launch_chain(hash_topk_fast_kernel, (unsigned)rows, 1024, 0, st, kcodes, kc_stride, qcodes, nbits, Sq, S,
                                                             W, prev_bits, k, out_bits);
   } else if (dtype == SAH_BF16) {
-    sah_launch_chain(hash_topk_kernel<__nv_bfloat16, 16, true>, (unsigned)rows, SAH_SELECT_THREADS, 0, st,
-        kcodes, kc_stride, qcodes, nbits, (const __nv_bfloat16*)bias, bias_s_b, bias_s_h, bias_s_q, Hq, Sq,
-        S, W, prev_bits, k, out_bits);
+    const HashBiasedKeys<__nv_bfloat16, 16> keys{kcodes, kc_stride, qcodes, nbits, (const __nv_bfloat16*)bias,
+                                                 bias_s_b, bias_s_h, bias_s_q, Hq, Sq, S};
+    const int rc = sah_select_launch<16>(keys, prev_bits, out_bits, rows, S, W, 0, S, k, st);
+    if (rc != SAH_OK) return rc;
   } else if (dtype == SAH_F32) {
-    sah_launch_chain(hash_topk_kernel<float, 32, true>, (unsigned)rows, SAH_SELECT_THREADS, 0, st, kcodes,
-        kc_stride, qcodes, nbits, (const float*)bias, bias_s_b, bias_s_h, bias_s_q, Hq, Sq, S, W,
-        prev_bits, k, out_bits);
+    const HashBiasedKeys<float, 32> keys{kcodes, kc_stride, qcodes, nbits, (const float*)bias,
+                                         bias_s_b, bias_s_h, bias_s_q, Hq, Sq, S};
+    const int rc = sah_select_launch<32>(keys, prev_bits, out_bits, rows, S, W, 0, S, k, st);
+    if (rc != SAH_OK) return rc;
   } else {
     return sah_fail(SAH_ERR_INVALID, "hash_topk: unknown dtype %d", dtype);
   }

@@ -1,36 +1,33 @@
-// Exact per-row top-k by radix select over order-preserving integer keys, with
-// ties going to the lowest column.  One CTA (SAH_SELECT_THREADS threads) owns
-// one mask row.  Only columns inside [col_begin, col_end) whose `prev` bit is
+// Exact per-row top-k by radix select over order-preserving integer keys, with ties going to the
+// lowest column, in one launch: a row belongs to a cluster of up to eight CTAs, each with a
+// contiguous range of its columns.  Only columns inside [col_begin, col_end) whose `prev` bit is
 // clear compete; the row written is prev | winners.
 //
-// Passes over the row's keys: KEYBITS / 8 histogram passes (most significant
-// digit first) fix the k-th largest key T and how many keys equal to T are
-// still needed; one counting pass and one emit pass then resolve ties in
-// column order: each warp owns a contiguous run of bitmap words, counts its
-// keys equal to T, a 32-entry scan orders the warps, and the warp emits its
-// words front to back taking "equal" keys while the quota lasts.
+// Two (16-bit keys: 11 + 5 bits) or three (32-bit keys: 11 + 11 + 10) histogram passes, most
+// significant digit first, fix the k-th largest key T and how many keys equal to T are still
+// needed; every CTA reads the other CTAs' histograms over distributed shared memory and finds the
+// digit itself, one cluster barrier per digit.  Wide first digits because scores share their
+// exponents: 8-bit digits put most keys of a warp into the same few counters.  One more pass
+// emits; where the keys equal to T are more than are needed a counting pass in front of it orders
+// them: a warp owns a contiguous run of columns, 32 lanes x 8 columns at a time, so reads are
+// coalesced and a scan over the warps' counts is all the ordering that is left.
+//
+// The first pass leaves the keys, zero where a column does not compete, in shared memory (up to
+// 81920 columns of 16 bits or 40960 of 32 per CTA), and the others test two 16-bit keys with one
+// integer operation; a longer range is read and converted again in every pass.  Bound by
+// instruction issue (the passes make about 20 instructions per 16-bit key) and, for short rows,
+// by the barriers.  128 rows x 65536 bfloat16 scores: 35.2 us as three launches with a grid-wide
+// histogram each, 45.6 us with the keys converted in every pass, 27.6 us now (32 rows x 8191: 23.5 us before, 10.7 us now).
 #pragma once
 
 #include "sah_common.cuh"
+#include <cooperative_groups.h>
 
 #define SAH_SELECT_THREADS 1024
-
-struct SahSelectSmem {
-  unsigned int hist[256];
-  long long scan[33];
-  unsigned int prefix;       // key bits fixed so far
-  unsigned int prefix_mask;  // which bits are fixed
-  long long need;            // keys still to take among the current candidates
-  int take_all;              // fewer candidates than k: take every candidate
-};
-
-// Adds 1 to hist[digit] for every lane with digit < 256, one atomic per
-// distinct digit in the warp.
-__device__ __forceinline__ void sah_hist_add(unsigned int* hist, unsigned int digit) {
-  unsigned int peers = __match_any_sync(0xffffffffu, digit);
-  int lane = threadIdx.x & 31;
-  if (digit < 256u && lane == (__ffs(peers) - 1)) atomicAdd(&hist[digit], (unsigned)__popc(peers));
-}
+#define SAH_SELECT_MIN_THREADS 512  // four counters of a digit each
+#define SAH_SELECT_BINS 2048
+#define SAH_SELECT_MAX_CLUSTER 8
+#define SAH_SELECT_KEY_BYTES (160 * 1024)  // keys of a CTA's columns in shared memory
 
 // Keep the lowest n set bits of m.
 __device__ __forceinline__ uint32_t sah_lowest_bits(uint32_t m, int n) {
@@ -41,131 +38,369 @@ __device__ __forceinline__ uint32_t sah_lowest_bits(uint32_t m, int n) {
   return m & ((1u << pos) - 1u);
 }
 
-template <int KEYBITS, typename KeyFn>
-__device__ void sah_select_row(const KeyFn& keyf, const uint32_t* __restrict__ prev_row,
-                               uint32_t* __restrict__ out_row, int64_t S, int64_t W,
-                               int64_t col_begin, int64_t col_end, int64_t k,
-                               SahSelectSmem& sm) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int NT = SAH_SELECT_THREADS;
+
+// Eight keys from column c0 of a row, two 16-bit ones or one 32-bit one per word (anything past
+// the end).  No key is 0: that would be a negative not-a-number, and -0 and not-a-numbers are
+// made +0 and the positive one by an addition of +0.
+template <typename T, int KEYBITS>
+struct SahScoreKeys;
+template <>
+struct SahScoreKeys<__nv_bfloat16, 16> {
+  const __nv_bfloat16* scores;
+  int64_t S;
+  const __nv_bfloat16* s;
+  bool vec;
+  __device__ __forceinline__ void open(int64_t row) {
+    s = scores + row * S;
+    vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
+  }
+  __device__ __forceinline__ void load(int64_t c0, uint32_t* w) const {
+    if (vec && c0 + 8 <= S) {
+      const uint4 v = *reinterpret_cast<const uint4*>(s + c0);
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else {
+      const uint16_t* u = reinterpret_cast<const uint16_t*>(s);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t lo = c0 + 2 * i < S ? u[c0 + 2 * i] : 0u, hi = c0 + 2 * i + 1 < S ? u[c0 + 2 * i + 1] : 0u;
+        w[i] = lo | hi << 16;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 z = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]), __float2bfloat162_rn(0.f));
+      const uint32_t u = *reinterpret_cast<const uint32_t*>(&z);
+      w[i] = u ^ ((((u >> 15) & 0x00010001u) * 0xFFFFu) | 0x80008000u);
+    }
+  }
+};
+template <>
+struct SahScoreKeys<float, 32> {
+  const float* scores;
+  int64_t S;
+  const float* s;
+  bool vec;
+  __device__ __forceinline__ void open(int64_t row) {
+    s = scores + row * S;
+    vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
+  }
+  __device__ __forceinline__ void load(int64_t c0, uint32_t* w) const {
+    float f[8];
+    if (vec && c0 + 8 <= S) {
+      sah_load8<float>(s + c0, f);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = c0 + i < S ? s[c0 + i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = sah_float_key(f[i] + 0.0f);
+  }
+};
+
+template <int KEYBITS, typename Keys, bool RESIDENT>
+__global__ void __launch_bounds__(SAH_SELECT_THREADS)
+sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, uint32_t* __restrict__ out_bits, int64_t S,
+                  int64_t W, int64_t col_begin, int64_t col_end, long long k) {
+  sah_pdl_entry();
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  constexpr int NW = KEYBITS == 16 ? 4 : 8;  // words of eight keys
+  extern __shared__ __align__(16) unsigned char sel_smem[];
+  uint4* store = reinterpret_cast<uint4*>(sel_smem);  // [NW / 4][bytes of this CTA]
+  __shared__ unsigned int hist[2][SAH_SELECT_BINS];  // alternate digits: a CTA may count the next
+                                                     // one while others still read this one
+  __shared__ unsigned int scan[33];
+  __shared__ unsigned int prefix_sm;
+  __shared__ long long need_sm;
+  __shared__ unsigned int ties_sm;  // keys equal to the prefix in the whole row
+  __shared__ int mode_sm;           // 0: threshold, 1: all candidates, 2: none
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int64_t row = blockIdx.x / ranks;
+  keys.open(row);
+  const unsigned char* pb = reinterpret_cast<const unsigned char*>(prev_bits + row * W);
+  unsigned char* ob = reinterpret_cast<unsigned char*>(out_bits + row * W);
   if (col_begin < 0) col_begin = 0;
   if (col_end > S) col_end = S;
 
-  if (tid == 0) {
-    sm.prefix = 0u;
-    sm.prefix_mask = 0u;
-    sm.need = k;
-    sm.take_all = (k <= 0) ? 2 : 0;  // 2: take nothing
-  }
-  __syncthreads();
+  // this CTA's words in bytes of eight columns; a warp's run in blocks of 32 bytes
+  const int64_t y_lo = W * rank / ranks * 4, y_hi = W * (rank + 1) / ranks * 4;
+  const int ny = (int)(y_hi - y_lo);
+  const int blocks = (ny + 31) / 32;
+  const int q_lo = (int)((int64_t)blocks * warp / nw), q_hi = (int)((int64_t)blocks * (warp + 1) / nw);
+  pb += y_lo;
+  ob += y_lo;
+  // columns of byte y (of this CTA) that compete
+  auto competing = [&](int y) -> unsigned int {
+    const int64_t c0 = (y_lo + y) * 8;
+    if (c0 >= col_end || c0 + 8 <= col_begin) return 0u;
+    unsigned int m = ~(unsigned int)pb[y] & 255u;
+    if (c0 < col_begin) m &= 255u << (int)(col_begin - c0);
+    if (c0 + 8 > col_end) m &= (1u << (int)(col_end - c0)) - 1u;
+    return m;
+  };
+  // the byte's keys from memory, 0 where a column does not compete; false if none does
+  auto convert = [&](int y, uint32_t* w) -> bool {
+    const unsigned int m = competing(y);
+#pragma unroll
+    for (int i = 0; i < NW; ++i) w[i] = 0u;
+    if (m == 0u) return false;
+    keys.load((y_lo + y) * 8, w);
+    if (m != 255u) {
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        if (NW == 4)
+          w[i] &= ((m >> (2 * i)) & 1u ? 0xFFFFu : 0u) | ((m >> (2 * i + 1)) & 1u ? 0xFFFF0000u : 0u);
+        else
+          w[i] = (m >> i) & 1u ? w[i] : 0u;
+      }
+    }
+    return true;
+  };
+  auto fetch = [&](int y, uint32_t* w) -> bool {
+    if (!RESIDENT) return convert(y, w);
+#pragma unroll
+    for (int i = 0; i < NW / 4; ++i) {
+      const uint4 v = store[i * ny + y];
+      w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+    }
+    return true;
+  };
+  auto key_at = [](const uint32_t* w, int i) -> uint32_t {
+    return NW == 8 ? w[i] : (i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu;
+  };
 
-  // ---- histogram passes ----
-  if (k > 0) {
-    for (int shift = KEYBITS - 8; shift >= 0; shift -= 8) {
-      if (tid < 256) sm.hist[tid] = 0u;
+  uint32_t prefix = 0u, pmask = 0u;
+  long long need = k;
+  int mode = k <= 0 ? 2 : 0;
+  unsigned int ties = 0u;   // keys equal to the threshold in the whole row
+  unsigned int lower = 0u;  // and in the CTAs in front of this one
+  constexpr int DIGITS = KEYBITS == 16 ? 2 : 3;
+#pragma unroll
+  for (int d = 0; d < DIGITS; ++d) {
+    constexpr int LAST = KEYBITS == 16 ? 5 : 10;
+    const int bits = d == DIGITS - 1 ? LAST : 11;
+    const int shift = d == DIGITS - 1 ? 0 : KEYBITS - 11 * (d + 1);
+    const int nbins = 1 << bits;
+    unsigned int* h = hist[d & 1];
+    if (mode == 0) {  // the same in the whole cluster
+      for (int i = tid; i < nbins; i += nt) h[i] = 0u;
+      if (tid == 0) mode_sm = 0;
       __syncthreads();
-      const unsigned int pfx = sm.prefix, pmask = sm.prefix_mask;
-      const int stop = sm.take_all;
-      if (!stop) {
-        // The loop bound is warp-uniform so that every lane reaches the
-        // warp-wide match inside sah_hist_add.
-        int64_t j0 = col_begin - (col_begin & 31);
-        for (int64_t base = j0 + (tid & ~31); base < col_end; base += NT) {
-          const int64_t j = base + lane;
-          unsigned int digit = 256u;
-          if (j >= col_begin && j < col_end) {
-            uint32_t pw = prev_row[j >> 5];
-            if (!((pw >> (j & 31)) & 1u)) {
-              unsigned int key = keyf(j);
-              if ((key & pmask) == pfx) digit = (key >> shift) & 255u;
+      for (int q = q_lo; q < q_hi; ++q) {
+        const int y = q * 32 + lane;
+        if (y >= ny) break;
+        uint32_t w[NW];
+        if (d == 0) {
+          const bool any = convert(y, w);
+          if (RESIDENT) {
+#pragma unroll
+            for (int i = 0; i < NW / 4; ++i)
+              store[i * ny + y] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+          }
+          if (any) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint32_t key = key_at(w, i);
+              if (key) atomicAdd(&h[key >> shift], 1u);
             }
           }
-          sah_hist_add(sm.hist, digit);
-        }
-      }
-      __syncthreads();
-      if (warp == 0 && !stop) {
-        // lane l owns bins [8l, 8l+8); find the bin where the descending
-        // cumulative count reaches `need`.
-        unsigned int loc[8];
-        unsigned int s = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { loc[i] = sm.hist[lane * 8 + i]; s += loc[i]; }
-        // suffix sum over lanes: above = sum of lanes > lane
-        unsigned int incl = s;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          unsigned int n = __shfl_down_sync(0xffffffffu, incl, o);
-          if (lane + o < 32) incl += n;
-        }
-        unsigned int above = incl - s;
-        unsigned int total = __shfl_sync(0xffffffffu, incl, 0);
-        long long need = sm.need;
-        if ((long long)total < need || (shift == KEYBITS - 8 && (long long)total <= need)) {
-          if (lane == 0) sm.take_all = 1;
         } else {
-          bool mine = ((long long)above < need) && ((long long)above + s >= need);
-          if (mine) {
-            long long cum = above;
-            int d = 7;
-            for (; d >= 0; --d) {
-              if (cum + loc[d] >= need) break;
-              cum += loc[d];
+          if (!fetch(y, w)) continue;
+          bool any = true;
+          if (NW == 4) {  // some half agrees with the prefix (nothing is left below the mask, so the test is exact)
+            uint32_t z = 0u;
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+              const uint32_t x = (w[i] ^ (prefix * 0x00010001u)) & (pmask * 0x00010001u);
+              z |= (x - 0x00010001u) & ~x;
             }
-            sm.prefix = pfx | ((unsigned int)(lane * 8 + d) << shift);
-            sm.prefix_mask = pmask | (255u << shift);
-            sm.need = need - cum;
+            any = (z & 0x80008000u) != 0u;
+          }
+          if (any) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint32_t key = key_at(w, i);
+              if (((key ^ prefix) & pmask) == 0u && key) atomicAdd(&h[(key >> shift) & (nbins - 1)], 1u);
+            }
           }
         }
       }
+      if (ranks > 1) cluster.sync(); else __syncthreads();
+      // thread t owns PER neighbouring bins, the highest first; all reads are on their way before
+      // the first is added
+      constexpr int PER = SAH_SELECT_BINS / SAH_SELECT_MIN_THREADS;
+      unsigned int cnt[PER], mine = 0u;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int bin = nbins - 1 - (tid * PER + j);
+        cnt[j] = 0u;
+        if (bin >= 0) {
+          if (ranks == 1) {
+            cnt[j] = h[bin];
+          } else {
+#pragma unroll
+            for (int r = 0; r < SAH_SELECT_MAX_CLUSTER; ++r)
+              if (r < ranks) cnt[j] += cluster.map_shared_rank(h, r)[bin];
+          }
+        }
+        mine += cnt[j];
+      }
+      unsigned int total;
+      unsigned int above = sah_block_excl_scan<unsigned int>(mine, scan, &total);
+      if ((long long)total < need || (d == 0 && (long long)total <= need)) {
+        if (tid == 0) mode_sm = 1;
+      } else if ((long long)above < need && (long long)above + mine >= need) {
+        bool found = false;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+          if (!found && (long long)above + cnt[j] >= need) {
+            prefix_sm = prefix | ((uint32_t)(nbins - 1 - (tid * PER + j)) << shift);
+            need_sm = need - above;
+            ties_sm = cnt[j];
+            found = true;
+          }
+          above += cnt[j];
+        }
+      }
       __syncthreads();
-    }
-  }
-
-  // ---- tie resolution in column order ----
-  const unsigned int T = sm.prefix;
-  const int mode = sm.take_all;          // 0: threshold, 1: all candidates, 2: none
-  const long long need = sm.need;        // keys equal to T to take
-  const int64_t words_per_warp = (W + 31) / 32;
-  const int64_t w_lo = (int64_t)warp * words_per_warp;
-  int64_t w_hi = w_lo + words_per_warp;
-  if (w_hi > W) w_hi = W;
-
-  long long eq_here = 0;
-  if (mode == 0) {
-    for (int64_t w = w_lo; w < w_hi; ++w) {
-      int64_t j = w * 32 + lane;
-      bool eq = false;
-      if (j >= col_begin && j < col_end) {
-        uint32_t pw = prev_row[w];
-        if (!((pw >> lane) & 1u)) eq = (keyf(j) == T);
+      mode = mode_sm;
+      if (mode == 0) {
+        prefix = prefix_sm;
+        need = need_sm;
+        ties = ties_sm;
+        pmask |= (uint32_t)(nbins - 1) << shift;
+        if (d == DIGITS - 1)
+          for (int r = 0; r < rank; ++r) lower += cluster.map_shared_rank(h, r)[prefix & (nbins - 1)];
       }
-      eq_here += __popc(__ballot_sync(0xffffffffu, eq));
+      __syncthreads();  // before the shared state is written again
     }
   }
-  long long total_eq;
-  long long before = sah_block_excl_scan<long long>(lane == 0 ? eq_here : 0, sm.scan, &total_eq);
-  before = __shfl_sync(0xffffffffu, before, 0);
 
-  long long quota = need - before;  // equal keys this warp may still take
-  for (int64_t w = w_lo; w < w_hi; ++w) {
-    int64_t j = w * 32 + lane;
-    uint32_t pw = prev_row[w];
-    bool gt = false, eq = false;
-    if (mode != 2 && j >= col_begin && j < col_end && !((pw >> lane) & 1u)) {
-      if (mode == 1) {
-        gt = true;
-      } else {
-        unsigned int key = keyf(j);
-        gt = key > T;
-        eq = key == T;
+  // one bit per key of the byte: equal to the threshold
+  auto equal = [&](const uint32_t* w) -> uint32_t {
+    uint32_t eq = 0u;
+    if (NW == 4) {
+      uint32_t z[4], any = 0u;  // bits 15 and 31: the half is zero
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t x = w[i] ^ (prefix * 0x00010001u);
+        z[i] = ~(((x & 0x7FFF7FFFu) + 0x7FFF7FFFu) | x) & 0x80008000u;
+        any |= z[i];
+      }
+      if (any) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) eq |= ((z[i] >> 15) & 1u) << (2 * i) | (z[i] >> 31) << (2 * i + 1);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) eq |= (w[i % NW] == prefix ? 1u : 0u) << i;
+    }
+    return eq;
+  };
+
+  // keys equal to the threshold in the columns in front of this warp's
+  long long quota = need;
+  if (mode == 0 && (long long)ties > need) {
+    unsigned int eq = 0u;
+    for (int q = q_lo; q < q_hi; ++q) {
+      const int y = q * 32 + lane;
+      uint32_t w[NW];
+      if (y < ny && fetch(y, w)) eq += __popc(equal(w));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) eq += __shfl_xor_sync(0xffffffffu, eq, o);
+    unsigned int total;
+    unsigned int before = sah_block_excl_scan<unsigned int>(lane == 0 ? eq : 0u, scan, &total);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    quota = need - (long long)lower - (long long)before;
+  }
+  for (int q = q_lo; q < q_hi; ++q) {
+    const int y = q * 32 + lane;
+    const unsigned int prev = y < ny ? pb[y] : 0u;
+    unsigned int gt = 0u, eq = 0u;
+    if (mode == 1) {
+      if (y < ny) gt = competing(y);
+    } else if (mode == 0 && y < ny) {
+      uint32_t w[NW];
+      if (fetch(y, w)) {
+        uint32_t below = 0u;  // the threshold is not 0, so a column that does not compete is below it
+        if (NW == 4) {
+#pragma unroll
+          for (int i = 7; i >= 0; --i) below = __funnelshift_l(key_at(w, i) - prefix, below, 1);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) below |= (w[i % NW] < prefix ? 1u : 0u) << i;
+        }
+        eq = equal(w);
+        gt = ~below & 255u & ~eq;
       }
     }
-    uint32_t gm = __ballot_sync(0xffffffffu, gt);
-    uint32_t em = __ballot_sync(0xffffffffu, eq);
-    int take = quota > 32 ? 32 : (quota < 0 ? 0 : (int)quota);
-    uint32_t sel = gm | sah_lowest_bits(em, take);
-    quota -= __popc(em);
-    if (lane == 0) out_row[w] = pw | sel;
+    if (mode == 0 && quota > 0 && __any_sync(0xffffffffu, eq != 0u)) {  // uniform but for the vote
+      int incl = __popc(eq);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+      }
+      const long long left = quota - (incl - __popc(eq));
+      gt |= sah_lowest_bits(eq, left > 8 ? 8 : left < 0 ? 0 : (int)left);
+      quota -= __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (y < ny) ob[y] = (unsigned char)(prev | gt);
   }
+  if (ranks > 1) cluster.sync();  // nobody leaves while its counters may be read
+}
+
+// CTAs per row: a power of two, as long as one wave of 148 holds all of them and each keeps 8192
+// columns, one byte of the bitmap per thread and pass (with 2048 columns per CTA 32 rows x 8191
+// bfloat16 scores took 20.4 us: the cluster barriers and the counters of the other CTAs cost more
+// than the passes)
+static inline int sah_select_ranks(int64_t rows, int64_t S) {
+  int ranks = 1;
+  while (ranks < SAH_SELECT_MAX_CLUSTER && rows * ranks * 2 <= 148 && S >= (int64_t)ranks * 2 * 8192) ranks *= 2;
+  return ranks;
+}
+
+// bytes of shared memory for the keys of a CTA's columns
+static inline int64_t sah_select_key_bytes(int64_t rows, int64_t S, int64_t W, int keybits) {
+  const int ranks = sah_select_ranks(rows, S);
+  return (W + ranks - 1) / ranks * 4 * keybits;
+}
+
+template <int KEYBITS, typename Keys>
+static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits, uint32_t* out_bits, int64_t rows,
+                                    int64_t S, int64_t W, int64_t col_begin, int64_t col_end, int64_t k,
+                                    cudaStream_t st) {
+  const int ranks = sah_select_ranks(rows, S);
+  // half-size CTAs for short rows and when rows queue for SMs
+  const int nt = W * 4 / ranks <= SAH_SELECT_MIN_THREADS || rows * ranks > 148 ? SAH_SELECT_MIN_THREADS
+                                                                                : SAH_SELECT_THREADS;
+  const int64_t key_bytes = sah_select_key_bytes(rows, S, W, KEYBITS);
+  const bool resident = key_bytes <= SAH_SELECT_KEY_BYTES;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(rows * ranks));
+  cfg.blockDim = dim3((unsigned)nt);
+  cfg.dynamicSmemBytes = resident ? (size_t)key_bytes : 0;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (resident) {
+    if (key_bytes > 24 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(sah_select_kernel<KEYBITS, Keys, true>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, SAH_SELECT_KEY_BYTES);
+      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "select attr: %s", cudaGetErrorString(e));
+    }
+    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, true>, keys, prev_bits, out_bits, S, W,
+                             col_begin, col_end, (long long)k);
+  } else {
+    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, false>, keys, prev_bits, out_bits, S, W,
+                             col_begin, col_end, (long long)k);
+  }
+  return SAH_OK;  // a launch error stays for SAH_LAUNCH_CHECK
 }

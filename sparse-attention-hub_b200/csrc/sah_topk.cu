@@ -202,28 +202,6 @@ extern "C" int sah_qk_scores(const void* q, const void* k, int dtype, int64_t qs
 // ---------------------------------------------------------------------------
 // Generic top-k over a score tensor.
 // ---------------------------------------------------------------------------
-template <typename T, int KEYBITS>
-struct ScoreKey {
-  const T* s;
-  __device__ __forceinline__ unsigned int operator()(int64_t j) const {
-    unsigned int key = sah_float_key(sah_to_float<T>(s[j]) + 0.0f);  // -0 ranks with +0
-    return KEYBITS == 16 ? (key >> 16) : key;
-  }
-};
-
-template <typename T, int KEYBITS>
-__global__ void __launch_bounds__(SAH_SELECT_THREADS)
-topk_select_kernel(const T* __restrict__ scores, int64_t S, int64_t W, int64_t col_begin,
-                   int64_t col_end, const uint32_t* __restrict__ prev_bits, int64_t k,
-                   uint32_t* __restrict__ out_bits) {
-  sah_pdl_entry();
-  __shared__ SahSelectSmem sm;
-  const int64_t row = blockIdx.x;
-  ScoreKey<T, KEYBITS> kf{scores + row * S};
-  sah_select_row<KEYBITS>(kf, prev_bits + row * W, out_bits + row * W, S, W, col_begin, col_end,
-                          k, sm);
-}
-
 extern "C" int sah_topk_select(const void* scores, int dtype, int64_t rows, int64_t S, int64_t W,
                                int64_t col_begin, int64_t col_end, const uint32_t* prev_bits,
                                int64_t k, uint32_t* out_bits, void* stream) {
@@ -233,11 +211,13 @@ extern "C" int sah_topk_select(const void* scores, int dtype, int64_t rows, int6
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_TOPK_SELECT, (cudaStream_t)stream);
   if (dtype == SAH_BF16) {
-    sah_launch_chain(topk_select_kernel<__nv_bfloat16, 16>, (unsigned)rows, SAH_SELECT_THREADS, 0, st,
-        (const __nv_bfloat16*)scores, S, W, col_begin, col_end, prev_bits, k, out_bits);
+    const SahScoreKeys<__nv_bfloat16, 16> keys{(const __nv_bfloat16*)scores, S};
+    const int rc = sah_select_launch<16>(keys, prev_bits, out_bits, rows, S, W, col_begin, col_end, k, st);
+    if (rc != SAH_OK) return rc;
   } else if (dtype == SAH_F32) {
-    sah_launch_chain(topk_select_kernel<float, 32>, (unsigned)rows, SAH_SELECT_THREADS, 0, st,
-        (const float*)scores, S, W, col_begin, col_end, prev_bits, k, out_bits);
+    const SahScoreKeys<float, 32> keys{(const float*)scores, S};
+    const int rc = sah_select_launch<32>(keys, prev_bits, out_bits, rows, S, W, col_begin, col_end, k, st);
+    if (rc != SAH_OK) return rc;
   } else {
     return sah_fail(SAH_ERR_INVALID, "topk_select: unknown dtype %d", dtype);
   }
@@ -772,6 +752,11 @@ extern "C" int sah_topk_select_ws(const void* scores, int dtype, int64_t rows, i
   if (col_begin < 0) col_begin = 0;
   if (col_end > S) col_end = S;
   cudaStream_t st = (cudaStream_t)stream;
+  // One launch, a cluster per row, while the keys of a CTA's columns fit in its shared memory; the
+  // grid-wide form for longer rows (32 rows of a million keys: four CTAs per row would leave most
+  // of the chip idle).
+  if (sah_select_key_bytes(rows, S, W, dtype == SAH_BF16 ? 16 : 32) <= SAH_SELECT_KEY_BYTES)
+    return sah_topk_select(scores, dtype, rows, S, W, col_begin, col_end, prev_bits, k, out_bits, stream);
   sah_prof_begin(SAH_PROF_TOPK_SELECT, st);
   int rc;
   if (dtype == SAH_BF16)

@@ -482,3 +482,61 @@ def test_hash_signatures_of_tiles_equal_those_of_single_vectors(dtype, widths, n
     for s0 in range(n0, n0 + n, 16):
         _native_ops.hash_encode(k, Hq, weights, biases, act, single, s0, min(n0 + n, s0 + 16))
     assert torch.equal(whole, single)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,S,k,b0,b1,dtype", [
+    (1, 131072, 2048, 64, 131072, "bf16"), (3, 16385, 300, 0, 16385, "f32"), (30, 8200, 82, 5, 8190, "bf16"),
+    (70, 4097, 1, 0, 4097, "f32"), (200, 519, 26, 0, 519, "bf16"), (2, 33, 32, 31, 33, "bf16"),
+    (5, 70000, 70000, 0, 70000, "bf16"), (4, 9000, 0, 0, 9000, "f32"), (2, 700000, 5000, 0, 700000, "bf16")])
+def test_topk_select_over_cluster_sizes(rows, S, k, b0, b1, dtype):
+    """Rows cut between 8, 4, 2 and 1 CTAs (and, for the longest, over the whole grid or with the
+    keys read again in every pass): the restatement's set, ties in column order across the cuts,
+    both signs of zero, column bounds inside a byte of the bitmap."""
+    from oracle import topk as o_topk
+
+    rng = np.random.default_rng(S + k)
+    x = rng.standard_normal((1, rows, 1, S)).astype(np.float32)
+    x[0, 0] = np.round(x[0, 0] * 2) / 2                  # a few hundred-fold ties, +0 and -0
+    x[0, rows - 1, 0, S // 3:] = 1.5                       # the cut inside one long run
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    sc = torch.from_numpy(x).to(DEV).to(dt)
+    active = rng.random((1, rows, 1, S)) < 0.05
+    prev = Mask.create_mask_from_dense_mask((1, rows, 1, S), torch.from_numpy(active.astype(np.float32)).to(DEV),
+                                            torch.float32)
+    want = o_topk.topk_inactive(sc.float().cpu().numpy(), active, k, b0, b1) | active
+    for per_row in (False, True):
+        sel = _native_ops.topk_select(sc, prev, k, b0, b1, per_row=per_row)
+        got = Mask._from_native((1, rows, 1, S), torch.float32, sel).get_dense_mask().cpu().numpy() != 0
+        np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Hq,Sq,S,k,dtype", [(1, 4, 1, 20000, 700, "bf16"), (2, 3, 24, 1031, 60, "bf16"),
+                                               (1, 5, 2, 260, 9, "f32")])
+def test_hash_topk_under_an_additive_mask(B, Hq, Sq, S, k, dtype):
+    """Hamming scores plus an additive mask (rounded to the dtype): rows over clusters, ragged
+    lengths, a mask shared by the heads with the lowest value, -inf and small offsets."""
+    from oracle import topk as o_topk
+
+    rng = np.random.default_rng(S)
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    cap = S + 3
+    kc = rng.integers(0, 2 ** 32, (B, Hq, cap), dtype=np.uint32)
+    kc[..., : S // 2] &= np.uint32(0xFF)
+    qc = rng.integers(0, 2 ** 32, (B, Hq, Sq), dtype=np.uint32)
+    am = torch.zeros((B, 1, Sq, S))
+    am[:, :, 0, S // 2: S // 2 + 50] = torch.finfo(dt).min
+    am[..., 7] = -float("inf")
+    am[..., 9] = 0.75
+    am = am.to(dt).to(DEV)
+    pop = np.array([bin(i).count("1") for i in range(65536)], np.int64)
+    d = kc[:, :, None, :S] ^ qc[..., None]
+    score = (32 - 2 * (pop[d & 0xFFFF] + pop[d >> 16])).astype(np.float32)
+    biased = (torch.from_numpy(score).to(DEV) + am.float()).to(dt).float().cpu().numpy()
+    active = rng.random((B, Hq, Sq, S)) < 0.1
+    prev = Mask.create_mask_from_dense_mask(active.shape, torch.from_numpy(active.astype(np.float32)).to(DEV), dt)
+    sel = _native_ops.hash_topk(torch.from_numpy(kc.view(np.int32)).to(DEV), S,
+                                torch.from_numpy(qc.view(np.int32)).to(DEV), 32, am, dt, prev, k, (B, Hq, Sq, S))
+    got = Mask._from_native(active.shape, dt, sel).get_dense_mask().float().cpu().numpy() != 0
+    np.testing.assert_array_equal(got, o_topk.topk_inactive(biased, active, k) | active)
