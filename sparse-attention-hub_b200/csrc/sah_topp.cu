@@ -20,9 +20,12 @@
 // added by one thread, run by run, and the scan starts again behind it (about a dozen times).
 //
 // A row is shared by a cluster of up to eight CTAs where there are few rows.  What bounds the
-// kernel is the instruction issue of the three passes over the row (maximum, histogram, emit;
-// the row stays in L1/L2).  128 rows x 65536 keys: 186 us with scalar loads, two gathers of the
-// weight per key from global memory and the accumulator replayed by one thread; 62 us now.
+// kernel is the instruction issue of the three passes over the row (maximum, histogram, emit), so
+// the logits of the first pass stay in shared memory (81920 columns per CTA; longer ranges are
+// converted again in every pass), the second replaces them by their bins, and where it can a pass
+// handles two 16-bit values per integer instruction.  128 rows x 65536 keys: 186 us with scalar
+// loads, two gathers of the weight per key from global memory and the accumulator replayed by one
+// thread; 62 us with the logits converted in every pass; 47 us now.
 // ---------------------------------------------------------------------------
 #include "sah_common.cuh"
 #include <cooperative_groups.h>
@@ -33,6 +36,7 @@
 #define TP_BINS (TP_D1 - TP_D0 + 2)  // bin 0: weight 1; bins 1 .. : d = TP_D0 ..; last bin: weight 0
 #define TP_PER 3                     // bins per thread
 #define TP_MAX_CLUSTER 8
+#define TP_ROW_BYTES (160 * 1024)    // logits of a CTA's columns in shared memory
 
 struct ToppArgs {
   const void* scores;      // [rows][S] unscaled q.k in bf16
@@ -87,13 +91,19 @@ __device__ __forceinline__ bool tp_add_run(float& acc, float v, unsigned int cou
   return true;
 }
 
-// bin of d = logit - maximum: ascending bins have descending weights.  A NaN (an infinite or NaN
-// logit) counts as weight 1.
-__device__ __forceinline__ int tp_bin(float d) {
-  const uint32_t b = __float_as_uint(d) >> 16;
-  if (b > 0xFF80u) return 0;
-  return min(max((int)b - (TP_D0 - 1), 0), TP_BINS - 1);
+// Bins of two values d = logit - maximum (packed bf16): ascending bins have descending weights.
+// As unsigned 16-bit numbers the d of bins 1 .. are TP_D0 .., the smaller magnitudes, +0 and the
+// positive not-a-number (an infinite or NaN logit; counts as weight 1) are below.
+__device__ __forceinline__ uint32_t tp_bins2(uint32_t d2) {
+  constexpr uint32_t LO = (TP_D0 - 1) * 0x00010001u, HI = TP_D1 * 0x00010001u;
+  return __vminu2(__vmaxu2(d2, LO), HI) - LO;  // neither half borrows
 }
+__device__ __forceinline__ uint32_t tp_pack2(float lo, float hi) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float tp_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float tp_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
 // 8 columns from column c0 of a row (zeros past the end); `vec`: rows are 16-byte aligned
 __device__ __forceinline__ void tp_load8(const __nv_bfloat16* __restrict__ s, int64_t c0, int64_t S, bool vec,
@@ -148,10 +158,12 @@ __device__ __forceinline__ TpMove tp_move(unsigned int vb, unsigned int count, i
   return r;
 }
 
+template <bool RESIDENT>
 __global__ void __launch_bounds__(TP_THREADS)
 topp_select_kernel(ToppArgs a) {
   sah_pdl_entry();
   namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) uint4 tp_row[];     // logits, then bins, of this CTA's columns
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ unsigned int hist[TP_PER * TP_THREADS];  // this CTA's counts; in rank 0 the row's
   __shared__ uint16_t weight[TP_PER * TP_THREADS];    // bf16 bits of exp(d) by bin
@@ -175,28 +187,37 @@ topp_select_kernel(ToppArgs a) {
   const bool vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
   const bool bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
   const unsigned char* pb = reinterpret_cast<const unsigned char*>(a.prev_bits + row * a.W);
-  const float lowest = __uint_as_float(0xFF7F0000u);   // the most negative finite bf16
 
   // the row in bytes of the bitmap, 8 columns each, cut into one range per CTA of the cluster
   const int64_t nb = a.W * 4;
-  const int64_t b_lo = nb * rank / ranks, b_hi = nb * (rank + 1) / ranks;
+  const int64_t b_lo = nb * rank / ranks;
+  const int ny = (int)(nb * (rank + 1) / ranks - b_lo);
+  pb += b_lo;
 
-  // scaled logits of a byte's columns, previously active positions pushed to the lowest value
-  // (:96-104)
-  auto logits = [&](int64_t byte, float* f) {
-    const int64_t c0 = byte * 8;
+  // scaled logits of a byte's columns, packed in pairs, previously active positions pushed to the
+  // lowest value (:96-104) and columns past the end to -inf
+  auto convert = [&](int y, uint32_t* w) {
+    const int64_t c0 = (b_lo + y) * 8;
+    float f[8];
     tp_load8(s, c0, a.S, vec, f);
-    const unsigned int act = pb[byte];
+    const unsigned int act = pb[y];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = sah_round_to<T>(__fmul_rn(f[i], a.scaling));
+    for (int i = 0; i < 4; ++i) w[i] = tp_pack2(__fmul_rn(f[2 * i], a.scaling), __fmul_rn(f[2 * i + 1], a.scaling));
     if (bias) {
       float bv[8];
       tp_load8(bias, c0, a.S, bias_vec, bv);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = sah_round_to<T>(__fadd_rn(f[i], bv[i]));
+      for (int i = 0; i < 4; ++i)
+        w[i] = tp_pack2(__fadd_rn(tp_lo(w[i]), bv[2 * i]), __fadd_rn(tp_hi(w[i]), bv[2 * i + 1]));
     }
+    if (act || c0 + 8 > a.S) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = (act >> i) & 1u ? lowest : f[i];
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t v = c0 + i >= a.S ? 0xFF80u : 0xFF7Fu;
+        if (((act >> i) & 1u) || c0 + i >= a.S)
+          w[i >> 1] = (i & 1) ? (w[i >> 1] & 0xFFFFu) | v << 16 : (w[i >> 1] & 0xFFFF0000u) | v;
+      }
+    }
   };
 
   for (int i = tid; i < TP_PER * TP_THREADS; i += TP_THREADS) {
@@ -207,13 +228,12 @@ topp_select_kernel(ToppArgs a) {
   }
 
   float mx = -INFINITY;
-  for (int64_t y = b_lo + tid; y < b_hi; y += TP_THREADS) {
-    if (y * 8 >= a.S) break;
-    float f[8];
-    logits(y, f);
+  for (int y = tid; y < ny; y += TP_THREADS) {
+    uint32_t w[4];
+    convert(y, w);
+    if (RESIDENT) tp_row[y] = make_uint4(w[0], w[1], w[2], w[3]);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (y * 8 + i < a.S) mx = fmaxf(mx, f[i]);
+    for (int i = 0; i < 4; ++i) mx = fmaxf(fmaxf(mx, tp_lo(w[i])), tp_hi(w[i]));
   }
   mx = tp_block_max(mx, scratch);
   if (ranks > 1) {
@@ -223,13 +243,33 @@ topp_select_kernel(ToppArgs a) {
   }
 
   // histogram over d
-  for (int64_t y = b_lo + tid; y < b_hi; y += TP_THREADS) {
-    if (y * 8 >= a.S) break;
-    float f[8];
-    logits(y, f);
+  auto bins = [&](int y, uint32_t* w) {
+    if (RESIDENT) {
+      const uint4 v = tp_row[y];
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else {
+      convert(y, w);
+    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (y * 8 + i < a.S) atomicAdd(&hist[tp_bin(sah_round_to<T>(__fsub_rn(f[i], mx)))], 1u);
+    for (int i = 0; i < 4; ++i)
+      w[i] = tp_bins2(tp_pack2(__fsub_rn(tp_lo(w[i]), mx), __fsub_rn(tp_hi(w[i]), mx)));
+  };
+  for (int y = tid; y < ny; y += TP_THREADS) {
+    uint32_t w[4];
+    bins(y, w);
+    if (RESIDENT) tp_row[y] = make_uint4(w[0], w[1], w[2], w[3]);
+    const int64_t left = a.S - (b_lo + y) * 8;
+    if (left >= 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        atomicAdd(&hist[w[i] & 0xFFFFu], 1u);
+        atomicAdd(&hist[w[i] >> 16], 1u);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < left) atomicAdd(&hist[(i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu], 1u);
+    }
   }
   __syncthreads();
   if (ranks > 1) {
@@ -377,16 +417,21 @@ topp_select_kernel(ToppArgs a) {
     last_bin = thr_sm;
   }
 
-  unsigned char* out = reinterpret_cast<unsigned char*>(a.out_bits + row * a.W);
-  for (int64_t y = b_lo + tid; y < b_hi; y += TP_THREADS) {
-    unsigned int bits = 0u;
-    if (y * 8 < a.S) {
-      float f[8];
-      logits(y, f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (y * 8 + i < a.S && tp_bin(sah_round_to<T>(__fsub_rn(f[i], mx))) <= last_bin) bits |= 1u << i;
+  unsigned char* out = reinterpret_cast<unsigned char*>(a.out_bits + row * a.W) + b_lo;
+  for (int y = tid; y < ny; y += TP_THREADS) {
+    uint32_t w[4];
+    if (RESIDENT) {
+      const uint4 v = tp_row[y];
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else {
+      bins(y, w);
     }
+    uint32_t bits = 0u;  // the sign of bin - (last_bin + 1)
+#pragma unroll
+    for (int i = 7; i >= 0; --i)
+      bits = __funnelshift_l(((i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu) - (uint32_t)(last_bin + 1), bits, 1);
+    const int64_t left = a.S - (b_lo + y) * 8;
+    if (left < 8) bits &= left <= 0 ? 0u : (1u << (int)left) - 1u;
     out[y] = (unsigned char)(a.or_prev ? (bits | pb[y]) : bits);
   }
 }
@@ -415,9 +460,17 @@ extern "C" int sah_topp_select(const void* scores, int dtype, float scaling, con
   int ranks = 1;
   while (ranks < TP_MAX_CLUSTER && rows * ranks * 2 <= 148 && S >= (int64_t)ranks * 2 * 8 * TP_THREADS) ranks *= 2;
   sah_prof_begin(SAH_PROF_TOPP, (cudaStream_t)stream);
+  const int64_t row_bytes = (W * 4 + ranks - 1) / ranks * 16;
+  const bool resident = row_bytes <= TP_ROW_BYTES;
+  if (resident) {
+    const cudaError_t e = cudaFuncSetAttribute(topp_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               TP_ROW_BYTES);
+    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "topp_select attr: %s", cudaGetErrorString(e));
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(rows * ranks));
   cfg.blockDim = dim3(TP_THREADS);
+  cfg.dynamicSmemBytes = resident ? (size_t)row_bytes : 0;
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -426,7 +479,9 @@ extern "C" int sah_topp_select(const void* scores, int dtype, float scaling, con
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  (void)cudaLaunchKernelEx(&cfg, topp_select_kernel, a);  // the error stays for SAH_LAUNCH_CHECK
+  // (a launch error stays for SAH_LAUNCH_CHECK)
+  if (resident) (void)cudaLaunchKernelEx(&cfg, topp_select_kernel<true>, a);
+  else (void)cudaLaunchKernelEx(&cfg, topp_select_kernel<false>, a);
   SAH_LAUNCH_CHECK("topp_select");
   sah_prof_end(SAH_PROF_TOPP, (cudaStream_t)stream);
   return SAH_OK;
