@@ -17,7 +17,7 @@
 // from the fixed-order kernel.  Both sums are within 129 * 2^-24 * sum|x_c p_c| of the exact
 // value (the tensor core at least as close), and sum|x_c p_c| <= |x| |p| with |x| <= 1.01 for a
 // transformed key, so a projection whose magnitude exceeds tau = 2^-15 * |p| has the same sign in
-// both.  The epilogue (two threads per key, alternate groups of 32 columns) shifts the 32 sign
+// both.  The epilogue (one thread per key) shifts the 32 sign
 // bits of a group into a word of the key's signature row, takes the smallest magnitude of the
 // group, and only where that is within the group's largest tau looks at the columns one by one;
 // groups that hold a projection within tau go through a small queue per warp (one global counter
@@ -32,8 +32,8 @@
 // have to be an 8-bit one), nor closer than 2^-17 to it, so a float product with 1 / M, 2^-22
 // away at most, rounds to the same bfloat16 number; operands near the ends of the range take the
 // division (a division per channel, its slow path's branch and the load in front of it in series
-// were most of the 1495 us that the kernel took at that size; now 629 us, and the
-// recheck 507 -> 121 us).
+// were most of the 1495 us that the kernel took at that size; 629 us with one set of producers that
+// branched per row; now 531 us, and the recheck 507 -> 121 us).
 //
 // Every mbarrier wait is bounded (sah_tcgen05.cuh); a wait that runs out sets the error word,
 // all roles leave their loops, tensor memory is freed.
@@ -43,8 +43,9 @@
 #define LTC_TILE 128
 #define LTC_NCHUNK 256   // hyperplanes per CTA
 #define LTC_KSTEPS 9     // 144 = 9 x 16 channels (129 used)
-#define LTC_EPI 8        // epilogue warps
-#define LTC_THREADS (32 * (LTC_EPI + 4 + 1))  // and 4 producer warps, 1 issuing warp
+#define LTC_EPI 4        // epilogue warps, one per 32 keys
+#define LTC_PROD 8       // producer warps, in two sets that take alternate tiles
+#define LTC_THREADS (32 * (LTC_EPI + LTC_PROD + 1))  // and 1 issuing warp
 #define LTC_QUEUE 64     // entries of a warp's queue of groups to redo
 #define LTC_TAU_SCALE 3.0517578125e-05f  // 2^-15
 
@@ -132,7 +133,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     *abort_sm = 0;
   }
-  if (warp == LTC_EPI + 4) {
+  if (warp == LTC_EPI + LTC_PROD) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::
                      "r"((uint32_t)__cvta_generic_to_shared(tmem_slot)),
                  "r"(512));
@@ -177,11 +178,11 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
   const uint32_t tmem = *tmem_slot;
   const float M = __uint_as_float(*max_bits);
 
-  if (warp >= LTC_EPI && warp < LTC_EPI + 4) {
+  if (warp >= LTC_EPI && warp < LTC_EPI + LTC_PROD) {
     // =========================== producers: transformed keys ===========================
     // 16 lanes cover one key row (8 channels each), two rows per pass, 32 rows per warp.
-    // The rows of the next tile are requested before the present one is handed over.
-    const int pw = warp - LTC_EPI;
+    // The rows of a set's next tile are requested before its present one is handed over.
+    const int pw = (warp - LTC_EPI) & 3, set = (warp - LTC_EPI) >> 2;
     const int my_chunk = lane & 15, my_sub = lane >> 4;
     const float rM = __frcp_rn(M);
     // the multiplication stands for the division only for a bfloat16 M well inside the range
@@ -200,9 +201,9 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
         if (key0 + it * 2 < s1) raw[it] = *reinterpret_cast<const uint4*>(kb + (key0 + it * 2) * ks_s);
       }
     };
-    if (my_tiles > 0) fetch(0);
-    for (int t = 0; t < my_tiles; ++t) {
-      const int buf = t & 1;
+    if (set < my_tiles) fetch(set);
+    for (int t = set; t < my_tiles; t += 2) {
+      const int buf = set;
       const int64_t flat = first + (int64_t)t * stride;
       const int64_t bh = flat / tiles_per_bh;
       const int64_t key0 = s0 + (flat - bh * tiles_per_bh) * LTC_TILE;
@@ -213,51 +214,61 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
       const float nk = key0 + pw * 32 + lane < s1 ? norms[bh * cap + key0 + pw * 32 + lane] : 0.f;
       if (t >= 2 && !aum_wait_warp(a_empty + buf * 8, (uint32_t)(((t >> 1) - 1) & 1), abort_sm, errflag)) break;
       unsigned char* at = sm + C::A_OFF + buf * C::A_TILE;
+      auto chunk_at = [&](int r) -> unsigned char* {
+        return at + (my_chunk >> 3) * C::A_ATOM + r * 128 + (((my_chunk & 7) ^ (r & 7)) << 4);
+      };
+      uint32_t slow = 0u;  // rows with an operand that has to be divided
 #pragma unroll
       for (int it = 0; it < 16; ++it) {
         const int r = pw * 32 + it * 2 + my_sub;
-        const bool live = key0 + r < s1;
-        float c[8];
-        sah_unpack8(raw[it], c);
-        bool slow = divide;
+        uint32_t w[4] = {raw[it].x, raw[it].y, raw[it].z, raw[it].w};
+        bool odd = divide;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (mean != nullptr) c[e] = sah_round_to<__nv_bfloat16>(__fsub_rn(c[e], m8[e]));
-          slow = slow || fabsf(c[e]) < 8.673617e-19f;  // 2^-60: a quotient that might be denormal (or zero)
+        for (int i = 0; i < 4; ++i) {
+          float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xffff0000u);
+          if (mean != nullptr) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(__fsub_rn(lo, m8[2 * i]), __fsub_rn(hi, m8[2 * i + 1]));
+            const uint32_t u = *reinterpret_cast<const uint32_t*>(&h);
+            lo = __uint_as_float(u << 16);
+            hi = __uint_as_float(u & 0xffff0000u);
+          }
+          // below 2^-60 the quotient might be denormal (or zero)
+          odd = odd || fabsf(lo) < 8.673617e-19f || fabsf(hi) < 8.673617e-19f;
+          const __nv_bfloat162 q = __floats2bfloat162_rn(__fmul_rn(lo, rM), __fmul_rn(hi, rM));
+          w[i] = *reinterpret_cast<const uint32_t*>(&q);
         }
-        if (slow && live) {
+        const bool live = key0 + r < s1;
+        if (odd && live) slow |= 1u << it;
+        *reinterpret_cast<uint4*>(chunk_at(r)) =
+            live ? make_uint4(w[0], w[1], w[2], w[3]) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      if (slow) {  // rare
+#pragma unroll 1
+        for (int it = 0; it < 16; ++it) {
+          if (!((slow >> it) & 1u)) continue;
+          const int r = pw * 32 + it * 2 + my_sub;
+          const __nv_bfloat16* kr = k + (bh / Hkv) * ks_b + (bh % Hkv) * ks_h + (key0 + r) * ks_s + my_chunk * 8;
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(chunk_at(r));
 #pragma unroll 1
           for (int e = 0; e < 8; ++e) {
-            float x = c[0];
-#pragma unroll
-            for (int f = 1; f < 8; ++f) x = e == f ? c[f] : x;
-            x = __fdiv_rn(x, M);
-#pragma unroll
-            for (int f = 0; f < 8; ++f) c[f] = e == f ? x : c[f];
+            float x = __bfloat162float(kr[e]);
+            if (mean != nullptr)
+              x = sah_round_to<__nv_bfloat16>(__fsub_rn(x, __bfloat162float(mean[bh * D + my_chunk * 8 + e])));
+            dst[e] = __float2bfloat16_rn(__fdiv_rn(x, M));
           }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) c[e] = live ? __fmul_rn(c[e], rM) : 0.f;
         }
-        uint4 v;
-        __nv_bfloat162 h;
-        h = __floats2bfloat162_rn(c[0], c[1]); v.x = *reinterpret_cast<const uint32_t*>(&h);
-        h = __floats2bfloat162_rn(c[2], c[3]); v.y = *reinterpret_cast<const uint32_t*>(&h);
-        h = __floats2bfloat162_rn(c[4], c[5]); v.z = *reinterpret_cast<const uint32_t*>(&h);
-        h = __floats2bfloat162_rn(c[6], c[7]); v.w = *reinterpret_cast<const uint32_t*>(&h);
-        *reinterpret_cast<uint4*>(at + (my_chunk >> 3) * C::A_ATOM + r * 128 + (((my_chunk & 7) ^ (r & 7)) << 4)) = v;
       }
       {  // channel 128: the augmentation column (chunk 0 of the third atom), one row per lane
         const int r = pw * 32 + lane;
         const float aug = key0 + r < s1 ? lsh_augment<__nv_bfloat16>(nk, M) : 0.f;
         *reinterpret_cast<__nv_bfloat16*>(at + 2 * C::A_ATOM + r * 128 + ((r & 7) << 4)) = __float2bfloat16_rn(aug);
       }
-      if (t + 1 < my_tiles) fetch(t + 1);
+      if (t + 2 < my_tiles) fetch(t + 2);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) aum_arrive(a_full + buf * 8);
     }
-  } else if (warp == LTC_EPI + 4) {
+  } else if (warp == LTC_EPI + LTC_PROD) {
     // =========================== tensor-core issuer ===========================
     if (lane == 0) {
       const uint32_t idesc = aum_idesc(false, false, n_mma);
@@ -279,9 +290,9 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
     }
     __syncwarp();
   } else {
-    // =================== epilogue: two threads per key, alternate column groups ===================
-    const int keyl = tid & 127, half = warp >> 2;  // warp w reads the tensor-memory lanes of quadrant w % 4
-    const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
+    // =========================== epilogue: one thread per key ===========================
+    const int keyl = tid;  // 0..127
+    const uint32_t lane_base = ((uint32_t)(warp * 32)) << 16;
     const int groups = (ncols + 31) / 32;
     LtcUncertain* queue = reinterpret_cast<LtcUncertain*>(sm + C::QUEUE_OFF) + warp * LTC_QUEUE;
     int queued = 0;  // the same in every lane
@@ -298,12 +309,12 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
     };
     // largest tau of each of this warp's groups; a group with columns past the end is looked at
     // one by one (a threshold that every magnitude is within)
-    for (int gq = half; gq < groups; gq += 2) {
+    for (int gq = 0; gq < groups; ++gq) {
       float g = tau_sm[gq * 32 + lane];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) g = fmaxf(g, __shfl_xor_sync(0xffffffffu, g, o));
       if (!(g >= 0.f)) g = INFINITY;  // a NaN among the hyperplanes
-      if (lane == 0 && (warp & 3) == 0) gtau_sm[gq] = gq * 32 + 32 <= ncols ? g : INFINITY;
+      if (lane == 0 && warp == 0) gtau_sm[gq] = gq * 32 + 32 <= ncols ? g : INFINITY;
     }
     asm volatile("bar.sync 1, %0;\n" ::"n"(LTC_EPI * 32) : "memory");
     for (int t = 0; t < my_tiles; ++t) {
@@ -314,7 +325,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
       if (!aum_wait_warp(d_full + buf * 8, (uint32_t)((t >> 1) & 1), abort_sm, errflag)) break;
       aum_fence_after();
       const int64_t row = bh * cap + s;
-      for (int gq = half; gq < groups; gq += 2) {
+      for (int gq = 0; gq < groups; ++gq) {
         uint32_t acc[32];
         ltc_tmem_ld32(tmem + lane_base + buf * LTC_NCHUNK + gq * 32, acc);
         uint32_t neg[4] = {0u, 0u, 0u, 0u};
@@ -366,7 +377,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
         }
       }
       // the row's padding bytes beyond the last table (the last chunk owns them)
-      if (blockIdx.y == gridDim.y - 1 && half == 0 && s < s1)
+      if (blockIdx.y == gridDim.y - 1 && s < s1)
         for (int bq = (col_base >> 3) + groups * 4; bq < LP; bq += 4)
           *reinterpret_cast<uint32_t*>(codes + row * LP + bq) = 0u;
       aum_fence_before();
@@ -377,7 +388,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
   }
   aum_fence_before();
   __syncthreads();
-  if (warp == LTC_EPI + 4) {
+  if (warp == LTC_EPI + LTC_PROD) {
     aum_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
   }
