@@ -71,6 +71,33 @@ template <>
 // same recipe reproduces the value (expf differs between libraries in the last place)
 __device__ __forceinline__ float ad_exp<float>(float x, const uint16_t*) { return (float)exp((double)x); }
 
+// Calls f(j) for the set bits j = threadIdx.x, threadIdx.x + 1024, ... below S of a bitmap, in that
+// order (1024 threads).  A thread's bits are the same bit of every 32nd word, so 32 words of a warp
+// are turned over (a 32 x 32 bit transposition, five exchanges) and each lane walks its own bits:
+// testing word after word, every warp went through the body for nearly all of them.
+template <typename F>
+__device__ __forceinline__ void ad_own_columns(const uint32_t* bits, int64_t S, F f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t words = (S + 31) / 32;
+  for (int64_t n0 = 0; n0 * 32 < words; n0 += 32) {  // words warp + 32 (n0 + lane)
+    const int64_t w = warp + 32 * (n0 + lane);
+    uint32_t m = w < words ? bits[w] : 0u;
+    if (w == words - 1 && (S & 31)) m &= (1u << (int)(S & 31)) - 1u;
+#pragma unroll
+    for (int o = 16, keep = 0x0000FFFF; o > 0; o >>= 1, keep ^= keep << o) {
+      // exchange the off-diagonal blocks of size o
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, m, o);
+      m = (lane & o) ? ((m & ~(uint32_t)keep) | ((other >> o) & (uint32_t)keep))
+                     : ((m & (uint32_t)keep) | ((other << o) & ~(uint32_t)keep));
+    }
+    while (m) {  // bit i: column lane of word warp + 32 (n0 + i)
+      const int i = __ffs(m) - 1;
+      m &= m - 1u;
+      f((warp + 32 * (n0 + i)) * 32 + lane);
+    }
+  }
+}
+
 struct AdaptiveArgs {
   const void* scores;      // [rows][S] unscaled q.k in dtype
   float scaling;
@@ -91,14 +118,26 @@ struct AdaptiveArgs {
   float* stats;  // optional [rows][4]: static denominator, std, estimated denominator, budget^2
 };
 
+// bfloat16 weights: exp rounds to 1 for |d| < 2^-10 and to 0 from |d| = 128 on; the part of the
+// table between (d negative) is kept in shared memory.
+#define AD_D0 0xBA80  // bf16 bits of -2^-10
+#define AD_D1 0xC300  // -128
+#define AD_ROW_BYTES (160 * 1024)  // logits of a bfloat16 row in shared memory: 81920 keys
+
 // One CTA (1024 threads) per mask row.  Every tensor operation of the reference is one
 // rounding to the dtype here; reductions use the fixed order above.
-template <typename T>
+// RESIDENT (bfloat16): the scaled logits of the row are formed once, eight at a time, and stay in
+// shared memory beside the table, because the sums visit scattered keys (the previous mask's, the
+// sample's) one after the other: with a load of the score and a gather of the weight from global
+// memory for each of them 128 rows x 65536 keys took 44.6 us, all of it latency; 19.3 us now.
+template <typename T, bool RESIDENT>
 __global__ void __launch_bounds__(1024)
 adaptive_budget_kernel(AdaptiveArgs a) {
   sah_pdl_entry();
-  extern __shared__ uint32_t ad_base_bits[];  // W words: distinct base-sample columns
+  extern __shared__ __align__(16) uint32_t ad_base_bits[];  // W words: distinct base-sample columns
   __shared__ float scratch[32];
+  __shared__ uint16_t table_sm[RESIDENT ? AD_D1 - AD_D0 : 1];
+  T* row_sm = reinterpret_cast<T*>(ad_base_bits + (a.W + 3) / 4 * 4);  // [W * 32] logits
   const int tid = threadIdx.x;
   const int64_t row = blockIdx.x;
   const int qi = (int)(row % a.Sq);
@@ -111,7 +150,7 @@ adaptive_budget_kernel(AdaptiveArgs a) {
                          : nullptr;
   const int64_t n = a.end - a.start;
 
-  auto logit = [&](int64_t j) {
+  auto make_logit = [&](int64_t j) {
     float t = sah_round_to<T>(__fmul_rn(sah_to_float<T>(s[j]), a.scaling));
     if (bias) t = sah_round_to<T>(__fadd_rn(t, sah_to_float<T>(bias[j])));
     return t;
@@ -120,31 +159,65 @@ adaptive_budget_kernel(AdaptiveArgs a) {
 
   // 1. row maximum over all keys
   float mx = -INFINITY;
-  for (int64_t j = tid; j < a.S; j += 1024) mx = fmaxf(mx, logit(j));
-  mx = sah_block_max(mx, scratch);
-  auto expw = [&](int64_t j) { return ad_exp<T>(sah_round_to<T>(__fsub_rn(logit(j), mx)), a.exp_table); };
+  if constexpr (RESIDENT) {
+    for (int i = tid; i < AD_D1 - AD_D0; i += 1024) table_sm[i] = a.exp_table[AD_D0 + i];
+    const bool vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
+    const bool bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
+    for (int64_t c0 = (int64_t)tid * 8; c0 < a.S; c0 += 1024 * 8) {
+      if (vec && (bias == nullptr || bias_vec) && c0 + 8 <= a.S) {
+        float f[8], bv[8];
+        sah_load8<T>(s + c0, f);
+        if (bias) sah_load8<T>(bias + c0, bv);
+        __align__(16) T out[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float t = sah_round_to<T>(__fmul_rn(f[i], a.scaling));
+          if (bias) t = sah_round_to<T>(__fadd_rn(t, bv[i]));
+          mx = fmaxf(mx, t);
+          out[i] = sah_from_float<T>(t);
+        }
+        *reinterpret_cast<uint4*>(row_sm + c0) = *reinterpret_cast<const uint4*>(out);
+      } else {
+        for (int64_t j = c0; j < c0 + 8 && j < a.S; ++j) {
+          const float t = make_logit(j);
+          mx = fmaxf(mx, t);
+          row_sm[j] = sah_from_float<T>(t);
+        }
+      }
+    }
+  } else {
+    for (int64_t j = tid; j < a.S; j += 1024) mx = fmaxf(mx, make_logit(j));
+  }
+  mx = sah_block_max(mx, scratch);  // (its barriers also publish the logits and the table)
+  auto expw = [&](int64_t j) {
+    if constexpr (RESIDENT) {
+      const float d = sah_round_to<T>(__fsub_rn(sah_to_float<T>(row_sm[j]), mx));
+      const uint32_t b = __float_as_uint(d) >> 16;
+      const uint32_t e = b - AD_D0 < AD_D1 - AD_D0 ? table_sm[b - AD_D0] : a.exp_table[b];
+      return __uint_as_float(e << 16);
+    } else {
+      return ad_exp<T>(sah_round_to<T>(__fsub_rn(make_logit(j), mx)), a.exp_table);
+    }
+  };
 
   // 2. static denominator: exp weights of the previous mask under its inverse weights
   float part = 0.f;
   const float unit_w = sah_inv_weight<T>(1.f);
   const uint32_t* pb = a.prev_bits ? a.prev_bits + row * a.W : nullptr;
-  for (int64_t j = tid; j < a.S; j += 1024) {
-    float term = 0.f;
-    if (pb == nullptr) {
-      term = expw(j);
-    } else {
-      const uint32_t word = pb[j >> 5];
-      const int bit = (int)(j & 31);
-      if ((word >> bit) & 1u) {
-        float w = unit_w;  // unit weights still pass through 1 / (1 + 1e-6)
-        if (a.prev_data != nullptr) {
-          const int64_t pos = a.ptr[row] + a.wpre[row * a.W + (j >> 5)] + __popc(word & ((1u << bit) - 1u));
-          w = sah_inv_weight<T>(sah_to_float<T>(reinterpret_cast<const T*>(a.prev_data)[pos]));
-        }
-        term = sah_round_to<T>(__fmul_rn(expw(j), w));
+  if (pb == nullptr) {
+    for (int64_t j = tid; j < a.S; j += 1024) part = __fadd_rn(part, expw(j));
+  } else {
+    // (the keys outside the mask would add +0)
+    ad_own_columns(pb, a.S, [&](int64_t j) {
+      float w = unit_w;  // unit weights still pass through 1 / (1 + 1e-6)
+      if (a.prev_data != nullptr) {
+        const uint32_t word = pb[j >> 5];
+        const int bit = (int)(j & 31);
+        const int64_t pos = a.ptr[row] + a.wpre[row * a.W + (j >> 5)] + __popc(word & ((1u << bit) - 1u));
+        w = sah_inv_weight<T>(sah_to_float<T>(reinterpret_cast<const T*>(a.prev_data)[pos]));
       }
-    }
-    part = __fadd_rn(part, term);
+      part = __fadd_rn(part, sah_round_to<T>(__fmul_rn(expw(j), w)));
+    });
   }
   const float static_den = sah_round_to<T>(sah_block_sum_fixed(part, scratch));
 
@@ -153,15 +226,35 @@ adaptive_budget_kernel(AdaptiveArgs a) {
     return a.base_draws ? a.base_draws[row * a.nb + i]
                         : sah_draw_column(a.seed, (uint64_t)(row * a.nb + i), a.start, n);
   };
+  // the weights of a thread's first four draws (5 % of 65536 keys) are kept for the second sum
+  constexpr int KEEP = 4;
+  float drawn[KEEP];
   part = 0.f;
-  for (int64_t i = tid; i < a.nb; i += 1024) {
+#pragma unroll
+  for (int n = 0; n < KEEP; ++n) {
+    const int64_t i = tid + n * 1024;
+    drawn[n] = 0.f;
+    if (i < a.nb) {
+      const int64_t c = base_col(i);
+      atomicOr(&ad_base_bits[c >> 5], 1u << (c & 31));
+      drawn[n] = expw(c);
+      part = __fadd_rn(part, drawn[n]);
+    }
+  }
+  for (int64_t i = tid + KEEP * 1024; i < a.nb; i += 1024) {
     const int64_t c = base_col(i);
     atomicOr(&ad_base_bits[c >> 5], 1u << (c & 31));
     part = __fadd_rn(part, expw(c));
   }
   const float mean = __fdiv_rn(sah_block_sum_fixed(part, scratch), (float)a.nb);
   part = 0.f;
-  for (int64_t i = tid; i < a.nb; i += 1024) {
+#pragma unroll
+  for (int n = 0; n < KEEP; ++n)
+    if (tid + n * 1024 < a.nb) {
+      const float d = __fsub_rn(drawn[n], mean);
+      part = __fadd_rn(part, __fmul_rn(d, d));
+    }
+  for (int64_t i = tid + KEEP * 1024; i < a.nb; i += 1024) {
     const float d = __fsub_rn(expw(base_col(i)), mean);
     part = __fadd_rn(part, __fmul_rn(d, d));
   }
@@ -174,10 +267,8 @@ adaptive_budget_kernel(AdaptiveArgs a) {
   const float w_base = sah_inv_weight<T>(p_base);
   __syncthreads();
   part = 0.f;
-  for (int64_t j = tid; j < a.S; j += 1024) {
-    if ((ad_base_bits[j >> 5] >> (j & 31)) & 1u)
-      part = __fadd_rn(part, sah_round_to<T>(__fmul_rn(expw(j), w_base)));
-  }
+  ad_own_columns(ad_base_bits, a.S,
+                 [&](int64_t j) { part = __fadd_rn(part, sah_round_to<T>(__fmul_rn(expw(j), w_base))); });
   const float sampled_den = sah_round_to<T>(sah_block_sum_fixed(part, scratch));
   const float est_den = sah_round_to<T>(__fadd_rn(static_den, sampled_den));
 
@@ -234,12 +325,23 @@ extern "C" int sah_adaptive_budget(const void* scores, int dtype, float scaling,
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_ADAPTIVE, st);
   SAH_DISPATCH_DTYPE(dtype, T, {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // bfloat16 rows that fit stay in shared memory; float32 weights come from a double-precision
+    // exponential, not from a table, and longer rows are read again
+    const size_t row_bytes = (size_t)W * 32 * sizeof(T);
+    if (sizeof(T) == 2 && row_bytes <= AD_ROW_BYTES) {
+      const size_t bytes = (size_t)(W + 3) / 4 * 16 + row_bytes;
+      cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, sizeof(T) == 2>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e));
+      sah_launch_chain(adaptive_budget_kernel<T, sizeof(T) == 2>, (unsigned)rows, 1024, bytes, st, a);
+    } else {
+      if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, false>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e));
+      }
+      sah_launch_chain(adaptive_budget_kernel<T, false>, (unsigned)rows, 1024, smem, st, a);
     }
-    sah_launch_chain(adaptive_budget_kernel<T>, (unsigned)rows, 1024, smem, st, a);
   });
   SAH_LAUNCH_CHECK("adaptive_budget");
   sah_prof_end(SAH_PROF_ADAPTIVE, st);
