@@ -292,6 +292,38 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
       dcol[j] = col < p.S ? __ldg(gd + col) : 1.f;
     }
   }
+  if (!LSH && RMAX == 4 && weighted) {
+    // Weights: the entries of eight words are requested together and then written (one dependent
+    // load per word and row in turn took 44 us for 32 groups x 65536 keys, 7 % of them selected;
+    // 27 us this way).
+#pragma unroll 1
+    for (int j0 = 0; j0 < 32; j0 += 8) {
+      T raw[8][RMAX];
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj)
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) {
+          const uint32_t wd = words_sm[wl][r][j0 + jj];
+          raw[jj][r] = sah_from_float<T>(0.f);
+          if ((wd >> lane) & 1u) raw[jj][r] = data[dbase_sm[wl][r][j0 + jj] + __popc(wd & lt)];
+        }
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        const int j = j0 + jj;
+        const uint32_t uj = union_sm[wl][j];
+        if (!((uj >> lane) & 1u)) continue;
+        const int64_t pos = list0 + before_sm[wl][j] + __popc(uj & lt);
+        unsigned int memb = 0u;
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) memb |= ((words_sm[wl][r][j] >> lane) & 1u) << r;
+        ucols[pos] = (int32_t)((c * PLAN_CHUNK_WORDS + j) * 32 + lane);
+        umemb[pos] = (uint16_t)memb;
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r)
+          if (r < p.R) uw[pos * p.R + r] = (memb >> r) & 1u ? sah_inv_weight<T>(sah_to_float<T>(raw[jj][r])) : 0.f;
+      }
+    }
+  } else {
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
     const uint32_t uj = union_sm[wl][j];
@@ -322,6 +354,7 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
         }
       }
     }
+  }
   }
   if (c == p.nchunks - 1) {
     int total = __shfl_sync(0xffffffffu, incl, 31);
