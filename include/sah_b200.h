@@ -231,8 +231,11 @@ int sah_topk_select(const void* scores, int dtype, int64_t rows, int64_t S, int6
                     int64_t col_begin, int64_t col_end, const uint32_t* prev_bits,
                     int64_t k, uint32_t* out_bits, void* stream);
 
-/* The same selection with every row spread over many CTAs (sah_topk_select gives
- * a row to one CTA, which leaves most SMs idle when there are few, long rows).
+/* 1 when the keys of such rows fit in the shared memory of the cluster of CTAs that
+ * sah_topk_select gives a row to (then it is the faster form), else 0. */
+int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W);
+/* The same selection for rows that do not fit: every row spread over the whole grid
+ * (calls sah_topk_select for rows that do).
  * Needs a 16-byte aligned device workspace of sah_topk_select_ws_bytes(rows, W)
  * bytes (SAH_ERR_WORKSPACE when smaller); rows <= 65535.  out_bits may alias
  * prev_bits.  Same result as sah_topk_select, bit for bit. */

@@ -737,6 +737,11 @@ static int sel_run(const T* scores, int64_t rows, int64_t S, int64_t W, int64_t 
   return SAH_OK;
 }
 
+extern "C" int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W) {
+  if (rows <= 0 || S <= 0 || W * 32 < S) return 0;
+  return sah_select_key_bytes(rows, S, W, dtype == SAH_BF16 ? 16 : 32) <= SAH_SELECT_KEY_BYTES ? 1 : 0;
+}
+
 extern "C" int sah_topk_select_ws(const void* scores, int dtype, int64_t rows, int64_t S, int64_t W,
                                   int64_t col_begin, int64_t col_end, const uint32_t* prev_bits,
                                   int64_t k, uint32_t* out_bits, void* workspace,
@@ -755,7 +760,7 @@ extern "C" int sah_topk_select_ws(const void* scores, int dtype, int64_t rows, i
   // One launch, a cluster per row, while the keys of a CTA's columns fit in its shared memory; the
   // grid-wide form for longer rows (32 rows of a million keys: four CTAs per row would leave most
   // of the chip idle).
-  if (sah_select_key_bytes(rows, S, W, dtype == SAH_BF16 ? 16 : 32) <= SAH_SELECT_KEY_BYTES)
+  if (sah_topk_select_fits(dtype, rows, S, W))
     return sah_topk_select(scores, dtype, rows, S, W, col_begin, col_end, prev_bits, k, out_bits, stream);
   sah_prof_begin(SAH_PROF_TOPK_SELECT, st);
   int rc;

@@ -20,6 +20,7 @@ from ctypes import (
     c_int64,
     c_void_p,
 )
+from functools import lru_cache
 from pathlib import Path
 from typing import Optional
 
@@ -76,6 +77,7 @@ _SIGNATURES = {
     "sah_qk_scores": [_P, _P, _I, _L, _L, _L, _L, _L, _L, _I, _I, _I, _I, _L, _I, _P, _L, _L,
                       _L, _P, _P],
     "sah_topk_select": [_P, _I, _L, _L, _L, _L, _L, _P, _L, _P, _P],
+    "sah_topk_select_fits": [_I, _L, _L, _L],  # returns 0 or 1
     "sah_topk_select_ws_bytes": [_L, _L],  # returns int64
     "sah_topk_sel_hist_offset": [_L, _L],  # returns int64
     "sah_topk_sel_begin": [_L, _L, _L, _P, _L, _P],
@@ -239,7 +241,18 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_of(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the current stream of a CUDA device (without building a `torch.cuda.Stream`)."""
+    idx = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if idx is None else idx)
+
+
+@lru_cache(maxsize=256)
+def attn_sizes(B: int, Hq: int, Hkv: int, Sq: int, S: int, D: int, has_data: int, sms: int) -> AttnSizes:
+    """`sah_attn_query_sizes`, a pure function of the extents; callers do not write to the result."""
+    sizes = AttnSizes()
+    check(load().sah_attn_query_sizes(B, Hq, Hkv, Sq, S, D, has_data, sms, ctypes.byref(sizes)),
+          "sah_attn_query_sizes")
+    return sizes
 
 
 _sm_count_cache: dict = {}

@@ -8,6 +8,7 @@ current CUDA stream of the tensors' device.
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -18,11 +19,13 @@ from .utils.mask import Mask, NativeBits, words_per_row
 
 
 def _rows(shape: Sequence[int]) -> int:
-    return int(np.prod(shape[:-1]))
+    return math.prod(shape[:-1])
 
 
 def bias_args(attention_mask: Optional[torch.Tensor], dtype: torch.dtype, n_keys: int):
     """(keep-alive tensor, pointer, stride_b, stride_h, stride_q) for an additive bias."""
+    if attention_mask is None:
+        return None, None, 0, 0, 0
     from .utils.mask_attention_utils import _bias_args
 
     return _bias_args(attention_mask, dtype, n_keys)
@@ -61,8 +64,9 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
                 per_row: bool = False) -> NativeBits:
     """previous | top-k of `scores` over inactive columns in [col_begin, col_end).
 
-    `per_row`: one CTA per row in a single launch instead of rows spread over many CTAs with
-    histograms in a scratch buffer; the better choice for many short rows (page scores)."""
+    `per_row`: the one-launch form (a cluster of CTAs per row) whatever the row length; otherwise
+    rows whose keys do not fit in a cluster's shared memory are spread over the whole grid, with
+    histograms in a scratch buffer."""
     _native.require_cuda(scores, "scores")
     lib = _native.load()
     S = scores.shape[-1]
@@ -72,7 +76,8 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
     sc = scores.contiguous()
     st = _native.stream_of(sc.device)
     end = S if col_end is None else col_end
-    if rows <= 65535 and not per_row:
+    if rows <= 65535 and not per_row and not lib.sah_topk_select_fits(_native.dtype_code(sc.dtype), rows, S,
+                                                                      prev.words):
         # rows are spread over many CTAs; the histograms live in a scratch buffer
         nbytes = int(lib.sah_topk_select_ws_bytes(rows, prev.words))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=sc.device)

@@ -20,6 +20,8 @@ maskers/fixed/implementations/basic_fixed.py:361-363).
 
 from __future__ import annotations
 
+import ctypes
+import math
 import warnings
 from typing import Literal, Optional, Tuple
 
@@ -30,13 +32,17 @@ from ... import _native
 
 
 def _n_rows(shape: Tuple[int, ...]) -> int:
-    return int(np.prod(shape[:-1])) if len(shape) > 1 else 1
+    return math.prod(shape[:-1])
 
 
 def words_per_row(n_cols: int) -> int:
     """Bitmap words per row: ceil(n/32) rounded up to 16 bytes."""
     w = (n_cols + 31) // 32
     return (w + 3) // 4 * 4
+
+
+# a fixed length, so that the array type is made once; a call reads what its band count says
+_BandArray = ctypes.c_int64 * (5 * 6)
 
 
 class NativeBits:
@@ -55,7 +61,7 @@ class NativeBits:
     __slots__ = ("_bits", "_lazy", "_data", "ptr", "wpre", "rows", "n_cols", "words", "deferred",
                  "_device")
 
-    MAX_BANDS = 6
+    MAX_BANDS = 6  # _BandArray's length
 
     def __init__(self, bits: Optional[torch.Tensor], rows: int, n_cols: int,
                  data: Optional[torch.Tensor] = None, zero_pending: bool = False,
@@ -142,11 +148,8 @@ class NativeBits:
         bands = lazy["bands"]
         if not lazy["zero"] and not bands:
             return
-        import ctypes
-
         lib = _native.load()
-        flat = [x for band in bands for x in band]
-        arr = (ctypes.c_int64 * max(len(flat), 1))(*flat)
+        arr = _BandArray(*[x for band in bands for x in band])
         _native.check(
             lib.sah_mask_fill_bands(self._bits.data_ptr(), self.rows, lazy["sq"], self.n_cols, self.words,
                                     len(bands), arr, int(lazy["zero"]),

@@ -121,16 +121,12 @@ def native_masked_attention(
     if has_data == 1:
         nb.ensure_scan()
 
-    sizes = _native.AttnSizes()
-    _native.check(lib.sah_attn_query_sizes(B, Hq, Hkv, Sq, S, D, has_data,
-                                           _native.sm_count(dev), ctypes.byref(sizes)),
-                  "sah_attn_query_sizes")
+    sms = _native.sm_count(dev)
+    sizes = _native.attn_sizes(B, Hq, Hkv, Sq, S, D, has_data, sms)
     if payload is not None and (sizes.rows_per_group > 4 or dtype != torch.bfloat16):
         payload, has_data = None, int(nb.data is not None)  # materialises the weights
         nb.ensure_scan()
-        _native.check(lib.sah_attn_query_sizes(B, Hq, Hkv, Sq, S, D, has_data,
-                                               _native.sm_count(dev), ctypes.byref(sizes)),
-                      "sah_attn_query_sizes")
+        sizes = _native.attn_sizes(B, Hq, Hkv, Sq, S, D, has_data, sms)
     # scratch is reused across calls of one shape; calls that could overlap on the device
     # (another stream, another host thread) get their own
     key = (dev.index, st, threading.get_ident(), B, Hq, Hkv, Sq, S, D, has_data)
@@ -147,8 +143,7 @@ def native_masked_attention(
     out = torch.empty((B, Sq, Hq, D), dtype=dtype, device=dev)
     rows = B * Hq * Sq
     part = torch.empty((rows, D + 2), dtype=torch.float32, device=dev) if return_partials else None
-    strides = (q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
-               v.stride(0), v.stride(1), v.stride(2))
+    strides = (*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
     try:
         if payload is not None:
             sig = payload.sig
