@@ -15,87 +15,92 @@
 // exact in fp32, so fma and mul+add agree there; fp32 inputs use an explicit
 // mul then add so that a CPU restatement without fma gets the same bits.
 // ---------------------------------------------------------------------------
+//
+// Bound by shared-memory reads (a key's own row and the broadcast query values) and, behind them,
+// the stream of K.  A thread therefore owns two keys where the head dimension is known, which
+// halves the query reads: 32 rows x 65536 keys x 4 sequences in bfloat16 (537 MB, 82 us at the
+// measured copy rate) 123 us with one key per thread, 113.7 us with two.
 #define QK_THREADS 128
-#define QK_MAXR 16
-#define QK_STAGES 1
-#define QK_TILES_PER_CTA 1
 
-// Two of those at once: sm_100 issues a pair of fp32 operations per instruction
-// (fma.rn.f32x2), each lane rounding exactly as the scalar fma; used for bf16 inputs, whose
+// Two partial sums at once: sm_100 issues a pair of fp32 operations per instruction
+// (fma.rn.f32x2), each half rounding exactly as the scalar fma; used for bf16 inputs, whose
 // products are exact in fp32.
 template <typename T>
-__device__ __forceinline__ void qk_mac2(float& c0, float& c1, float a0, float a1, float b0, float b1);
+__device__ __forceinline__ void qk_mac2(unsigned long long& c, unsigned long long a, unsigned long long b);
 template <>
-__device__ __forceinline__ void qk_mac2<__nv_bfloat16>(float& c0, float& c1, float a0, float a1,
-                                                       float b0, float b1) {
-  unsigned long long a, b, c;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(a0), "f"(a1));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(b0), "f"(b1));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(c) : "f"(c0), "f"(c1));
+__device__ __forceinline__ void qk_mac2<__nv_bfloat16>(unsigned long long& c, unsigned long long a,
+                                                       unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(c0), "=f"(c1) : "l"(c));
+}
+__device__ __forceinline__ float2 qk_halves(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
 }
 template <>
-__device__ __forceinline__ void qk_mac2<float>(float& c0, float& c1, float a0, float a1, float b0,
-                                               float b1) {
-  // fp32 inputs: a rounded product, then a rounded sum (no fma), one lane at a time
-  c0 = __fadd_rn(c0, __fmul_rn(a0, b0));
-  c1 = __fadd_rn(c1, __fmul_rn(a1, b1));
+__device__ __forceinline__ void qk_mac2<float>(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  // fp32 inputs: a rounded product, then a rounded sum, one half at a time (the assembler joins a
+  // packed product and a packed sum into one packed fma)
+  float2 cf = qk_halves(c);
+  const float2 af = qk_halves(a), bf = qk_halves(b);
+  cf.x = __fadd_rn(cf.x, __fmul_rn(af.x, bf.x));
+  cf.y = __fadd_rn(cf.y, __fmul_rn(af.y, bf.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(c) : "f"(cf.x), "f"(cf.y));
 }
-
+// eight elements of a key as four pairs of floats
 template <typename T>
-__device__ __forceinline__ float qk_mac(float a, float b, float c);
+__device__ __forceinline__ void qk_load_pairs(const T* p, unsigned long long* v);
 template <>
-__device__ __forceinline__ float qk_mac<__nv_bfloat16>(float a, float b, float c) {
-  return fmaf(a, b, c);
+__device__ __forceinline__ void qk_load_pairs<__nv_bfloat16>(const __nv_bfloat16* p, unsigned long long* v) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v[i]) : "r"(w[i] << 16), "r"(w[i] & 0xffff0000u));
 }
 template <>
-__device__ __forceinline__ float qk_mac<float>(float a, float b, float c) {
-  return __fadd_rn(c, __fmul_rn(a, b));
+__device__ __forceinline__ void qk_load_pairs<float>(const float* p, unsigned long long* v) {
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p), b = *reinterpret_cast<const ulonglong2*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
 // DT: head dim known at compile time (0: use the runtime value); FULL4: the number of rows
 // per KV head is a multiple of 4, so no row needs a bounds test.  Both only remove
 // instructions; the arithmetic is the same.
-template <typename T, int DT, bool FULL4>
-__global__ void __launch_bounds__(QK_THREADS, 5)
+// KEYS: keys per thread, QK_THREADS apart.
+template <typename T, int DT, bool FULL4, int KEYS>
+__global__ void __launch_bounds__(QK_THREADS, KEYS == 2 ? 3 : 5)
 qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b, int64_t qs_h,
                  int64_t qs_q, int64_t ks_b, int64_t ks_h, int64_t ks_s, int Hq, int Hkv, int Sq,
                  int64_t S, int D_rt, const T* __restrict__ bias, int64_t bias_s_b,
                  int64_t bias_s_h, int64_t bias_s_q, T* __restrict__ scores) {
   sah_pdl_entry();
+  constexpr int TILE = QK_THREADS * KEYS;
   extern __shared__ __align__(16) float q_sm[];  // [R][D] queries, then the K tile
   const int D = DT ? DT : D_rt;
   const int G = Hq / Hkv;
   const int R = G * Sq;  // rows sharing this KV head
   const int kvh = blockIdx.y, b = blockIdx.z;
-  // The CTA's QK_THREADS keys are copied to shared memory with coalesced 16-byte cp.async
-  // (a thread walking its own row in global memory would touch a new 128-byte line per
-  // load); rows are padded by 16 bytes so that the per-thread row reads do not collide.
+  // The CTA's keys are copied to shared memory with coalesced 16-byte cp.async (a thread walking
+  // its own row in global memory would touch a new 128-byte line per load); rows are padded by 16
+  // bytes so that the per-thread row reads do not collide.
   const int row_bytes = D * (int)sizeof(T);
   const int row_stride = row_bytes + 16;
-  const int stage_bytes = QK_THREADS * row_stride;
-  unsigned char* k_sm = reinterpret_cast<unsigned char*>(q_sm + R * D);  // QK_STAGES tiles
-  const int64_t n_tiles = (S + QK_THREADS - 1) / QK_THREADS;
-  const int64_t t_first = (int64_t)blockIdx.x * QK_TILES_PER_CTA;
-  const int64_t t_last = t_first + QK_TILES_PER_CTA < n_tiles ? t_first + QK_TILES_PER_CTA : n_tiles;
+  unsigned char* k_sm = reinterpret_cast<unsigned char*>(q_sm + R * D);
   const int cpr = row_bytes / 16;
-  const unsigned char* kbase = reinterpret_cast<const unsigned char*>(k + b * ks_b + kvh * ks_h);
-  const int64_t src_stride = ks_s * (int64_t)sizeof(T);
-  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(k_sm);
-  auto issue = [&](int64_t tile, int stage) {
-    const int64_t j0 = tile * QK_THREADS;
-    const int nkeys = (int)(S - j0 < QK_THREADS ? S - j0 : QK_THREADS);
-    const unsigned char* src = kbase + j0 * src_stride;
-    const uint32_t dst0 = sm0 + stage * stage_bytes;
+  const int64_t j0 = (int64_t)blockIdx.x * TILE;
+  {
+    const int nkeys = (int)(S - j0 < TILE ? S - j0 : TILE);
+    const int64_t src_stride = ks_s * (int64_t)sizeof(T);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(k + b * ks_b + kvh * ks_h) + j0 * src_stride;
+    const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(k_sm);
     for (int c = threadIdx.x; c < nkeys * cpr; c += QK_THREADS) {
       const int row = c / cpr, col = c - row * cpr;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst0 + row * row_stride + col * 16),
                    "l"(src + row * src_stride + col * 16));
     }
     asm volatile("cp.async.commit_group;\n" ::);
-  };
-  if (t_first < t_last) issue(t_first, 0);
+  }
   // Stage the group's queries as fp32: row r = g * Sq + qi.
   for (int idx = threadIdx.x; idx < R * D; idx += QK_THREADS) {
     int r = idx / D, d = idx - r * D;
@@ -103,58 +108,61 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
     q_sm[idx] = sah_to_float<T>(q[b * qs_b + (int64_t)(kvh * G + g) * qs_h + qi * qs_q + d]);
   }
   const int chunks = D / 8;
-  for (int64_t tile = t_first; tile < t_last; ++tile) {
-    const int stage = (int)((tile - t_first) & 1);
-    if (tile + 1 < t_last) {
-      issue(tile + 1, stage ^ 1);  // the other stage was released by the barrier below
-      asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::);
-    }
-    __syncthreads();
-    const int64_t j = tile * QK_THREADS + threadIdx.x;
-    if (j < S) {
-      const T* kr = reinterpret_cast<const T*>(k_sm + stage * stage_bytes + threadIdx.x * row_stride);
-      for (int r0 = 0; r0 < R; r0 += 4) {
-        float acc[4][8];
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  if (j0 + threadIdx.x >= S) return;  // (the thread's other key lies further on)
+  const unsigned char* kr = k_sm + threadIdx.x * row_stride;
+  for (int r0 = 0; r0 < R; r0 += 4) {
+    unsigned long long acc[KEYS][4][4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+    for (int u = 0; u < KEYS; ++u)
 #pragma unroll
-          for (int i = 0; i < 8; ++i) acc[r][i] = 0.f;
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[u][r][i] = 0ull;
 #pragma unroll(DT ? 4 : 1)
-        for (int t = 0; t < chunks; ++t) {
-          float kf[8];
-          sah_load8<T>(kr + t * 8, kf);
+    for (int t = 0; t < chunks; ++t) {
+      unsigned long long kp[KEYS][4];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            if (FULL4 || r0 + r < R) {
-              const float4 qa = *reinterpret_cast<const float4*>(q_sm + (r0 + r) * D + t * 8);
-              const float4 qb = *reinterpret_cast<const float4*>(q_sm + (r0 + r) * D + t * 8 + 4);
-              qk_mac2<T>(acc[r][0], acc[r][1], qa.x, qa.y, kf[0], kf[1]);
-              qk_mac2<T>(acc[r][2], acc[r][3], qa.z, qa.w, kf[2], kf[3]);
-              qk_mac2<T>(acc[r][4], acc[r][5], qb.x, qb.y, kf[4], kf[5]);
-              qk_mac2<T>(acc[r][6], acc[r][7], qb.z, qb.w, kf[6], kf[7]);
-            }
-          }
-        }
+      for (int u = 0; u < KEYS; ++u)  // (a key past the end: whatever lies there, not stored)
+        qk_load_pairs<T>(reinterpret_cast<const T*>(kr + u * QK_THREADS * row_stride) + t * 8, kp[u]);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          if (FULL4 || r0 + r < R) {
-            float s = __fadd_rn(__fadd_rn(__fadd_rn(acc[r][0], acc[r][1]), __fadd_rn(acc[r][2], acc[r][3])),
-                                __fadd_rn(__fadd_rn(acc[r][4], acc[r][5]), __fadd_rn(acc[r][6], acc[r][7])));
-            s = sah_round_to<T>(s);
-            const int rr = r0 + r, g = rr / Sq, qi = rr - g * Sq, h = kvh * G + g;
-            if (bias != nullptr) {
-              float bv = sah_to_float<T>(bias[b * bias_s_b + h * bias_s_h + qi * bias_s_q + j]);
-              s = sah_round_to<T>(__fadd_rn(s, bv));
-            }
-            const int64_t row = ((int64_t)b * Hq + h) * Sq + qi;
-            scores[row * S + j] = sah_from_float<T>(s);
+      for (int r = 0; r < 4; ++r) {
+        if (FULL4 || r0 + r < R) {
+          const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(q_sm + (r0 + r) * D + t * 8);
+          const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(q_sm + (r0 + r) * D + t * 8 + 4);
+#pragma unroll
+          for (int u = 0; u < KEYS; ++u) {
+            qk_mac2<T>(acc[u][r][0], qa.x, kp[u][0]);
+            qk_mac2<T>(acc[u][r][1], qa.y, kp[u][1]);
+            qk_mac2<T>(acc[u][r][2], qb.x, kp[u][2]);
+            qk_mac2<T>(acc[u][r][3], qb.y, kp[u][3]);
           }
         }
       }
     }
-    __syncthreads();  // the tile may be overwritten by the copy issued two iterations on
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (FULL4 || r0 + r < R) {
+        const int rr = r0 + r, g = rr / Sq, qi = rr - g * Sq, h = kvh * G + g;
+        const int64_t row = ((int64_t)b * Hq + h) * Sq + qi;
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+          const int64_t j = j0 + u * QK_THREADS + threadIdx.x;
+          if (j >= S) continue;
+          const float2 p0 = qk_halves(acc[u][r][0]), p1 = qk_halves(acc[u][r][1]);
+          const float2 p2 = qk_halves(acc[u][r][2]), p3 = qk_halves(acc[u][r][3]);
+          float s = __fadd_rn(__fadd_rn(__fadd_rn(p0.x, p0.y), __fadd_rn(p1.x, p1.y)),
+                              __fadd_rn(__fadd_rn(p2.x, p2.y), __fadd_rn(p3.x, p3.y)));
+          s = sah_round_to<T>(s);
+          if (bias != nullptr) {
+            float bv = sah_to_float<T>(bias[b * bias_s_b + h * bias_s_h + qi * bias_s_q + j]);
+            s = sah_round_to<T>(__fadd_rn(s, bv));
+          }
+          scores[row * S + j] = sah_from_float<T>(s);
+        }
+      }
+    }
   }
 }
 
@@ -171,28 +179,39 @@ extern "C" int sah_qk_scores(const void* q, const void* k, int dtype, int64_t qs
               "qk_scores: K rows must be 32-byte aligned");
   const int R = (Hq / Hkv) * Sq;
   const size_t elt = dtype == SAH_BF16 ? 2 : 4;
-  const size_t smem = (size_t)R * D * sizeof(float) + (size_t)QK_STAGES * QK_THREADS * (D * elt + 16);
+  size_t smem = (size_t)R * D * sizeof(float) + (size_t)QK_THREADS * (D * elt + 16);
   if (smem > 200 * 1024)
     return sah_fail(SAH_ERR_UNSUPPORTED, "qk_scores: %d query rows per KV head do not fit", R);
-  dim3 grid((unsigned)sah_ceil_div(sah_ceil_div(S, QK_THREADS), QK_TILES_PER_CTA), (unsigned)Hkv, (unsigned)B);
+  // Two keys per thread for the head dimensions that are compiled in, as long as three tiles fit
+  // on an SM beside the queries and the smaller grid still has four CTAs per SM (below that the
+  // first tile's latency, not the reads, is what a launch takes).
+  const int64_t pairs = sah_ceil_div(S, (int64_t)QK_THREADS * 2) * Hkv * B;
+  const bool two = (D == 128 || D == 64) && R % 4 == 0 && pairs >= 4 * 148 &&
+                   smem + (size_t)QK_THREADS * (D * elt + 16) <= 75 * 1024;
+  if (two) smem += (size_t)QK_THREADS * (D * elt + 16);
+  const dim3 grid((unsigned)sah_ceil_div(S, (int64_t)QK_THREADS * (two ? 2 : 1)), (unsigned)Hkv, (unsigned)B);
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_QK_SCORES, (cudaStream_t)stream);
-#define QK_LAUNCH(T, DT, F4)                                                                        \
+#define QK_LAUNCH(T, DT, F4, KEYS)                                                                  \
   do {                                                                                              \
     if (smem > 48 * 1024) {                                                                         \
-      cudaError_t e = cudaFuncSetAttribute(qk_scores_kernel<T, DT, F4>,                             \
+      cudaError_t e = cudaFuncSetAttribute(qk_scores_kernel<T, DT, F4, KEYS>,                       \
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "qk_scores attr: %s", cudaGetErrorString(e)); \
     }                                                                                               \
-    sah_launch_chain(qk_scores_kernel<T, DT, F4>, grid, QK_THREADS, smem, st, \
+    sah_launch_chain(qk_scores_kernel<T, DT, F4, KEYS>, grid, QK_THREADS, smem, st, \
         (const T*)q, (const T*)k, qs_b, qs_h, qs_q, ks_b, ks_h, ks_s, Hq, Hkv, Sq, S, D,            \
         (const T*)bias, bias_s_b, bias_s_h, bias_s_q, (T*)scores);                                  \
   } while (0)
   const bool full4 = (R % 4) == 0;
   SAH_DISPATCH_DTYPE(dtype, T, {
-    if (D == 128 && full4) QK_LAUNCH(T, 128, true);
-    else if (D == 64 && full4) QK_LAUNCH(T, 64, true);
-    else QK_LAUNCH(T, 0, false);
+    if (two && D == 128) QK_LAUNCH(T, 128, true, 2);
+    else if (two) QK_LAUNCH(T, 64, true, 2);
+    else if (D == 128 && full4) QK_LAUNCH(T, 128, true, 1);
+    else if (D == 64 && full4) QK_LAUNCH(T, 64, true, 1);
+    else if (D == 128) QK_LAUNCH(T, 128, false, 1);
+    else if (D == 64) QK_LAUNCH(T, 64, false, 1);
+    else QK_LAUNCH(T, 0, false, 1);
   });
   SAH_LAUNCH_CHECK("qk_scores");
   sah_prof_end(SAH_PROF_QK_SCORES, (cudaStream_t)stream);

@@ -540,3 +540,30 @@ def test_hash_topk_under_an_additive_mask(B, Hq, Sq, S, k, dtype):
                                 torch.from_numpy(qc.view(np.int32)).to(DEV), 32, am, dt, prev, k, (B, Hq, Sq, S))
     got = Mask._from_native(active.shape, dt, sel).get_dense_mask().float().cpu().numpy() != 0
     np.testing.assert_array_equal(got, o_topk.topk_inactive(biased, active, k) | active)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,S,D,masked", [
+    (1, 4, 1, 1, 1, 128, False), (2, 3, 3, 1, 17, 128, True), (1, 16, 2, 1, 1003, 128, False),
+    (1, 6, 2, 3, 333, 64, True), (3, 2, 2, 1, 64, 64, False), (1, 8, 2, 24, 79, 128, True),
+    (1, 4, 2, 2, 140, 80, True), (1, 6, 2, 1, 1601, 64, True), (1, 8, 8, 1, 30000, 128, False)])
+def test_score_bits_at_the_edges(dtype, B, Hq, Hkv, Sq, S, D, masked):
+    """q.k bit for bit in the fixed order: group sizes that are no multiple of four, key counts
+    around the 16-key groups of a warp, more rows than stay in registers, head dims with and
+    without the four-lane kernel, strided keys and queries."""
+    torch.manual_seed(S + D)
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    q = torch.randn((B, Sq, Hq, D), device=DEV).to(dt).transpose(1, 2)
+    k = torch.randn((B, S, Hkv, D + 8), device=DEV).to(dt)[..., :D].transpose(1, 2)
+    am = None
+    if masked:
+        am = torch.zeros((B, 1, Sq, S + 3), device=DEV).to(dt)
+        am[:, :, 0, S // 2:] = torch.finfo(dt).min
+        am[..., 0] = 0.37
+    got = _native_ops.qk_scores(q, k, am).float().cpu().numpy()
+    n = min(S, 1100)  # the ends of a long row
+    cols = np.r_[0:n, S - n:S]
+    want = o_qk.qk_scores(q.float().cpu().numpy(), k[:, :, cols].float().cpu().numpy(), dtype,
+                          None if am is None else am[..., cols].float().cpu().numpy())
+    np.testing.assert_array_equal(got[..., cols], want)
