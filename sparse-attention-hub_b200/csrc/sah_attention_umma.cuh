@@ -587,11 +587,18 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
 // keys 99 against 108 us; 64K keys 63 against 73 us (two waves from 512K down: 337, 185 and
 // 111 us -- a CTA's prologue, pipeline fill and merge are paid once per SM instead of twice).  64 KV groups with lists of a few
 // thousand rows (HashAttention and Quest at B = 8, S = 32768): 63 against 69 us and 56 against
-// 61 us.  In between -- 8 to 32 groups with lists of 10^4..10^5 rows -- the mma.sync kernel,
-// with two CTAs per SM and lower fixed costs, was ahead by 5-40 % (measured with two waves).
+// 61 us.  8 groups and fewer, whole decode step:
+// Sink + Local 20.6 against 24.2 us (1024 keys), 21.3 against 22.7 (4096); oracle top-k 30.8 against
+// 32.9 (2048), 39.5 against 41.4 (8192); hash 37.8 against 43.8 us (4096 keys), 40.1 against 45.5 (8192), 43.9 against 45.3 (16384); Quest
+// 38.2 against 42.0 (8192); PQCache 131072 keys 81.7 against 86.1; top-p 74.0 against 76.6 (8192),
+// 147.5 against 150.3 (65536); MagicPig 45.9 against 54.6 (8192), 54.5 against 58.4 (16384), 94.9
+// against 105.9 (65500), and with 16 groups 96.4 against 104.4 (32768).  In between -- 16 to 32
+// groups with lists of 10^4..10^5 rows -- the mma.sync kernel, with two CTAs per SM and lower fixed
+// costs, is ahead or even (top-p, 32 groups of 65536 keys: 369 against 394 us; MagicPig, 32 groups
+// of 49152: 207 against 209).
 #define AUM_DEFAULT_MIN_KEYS (64 * 1024)
 static bool aum_default(bool lsh, int64_t S, int groups) {
-  return (lsh && S >= AUM_DEFAULT_MIN_KEYS) || (groups >= 64 && S <= 65536);
+  return (lsh && S >= AUM_DEFAULT_MIN_KEYS) || (groups >= 64 && S <= 65536) || groups <= (lsh ? 16 : 8);
 }
 
 // The kernel choice: a process-wide setting (sah_attn_select_kernel), else SAH_ATTN_UMMA in the
