@@ -225,13 +225,14 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
 // centroid's keys, each adding half of the channels into fp64 registers that live across the
 // strips; the registers go to global memory with one atomic per (centroid, channel) and CTA.
 // Bound: shared-memory integer atomics and L2 (every 32-byte sector of a key is fetched by the
-// CTAs of two sub-vectors).  8 KV heads x 65472 keys x 16 sub-vectors: 134 us; with one fp64
-// shared-memory atomic per key and channel -- a compare-and-swap loop -- it took 812 us.
+// CTAs of two sub-vectors).  8 KV heads x 65472 keys x 16 sub-vectors: 96 us with eight keys of a
+// centroid in flight, 122 us with four and three CTAs per SM; with one fp64 shared-memory atomic
+// per key and channel -- a compare-and-swap loop -- it took 812 us.
 #define PQA_THREADS 512
 #define PQA_STRIP 4096
 
 template <typename T>
-__global__ void __launch_bounds__(PQA_THREADS, 3)
+__global__ void __launch_bounds__(PQA_THREADS, 2)
 pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
                      int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int vec8,
                      const uint8_t* __restrict__ codes, int64_t cap, double* __restrict__ sums,
@@ -283,25 +284,33 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
     int e = start_sm[cent];
     count += e1 - e;
     const T* xs = xg + j0 * xs_s;
-    if (sizeof(T) == 2 && vec8) {  // four channels in 8 aligned bytes; four keys in flight
-      for (; e + 4 <= e1; e += 4) {
-        uint2 v[4];
+    if (sizeof(T) == 2 && vec8) {  // four channels in 8 aligned bytes; eight keys in flight
+      for (; e + 8 <= e1; e += 8) {
+        uint2 v[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u] * xs_s);
+        for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u] * xs_s);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 8; ++u) {
           acc[0] += (double)__uint_as_float(v[u].x << 16);
           acc[1] += (double)__uint_as_float(v[u].x & 0xffff0000u);
           acc[2] += (double)__uint_as_float(v[u].y << 16);
           acc[3] += (double)__uint_as_float(v[u].y & 0xffff0000u);
         }
       }
-      for (; e < e1; ++e) {
-        const uint2 v = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e] * xs_s);
-        acc[0] += (double)__uint_as_float(v.x << 16);
-        acc[1] += (double)__uint_as_float(v.x & 0xffff0000u);
-        acc[2] += (double)__uint_as_float(v.y << 16);
-        acc[3] += (double)__uint_as_float(v.y & 0xffff0000u);
+      {  // the last few, all in flight as well
+        uint2 v[8];
+        const int left = e1 - e;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          v[u] = u < left ? *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u] * xs_s) : make_uint2(0u, 0u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (u < left) {
+            acc[0] += (double)__uint_as_float(v[u].x << 16);
+            acc[1] += (double)__uint_as_float(v[u].x & 0xffff0000u);
+            acc[2] += (double)__uint_as_float(v[u].y << 16);
+            acc[3] += (double)__uint_as_float(v[u].y & 0xffff0000u);
+          }
       }
     } else {
       for (; e < e1; ++e) {
@@ -333,9 +342,9 @@ extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t
   if (sub_d > PQ_MAX_SUBD || n_cent > 256)
     return sah_fail(SAH_ERR_UNSUPPORTED, "pq_accumulate: sub-vector dim %d (<= %d) / %d centroids (<= 256)",
                     sub_d, PQ_MAX_SUBD, n_cent);
-  // one wave of three CTAs per SM; the strips of a slice share the CTA's registers
+  // one wave of two CTAs per SM; the strips of a slice share the CTA's registers
   const int64_t groups = (int64_t)B * Hkv * n_sub;
-  int64_t slices = (int64_t)3 * 148 / groups;
+  int64_t slices = (int64_t)2 * 148 / groups;
   if (slices < 1) slices = 1;
   const int64_t strips = sah_ceil_div(n_keys, (int64_t)PQA_STRIP);
   if (slices > strips) slices = strips;
@@ -369,21 +378,29 @@ __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t 
   float move = 0.f;
   const int c = threadIdx.x;
   if (c < n_cent) {
+    // everything that may be needed is requested before the first use (a channel at a time, each
+    // with its own loads, took 16 to 29 us for 128 groups of 256 centres; 4.3 us this way)
     const int cnt = counts[grp * n_cent + c];
-    float d2 = 0.f;
-    for (int d = 0; d < sub_d; ++d) {
-      float nv;
-      if (cnt > 0) {
-        nv = __fdiv_rn((float)sums[(grp * n_cent + c) * sub_d + d], (float)cnt);
-      } else {
-        const int64_t j = reseed[grp * n_cent + c];
-        nv = sah_to_float<T>(x[b * xs_b + kvh * xs_h + (j + init_offset) * xs_s + sub * sub_d + d]);
-      }
-      float* cp = centroids + (grp * n_cent + c) * sub_d + d;
-      const float t = __fsub_rn(nv, *cp);
-      d2 = __fadd_rn(d2, __fmul_rn(t, t));
-      *cp = nv;
+    const double* sp = sums + (grp * n_cent + c) * sub_d;
+    float* cp = centroids + (grp * n_cent + c) * sub_d;
+    double sv[PQ_MAX_SUBD];
+    float old[PQ_MAX_SUBD];
+#pragma unroll
+    for (int d = 0; d < PQ_MAX_SUBD; ++d) {
+      sv[d] = d < sub_d ? sp[d] : 0.0;
+      old[d] = d < sub_d ? cp[d] : 0.f;
     }
+    const T* xr = nullptr;
+    if (cnt <= 0) xr = x + b * xs_b + kvh * xs_h + (reseed[grp * n_cent + c] + init_offset) * xs_s + sub * sub_d;
+    float d2 = 0.f;
+#pragma unroll
+    for (int d = 0; d < PQ_MAX_SUBD; ++d)
+      if (d < sub_d) {
+        const float nv = cnt > 0 ? __fdiv_rn((float)sv[d], (float)cnt) : sah_to_float<T>(xr[d]);
+        const float t = __fsub_rn(nv, old[d]);
+        d2 = __fadd_rn(d2, __fmul_rn(t, t));
+        cp[d] = nv;
+      }
     move = sqrtf(d2);
   }
   float total;
