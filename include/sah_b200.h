@@ -231,6 +231,11 @@ int sah_topk_select(const void* scores, int dtype, int64_t rows, int64_t S, int6
                     int64_t col_begin, int64_t col_end, const uint32_t* prev_bits,
                     int64_t k, uint32_t* out_bits, void* stream);
 
+/* The same when the previous mask is nothing but bands on an empty bitmap (bands as for
+ * sah_mask_fill_bands; row r has query position r % Sq): no bitmap is read. */
+int sah_topk_select_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S,
+                          int64_t W, int64_t col_begin, int64_t col_end, int n_bands,
+                          const int64_t* bands, int64_t k, uint32_t* out_bits, void* stream);
 /* 1 when the keys of such rows fit in the shared memory of the cluster of CTAs that
  * sah_topk_select gives a row to (then it is the faster form), else 0. */
 int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W);
@@ -603,6 +608,12 @@ int sah_attn_plan(const uint32_t* bits, const void* data, const int32_t* wpre,
                   const int64_t* ptr, int dtype, int B, int Hq, int Hkv, int Sq, int64_t S,
                   int64_t W, const sah_attn_sizes* sizes, int32_t* ucols, uint16_t* umemb,
                   float* uw, int32_t* ucount, void* stream);
+
+/* The same for a mask that is nothing but bands on an empty bitmap (sink and local window; bands
+ * as for sah_mask_fill_bands, unit weights), without the bitmap; S <= 32768. */
+int sah_attn_plan_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv,
+                        int Sq, int64_t S, const sah_attn_sizes* sizes, int32_t* ucols,
+                        uint16_t* umemb, int32_t* ucount, void* stream);
 
 /* The same for a MagicPig mask whose weights sah_masked_attention_lsh evaluates itself
  * (sizes queried with has_data = 2; at most 4 mask rows per KV group).  `bits` are the

@@ -136,9 +136,13 @@ template <typename T, int RMAX>
 __global__ void __launch_bounds__(PLAN_FUSED_THREADS)
 attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ data,
                        const int32_t* __restrict__ wpre, const int64_t* __restrict__ ptr,
-                       PlanGeom p, int32_t* __restrict__ ucols, uint16_t* __restrict__ umemb,
-                       float* __restrict__ uw, int32_t* __restrict__ ucount) {
+                       PlanGeom p, const __grid_constant__ MaskBands bands, int32_t* __restrict__ ucols,
+                       uint16_t* __restrict__ umemb, float* __restrict__ uw, int32_t* __restrict__ ucount) {
   sah_pdl_entry_early();
+  // word of a mask row: from the bitmap, or (no bitmap) from the mask's bands
+  auto row_word = [&](int64_t row, int64_t wi) -> uint32_t {
+    return bits != nullptr ? bits[row * p.W + wi] : sah_band_bits(bands, row % p.Sq, wi * 32, 32, p.S, 0u);
+  };
   __shared__ int scan[33];
   __shared__ int64_t rows_sm[RMAX];
   const int64_t g = blockIdx.x;
@@ -157,7 +161,7 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
     uint32_t ua = 0u;
 #pragma unroll
     for (int r = 0; r < RMAX; ++r)
-      if (rows[r] >= 0) ua |= bits[rows[r] * p.W + wa];
+      if (rows[r] >= 0) ua |= row_word(rows[r], wa);
     ahead += __popc(ua);
   }
 #pragma unroll
@@ -167,7 +171,7 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
     if (w < p.Wv && rows[r] >= 0) {
       // wpre counts every set bit of the caller's words; bits past S are dropped after
       // the CSR offsets were taken from the unmasked prefix (they can only sit last)
-      words[r] = plan_word(p, bits[rows[r] * p.W + w], w);
+      words[r] = plan_word(p, row_word(rows[r], w), w);
       if (uw != nullptr && words[r]) dbase[r] = ptr[rows[r]] + wpre[rows[r] * p.W + w];
     }
     u |= words[r];
@@ -386,13 +390,10 @@ static int plan_geometry(int B, int Hq, int Hkv, int Sq, int64_t S, int64_t W,
   return SAH_OK;
 }
 
-extern "C" int sah_attn_plan(const uint32_t* bits, const void* data, const int32_t* wpre,
-                             const int64_t* ptr, int dtype, int B, int Hq, int Hkv, int Sq,
-                             int64_t S, int64_t W, const sah_attn_sizes* sizes, int32_t* ucols,
-                             uint16_t* umemb, float* uw, int32_t* ucount, void* stream) {
-  SAH_REQUIRE(bits && sizes && ucols && umemb && ucount, "attn_plan: null pointer");
-  SAH_REQUIRE(data == nullptr || (wpre && ptr && uw), "attn_plan: data needs wpre, ptr and uw");
-  SAH_REQUIRE(W * 32 >= S, "attn_plan: W too small");
+static int attn_plan_impl(const uint32_t* bits, const MaskBands& bands, const void* data, const int32_t* wpre,
+                          const int64_t* ptr, int dtype, int B, int Hq, int Hkv, int Sq,
+                          int64_t S, int64_t W, const sah_attn_sizes* sizes, int32_t* ucols,
+                          uint16_t* umemb, float* uw, int32_t* ucount, void* stream) {
   PlanGeom p;
   int rc0 = plan_geometry(B, Hq, Hkv, Sq, S, W, sizes, &p);
   if (rc0 != SAH_OK) return rc0;
@@ -403,15 +404,17 @@ extern "C" int sah_attn_plan(const uint32_t* bits, const void* data, const int32
   const int64_t blocks = sah_ceil_div(warps * 32, threads);
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_ATTN_PLAN, (cudaStream_t)stream);
+  if (bits == nullptr && p.Wv > 1024)
+    return sah_fail(SAH_ERR_UNSUPPORTED, "attn_plan_bands: %lld keys (at most 32768)", (long long)S);
   if (p.Wv <= 1024) {
     const dim3 fgrid((unsigned)groups, (unsigned)sah_ceil_div(p.Wv, PLAN_FUSED_THREADS));
     SAH_DISPATCH_DTYPE(dtype, T, {
       if (p.R <= 4)
         sah_launch_chain(attn_plan_fused_kernel<T, 4>, fgrid, PLAN_FUSED_THREADS, 0, st, bits, (const T*)data,
-            wpre, ptr, p, ucols, umemb, data ? uw : nullptr, ucount);
+            wpre, ptr, p, bands, ucols, umemb, data ? uw : nullptr, ucount);
       else
         sah_launch_chain(attn_plan_fused_kernel<T, AT_MAXR>, fgrid, PLAN_FUSED_THREADS, 0, st, bits,
-            (const T*)data, wpre, ptr, p, ucols, umemb, data ? uw : nullptr, ucount);
+            (const T*)data, wpre, ptr, p, bands, ucols, umemb, data ? uw : nullptr, ucount);
     });
     SAH_LAUNCH_CHECK("attn_plan_fused");
     sah_prof_end(SAH_PROF_ATTN_PLAN, (cudaStream_t)stream);
@@ -433,6 +436,28 @@ extern "C" int sah_attn_plan(const uint32_t* bits, const void* data, const int32
   SAH_LAUNCH_CHECK("attn_plan_emit");
   sah_prof_end(SAH_PROF_ATTN_PLAN, (cudaStream_t)stream);
   return SAH_OK;
+}
+
+extern "C" int sah_attn_plan(const uint32_t* bits, const void* data, const int32_t* wpre,
+                             const int64_t* ptr, int dtype, int B, int Hq, int Hkv, int Sq,
+                             int64_t S, int64_t W, const sah_attn_sizes* sizes, int32_t* ucols,
+                             uint16_t* umemb, float* uw, int32_t* ucount, void* stream) {
+  SAH_REQUIRE(bits && sizes && ucols && umemb && ucount, "attn_plan: null pointer");
+  SAH_REQUIRE(data == nullptr || (wpre && ptr && uw), "attn_plan: data needs wpre, ptr and uw");
+  SAH_REQUIRE(W * 32 >= S, "attn_plan: W too small");
+  return attn_plan_impl(bits, MaskBands(), data, wpre, ptr, dtype, B, Hq, Hkv, Sq, S, W, sizes, ucols, umemb, uw,
+                        ucount, stream);
+}
+
+extern "C" int sah_attn_plan_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv, int Sq,
+                                   int64_t S, const sah_attn_sizes* sizes, int32_t* ucols, uint16_t* umemb,
+                                   int32_t* ucount, void* stream) {
+  SAH_REQUIRE(sizes && ucols && umemb && ucount, "attn_plan_bands: null pointer");
+  SAH_REQUIRE(n_bands >= 0 && n_bands <= SAH_MAX_BANDS && (n_bands == 0 || bands != nullptr),
+              "attn_plan_bands: 0..%d bands", SAH_MAX_BANDS);
+  SAH_REQUIRE(S > 0 && Sq > 0, "attn_plan_bands: bad extents");
+  return attn_plan_impl(nullptr, sah_make_bands(n_bands, bands), nullptr, nullptr, nullptr, dtype, B, Hq, Hkv, Sq, S,
+                        (S + 31) / 32, sizes, ucols, umemb, nullptr, ucount, stream);
 }
 
 extern "C" int sah_attn_plan_lsh(const uint32_t* bits, const uint32_t* unit_bits, const float* dens,

@@ -143,6 +143,48 @@ __device__ __forceinline__ V sah_block_excl_scan(V c, V* scratch, V* total) {
     }                                                                  \
   } while (0)
 
+// ---- band edits of a bitmap --------------------------------------------------------
+// The sink and local-window part of a mask, as its bands: [lo_base + q lo_qstep, hi_base + q
+// hi_qstep) of the row with query position q is set (value 1) or cleared (0), in order.  Kernels
+// that read such a mask once take the bands instead of a bitmap that a launch of its own fills.
+#define SAH_MAX_BANDS 6
+struct MaskBands {
+  int n;
+  int64_t lo_base[SAH_MAX_BANDS], lo_qstep[SAH_MAX_BANDS], hi_base[SAH_MAX_BANDS], hi_qstep[SAH_MAX_BANDS];
+  int value[SAH_MAX_BANDS];
+};
+static inline MaskBands sah_make_bands(int n_bands, const int64_t* bands) {
+  MaskBands mb;
+  mb.n = n_bands;
+  for (int i = 0; i < SAH_MAX_BANDS; ++i) {
+    const bool on = i < n_bands;
+    mb.lo_base[i] = on ? bands[5 * i + 0] : 0;
+    mb.lo_qstep[i] = on ? bands[5 * i + 1] : 0;
+    mb.hi_base[i] = on ? bands[5 * i + 2] : 0;
+    mb.hi_qstep[i] = on ? bands[5 * i + 3] : 0;
+    mb.value[i] = on ? (int)bands[5 * i + 4] : 0;
+  }
+  return mb;
+}
+// the bands applied to `v`, the bits of columns [c0, c0 + width) (width <= 32) of a row of S columns
+__device__ __forceinline__ uint32_t sah_band_bits(const MaskBands& bands, int64_t q, int64_t c0, int width, int64_t S,
+                                                  uint32_t v) {
+#pragma unroll
+  for (int i = 0; i < SAH_MAX_BANDS; ++i) {
+    if (i >= bands.n) break;
+    int64_t lo = bands.lo_base[i] + q * bands.lo_qstep[i];
+    int64_t hi = bands.hi_base[i] + q * bands.hi_qstep[i];
+    if (lo < 0) lo = 0;
+    if (hi > S) hi = S;
+    if (hi <= c0 || lo >= c0 + width || lo >= hi) continue;
+    const int a = lo > c0 ? (int)(lo - c0) : 0;                  // first bit
+    const int b = hi < c0 + width ? (int)(hi - c0) : width;      // one past the last
+    const uint32_t m = (b >= 32 ? 0xffffffffu : ((1u << b) - 1u)) & ~((1u << a) - 1u);
+    if (bands.value[i]) v |= m; else v &= ~m;
+  }
+  return v;
+}
+
 // ---- launch accounting and optional per-kernel event timing -------------------
 // Slots name the kernels whose device time a caller may want in isolation.
 enum SahProfSlot {

@@ -99,8 +99,9 @@ struct SahScoreKeys<float, 32> {
 
 template <int KEYBITS, typename Keys, bool RESIDENT>
 __global__ void __launch_bounds__(SAH_SELECT_THREADS)
-sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, uint32_t* __restrict__ out_bits, int64_t S,
-                  int64_t W, int64_t col_begin, int64_t col_end, long long k) {
+sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __grid_constant__ MaskBands bands, int Sq,
+                  uint32_t* __restrict__ out_bits, int64_t S, int64_t W, int64_t col_begin, int64_t col_end,
+                  long long k) {
   sah_pdl_entry();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -118,7 +119,8 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, uint32_t* _
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int64_t row = blockIdx.x / ranks;
   keys.open(row);
-  const unsigned char* pb = reinterpret_cast<const unsigned char*>(prev_bits + row * W);
+  // the previous mask: a bitmap, or (no bitmap) its bands
+  const unsigned char* pb = prev_bits == nullptr ? nullptr : reinterpret_cast<const unsigned char*>(prev_bits + row * W);
   unsigned char* ob = reinterpret_cast<unsigned char*>(out_bits + row * W);
   if (col_begin < 0) col_begin = 0;
   if (col_end > S) col_end = S;
@@ -128,13 +130,35 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, uint32_t* _
   const int ny = (int)(y_hi - y_lo);
   const int blocks = (ny + 31) / 32;
   const int q_lo = (int)((int64_t)blocks * warp / nw), q_hi = (int)((int64_t)blocks * (warp + 1) / nw);
-  pb += y_lo;
+  if (pb != nullptr) pb += y_lo;
   ob += y_lo;
+  // bytes [gap_lo, gap_hi) of this CTA lie between the bands that begin the row and the others:
+  // nearly all of them, and empty
+  const int64_t qpos = row % Sq;
+  int gap_lo = 0, gap_hi = 0;
+  if (pb == nullptr) {
+    int64_t a = 0, e = S;
+#pragma unroll
+    for (int i = 0; i < SAH_MAX_BANDS; ++i) {
+      if (i >= bands.n) break;
+      const int64_t lo = bands.lo_base[i] + qpos * bands.lo_qstep[i], hi = bands.hi_base[i] + qpos * bands.hi_qstep[i];
+      if (lo <= 0) a = hi > a ? hi : a;
+      else e = lo < e ? lo : e;
+    }
+    a = (a + 7) / 8 - y_lo;
+    e = e / 8 - y_lo;
+    gap_lo = (int)(a < 0 ? 0 : a > ny ? ny : a);
+    gap_hi = (int)(e < 0 ? 0 : e > ny ? ny : e);
+  }
+  auto previous = [&](int y) -> unsigned int {
+    if (pb != nullptr) return pb[y];
+    return y >= gap_lo && y < gap_hi ? 0u : sah_band_bits(bands, qpos, (y_lo + y) * 8, 8, S, 0u);
+  };
   // columns of byte y (of this CTA) that compete
   auto competing = [&](int y) -> unsigned int {
     const int64_t c0 = (y_lo + y) * 8;
     if (c0 >= col_end || c0 + 8 <= col_begin) return 0u;
-    unsigned int m = ~(unsigned int)pb[y] & 255u;
+    unsigned int m = ~previous(y) & 255u;
     if (c0 < col_begin) m &= 255u << (int)(col_begin - c0);
     if (c0 + 8 > col_end) m &= (1u << (int)(col_end - c0)) - 1u;
     return m;
@@ -317,7 +341,7 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, uint32_t* _
   }
   for (int q = q_lo; q < q_hi; ++q) {
     const int y = q * 32 + lane;
-    const unsigned int prev = y < ny ? pb[y] : 0u;
+    const unsigned int prev = y < ny ? previous(y) : 0u;
     unsigned int gt = 0u, eq = 0u;
     if (mode == 1) {
       if (y < ny) gt = competing(y);
@@ -371,7 +395,7 @@ static inline int64_t sah_select_key_bytes(int64_t rows, int64_t S, int64_t W, i
 template <int KEYBITS, typename Keys>
 static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits, uint32_t* out_bits, int64_t rows,
                                     int64_t S, int64_t W, int64_t col_begin, int64_t col_end, int64_t k,
-                                    cudaStream_t st) {
+                                    cudaStream_t st, const MaskBands& bands = MaskBands(), int Sq = 1) {
   const int ranks = sah_select_ranks(rows, S);
   // half-size CTAs for short rows and when rows queue for SMs
   const int nt = W * 4 / ranks <= SAH_SELECT_MIN_THREADS || rows * ranks > 148 ? SAH_SELECT_MIN_THREADS
@@ -396,11 +420,11 @@ static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, SAH_SELECT_KEY_BYTES);
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "select attr: %s", cudaGetErrorString(e));
     }
-    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, true>, keys, prev_bits, out_bits, S, W,
-                             col_begin, col_end, (long long)k);
+    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, true>, keys, prev_bits, bands, Sq,
+                             out_bits, S, W, col_begin, col_end, (long long)k);
   } else {
-    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, false>, keys, prev_bits, out_bits, S, W,
-                             col_begin, col_end, (long long)k);
+    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, false>, keys, prev_bits, bands, Sq,
+                             out_bits, S, W, col_begin, col_end, (long long)k);
   }
   return SAH_OK;  // a launch error stays for SAH_LAUNCH_CHECK
 }

@@ -72,12 +72,21 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
     S = scores.shape[-1]
     rows = _rows(scores.shape)
     prev = previous_mask.native_bits()
-    dst = out if out is not None else NativeBits(torch.empty_like(prev.bits), rows, S)
     sc = scores.contiguous()
     st = _native.stream_of(sc.device)
     end = S if col_end is None else col_end
-    if rows <= 65535 and not per_row and not lib.sah_topk_select_fits(_native.dtype_code(sc.dtype), rows, S,
-                                                                      prev.words):
+    dst = out if out is not None else NativeBits(
+        torch.empty((prev.rows, prev.words), dtype=torch.int32, device=sc.device), rows, S)
+    fits = lib.sah_topk_select_fits(_native.dtype_code(sc.dtype), rows, S, prev.words)
+    bands = prev.pending_bands() if fits and prev.rows == rows else None
+    if bands is not None:
+        # the previous mask is a sink and a window that nobody has needed as a bitmap so far
+        _native.check(
+            lib.sah_topk_select_bands(sc.data_ptr(), _native.dtype_code(sc.dtype), rows, bands[2], S, prev.words,
+                                      col_begin, end, bands[0], bands[1], k, dst.bits.data_ptr(), st),
+            "sah_topk_select_bands")
+        return dst
+    if rows <= 65535 and not per_row and not fits:
         # rows are spread over many CTAs; the histograms live in a scratch buffer
         nbytes = int(lib.sah_topk_select_ws_bytes(rows, prev.words))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=sc.device)

@@ -142,6 +142,17 @@ class NativeBits:
         self.ptr = None   # the CSR companions describe the old bits
         self.wpre = None
 
+    def pending_bands(self):
+        """(number of bands, host array, query rows per (batch, head)) of a bitmap that is nothing
+        but noted bands on an empty mask, else None.  A kernel that takes the bands saves the
+        launch that would fill the words; the notes stay, so whoever asks for the words gets
+        them."""
+        lazy = self._lazy
+        if self._bits is None or not lazy["zero"]:
+            return None
+        bands = lazy["bands"]
+        return len(bands), _BandArray(*[x for band in bands for x in band]), lazy["sq"]
+
     def flush(self) -> None:
         """Apply the pending clear and band edits with one launch."""
         lazy = self._lazy

@@ -168,12 +168,19 @@ def native_masked_attention(
                     _native.ptr(part), _native.ptr(dump), st),
                 "sah_masked_attention_lsh")
         else:
-            _native.check(
-                lib.sah_attn_plan(nb.bits.data_ptr(), _native.ptr(nb.data), _native.ptr(nb.wpre),
-                                  _native.ptr(nb.ptr), code, B, Hq, Hkv, Sq, S, nb.words,
-                                  ctypes.byref(sizes), ws["ucols"].data_ptr(), ws["umemb"].data_ptr(),
-                                  _native.ptr(ws["uw"]) if has_data else None, ws["ucount"].data_ptr(), st),
-                "sah_attn_plan")
+            bands = nb.pending_bands() if has_data == 0 and S <= 32768 and nb.rows == B * Hq * Sq else None
+            if bands is not None and bands[2] == Sq:
+                _native.check(
+                    lib.sah_attn_plan_bands(bands[0], bands[1], code, B, Hq, Hkv, Sq, S, ctypes.byref(sizes),
+                                            ws["ucols"].data_ptr(), ws["umemb"].data_ptr(),
+                                            ws["ucount"].data_ptr(), st), "sah_attn_plan_bands")
+            else:
+                _native.check(
+                    lib.sah_attn_plan(nb.bits.data_ptr(), _native.ptr(nb.data), _native.ptr(nb.wpre),
+                                      _native.ptr(nb.ptr), code, B, Hq, Hkv, Sq, S, nb.words,
+                                      ctypes.byref(sizes), ws["ucols"].data_ptr(), ws["umemb"].data_ptr(),
+                                      _native.ptr(ws["uw"]) if has_data else None, ws["ucount"].data_ptr(), st),
+                    "sah_attn_plan")
             _native.check(
                 lib.sah_masked_attention(
                     q.data_ptr(), k.data_ptr(), v.data_ptr(), code, *strides,

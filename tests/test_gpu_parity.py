@@ -567,3 +567,34 @@ def test_score_bits_at_the_edges(dtype, B, Hq, Hkv, Sq, S, D, masked):
     want = o_qk.qk_scores(q.float().cpu().numpy(), k[:, :, cols].float().cpu().numpy(), dtype,
                           None if am is None else am[..., cols].float().cpu().numpy())
     np.testing.assert_array_equal(got[..., cols], want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,S,Sq,stack", [
+    ("f32", 700, 1, "fixed"), ("bf16", 131, 3, "fixed"), ("bf16", 32768, 1, "fixed"), ("bf16", 33000, 2, "fixed"),
+    ("bf16", 4097, 1, "topk"), ("f32", 1000, 4, "topk"), ("bf16", 90000, 1, "topk"), ("bf16", 260, 2, "topk")])
+def test_band_masks_without_a_bitmap(dtype, S, Sq, stack, monkeypatch):
+    """A mask of bands alone (sink and window, the future cleared for several query positions) goes
+    to the selection and to the attention plan as bands: the same masks and the same output as
+    with the bitmap filled first."""
+    from sparse_attention_hub.sparse_attention.utils.mask import NativeBits
+
+    torch.manual_seed(S)
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    q = torch.randn((2, 4, Sq, 64), device=DEV).to(dt)
+    k, v = (torch.randn((2, 2, S, 64), device=DEV).to(dt) for _ in range(2))
+    maskers = [("sink", {"sink_size": 5}), ("local", {"window_size": 37})]
+    if stack == "topk":
+        maskers.append(("oracle_topk", {"heavy_size": 0.05}))
+    ra = workloads.research_attention(maskers, dtype, DEV)
+
+    def run():
+        mask = ra.build_mask(q, k, v, None, 0.125, 0.0, {}, layer_idx=0)
+        out = get_masked_attention_output(None, q, k, v, None, None, 0.125, 0.0, mask)
+        return out, mask.get_dense_mask()
+
+    out, dense = run()
+    monkeypatch.setattr(NativeBits, "pending_bands", lambda self: None)
+    want_out, want_dense = run()
+    assert torch.equal(dense, want_dense)
+    assert torch.equal(out, want_out)
