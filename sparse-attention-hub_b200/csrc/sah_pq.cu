@@ -483,7 +483,7 @@ pq_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs
   const int entries = n_sub * n_cent;
   const int Dh = n_sub * sub_d;
   Entry* lut = reinterpret_cast<Entry*>(pq_sm_raw);                  // [n_sub][n_cent]
-  float* q_sm = reinterpret_cast<float*>(lut + entries);             // [PQ_ROWS][Dh]
+  float* q_sm = reinterpret_cast<float*>(lut + entries);             // [Dh][PQ_ROWS]
   for (int idx = threadIdx.x; idx < PQ_ROWS * Dh; idx += PQ_TILE) {
     const int rr = idx / Dh, d = idx - rr * Dh;
     const int r = rblk * PQ_ROWS + rr;
@@ -492,36 +492,52 @@ pq_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs
       const int g = r / Sq, qi = r - g * Sq;
       v = sah_to_float<T>(q[b * qs_b + (int64_t)(kvh * G + g) * qs_h + qi * qs_q + d]);
     }
-    q_sm[idx] = v;
+    q_sm[d * PQ_ROWS + rr] = v;
   }
   __syncthreads();
   constexpr int PER16 = 16 / (int)sizeof(T);  // elements per 16-byte load
-  for (int idx = threadIdx.x; idx < entries; idx += PQ_TILE) {
-    const int sub = idx / n_cent;
-    const T* cp = centroids + (bk * n_sub * (int64_t)n_cent + idx) * sub_d;
-    float acc[PQ_ROWS] = {0.f, 0.f, 0.f, 0.f};
+  // Four entries of a thread at a time, their centroids' first 16 bytes (all of them, for 8 bf16
+  // channels) requested together; channels ascending.
+  constexpr int AHEAD = 4;
+  const int log_cent = (n_cent & (n_cent - 1)) == 0 ? 31 - __clz(n_cent) : -1;  // a division per entry otherwise
+  for (int idx0 = threadIdx.x; idx0 < entries; idx0 += AHEAD * PQ_TILE) {
+    uint4 first[AHEAD];
     if constexpr (VEC) {
-      for (int d0 = 0; d0 < sub_d; d0 += PER16) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(cp + d0);
-        const T* cv = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-        for (int e = 0; e < PER16; ++e) {
-          const float c = sah_to_float<T>(cv[e]);
-#pragma unroll
-          for (int rr = 0; rr < PQ_ROWS; ++rr) acc[rr] = fmaf(q_sm[rr * Dh + sub * sub_d + d0 + e], c, acc[rr]);
-        }
-      }
-    } else {
-      for (int d = 0; d < sub_d; ++d) {
-        const float c = sah_to_float<T>(cp[d]);
-#pragma unroll
-        for (int rr = 0; rr < PQ_ROWS; ++rr) acc[rr] = fmaf(q_sm[rr * Dh + sub * sub_d + d], c, acc[rr]);
-      }
+      for (int n = 0; n < AHEAD; ++n)
+        if (idx0 + n * PQ_TILE < entries)
+          first[n] = *reinterpret_cast<const uint4*>(centroids + (bk * n_sub * (int64_t)n_cent + idx0 + n * PQ_TILE) * sub_d);
     }
-    float out[PQ_ROWS];
 #pragma unroll
-    for (int rr = 0; rr < PQ_ROWS; ++rr) out[rr] = (rblk * PQ_ROWS + rr < R) ? sah_round_to<T>(acc[rr]) : 0.f;
-    lut[idx] = PqEntry<T>::pack(out);
+    for (int n = 0; n < AHEAD; ++n) {
+      const int idx = idx0 + n * PQ_TILE;
+      if (idx >= entries) break;
+      const int sub = log_cent >= 0 ? idx >> log_cent : idx / n_cent;
+      const T* cp = centroids + (bk * n_sub * (int64_t)n_cent + idx) * sub_d;
+      const float4* qv = reinterpret_cast<const float4*>(q_sm) + sub * sub_d;
+      float acc[PQ_ROWS] = {0.f, 0.f, 0.f, 0.f};
+      auto channel = [&](float c, const float4& x) {
+        acc[0] = fmaf(x.x, c, acc[0]);
+        acc[1] = fmaf(x.y, c, acc[1]);
+        acc[2] = fmaf(x.z, c, acc[2]);
+        acc[3] = fmaf(x.w, c, acc[3]);
+      };
+      if constexpr (VEC) {
+        uint4 raw = first[n];
+        for (int d0 = 0; d0 < sub_d; d0 += PER16) {
+          if (d0 > 0) raw = *reinterpret_cast<const uint4*>(cp + d0);
+          const T* cv = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+          for (int e = 0; e < PER16; ++e) channel(sah_to_float<T>(cv[e]), qv[d0 + e]);
+        }
+      } else {
+        for (int d = 0; d < sub_d; ++d) channel(sah_to_float<T>(cp[d]), qv[d]);
+      }
+      float out[PQ_ROWS];
+#pragma unroll
+      for (int rr = 0; rr < PQ_ROWS; ++rr) out[rr] = (rblk * PQ_ROWS + rr < R) ? sah_round_to<T>(acc[rr]) : 0.f;
+      lut[idx] = PqEntry<T>::pack(out);
+    }
   }
   __syncthreads();
   const bool vec = (n_sub == 16) && ((reinterpret_cast<uintptr_t>(codes) & 15) == 0);
@@ -534,11 +550,20 @@ pq_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs
   }
   const int64_t j0 = (int64_t)blockIdx.x * keys_per_cta;
   const int64_t j1 = j0 + keys_per_cta < n_keys ? j0 + keys_per_cta : n_keys;
+  // the codes of the next two keys of a thread are requested before the present one is scored
+  uint4 ahead[2];
+  auto fetch = [&](int64_t j) -> uint4 {
+    return vec && j < j1 ? *reinterpret_cast<const uint4*>(codes + (bk * cap + j) * n_sub) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  ahead[0] = fetch(j0 + threadIdx.x);
+  ahead[1] = fetch(j0 + threadIdx.x + PQ_TILE);
   for (int64_t j = j0 + threadIdx.x; j < j1; j += PQ_TILE) {
     const uint8_t* cj = codes + (bk * cap + j) * n_sub;
     float s[PQ_ROWS] = {0.f, 0.f, 0.f, 0.f};
     if (vec) {
-      const uint4 cv = *reinterpret_cast<const uint4*>(cj);
+      const uint4 cv = ahead[0];
+      ahead[0] = ahead[1];
+      ahead[1] = fetch(j + 2 * PQ_TILE);
       const uint32_t w[4] = {cv.x, cv.y, cv.z, cv.w};
 #pragma unroll
       for (int sub = 0; sub < 16; ++sub) {

@@ -17,15 +17,19 @@
 // move depends on A's parity and every later add of the same v moves by the even one of k, k + 1.
 // A bin is therefore a function of A's parity (two moves), such functions compose, and a scan
 // over the bins gives every prefix up to the first one that reaches the next binade; that bin is
-// added by one thread, run by run, and the scan starts again behind it (about a dozen times).
+// added run by run, and the scan starts again behind it.  One warp does this over the list of
+// non-empty bins, 64 at a time, some two dozen scans for a row of 65536 keys (all threads over all
+// bins, with four barriers per binade, took 28 us for it).
 //
 // A row is shared by a cluster of up to eight CTAs where there are few rows.  What bounds the
 // kernel is the instruction issue of the three passes over the row (maximum, histogram, emit), so
 // the logits of the first pass stay in shared memory (81920 columns per CTA; longer ranges are
 // converted again in every pass), the second replaces them by their bins, and where it can a pass
-// handles two 16-bit values per integer instruction.  128 rows x 65536 keys: 186 us with scalar
+// handles two 16-bit values per integer instruction; four blocks of a pass are requested at a time.
+// 128 rows x 65536 keys: 186 us with scalar
 // loads, two gathers of the weight per key from global memory and the accumulator replayed by one
-// thread; 62 us with the logits converted in every pass; 47 us now.
+// thread; 62 us with the logits converted in every pass; 47 us with the replay by all threads;
+// 30 us now.
 // ---------------------------------------------------------------------------
 #include "sah_common.cuh"
 #include <cooperative_groups.h>
@@ -65,32 +69,6 @@ __device__ __forceinline__ float tp_block_max(float v, float* scratch32) {
   return w;
 }
 
-// Adds `count` copies of v (> 0) to acc one after the other in float32; returns false when an
-// add left acc unchanged (then no smaller value changes it either).
-__device__ __forceinline__ bool tp_add_run(float& acc, float v, unsigned int count) {
-  int same = 0;   // consecutive single steps that stayed in the binade they started in
-  while (count > 0u) {
-    const float next = __fadd_rn(acc, v);
-    if (next == acc) return false;
-    const bool stay = (__float_as_uint(next) >> 23) == (__float_as_uint(acc) >> 23);
-    const float step = __fsub_rn(next, acc);   // exact when both lie in one binade
-    acc = next;
-    --count;
-    same = stay ? same + 1 : 0;
-    if (same >= 2 && count > 0u) {
-      // acc is a multiple of the binade's spacing, `step` too; every further add moves acc by
-      // `step` until it reaches the next power of two
-      const float hi = __uint_as_float(((__float_as_uint(acc) >> 23) + 1u) << 23);
-      double n = floor(((double)hi - (double)acc) / (double)step);
-      if (n > (double)count) n = (double)count;
-      acc = (float)((double)acc + n * (double)step);
-      count -= (unsigned int)n;
-      same = 0;
-    }
-  }
-  return true;
-}
-
 // Bins of two values d = logit - maximum (packed bf16): ascending bins have descending weights.
 // As unsigned 16-bit numbers the d of bins 1 .. are TP_D0 .., the smaller magnitudes, +0 and the
 // positive not-a-number (an infinite or NaN logit; counts as weight 1) are below.
@@ -127,35 +105,66 @@ __device__ __forceinline__ TpMove tp_then(const TpMove& f, const TpMove& g) {
   r.d1 = min(f.d1 + ((f.d1 & 1u) ? g.d0 : g.d1), TP_FAR);
   return r;
 }
-// `count` adds of the positive bf16 value with bits `vb` to an accumulator whose binade has
-// exponent field `ea` (spacing 2^(ea - 150))
-__device__ __forceinline__ TpMove tp_move(unsigned int vb, unsigned int count, int ea) {
+// One add of the positive bf16 value with bits `vb` to an accumulator whose binade has exponent
+// field `ea` (spacing 2^(ea - 150)): A moves by `step` from an even A, by `first1` from an odd one
+// (to an even A where the two differ).
+__device__ __forceinline__ void tp_steps(unsigned int vb, int ea, unsigned int& step, unsigned int& first1) {
   int ev = (int)(vb >> 7);
   unsigned int m = vb & 127u;
   if (ev) m |= 128u; else ev = 1;   // v = m * 2^(ev - 134)
   const int sh = ea - 16 - ev;      // v / u = m * 2^-sh
-  unsigned int k, first1, step;
   if (sh <= 0) {
-    k = m << -sh;                   // v is not above the accumulator, so at most 2^24
-    first1 = step = k;
+    first1 = step = m << -sh;       // v is not above the accumulator, so at most 2^24
   } else if (sh > 8) {
-    k = first1 = step = 0u;         // below half a spacing
+    first1 = step = 0u;             // below half a spacing
   } else {
-    k = m >> sh;
-    const unsigned int rem = m & ((1u << sh) - 1u), half = 1u << (sh - 1);
+    const unsigned int k = m >> sh, rem = m & ((1u << sh) - 1u), half = 1u << (sh - 1);
     if (rem == half) {
-      step = k + (k & 1u);          // from an even A to an even A
-      first1 = k + 1u - (k & 1u);   // from an odd A to an even A
+      step = k + (k & 1u);
+      first1 = k + 1u - (k & 1u);
     } else {
-      if (rem > half) ++k;
-      first1 = step = k;
+      first1 = step = k + (rem > half ? 1u : 0u);
     }
   }
+}
+// `count` such adds, as moves by A's parity at entry
+__device__ __forceinline__ TpMove tp_move(unsigned int vb, unsigned int count, int ea) {
+  unsigned int step, first1;
+  tp_steps(vb, ea, step, first1);
   const unsigned long long rest = (unsigned long long)(count - 1u) * step;
   TpMove r;
   r.d0 = (unsigned int)min(rest + step, (unsigned long long)TP_FAR);
   r.d1 = (unsigned int)min(rest + first1, (unsigned long long)TP_FAR);
   return r;
+}
+// `count` adds of the bf16 value with bits `vb` to acc (not below the value; 0 before the first run,
+// whose weight is 1: the maximum itself), binade by
+// binade: all that stay below the next power of two at once, then one real add across it.
+__device__ __forceinline__ float tp_add_run(float acc, unsigned int vb, unsigned int count) {
+  const float v = __uint_as_float(vb << 16);
+  if (acc == 0.f) {
+    acc = v;
+    --count;
+  }
+  while (count > 0u) {
+    const unsigned int ea = __float_as_uint(acc) >> 23;
+    unsigned int A = (__float_as_uint(acc) & 0x7FFFFFu) | 0x800000u, step, first1;
+    tp_steps(vb, (int)ea, step, first1);
+    const unsigned int first = (A & 1u) ? first1 : step, room = (1u << 24) - 1u - A;  // A may grow by `room`
+    if (first <= room) {
+      unsigned int more = step == 0u ? count - 1u : (room - first) / step;  // adds after the first
+      if (more > count - 1u) more = count - 1u;
+      A += first + more * step;
+      count -= 1u + more;
+      acc = __uint_as_float(ea << 23 | (A & 0x7FFFFFu));
+      if (step == 0u) break;  // nothing moves any more
+    }
+    if (count > 0u) {
+      acc = __fadd_rn(acc, v);
+      --count;
+    }
+  }
+  return acc;
 }
 
 template <bool RESIDENT>
@@ -168,10 +177,12 @@ topp_select_kernel(ToppArgs a) {
   __shared__ unsigned int hist[TP_PER * TP_THREADS];  // this CTA's counts; in rank 0 the row's
   __shared__ uint16_t weight[TP_PER * TP_THREADS];    // bf16 bits of exp(d) by bin
   __shared__ float scratch[32];
-  __shared__ uint2 warp_move[32];
+  __shared__ uint16_t list[TP_PER * TP_THREADS];      // non-empty bins of positive weight, ascending
+  __shared__ float list_sum[TP_PER * TP_THREADS];     // the accumulator behind each of them
+  __shared__ int scan_sm[33];
   __shared__ float max_sm;                            // this CTA's maximum
   __shared__ float acc_sm;
-  __shared__ int cross_sm, pick_sm, last_sm, thr_sm;
+  __shared__ int cross_sm, pick_sm, thr_sm;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int64_t row = blockIdx.x / ranks;
@@ -196,13 +207,23 @@ topp_select_kernel(ToppArgs a) {
 
   // scaled logits of a byte's columns, packed in pairs, previously active positions pushed to the
   // lowest value (:96-104) and columns past the end to -inf
-  auto convert = [&](int y, uint32_t* w) {
+  auto load = [&](int y) -> uint4 {
     const int64_t c0 = (b_lo + y) * 8;
-    float f[8];
-    tp_load8(s, c0, a.S, vec, f);
-    const unsigned int act = pb[y];
+    if (vec && c0 + 8 <= a.S) return *reinterpret_cast<const uint4*>(s + c0);
+    const uint16_t* u = reinterpret_cast<const uint16_t*>(s);
+    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = tp_pack2(__fmul_rn(f[2 * i], a.scaling), __fmul_rn(f[2 * i + 1], a.scaling));
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t lo = c0 + 2 * i < a.S ? u[c0 + 2 * i] : 0u, hi = c0 + 2 * i + 1 < a.S ? u[c0 + 2 * i + 1] : 0u;
+      w[i] = lo | hi << 16;
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  };
+  auto scale = [&](int y, const uint4& raw, unsigned int act, uint32_t* w) {
+    const int64_t c0 = (b_lo + y) * 8;
+    w[0] = raw.x; w[1] = raw.y; w[2] = raw.z; w[3] = raw.w;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = tp_pack2(__fmul_rn(tp_lo(w[i]), a.scaling), __fmul_rn(tp_hi(w[i]), a.scaling));
     if (bias) {
       float bv[8];
       tp_load8(bias, c0, a.S, bias_vec, bv);
@@ -219,6 +240,7 @@ topp_select_kernel(ToppArgs a) {
       }
     }
   };
+  auto convert = [&](int y, uint32_t* w) { scale(y, load(y), pb[y], w); };
 
   for (int i = tid; i < TP_PER * TP_THREADS; i += TP_THREADS) {
     hist[i] = 0u;
@@ -228,12 +250,30 @@ topp_select_kernel(ToppArgs a) {
   }
 
   float mx = -INFINITY;
-  for (int y = tid; y < ny; y += TP_THREADS) {
-    uint32_t w[4];
-    convert(y, w);
-    if (RESIDENT) tp_row[y] = make_uint4(w[0], w[1], w[2], w[3]);
+  constexpr int AHEAD = 4;
+  for (int y0 = tid; y0 < ny; y0 += AHEAD * TP_THREADS) {
+    uint4 raw[AHEAD];
+    unsigned int act[AHEAD];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) mx = fmaxf(fmaxf(mx, tp_lo(w[i])), tp_hi(w[i]));
+    for (int n = 0; n < AHEAD; ++n) {
+      const int y = y0 + n * TP_THREADS;
+      raw[n] = make_uint4(0u, 0u, 0u, 0u);
+      act[n] = 0u;
+      if (y < ny) {
+        raw[n] = load(y);
+        act[n] = pb[y];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < AHEAD; ++n) {
+      const int y = y0 + n * TP_THREADS;
+      if (y >= ny) break;
+      uint32_t w[4];
+      scale(y, raw[n], act[n], w);
+      if (RESIDENT) tp_row[y] = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mx = fmaxf(fmaxf(mx, tp_lo(w[i])), tp_hi(w[i]));
+    }
   }
   mx = tp_block_max(mx, scratch);
   if (ranks > 1) {
@@ -283,36 +323,51 @@ topp_select_kernel(ToppArgs a) {
   }
 
   if (rank == 0) {
-    // replay of the accumulator, largest weight first; thread t holds bins 3 t .. 3 t + 2
-    unsigned int cnt[TP_PER], val[TP_PER];
-    float sum[TP_PER];
-    int last = -1;
+    // the non-empty bins, thread t looks at bins 3 t .. 3 t + 2
+    unsigned int val[TP_PER];
+    bool full[TP_PER];
+    int n_here = 0;
 #pragma unroll
     for (int i = 0; i < TP_PER; ++i) {
-      const int bin = tid * TP_PER + i;
-      val[i] = weight[bin];
-      cnt[i] = val[i] ? hist[bin] : 0u;
-      sum[i] = 0.f;
-      if (cnt[i]) last = bin;
+      val[i] = weight[tid * TP_PER + i];
+      full[i] = val[i] != 0u && hist[tid * TP_PER + i] != 0u;
+      n_here += full[i] ? 1 : 0;
     }
-    if (tid == 0) { acc_sm = 0.f; pick_sm = -1; last_sm = -1; thr_sm = -1; }
-    int pos = 0;   // bins before it are done
-    for (;;) {
-      if (tid == 0) cross_sm = TP_BINS;
-      __syncthreads();
-      const float acc = acc_sm;
-      const int ea = (int)(__float_as_uint(acc) >> 23);
-      unsigned int A = (__float_as_uint(acc) & 0x7FFFFFu) | 0x800000u;
-      TpMove mv[TP_PER], all;
-      all.d0 = all.d1 = 0u;
-      if (acc > 0.f) {
+    if (tid == 0) { pick_sm = -1; thr_sm = -1; cross_sm = TP_BINS; }
+    int n_list;
+    int at = sah_block_excl_scan<int>(n_here, scan_sm, &n_list);
 #pragma unroll
-        for (int i = 0; i < TP_PER; ++i) {
-          mv[i].d0 = mv[i].d1 = 0u;
-          if (cnt[i] && tid * TP_PER + i >= pos) mv[i] = tp_move(val[i], cnt[i], ea);
-          all = tp_then(all, mv[i]);
+    for (int i = 0; i < TP_PER; ++i)
+      if (full[i]) list[at++] = (uint16_t)(tid * TP_PER + i);
+    __syncthreads();
+    // replay of the accumulator, largest weight first: lane l takes entries base + 2 l, + 1
+    if (warp == 0) {
+      float acc = 0.f;
+      for (int base = 0; base < n_list;) {
+        if (acc == 0.f) {
+          const int bin = list[0];
+          acc = tp_add_run(0.f, weight[bin], hist[bin]);
+          if (lane == 0) list_sum[0] = acc;
+          base = 1;
+          continue;
         }
-        // exclusive scan over the threads
+        const int ea = (int)(__float_as_uint(acc) >> 23);
+        const unsigned int A0 = (__float_as_uint(acc) & 0x7FFFFFu) | 0x800000u;
+        unsigned int v[2], c[2];
+        TpMove mv[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int e = base + 2 * lane + i;
+          v[i] = c[i] = 0u;
+          mv[i].d0 = mv[i].d1 = 0u;
+          if (e < n_list) {
+            const int bin = list[e];
+            v[i] = weight[bin];
+            c[i] = hist[bin];
+            mv[i] = tp_move(v[i], c[i], ea);
+          }
+        }
+        TpMove all = tp_then(mv[0], mv[1]);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           TpMove left;
@@ -320,77 +375,53 @@ topp_select_kernel(ToppArgs a) {
           left.d1 = __shfl_up_sync(0xffffffffu, all.d1, o);
           if (lane >= o) all = tp_then(left, all);
         }
-        if (lane == 31) warp_move[warp] = make_uint2(all.d0, all.d1);
         TpMove ex;
         ex.d0 = __shfl_up_sync(0xffffffffu, all.d0, 1);
         ex.d1 = __shfl_up_sync(0xffffffffu, all.d1, 1);
         if (lane == 0) ex.d0 = ex.d1 = 0u;
-        __syncthreads();
-        TpMove w;
-        w.d0 = warp_move[lane].x;
-        w.d1 = warp_move[lane].y;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          TpMove left;
-          left.d0 = __shfl_up_sync(0xffffffffu, w.d0, o);
-          left.d1 = __shfl_up_sync(0xffffffffu, w.d1, o);
-          if (lane >= o) w = tp_then(left, w);
+        // A in front of this lane's entries and behind each of them; from the first that reaches
+        // the next binade on the numbers mean nothing
+        const unsigned int before = A0 + ((A0 & 1u) ? ex.d1 : ex.d0);
+        const unsigned int mid = before + ((before & 1u) ? mv[0].d1 : mv[0].d0);
+        const unsigned int end = mid + ((mid & 1u) ? mv[1].d1 : mv[1].d0);
+        const unsigned int over = __ballot_sync(0xffffffffu, end >= (1u << 24));  // moves only add up
+        const int first = over ? __ffs(over) - 1 : 32;
+        auto value = [&](unsigned int A) { return __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu)); };
+        const int e0 = base + 2 * lane;
+        if (lane < first) {
+          if (e0 < n_list) list_sum[e0] = value(mid);
+          if (e0 + 1 < n_list) list_sum[e0 + 1] = value(end);
+        } else if (lane == first && mid < (1u << 24)) {
+          list_sum[e0] = value(mid);
         }
-        TpMove before;
-        before.d0 = __shfl_sync(0xffffffffu, w.d0, (warp + 31) & 31);
-        before.d1 = __shfl_sync(0xffffffffu, w.d1, (warp + 31) & 31);
-        if (warp == 0) before.d0 = before.d1 = 0u;
-        before = tp_then(before, ex);
-        A += (A & 1u) ? before.d1 : before.d0;
-      }
-      // own bins: a prefix below the next binade is final, the first that reaches it is added
-      // run by run below
-      float entry = acc;
-      int mine = TP_BINS;
-#pragma unroll
-      for (int i = 0; i < TP_PER; ++i) {
-        const int bin = tid * TP_PER + i;
-        if (mine == TP_BINS && cnt[i] && bin >= pos) {
-          const unsigned int next = acc > 0.f ? A + ((A & 1u) ? mv[i].d1 : mv[i].d0) : TP_FAR;
-          if (A < (1u << 24)) entry = acc > 0.f ? __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu)) : 0.f;
-          if (next < (1u << 24)) {
-            A = next;
-            sum[i] = __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu));
-          } else {
-            mine = bin;
-          }
+        if (first == 32) {
+          acc = value(__shfl_sync(0xffffffffu, end, 31));
+          base += 64;
+        } else {
+          const bool second = __shfl_sync(0xffffffffu, mid, first) < (1u << 24);  // which of the lane's entries
+          const unsigned int A = __shfl_sync(0xffffffffu, second ? mid : before, first);
+          const unsigned int vb = __shfl_sync(0xffffffffu, second ? v[1] : v[0], first);
+          const unsigned int n = __shfl_sync(0xffffffffu, second ? c[1] : c[0], first);
+          acc = tp_add_run(value(A), vb, n);
+          base += 2 * first + (second ? 1 : 0);
+          if (lane == 0) list_sum[base] = acc;
+          ++base;
         }
       }
-      if (mine < TP_BINS) atomicMin(&cross_sm, mine);
-      if (tid == TP_THREADS - 1 && mine == TP_BINS && acc > 0.f && A < (1u << 24))
-        acc_sm = __uint_as_float((uint32_t)ea << 23 | (A & 0x7FFFFFu));  // no crossing at all: the total
-      __syncthreads();
-      const int cross = cross_sm;
-      if (cross == TP_BINS) break;
-      if (mine == cross) {
-#pragma unroll
-        for (int i = 0; i < TP_PER; ++i)
-          if (tid * TP_PER + i == cross) {
-            tp_add_run(entry, __uint_as_float(val[i] << 16), cnt[i]);
-            sum[i] = entry;
-          }
-        acc_sm = entry;
-      }
-      pos = cross + 1;
-      __syncthreads();
+      if (lane == 0) acc_sm = acc;
     }
+    __syncthreads();
 
     // first run (largest value) whose normalised prefix exceeds top_p (:118-131)
     const float total = sah_round_to<T>(acc_sm);
     const float p = sah_round_to<T>(a.top_p);
-    int best = TP_BINS;
-#pragma unroll
-    for (int i = TP_PER - 1; i >= 0; --i)
-      if (cnt[i] && sah_round_to<T>(__fdiv_rn(sah_round_to<T>(sum[i]), total)) > p) best = tid * TP_PER + i;
-    if (tid == 0) cross_sm = TP_BINS;
-    __syncthreads();
+    int best = TP_BINS;  // place in the list
+    for (int e = tid; e < n_list; e += TP_THREADS)
+      if (sah_round_to<T>(__fdiv_rn(sah_round_to<T>(list_sum[e]), total)) > p) {
+        best = e;
+        break;
+      }
     if (best < TP_BINS) atomicMin(&cross_sm, best);
-    if (last >= 0) atomicMax(&last_sm, last);
     // weight 0 among the keys: bins whose weight is 0
 #pragma unroll
     for (int i = 0; i < TP_PER; ++i)
@@ -398,8 +429,8 @@ topp_select_kernel(ToppArgs a) {
     __syncthreads();
     // nothing exceeds top_p: the search position is clamped to the last sorted element (:127-130)
     unsigned int thr;
-    if (cross_sm < TP_BINS) thr = weight[cross_sm];
-    else thr = (pick_sm > 0 || last_sm < 0) ? 0u : weight[last_sm];
+    if (cross_sm < TP_BINS) thr = weight[list[cross_sm]];
+    else thr = (pick_sm > 0 || n_list == 0) ? 0u : weight[list[n_list - 1]];
     // the last bin that is selected (weight >= threshold, :158-160)
     int keep = -1;
 #pragma unroll
