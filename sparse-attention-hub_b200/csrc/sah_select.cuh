@@ -54,7 +54,11 @@ struct SahScoreKeys<__nv_bfloat16, 16> {
     s = scores + row * S;
     vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
   }
-  __device__ __forceinline__ void load(int64_t c0, uint32_t* w) const {
+  static constexpr int AHEAD = 4;  // blocks requested together, as registers allow
+  static constexpr bool BANDS = true;  // the previous mask may come as bands
+  struct Raw { uint32_t w[4]; };
+  __device__ __forceinline__ void load(int64_t c0, Raw& raw) const {
+    uint32_t* w = raw.w;
     if (vec && c0 + 8 <= S) {
       const uint4 v = *reinterpret_cast<const uint4*>(s + c0);
       w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
@@ -66,9 +70,11 @@ struct SahScoreKeys<__nv_bfloat16, 16> {
         w[i] = lo | hi << 16;
       }
     }
+  }
+  __device__ __forceinline__ void make(const Raw& raw, uint32_t* w) const {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const __nv_bfloat162 z = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]), __float2bfloat162_rn(0.f));
+      const __nv_bfloat162 z = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&raw.w[i]), __float2bfloat162_rn(0.f));
       const uint32_t u = *reinterpret_cast<const uint32_t*>(&z);
       w[i] = u ^ ((((u >> 15) & 0x00010001u) * 0xFFFFu) | 0x80008000u);
     }
@@ -84,16 +90,21 @@ struct SahScoreKeys<float, 32> {
     s = scores + row * S;
     vec = (reinterpret_cast<uintptr_t>(s) & 15) == 0;
   }
-  __device__ __forceinline__ void load(int64_t c0, uint32_t* w) const {
-    float f[8];
+  static constexpr int AHEAD = 2;
+  static constexpr bool BANDS = true;
+  struct Raw { float f[8]; };
+  __device__ __forceinline__ void load(int64_t c0, Raw& raw) const {
+    float* f = raw.f;
     if (vec && c0 + 8 <= S) {
       sah_load8<float>(s + c0, f);
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = c0 + i < S ? s[c0 + i] : 0.f;
     }
+  }
+  __device__ __forceinline__ void make(const Raw& raw, uint32_t* w) const {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w[i] = sah_float_key(f[i] + 0.0f);
+    for (int i = 0; i < 8; ++i) w[i] = sah_float_key(raw.f[i] + 0.0f);
   }
 };
 
@@ -136,7 +147,7 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
   // nearly all of them, and empty
   const int64_t qpos = row % Sq;
   int gap_lo = 0, gap_hi = 0;
-  if (pb == nullptr) {
+  if (Keys::BANDS && pb == nullptr) {
     int64_t a = 0, e = S;
 #pragma unroll
     for (int i = 0; i < SAH_MAX_BANDS; ++i) {
@@ -151,7 +162,7 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
     gap_hi = (int)(e < 0 ? 0 : e > ny ? ny : e);
   }
   auto previous = [&](int y) -> unsigned int {
-    if (pb != nullptr) return pb[y];
+    if (!Keys::BANDS || pb != nullptr) return pb[y];
     return y >= gap_lo && y < gap_hi ? 0u : sah_band_bits(bands, qpos, (y_lo + y) * 8, 8, S, 0u);
   };
   // columns of byte y (of this CTA) that compete
@@ -164,12 +175,11 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
     return m;
   };
   // the byte's keys from memory, 0 where a column does not compete; false if none does
-  auto convert = [&](int y, uint32_t* w) -> bool {
-    const unsigned int m = competing(y);
+  auto finish = [&](const typename Keys::Raw& raw, unsigned int m, uint32_t* w) -> bool {
 #pragma unroll
     for (int i = 0; i < NW; ++i) w[i] = 0u;
     if (m == 0u) return false;
-    keys.load((y_lo + y) * 8, w);
+    keys.make(raw, w);
     if (m != 255u) {
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
@@ -180,6 +190,12 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
       }
     }
     return true;
+  };
+  auto convert = [&](int y, uint32_t* w) -> bool {
+    const unsigned int m = competing(y);
+    typename Keys::Raw raw;
+    if (m) keys.load((y_lo + y) * 8, raw);
+    return finish(raw, m, w);
   };
   auto fetch = [&](int y, uint32_t* w) -> bool {
     if (!RESIDENT) return convert(y, w);
@@ -211,25 +227,43 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
       for (int i = tid; i < nbins; i += nt) h[i] = 0u;
       if (tid == 0) mode_sm = 0;
       __syncthreads();
-      for (int q = q_lo; q < q_hi; ++q) {
-        const int y = q * 32 + lane;
-        if (y >= ny) break;
-        uint32_t w[NW];
-        if (d == 0) {
-          const bool any = convert(y, w);
-          if (RESIDENT) {
+      if (d == 0) {
+        // a few blocks' keys are requested before the first is converted
+        constexpr int AHEAD = Keys::AHEAD;
+        for (int q0 = q_lo; q0 < q_hi; q0 += AHEAD) {
+          typename Keys::Raw raw[AHEAD];
+          unsigned int m[AHEAD];
 #pragma unroll
-            for (int i = 0; i < NW / 4; ++i)
-              store[i * ny + y] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+          for (int n = 0; n < AHEAD; ++n) {
+            const int y = (q0 + n) * 32 + lane;
+            m[n] = q0 + n < q_hi && y < ny ? competing(y) : 0u;
+            if (m[n]) keys.load((y_lo + y) * 8, raw[n]);
           }
-          if (any) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint32_t key = key_at(w, i);
-              if (key) atomicAdd(&h[key >> shift], 1u);
+          for (int n = 0; n < AHEAD; ++n) {
+            const int y = (q0 + n) * 32 + lane;
+            if (q0 + n >= q_hi || y >= ny) break;
+            uint32_t w[NW];
+            const bool any = finish(raw[n], m[n], w);
+            if (RESIDENT) {
+#pragma unroll
+              for (int i = 0; i < NW / 4; ++i)
+                store[i * ny + y] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+            }
+            if (any) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint32_t key = key_at(w, i);
+                if (key) atomicAdd(&h[key >> shift], 1u);
+              }
             }
           }
-        } else {
+        }
+      } else {
+        for (int q = q_lo; q < q_hi; ++q) {
+          const int y = q * 32 + lane;
+          if (y >= ny) break;
+          uint32_t w[NW];
           if (!fetch(y, w)) continue;
           bool any = true;
           if (NW == 4) {  // some half agrees with the prefix (nothing is left below the mask, so the test is exact)
