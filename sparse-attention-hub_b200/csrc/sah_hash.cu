@@ -20,7 +20,8 @@
 // whose 64 multiply-adds need four broadcast reads of activations and one of weights.
 // 32 heads x 16384 keys through 128-128-128-32: 1963 us with tiles of 64 vectors, 8 x 4 outputs
 // per thread, scalar fma and the weights staged per tile; 981 us with one tile of 128 vectors per
-// CTA; 907 us in groups, 863 us with the channel loop unrolled eight times (19.3 G multiply-adds; 540 us at 128 per clock and SM).
+// CTA; 907 us in groups, 863 us with the channel loop unrolled eight times, 851 us sixteen times
+// (19.3 G multiply-adds; 540 us at 128 per clock and SM).
 // ---------------------------------------------------------------------------
 #define HE_TK 32        // vectors per tile
 #define HE_GT 64        // threads per group
@@ -99,7 +100,7 @@ __device__ __forceinline__ void he_layer(float* __restrict__ act, const float* _
 
   const float* ap = act + kg * KP;
   const float* wp = w_sm + og * OP;
-#pragma unroll 8
+#pragma unroll 16
   for (int d = 0; d < din; ++d) {
     unsigned long long a[KP / 2], w[OP];
 #pragma unroll

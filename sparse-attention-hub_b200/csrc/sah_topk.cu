@@ -19,7 +19,8 @@
 // Bound by shared-memory reads (a key's own row and the broadcast query values) and, behind them,
 // the stream of K.  A thread therefore owns two keys where the head dimension is known, which
 // halves the query reads: 32 rows x 65536 keys x 4 sequences in bfloat16 (537 MB, 82 us at the
-// measured copy rate) 123 us with one key per thread, 113.7 us with two.
+// measured copy rate) 123 us with one key per thread, 113.7 us with two,
+// 110.3 us without the division of the row number that a single query does not need.
 #define QK_THREADS 128
 
 // Two partial sums at once: sm_100 issues a pair of fp32 operations per instruction
@@ -144,7 +145,7 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (FULL4 || r0 + r < R) {
-        const int rr = r0 + r, g = rr / Sq, qi = rr - g * Sq, h = kvh * G + g;
+        const int rr = r0 + r, g = Sq == 1 ? rr : rr / Sq, qi = rr - g * Sq, h = kvh * G + g;
         const int64_t row = ((int64_t)b * Hq + h) * Sq + qi;
 #pragma unroll
         for (int u = 0; u < KEYS; ++u) {
