@@ -420,3 +420,48 @@ def test_gpu_signatures_of_single_keys_equal_those_of_a_tile(dtype, L, K, D, cen
     for s0, s1 in ((0, 1), (1, 5), (5, 7), (7, 8), (8, 9)):
         sign(parts, s0, s1)
     assert torch.equal(whole, parts)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S,scale,centred", [(1024, 1.0, True), (1055, 1.0, False), (4097, 5e-20, True),
+                                             (1300, 3e17, False)])
+def test_gpu_norms_of_many_keys_equal_those_of_few(S, scale, centred):
+    """Norms and transformed norms of 1024 keys and more are made 32 keys per warp, fewer a key per
+    warp: the same bits and the same maximum, zero keys and operands that have to be divided
+    included."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, D, cap = 2, 2, 128, S + 3
+    gen = torch.Generator(device=dev).manual_seed(S)
+    keys = torch.randn((B, Hkv, cap, D), generator=gen, device=dev) * scale
+    keys[:, :, 7] = 0.0
+    keys[..., 64] *= 2.0 ** -75
+    keys = keys.to(torch.bfloat16)[:, :, :S]
+    mean = keys.float().mean(dim=2).to(torch.bfloat16).contiguous() if centred else None
+    st = _native.stream_of(torch.device(dev))
+    kargs = (keys.data_ptr(), _native.SAH_BF16, keys.stride(0), keys.stride(1), keys.stride(2), B, Hkv)
+
+    def stats(norms, top, s0, s1):
+        _native.check(lib.sah_lsh_key_stats(*kargs, s0, s1, D, _native.ptr(mean), cap, norms.data_ptr(),
+                                            top.data_ptr(), 148, st), "sah_lsh_key_stats")
+
+    norms, parts = (torch.full((B, Hkv, cap), -1.0, device=dev) for _ in range(2))
+    top, top_parts = (torch.zeros(1, dtype=torch.int32, device=dev) for _ in range(2))
+    stats(norms, top, 0, S)
+    for s0 in range(0, S, 1000):
+        stats(parts, top_parts, s0, min(S, s0 + 1000))
+    assert torch.equal(norms, parts) and torch.equal(top, top_parts)
+
+    def dens(out, s0, last):
+        committed = torch.full((1,), last, dtype=torch.int32, device=dev)
+        _native.check(lib.sah_lsh_key_den(*kargs, s0, S, D, _native.ptr(mean), norms.data_ptr(), cap, top.data_ptr(),
+                                          committed.data_ptr(), out.data_ptr(), 148, st), "sah_lsh_key_den")
+        assert torch.equal(committed, top)
+
+    whole, again = (torch.full((B, Hkv, cap), -1.0, device=dev) for _ in range(2))
+    dens(whole, 0, 0)
+    dens(again, 1, 0)  # the maximum moved: every key, through the kernel of the decode step
+    assert torch.equal(whole, again)
