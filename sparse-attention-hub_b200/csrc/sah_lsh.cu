@@ -1170,10 +1170,16 @@ lsh_key_rows_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_t k
   }
 }
 
-#define LSH_ROWS_MIN_KEYS 1024  // below this a key per warp spreads better over the chip
-static bool lsh_rows_fits(const void* keys, int dtype, int64_t ks_b, int64_t ks_h, int64_t ks_s, int64_t n, int D) {
-  return dtype == SAH_BF16 && D == 128 && n >= LSH_ROWS_MIN_KEYS && ((uintptr_t)keys & 7) == 0 && ks_b % 4 == 0 &&
-         ks_h % 4 == 0 && ks_s % 4 == 0;
+// From how many keys on, all heads together, 32 keys per warp are ahead of a key per warp, which
+// spreads fewer keys better over the chip.  Norms: 2 x 1024 keys 6.2 against 4.2 us, 2 x 2048 equal,
+// 8 x 1024 6.2 against 8.4 us.  Transformed norms (with the clearing of a word, 2 us): 8 x 2048 16.4
+// against 14.4 us, 2 x 16384 16.4 against 18.5 us, 8 x 4096 16.4 against 20.5 us.
+#define LSH_ROWS_MIN_STATS 4096
+#define LSH_ROWS_MIN_DENS 32768
+static bool lsh_rows_fits(const void* keys, int dtype, int64_t ks_b, int64_t ks_h, int64_t ks_s, int64_t n,
+                          int64_t heads, int64_t least, int D) {
+  return dtype == SAH_BF16 && D == 128 && n >= 1024 && n * heads >= least && ((uintptr_t)keys & 7) == 0 &&
+         ks_b % 4 == 0 && ks_h % 4 == 0 && ks_s % 4 == 0;
 }
 static dim3 lsh_rows_grid(int64_t n, int64_t heads, int sm_count) {
   int64_t gx = (n + 255) / 256;
@@ -1190,7 +1196,7 @@ extern "C" int sah_lsh_key_stats(const void* keys, int dtype, int64_t ks_b, int6
   SAH_REQUIRE(s0 >= 0 && s1 >= s0 && s1 <= cap, "lsh_key_stats: bad key range");
   if (s1 == s0) return SAH_OK;
   if (sm_count <= 0) sm_count = 148;
-  if (lsh_rows_fits(keys, dtype, ks_b, ks_h, ks_s, s1 - s0, D)) {
+  if (lsh_rows_fits(keys, dtype, ks_b, ks_h, ks_s, s1 - s0, (int64_t)B * Hkv, LSH_ROWS_MIN_STATS, D)) {
     lsh_key_rows_kernel<false><<<lsh_rows_grid(s1 - s0, (int64_t)B * Hkv, sm_count), 256, 0, (cudaStream_t)stream>>>(
         reinterpret_cast<const __nv_bfloat16*>(keys), ks_b, ks_h, ks_s, Hkv, s0, s1,
         reinterpret_cast<const __nv_bfloat16*>(mean), cap, norms, max_norm_bits, nullptr);
@@ -1221,7 +1227,7 @@ extern "C" int sah_lsh_key_den(const void* keys, int dtype, int64_t ks_b, int64_
   if (sm_count <= 0) sm_count = 148;
   cudaStream_t st = (cudaStream_t)stream;
   // An index build: every key is new (whether M moved or not), so the first key is known here.
-  if (s_new0 == 0 && lsh_rows_fits(keys, dtype, ks_b, ks_h, ks_s, s1, D)) {
+  if (s_new0 == 0 && lsh_rows_fits(keys, dtype, ks_b, ks_h, ks_s, s1, (int64_t)B * Hkv, LSH_ROWS_MIN_DENS, D)) {
     lsh_key_rows_kernel<true><<<lsh_rows_grid(s1, (int64_t)B * Hkv, sm_count), 256, 0, st>>>(
         reinterpret_cast<const __nv_bfloat16*>(keys), ks_b, ks_h, ks_s, Hkv, 0, s1,
         reinterpret_cast<const __nv_bfloat16*>(mean), cap, const_cast<float*>(norms),
