@@ -587,18 +587,18 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
 // keys 99 against 108 us; 64K keys 63 against 73 us (two waves from 512K down: 337, 185 and
 // 111 us -- a CTA's prologue, pipeline fill and merge are paid once per SM instead of twice).  64 KV groups with lists of a few
 // thousand rows (HashAttention and Quest at B = 8, S = 32768): 63 against 69 us and 56 against
-// 61 us.  8 groups and fewer, whole decode step:
-// Sink + Local 20.6 against 24.2 us (1024 keys), 21.3 against 22.7 (4096); oracle top-k 30.8 against
-// 32.9 (2048), 39.5 against 41.4 (8192); hash 37.8 against 43.8 us (4096 keys), 40.1 against 45.5 (8192), 43.9 against 45.3 (16384); Quest
-// 38.2 against 42.0 (8192); PQCache 131072 keys 81.7 against 86.1; top-p 74.0 against 76.6 (8192),
-// 147.5 against 150.3 (65536); MagicPig 45.9 against 54.6 (8192), 54.5 against 58.4 (16384), 94.9
-// against 105.9 (65500), and with 16 groups 96.4 against 104.4 (32768).  In between -- 16 to 32
-// groups with lists of 10^4..10^5 rows -- the mma.sync kernel, with two CTAs per SM and lower fixed
-// costs, is ahead or even (top-p, 32 groups of 65536 keys: 369 against 394 us; MagicPig, 32 groups
-// of 49152: 207 against 209).
+// 61 us.  In between -- 8 to 32 groups with lists of 10^4..10^5 rows -- the mma.sync kernel,
+// with two CTAs per SM and lower fixed costs, was ahead by 5-40 % (measured with two waves).
+// Few groups with short lists stay on the mma.sync kernel although this one is ahead there (one
+// query, 8 groups: 18 to 30 against 22 to 36 us for lists of 400 to 6000 rows), because it is less
+// exact: the maximum that P is taken against is shared by tiles of 128 entries and may lie up to
+// AUM_RESCALE_T below the true one, so a row's largest weights are rounded to bfloat16, while a warp
+// of the mma.sync kernel holds the largest of its 16 to 100 entries exactly (as 1).  Relative error
+// against float64 where one key of a hundred carries the weight (HashAttention, 8 groups, 4096 to
+// 97000 keys): 1.8e-3 to 2.3e-3 here, 1.7e-3 there; flat rows: 1.7e-3 in both.
 #define AUM_DEFAULT_MIN_KEYS (64 * 1024)
 static bool aum_default(bool lsh, int64_t S, int groups) {
-  return (lsh && S >= AUM_DEFAULT_MIN_KEYS) || (groups >= 64 && S <= 65536) || groups <= (lsh ? 16 : 8);
+  return (lsh && S >= AUM_DEFAULT_MIN_KEYS) || (groups >= 64 && S <= 65536);
 }
 
 // The kernel choice: a process-wide setting (sah_attn_select_kernel), else SAH_ATTN_UMMA in the

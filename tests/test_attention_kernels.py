@@ -102,6 +102,35 @@ def test_magicpig_weights_inside_the_kernel(kernel, S):
     np.testing.assert_allclose(out.float().cpu().numpy(), ref, atol=TOL, rtol=TOL)
 
 
+def test_default_kernel_for_few_groups_is_as_exact_as_the_mma_kernel():
+    """One key of a hundred carries e^6.5 times the weight of the others, 8 KV groups: the relative
+    error against float64 of the kernel that is taken by default is that of the mma.sync kernel, in
+    which the largest weight of every warp's share is exactly 1.  (Rounding those weights too makes it 1.06
+    times as large here and up to 1.33 times on HashAttention; 2 % is left for the order of sums.)"""
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    direction = torch.nn.functional.normalize(torch.randn((1, 8, 1, 128), generator=gen, device=DEV), dim=-1)
+    heavy = torch.rand((1, 8, 24000, 1), generator=gen, device=DEV) < 0.01
+    k, v = (torch.randn((1, 8, 24000, 128), generator=gen, device=DEV) for _ in range(2))
+    k, v = (k + 6.5 * direction * heavy).bfloat16(), v.bfloat16()
+    q = torch.randn((1, 32, 1, 128), generator=gen, device=DEV)
+    q = (0.3 * q + 128 ** 0.5 * direction.repeat_interleave(4, 1)).bfloat16()
+    few = torch.rand((1, 32, 1, 24000), generator=gen, device=DEV) < 0.06
+    dense = (few | heavy.transpose(2, 3).repeat_interleave(4, 1)).bfloat16()
+    scaling = 128 ** -0.5
+    logits = torch.matmul(q.double(), k.repeat_interleave(4, 1).double().transpose(2, 3)) * scaling
+    p = torch.softmax(logits.masked_fill(dense == 0, -float("inf")), dim=-1)
+    exact = torch.matmul(p, v.repeat_interleave(4, 1).double()).transpose(1, 2)
+
+    def error(choice):
+        prev = select_attention_kernel(choice)
+        m = Mask.create_mask_from_dense_mask(tuple(dense.shape), dense, torch.bfloat16)
+        out = native_masked_attention(q, k, v, None, None, scaling, m)
+        select_attention_kernel(prev)
+        return float((out.double() - exact).norm() / exact.norm())
+
+    assert error("auto") <= 1.02 * error("mma")
+
+
 def test_bounded_wait_runs_out_and_reports_without_hanging():
     """Every mbarrier wait of the tcgen05 kernels is bounded.  `sah_wait_selftest` waits 2 ms for an
     arrival that never comes: the error word is set, the measured wait is about the limit, the
