@@ -465,6 +465,11 @@ struct PqEntry<__nv_bfloat16> {
   }
 };
 
+// bytes of the table in front of the staged queries, which are read 16 bytes at a time
+__host__ __device__ __forceinline__ size_t pq_table_bytes(size_t entry, int n_sub, int n_cent) {
+  return (entry * (size_t)n_sub * (size_t)n_cent + 15) / 16 * 16;
+}
+
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(PQ_TILE)
 pq_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs_q,
@@ -483,7 +488,7 @@ pq_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs
   const int entries = n_sub * n_cent;
   const int Dh = n_sub * sub_d;
   Entry* lut = reinterpret_cast<Entry*>(pq_sm_raw);                  // [n_sub][n_cent]
-  float* q_sm = reinterpret_cast<float*>(lut + entries);             // [Dh][PQ_ROWS]
+  float* q_sm = reinterpret_cast<float*>(pq_sm_raw + pq_table_bytes(sizeof(Entry), n_sub, n_cent));  // [Dh][PQ_ROWS]
   for (int idx = threadIdx.x; idx < PQ_ROWS * Dh; idx += PQ_TILE) {
     const int rr = idx / Dh, d = idx - rr * Dh;
     const int r = rblk * PQ_ROWS + rr;
@@ -601,7 +606,7 @@ extern "C" int sah_pq_scores(const void* q, int dtype, int64_t qs_b, int64_t qs_
   const int R = (Hq / Hkv) * Sq;
   const int rblocks = (R + PQ_ROWS - 1) / PQ_ROWS;
   const size_t esz = (dtype == SAH_BF16) ? 8 : 16;  // one table entry: the four rows of a centroid
-  const size_t smem = esz * n_sub * n_cent + (size_t)PQ_ROWS * n_sub * sub_d * sizeof(float);
+  const size_t smem = pq_table_bytes(esz, n_sub, n_cent) + (size_t)PQ_ROWS * n_sub * sub_d * sizeof(float);
   if (smem > 200 * 1024)
     return sah_fail(SAH_ERR_UNSUPPORTED, "pq_scores: %d x %d lookup table does not fit", n_sub, n_cent);
   SAH_REQUIRE(rblocks <= 65535 && (int64_t)B * Hkv <= 65535, "pq_scores: too many rows per launch");

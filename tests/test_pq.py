@@ -343,3 +343,39 @@ def test_gpu_few_appended_keys_equal_the_tile_kernel(dtype, n_sub, sub_d, n_cent
     for s0, s1 in ((off, off + 1), (off + 1, off + 17), (off + 17, off + 20), (off + 20, off + 36), (off + 36, S)):
         assign(parts, s0, s1)
     assert torch.equal(whole, parts)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,n_sub,sub_d,n_cent,S", [("bf16", 3, 8, 33, 700), ("bf16", 1, 16, 255, 40),
+                                                        ("bf16", 5, 5, 1, 300), ("f32", 3, 4, 7, 90)])
+def test_gpu_scores_with_odd_tables(dtype, n_sub, sub_d, n_cent, S):
+    """`sah_pq_scores` with an odd number of table entries (8 bytes each in bfloat16: the queries
+    behind them start on the next 16-byte boundary): table entries summed over ascending channels and
+    rounded, an entry per sub-vector added in float32 and rounded once."""
+    import torch
+    from oracle.bf16 import round_bf16
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    dt = workloads.torch_dtype(dtype)
+    rnd = round_bf16 if dtype == "bf16" else (lambda a: a.astype(np.float32))
+    B, Hq, Hkv, Sq, off = 2, 6, 2, 1, 3
+    gen = torch.Generator(device=dev).manual_seed(n_cent)
+    # multiples of 1/8 below 4: every product and partial sum is exact in float32
+    q = (torch.randint(-31, 32, (B, Hq, Sq, n_sub * sub_d), generator=gen, device=dev) / 8.0).to(dt)
+    cent = (torch.randint(-31, 32, (B * Hkv * n_sub, n_cent, sub_d), generator=gen, device=dev) / 8.0).to(dt)
+    codes = torch.randint(0, n_cent, (B, Hkv, S, n_sub), generator=gen, device=dev).to(torch.uint8)
+    got = torch.zeros((B, Hq, Sq, S), dtype=dt, device=dev)
+    _native.check(lib.sah_pq_scores(q.data_ptr(), _native.dtype_code(dt), q.stride(0), q.stride(1), q.stride(2),
+                                    cent.data_ptr(), codes.data_ptr(), S, B, Hq, Hkv, Sq, S - off, off, S, n_sub, sub_d,
+                                    n_cent, got.data_ptr(), None, 0, _native.stream_of(torch.device(dev))), "sah_pq_scores")
+    qn = q.float().cpu().numpy().reshape(B, Hkv, Hq // Hkv, n_sub, sub_d)
+    cn = cent.float().cpu().numpy().reshape(B, Hkv, n_sub, n_cent, sub_d)
+    table = rnd(np.einsum("bhgsd,bhscd->bhgsc", qn, cn).astype(np.float32)).astype(np.float32)
+    want = np.zeros((B, Hkv, Hq // Hkv, S - off), np.float32)
+    c = codes.cpu().numpy()[:, :, :S - off].astype(np.int64)
+    for s in range(n_sub):
+        want += np.take_along_axis(table[:, :, :, s], np.broadcast_to(c[:, :, None, :, s], want.shape), axis=3)
+    np.testing.assert_array_equal(got.float().cpu().numpy()[..., off:].reshape(want.shape), rnd(want))
+    assert bool((got[..., :off] == 0).all())
