@@ -227,14 +227,15 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
 // Bound: shared-memory integer atomics and L2 (every 32-byte sector of a key is fetched by the
 // CTAs of two sub-vectors).  8 KV heads x 65472 keys x 16 sub-vectors: 96 us with eight keys of a
 // centroid in flight, 122 us with four and three CTAs per SM; with one fp64 shared-memory atomic
-// per key and channel -- a compare-and-swap loop -- it took 812 us.
+// per key and channel -- a compare-and-swap loop -- it took 812 us.  Sub-vectors
+// of more than 16 channels are cut into blocks of 16 (`cblocks`), a CTA each; the first block counts.
 #define PQA_THREADS 512
 #define PQA_STRIP 4096
 
 template <typename T>
 __global__ void __launch_bounds__(PQA_THREADS, 2)
 pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
-                     int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int vec8,
+                     int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int cblocks, int vec8,
                      const uint8_t* __restrict__ codes, int64_t cap, double* __restrict__ sums,
                      int* __restrict__ counts) {
   __shared__ int pos_sm[256];              // histogram, then the next free slot of every centroid
@@ -244,14 +245,15 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
   constexpr int HALF = (PQ_MAX_SUBD + 1) / 2;
   constexpr int PER = PQA_STRIP / PQA_THREADS;
   const int tid = threadIdx.x;
-  const int sub = blockIdx.y;
+  const int sub = blockIdx.y / cblocks, c_lo = (blockIdx.y - sub * cblocks) * PQ_MAX_SUBD;
   const int64_t bk = blockIdx.z;
   const int kvh = (int)(bk % Hkv);
   const int64_t b = bk / Hkv;
   const int64_t grp = bk * n_sub + sub;
   const int cent = tid >> 1;
-  const int half = (sub_d + 1) / 2;        // channels of the even threads
-  const int d0 = (tid & 1) ? half : 0, nd = (tid & 1) ? sub_d - half : half;
+  const int nch = sub_d - c_lo < PQ_MAX_SUBD ? sub_d - c_lo : PQ_MAX_SUBD;  // channels of this CTA
+  const int half = (nch + 1) / 2;          // channels of the even threads
+  const int d0 = c_lo + ((tid & 1) ? half : 0), nd = (tid & 1) ? nch - half : half;
   const T* xg = x + b * xs_b + kvh * xs_h + init_offset * xs_s + sub * sub_d + d0;
   const uint8_t* cg = codes + bk * cap * n_sub + sub;
   double acc[HALF];
@@ -327,7 +329,7 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
 #pragma unroll
     for (int i = 0; i < HALF; ++i)
       if (i < nd) atomicAdd(out + i, acc[i]);
-    if ((tid & 1) == 0) atomicAdd(&counts[grp * n_cent + cent], count);
+    if ((tid & 1) == 0 && c_lo == 0) atomicAdd(&counts[grp * n_cent + cent], count);
   }
 }
 
@@ -339,21 +341,19 @@ extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t
   SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_cent > 0 && n_keys >= 0,
               "pq_accumulate: bad extents");
   if (n_keys == 0) return SAH_OK;
-  if (sub_d > PQ_MAX_SUBD || n_cent > 256)
-    return sah_fail(SAH_ERR_UNSUPPORTED, "pq_accumulate: sub-vector dim %d (<= %d) / %d centroids (<= 256)",
-                    sub_d, PQ_MAX_SUBD, n_cent);
   // one wave of two CTAs per SM; the strips of a slice share the CTA's registers
-  const int64_t groups = (int64_t)B * Hkv * n_sub;
+  const int cblocks = (sub_d + PQ_MAX_SUBD - 1) / PQ_MAX_SUBD;
+  const int64_t groups = (int64_t)B * Hkv * n_sub * cblocks;
   int64_t slices = (int64_t)2 * 148 / groups;
   if (slices < 1) slices = 1;
   const int64_t strips = sah_ceil_div(n_keys, (int64_t)PQA_STRIP);
   if (slices > strips) slices = strips;
-  dim3 grid((unsigned)slices, (unsigned)n_sub, (unsigned)((int64_t)B * Hkv));
+  dim3 grid((unsigned)slices, (unsigned)(n_sub * cblocks), (unsigned)((int64_t)B * Hkv));
   const int vec8 = sub_d == 8 && (reinterpret_cast<uintptr_t>(x) & 7) == 0 && xs_s % 4 == 0 && xs_h % 4 == 0 &&
                    xs_b % 4 == 0;
   SAH_DISPATCH_DTYPE(dtype, T, {
     pq_accumulate_kernel<T><<<grid, PQA_THREADS, 0, (cudaStream_t)stream>>>(
-        (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, vec8, codes, cap,
+        (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, cblocks, vec8, codes, cap,
         sums, counts);
   });
   SAH_LAUNCH_CHECK("pq_accumulate");
@@ -378,29 +378,33 @@ __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t 
   float move = 0.f;
   const int c = threadIdx.x;
   if (c < n_cent) {
-    // everything that may be needed is requested before the first use (a channel at a time, each
-    // with its own loads, took 16 to 29 us for 128 groups of 256 centres; 4.3 us this way)
+    // everything that may be needed is requested before the first use, 16 channels at a time (a
+    // channel at a time, each with its own loads, took 16 to 29 us for 128 groups of 256 centres of
+    // 8 channels; 4.3 us this way)
     const int cnt = counts[grp * n_cent + c];
-    const double* sp = sums + (grp * n_cent + c) * sub_d;
-    float* cp = centroids + (grp * n_cent + c) * sub_d;
-    double sv[PQ_MAX_SUBD];
-    float old[PQ_MAX_SUBD];
-#pragma unroll
-    for (int d = 0; d < PQ_MAX_SUBD; ++d) {
-      sv[d] = d < sub_d ? sp[d] : 0.0;
-      old[d] = d < sub_d ? cp[d] : 0.f;
-    }
     const T* xr = nullptr;
     if (cnt <= 0) xr = x + b * xs_b + kvh * xs_h + (reseed[grp * n_cent + c] + init_offset) * xs_s + sub * sub_d;
     float d2 = 0.f;
+    for (int c_lo = 0; c_lo < sub_d; c_lo += PQ_MAX_SUBD) {
+      const double* sp = sums + (grp * n_cent + c) * sub_d + c_lo;
+      float* cp = centroids + (grp * n_cent + c) * sub_d + c_lo;
+      const int nch = sub_d - c_lo;
+      double sv[PQ_MAX_SUBD];
+      float old[PQ_MAX_SUBD];
 #pragma unroll
-    for (int d = 0; d < PQ_MAX_SUBD; ++d)
-      if (d < sub_d) {
-        const float nv = cnt > 0 ? __fdiv_rn((float)sv[d], (float)cnt) : sah_to_float<T>(xr[d]);
-        const float t = __fsub_rn(nv, old[d]);
-        d2 = __fadd_rn(d2, __fmul_rn(t, t));
-        cp[d] = nv;
+      for (int d = 0; d < PQ_MAX_SUBD; ++d) {
+        sv[d] = d < nch ? sp[d] : 0.0;
+        old[d] = d < nch ? cp[d] : 0.f;
       }
+#pragma unroll
+      for (int d = 0; d < PQ_MAX_SUBD; ++d)
+        if (d < nch) {
+          const float nv = cnt > 0 ? __fdiv_rn((float)sv[d], (float)cnt) : sah_to_float<T>(xr[c_lo + d]);
+          const float t = __fsub_rn(nv, old[d]);
+          d2 = __fadd_rn(d2, __fmul_rn(t, t));
+          cp[d] = nv;
+        }
+    }
     move = sqrtf(d2);
   }
   float total;

@@ -379,3 +379,54 @@ def test_gpu_scores_with_odd_tables(dtype, n_sub, sub_d, n_cent, S):
         want += np.take_along_axis(table[:, :, :, s], np.broadcast_to(c[:, :, None, :, s], want.shape), axis=3)
     np.testing.assert_array_equal(got.float().cpu().numpy()[..., off:].reshape(want.shape), rnd(want))
     assert bool((got[..., :off] == 0).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,n_sub,sub_d,n_cent", [("bf16", 2, 32, 40), ("f32", 3, 17, 33), ("bf16", 4, 16, 256),
+                                                      ("f32", 1, 50, 300)])
+def test_gpu_centres_of_wide_subvectors(dtype, n_sub, sub_d, n_cent):
+    """`sah_pq_accumulate` and `sah_pq_update` with sub-vectors of up to and over 16 channels (and,
+    for the sums, more centroids than a byte can name): exact sums and counts; every channel of every
+    centre replaced, empty clusters by their key, and the moves of all channels in `shift2`."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, n_keys = 1, 2, 4500
+    dt = workloads.torch_dtype(dtype)
+    gen = torch.Generator(device=dev).manual_seed(sub_d)
+    # multiples of 1/16 below 16 (8 significant bits): sums are exact in any order
+    keys = (torch.randint(-255, 256, (B, Hkv, n_keys, n_sub * sub_d), generator=gen, device=dev) / 16.0).to(dt)
+    used = min(n_cent, 256) - 1                      # the last centroid that a code names stays empty
+    codes = torch.randint(0, used, (B, Hkv, n_keys, n_sub), generator=gen, device=dev).to(torch.uint8)
+    groups = B * Hkv * n_sub
+    sums = torch.zeros((groups, n_cent, sub_d), dtype=torch.float64, device=dev)
+    counts = torch.zeros((groups, n_cent), dtype=torch.int32, device=dev)
+    st = _native.stream_of(torch.device(dev))
+    kargs = (keys.data_ptr(), _native.dtype_code(dt), keys.stride(0), keys.stride(1), keys.stride(2), B, Hkv)
+    _native.check(lib.sah_pq_accumulate(*kargs, n_keys, 0, n_sub, sub_d, n_cent, codes.data_ptr(), n_keys,
+                                        sums.data_ptr(), counts.data_ptr(), st), "sah_pq_accumulate")
+    x = keys.double().cpu().numpy().reshape(B * Hkv, n_keys, n_sub, sub_d)
+    c = codes.cpu().numpy().reshape(B * Hkv, n_keys, n_sub)
+    want, cnt = np.zeros((groups, n_cent, sub_d)), np.zeros((groups, n_cent), np.int64)
+    for g in range(groups):
+        np.add.at(want[g], c[g // n_sub, :, g % n_sub], x[g // n_sub, :, g % n_sub])
+        cnt[g] = np.bincount(c[g // n_sub, :, g % n_sub], minlength=n_cent)
+    np.testing.assert_array_equal(counts.cpu().numpy(), cnt)
+    np.testing.assert_array_equal(sums.cpu().numpy(), want)
+    if n_cent > 256:
+        return
+    cent = torch.randn((groups, n_cent, sub_d), generator=gen, device=dev)
+    reseed = torch.randint(0, n_keys, (groups, n_cent), generator=gen, device=dev)
+    new, shift2 = cent.clone(), torch.zeros(groups, device=dev)
+    _native.check(lib.sah_pq_update(*kargs, 0, n_sub, sub_d, n_cent, sums.data_ptr(), counts.data_ptr(),
+                                    reseed.data_ptr(), new.data_ptr(), shift2.data_ptr(), st), "sah_pq_update")
+    g = np.arange(groups)[:, None]
+    seeds = x[g // n_sub, reseed.cpu().numpy(), g % n_sub].astype(np.float32)
+    mean = want.astype(np.float32) / np.maximum(cnt, 1).astype(np.float32)[..., None]
+    centres = np.where(cnt[..., None] > 0, mean, seeds).astype(np.float32)
+    np.testing.assert_array_equal(new.cpu().numpy(), centres)
+    moves = np.sqrt(((centres.astype(np.float64) - cent.double().cpu().numpy()) ** 2).sum(-1)).sum(-1) ** 2
+    # float32 sums of sub_d squares and of n_cent roots, squared: within (sub_d + 2 n_cent) 2^-23 < 1e-4
+    np.testing.assert_allclose(shift2.cpu().numpy(), moves, rtol=1e-4)
