@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t ptc_candidates(const uint32_t* v, float thr)
   return ~((below[0] << 24) | (below[1] << 16) | (below[2] << 8) | below[3]);
 }
 
-// NB: blocks of 32 accumulator columns (n_cent <= 32 NB; the columns past n_cent hold -5e29)
+// NB: blocks of 32 accumulator columns (n_cent <= 32 NB; the columns past n_cent hold -inf)
 template <int NS, int NB>
 __global__ void __launch_bounds__(PTC_THREADS, 1)
 pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
@@ -178,7 +178,8 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
         ptc_split3(v, hi + d, mi + d, lo + d);
         nn[d] = __float2bfloat16_rn(0.f);
       }
-      ptc_split3(c < n_cent ? -0.5f * n2 : -5e29f, nn, nn + 1, nn + 2);
+      if (c < n_cent) ptc_split3(-0.5f * n2, nn, nn + 1, nn + 2);
+      else nn[0] = __float2bfloat16_rn(-INFINITY);  // below every centroid, however far out those lie
       // a NaN or infinite norm makes the margin NaN or infinite: every centroid is then measured
       if (c < n_cent) atomicMax(cmax_sm + s, __float_as_uint(n2));
       unsigned char* row = sm + C::B_OFF + s * (256 * 128) + c * 128;

@@ -430,3 +430,31 @@ def test_gpu_centres_of_wide_subvectors(dtype, n_sub, sub_d, n_cent):
     moves = np.sqrt(((centres.astype(np.float64) - cent.double().cpu().numpy()) ** 2).sum(-1)).sum(-1) ** 2
     # float32 sums of sub_d squares and of n_cent roots, squared: within (sub_d + 2 n_cent) 2^-23 < 1e-4
     np.testing.assert_allclose(shift2.cpu().numpy(), moves, rtol=1e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_cent,scale", [(16, 2.0 ** 52), (48, 2.0 ** 60), (80, 2.0 ** -40), (256, 2.0 ** 60)])
+def test_gpu_assignment_of_keys_far_from_one(n_cent, scale):
+    """Columns that pad the centroids of `sah_pq_assign_tc` to a power of two lie below every
+    centroid's, whatever the keys' magnitude: the codes of `sah_pq_assign`."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, n_sub, n_keys = 1, 2, 4, 700
+    gen = torch.Generator(device=dev).manual_seed(n_cent)
+    keys = (torch.randn((B, Hkv, n_keys, n_sub * 8), generator=gen, device=dev) * scale).to(torch.bfloat16)
+    cent = (torch.randn((B * Hkv * n_sub, n_cent, 8), generator=gen, device=dev) + 3.0) * scale
+    st = _native.stream_of(torch.device(dev))
+    want = torch.full((B, Hkv, n_keys, n_sub), 255, dtype=torch.uint8, device=dev)
+    got = want.clone()
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    strides = (keys.stride(0), keys.stride(1), keys.stride(2))
+    _native.check(lib.sah_pq_assign(keys.data_ptr(), _native.SAH_BF16, *strides, B, Hkv, 0, n_keys, 0, n_sub, 8, n_cent,
+                                    cent.data_ptr(), want.data_ptr(), n_keys, 0, st), "sah_pq_assign")
+    _native.check(lib.sah_pq_assign_tc(keys.data_ptr(), *strides, B, Hkv, 0, n_keys, 0, n_sub, 8, n_cent,
+                                       cent.data_ptr(), got.data_ptr(), n_keys, err.data_ptr(), 148, st),
+                  "sah_pq_assign_tc")
+    assert int(err.item()) == 0 and torch.equal(got, want)
+    assert len(torch.unique(want)) > 4
