@@ -236,6 +236,12 @@ int sah_topk_select(const void* scores, int dtype, int64_t rows, int64_t S, int6
 int sah_topk_select_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S,
                           int64_t W, int64_t col_begin, int64_t col_end, int n_bands,
                           const int64_t* bands, int64_t k, uint32_t* out_bits, void* stream);
+/* The same; prev_bits also receives the bands as a bitmap (every word of it), for readers of the
+ * previous mask.  It must not be out_bits. */
+int sah_topk_select_fill_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S,
+                               int64_t W, int64_t col_begin, int64_t col_end, int n_bands,
+                               const int64_t* bands, uint32_t* prev_bits, int64_t k,
+                               uint32_t* out_bits, void* stream);
 /* 1 when the keys of such rows fit in the shared memory of the cluster of CTAs that
  * sah_topk_select gives a row to (then it is the faster form), else 0. */
 int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W);
@@ -614,6 +620,12 @@ int sah_attn_plan(const uint32_t* bits, const void* data, const int32_t* wpre,
 int sah_attn_plan_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv,
                         int Sq, int64_t S, const sah_attn_sizes* sizes, int32_t* ucols,
                         uint16_t* umemb, int32_t* ucount, void* stream);
+/* The same; bits [rows][W] also receives the mask as a bitmap (every word of it; W as the library
+ * rounds it, the words of S keys up to a multiple of four). */
+int sah_attn_plan_fill_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv,
+                             int Sq, int64_t S, int64_t W, const sah_attn_sizes* sizes,
+                             uint32_t* bits, int32_t* ucols, uint16_t* umemb, int32_t* ucount,
+                             void* stream);
 
 /* The same for a MagicPig mask whose weights sah_masked_attention_lsh evaluates itself
  * (sizes queried with has_data = 2; at most 4 mask rows per KV group).  `bits` are the

@@ -136,10 +136,12 @@ template <typename T, int RMAX>
 __global__ void __launch_bounds__(PLAN_FUSED_THREADS)
 attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ data,
                        const int32_t* __restrict__ wpre, const int64_t* __restrict__ ptr,
-                       PlanGeom p, const __grid_constant__ MaskBands bands, int32_t* __restrict__ ucols,
-                       uint16_t* __restrict__ umemb, float* __restrict__ uw, int32_t* __restrict__ ucount) {
+                       PlanGeom p, const __grid_constant__ MaskBands bands, uint32_t* __restrict__ band_bits,
+                       int32_t* __restrict__ ucols, uint16_t* __restrict__ umemb, float* __restrict__ uw,
+                       int32_t* __restrict__ ucount) {
   sah_pdl_entry_early();
-  // word of a mask row: from the bitmap, or (no bitmap) from the mask's bands
+  // word of a mask row: from the bitmap, or (no bitmap) from the mask's bands; those are written
+  // out as a bitmap for whoever reads the mask later, if there is a place for it
   auto row_word = [&](int64_t row, int64_t wi) -> uint32_t {
     return bits != nullptr ? bits[row * p.W + wi] : sah_band_bits(bands, row % p.Sq, wi * 32, 32, p.S, 0u);
   };
@@ -175,6 +177,7 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
       if (uw != nullptr && words[r]) dbase[r] = ptr[rows[r]] + wpre[rows[r] * p.W + w];
     }
     u |= words[r];
+    if (band_bits != nullptr && w < p.W && rows[r] >= 0) band_bits[rows[r] * p.W + w] = words[r];
   }
   int base = 0;
   if (w0 > 0) {
@@ -392,7 +395,7 @@ static int plan_geometry(int B, int Hq, int Hkv, int Sq, int64_t S, int64_t W,
 
 static int attn_plan_impl(const uint32_t* bits, const MaskBands& bands, const void* data, const int32_t* wpre,
                           const int64_t* ptr, int dtype, int B, int Hq, int Hkv, int Sq,
-                          int64_t S, int64_t W, const sah_attn_sizes* sizes, int32_t* ucols,
+                          int64_t S, int64_t W, const sah_attn_sizes* sizes, uint32_t* band_bits, int32_t* ucols,
                           uint16_t* umemb, float* uw, int32_t* ucount, void* stream) {
   PlanGeom p;
   int rc0 = plan_geometry(B, Hq, Hkv, Sq, S, W, sizes, &p);
@@ -411,10 +414,10 @@ static int attn_plan_impl(const uint32_t* bits, const MaskBands& bands, const vo
     SAH_DISPATCH_DTYPE(dtype, T, {
       if (p.R <= 4)
         sah_launch_chain(attn_plan_fused_kernel<T, 4>, fgrid, PLAN_FUSED_THREADS, 0, st, bits, (const T*)data,
-            wpre, ptr, p, bands, ucols, umemb, data ? uw : nullptr, ucount);
+            wpre, ptr, p, bands, band_bits, ucols, umemb, data ? uw : nullptr, ucount);
       else
         sah_launch_chain(attn_plan_fused_kernel<T, AT_MAXR>, fgrid, PLAN_FUSED_THREADS, 0, st, bits,
-            (const T*)data, wpre, ptr, p, bands, ucols, umemb, data ? uw : nullptr, ucount);
+            (const T*)data, wpre, ptr, p, bands, band_bits, ucols, umemb, data ? uw : nullptr, ucount);
     });
     SAH_LAUNCH_CHECK("attn_plan_fused");
     sah_prof_end(SAH_PROF_ATTN_PLAN, (cudaStream_t)stream);
@@ -445,19 +448,37 @@ extern "C" int sah_attn_plan(const uint32_t* bits, const void* data, const int32
   SAH_REQUIRE(bits && sizes && ucols && umemb && ucount, "attn_plan: null pointer");
   SAH_REQUIRE(data == nullptr || (wpre && ptr && uw), "attn_plan: data needs wpre, ptr and uw");
   SAH_REQUIRE(W * 32 >= S, "attn_plan: W too small");
-  return attn_plan_impl(bits, MaskBands(), data, wpre, ptr, dtype, B, Hq, Hkv, Sq, S, W, sizes, ucols, umemb, uw,
-                        ucount, stream);
+  return attn_plan_impl(bits, MaskBands(), data, wpre, ptr, dtype, B, Hq, Hkv, Sq, S, W, sizes, nullptr, ucols,
+                        umemb, uw, ucount, stream);
 }
 
-extern "C" int sah_attn_plan_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv, int Sq,
-                                   int64_t S, const sah_attn_sizes* sizes, int32_t* ucols, uint16_t* umemb,
-                                   int32_t* ucount, void* stream) {
+static int attn_plan_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv, int Sq, int64_t S,
+                           int64_t W, const sah_attn_sizes* sizes, uint32_t* bits, int32_t* ucols, uint16_t* umemb,
+                           int32_t* ucount, void* stream) {
   SAH_REQUIRE(sizes && ucols && umemb && ucount, "attn_plan_bands: null pointer");
   SAH_REQUIRE(n_bands >= 0 && n_bands <= SAH_MAX_BANDS && (n_bands == 0 || bands != nullptr),
               "attn_plan_bands: 0..%d bands", SAH_MAX_BANDS);
   SAH_REQUIRE(S > 0 && Sq > 0, "attn_plan_bands: bad extents");
   return attn_plan_impl(nullptr, sah_make_bands(n_bands, bands), nullptr, nullptr, nullptr, dtype, B, Hq, Hkv, Sq, S,
-                        (S + 31) / 32, sizes, ucols, umemb, nullptr, ucount, stream);
+                        W, sizes, bits, ucols, umemb, nullptr, ucount, stream);
+}
+
+extern "C" int sah_attn_plan_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv, int Sq,
+                                   int64_t S, const sah_attn_sizes* sizes, int32_t* ucols, uint16_t* umemb,
+                                   int32_t* ucount, void* stream) {
+  return attn_plan_bands(n_bands, bands, dtype, B, Hq, Hkv, Sq, S, (S + 31) / 32, sizes, nullptr, ucols, umemb,
+                         ucount, stream);
+}
+
+extern "C" int sah_attn_plan_fill_bands(int n_bands, const int64_t* bands, int dtype, int B, int Hq, int Hkv, int Sq,
+                                        int64_t S, int64_t W, const sah_attn_sizes* sizes, uint32_t* bits,
+                                        int32_t* ucols, uint16_t* umemb, int32_t* ucount, void* stream) {
+  SAH_REQUIRE(bits != nullptr, "attn_plan_fill_bands: null pointer");
+  // the words of a row are those of the CTAs that plan it
+  SAH_REQUIRE(S > 0 && W * 32 >= S &&
+                  sah_ceil_div(W, PLAN_FUSED_THREADS) == sah_ceil_div(sah_ceil_div(S, 32), PLAN_FUSED_THREADS),
+              "attn_plan_fill_bands: rows of %lld words for %lld keys", (long long)W, (long long)S);
+  return attn_plan_bands(n_bands, bands, dtype, B, Hq, Hkv, Sq, S, W, sizes, bits, ucols, umemb, ucount, stream);
 }
 
 extern "C" int sah_attn_plan_lsh(const uint32_t* bits, const uint32_t* unit_bits, const float* dens,

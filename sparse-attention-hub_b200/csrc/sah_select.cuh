@@ -111,7 +111,7 @@ struct SahScoreKeys<float, 32> {
 template <int KEYBITS, typename Keys, bool RESIDENT>
 __global__ void __launch_bounds__(SAH_SELECT_THREADS)
 sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __grid_constant__ MaskBands bands, int Sq,
-                  uint32_t* __restrict__ out_bits, int64_t S, int64_t W, int64_t col_begin, int64_t col_end,
+                  uint32_t* __restrict__ band_bits, uint32_t* __restrict__ out_bits, int64_t S, int64_t W, int64_t col_begin, int64_t col_end,
                   long long k) {
   sah_pdl_entry();
   namespace cg = cooperative_groups;
@@ -130,8 +130,10 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int64_t row = blockIdx.x / ranks;
   keys.open(row);
-  // the previous mask: a bitmap, or (no bitmap) its bands
+  // the previous mask: a bitmap, or (no bitmap) its bands, written out as a bitmap for whoever
+  // reads that mask later if there is a place for it
   const unsigned char* pb = prev_bits == nullptr ? nullptr : reinterpret_cast<const unsigned char*>(prev_bits + row * W);
+  unsigned char* bb = band_bits == nullptr ? nullptr : reinterpret_cast<unsigned char*>(band_bits + row * W);
   unsigned char* ob = reinterpret_cast<unsigned char*>(out_bits + row * W);
   if (col_begin < 0) col_begin = 0;
   if (col_end > S) col_end = S;
@@ -142,6 +144,7 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
   const int blocks = (ny + 31) / 32;
   const int q_lo = (int)((int64_t)blocks * warp / nw), q_hi = (int)((int64_t)blocks * (warp + 1) / nw);
   if (pb != nullptr) pb += y_lo;
+  if (bb != nullptr) bb += y_lo;
   ob += y_lo;
   // bytes [gap_lo, gap_hi) of this CTA lie between the bands that begin the row and the others:
   // nearly all of them, and empty
@@ -406,6 +409,7 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
       quota -= __shfl_sync(0xffffffffu, incl, 31);
     }
     if (y < ny) ob[y] = (unsigned char)(prev | gt);
+    if (Keys::BANDS && bb != nullptr && y < ny) bb[y] = (unsigned char)prev;
   }
   if (ranks > 1) cluster.sync();  // nobody leaves while its counters may be read
 }
@@ -429,7 +433,8 @@ static inline int64_t sah_select_key_bytes(int64_t rows, int64_t S, int64_t W, i
 template <int KEYBITS, typename Keys>
 static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits, uint32_t* out_bits, int64_t rows,
                                     int64_t S, int64_t W, int64_t col_begin, int64_t col_end, int64_t k,
-                                    cudaStream_t st, const MaskBands& bands = MaskBands(), int Sq = 1) {
+                                    cudaStream_t st, const MaskBands& bands = MaskBands(), int Sq = 1,
+                                    uint32_t* band_bits = nullptr) {
   const int ranks = sah_select_ranks(rows, S);
   // half-size CTAs for short rows and when rows queue for SMs
   const int nt = W * 4 / ranks <= SAH_SELECT_MIN_THREADS || rows * ranks > 148 ? SAH_SELECT_MIN_THREADS
@@ -455,10 +460,10 @@ static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits,
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "select attr: %s", cudaGetErrorString(e));
     }
     (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, true>, keys, prev_bits, bands, Sq,
-                             out_bits, S, W, col_begin, col_end, (long long)k);
+                             band_bits, out_bits, S, W, col_begin, col_end, (long long)k);
   } else {
     (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, false>, keys, prev_bits, bands, Sq,
-                             out_bits, S, W, col_begin, col_end, (long long)k);
+                             band_bits, out_bits, S, W, col_begin, col_end, (long long)k);
   }
   return SAH_OK;  // a launch error stays for SAH_LAUNCH_CHECK
 }

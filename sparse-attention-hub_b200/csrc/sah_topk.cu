@@ -757,13 +757,15 @@ static int sel_run(const T* scores, int64_t rows, int64_t S, int64_t W, int64_t 
   return SAH_OK;
 }
 
-extern "C" int sah_topk_select_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S, int64_t W,
-                                     int64_t col_begin, int64_t col_end, int n_bands, const int64_t* bands,
-                                     int64_t k, uint32_t* out_bits, void* stream) {
+// The previous mask as its bands; prev_bits (may be NULL) receives them as a bitmap.
+static int select_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S, int64_t W, int64_t col_begin,
+                        int64_t col_end, int n_bands, const int64_t* bands, uint32_t* prev_bits, int64_t k,
+                        uint32_t* out_bits, void* stream) {
   SAH_REQUIRE(scores && out_bits, "topk_select_bands: null pointer");
   SAH_REQUIRE(rows >= 0 && Sq > 0 && S > 0 && W * 32 >= S, "topk_select_bands: bad extents");
   SAH_REQUIRE(n_bands >= 0 && n_bands <= SAH_MAX_BANDS && (n_bands == 0 || bands != nullptr),
               "topk_select_bands: 0..%d bands", SAH_MAX_BANDS);
+  SAH_REQUIRE(prev_bits != out_bits, "topk_select_fill_bands: the two bitmaps must be different ones");
   if (rows == 0) return SAH_OK;
   const MaskBands mb = sah_make_bands(n_bands, bands);
   cudaStream_t st = (cudaStream_t)stream;
@@ -771,10 +773,10 @@ extern "C" int sah_topk_select_bands(const void* scores, int dtype, int64_t rows
   int rc;
   if (dtype == SAH_BF16) {
     const SahScoreKeys<__nv_bfloat16, 16> keys{(const __nv_bfloat16*)scores, S};
-    rc = sah_select_launch<16>(keys, nullptr, out_bits, rows, S, W, col_begin, col_end, k, st, mb, Sq);
+    rc = sah_select_launch<16>(keys, nullptr, out_bits, rows, S, W, col_begin, col_end, k, st, mb, Sq, prev_bits);
   } else if (dtype == SAH_F32) {
     const SahScoreKeys<float, 32> keys{(const float*)scores, S};
-    rc = sah_select_launch<32>(keys, nullptr, out_bits, rows, S, W, col_begin, col_end, k, st, mb, Sq);
+    rc = sah_select_launch<32>(keys, nullptr, out_bits, rows, S, W, col_begin, col_end, k, st, mb, Sq, prev_bits);
   } else {
     return sah_fail(SAH_ERR_INVALID, "topk_select_bands: unknown dtype %d", dtype);
   }
@@ -782,6 +784,19 @@ extern "C" int sah_topk_select_bands(const void* scores, int dtype, int64_t rows
   SAH_LAUNCH_CHECK("topk_select_bands");
   sah_prof_end(SAH_PROF_TOPK_SELECT, st);
   return SAH_OK;
+}
+
+extern "C" int sah_topk_select_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S, int64_t W,
+                                     int64_t col_begin, int64_t col_end, int n_bands, const int64_t* bands,
+                                     int64_t k, uint32_t* out_bits, void* stream) {
+  return select_bands(scores, dtype, rows, Sq, S, W, col_begin, col_end, n_bands, bands, nullptr, k, out_bits, stream);
+}
+
+extern "C" int sah_topk_select_fill_bands(const void* scores, int dtype, int64_t rows, int Sq, int64_t S, int64_t W,
+                                          int64_t col_begin, int64_t col_end, int n_bands, const int64_t* bands,
+                                          uint32_t* prev_bits, int64_t k, uint32_t* out_bits, void* stream) {
+  SAH_REQUIRE(prev_bits != nullptr, "topk_select_fill_bands: null pointer");
+  return select_bands(scores, dtype, rows, Sq, S, W, col_begin, col_end, n_bands, bands, prev_bits, k, out_bits, stream);
 }
 
 extern "C" int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W) {

@@ -78,6 +78,7 @@ _SIGNATURES = {
                       _L, _P, _P],
     "sah_topk_select": [_P, _I, _L, _L, _L, _L, _L, _P, _L, _P, _P],
     "sah_topk_select_bands": [_P, _I, _L, _I, _L, _L, _L, _L, _I, _P, _L, _P, _P],
+    "sah_topk_select_fill_bands": [_P, _I, _L, _I, _L, _L, _L, _L, _I, _P, _P, _L, _P, _P],
     "sah_topk_select_fits": [_I, _L, _L, _L],  # returns 0 or 1
     "sah_topk_select_ws_bytes": [_L, _L],  # returns int64
     "sah_topk_sel_hist_offset": [_L, _L],  # returns int64
@@ -90,6 +91,7 @@ _SIGNATURES = {
     "sah_attn_plan": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _L, POINTER(AttnSizes), _P, _P,
                       _P, _P, _P],
     "sah_attn_plan_bands": [_I, _P, _I, _I, _I, _I, _I, _L, POINTER(AttnSizes), _P, _P, _P, _P],
+    "sah_attn_plan_fill_bands": [_I, _P, _I, _I, _I, _I, _I, _L, _L, POINTER(AttnSizes), _P, _P, _P, _P, _P],
     "sah_masked_attention": [_P, _P, _P, _I, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _I, _I, _I,
                              _L, _I, c_float, _P, _L, _L, _L, _P, POINTER(AttnSizes), _P, _P, _P,
                              _P, _P, _P, _P, _P],

@@ -78,13 +78,15 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
     dst = out if out is not None else NativeBits(
         torch.empty((prev.rows, prev.words), dtype=torch.int32, device=sc.device), rows, S)
     fits = lib.sah_topk_select_fits(_native.dtype_code(sc.dtype), rows, S, prev.words)
-    bands = prev.pending_bands() if fits and prev.rows == rows else None
+    bands = prev.pending_bands() if fits and prev.rows == rows and out is None else None
     if bands is not None:
-        # the previous mask is a sink and a window that nobody has needed as a bitmap so far
+        # the previous mask is a sink and a window that nobody has needed as a bitmap so far; the
+        # kernel fills its words on the way
         _native.check(
-            lib.sah_topk_select_bands(sc.data_ptr(), _native.dtype_code(sc.dtype), rows, bands[2], S, prev.words,
-                                      col_begin, end, bands[0], bands[1], k, dst.bits.data_ptr(), st),
-            "sah_topk_select_bands")
+            lib.sah_topk_select_fill_bands(sc.data_ptr(), _native.dtype_code(sc.dtype), rows, bands[2], S, prev.words,
+                                           col_begin, end, bands[0], bands[1], prev.storage.data_ptr(), k,
+                                           dst.bits.data_ptr(), st), "sah_topk_select_fill_bands")
+        prev.bands_written()
         return dst
     if rows <= 65535 and not per_row and not fits:
         # rows are spread over many CTAs; the histograms live in a scratch buffer

@@ -144,14 +144,23 @@ class NativeBits:
 
     def pending_bands(self):
         """(number of bands, host array, query rows per (batch, head)) of a bitmap that is nothing
-        but noted bands on an empty mask, else None.  A kernel that takes the bands saves the
-        launch that would fill the words; the notes stay, so whoever asks for the words gets
-        them."""
+        but noted bands on an empty mask, else None.  A kernel that takes the bands and writes the
+        words beside its own work (`bands_written`) saves the launch that would fill them."""
         lazy = self._lazy
         if self._bits is None or not lazy["zero"]:
             return None
         bands = lazy["bands"]
         return len(bands), _BandArray(*[x for band in bands for x in band]), lazy["sq"]
+
+    @property
+    def storage(self) -> torch.Tensor:
+        """The words as they lie in memory, pending edits not applied."""
+        return self._bits
+
+    def bands_written(self) -> None:
+        """The pending bands have been written to the words by a kernel on the current stream."""
+        self._lazy["zero"] = False
+        self._lazy["bands"] = []
 
     def flush(self) -> None:
         """Apply the pending clear and band edits with one launch."""
@@ -165,8 +174,7 @@ class NativeBits:
             lib.sah_mask_fill_bands(self._bits.data_ptr(), self.rows, lazy["sq"], self.n_cols, self.words,
                                     len(bands), arr, int(lazy["zero"]),
                                     _native.stream_of(self._bits.device)), "sah_mask_fill_bands")
-        lazy["zero"] = False
-        lazy["bands"] = []
+        self.bands_written()
 
     def ensure_scan(self) -> None:
         """Fill ptr (int64 [rows+1]) and wpre (int32 [rows, W])."""

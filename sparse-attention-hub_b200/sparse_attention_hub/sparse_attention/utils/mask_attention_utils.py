@@ -171,9 +171,11 @@ def native_masked_attention(
             bands = nb.pending_bands() if has_data == 0 and S <= 32768 and nb.rows == B * Hq * Sq else None
             if bands is not None and bands[2] == Sq:
                 _native.check(
-                    lib.sah_attn_plan_bands(bands[0], bands[1], code, B, Hq, Hkv, Sq, S, ctypes.byref(sizes),
-                                            ws["ucols"].data_ptr(), ws["umemb"].data_ptr(),
-                                            ws["ucount"].data_ptr(), st), "sah_attn_plan_bands")
+                    lib.sah_attn_plan_fill_bands(bands[0], bands[1], code, B, Hq, Hkv, Sq, S, nb.words,
+                                                 ctypes.byref(sizes), nb.storage.data_ptr(),
+                                                 ws["ucols"].data_ptr(), ws["umemb"].data_ptr(),
+                                                 ws["ucount"].data_ptr(), st), "sah_attn_plan_fill_bands")
+                nb.bands_written()
             else:
                 _native.check(
                     lib.sah_attn_plan(nb.bits.data_ptr(), _native.ptr(nb.data), _native.ptr(nb.wpre),

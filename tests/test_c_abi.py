@@ -43,6 +43,14 @@ def test_bad_arguments_return_a_status_and_a_message():
     assert b"null" in lib.sah_last_error()
     assert lib.sah_hash_topk(None, 0, None, 32, None, 1, 0, 0, 0, 1, 1, 1, 32, 1, None, 1, None, None) == 1
     assert lib.sah_lsh_match(None, 32, None, 1, 4, 1, 4, 5, 4, 32, 1, None, None, None) == 1
+    # a bitmap of bands is written beside the result, not over it, in rows of the library's width
+    one = ctypes.c_void_p(16)  # never dereferenced: the calls are refused first
+    assert lib.sah_topk_select_fill_bands(one, 1, 1, 1, 32, 1, 0, 32, 0, None, one, 1, one, None) == 1
+    assert b"different" in lib.sah_last_error()
+    sizes = _native.AttnSizes()
+    assert lib.sah_attn_query_sizes(1, 8, 2, 1, 700, 128, 0, 148, ctypes.byref(sizes)) == 0
+    assert lib.sah_attn_plan_fill_bands(0, None, 1, 1, 8, 2, 1, 700, 257, ctypes.byref(sizes), one, one, one, one,
+                                        None) == 1
     with pytest.raises(_native.NativeLibraryError):
         _native.check(1, "sah_lsh_match")
     with pytest.raises(NotImplementedError):

@@ -576,8 +576,22 @@ def test_score_bits_at_the_edges(dtype, B, Hq, Hkv, Sq, S, D, masked):
 def test_band_masks_without_a_bitmap(dtype, S, Sq, stack, monkeypatch):
     """A mask of bands alone (sink and window, the future cleared for several query positions) goes
     to the selection and to the attention plan as bands: the same masks and the same output as
-    with the bitmap filled first."""
+    with the bitmap filled first.  The words of the mask that was handed over are written by the
+    kernel that took the bands, on its stream: whoever reads them afterwards, on whatever stream
+    that waited for the call, finds them without a launch of its own."""
+    from sparse_attention_hub import _native
     from sparse_attention_hub.sparse_attention.utils.mask import NativeBits
+
+    taken = []
+    pending = NativeBits.pending_bands
+
+    def noted(self):
+        bands = pending(self)
+        if bands is not None:
+            taken.append(self)
+        return bands
+
+    monkeypatch.setattr(NativeBits, "pending_bands", noted)
 
     torch.manual_seed(S)
     dt = torch.bfloat16 if dtype == "bf16" else torch.float32
@@ -591,10 +605,23 @@ def test_band_masks_without_a_bitmap(dtype, S, Sq, stack, monkeypatch):
     def run():
         mask = ra.build_mask(q, k, v, None, 0.125, 0.0, {}, layer_idx=0)
         out = get_masked_attention_output(None, q, k, v, None, None, 0.125, 0.0, mask)
+        before = _native.launch_count()
+        mask.native_bits().bits
+        assert _native.launch_count() == before
         return out, mask.get_dense_mask()
 
     out, dense = run()
+    assert (S > 32768 and stack == "fixed") or taken
     monkeypatch.setattr(NativeBits, "pending_bands", lambda self: None)
     want_out, want_dense = run()
+    fixed = workloads.research_attention(maskers[:2], dtype, DEV)
+    fixed_dense = fixed.build_mask(q, k, v, None, 0.125, 0.0, {}, layer_idx=0).get_dense_mask()
     assert torch.equal(dense, want_dense)
     assert torch.equal(out, want_out)
+    for bits in taken:
+        before = _native.launch_count()
+        words = bits.bits
+        assert _native.launch_count() == before
+        got = Mask._from_native((2, 4, Sq, S), dt, NativeBits(words, bits.rows, S)).get_dense_mask()
+        assert torch.equal(got, fixed_dense)
+        assert bool((words[:, (S + 31) // 32:] == 0).all())
