@@ -1105,11 +1105,11 @@ extern "C" int sah_attn_gather_probe(const void* k, const void* v, int64_t ks_b,
   cudaError_t e;
   sah_prof_begin(SAH_PROF_OTHER, st);
   if (D == 128) {
-    e = atm_allow_smem(attention_gather_probe_kernel<128>, AtmCfg<128>::SMEM, allowed[0]);
+    e = sah_allow_smem(attention_gather_probe_kernel<128>, AtmCfg<128>::SMEM, allowed[0]);
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "gather probe attr: %s", cudaGetErrorString(e));
     attention_gather_probe_kernel<128><<<grid, ATM_THREADS, AtmCfg<128>::SMEM, st>>>(a, sink);
   } else {
-    e = atm_allow_smem(attention_gather_probe_kernel<64>, AtmCfg<64>::SMEM, allowed[1]);
+    e = sah_allow_smem(attention_gather_probe_kernel<64>, AtmCfg<64>::SMEM, allowed[1]);
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "gather probe attr: %s", cudaGetErrorString(e));
     attention_gather_probe_kernel<64><<<grid, ATM_THREADS, AtmCfg<64>::SMEM, st>>>(a, sink);
   }

@@ -773,19 +773,6 @@ attention_gather_probe_kernel(AttnArgs a, unsigned int* __restrict__ sink) {
   if (acc == 0x9e3779b9u) *sink = acc;  // keeps the reads alive; practically never true
 }
 
-// The kernels ask for more dynamic shared memory than the default limit; the attribute is
-// set once per device and instantiation.
-template <typename Kernel>
-static cudaError_t atm_allow_smem(Kernel kernel, int smem, bool* done_by_device) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && done_by_device[dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done_by_device[dev] = true;
-  return e;
-}
-
 // ---- tensor maps of K and V for the TMA copy stage --------------------------------------
 typedef CUresult (*AtmEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -880,7 +867,7 @@ static int launch_attention_mma(AttnArgs a, int B, int groups, int* tickets, int
     const int smem = AtmCfg<D, TMA, NST>::SMEM;                                                     \
     if (merge_bytes > (size_t)ATM_WARPS * AtmCfg<D, TMA, NST>::WARP_BYTES)                          \
       return sah_fail(SAH_ERR_UNSUPPORTED, "attention: %d splits do not fit the merge scratch", a.nsplit); \
-    e = atm_allow_smem(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, smem, allowed[SLOT]);  \
+    e = sah_allow_smem(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, smem, allowed[SLOT]);  \
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "attention attr: %s", cudaGetErrorString(e)); \
     sah_launch_chain(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, grid, ATM_THREADS, smem, st, \
         a, maps, tickets, errflag, sinks, (__nv_bfloat16*)out, part_out);                           \

@@ -651,7 +651,7 @@ static int launch_attention_umma(AttnArgs a, int B, int groups, int* tickets, in
   cudaError_t e = cudaSuccess;
 #define AUM_LAUNCH(LSHW, RMAX, SLOT)                                                                  \
   do {                                                                                                \
-    e = atm_allow_smem(masked_attention_umma_kernel<LSHW, RMAX>, AumCfg::SMEM, allowed[SLOT]);        \
+    e = sah_allow_smem(masked_attention_umma_kernel<LSHW, RMAX>, AumCfg::SMEM, allowed[SLOT]);        \
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "attention attr: %s", cudaGetErrorString(e)); \
     sah_launch_chain(masked_attention_umma_kernel<LSHW, RMAX>, grid, AUM_THREADS, AumCfg::SMEM, st, \
         a, tickets, errflag, sinks, (__nv_bfloat16*)out, part_out);                             \

@@ -256,6 +256,20 @@ __device__ __forceinline__ void sah_pdl_entry_early() {
 // (SAH_PDL_MAX_WARPS replaces the 1024); 0 = no chaining at all, the default.
 int sah_pdl_max_warps();
 
+// Leave to launch `kernel` with up to `smem` bytes of dynamic shared memory on the current device.
+// The limit belongs to a device, so it is noted for each; a refusal is not.  `smem` is one constant
+// per kernel, so that threads that get here together cannot leave a smaller limit behind.
+template <typename Kernel>
+static cudaError_t sah_allow_smem(Kernel kernel, int smem, bool* done_by_device /* [64] */) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 0 && dev < 64 && done_by_device[dev]) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done_by_device[dev] = true;
+  return e;
+}
+
 template <typename... KArgs, typename... Args>
 static inline void sah_launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                     cudaStream_t st, Args&&... args) {

@@ -28,6 +28,7 @@
 #define HE_GROUPS 4
 #define HE_THREADS (HE_GT * HE_GROUPS)
 #define HE_MAXD 128     // widest layer
+#define HE_SMEM (227 * 1024)  // shared memory of a CTA at most
 #define HE_PITCH 36     // floats per activation channel: lanes that write neighbouring channels
                         // four vectors at a time hit different banks
 
@@ -404,7 +405,7 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
       const int wbytes = n_layers * HE_MAXD * HE_MAXD * (int)sizeof(T);
       if (wbytes > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(hash_encode_small_kernel<T>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, wbytes);
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "hash_encode attr: %s", cudaGetErrorString(e));
       }
       for (int l = 0; l < n_layers; ++l)
@@ -449,12 +450,9 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
     a.act_table = act_table;
     a.codes = codes;
     const int tc_smem = 1024 + off;
-    static int tc_allowed = 0;
-    if (tc_smem > tc_allowed) {
-      cudaError_t e = cudaFuncSetAttribute(hash_encode_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem);
-      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "hash_encode_tc attr: %s", cudaGetErrorString(e));
-      tc_allowed = tc_smem;
-    }
+    static bool tc_allowed[64] = {};
+    const cudaError_t e = sah_allow_smem(hash_encode_tc_kernel, HE_SMEM, tc_allowed);
+    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "hash_encode_tc attr: %s", cudaGetErrorString(e));
     // about two CTAs per SM in all, each with a contiguous slice of the key tiles
     const int64_t n_tiles = sah_ceil_div(n_end - n_begin, (int64_t)HTC_TILE);
     int64_t slices = sah_ceil_div((int64_t)2 * 148, (int64_t)H_out * B);
@@ -476,7 +474,7 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
     w_max = w > w_max ? w : w_max;
   }
   const size_t act_bytes = (size_t)HE_GROUPS * HE_MAXD * HE_PITCH * sizeof(float);
-  p.resident = act_bytes + w_all <= 227 * 1024 ? 1 : 0;
+  p.resident = act_bytes + w_all <= HE_SMEM ? 1 : 0;
   const size_t smem = act_bytes + (p.resident ? w_all : w_max);
   p.tiles_per_head = sah_ceil_div(n_end - n_begin, (int64_t)HE_TK);
   p.tiles = p.tiles_per_head * H_out * B;
@@ -485,7 +483,7 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
   sah_prof_begin(SAH_PROF_HASH_ENCODE, (cudaStream_t)stream);
   SAH_DISPATCH_DTYPE(dtype, T, {
     cudaError_t e = cudaFuncSetAttribute(hash_encode_kernel<T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, HE_SMEM);
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "hash_encode attr: %s", cudaGetErrorString(e));
     hash_encode_kernel<T><<<grid, HE_THREADS, smem, st>>>(p);
   });

@@ -156,6 +156,8 @@ __device__ __forceinline__ float lsh_augment(float nk, float M) {
 // copy requested before the first is waited for (no wait in here).
 #define LSH_COLS 64
 #define LSH_COLS_THREADS 128
+// the hyperplanes, a row of head dim + 1 and the signs: at most, for head dim 256
+#define LSH_COLS_SMEM(T) (257 * (LSH_COLS * (int)sizeof(T) + 4) + LSH_COLS)
 template <typename T>
 __device__ __forceinline__ void lsh_stage_columns(const T* __restrict__ proj, int nbits, int Dp, int c0, int nc,
                                                   T* __restrict__ sm) {
@@ -334,7 +336,7 @@ extern "C" int sah_lsh_key_sign(const void* keys, int dtype, int64_t ks_b, int64
     const int bytes = (D + 1) * (LSH_COLS * (int)sizeof(T) + 4) + LSH_COLS;                        \
     if (bytes > 48 * 1024) {                                                                       \
       cudaError_t e = cudaFuncSetAttribute(lsh_key_sign_few_kernel<T, CodeT>,                      \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);    \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, LSH_COLS_SMEM(T)); \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign attr: %s", cudaGetErrorString(e)); \
     }                                                                                              \
     sah_launch_chain(lsh_key_sign_few_kernel<T, CodeT>, fgrid, LSH_COLS_THREADS, bytes, st, \
@@ -352,7 +354,7 @@ extern "C" int sah_lsh_key_sign(const void* keys, int dtype, int64_t ks_b, int64
 #define LSH_SIGN_LAUNCH(T, CodeT)                                                                  \
   do {                                                                                             \
     cudaError_t e = cudaFuncSetAttribute(lsh_key_sign_kernel<T, CodeT>,                            \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign attr: %s", cudaGetErrorString(e)); \
     sah_launch_chain(lsh_key_sign_kernel<T, CodeT>, grid, 256, smem, st, \
         reinterpret_cast<const T*>(keys), ks_b, ks_h, ks_s, Hkv, s0, s1, D,                        \
@@ -402,14 +404,11 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
                                  : (1ll << 30));
   cudaError_t e = cudaMemsetAsync(status, 0, 16, st);
   if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign_tc memset: %s", cudaGetErrorString(e));
-  static bool allowed = false;
-  if (!allowed) {
-    e = cudaFuncSetAttribute(lsh_key_sign_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LtcCfg::SMEM);
-    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign_tc attr: %s", cudaGetErrorString(e));
-    e = cudaFuncSetAttribute(lsh_sign_recheck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LTC_RC_SMEM);
-    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_sign_recheck attr: %s", cudaGetErrorString(e));
-    allowed = true;
-  }
+  static bool allowed[2][64] = {};
+  e = sah_allow_smem(lsh_key_sign_tc_kernel, LtcCfg::SMEM, allowed[0]);
+  if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign_tc attr: %s", cudaGetErrorString(e));
+  e = sah_allow_smem(lsh_sign_recheck_kernel, LTC_RC_SMEM, allowed[1]);
+  if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_sign_recheck attr: %s", cudaGetErrorString(e));
   if (sm_count <= 0) sm_count = 148;
   // chunks of equal width: every CTA transforms as many keys and reads as many columns
   int chunks = (L * 8 + LTC_NCHUNK - 1) / LTC_NCHUNK;
@@ -541,7 +540,7 @@ extern "C" int sah_lsh_query(const void* q, int dtype, int64_t qs_b, int64_t qs_
     const int bytes = (D + 1) * LSH_COLS * (int)sizeof(T) + D * 4 + LSH_COLS;                      \
     if (bytes > 48 * 1024) {                                                                       \
       cudaError_t e = cudaFuncSetAttribute(lsh_query_kernel<T, CodeT>,                             \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);    \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, LSH_COLS_SMEM(T)); \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_query attr: %s", cudaGetErrorString(e)); \
     }                                                                                              \
     sah_launch_chain(lsh_query_kernel<T, CodeT>, grid, LSH_COLS_THREADS, bytes, st, \

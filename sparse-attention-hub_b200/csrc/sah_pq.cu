@@ -197,9 +197,9 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
   const cudaStream_t st = (cudaStream_t)stream;
 #define PTC_LAUNCH(NS, NB)                                                                                       \
   do {                                                                                                           \
-    static const cudaError_t allowed = cudaFuncSetAttribute(                                                     \
-        pq_assign_tc_kernel<NS, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, PtcCfg<NS>::SMEM);             \
-    if (allowed != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_assign_tc attr: %s", cudaGetErrorString(allowed)); \
+    static bool allowed[64] = {};                                                                                \
+    const cudaError_t e = sah_allow_smem(pq_assign_tc_kernel<NS, NB>, PtcCfg<NS>::SMEM, allowed);                \
+    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_assign_tc attr: %s", cudaGetErrorString(e));         \
     pq_assign_tc_kernel<NS, NB><<<grid, PTC_THREADS, PtcCfg<NS>::SMEM, st>>>(                                    \
         reinterpret_cast<const __nv_bfloat16*>(x), xs_b, xs_h, xs_s, Hkv, key_begin, key_end, init_offset,       \
         n_sub, n_cent, n_blocks, centroids, codes, cap, errflag);                                                \
@@ -436,6 +436,7 @@ extern "C" int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_
 // with an fp32 accumulator, pq_top_k.py:481-488).
 // ---------------------------------------------------------------------------
 #define PQ_ROWS 4
+#define PQ_SCORES_SMEM (200 * 1024)  // tables and queries of a CTA
 
 // One CTA: builds the table of one (KV group, block of 4 rows) in shared memory --
 // lut[sub][c][rr] = q_sub(row rblk*4 + rr) . centroid(sub, c), fma over ascending dims, rounded
@@ -611,7 +612,7 @@ extern "C" int sah_pq_scores(const void* q, int dtype, int64_t qs_b, int64_t qs_
   const int rblocks = (R + PQ_ROWS - 1) / PQ_ROWS;
   const size_t esz = (dtype == SAH_BF16) ? 8 : 16;  // one table entry: the four rows of a centroid
   const size_t smem = pq_table_bytes(esz, n_sub, n_cent) + (size_t)PQ_ROWS * n_sub * sub_d * sizeof(float);
-  if (smem > 200 * 1024)
+  if (smem > PQ_SCORES_SMEM)
     return sah_fail(SAH_ERR_UNSUPPORTED, "pq_scores: %d x %d lookup table does not fit", n_sub, n_cent);
   SAH_REQUIRE(rblocks <= 65535 && (int64_t)B * Hkv <= 65535, "pq_scores: too many rows per launch");
   cudaStream_t st = (cudaStream_t)stream;
@@ -626,14 +627,12 @@ extern "C" int sah_pq_scores(const void* q, int dtype, int64_t qs_b, int64_t qs_
   dim3 grid((unsigned)sah_ceil_div(n_keys, keys_per_cta), (unsigned)rblocks, (unsigned)((int64_t)B * Hkv));
   const int64_t tsz = (dtype == SAH_BF16) ? 2 : 4;
   const bool vecc = (sub_d * tsz) % 16 == 0 && (reinterpret_cast<uintptr_t>(centroids) & 15) == 0;
-  static int smem_allowed[4] = {0, 0, 0, 0};  // largest dynamic shared memory granted per instantiation
+  static bool allowed[4][64] = {};
 #define PQ_SCORES_LAUNCH(T, VEC, SLOT)                                                                    \
   do {                                                                                                    \
-    if ((int)smem > 48 * 1024 && (int)smem > smem_allowed[SLOT]) {                                        \
-      cudaError_t e = cudaFuncSetAttribute(pq_scores_kernel<T, VEC>,                                      \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+    if ((int)smem > 48 * 1024) {                                                                          \
+      const cudaError_t e = sah_allow_smem(pq_scores_kernel<T, VEC>, PQ_SCORES_SMEM, allowed[SLOT]);      \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_scores attr: %s", cudaGetErrorString(e));   \
-      smem_allowed[SLOT] = (int)smem;                                                                     \
     }                                                                                                     \
     sah_launch_chain(pq_scores_kernel<T, VEC>, grid, PQ_TILE, smem, st, (const T*)q, qs_b, qs_h, qs_q, (const T*)centroids, \
                                                           codes, cap, Hq, Hkv, Sq, n_keys, init_offset, S, \

@@ -237,7 +237,7 @@ extern "C" int sah_quest_scores(const void* q, int dtype, int64_t qs_b, int64_t 
   SAH_DISPATCH_DTYPE(dtype, T, {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(quest_scores_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+                                           160 * 1024);  // 139 KB: 32 pages of 512 float32 channels
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "quest_scores attr: %s", cudaGetErrorString(e));
     }
     sah_launch_chain(quest_scores_kernel<T>, grid, dim3((unsigned)pages, QS_ROWS), smem, (cudaStream_t)stream, (const T*)q, qs_b,

@@ -331,13 +331,14 @@ extern "C" int sah_adaptive_budget(const void* scores, int dtype, float scaling,
     if (sizeof(T) == 2 && row_bytes <= AD_ROW_BYTES) {
       const size_t bytes = (size_t)(W + 3) / 4 * 16 + row_bytes;
       cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, sizeof(T) == 2>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           AD_ROW_BYTES / 16 + AD_ROW_BYTES);
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e));
       sah_launch_chain(adaptive_budget_kernel<T, sizeof(T) == 2>, (unsigned)rows, 1024, bytes, st, a);
     } else {
       if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e));
       }
       sah_launch_chain(adaptive_budget_kernel<T, false>, (unsigned)rows, 1024, smem, st, a);

@@ -197,7 +197,7 @@ extern "C" int sah_qk_scores(const void* q, const void* k, int dtype, int64_t qs
   do {                                                                                              \
     if (smem > 48 * 1024) {                                                                         \
       cudaError_t e = cudaFuncSetAttribute(qk_scores_kernel<T, DT, F4, KEYS>,                       \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "qk_scores attr: %s", cudaGetErrorString(e)); \
     }                                                                                               \
     sah_launch_chain(qk_scores_kernel<T, DT, F4, KEYS>, grid, QK_THREADS, smem, st, \

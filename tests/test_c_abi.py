@@ -114,3 +114,21 @@ def test_every_chained_launch_names_a_kernel_that_waits_for_its_predecessors():
         assert body.lstrip().startswith(("sah_pdl_entry();", "sah_pdl_entry_early();")), name
     # and nothing else sets the attribute
     assert text.count("cudaLaunchAttributeProgrammaticStreamSerialization") == 1
+
+
+def test_shared_memory_limits_belong_to_a_device_and_do_not_vary():
+    """A kernel's limit on dynamic shared memory holds for one device, and the last call that sets it
+    wins.  Read from the sources: what has been granted is remembered per device or not at all,
+    and every kernel asks for one constant, so that neither a second GPU of the process nor a second
+    host thread finds the limit of another call."""
+    csrc = HEADER.parent.parent / "sparse-attention-hub_b200" / "csrc"
+    text = "\n".join(p.read_text() for p in sorted(csrc.glob("*.cu*"))).replace("\\\n", "\n")
+    assert not re.findall(r"static const cudaError_t", text)
+    flags = re.findall(r"static (?:bool|int) (\w*allowed\w*)((?:\[\w+\])*)", text)
+    assert flags and all(dims.endswith("[64]") for _, dims in flags), flags
+    sizes = re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\);", text)
+    sizes.remove("smem")  # sah_allow_smem's own parameter
+    sizes.remove("(int)smem")  # the float32 attention kernel, whose size follows its query block alone
+    assert len(sizes) >= 10
+    for size in sizes:
+        assert not re.search(r"\b[a-z]\w*\b", re.sub(r"\bsizeof\b|\bint\b", "", size)), size
