@@ -8,7 +8,10 @@
 // Encode.  A persistent CTA hashes tiles of HE_TK vectors; its tiles are a contiguous range of
 // the (batch, output head, tile) list, so that a head's weights (fp32, every layer) are staged
 // once and stay in shared memory while the head lasts, and every SM gets the same share of the
-// list.  Four groups of two warps each take a tile at a time, with barriers of their own, so that
+// list, cut between units of HE_GROUPS tiles of one head, or of two tiles or one as long as every
+// unit has an SM to itself: staging takes about 10 us, and a tile alone on an SM 12 us less than
+// four (cut anywhere, with four tiles per CTA, the heads of a short range shared CTAs in turn: 97 us
+// for 32 heads x 17 to 32 vectors, 26 us now; 64 to 256 vectors 38 to 59 us, 26 us now).  Four groups of two warps each take a tile at a time, with barriers of their own, so that
 // one group's rounding, activation look-ups and stores run under another's multiply-adds.
 // Activations are fp32 [channel][vector] and overwritten layer by layer.
 //
@@ -44,7 +47,7 @@ struct HashEncodeArgs {
   int act;
   const uint16_t* act_table;
   uint32_t* codes;
-  int64_t tiles_per_head, tiles;  // the tiled kernel's list
+  int tiles_per_head, unit, units_per_head, units;  // the tiled kernel's list
   int resident;                   // every layer's weights fit beside the activations
 };
 
@@ -174,7 +177,12 @@ hash_encode_kernel(HashEncodeArgs p) {
   float* act = reinterpret_cast<float*>(he_smem) + grp * HE_MAXD * HE_PITCH;  // [HE_MAXD][HE_PITCH] per group
   float* w_sm = reinterpret_cast<float*>(he_smem) + HE_GROUPS * HE_MAXD * HE_PITCH;
   const int D = p.dims[0], cpr = D / 8;
-  const int64_t t_first = p.tiles * blockIdx.x / gridDim.x, t_last = p.tiles * (blockIdx.x + 1) / gridDim.x;
+  auto unit_tile = [&](int u) {  // first tile of a unit
+    const int bh = u / p.units_per_head;
+    return bh * p.tiles_per_head + (u - bh * p.units_per_head) * p.unit;
+  };
+  const int t_first = unit_tile((int)((int64_t)p.units * blockIdx.x / gridDim.x));
+  const int t_last = unit_tile((int)((int64_t)p.units * (blockIdx.x + 1) / gridDim.x));
 
   auto stage_weights = [&](int l, int h, float* dst) {
     const int din = p.dims[l], dout = p.dims[l + 1];
@@ -188,14 +196,15 @@ hash_encode_kernel(HashEncodeArgs p) {
   // of the tile before is computed.
   constexpr int FETCH = HE_TK * HE_MAXD / 8 / HE_GT;
   uint4 raw[FETCH];
-  auto row_of = [&](int64_t t) -> const T* {
-    const int64_t bh = t / p.tiles_per_head;
-    const int64_t n = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK + gt % HE_TK;
+  const int G = p.H_out / p.H_in;
+  auto row_of = [&](int t) -> const T* {
+    const int bh = t / p.tiles_per_head;
+    const int64_t n = p.n_begin + (int64_t)(t - bh * p.tiles_per_head) * HE_TK + gt % HE_TK;
     if (t >= t_last || n >= p.n_end) return nullptr;
-    const int h = (int)(bh % p.H_out);
-    return reinterpret_cast<const T*>(p.x) + bh / p.H_out * p.xs_b + h / (p.H_out / p.H_in) * p.xs_h + n * p.xs_n;
+    const int b = bh / p.H_out, h = bh - b * p.H_out;
+    return reinterpret_cast<const T*>(p.x) + b * p.xs_b + h / G * p.xs_h + n * p.xs_n;
   };
-  auto fetch = [&](int64_t t) {
+  auto fetch = [&](int t) {
     const T* row = row_of(t);
 #pragma unroll
     for (int f = 0; f < FETCH; ++f) {
@@ -206,12 +215,12 @@ hash_encode_kernel(HashEncodeArgs p) {
   };
 
   // the range head by head; within a head group g takes the tiles g, g + HE_GROUPS, ...
-  for (int64_t t0 = t_first; t0 < t_last;) {
-    const int64_t bh = t0 / p.tiles_per_head;
-    const int h = (int)(bh % p.H_out);
-    int64_t t1 = (bh + 1) * p.tiles_per_head;
+  for (int t0 = t_first; t0 < t_last;) {
+    const int bh = t0 / p.tiles_per_head;
+    const int h = bh % p.H_out;
+    int t1 = (bh + 1) * p.tiles_per_head;
     if (t1 > t_last) t1 = t_last;
-    int64_t t = t0 + grp;
+    int t = t0 + grp;
     if (sizeof(T) == 2) fetch(t < t1 ? t : t_last);  // zeros where the group has no tile
     if (p.resident) {
       __syncthreads();  // the weights of the head before are done with
@@ -224,9 +233,9 @@ hash_encode_kernel(HashEncodeArgs p) {
     }
     // weights that are staged layer by layer keep the groups together: all of them go round
     // equally often, with nothing to write where a group has no tile left
-    const int64_t rounds = p.resident ? (t < t1 ? (t1 - t + HE_GROUPS - 1) / HE_GROUPS : 0)
-                                      : (t1 - t0 + HE_GROUPS - 1) / HE_GROUPS;
-    for (int64_t round = 0; round < rounds; ++round, t += HE_GROUPS) {
+    const int rounds = p.resident ? (t < t1 ? (t1 - t + HE_GROUPS - 1) / HE_GROUPS : 0)
+                                  : (t1 - t0 + HE_GROUPS - 1) / HE_GROUPS;
+    for (int round = 0; round < rounds; ++round, t += HE_GROUPS) {
       {  // (the last layer's barrier stands between the reads of the tile before and these writes)
         const T* row = sizeof(T) == 2 ? nullptr : (t < t1 ? row_of(t) : nullptr);
 #pragma unroll
@@ -242,7 +251,7 @@ hash_encode_kernel(HashEncodeArgs p) {
         }
       }
       const float* w_l = w_sm;
-      const int64_t n0 = p.n_begin + (t - bh * p.tiles_per_head) * HE_TK;
+      const int64_t n0 = p.n_begin + (int64_t)(t - bh * p.tiles_per_head) * HE_TK;
       uint32_t* codes = p.codes + bh * p.n_total + n0;
       const int nvalid = t >= t1 ? 0 : (int)(p.n_end - n0 < HE_TK ? p.n_end - n0 : HE_TK);
       for (int l = 0; l < p.n_layers; ++l) {
@@ -476,10 +485,14 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
   const size_t act_bytes = (size_t)HE_GROUPS * HE_MAXD * HE_PITCH * sizeof(float);
   p.resident = act_bytes + w_all <= HE_SMEM ? 1 : 0;
   const size_t smem = act_bytes + (p.resident ? w_all : w_max);
-  p.tiles_per_head = sah_ceil_div(n_end - n_begin, (int64_t)HE_TK);
-  p.tiles = p.tiles_per_head * H_out * B;
-  const int64_t ctas = sah_ceil_div(p.tiles, (int64_t)HE_GROUPS);
-  const unsigned grid = (unsigned)(ctas < 148 ? ctas : 148);
+  const int64_t tiles_per_head = sah_ceil_div(n_end - n_begin, (int64_t)HE_TK), heads = (int64_t)H_out * B;
+  SAH_REQUIRE(tiles_per_head * heads < (1ll << 31), "hash_encode: too many vectors");
+  p.unit = 1;
+  while (p.unit < HE_GROUPS && sah_ceil_div(tiles_per_head, (int64_t)p.unit) * heads > 148) p.unit *= 2;
+  p.tiles_per_head = (int)tiles_per_head;
+  p.units_per_head = (int)sah_ceil_div(tiles_per_head, (int64_t)p.unit);
+  p.units = (int)(p.units_per_head * heads);
+  const unsigned grid = (unsigned)(p.units < 148 ? p.units : 148);
   sah_prof_begin(SAH_PROF_HASH_ENCODE, (cudaStream_t)stream);
   SAH_DISPATCH_DTYPE(dtype, T, {
     cudaError_t e = cudaFuncSetAttribute(hash_encode_kernel<T>,

@@ -464,11 +464,14 @@ def test_hash_signatures_from_tensor_cores_equal_the_fixed_order_kernel(hidden, 
     ("bf16", (128, 128, 128, 32), 0, 17, "silu"), ("bf16", (128, 128, 128, 32), 5, 128, "silu"),
     ("bf16", (64, 32, 16), 3, 129, "relu"), ("bf16", (72, 16, 64, 128, 32), 0, 300, "tanh"),
     ("bf16", (128, 128, 128, 128, 32), 0, 257, "gelu"), ("bf16", (128, 128, 128, 32), 0, 12000, "silu"),
-    ("f32", (128, 128, 128, 32), 1, 255, "silu"), ("f32", (8, 16), 0, 130, "relu")])
+    ("f32", (128, 128, 128, 32), 1, 255, "silu"), ("f32", (8, 16), 0, 130, "relu"),
+    ("bf16", (128, 128, 128, 32), 2, 592, "silu"), ("bf16", (128, 128, 128, 32), 0, 593, "silu"),
+    ("bf16", (128, 128, 128, 128, 32), 3, 700, "relu"), ("bf16", (128, 128, 128, 32), 0, 1153, "silu"),
+    ("f32", (64, 32, 16), 0, 1186, "tanh")])
 def test_hash_signatures_of_tiles_equal_those_of_single_vectors(dtype, widths, n0, n, act):
-    """Ranges of more than 16 vectors go through tiles of 128 (weights of all layers resident in
-    shared memory, or layer by layer where they do not fit; several heads per CTA), shorter ones
-    one vector per CTA.  Both walk the channels in the same order: the same words, and words
+    """Ranges of more than 16 vectors go through tiles of 32 (weights of all layers resident in
+    shared memory, or layer by layer where they do not fit; one, two or four tiles of a head as the
+    unit that CTAs share, and several units per CTA), shorter ones one vector per CTA.  Both walk the channels in the same order: the same words, and words
     outside the range untouched."""
     torch.manual_seed(sum(widths) + n)
     B, Hkv, Hq, S = 2, 2, 4, n0 + n + 3
