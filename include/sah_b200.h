@@ -242,11 +242,12 @@ int sah_topk_select_fill_bands(const void* scores, int dtype, int64_t rows, int 
                                int64_t W, int64_t col_begin, int64_t col_end, int n_bands,
                                const int64_t* bands, uint32_t* prev_bits, int64_t k,
                                uint32_t* out_bits, void* stream);
-/* 1 when the keys of such rows fit in the shared memory of the cluster of CTAs that
- * sah_topk_select gives a row to (then it is the faster form), else 0. */
+/* Which form is the faster one for such rows: 2, sah_topk_select (the keys of a row fit in the shared
+ * memory of its cluster of CTAs); 1, sah_topk_select_bands where it saves filling a bitmap, else
+ * sah_topk_select_ws; 0, sah_topk_select_ws. */
 int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W);
-/* The same selection for rows that do not fit: every row spread over the whole grid
- * (calls sah_topk_select for rows that do).
+/* The same selection with every row spread over the whole grid (calls sah_topk_select where that
+ * is the faster form).
  * Needs a 16-byte aligned device workspace of sah_topk_select_ws_bytes(rows, W)
  * bytes (SAH_ERR_WORKSPACE when smaller); rows <= 65535.  out_bits may alias
  * prev_bits.  Same result as sah_topk_select, bit for bit. */

@@ -256,6 +256,11 @@ __device__ __forceinline__ void sah_pdl_entry_early() {
 // (SAH_PDL_MAX_WARPS replaces the 1024); 0 = no chaining at all, the default.
 int sah_pdl_max_warps();
 
+// CTAs of one wave when clusters of `ranks` of them, one CTA per SM, have to find their SMs in one
+// GPC each.  148 SMs hold 15 clusters of eight and 35 of four (16 and 36 rows took twice the time of
+// 15 and 35); one fewer is counted on, since the SMs of a GPC differ from device to device.
+static inline int sah_cluster_wave(int ranks) { return ranks <= 2 ? 148 : ranks == 4 ? 136 : 112; }
+
 // Leave to launch `kernel` with up to `smem` bytes of dynamic shared memory on the current device.
 // The limit belongs to a device, so it is noted for each; a refusal is not.  `smem` is one constant
 // per kernel, so that threads that get here together cannot leave a smaller limit behind.

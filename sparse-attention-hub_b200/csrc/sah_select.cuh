@@ -18,16 +18,19 @@
 // instruction issue (the passes make about 20 instructions per 16-bit key) and, for short rows,
 // by the barriers.  128 rows x 65536 bfloat16 scores: 35.2 us as three launches with a grid-wide
 // histogram each, 45.6 us with the keys converted in every pass, 27.6 us now (32 rows x 8191: 23.5 us before, 10.7 us now).
+// Rows of up to 2048 columns (page scores) take digits of 8 bits and CTAs of 64 to 256 threads: 32
+// rows x 512 bfloat16 scores 7.0 us with the wide digits, 5.9 us this way.
 #pragma once
 
 #include "sah_common.cuh"
 #include <cooperative_groups.h>
 
 #define SAH_SELECT_THREADS 1024
-#define SAH_SELECT_MIN_THREADS 512  // four counters of a digit each
-#define SAH_SELECT_BINS 2048
+#define SAH_SELECT_PER 4             // counters of a digit per thread: at least 512 threads of 2048 ...
+#define SAH_SELECT_SHORT_BYTES 256   // ... and 64 of 256, for rows of up to 2048 columns
 #define SAH_SELECT_MAX_CLUSTER 8
 #define SAH_SELECT_KEY_BYTES (160 * 1024)  // keys of a CTA's columns in shared memory
+#define SAH_SELECT_HALF_BYTES (90 * 1024)  // two such CTAs share an SM
 
 // Keep the lowest n set bits of m.
 __device__ __forceinline__ uint32_t sah_lowest_bits(uint32_t m, int n) {
@@ -108,8 +111,9 @@ struct SahScoreKeys<float, 32> {
   }
 };
 
-template <int KEYBITS, typename Keys, bool RESIDENT>
-__global__ void __launch_bounds__(SAH_SELECT_THREADS)
+// SHORT: digits of 8 bits, whose 256 counters a small CTA clears and scans in no time
+template <int KEYBITS, typename Keys, bool RESIDENT, bool SHORT>
+__global__ void __launch_bounds__(SHORT ? SAH_SELECT_SHORT_BYTES : SAH_SELECT_THREADS)
 sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __grid_constant__ MaskBands bands, int Sq,
                   uint32_t* __restrict__ band_bits, uint32_t* __restrict__ out_bits, int64_t S, int64_t W, int64_t col_begin, int64_t col_end,
                   long long k) {
@@ -117,9 +121,10 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   constexpr int NW = KEYBITS == 16 ? 4 : 8;  // words of eight keys
+  constexpr int DIGIT = SHORT ? 8 : 11, DIGITS = (KEYBITS + DIGIT - 1) / DIGIT, BINS = 1 << DIGIT;
   extern __shared__ __align__(16) unsigned char sel_smem[];
   uint4* store = reinterpret_cast<uint4*>(sel_smem);  // [NW / 4][bytes of this CTA]
-  __shared__ unsigned int hist[2][SAH_SELECT_BINS];  // alternate digits: a CTA may count the next
+  __shared__ unsigned int hist[2][BINS];  // alternate digits: a CTA may count the next
                                                      // one while others still read this one
   __shared__ unsigned int scan[33];
   __shared__ unsigned int prefix_sm;
@@ -218,12 +223,10 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
   int mode = k <= 0 ? 2 : 0;
   unsigned int ties = 0u;   // keys equal to the threshold in the whole row
   unsigned int lower = 0u;  // and in the CTAs in front of this one
-  constexpr int DIGITS = KEYBITS == 16 ? 2 : 3;
 #pragma unroll
   for (int d = 0; d < DIGITS; ++d) {
-    constexpr int LAST = KEYBITS == 16 ? 5 : 10;
-    const int bits = d == DIGITS - 1 ? LAST : 11;
-    const int shift = d == DIGITS - 1 ? 0 : KEYBITS - 11 * (d + 1);
+    const int bits = d == DIGITS - 1 ? KEYBITS - DIGIT * (DIGITS - 1) : DIGIT;
+    const int shift = d == DIGITS - 1 ? 0 : KEYBITS - DIGIT * (d + 1);
     const int nbins = 1 << bits;
     unsigned int* h = hist[d & 1];
     if (mode == 0) {  // the same in the whole cluster
@@ -290,7 +293,7 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
       if (ranks > 1) cluster.sync(); else __syncthreads();
       // thread t owns PER neighbouring bins, the highest first; all reads are on their way before
       // the first is added
-      constexpr int PER = SAH_SELECT_BINS / SAH_SELECT_MIN_THREADS;
+      constexpr int PER = SAH_SELECT_PER;
       unsigned int cnt[PER], mine = 0u;
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
@@ -414,13 +417,15 @@ sah_select_kernel(Keys keys, const uint32_t* __restrict__ prev_bits, const __gri
   if (ranks > 1) cluster.sync();  // nobody leaves while its counters may be read
 }
 
-// CTAs per row: a power of two, as long as one wave of 148 holds all of them and each keeps 8192
+// CTAs per row: a power of two, as long as one wave holds all of them and each keeps 8192
 // columns, one byte of the bitmap per thread and pass (with 2048 columns per CTA 32 rows x 8191
 // bfloat16 scores took 20.4 us: the cluster barriers and the counters of the other CTAs cost more
 // than the passes)
 static inline int sah_select_ranks(int64_t rows, int64_t S) {
   int ranks = 1;
-  while (ranks < SAH_SELECT_MAX_CLUSTER && rows * ranks * 2 <= 148 && S >= (int64_t)ranks * 2 * 8192) ranks *= 2;
+  while (ranks < SAH_SELECT_MAX_CLUSTER && rows * ranks * 2 <= sah_cluster_wave(ranks * 2) &&
+         S >= (int64_t)ranks * 2 * 8192)
+    ranks *= 2;
   return ranks;
 }
 
@@ -436,11 +441,15 @@ static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits,
                                     cudaStream_t st, const MaskBands& bands = MaskBands(), int Sq = 1,
                                     uint32_t* band_bits = nullptr) {
   const int ranks = sah_select_ranks(rows, S);
-  // half-size CTAs for short rows and when rows queue for SMs
-  const int nt = W * 4 / ranks <= SAH_SELECT_MIN_THREADS || rows * ranks > 148 ? SAH_SELECT_MIN_THREADS
-                                                                                : SAH_SELECT_THREADS;
   const int64_t key_bytes = sah_select_key_bytes(rows, S, W, KEYBITS);
   const bool resident = key_bytes <= SAH_SELECT_KEY_BYTES;
+  const int64_t row_bytes = W * 4 / ranks;  // a thread looks at one at a time
+  const bool shrt = W * 4 <= SAH_SELECT_SHORT_BYTES;
+  // half-size CTAs for shorter rows, and when rows queue for SMs that hold two of them (256 rows x
+  // 65536 bfloat16 scores, of which an SM holds one: 59.0 us in half-size CTAs, 48.1 us in whole ones)
+  const bool two = rows * ranks > 148 && key_bytes <= SAH_SELECT_HALF_BYTES;
+  const int nt = shrt ? (row_bytes <= 64 ? 64 : row_bytes <= 128 ? 128 : 256)
+                      : row_bytes <= SAH_SELECT_THREADS / 2 || two ? SAH_SELECT_THREADS / 2 : SAH_SELECT_THREADS;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(rows * ranks));
   cfg.blockDim = dim3((unsigned)nt);
@@ -452,18 +461,22 @@ static inline int sah_select_launch(const Keys& keys, const uint32_t* prev_bits,
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (resident) {
+  cfg.numAttrs = ranks > 1 ? 1 : 0;
+  auto launch = [&](auto kernel) {
+    (void)cudaLaunchKernelEx(&cfg, kernel, keys, prev_bits, bands, Sq, band_bits, out_bits, S, W, col_begin, col_end,
+                             (long long)k);
+  };
+  if (shrt) {
+    launch(sah_select_kernel<KEYBITS, Keys, true, true>);
+  } else if (resident) {
     if (key_bytes > 24 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(sah_select_kernel<KEYBITS, Keys, true>,
+      const cudaError_t e = cudaFuncSetAttribute(sah_select_kernel<KEYBITS, Keys, true, false>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, SAH_SELECT_KEY_BYTES);
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "select attr: %s", cudaGetErrorString(e));
     }
-    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, true>, keys, prev_bits, bands, Sq,
-                             band_bits, out_bits, S, W, col_begin, col_end, (long long)k);
+    launch(sah_select_kernel<KEYBITS, Keys, true, false>);
   } else {
-    (void)cudaLaunchKernelEx(&cfg, sah_select_kernel<KEYBITS, Keys, false>, keys, prev_bits, bands, Sq,
-                             band_bits, out_bits, S, W, col_begin, col_end, (long long)k);
+    launch(sah_select_kernel<KEYBITS, Keys, false, false>);
   }
   return SAH_OK;  // a launch error stays for SAH_LAUNCH_CHECK
 }

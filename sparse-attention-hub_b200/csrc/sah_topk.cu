@@ -799,9 +799,30 @@ extern "C" int sah_topk_select_fill_bands(const void* scores, int dtype, int64_t
   return select_bands(scores, dtype, rows, Sq, S, W, col_begin, col_end, n_bands, bands, prev_bits, k, out_bits, stream);
 }
 
+// Which form is ahead, measured over 1 to 2048 rows of 512 to 262144 scores (us; cluster form against
+// the grid-wide one, which in bfloat16 is three launches and in float32 five):
+//   float32: the cluster form (32 rows x 65536 23 / 35, 256 x 24000 22 / 73) unless eight CTAs
+//     share a row (8 x 65536 31 / 28);
+//   bfloat16, eight or four CTAs per row: the grid-wide form (8 x 65536 21 / 13, 32 x 32768 16 / 13),
+//     but for some thirty long rows the cluster form, at first if it also saves the launch that fills
+//     a bitmap of bands (32 x 131072 23.2 / 24.0), then in any case (32 x 262144 32 / 37);
+//   two: they are even (1 to 74 rows x 16384 13.4 to 13.8 / 12.4 to 13.4, 48 x 65536 20 / 18), so the
+//     saved launch decides, until the rows fill the chip (64 x 81920 23 / 30, 48 x 131072 29 / 31);
+//   one: the cluster form (128 x 65536 26 / 34, 256 x 8192 12 / 15), but the grid-wide one where rows
+//     that fill an SM leave most of the last wave empty (149 x 65536 48 / 42) and for a thousand
+//     rows of 2049 to 8192 scores (2048 x 8192 67 / 61).
 extern "C" int sah_topk_select_fits(int dtype, int64_t rows, int64_t S, int64_t W) {
   if (rows <= 0 || S <= 0 || W * 32 < S) return 0;
-  return sah_select_key_bytes(rows, S, W, dtype == SAH_BF16 ? 16 : 32) <= SAH_SELECT_KEY_BYTES ? 1 : 0;
+  const int64_t key_bytes = sah_select_key_bytes(rows, S, W, dtype == SAH_BF16 ? 16 : 32);
+  if (key_bytes > SAH_SELECT_KEY_BYTES) return 0;
+  const int ranks = sah_select_ranks(rows, S);
+  if (dtype != SAH_BF16) return ranks == 8 ? 0 : 2;
+  if (ranks == 8) return 0;
+  if (ranks == 4) return rows * S >= 7000000 ? 2 : rows >= 28 && rows * S >= 2500000 ? 1 : 0;
+  if (ranks == 2) return (rows >= 60 && S >= 20000) || rows * S >= 6000000 ? 2 : 1;
+  const int64_t waves = sah_ceil_div(rows, 148);
+  if (key_bytes > SAH_SELECT_HALF_BYTES && rows > 148 && rows * 100 < waves * 148 * 62) return 0;
+  return rows >= 1024 && S > 2048 && S <= 8192 ? 0 : 2;
 }
 
 extern "C" int sah_topk_select_ws(const void* scores, int dtype, int64_t rows, int64_t S, int64_t W,
@@ -819,10 +840,7 @@ extern "C" int sah_topk_select_ws(const void* scores, int dtype, int64_t rows, i
   if (col_begin < 0) col_begin = 0;
   if (col_end > S) col_end = S;
   cudaStream_t st = (cudaStream_t)stream;
-  // One launch, a cluster per row, while the keys of a CTA's columns fit in its shared memory; the
-  // grid-wide form for longer rows (32 rows of a million keys: four CTAs per row would leave most
-  // of the chip idle).
-  if (sah_topk_select_fits(dtype, rows, S, W))
+  if (sah_topk_select_fits(dtype, rows, S, W) == 2)
     return sah_topk_select(scores, dtype, rows, S, W, col_begin, col_end, prev_bits, k, out_bits, stream);
   sah_prof_begin(SAH_PROF_TOPK_SELECT, st);
   int rc;

@@ -487,9 +487,11 @@ extern "C" int sah_topp_select(const void* scores, int dtype, float scaling, con
   const int64_t rows = (int64_t)B * Hq * Sq;
   SAH_REQUIRE(rows <= 2147483647, "topp_select: too many rows");
   // Few rows: several CTAs per row (a power of two, so that the bitmap bytes split evenly), as
-  // long as one wave of 148 holds them all and each still has a pass of 8 columns per thread.
+  // long as one wave holds them all and each still has a pass of 8 columns per thread.
   int ranks = 1;
-  while (ranks < TP_MAX_CLUSTER && rows * ranks * 2 <= 148 && S >= (int64_t)ranks * 2 * 8 * TP_THREADS) ranks *= 2;
+  while (ranks < TP_MAX_CLUSTER && rows * ranks * 2 <= sah_cluster_wave(ranks * 2) &&
+         S >= (int64_t)ranks * 2 * 8 * TP_THREADS)
+    ranks *= 2;
   sah_prof_begin(SAH_PROF_TOPP, (cudaStream_t)stream);
   const int64_t row_bytes = (W * 4 + ranks - 1) / ranks * 16;
   const bool resident = row_bytes <= TP_ROW_BYTES;

@@ -79,7 +79,7 @@ _SIGNATURES = {
     "sah_topk_select": [_P, _I, _L, _L, _L, _L, _L, _P, _L, _P, _P],
     "sah_topk_select_bands": [_P, _I, _L, _I, _L, _L, _L, _L, _I, _P, _L, _P, _P],
     "sah_topk_select_fill_bands": [_P, _I, _L, _I, _L, _L, _L, _L, _I, _P, _P, _L, _P, _P],
-    "sah_topk_select_fits": [_I, _L, _L, _L],  # returns 0 or 1
+    "sah_topk_select_fits": [_I, _L, _L, _L],  # returns 0, 1 or 2
     "sah_topk_select_ws_bytes": [_L, _L],  # returns int64
     "sah_topk_sel_hist_offset": [_L, _L],  # returns int64
     "sah_topk_sel_begin": [_L, _L, _L, _P, _L, _P],

@@ -65,8 +65,8 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
     """previous | top-k of `scores` over inactive columns in [col_begin, col_end).
 
     `per_row`: the one-launch form (a cluster of CTAs per row) whatever the row length; otherwise
-    rows whose keys do not fit in a cluster's shared memory are spread over the whole grid, with
-    histograms in a scratch buffer."""
+    rows for which the library counts it as the faster form (`sah_topk_select_fits`) are spread over
+    the whole grid, with histograms in a scratch buffer."""
     _native.require_cuda(scores, "scores")
     lib = _native.load()
     S = scores.shape[-1]
@@ -77,8 +77,8 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
     end = S if col_end is None else col_end
     dst = out if out is not None else NativeBits(
         torch.empty((prev.rows, prev.words), dtype=torch.int32, device=sc.device), rows, S)
-    fits = lib.sah_topk_select_fits(_native.dtype_code(sc.dtype), rows, S, prev.words)
-    bands = prev.pending_bands() if fits and prev.rows == rows and out is None else None
+    form = lib.sah_topk_select_fits(_native.dtype_code(sc.dtype), rows, S, prev.words)
+    bands = prev.pending_bands() if form and prev.rows == rows and out is None else None
     if bands is not None:
         # the previous mask is a sink and a window that nobody has needed as a bitmap so far; the
         # kernel fills its words on the way
@@ -88,7 +88,7 @@ def topk_select(scores: torch.Tensor, previous_mask: Mask, k: int, col_begin: in
                                            dst.bits.data_ptr(), st), "sah_topk_select_fill_bands")
         prev.bands_written()
         return dst
-    if rows <= 65535 and not per_row and not fits:
+    if rows <= 65535 and not per_row and form != 2:
         # rows are spread over many CTAs; the histograms live in a scratch buffer
         nbytes = int(lib.sah_topk_select_ws_bytes(rows, prev.words))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=sc.device)

@@ -66,6 +66,20 @@ def test_workspace_size_queries():
     assert sizes.groups == 64 and sizes.ucols_bytes > 0
 
 
+@pytest.mark.parametrize("dtype,rows,S,form", [
+    (1, 32, 512, 2), (1, 32, 8191, 2), (1, 32, 16384, 1), (1, 32, 32768, 0), (1, 8, 65536, 0), (1, 16, 65536, 0),
+    (1, 32, 131072, 1), (1, 32, 262144, 2), (1, 24, 131072, 0), (1, 48, 65536, 1), (1, 74, 98304, 2),
+    (1, 128, 65536, 2), (1, 149, 65536, 0), (1, 192, 65536, 2), (1, 256, 65536, 2),
+    (1, 160, 32768, 2), (1, 2048, 8192, 0), (1, 2048, 2048, 2), (1, 75, 98304, 0), (0, 32, 65536, 2),
+    (0, 8, 65536, 0), (0, 16, 131072, 2), (0, 256, 24000, 2), (0, 160, 49152, 0), (1, 0, 512, 0)])
+def test_form_of_the_selection(dtype, rows, S, form):
+    """The rule that spreads rows over clusters of CTAs (2), over the grid (0), or over clusters only
+    where that saves the launch that fills a bitmap of bands (1), at the points that it was
+    measured at."""
+    words = ((S + 31) // 32 + 3) // 4 * 4
+    assert _native.load().sah_topk_select_fits(dtype, rows, S, words) == form
+
+
 def test_plan_refuses_sizes_of_another_key_count():
     """The counter block is laid out by the key count: a plan call whose `sizes` came from a
     query for fewer keys (too few chunk counters) is refused before anything is launched, and
