@@ -64,11 +64,16 @@ extern "C" int sah_quest_page_minmax(const void* k, int dtype, int64_t ks_b, int
 // first is waited for.  Bound by that latency and by the rounded products, two per channel; in
 // bfloat16 they are made in pairs (the product of two bfloat16 numbers rounds once either way).
 // 256 rows x 512 pages x 128 channels: 14.2 us with every row reading the bounds for itself,
-// 8.0 us now.
+// 8.0 us now.  In float32, where a page's bounds are twice as long and there are no pairs, that gains
+// where a launch is short of warps (32 rows x 512 pages 5.9 us row by row, 4.3 us staged; 512
+// channels 16 and 9 us) and loses where it is not (256 x 512 11 and 15 us): from QS_DIRECT scores on
+// and up to 256 channels a thread reads the bounds of its page for its own row.
 #define QS_ROWS 4
 #define QS_PAGES 128            // pages per CTA; halved until the bounds fit
-#define QS_BOUND_BYTES (96 * 1024)
+#define QS_BOUND_BYTES(elt) ((elt) == 2 ? 96 * 1024 : 36 * 1024)
+#define QS_DIRECT (48 * 1024)
 #define QS_MAXD 512
+#define QS_SMEM (160 * 1024)    // 139 KB at most: 32 pages of 512 float32 channels
 
 template <typename T>
 struct QuestVec {  // elements one vector load of the reference's reduction brings
@@ -92,12 +97,17 @@ __device__ __forceinline__ void quest_max8(const __nv_bfloat16* q, const __nv_bf
   }
 }
 __device__ __forceinline__ void quest_max8(const float* q, const float* lo, const float* hi, float* out) {
+  float qf[8], a[8], c[8];
+  sah_load8<float>(q, qf);
+  sah_load8<float>(lo, a);
+  sah_load8<float>(hi, c);
 #pragma unroll
-  for (int l = 0; l < 8; ++l) out[l] = fmaxf(__fmul_rn(q[l], lo[l]), __fmul_rn(q[l], hi[l]));
+  for (int l = 0; l < 8; ++l) out[l] = fmaxf(__fmul_rn(qf[l], a[l]), __fmul_rn(qf[l], c[l]));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(QS_PAGES * QS_ROWS)
+// STAGED: bounds in shared memory, blockDim.y = QS_ROWS; else read where they lie, blockDim.y = 1
+template <typename T, bool STAGED>
+__global__ void __launch_bounds__(STAGED ? QS_PAGES * QS_ROWS : QS_PAGES)
 quest_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs_q,
                     const T* __restrict__ pmin, const T* __restrict__ pmax, int64_t P_cap, int Hq,
                     int Hkv, int Sq, int64_t S, int D, int page_size, const T* __restrict__ bias,
@@ -107,12 +117,12 @@ quest_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t
   const int NP = blockDim.x, chunks = D / 8;
   T* lo_sm = reinterpret_cast<T*>(qs_smem);                 // [chunks][NP][8]
   T* hi_sm = lo_sm + (size_t)chunks * NP * 8;
-  T* q_sm = hi_sm + (size_t)chunks * NP * 8;                // [QS_ROWS][D]
+  T* q_sm = STAGED ? hi_sm + (size_t)chunks * NP * 8 : lo_sm;  // [rows][D]
   const int G = Hq / Hkv, R = G * Sq;                       // rows that share a KV head
   const int64_t bk = blockIdx.z;                            // b * Hkv + kvh
   const int kvh = (int)(bk % Hkv);
   const int64_t b = bk / Hkv;
-  const int r = blockIdx.y * QS_ROWS + threadIdx.y;         // row r = g * Sq + qi of the KV head
+  const int r = blockIdx.y * blockDim.y + threadIdx.y;      // row r = g * Sq + qi of the KV head
   const int64_t P = (S + page_size - 1) / page_size;
   const int64_t page0 = (int64_t)blockIdx.x * NP;
   const int np = (int)(P - page0 < NP ? P - page0 : NP);
@@ -121,7 +131,7 @@ quest_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t
   constexpr int PIECES = 8 * (int)sizeof(T) / 16;           // 16-byte pieces of a chunk
   const T* lo_g = pmin + bk * (int64_t)D * P_cap + page0 * 8;
   const T* hi_g = pmax + bk * (int64_t)D * P_cap + page0 * 8;
-  for (int i = tid; i < chunks * NP * PIECES; i += nt) {
+  for (int i = tid; STAGED && i < chunks * NP * PIECES; i += nt) {
     const int c = i / (NP * PIECES), x = i - c * (NP * PIECES);  // piece x of the chunk's row of pages
     if (x < np * PIECES) {
       const int64_t src = c * P_cap * 8 + (int64_t)x * (8 / PIECES);
@@ -143,10 +153,10 @@ quest_scores_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t
   const int64_t page = page0 + threadIdx.x;
   if (r >= R || page >= P) return;
   const int64_t row = (b * Hq + h) * Sq + qi;
-  const T* lo = lo_sm + threadIdx.x * 8;
-  const T* hi = hi_sm + threadIdx.x * 8;
+  const T* lo = (STAGED ? lo_sm : lo_g) + threadIdx.x * 8;
+  const T* hi = (STAGED ? hi_sm : hi_g) + threadIdx.x * 8;
   const T* qs = q_sm + threadIdx.y * D;
-  const int cstride = NP * 8;
+  const int64_t cstride = STAGED ? NP * 8 : P_cap * 8;
 
   constexpr int VEC = QuestVec<T>::N;
   const int nv = D / VEC;
@@ -229,21 +239,30 @@ extern "C" int sah_quest_scores(const void* q, int dtype, int64_t qs_b, int64_t 
   SAH_REQUIRE(rows <= 65535, "quest_scores: more than 65535 mask rows");
   const int64_t elt = dtype == SAH_BF16 ? 2 : 4;
   int pages = QS_PAGES;
-  while (pages > 32 && (2 * pages * D * elt > QS_BOUND_BYTES || P <= pages / 2)) pages /= 2;
-  const size_t smem = (size_t)(2 * pages + QS_ROWS) * D * elt;
-  dim3 grid((unsigned)sah_ceil_div(P, pages), (unsigned)sah_ceil_div((int64_t)(Hq / Hkv) * Sq, QS_ROWS),
+  const bool direct = dtype != SAH_BF16 && rows * P >= QS_DIRECT && D <= 256;
+  while (!direct && pages > 32 && (2 * pages * D * elt > QS_BOUND_BYTES(elt) || P <= pages / 2)) pages /= 2;
+  const int qrows = direct ? 1 : QS_ROWS;
+  const size_t smem = (size_t)((direct ? 0 : 2 * pages) + qrows) * D * elt;
+  dim3 grid((unsigned)sah_ceil_div(P, pages), (unsigned)sah_ceil_div((int64_t)(Hq / Hkv) * Sq, qrows),
             (unsigned)((int64_t)B * Hkv));
   sah_prof_begin(SAH_PROF_QUEST, (cudaStream_t)stream);
-  SAH_DISPATCH_DTYPE(dtype, T, {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(quest_scores_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           160 * 1024);  // 139 KB: 32 pages of 512 float32 channels
-      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "quest_scores attr: %s", cudaGetErrorString(e));
-    }
-    sah_launch_chain(quest_scores_kernel<T>, grid, dim3((unsigned)pages, QS_ROWS), smem, (cudaStream_t)stream, (const T*)q, qs_b,
-        qs_h, qs_q, (const T*)pmin, (const T*)pmax, P_cap, Hq, Hkv, Sq, S, D, page_size,
-        (const T*)bias, bias_s_b, bias_s_q, (T*)scores);
-  });
+  const dim3 block((unsigned)pages, (unsigned)qrows);
+#define QS_LAUNCH(T, STAGED)                                                                                       \
+  do {                                                                                                             \
+    if (smem > 48 * 1024) {                                                                                        \
+      const cudaError_t e = cudaFuncSetAttribute(                                                                  \
+          quest_scores_kernel<T, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, QS_SMEM);                   \
+      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "quest_scores attr: %s", cudaGetErrorString(e));         \
+    }                                                                                                              \
+    sah_launch_chain(quest_scores_kernel<T, STAGED>, grid, block, smem, (cudaStream_t)stream, (const T*)q, qs_b,   \
+        qs_h, qs_q, (const T*)pmin, (const T*)pmax, P_cap, Hq, Hkv, Sq, S, D, page_size, (const T*)bias, bias_s_b, \
+        bias_s_q, (T*)scores);                                                                                     \
+  } while (0)
+  if (dtype == SAH_BF16) QS_LAUNCH(__nv_bfloat16, true);
+  else if (dtype != SAH_F32) return sah_fail(SAH_ERR_INVALID, "unknown dtype %d", dtype);
+  else if (direct) QS_LAUNCH(float, false);
+  else QS_LAUNCH(float, true);
+#undef QS_LAUNCH
   SAH_LAUNCH_CHECK("quest_scores");
   sah_prof_end(SAH_PROF_QUEST, (cudaStream_t)stream);
   return SAH_OK;

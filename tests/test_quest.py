@@ -182,3 +182,42 @@ def test_gpu_appended_keys_update_only_their_pages():
         assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
         ref_mask, _, _ = stacks.run_stack(stack, wl.q, wl.k[:, :, :n], wl.v[:, :, :n], wl.scaling, "bf16")
         np.testing.assert_array_equal(a[0].cpu().numpy(), mask_ops.to_csr(ref_mask)[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,P,masked", [(128, 771, False), (72, 771, True), (256, 1029, False), (64, 800, True)])
+def test_gpu_float32_scores_of_many_rows_equal_those_of_few(D, P, masked):
+    """From 48 K float32 scores on a row reads the page bounds where they lie, below that four rows
+    share a copy in shared memory: the same bits for the same row."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hq, Hkv, Sq, page = 2, 8, 2, 4, 16
+    S, P_cap = P * page - 5, P + 3
+    gen = torch.Generator(device=dev).manual_seed(D)
+    q = torch.randn((B, Sq, Hq, D), generator=gen, device=dev).transpose(1, 2)
+    lo = torch.randn((B, Hkv, D // 8, P_cap, 8), generator=gen, device=dev)
+    hi = lo + torch.rand((B, Hkv, D // 8, P_cap, 8), generator=gen, device=dev)
+    bias = None
+    if masked:
+        bias = torch.zeros((B, 1, Sq, S), device=dev)
+        bias[..., page * 7:page * 9 + 1] = torch.finfo(torch.float32).min
+
+    def scores(n):
+        out = torch.zeros((B, Hq, n, P), device=dev)
+        _native.check(lib.sah_quest_scores(q.data_ptr(), _native.SAH_F32, q.stride(0), q.stride(1), q.stride(2),
+                                           lo.data_ptr(), hi.data_ptr(), P_cap, B, Hq, Hkv, n, S, D, page,
+                                           _native.ptr(bias), S * Sq, 0, S, out.data_ptr(),
+                                           _native.stream_of(torch.device(dev))), "sah_quest_scores")
+        return out
+
+    many, few = scores(Sq), scores(1)
+    assert B * Hq * Sq * P >= 48 * 1024 > B * Hq * P
+    assert torch.equal(many[:, :, :1], few)
+    want = torch.maximum(q[:, :, 1, None] * lo[:, :, :, :P].permute(0, 1, 3, 2, 4).reshape(B, Hkv, P, D).repeat_interleave(
+        Hq // Hkv, 1), q[:, :, 1, None] * hi[:, :, :, :P].permute(0, 1, 3, 2, 4).reshape(B, Hkv, P, D).repeat_interleave(
+            Hq // Hkv, 1)).sum(-1, dtype=torch.float64)
+    if not masked:  # D float32 products added in float32: within D 2^-24 of the sum of magnitudes, 4 D here
+        assert float((many[:, :, 1].double() - want).abs().max()) < D * 2.0 ** -24 * 4 * D
