@@ -550,11 +550,15 @@ def test_hash_topk_under_an_additive_mask(B, Hq, Sq, S, k, dtype):
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,S,D,masked", [
     (1, 4, 1, 1, 1, 128, False), (2, 3, 3, 1, 17, 128, True), (1, 16, 2, 1, 1003, 128, False),
     (1, 6, 2, 3, 333, 64, True), (3, 2, 2, 1, 64, 64, False), (1, 8, 2, 24, 79, 128, True),
-    (1, 4, 2, 2, 140, 80, True), (1, 6, 2, 1, 1601, 64, True), (1, 8, 8, 1, 30000, 128, False)])
+    (1, 4, 2, 2, 140, 80, True), (1, 6, 2, 1, 1601, 64, True), (1, 8, 8, 1, 30000, 128, False),
+    (1, 32, 8, 1, 19001, 128, False), (1, 32, 8, 1, 19100, 128, True), (2, 32, 8, 1, 9700, 64, False),
+    (2, 16, 8, 2, 9770, 64, True), (1, 32, 8, 2, 18945, 128, False)])
 def test_score_bits_at_the_edges(dtype, B, Hq, Hkv, Sq, S, D, masked):
     """q.k bit for bit in the fixed order: group sizes that are no multiple of four, key counts
-    around the 16-key groups of a warp, more rows than stay in registers, head dims with and
-    without the four-lane kernel, strided keys and queries."""
+    around the ends of a CTA's tile, more rows than stay in registers, head dims that are and are not
+    compiled in, strided keys and queries; and, in the last five in bfloat16, two keys per thread (rows in
+    fours, 592 CTAs of 256 keys or more) with a last tile of 1, 42, 57, 156 and 228 keys, of which a thread's
+    second one may lie past the end."""
     torch.manual_seed(S + D)
     dt = torch.bfloat16 if dtype == "bf16" else torch.float32
     q = torch.randn((B, Sq, Hq, D), device=DEV).to(dt).transpose(1, 2)
