@@ -188,12 +188,16 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
               "pq_assign_tc: key rows must be 16-byte aligned");
   if (key_begin == key_end) return SAH_OK;
   if (sm_count <= 0) sm_count = 148;
-  // four neighbouring sub-vectors per CTA (a key's 64 bytes, one 4-byte store of codes) when the
-  // layout allows it, else one; n_cent padded to a power-of-two number of 32-column blocks
-  const int ns = (n_sub % 4 == 0 && (reinterpret_cast<uintptr_t>(codes) & 3) == 0) ? 4 : 1;
-  const int64_t n_blocks = (int64_t)B * Hkv * (n_sub / ns);
-  const int64_t items = n_blocks * sah_ceil_div(key_end - key_begin, (int64_t)PTC_TILE);
-  const unsigned grid = (unsigned)(items < 2 * (int64_t)sm_count ? (items + 1) / 2 : sm_count);
+  // Four neighbouring sub-vectors per CTA (a key's 64 bytes, one 4-byte store of codes) when the
+  // layout allows it, else one; also one while every (sub-vector, tile) has a group of warps to itself
+  // (128 groups x 64 keys x 256 centroids 23.4 us by fours, 7.3 us one by one).  n_cent padded to a
+  // power-of-two number of 32-column blocks.
+  const int64_t tiles = sah_ceil_div(key_end - key_begin, (int64_t)PTC_TILE);
+  auto ctas = [&](int64_t blocks) { return tiles == 1 ? blocks : (blocks * tiles + 1) / 2; };  // two tiles of a block each
+  const int64_t groups = (int64_t)B * Hkv * n_sub;
+  const int ns = n_sub % 4 == 0 && (reinterpret_cast<uintptr_t>(codes) & 3) == 0 && ctas(groups) > sm_count ? 4 : 1;
+  const int64_t n_blocks = groups / ns;
+  const unsigned grid = (unsigned)(ctas(n_blocks) < sm_count ? ctas(n_blocks) : sm_count);
   const cudaStream_t st = (cudaStream_t)stream;
 #define PTC_LAUNCH(NS, NB)                                                                                       \
   do {                                                                                                           \

@@ -248,10 +248,11 @@ def test_gpu_ip_metric_build_decode_and_append_equal_the_reference():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n_sub,n_cent,n_keys", [(16, 256, 1), (16, 64, 129), (4, 128, 300), (6, 256, 255), (3, 32, 128)])
+@pytest.mark.parametrize("n_sub,n_cent,n_keys", [(16, 256, 1), (16, 64, 129), (4, 128, 300), (6, 256, 255), (3, 32, 128),
+                                                 (16, 256, 1281), (16, 16, 1200), (8, 64, 2600), (4, 128, 9700)])
 def test_gpu_assignment_tile_edges_and_layouts(n_sub, n_cent, n_keys):
     """`sah_pq_assign_tc` at the edges of its tiles (one key, a tile, a tile and one), for every
-    padded centroid count and with one or four sub-vectors per CTA, on integer-valued keys and
+    padded centroid count and with one sub-vector per CTA or (the last four) four, on integer-valued keys and
     centroids (many exact ties): the codes of `sah_pq_assign`."""
     import torch
     from sparse_attention_hub import _native
