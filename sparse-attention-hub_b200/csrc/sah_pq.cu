@@ -228,6 +228,9 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
 // counting sort with integer atomics in shared memory), then two threads per centroid walk the
 // centroid's keys, each adding half of the channels into fp64 registers that live across the
 // strips; the registers go to global memory with one atomic per (centroid, channel) and CTA.
+// Below 129 centroids several such pairs of lanes (`shares`) take every so many-th key of a centroid
+// and add up in the warp (16 centroids, 128 groups x 65472 keys: 258 us in bfloat16 and 1374 us in
+// float32 with a pair each, 76 us and 176 us this way).
 // Bound: shared-memory integer atomics and L2 (every 32-byte sector of a key is fetched by the
 // CTAs of two sub-vectors).  8 KV heads x 65472 keys x 16 sub-vectors: 96 us with eight keys of a
 // centroid in flight, 122 us with four and three CTAs per SM; with one fp64 shared-memory atomic
@@ -239,7 +242,7 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
 template <typename T>
 __global__ void __launch_bounds__(PQA_THREADS, 2)
 pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
-                     int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int cblocks, int vec8,
+                     int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int cblocks, int shares, int vec8,
                      const uint8_t* __restrict__ codes, int64_t cap, double* __restrict__ sums,
                      int* __restrict__ counts) {
   __shared__ int pos_sm[256];              // histogram, then the next free slot of every centroid
@@ -254,7 +257,7 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
   const int kvh = (int)(bk % Hkv);
   const int64_t b = bk / Hkv;
   const int64_t grp = bk * n_sub + sub;
-  const int cent = tid >> 1;
+  const int cent = (tid >> 1) / shares, share = (tid >> 1) - cent * shares;
   const int nch = sub_d - c_lo < PQ_MAX_SUBD ? sub_d - c_lo : PQ_MAX_SUBD;  // channels of this CTA
   const int half = (nch + 1) / 2;          // channels of the even threads
   const int d0 = c_lo + ((tid & 1) ? half : 0), nd = (tid & 1) ? nch - half : half;
@@ -288,13 +291,15 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
     __syncthreads();
     const int e1 = start_sm[cent + 1];
     int e = start_sm[cent];
-    count += e1 - e;
+    if (share == 0) count += e1 - e;
+    e += share;
     const T* xs = xg + j0 * xs_s;
     if (sizeof(T) == 2 && vec8) {  // four channels in 8 aligned bytes; eight keys in flight
-      for (; e + 8 <= e1; e += 8) {
+      for (; e + 7 * shares < e1; e += 8 * shares) {
         uint2 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u] * xs_s);
+        for (int u = 0; u < 8; ++u)
+          v[u] = *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u * shares] * xs_s);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           acc[0] += (double)__uint_as_float(v[u].x << 16);
@@ -305,13 +310,13 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
       }
       {  // the last few, all in flight as well
         uint2 v[8];
-        const int left = e1 - e;
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-          v[u] = u < left ? *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u] * xs_s) : make_uint2(0u, 0u);
+          v[u] = e + u * shares < e1 ? *reinterpret_cast<const uint2*>(xs + (int64_t)order_sm[e + u * shares] * xs_s)
+                                     : make_uint2(0u, 0u);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-          if (u < left) {
+          if (e + u * shares < e1) {
             acc[0] += (double)__uint_as_float(v[u].x << 16);
             acc[1] += (double)__uint_as_float(v[u].x & 0xffff0000u);
             acc[2] += (double)__uint_as_float(v[u].y << 16);
@@ -319,7 +324,7 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
           }
       }
     } else {
-      for (; e < e1; ++e) {
+      for (; e < e1; e += shares) {
         const T* xr = xs + (int64_t)order_sm[e] * xs_s;
 #pragma unroll
         for (int i = 0; i < HALF; ++i)
@@ -328,12 +333,21 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
     }
     __syncthreads();  // the sorted list and the starts are done with
   }
-  if (cent < n_cent && count > 0) {
+  bool any = count > 0;
+  if (shares > 1) {  // up to 16 shares of a centroid lie in one warp
+    const int width = shares < 16 ? shares : 16;
+    for (int o = 1; o < width; o <<= 1)
+#pragma unroll
+      for (int i = 0; i < HALF; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 2 * o);
+    if (share % width != 0) return;
+    any = shares > 16 || count > 0;
+  }
+  if (cent < n_cent && any) {
     double* out = sums + (grp * n_cent + cent) * sub_d + d0;
 #pragma unroll
     for (int i = 0; i < HALF; ++i)
       if (i < nd) atomicAdd(out + i, acc[i]);
-    if ((tid & 1) == 0 && c_lo == 0) atomicAdd(&counts[grp * n_cent + cent], count);
+    if ((tid & 1) == 0 && c_lo == 0 && count > 0) atomicAdd(&counts[grp * n_cent + cent], count);
   }
 }
 
@@ -353,11 +367,14 @@ extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t
   const int64_t strips = sah_ceil_div(n_keys, (int64_t)PQA_STRIP);
   if (slices > strips) slices = strips;
   dim3 grid((unsigned)slices, (unsigned)(n_sub * cblocks), (unsigned)((int64_t)B * Hkv));
+  // pairs of threads per centroid: what is left of 256 of them, a power of two
+  int shares = 1;
+  while (shares * 2 * n_cent <= PQA_THREADS / 2) shares *= 2;
   const int vec8 = sub_d == 8 && (reinterpret_cast<uintptr_t>(x) & 7) == 0 && xs_s % 4 == 0 && xs_h % 4 == 0 &&
                    xs_b % 4 == 0;
   SAH_DISPATCH_DTYPE(dtype, T, {
     pq_accumulate_kernel<T><<<grid, PQA_THREADS, 0, (cudaStream_t)stream>>>(
-        (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, cblocks, vec8, codes, cap,
+        (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, cblocks, shares, vec8, codes, cap,
         sums, counts);
   });
   SAH_LAUNCH_CHECK("pq_accumulate");

@@ -277,18 +277,21 @@ def test_gpu_assignment_tile_edges_and_layouts(n_sub, n_cent, n_keys):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dtype,n_sub,sub_d,n_keys", [("bf16", 16, 8, 1), ("bf16", 16, 8, 4097), ("bf16", 4, 9, 5000),
-                                                      ("f32", 3, 16, 4096), ("f32", 2, 5, 9000)])
-def test_gpu_cluster_sums_equal_float64_sums(dtype, n_sub, sub_d, n_keys):
+@pytest.mark.parametrize("dtype,n_sub,sub_d,n_keys,n_cent", [
+    ("bf16", 16, 8, 1, 32), ("bf16", 16, 8, 4097, 32), ("bf16", 4, 9, 5000, 32), ("f32", 3, 16, 4096, 32),
+    ("f32", 2, 5, 9000, 32), ("bf16", 16, 8, 4200, 256), ("f32", 2, 8, 4099, 129), ("bf16", 2, 8, 5001, 128),
+    ("bf16", 4, 8, 4301, 16), ("f32", 2, 6, 4301, 9), ("bf16", 2, 8, 130, 8), ("f32", 1, 3, 4099, 8)])
+def test_gpu_cluster_sums_equal_float64_sums(dtype, n_sub, sub_d, n_keys, n_cent):
     """`sah_pq_accumulate`: counts exact, and float64 sums that round to the float32 sums of numpy's
     float64 additions (values are multiples of 2^-8 below 8, so float64 sums are exact in any
-    order); one cluster holds half of the keys and one none."""
+    order); one cluster holds half of the keys and one none.  From 129 centroids on a pair of threads has
+    a centroid to itself, with 9 to 16 of them a warp has one, with 8 two warps share one."""
     import torch
     from sparse_attention_hub import _native
 
     lib = _native.load()
     dev = "cuda:0"
-    B, Hkv, off, n_cent = 2, 1, 2, 32
+    B, Hkv, off = 2, 1, 2
     gen = torch.Generator(device=dev).manual_seed(n_keys)
     keys = (torch.randint(-2047, 2048, (B, Hkv, n_keys + off, n_sub * sub_d), generator=gen, device=dev) / 256.0)
     keys = keys.to(workloads.torch_dtype(dtype))
