@@ -75,20 +75,30 @@ __device__ __forceinline__ float ad_exp<float>(float x, const uint16_t*) { retur
 // order (1024 threads).  A thread's bits are the same bit of every 32nd word, so 32 words of a warp
 // are turned over (a 32 x 32 bit transposition, five exchanges) and each lane walks its own bits:
 // testing word after word, every warp went through the body for nearly all of them.
+#define AD_FEW 2  // words per warp up to which the bits are picked one by one
 template <typename F>
 __device__ __forceinline__ void ad_own_columns(const uint32_t* bits, int64_t S, F f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t words = (S + 31) / 32;
   for (int64_t n0 = 0; n0 * 32 < words; n0 += 32) {  // words warp + 32 (n0 + lane)
-    const int64_t w = warp + 32 * (n0 + lane);
-    uint32_t m = w < words ? bits[w] : 0u;
-    if (w == words - 1 && (S & 31)) m &= (1u << (int)(S & 31)) - 1u;
+    uint32_t m = 0u;
+    if (words <= 32 * AD_FEW) {  // a few words per warp: every lane reads its own bit of each
 #pragma unroll
-    for (int o = 16, keep = 0x0000FFFF; o > 0; o >>= 1, keep ^= keep << o) {
-      // exchange the off-diagonal blocks of size o
-      const uint32_t other = __shfl_xor_sync(0xffffffffu, m, o);
-      m = (lane & o) ? ((m & ~(uint32_t)keep) | ((other >> o) & (uint32_t)keep))
-                     : ((m & (uint32_t)keep) | ((other << o) & ~(uint32_t)keep));
+      for (int i = 0; i < AD_FEW; ++i) {
+        const int64_t w = warp + 32 * i;
+        if (w * 32 + lane < S) m |= ((bits[w] >> lane) & 1u) << i;
+      }
+    } else {
+      const int64_t w = warp + 32 * (n0 + lane);
+      m = w < words ? bits[w] : 0u;
+      if (w == words - 1 && (S & 31)) m &= (1u << (int)(S & 31)) - 1u;
+#pragma unroll
+      for (int o = 16, keep = 0x0000FFFF; o > 0; o >>= 1, keep ^= keep << o) {
+        // exchange the off-diagonal blocks of size o
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, m, o);
+        m = (lane & o) ? ((m & ~(uint32_t)keep) | ((other >> o) & (uint32_t)keep))
+                       : ((m & (uint32_t)keep) | ((other << o) & ~(uint32_t)keep));
+      }
     }
     while (m) {  // bit i: column lane of word warp + 32 (n0 + i)
       const int i = __ffs(m) - 1;
@@ -122,6 +132,7 @@ struct AdaptiveArgs {
 // table between (d negative) is kept in shared memory.
 #define AD_D0 0xBA80  // bf16 bits of -2^-10
 #define AD_D1 0xC300  // -128
+#define AD_SMEM (200 * 1024)       // the base sample's bitmap, or that and the row
 #define AD_ROW_BYTES (160 * 1024)  // logits of a bfloat16 row in shared memory: 81920 keys
 
 // One CTA (1024 threads) per mask row.  Every tensor operation of the reference is one
@@ -130,8 +141,9 @@ struct AdaptiveArgs {
 // shared memory beside the table, because the sums visit scattered keys (the previous mask's, the
 // sample's) one after the other: with a load of the score and a gather of the weight from global
 // memory for each of them 128 rows x 65536 keys took 44.6 us, all of it latency; 19.3 us now.
-template <typename T, bool RESIDENT>
-__global__ void __launch_bounds__(1024)
+// KEEP: draws per thread whose weights stay in registers between the two sums over the sample.
+template <typename T, bool RESIDENT, int KEEP>
+__global__ void __launch_bounds__(1024, RESIDENT ? 1 : 2)
 adaptive_budget_kernel(AdaptiveArgs a) {
   sah_pdl_entry();
   extern __shared__ __align__(16) uint32_t ad_base_bits[];  // W words: distinct base-sample columns
@@ -226,8 +238,7 @@ adaptive_budget_kernel(AdaptiveArgs a) {
     return a.base_draws ? a.base_draws[row * a.nb + i]
                         : sah_draw_column(a.seed, (uint64_t)(row * a.nb + i), a.start, n);
   };
-  // the weights of a thread's first four draws (5 % of 65536 keys) are kept for the second sum
-  constexpr int KEEP = 4;
+  // the weights of a thread's first draws are kept for the second sum
   float drawn[KEEP];
   part = 0.f;
 #pragma unroll
@@ -318,32 +329,38 @@ extern "C" int sah_adaptive_budget(const void* scores, int dtype, float scaling,
   a.seed = seed; a.base_draws = base_draws; a.exp_table = exp_table;
   a.delta_ppf = delta_ppf; a.epsilon = epsilon; a.budget = budget; a.prob = prob; a.stats = stats;
   const size_t smem = (size_t)W * sizeof(uint32_t);
-  if (smem > 200 * 1024)
+  if (smem > AD_SMEM)
     return sah_fail(SAH_ERR_UNSUPPORTED, "adaptive_budget: %lld keys per row exceed the base-sample bitmap",
                     (long long)S);
   const int64_t rows = (int64_t)B * Hq * Sq;
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_ADAPTIVE, st);
+#define AD_LAUNCH(RESIDENT, KEEP)                                                                           \
+  do {                                                                                                      \
+    if (bytes > 40 * 1024) {                                                                                \
+      const cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, RESIDENT, KEEP>,                 \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, AD_SMEM);     \
+      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e)); \
+    }                                                                                                       \
+    sah_launch_chain(adaptive_budget_kernel<T, RESIDENT, KEEP>, (unsigned)rows, 1024, bytes, st, a);        \
+  } while (0)
   SAH_DISPATCH_DTYPE(dtype, T, {
-    // bfloat16 rows that fit stay in shared memory; float32 weights come from a double-precision
-    // exponential, not from a table, and longer rows are read again
+    // Bfloat16 rows that fit stay in shared memory, unless several of them can share an SM that would
+    // hold one (from 149 rows on, up to 65536 keys: 256 x 8192 15.0 us resident, 12.9 us not; 256 x
+    // 65536 even) or the table takes longer to copy than the row to read (below 2048 keys).  float32
+    // weights come from a double-precision exponential, not from a table, and longer rows are read
+    // again.
     const size_t row_bytes = (size_t)W * 32 * sizeof(T);
-    if (sizeof(T) == 2 && row_bytes <= AD_ROW_BYTES) {
-      const size_t bytes = (size_t)(W + 3) / 4 * 16 + row_bytes;
-      cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, sizeof(T) == 2>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           AD_ROW_BYTES / 16 + AD_ROW_BYTES);
-      if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e));
-      sah_launch_chain(adaptive_budget_kernel<T, sizeof(T) == 2>, (unsigned)rows, 1024, bytes, st, a);
-    } else {
-      if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(adaptive_budget_kernel<T, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "adaptive_budget attr: %s", cudaGetErrorString(e));
-      }
-      sah_launch_chain(adaptive_budget_kernel<T, false>, (unsigned)rows, 1024, smem, st, a);
-    }
+    const bool resident = sizeof(T) == 2 && row_bytes <= AD_ROW_BYTES && S >= 2048 && (rows <= 148 || S > 65536);
+    constexpr bool RES = sizeof(T) == 2;
+    const size_t bytes = resident ? (size_t)(W + 3) / 4 * 16 + row_bytes : smem;
+    // one draw per thread (5 % of 20480 keys), or up to four kept (of 81920) and the others made again
+    if (resident && nb <= 1024) AD_LAUNCH(RES, 1);
+    else if (resident) AD_LAUNCH(RES, 4);
+    else if (nb <= 1024) AD_LAUNCH(false, 1);
+    else AD_LAUNCH(false, 4);
   });
+#undef AD_LAUNCH
   SAH_LAUNCH_CHECK("adaptive_budget");
   sah_prof_end(SAH_PROF_ADAPTIVE, st);
   return SAH_OK;

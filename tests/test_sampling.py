@@ -225,3 +225,35 @@ def test_gpu_random_sampling_own_draws_statistics():
     # 1024 draws with replacement from 4096: about 4096 * (1 - exp(-1/4)) = 906 distinct
     assert np.all(per_row <= 1024) and abs(per_row.mean() - 906) < 30
     assert np.all(got[2] == np.float32(0.25))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,B,Hq,S,rate,masked", [
+    ("bf16", 1, 2, 40003, 0.05, False), ("bf16", 1, 2, 40003, 0.02, True), ("bf16", 1, 2, 90001, 0.05, True),
+    ("bf16", 1, 2, 90001, 0.011, False), ("bf16", 10, 16, 2100, 0.05, True), ("bf16", 2, 4, 700, 0.1, False),
+    ("f32", 1, 2, 40003, 0.05, True), ("f32", 10, 16, 1100, 0.05, False), ("f32", 1, 2, 2049, 0.04, True)])
+def test_gpu_adaptive_budgets_of_long_short_and_many_rows(dtype, B, Hq, S, rate, masked):
+    """Rows that stay in shared memory, rows too long for it, rows of which an SM takes several; one
+    draw per thread, up to four kept, more; lengths that are no multiple of 8 or 32; additive masks:
+    budget, probability and stats bit for bit."""
+    import torch
+
+    wl = workloads.oracle_adaptive(seed=S, dtype=dtype, B=B, Hq=Hq, Hkv=Hq // 2, S=S, D=64, sink=8, window=24,
+                                   heavy=0.02, base_rate=rate, epsilon=0.1, delta=0.1, Sq=1)
+    am = None
+    if masked:
+        am = np.zeros((B, 1, 1, S), np.float32)
+        am[..., S // 2:S // 2 + 41] = -np.inf
+        am[..., 3] = 0.5
+    dev = "cuda:0"
+    ra = workloads.research_attention(wl.stack, wl.dtype, dev)
+    q, k, v = (workloads.to_torch(a, wl.dtype, dev) for a in (wl.q, wl.k, wl.v))
+    meta = {"adaptive_sampling_seed": 5}
+    ra.build_mask(q, k, v, None if am is None else workloads.to_torch(am, wl.dtype, dev), float(wl.scaling), 0.0,
+                  meta, layer_idx=0)
+    budget, prob, stats = meta["adaptive_sampling_stats"][0]
+    _, _, ometa = stacks.run_stack(wl.stack, wl.q, wl.k, wl.v, wl.scaling, dtype, attention_mask=am,
+                                   meta={"adaptive_seed": 5 * 1000003})
+    np.testing.assert_array_equal(budget.cpu().numpy(), ometa["adaptive_budget"])
+    np.testing.assert_array_equal(prob.float().cpu().numpy(), ometa["adaptive_prob"])
+    np.testing.assert_array_equal(stats.cpu().numpy(), ometa["adaptive_stats"])
