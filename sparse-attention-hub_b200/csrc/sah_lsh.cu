@@ -156,8 +156,20 @@ __device__ __forceinline__ float lsh_augment(float nk, float M) {
 // copy requested before the first is waited for (no wait in here).
 #define LSH_COLS 64
 #define LSH_COLS_THREADS 128
+#define LSH_QUERY_FOUR (4 * 148)
 // the hyperplanes, a row of head dim + 1 and the signs: at most, for head dim 256
 #define LSH_COLS_SMEM(T) (257 * (LSH_COLS * (int)sizeof(T) + 4) + LSH_COLS)
+// Tables per CTA: as many as fit, but if rows of hyperplanes start on 16 bytes no more than leave
+// every CTA's columns starting there too (10 bits per table in bfloat16: four tables, not six).
+template <typename T>
+static int lsh_cta_tables(int K, int L) {
+  constexpr int PER = 16 / (int)sizeof(T);
+  const int most = LSH_COLS / K;
+  if ((L * K) % PER == 0)
+    for (int t = most; t > 0; --t)
+      if (t * K % PER == 0) return t;
+  return most;
+}
 template <typename T>
 __device__ __forceinline__ void lsh_stage_columns(const T* __restrict__ proj, int nbits, int Dp, int c0, int nc,
                                                   T* __restrict__ sm) {
@@ -191,14 +203,14 @@ __global__ void __launch_bounds__(LSH_COLS_THREADS)
 lsh_key_sign_few_kernel(const T* __restrict__ k, int64_t ks_b, int64_t ks_h, int64_t ks_s, int Hkv,
                         int64_t s0, int D, const T* __restrict__ mean, const float* __restrict__ norms,
                         const unsigned int* __restrict__ max_bits, const T* __restrict__ proj, int L, int K,
-                        int64_t cap, CodeT* __restrict__ codes) {
+                        int tables, int64_t cap, CodeT* __restrict__ codes) {
   sah_pdl_entry_early();
   extern __shared__ __align__(16) unsigned char lsh_smem[];
   const int nbits = L * K, Dp = D + 1;
   T* pr = reinterpret_cast<T*>(lsh_smem);                                         // [Dp][LSH_COLS]
   float* xt = reinterpret_cast<float*>(lsh_smem + (size_t)Dp * LSH_COLS * sizeof(T));  // [Dp]
   unsigned char* sb = reinterpret_cast<unsigned char*>(xt + Dp);                  // [LSH_COLS]
-  const int tables = LSH_COLS / K, l0 = blockIdx.x * tables;
+  const int l0 = blockIdx.x * tables;
   const int lt = L - l0 < tables ? L - l0 : tables;
   lsh_stage_columns<T>(proj, nbits, Dp, l0 * K, lt * K, pr);
   const int64_t bh = blockIdx.y, s = s0 + blockIdx.z;
@@ -329,10 +341,10 @@ extern "C" int sah_lsh_key_sign(const void* keys, int dtype, int64_t ks_b, int64
   dim3 grid((unsigned)((s1 - s0 + LSH_KT - 1) / LSH_KT), (unsigned)(B * Hkv));
   cudaStream_t st = (cudaStream_t)stream;
   if (s1 - s0 <= LSH_FEW_KEYS) {
-    const int tables = LSH_COLS / K;
-    dim3 fgrid((unsigned)((L + tables - 1) / tables), (unsigned)(B * Hkv), (unsigned)(s1 - s0));
 #define LSH_FEW_LAUNCH(T, CodeT)                                                                   \
   do {                                                                                             \
+    const int tables = lsh_cta_tables<T>(K, L);                                                    \
+    const dim3 fgrid((unsigned)((L + tables - 1) / tables), (unsigned)(B * Hkv), (unsigned)(s1 - s0)); \
     const int bytes = (D + 1) * (LSH_COLS * (int)sizeof(T) + 4) + LSH_COLS;                        \
     if (bytes > 48 * 1024) {                                                                       \
       cudaError_t e = cudaFuncSetAttribute(lsh_key_sign_few_kernel<T, CodeT>,                      \
@@ -342,7 +354,7 @@ extern "C" int sah_lsh_key_sign(const void* keys, int dtype, int64_t ks_b, int64
     sah_launch_chain(lsh_key_sign_few_kernel<T, CodeT>, fgrid, LSH_COLS_THREADS, bytes, st, \
         reinterpret_cast<const T*>(keys), ks_b, ks_h, ks_s, Hkv, s0, D,                            \
         reinterpret_cast<const T*>(mean), norms, max_norm_bits, reinterpret_cast<const T*>(proj),  \
-        L, K, cap, reinterpret_cast<CodeT*>(codes));                                               \
+        L, K, tables, cap, reinterpret_cast<CodeT*>(codes));                                       \
   } while (0)
     SAH_DISPATCH_DTYPE(dtype, T, {
       if (K <= 8) LSH_FEW_LAUNCH(T, uint8_t); else LSH_FEW_LAUNCH(T, uint16_t);
@@ -436,35 +448,39 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
 // ---------------------------------------------------------------------------------------
 // query: centre, normalise, signatures, unit vector
 // ---------------------------------------------------------------------------------------
-// A CTA takes one query row and LSH_COLS / K tables: the hyperplanes are requested at once, the
+// A CTA takes one query row and up to LSH_COLS / K tables: the hyperplanes are requested at once, the
 // first warp normalises the query meanwhile (every CTA of the row does; the first one writes it
 // out), then one thread per column adds up the channels in order.  This kernel sits on the
 // critical path of every decode step and is all latency: 32 rows took 12.5 us with one CTA per
-// row, 7.7 us now.
-template <typename T, typename CodeT>
+// row, 7.7 us now.  Where that makes more CTAs than an SM holds at once, the hyperplanes' way from L2
+// takes the time, and a CTA takes four rows, a warp normalising each: 512 rows x 75 tables of 8 bits
+// in float32 22.0 us with one CTA per row, 30.6 us with ROWS = 1, 14.4 us with 4 (bfloat16 25.2, 22.3,
+// 13.3).
+template <typename T, typename CodeT, int ROWS>
 __global__ void __launch_bounds__(LSH_COLS_THREADS)
 lsh_query_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs_q, int Hq, int Sq,
                  int G, int D, const T* __restrict__ mean, const T* __restrict__ proj, int L, int K,
-                 CodeT* __restrict__ qcodes, float* __restrict__ qunit, T* __restrict__ qhat,
+                 int tables, int64_t rows, CodeT* __restrict__ qcodes, float* __restrict__ qunit, T* __restrict__ qhat,
                  float* __restrict__ qmu) {
   sah_pdl_entry_early();
   extern __shared__ __align__(16) unsigned char lsh_smem[];
   const int nbits = L * K, Dp = D + 1;
   T* pr = reinterpret_cast<T*>(lsh_smem);                                         // [Dp][LSH_COLS]
-  float* qn = reinterpret_cast<float*>(lsh_smem + (size_t)Dp * LSH_COLS * sizeof(T));  // [D] normalised query
-  unsigned char* sb = reinterpret_cast<unsigned char*>(qn + D);                   // [LSH_COLS]
-  const int tables = LSH_COLS / K, l0 = blockIdx.y * tables;
+  float* qn_sm = reinterpret_cast<float*>(lsh_smem + (size_t)Dp * LSH_COLS * sizeof(T));  // [ROWS][D] normalised
+  unsigned char* sb = reinterpret_cast<unsigned char*>(qn_sm + ROWS * D);         // [ROWS][LSH_COLS]
+  const int l0 = blockIdx.y * tables;
   const int lt = L - l0 < tables ? L - l0 : tables;
   lsh_stage_columns<T>(proj, nbits, Dp, l0 * K, lt * K, pr);
   const bool writer = blockIdx.y == 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row = blockIdx.x;
-  const int qi = (int)(row % Sq);
-  const int64_t bh = row / Sq;
-  const int h = (int)(bh % Hq);
-  const int64_t b = bh / Hq;
+  const int64_t row0 = (int64_t)blockIdx.x * ROWS, row = row0 + warp;  // the row of this warp, if it has one
   const int per = D / 32;
-  if (warp == 0) {
+  if (warp < ROWS && row < rows) {
+    const int qi = (int)(row % Sq);
+    const int64_t bh = row / Sq;
+    const int h = (int)(bh % Hq);
+    const int64_t b = bh / Hq;
+    float* qn = qn_sm + warp * D;
     float x[LSH_MAX_PER_LANE], m[LSH_MAX_PER_LANE], c[LSH_MAX_PER_LANE];
     lsh_load_lane<T>(q + b * qs_b + h * qs_h + qi * qs_q, per, lane, x);
     if (mean) lsh_load_lane<T>(mean + (b * (Hq / G) + h / G) * D, per, lane, m);
@@ -504,19 +520,31 @@ lsh_query_kernel(const T* __restrict__ q, int64_t qs_b, int64_t qs_h, int64_t qs
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  if (threadIdx.x < lt * K) {  // one accumulator per column, channels ascending, as everywhere
-    float acc = 0.f;
+  // one accumulator per row and column, channels ascending, as everywhere; with four rows, two each
+  constexpr int PER = ROWS == 1 ? 1 : ROWS * LSH_COLS / LSH_COLS_THREADS;
+  const int col = ROWS == 1 ? threadIdx.x : threadIdx.x % LSH_COLS;
+  const int r0 = ROWS == 1 ? 0 : threadIdx.x / LSH_COLS * PER;
+  if (col < lt * K) {
+    float acc[PER];
+#pragma unroll
+    for (int r = 0; r < PER; ++r) acc[r] = 0.f;
 #pragma unroll 8
-    for (int c = 0; c < D; ++c)
-      acc = __fadd_rn(acc, __fmul_rn(qn[c], sah_to_float<T>(pr[c * LSH_COLS + threadIdx.x])));
-    acc = __fadd_rn(acc, __fmul_rn(0.f, sah_to_float<T>(pr[D * LSH_COLS + threadIdx.x])));
-    sb[threadIdx.x] = acc > 0.f ? 1 : 0;
+    for (int c = 0; c < D; ++c) {
+      const float p = sah_to_float<T>(pr[c * LSH_COLS + col]);
+#pragma unroll
+      for (int r = 0; r < PER; ++r) acc[r] = __fadd_rn(acc[r], __fmul_rn(qn_sm[(r0 + r) * D + c], p));
+    }
+    const float last = __fmul_rn(0.f, sah_to_float<T>(pr[D * LSH_COLS + col]));
+#pragma unroll
+    for (int r = 0; r < PER; ++r) sb[(r0 + r) * LSH_COLS + col] = __fadd_rn(acc[r], last) > 0.f ? 1 : 0;
   }
   __syncthreads();
-  for (int l = threadIdx.x; l < lt; l += LSH_COLS_THREADS) {
+  for (int i = threadIdx.x; i < ROWS * lt; i += LSH_COLS_THREADS) {
+    const int r = ROWS == 1 ? 0 : i / lt, l = i - r * lt;
+    if (row0 + r >= rows) break;
     unsigned int code = 0;
-    for (int j = 0; j < K; ++j) code |= (unsigned int)sb[l * K + j] << j;
-    qcodes[row * L + l0 + l] = (CodeT)code;
+    for (int j = 0; j < K; ++j) code |= (unsigned int)sb[r * LSH_COLS + l * K + j] << j;
+    qcodes[(row0 + r) * L + l0 + l] = (CodeT)code;
   }
 }
 
@@ -533,23 +561,28 @@ extern "C" int sah_lsh_query(const void* q, int dtype, int64_t qs_b, int64_t qs_
     return sah_fail(SAH_ERR_UNSUPPORTED, "lsh_query: %d x %d signature bits exceed shared memory", L, K);
   const int64_t rows = (int64_t)B * Hq * Sq;
   cudaStream_t st = (cudaStream_t)stream;
-  const int tables = LSH_COLS / K;
-  const dim3 grid((unsigned)rows, (unsigned)((L + tables - 1) / tables));
-#define LSH_QUERY_LAUNCH(T, CodeT)                                                                 \
+#define LSH_QUERY_LAUNCH(T, CodeT, ROWS)                                                           \
   do {                                                                                             \
-    const int bytes = (D + 1) * LSH_COLS * (int)sizeof(T) + D * 4 + LSH_COLS;                      \
+    const dim3 grid((unsigned)((rows + ROWS - 1) / ROWS), (unsigned)chunks);                       \
+    const int bytes = (D + 1) * LSH_COLS * (int)sizeof(T) + ROWS * (D * 4 + LSH_COLS);             \
     if (bytes > 48 * 1024) {                                                                       \
-      cudaError_t e = cudaFuncSetAttribute(lsh_query_kernel<T, CodeT>,                             \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, LSH_COLS_SMEM(T)); \
+      cudaError_t e = cudaFuncSetAttribute(lsh_query_kernel<T, CodeT, ROWS>,                             \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, LSH_COLS_SMEM(T) + ROWS * (256 * 4 + LSH_COLS)); \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_query attr: %s", cudaGetErrorString(e)); \
     }                                                                                              \
-    sah_launch_chain(lsh_query_kernel<T, CodeT>, grid, LSH_COLS_THREADS, bytes, st, \
+    sah_launch_chain(lsh_query_kernel<T, CodeT, ROWS>, grid, LSH_COLS_THREADS, bytes, st, \
         reinterpret_cast<const T*>(q), qs_b, qs_h, qs_q, Hq, Sq, G, D,                             \
-        reinterpret_cast<const T*>(mean), reinterpret_cast<const T*>(proj), L, K,                  \
+        reinterpret_cast<const T*>(mean), reinterpret_cast<const T*>(proj), L, K, tables, rows,    \
         reinterpret_cast<CodeT*>(qcodes), qunit, reinterpret_cast<T*>(qhat), qmu);                 \
   } while (0)
   SAH_DISPATCH_DTYPE(dtype, T, {
-    if (K <= 8) LSH_QUERY_LAUNCH(T, uint8_t); else LSH_QUERY_LAUNCH(T, uint16_t);
+    const int tables = lsh_cta_tables<T>(K, L), chunks = (L + tables - 1) / tables;
+    // four rows per CTA from four CTAs per SM on
+    const bool four = rows * chunks > LSH_QUERY_FOUR;
+    if (K <= 8 && four) LSH_QUERY_LAUNCH(T, uint8_t, 4);
+    else if (K <= 8) LSH_QUERY_LAUNCH(T, uint8_t, 1);
+    else if (four) LSH_QUERY_LAUNCH(T, uint16_t, 4);
+    else LSH_QUERY_LAUNCH(T, uint16_t, 1);
   });
 #undef LSH_QUERY_LAUNCH
   SAH_LAUNCH_CHECK("lsh_query");
@@ -611,50 +644,94 @@ lsh_match_kernel(const CodeT* __restrict__ codes, int64_t cap, const CodeT* __re
   const int64_t word0 = ((int64_t)blockIdx.x * LSH_MATCH_WARPS + warp) * LSH_MATCH_WORDS;
   if (word0 * 32 >= S) return;
   const uint4* base = reinterpret_cast<const uint4*>(codes + bh * cap * LP);
+  const int64_t words = (S + 31) / 32;
+  // the four words of a mask row as one 16-byte access
+  const bool quad = W % 4 == 0 && word0 + LSH_MATCH_WORDS <= words && (reinterpret_cast<uintptr_t>(out_bits) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(prev_bits) & 15) == 0;
   // A key's row is read once for 64 query rows (once per four of them, at 16 query positions, took
-  // 187 us for 8 x 65500 keys; 165 us now, the integer instructions).
+  // 187 us for 8 x 65500 keys of 75 tables; 165 us now, the integer instructions).  A lane keeps the
+  // words of two query rows until all four are there and stores them together.  Of short signatures it
+  // reads all four words' keys before it starts on the queries, so that a query row read from shared
+  // memory serves four words (16 tables, 8 rows x 65500 keys: 9.6 us reading the keys once per four
+  // queries, 12.1 us word by word, 10.2 us this way; 64 rows x 16384 26.4, 26.2 and 17.2).
   for (int rb = 0; rb < R; rb += 64) {
     const int re = R - rb < 64 ? R - rb : 64;
-#pragma unroll 1
-    for (int j = 0; j < LSH_MATCH_WORDS; ++j) {
-      const int64_t word = word0 + j, key = word * 32 + lane;
-      if (word * 32 >= S) break;
-      uint4 v[NC];
+    uint32_t keep[2][LSH_MATCH_WORDS];  // lane l: the words of rows rb + l and rb + 32 + l
 #pragma unroll
-      for (int c = 0; c < NC; ++c) v[c] = key < S ? __ldg(base + key * NC + c) : make_uint4(0u, 0u, 0u, 0u);
-      uint32_t mine[2] = {0u, 0u};  // lane l keeps the words of rows rb + l and rb + 32 + l
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int j = 0; j < LSH_MATCH_WORDS; ++j) keep[n][j] = 0u;
+    constexpr int JW = NC <= 2 ? LSH_MATCH_WORDS : 1;  // words whose keys a lane holds at once
+#pragma unroll 1
+    for (int j0 = 0; j0 < LSH_MATCH_WORDS; j0 += JW) {
+      if ((word0 + j0) * 32 >= S) break;
+      uint4 v[JW][NC];
+      uint32_t mine[JW][2];
+#pragma unroll
+      for (int j = 0; j < JW; ++j) {
+        const int64_t key = (word0 + j0 + j) * 32 + lane;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) v[j][c] = key < S ? __ldg(base + key * NC + c) : make_uint4(0u, 0u, 0u, 0u);
+        mine[j][0] = mine[j][1] = 0u;
+      }
       for (int r0 = 0; r0 < re; r0 += 4) {
-        uint32_t hit[4] = {0u, 0u, 0u, 0u};
+        uint32_t hit[JW][4];
+#pragma unroll
+        for (int j = 0; j < JW; ++j)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) hit[j][r] = 0u;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             if (r0 + r < re) {
               const uint4 q = qs[(rb + r0 + r) * NC + c];
-              lsh_match_word<CodeT>(v[c].x ^ q.x, hit[r]);
-              lsh_match_word<CodeT>(v[c].y ^ q.y, hit[r]);
-              lsh_match_word<CodeT>(v[c].z ^ q.z, hit[r]);
-              lsh_match_word<CodeT>(v[c].w ^ q.w, hit[r]);
+#pragma unroll
+              for (int j = 0; j < JW; ++j) {
+                lsh_match_word<CodeT>(v[j][c].x ^ q.x, hit[j][r]);
+                lsh_match_word<CodeT>(v[j][c].y ^ q.y, hit[j][r]);
+                lsh_match_word<CodeT>(v[j][c].z ^ q.z, hit[j][r]);
+                lsh_match_word<CodeT>(v[j][c].w ^ q.w, hit[j][r]);
+              }
             }
           }
         }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const uint32_t wbits = __ballot_sync(0xffffffffu, lsh_matched<CodeT>(hit[r]) && key < S);
-          if (lane == ((r0 + r) & 31)) {
-            if (r0 + r < 32) mine[0] = wbits; else mine[1] = wbits;
+        for (int j = 0; j < JW; ++j) {
+          const bool live = (word0 + j0 + j) * 32 + lane < S;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const uint32_t wbits = __ballot_sync(0xffffffffu, lsh_matched<CodeT>(hit[j][r]) && live);
+            if (lane == ((r0 + r) & 31)) {
+              if (r0 + r < 32) mine[j][0] = wbits; else mine[j][1] = wbits;
+            }
           }
         }
       }
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        const int r = rb + n * 32 + lane;
-        if (n * 32 + lane < re) {
-          const int g = r / Sq, qi = r % Sq;
-          const int64_t row = ((b * Hq) + hkv * G + g) * Sq + qi;
-          uint32_t bits = mine[n];  // keys past S never set a bit
-          if (prev_bits != nullptr) bits |= prev_bits[row * W + word];
-          out_bits[row * W + word] = bits;
+      for (int j = 0; j < LSH_MATCH_WORDS; ++j)
+        if (JW == LSH_MATCH_WORDS || j == j0) {
+          keep[0][j] = mine[j % JW][0];
+          keep[1][j] = mine[j % JW][1];
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int r = rb + n * 32 + lane;
+      if (n * 32 + lane < re) {
+        const int g = r / Sq, qi = r % Sq;
+        const int64_t at = (((b * Hq) + hkv * G + g) * Sq + qi) * W + word0;  // keys past S never set a bit
+        if (quad) {
+          uint4 bits = make_uint4(keep[n][0], keep[n][1], keep[n][2], keep[n][3]);
+          if (prev_bits != nullptr) {
+            const uint4 p = *reinterpret_cast<const uint4*>(prev_bits + at);
+            bits = make_uint4(bits.x | p.x, bits.y | p.y, bits.z | p.z, bits.w | p.w);
+          }
+          *reinterpret_cast<uint4*>(out_bits + at) = bits;
+        } else {
+#pragma unroll
+          for (int j = 0; j < LSH_MATCH_WORDS; ++j)
+            if (word0 + j < words) out_bits[at + j] = keep[n][j] | (prev_bits != nullptr ? prev_bits[at + j] : 0u);
         }
       }
     }

@@ -465,3 +465,82 @@ def test_gpu_norms_of_many_keys_equal_those_of_few(S, scale, centred):
     dens(whole, 0, 0)
     dens(again, 1, 0)  # the maximum moved: every key, through the kernel of the decode step
     assert torch.equal(whole, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,L,K,D,B,Hq,Sq,centred", [
+    ("bf16", 75, 8, 128, 3, 7, 3, True), ("f32", 75, 8, 128, 1, 61, 1, False), ("bf16", 40, 10, 128, 5, 5, 5, True),
+    ("f32", 33, 7, 32, 3, 51, 1, True), ("f32", 21, 16, 256, 1, 101, 1, True), ("bf16", 64, 1, 64, 1, 601, 1, False)])
+def test_gpu_queries_by_fours_equal_single_ones(dtype, L, K, D, B, Hq, Sq, centred):
+    """Many query rows go four to a CTA, few one to a CTA: the same codes, unit vectors and constants,
+    with a last CTA of one to three rows, whatever the table width and the alignment of the
+    hyperplanes' rows."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    torch.manual_seed(L + D)
+    q = torch.randn((B, Sq, Hq, D), device=dev).to(dt).transpose(1, 2)
+    proj = torch.randn((D + 1, L * K), device=dev).to(dt)
+    mean = (0.2 * torch.randn((B * Hq, D), device=dev)).to(dt) if centred else None
+    code = torch.uint8 if K <= 8 else torch.int16
+
+    def query(b, h, s):
+        """rows of batch b, head h, position s; None: all"""
+        part = q if b is None else q[b:b + 1, h:h + 1, s:s + 1]
+        rows = part.shape[0] * part.shape[1] * part.shape[2]
+        m = mean if mean is None or b is None else mean[b * Hq + h:b * Hq + h + 1].contiguous()
+        out = (torch.zeros((rows, L), dtype=code, device=dev), torch.zeros((rows, D), device=dev),
+               torch.zeros((rows, D), dtype=dt, device=dev), torch.zeros(rows, device=dev))
+        _native.check(lib.sah_lsh_query(part.data_ptr(), _native.dtype_code(dt), part.stride(0), part.stride(1),
+                                        part.stride(2), part.shape[0], part.shape[1], part.shape[2], 1, D,
+                                        _native.ptr(m), proj.data_ptr(), L, K, *(t.data_ptr() for t in out),
+                                        _native.stream_of(torch.device(dev))), "sah_lsh_query")
+        return out
+
+    whole = query(None, None, None)
+    parts = [query(b, h, s) for b in range(B) for h in range(Hq) for s in range(Sq)]
+    assert B * Hq * Sq % 4 and B * Hq * Sq * -(-L // (64 // K)) > 592
+    for i, got in enumerate(whole):
+        assert torch.equal(got, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,K,G,Sq,S,pad,joined", [
+    (16, 2, 4, 2, 1003, 0, True), (75, 8, 4, 16, 4100, 0, False), (5, 8, 3, 11, 129, 1, True), (40, 10, 2, 33, 300, 2, True),
+    (16, 8, 5, 13, 31, 0, False), (9, 12, 1, 5, 128, 3, True), (75, 8, 1, 70, 2049, 0, True)])
+def test_gpu_matches_of_several_positions(L, K, G, Sq, S, pad, joined):
+    """More than four query rows per KV head: up to and over 64 of them, rows of the bitmap that end
+    inside a 16-byte store and that do not start on one, byte and halfword codes, with and without
+    the previous mask: every word that holds keys, and no other."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, cap = 2, 2, S + 6
+    dt, width = (torch.uint8, 1) if K <= 8 else (torch.int16, 2)
+    pitch = (L * width + 15) // 16 * 16 // width
+    gen = torch.Generator(device=dev).manual_seed(S)
+    top = 1 << min(K, 6)
+    codes = torch.zeros((B * Hkv, cap, pitch), dtype=dt, device=dev)
+    codes[..., :L] = torch.randint(0, top, (B * Hkv, cap, L), generator=gen, device=dev).to(dt)
+    qcodes = torch.randint(0, top, (B, Hkv * G, Sq, L), generator=gen, device=dev).to(dt)
+    rows, used = B * Hkv * G * Sq, (S + 31) // 32
+    W = (used + 3) // 4 * 4 + pad
+    prev = torch.randint(-2 ** 31, 2 ** 31 - 1, (rows, W), generator=gen, device=dev, dtype=torch.int64).to(torch.int32)
+    out = torch.full((rows, W), 0x5A5A5A5A, dtype=torch.int32, device=dev)
+    _native.check(lib.sah_lsh_match(codes.data_ptr(), cap, qcodes.data_ptr(), B, Hkv * G, Sq, G, L, K, S, W,
+                                    prev.data_ptr() if joined else None, out.data_ptr(),
+                                    _native.stream_of(torch.device(dev))), "sah_lsh_match")
+    k = codes[:, :S, :L].reshape(B, Hkv, 1, 1, S, L)
+    hit = torch.stack([(k == qcodes.reshape(B, Hkv, G, Sq, 1, L)[:, :, g:g + 1]).any(-1)[:, :, 0] for g in range(G)], 2)
+    bits = torch.zeros((rows, used * 32), dtype=torch.int64, device=dev)
+    bits[:, :S] = hit.reshape(rows, S)
+    words = (bits.reshape(rows, used, 32) << torch.arange(32, device=dev)).sum(-1)
+    if joined:
+        words |= prev[:, :used].long() & 0xFFFFFFFF
+    assert torch.equal(out[:, :used].long() & 0xFFFFFFFF, words)
+    assert bool((out[:, used:] == 0x5A5A5A5A).all()) and 0 < int(hit.sum()) < hit.numel()
