@@ -880,11 +880,9 @@ static int lsh_match_launch(const void* codes, int64_t cap, const void* qcodes, 
   case NC: {                                                                                        \
     constexpr int RSMEM = LSH_MATCH_WARPS * LSH_MATCH_REG_STAGES * 32 * NC * 16;                    \
     static bool allowed[64] = {};                                                                   \
-    if (RSMEM > 48 * 1024 && dev >= 0 && dev < 64 && !allowed[dev]) {                               \
-      cudaError_t e = cudaFuncSetAttribute(lsh_match_reg_kernel<CodeT, NC>,                         \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, RSMEM);     \
+    if (RSMEM + 4 * NC * 16 > 48 * 1024) {  /* beside the four query rows */                        \
+      const cudaError_t e = sah_allow_smem(lsh_match_reg_kernel<CodeT, NC>, RSMEM, allowed);        \
       if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_match attr: %s", cudaGetErrorString(e)); \
-      allowed[dev] = true;                                                                          \
     }                                                                                               \
     sah_launch_chain(lsh_match_reg_kernel<CodeT, NC>, rgrid, LSH_MATCH_WARPS * 32, RSMEM, st,       \
         reinterpret_cast<const CodeT*>(codes), cap, reinterpret_cast<const CodeT*>(qcodes), Hq, Sq, \

@@ -510,11 +510,13 @@ def test_gpu_queries_by_fours_equal_single_ones(dtype, L, K, D, B, Hq, Sq, centr
 @pytest.mark.gpu
 @pytest.mark.parametrize("L,K,G,Sq,S,pad,joined", [
     (16, 2, 4, 2, 1003, 0, True), (75, 8, 4, 16, 4100, 0, False), (5, 8, 3, 11, 129, 1, True), (40, 10, 2, 33, 300, 2, True),
-    (16, 8, 5, 13, 31, 0, False), (9, 12, 1, 5, 128, 3, True), (75, 8, 1, 70, 2049, 0, True)])
+    (16, 8, 5, 13, 31, 0, False), (9, 12, 1, 5, 128, 3, True), (75, 8, 1, 70, 2049, 0, True),
+    (40, 8, 4, 1, 1003, 0, True), (24, 12, 2, 2, 700, 1, False), (96, 8, 4, 1, 300, 0, True)])
 def test_gpu_matches_of_several_positions(L, K, G, Sq, S, pad, joined):
     """More than four query rows per KV head: up to and over 64 of them, rows of the bitmap that end
     inside a 16-byte store and that do not start on one, byte and halfword codes, with and without
-    the previous mask: every word that holds keys, and no other."""
+    the previous mask: every word that holds keys, and no other.  The last three have four rows and
+    signatures of 48 and 96 bytes, whose keys go through a ring in shared memory (48 KB at 48 bytes)."""
     import torch
     from sparse_attention_hub import _native
 
