@@ -201,11 +201,13 @@ def test_restatement_three_query_positions_under_a_causal_mask():
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,S,spread,top_p,masked", [
     (1, 131072, 25.0, 0.9, False), (2, 70001, 60.0, 0.999, True), (20, 16384, 4.0, 0.7, False),
-    (75, 2040, 300.0, 0.5, True), (150, 1031, 25.0, 0.95, True), (3, 40, 900.0, 0.9, False)])
+    (75, 2040, 300.0, 0.5, True), (150, 1031, 25.0, 0.95, True), (3, 40, 900.0, 0.9, False),
+    (1, 700001, 40.0, 0.9, True), (38, 164001, 12.0, 0.8, False)])
 def test_gpu_rows_shared_by_clusters_and_ragged_rows(rows, S, spread, top_p, masked):
     """Rows cut between 8, 4, 2 and 1 CTAs; lengths that end inside a bitmap byte (no 16-byte
     loads); flat rows (every add near a tie of the accumulator) and steep ones (weights down to
-    the denormals and 0); additive masks with the lowest value and -inf."""
+    the denormals and 0); additive masks with the lowest value and -inf; ranges too long for a CTA's shared
+    memory (the last two), whose logits every pass makes again."""
     from oracle.bf16 import round_bf16
 
     rng = np.random.default_rng(S)
