@@ -292,6 +292,9 @@ lsh_key_sign_kernel(const T* __restrict__ k, int64_t ks_b, int64_t ks_h, int64_t
       float acc[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+      // unrolled by eight, the loads of as many channels are on their way (left to itself the loop
+      // took 416 us for 64 heads x 4096 keys of 16 tables of 2 bits, 352 us this way)
+#pragma unroll 8
       for (int c = 0; c < Dp; ++c) {
         const float p = sah_to_float<T>(proj[(int64_t)c * nbits + o]);
         const float4 a = *reinterpret_cast<const float4*>(xt + c * LSH_KT + k8);
