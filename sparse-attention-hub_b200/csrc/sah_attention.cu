@@ -130,9 +130,11 @@ __global__ void attn_plan_count_kernel(const uint32_t* __restrict__ bits,
 // one per thread, up to four CTAs per group.  A CTA first counts the union bits of the words in
 // front of its own (a few loads per thread from a bitmap that is cache resident), then a single
 // ordered block scan places every word's entries; no second kernel and no chunk counters.
+// BANDS: the mask as its bands (an instantiation of its own: looked up at run time, bitmap or bands,
+// they cost every plan from a bitmap 0.7 us of 2.6 to 4, and 3.6 of 7.1 us with eight rows per group).
 #define PLAN_FUSED_THREADS 256
 
-template <typename T, int RMAX>
+template <typename T, int RMAX, bool BANDS>
 __global__ void __launch_bounds__(PLAN_FUSED_THREADS)
 attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ data,
                        const int32_t* __restrict__ wpre, const int64_t* __restrict__ ptr,
@@ -143,7 +145,8 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
   // word of a mask row: from the bitmap, or (no bitmap) from the mask's bands; those are written
   // out as a bitmap for whoever reads the mask later, if there is a place for it
   auto row_word = [&](int64_t row, int64_t wi) -> uint32_t {
-    return bits != nullptr ? bits[row * p.W + wi] : sah_band_bits(bands, row % p.Sq, wi * 32, 32, p.S, 0u);
+    if constexpr (BANDS) return sah_band_bits(bands, row % p.Sq, wi * 32, 32, p.S, 0u);
+    else return bits[row * p.W + wi];
   };
   __shared__ int scan[33];
   __shared__ int64_t rows_sm[RMAX];
@@ -177,7 +180,7 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
       if (uw != nullptr && words[r]) dbase[r] = ptr[rows[r]] + wpre[rows[r] * p.W + w];
     }
     u |= words[r];
-    if (band_bits != nullptr && w < p.W && rows[r] >= 0) band_bits[rows[r] * p.W + w] = words[r];
+    if (BANDS && band_bits != nullptr && w < p.W && rows[r] >= 0) band_bits[rows[r] * p.W + w] = words[r];
   }
   int base = 0;
   if (w0 > 0) {
@@ -225,7 +228,8 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
 // ([groups][S]) the key's constant of the cosine, 1 / (M * |transformed key|).
 #define PLAN_EMIT_WARPS 4
 
-template <typename T, int RMAX, bool LSH>
+// BATCH: per-entry weights of up to four rows, the entries of eight words requested together.
+template <typename T, int RMAX, bool LSH, bool BATCH>
 __global__ void __launch_bounds__(PLAN_EMIT_WARPS * 32)
 attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ ubits,
                       const T* __restrict__ data, const int32_t* __restrict__ wpre,
@@ -251,7 +255,7 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
   for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
 
   const int64_t w = c * PLAN_CHUNK_WORDS + lane;
-  const bool weighted = !LSH && uw != nullptr;
+  const bool weighted = BATCH || (!LSH && uw != nullptr);
   uint32_t u = 0u;
 #pragma unroll
   for (int r = 0; r < RMAX; ++r) {
@@ -299,12 +303,17 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
       dcol[j] = col < p.S ? __ldg(gd + col) : 1.f;
     }
   }
-  if (!LSH && RMAX == 4 && weighted) {
-    // Weights: the entries of eight words are requested together and then written (one dependent
+  if constexpr (BATCH) {
+    // The entries of eight words are requested together and then written (one dependent
     // load per word and row in turn took 44 us for 32 groups x 65536 keys, 7 % of them selected;
-    // 27 us this way).
+    // 27 us this way; in one instantiation with the plans without weights it made those slower, 64
+    // groups x 131072 keys 25.5 -> 29.2 us).
 #pragma unroll 1
     for (int j0 = 0; j0 < 32; j0 += 8) {
+      uint32_t any = 0u;
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) any |= union_sm[wl][j0 + jj];
+      if (any == 0u) continue;  // the same for every lane
       T raw[8][RMAX];
 #pragma unroll
       for (int jj = 0; jj < 8; ++jj)
@@ -411,14 +420,16 @@ static int attn_plan_impl(const uint32_t* bits, const MaskBands& bands, const vo
     return sah_fail(SAH_ERR_UNSUPPORTED, "attn_plan_bands: %lld keys (at most 32768)", (long long)S);
   if (p.Wv <= 1024) {
     const dim3 fgrid((unsigned)groups, (unsigned)sah_ceil_div(p.Wv, PLAN_FUSED_THREADS));
+#define PLAN_FUSED_LAUNCH(RMAX, BANDS)                                                                    \
+  sah_launch_chain(attn_plan_fused_kernel<T, RMAX, BANDS>, fgrid, PLAN_FUSED_THREADS, 0, st, bits,         \
+      (const T*)data, wpre, ptr, p, bands, band_bits, ucols, umemb, data ? uw : nullptr, ucount)
     SAH_DISPATCH_DTYPE(dtype, T, {
-      if (p.R <= 4)
-        sah_launch_chain(attn_plan_fused_kernel<T, 4>, fgrid, PLAN_FUSED_THREADS, 0, st, bits, (const T*)data,
-            wpre, ptr, p, bands, band_bits, ucols, umemb, data ? uw : nullptr, ucount);
-      else
-        sah_launch_chain(attn_plan_fused_kernel<T, AT_MAXR>, fgrid, PLAN_FUSED_THREADS, 0, st, bits,
-            (const T*)data, wpre, ptr, p, bands, band_bits, ucols, umemb, data ? uw : nullptr, ucount);
+      if (bits != nullptr && p.R <= 4) PLAN_FUSED_LAUNCH(4, false);
+      else if (bits != nullptr) PLAN_FUSED_LAUNCH(AT_MAXR, false);
+      else if (p.R <= 4) PLAN_FUSED_LAUNCH(4, true);
+      else PLAN_FUSED_LAUNCH(AT_MAXR, true);
     });
+#undef PLAN_FUSED_LAUNCH
     SAH_LAUNCH_CHECK("attn_plan_fused");
     sah_prof_end(SAH_PROF_ATTN_PLAN, (cudaStream_t)stream);
     return SAH_OK;
@@ -426,16 +437,16 @@ static int attn_plan_impl(const uint32_t* bits, const MaskBands& bands, const vo
   sah_launch_chain(attn_plan_count_kernel, (unsigned)blocks, threads, 0, st, bits, nullptr, p, chunkcnt);
   SAH_LAUNCH_CHECK("attn_plan_count");
   const int64_t eblocks = sah_ceil_div(warps, PLAN_EMIT_WARPS);
+#define PLAN_EMIT_LAUNCH(RMAX, BATCH)                                                                     \
+  sah_launch_chain(attn_plan_emit_kernel<T, RMAX, false, BATCH>, (unsigned)eblocks, PLAN_EMIT_WARPS * 32, 0, \
+      st, bits, nullptr, (const T*)data, wpre, ptr, nullptr, 0, nullptr, p, chunkcnt, ucols, umemb,         \
+      data ? uw : nullptr, ucount)
   SAH_DISPATCH_DTYPE(dtype, T, {
-    if (p.R <= 4)
-      sah_launch_chain(attn_plan_emit_kernel<T, 4, false>, (unsigned)eblocks, PLAN_EMIT_WARPS * 32, 0, st,
-          bits, nullptr, (const T*)data, wpre, ptr, nullptr, 0, nullptr, p, chunkcnt, ucols, umemb,
-          data ? uw : nullptr, ucount);
-    else
-      sah_launch_chain(attn_plan_emit_kernel<T, AT_MAXR, false>, (unsigned)eblocks, PLAN_EMIT_WARPS * 32, 0,
-          st, bits, nullptr, (const T*)data, wpre, ptr, nullptr, 0, nullptr, p, chunkcnt, ucols, umemb,
-          data ? uw : nullptr, ucount);
+    if (p.R <= 4 && data != nullptr) PLAN_EMIT_LAUNCH(4, true);
+    else if (p.R <= 4) PLAN_EMIT_LAUNCH(4, false);
+    else PLAN_EMIT_LAUNCH(AT_MAXR, false);
   });
+#undef PLAN_EMIT_LAUNCH
   SAH_LAUNCH_CHECK("attn_plan_emit");
   sah_prof_end(SAH_PROF_ATTN_PLAN, (cudaStream_t)stream);
   return SAH_OK;
@@ -504,7 +515,7 @@ extern "C" int sah_attn_plan_lsh(const uint32_t* bits, const uint32_t* unit_bits
   sah_prof_begin(SAH_PROF_ATTN_PLAN, st);
   sah_launch_chain(attn_plan_count_kernel, (unsigned)blocks, threads, 0, st, bits, unit_bits, p, chunkcnt);
   SAH_LAUNCH_CHECK("attn_plan_count");
-  sah_launch_chain(attn_plan_emit_kernel<float, 4, true>, (unsigned)sah_ceil_div(warps, PLAN_EMIT_WARPS),
+  sah_launch_chain(attn_plan_emit_kernel<float, 4, true, false>, (unsigned)sah_ceil_div(warps, PLAN_EMIT_WARPS),
                    PLAN_EMIT_WARPS * 32, 0, st, bits, unit_bits, nullptr, nullptr, nullptr, dens, dens_cap,
                    max_norm_bits, p, chunkcnt, ucols, umemb, uinv, ucount);
   SAH_LAUNCH_CHECK("attn_plan_emit_lsh");
