@@ -11,8 +11,9 @@
 // list, cut between units of HE_GROUPS tiles of one head, or of two tiles or one as long as every
 // unit has an SM to itself: staging takes about 10 us, and a tile alone on an SM 12 us less than
 // four (cut anywhere, with four tiles per CTA, the heads of a short range shared CTAs in turn: 97 us
-// for 32 heads x 17 to 32 vectors, 26 us now; 64 to 256 vectors 38 to 59 us, 26 us now).  Four groups of two warps each take a tile at a time, with barriers of their own, so that
-// one group's rounding, activation look-ups and stores run under another's multiply-adds.
+// for 32 heads x 17 to 32 vectors, 26 us now; 64 to 256 vectors 38 to 59 us, 26 us now).  Four groups
+// of two warps each take a tile at a time, with barriers of their own, so that one group's rounding,
+// activation look-ups and stores run under another's multiply-adds.
 // Activations are fp32 [channel][vector] and overwritten layer by layer.
 //
 // One layer is a register-tiled product in which every output has a single fp32 accumulator
@@ -23,8 +24,8 @@
 // whose 64 multiply-adds need four broadcast reads of activations and one of weights.
 // 32 heads x 16384 keys through 128-128-128-32: 1963 us with tiles of 64 vectors, 8 x 4 outputs
 // per thread, scalar fma and the weights staged per tile; 981 us with one tile of 128 vectors per
-// CTA; 907 us in groups, 863 us with the channel loop unrolled eight times, 851 us sixteen times
-// (19.3 G multiply-adds; 540 us at 128 per clock and SM).
+// CTA; 907 us in groups, 863 us with the channel loop unrolled eight times, 851 us sixteen times,
+// 811 us with the list walked in 32-bit arithmetic (19.3 G multiply-adds; 540 us at 128 per clock and SM).
 // ---------------------------------------------------------------------------
 #define HE_TK 32        // vectors per tile
 #define HE_GT 64        // threads per group
@@ -430,7 +431,7 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
   // bfloat16, about 31 % of the accumulators lie within the error band of a rounding midpoint, so
   // nearly every warp repeats nearly every output in the fixed order and the build took 2.6x to
   // 4.6x as long as hash_encode_kernel did at 52 ms for 8 x 32768 keys x 32 heads (134 ms), which
-  // has halved since.
+  // has become 2.3x faster since.
   const char* tc_e = getenv("SAH_HASH_TC");
   const int tc_env = (tc_e != nullptr && tc_e[0] == '1') ? 1 : 0;
   bool tc = tc_env == 1 && dtype == SAH_BF16 && n_layers <= HTC_MAX_LAYERS && n_end - n_begin >= 1024 &&
