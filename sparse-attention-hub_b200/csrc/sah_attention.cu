@@ -228,7 +228,9 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
 // ([groups][S]) the key's constant of the cosine, 1 / (M * |transformed key|).
 #define PLAN_EMIT_WARPS 4
 
-// BATCH: per-entry weights of up to four rows, the entries of eight words requested together.
+// BATCH: per-entry weights of up to four rows, the entries of eight words requested together.  Without
+// it four rows have none (their code in the unrolled loop is fetched for nothing: 4 us of a decode step's
+// 23, whose instruction cache is cold); more rows ask at run time.
 template <typename T, int RMAX, bool LSH, bool BATCH>
 __global__ void __launch_bounds__(PLAN_EMIT_WARPS * 32)
 attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ ubits,
@@ -255,7 +257,7 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
   for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
 
   const int64_t w = c * PLAN_CHUNK_WORDS + lane;
-  const bool weighted = BATCH || (!LSH && uw != nullptr);
+  const bool weighted = BATCH || (!LSH && RMAX > 4 && uw != nullptr);
   uint32_t u = 0u;
 #pragma unroll
   for (int r = 0; r < RMAX; ++r) {
