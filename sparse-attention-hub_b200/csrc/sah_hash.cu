@@ -431,7 +431,7 @@ extern "C" int sah_hash_encode(const void* x, int dtype, int64_t xs_b, int64_t x
   // bfloat16, about 31 % of the accumulators lie within the error band of a rounding midpoint, so
   // nearly every warp repeats nearly every output in the fixed order and the build took 2.6x to
   // 4.6x as long as hash_encode_kernel did at 52 ms for 8 x 32768 keys x 32 heads (134 ms), which
-  // has become 2.3x faster since.
+  // has become 2.4x faster since.
   const char* tc_e = getenv("SAH_HASH_TC");
   const int tc_env = (tc_e != nullptr && tc_e[0] == '1') ? 1 : 0;
   bool tc = tc_env == 1 && dtype == SAH_BF16 && n_layers <= HTC_MAX_LAYERS && n_end - n_begin >= 1024 &&
