@@ -228,7 +228,7 @@ attn_plan_fused_kernel(const uint32_t* __restrict__ bits, const T* __restrict__ 
 // ([groups][S]) the key's constant of the cosine, 1 / (M * |transformed key|).
 #define PLAN_EMIT_WARPS 4
 
-// BATCH: per-entry weights of up to four rows, the entries of eight words requested together.  Without
+// BATCH: per-entry weights of up to four rows, the entries of four words requested together.  Without
 // it four rows have none (their code in the unrolled loop is fetched for nothing: 4 us of a decode step's
 // 23, whose instruction cache is cold); more rows ask at run time.
 template <typename T, int RMAX, bool LSH, bool BATCH>
@@ -306,19 +306,19 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
     }
   }
   if constexpr (BATCH) {
-    // The entries of eight words are requested together and then written (one dependent
-    // load per word and row in turn took 44 us for 32 groups x 65536 keys, 7 % of them selected;
-    // 27 us this way; in one instantiation with the plans without weights it made those slower, 64
-    // groups x 131072 keys 25.5 -> 29.2 us).
+    // The entries of four words are requested together and then written (one dependent load per word
+    // and row in turn took 34 us for 8 groups x 65536 keys, 10 % of them selected, and 44 us for 64
+    // groups; 26 and 40 us this way).  Eight words together need 96 registers, which holds two waves of
+    // CTAs where this is one and a half: 64 groups 56 us.
 #pragma unroll 1
-    for (int j0 = 0; j0 < 32; j0 += 8) {
+    for (int j0 = 0; j0 < 32; j0 += 4) {
       uint32_t any = 0u;
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) any |= union_sm[wl][j0 + jj];
+      for (int jj = 0; jj < 4; ++jj) any |= union_sm[wl][j0 + jj];
       if (any == 0u) continue;  // the same for every lane
-      T raw[8][RMAX];
+      T raw[4][RMAX];
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj)
+      for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
         for (int r = 0; r < RMAX; ++r) {
           const uint32_t wd = words_sm[wl][r][j0 + jj];
@@ -326,7 +326,7 @@ attn_plan_emit_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restr
           if ((wd >> lane) & 1u) raw[jj][r] = data[dbase_sm[wl][r][j0 + jj] + __popc(wd & lt)];
         }
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
+      for (int jj = 0; jj < 4; ++jj) {
         const int j = j0 + jj;
         const uint32_t uj = union_sm[wl][j];
         if (!((uj >> lane) & 1u)) continue;
