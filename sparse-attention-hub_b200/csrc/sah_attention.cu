@@ -15,6 +15,9 @@
 #define AT_THREADS 128
 #define AT_STAGES 3
 #define AT_MAXR 16
+// fp32 kernel: below this many tiles per CTA, one wave of CTAs instead of two (32 heads x 16384 keys of
+// which a head selects 968: 24.8 us with all 64 CTAs of a group, most of them with one tile, 15.8 us so)
+#define AT_ONE_WAVE_TILES 4
 #define PLAN_CHUNK_WORDS 32  // one warp scans 32 bitmap words = 1024 columns
 
 // Chunk counters per group: a function of the key count alone, so that the plan, the
@@ -559,6 +562,8 @@ struct AttnArgs {
   // TMA copy stage: K and V as 2-D [rows][D] tensors, row = b * rows_b + h * rows_h + key
   int64_t k_rows_b, k_rows_h, v_rows_b, v_rows_h;
   int k_rows_total, v_rows_total;
+  int wave;            // CTAs per group that the device holds at once, two per SM
+  int group_major;     // grid: 1 the splits of a group side by side, 0 the groups
   int one_wave_tiles;  // tcgen05 kernel: tiles per CTA below which only half of the grid works
 };
 
@@ -602,8 +607,8 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
   int* cols_sm = reinterpret_cast<int*>(alpha_sm + RP);  // [STAGES][TILE]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int split = blockIdx.x;
-  const int64_t g = blockIdx.y;
+  const int split = blockIdx.y;
+  const int64_t g = blockIdx.x;
   const int qb = (int)(g % a.nqb);
   const int64_t bk = g / a.nqb;
   const int kvh = (int)(bk % a.Hkv);
@@ -615,13 +620,16 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
   const uint16_t* gmemb = a.umemb + g * a.S;
   const float* guw = a.uw ? a.uw + g * a.S * a.R : nullptr;
 
-  // this CTA's slice of the group's union list
+  // this CTA's slice of the group's union list: whole tiles, shared evenly by as many CTAs as there
+  // are tiles, or as one wave of the device has for the group
   const int U = a.ucount[g];
-  int per = (U + a.nsplit - 1) / a.nsplit;
-  per = ((per + C::TILE - 1) / C::TILE) * C::TILE;
-  int start = split * per;
-  if (start > U) start = U;
-  int end = start + per;
+  const int total_tiles = (U + C::TILE - 1) / C::TILE;
+  int active = total_tiles < a.nsplit ? total_tiles : a.nsplit;
+  if (active > a.wave && total_tiles < a.nsplit * AT_ONE_WAVE_TILES) active = a.wave;
+  if (active < 1) active = 1;
+  if (split >= active) return;
+  const int start = (int)((int64_t)total_tiles * split / active) * C::TILE;
+  int end = (int)((int64_t)total_tiles * (split + 1) / active) * C::TILE;
   if (end > U) end = U;
   const int ntiles = (end - start + C::TILE - 1) / C::TILE;
 
@@ -869,10 +877,8 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
     pout[tid * (D + 2) + D] = m_sm[tid];
     pout[tid * (D + 2) + D + 1] = l_sm[tid];
   }
-  // the last CTA of the group to get here merges the splits and writes the output rows (every
-  // CTA of the grid writes a partial, an empty one included)
-  __syncthreads();  // the reduction buffer is read no more: it becomes the merge scratch
-  atm_finish_group<D, AT_THREADS, T>(a, g, a.nsplit, stage_base, &is_last_sm, tickets, sinks, out, part_out);
+  // the last CTA of the group to get here merges the splits and writes the output rows
+  atm_finish_group<D, AT_THREADS, D / 64, T>(a, g, active, &is_last_sm, tickets, sinks, out, part_out);
 }
 
 template <typename T, int D>
@@ -886,10 +892,9 @@ static int launch_attention(const AttnArgs& a, int groups, int* tickets, const f
                                  (size_t)C::TILE * RP + 3 * RP) +
                 sizeof(int) * AT_STAGES * C::TILE;
   size_t red = sizeof(float) * 4 * RP * D;
-  if (red > (size_t)AT_STAGES * C::STAGE_BYTES ||
-      sizeof(float) * (16 * (size_t)a.nsplit + 32) > (size_t)AT_STAGES * C::STAGE_BYTES)
+  if (red > (size_t)AT_STAGES * C::STAGE_BYTES)
     return sah_fail(SAH_ERR_UNSUPPORTED, "attention: reduction buffer does not fit");
-  dim3 grid((unsigned)a.nsplit, (unsigned)groups);
+  dim3 grid((unsigned)groups, (unsigned)a.nsplit);
 #define SAH_AT_LAUNCH(NQ)                                                                        \
   {                                                                                              \
     cudaError_t e = cudaFuncSetAttribute(masked_attention_kernel<T, D, NQ>,                      \
@@ -906,6 +911,11 @@ static int launch_attention(const AttnArgs& a, int groups, int* tickets, const f
   }
 #undef SAH_AT_LAUNCH
   return SAH_OK;
+}
+
+static int attn_wave(int groups) {
+  const int per_group = 2 * aum_sm_count() / groups;
+  return per_group < 1 ? 1 : per_group;
 }
 
 struct AttnLsh {
@@ -955,8 +965,9 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
   a.w_dump = lsh ? lsh->w_dump : nullptr;
   a.k_rows_b = a.k_rows_h = a.v_rows_b = a.v_rows_h = 0;
   a.k_rows_total = a.v_rows_total = 0;
-  a.one_wave_tiles = 0;
+  a.one_wave_tiles = a.group_major = 0;
   const int groups = sizes->groups;
+  a.wave = attn_wave(groups);
   SAH_REQUIRE((int64_t)groups == (int64_t)B * Hkv * a.nqb && a.R == a.G * a.q_block &&
                   a.R <= AT_MAXR && a.nsplit >= 1,
               "masked_attention: sizes do not match the extents");
@@ -1110,8 +1121,10 @@ extern "C" int sah_attn_gather_probe(const void* k, const void* v, int64_t ks_b,
   a.nsplit = sizes->nsplit;
   a.S = S;
   a.ucols = ucols; a.ucount = ucount;
+  a.wave = attn_wave(sizes->groups);
   SAH_REQUIRE((int64_t)sizes->groups == (int64_t)B * Hkv * a.nqb,
               "attn_gather_probe: sizes do not match the extents");
+  a.group_major = 1;
   dim3 grid((unsigned)a.nsplit, (unsigned)sizes->groups);
   cudaStream_t st = (cudaStream_t)stream;
   static bool allowed[2][64] = {};

@@ -45,7 +45,10 @@
 #endif
 #define ATM_THREADS (ATM_WARPS * 32)
 #define ATM_TILE 16
-#define ATM_MIN_TILES 8        // tiles a warp should have before a further CTA joins the group
+// Tiles a warp should have before a further CTA joins the group: a tile takes a warp 0.8 us, a further
+// split the merge next to nothing (8 tiles 13.2 us, 4 tiles 10.6, 2 tiles and 1 tile 9.1, 32 heads x 8191
+// keys, 90 tiles per group; 131072 keys, 560 tiles per group: 19.3, 16.1, 15.9, 15.9 us).
+#define ATM_MIN_TILES 2
 #define ATM_ONE_WAVE_TILES 48  // below this many tiles per warp, one wave of CTAs instead of two
 #define ATM_FINE_SPLITS 16     // ... when the grid has at least this many CTAs per group
 
@@ -110,12 +113,12 @@ __device__ __forceinline__ uint32_t atm_pack_bf16(float lo, float hi) {
 // CTAs that share one group's union list.  The grid holds nsplit per group: two waves of the
 // device for long lists (the second wave evens out groups of different length).  When the
 // groups are few (nsplit >= ATM_FINE_SPLITS) and a list would give a warp fewer than
-// ATM_ONE_WAVE_TILES tiles in that arrangement, half of the CTAs work on it: one wave, half as
-// many pipeline fills and partials.  A short list is shared by as few CTAs as give every warp
+// ATM_ONE_WAVE_TILES tiles in that arrangement, one wave of CTAs (`wave` per group) works on it:
+// half as many pipeline fills and partials.  A short list is shared by as few CTAs as give every warp
 // a run of ATM_MIN_TILES tiles; the others leave at once (they hold no ticket).
-__device__ __forceinline__ int atm_active_splits(int total_tiles, int nsplit) {
+__device__ __forceinline__ int atm_active_splits(int total_tiles, int nsplit, int wave) {
   int active = nsplit;
-  if (nsplit >= ATM_FINE_SPLITS && total_tiles < nsplit * ATM_WARPS * ATM_ONE_WAVE_TILES) active = nsplit / 2;
+  if (nsplit >= ATM_FINE_SPLITS && wave < nsplit && total_tiles < nsplit * ATM_WARPS * ATM_ONE_WAVE_TILES) active = wave;
   const int by_length = (total_tiles + ATM_WARPS * ATM_MIN_TILES - 1) / (ATM_WARPS * ATM_MIN_TILES);
   if (by_length < active) active = by_length;
   return active < 1 ? 1 : active;
@@ -157,8 +160,7 @@ __device__ __forceinline__ float atm_lsh_weight(float dot_hat, float qmu, float 
 // mask row).  It takes a ticket; the last CTA of the group to arrive merges the `active`
 // partials of the group, applies the sink logits and writes the output rows (and, when
 // `part_out` is given, the group's merged partial for a merge across sequence shards).
-// Called by all NT threads of the CTA; `scratch` is shared memory the CTA no longer needs
-// (16 * active + 32 floats).
+// Called by all NT threads of the CTA.
 __device__ __forceinline__ void atm_store2(__nv_bfloat16* p, float x, float y) {
   *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);
 }
@@ -166,73 +168,82 @@ __device__ __forceinline__ void atm_store2(float* p, float x, float y) {
   *reinterpret_cast<float2*>(p) = make_float2(x, y);
 }
 
-template <int D, int NT, typename OutT>
-__device__ __forceinline__ void atm_finish_group(const AttnArgs& a, int64_t g, int active,
-                                                 unsigned char* scratch, int* is_last_sm,
+// A warp takes a mask row, its lanes over the dims (PAIRS pairs each; where there are more warps than
+// rows, one: half of a row of 128): the splits' maxima and denominators (lane = split) and the accumulators of up to sixteen splits are requested together, so
+// a merge of few splits is one round trip to L2 and no barrier; the rescale factors go round by
+// shuffles.  (Three dependent round trips and two barriers took 5 to 6 us of a launch's 15 to 19 us:
+// 32 heads x 8191 bfloat16 keys of which a head selects 800, 16.3 us before, 13.2 us with this merge
+// and the first copies issued in front of the queries; 10.0 us with ATM_MIN_TILES lowered to 2 as well.)
+template <int D, int NT, int PAIRS, typename OutT>
+__device__ __forceinline__ void atm_finish_group(const AttnArgs& a, int64_t g, int active, int* is_last_sm,
                                                  int* __restrict__ tickets, const float* __restrict__ sinks,
                                                  OutT* __restrict__ out,
                                                  float* __restrict__ part_out) {
+  constexpr int V = PAIRS;            // pairs of dims per lane, 64 apart
+  constexpr int PARTS = D / 64 / V;   // warps per row
+  constexpr int AHEAD = 16;  // splits requested together
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int qb = (int)(g % a.nqb);
   const int64_t bk = g / a.nqb;
   const int kvh = (int)(bk % a.Hkv);
   const int64_t b = bk / a.Hkv;
-  __threadfence();
-  __syncthreads();
+  __syncthreads();  // the CTA's partial is stored
   if (tid == 0) {
-    const int old = atomicAdd(&tickets[g], 1);
-    const int last = (old == active - 1);
+    __threadfence();
+    const int last = atomicAdd(&tickets[g], 1) == active - 1;
     if (last) tickets[g] = 0;  // ready for the next call
+    __threadfence();
     *is_last_sm = last;
   }
   __syncthreads();
   if (!*is_last_sm) return;
-  __threadfence();
-  const float* p0 = a.partial + (int64_t)g * a.nsplit * a.R * (D + 2);
   const int64_t pstride = (int64_t)a.R * (D + 2);
-  // phase 1: one warp per row finds the row maximum, the per-split rescale
-  // factors and the denominator
-  float* sc_sm = reinterpret_cast<float*>(scratch);  // [R][active]
-  float* ml_sm = sc_sm + 16 * active;                // [R][2]
-  for (int r = warp; r < a.R; r += NT / 32) {
-    const float* pr = p0 + (int64_t)r * (D + 2);
-    float mloc = -INFINITY;
-    for (int s2 = lane; s2 < active; s2 += 32) mloc = fmaxf(mloc, __ldcg(pr + s2 * pstride + D));
-#pragma unroll
-    for (int of = 16; of > 0; of >>= 1) mloc = fmaxf(mloc, __shfl_xor_sync(0xffffffffu, mloc, of));
-    float lsum = 0.f;
-    for (int s2 = lane; s2 < active; s2 += 32) {
-      const float ms = __ldcg(pr + s2 * pstride + D);
-      const float sc = (ms == -INFINITY) ? 0.f : __expf(ms - mloc);
-      sc_sm[r * active + s2] = sc;
-      lsum += __ldcg(pr + s2 * pstride + D + 1) * sc;
-    }
-#pragma unroll
-    for (int of = 16; of > 0; of >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, of);
-    if (lane == 0) {
-      ml_sm[r * 2] = mloc;
-      ml_sm[r * 2 + 1] = lsum;
-    }
-  }
-  __syncthreads();
-  // phase 2: every thread owns (row, pair of dims) items and sums them over the splits with
-  // 8-byte loads, eight in flight
-  for (int idx = tid; idx < a.R * (D / 2); idx += NT) {
-    const int r = idx / (D / 2), d = (idx - r * (D / 2)) * 2;
+  for (int item = warp; item < a.R * PARTS; item += NT / 32) {
+    const int r = item / PARTS, d0 = (item - r * PARTS) * 64 + lane * 2;
     const int gi = r / a.q_block, qo = r - gi * a.q_block;
     const int qi = qb * a.q_block + qo;
-    if (qi >= a.Sq) continue;
+    if (qi >= a.Sq) continue;  // the same for the whole warp
     const int h = kvh * a.G + gi;
-    const float* pr = p0 + (int64_t)r * (D + 2) + d;
-    const float* sc = sc_sm + r * active;
-    float2 accv = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int s2 = 0; s2 < active; ++s2) {
-      const float2 x = __ldcg(reinterpret_cast<const float2*>(pr + s2 * pstride));
-      accv.x = fmaf(x.x, sc[s2], accv.x);
-      accv.y = fmaf(x.y, sc[s2], accv.y);
+    const float* pr = a.partial + (int64_t)g * a.nsplit * pstride + (int64_t)r * (D + 2);
+    float M = -INFINITY, L = 0.f;
+    float2 acc[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = make_float2(0.f, 0.f);
+    for (int s0 = 0; s0 < active; s0 += AHEAD) {
+      const float* p0 = pr + s0 * pstride;
+      const int n = active - s0 < AHEAD ? active - s0 : AHEAD;
+      float2 ml = make_float2(-INFINITY, 0.f);
+      if (lane < n) ml = __ldcg(reinterpret_cast<const float2*>(p0 + lane * pstride + D));
+      float2 x[AHEAD][V];
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          x[i][v] = i < n ? __ldcg(reinterpret_cast<const float2*>(p0 + i * pstride + v * 64 + d0))
+                          : make_float2(0.f, 0.f);
+      float mx = ml.x;
+#pragma unroll
+      for (int of = AHEAD / 2; of > 0; of >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, of));
+      mx = fmaxf(__shfl_sync(0xffffffffu, mx, 0), M);
+      const float old = (M == -INFINITY) ? 0.f : __expf(M - mx);
+      const float sc = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - mx);
+      float l = ml.y * sc;
+#pragma unroll
+      for (int of = AHEAD / 2; of > 0; of >>= 1) l += __shfl_xor_sync(0xffffffffu, l, of);
+      L = L * old + __shfl_sync(0xffffffffu, l, 0);
+      M = mx;
+#pragma unroll
+      for (int v = 0; v < V; ++v) { acc[v].x *= old; acc[v].y *= old; }
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        const float si = __shfl_sync(0xffffffffu, sc, i);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          acc[v].x = fmaf(x[i][v].x, si, acc[v].x);
+          acc[v].y = fmaf(x[i][v].y, si, acc[v].y);
+        }
+      }
     }
-    const float M = ml_sm[r * 2], L = ml_sm[r * 2 + 1];
     float Mx = M, sink_term = 0.f;
     if (sinks != nullptr) {
       const float sk = sinks[h];
@@ -242,12 +253,14 @@ __device__ __forceinline__ void atm_finish_group(const AttnArgs& a, int64_t g, i
     const float resc = (M == -INFINITY) ? 0.f : __expf(M - Mx);
     const float den = L * resc + sink_term;
     const int64_t row = (b * a.Hq + h) * a.Sq + qi;
-    if (part_out != nullptr) *reinterpret_cast<float2*>(part_out + row * (D + 2) + d) = accv;
-    atm_store2(out + ((b * a.Sq + qi) * a.Hq + h) * D + d, accv.x * resc / den, accv.y * resc / den);
-    if (part_out != nullptr && d == 0) {
-      part_out[row * (D + 2) + D] = M;
-      part_out[row * (D + 2) + D + 1] = L;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const int d = v * 64 + d0;
+      if (part_out != nullptr) *reinterpret_cast<float2*>(part_out + row * (D + 2) + d) = acc[v];
+      atm_store2(out + ((b * a.Sq + qi) * a.Hq + h) * D + d, acc[v].x * resc / den, acc[v].y * resc / den);
     }
+    if (part_out != nullptr && d0 == 0)
+      *reinterpret_cast<float2*>(part_out + row * (D + 2) + D) = make_float2(M, L);
   }
 }
 
@@ -273,12 +286,14 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
     atm_smem = atm_smem_raw + (((raw_s + 1023u) & ~1023u) - raw_s);
   }
   unsigned char* ring = atm_smem + warp * C::WARP_BYTES;
-  unsigned char* q_sm = atm_smem;  // the first ring, before any copy is issued
+  // the stage of the first ring that the first copies do not fill
+  unsigned char* q_sm = atm_smem + (NST - 1) * C::STAGE_BYTES;
   unsigned char* meta_base = atm_smem + ATM_WARPS * C::WARP_BYTES;
   int4* meta_sm = reinterpret_cast<int4*>(meta_base) + warp * NST * 16;
   const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
   const uint32_t bar_s = (uint32_t)__cvta_generic_to_shared(meta_base + C::META_BYTES) + warp * NST * 8;
   __shared__ int is_last_sm;
+  __shared__ float2 ml_sm[ATM_WARPS][16];  // maximum and denominator of every warp's rows
   if constexpr (TMA) {
     if (lane == 0) {
 #pragma unroll
@@ -287,8 +302,8 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
     }
   }
 
-  const int split = blockIdx.x;
-  const int64_t g = blockIdx.y;
+  const int split = a.group_major ? blockIdx.x : blockIdx.y;
+  const int64_t g = a.group_major ? blockIdx.y : blockIdx.x;
   const int qb = (int)(g % a.nqb);
   const int64_t bk = g / a.nqb;
   const int kvh = (int)(bk % a.Hkv);
@@ -303,7 +318,7 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
   // ---- this warp's tiles ----
   const int U = a.ucount[g];
   const int total_tiles = (U + ATM_TILE - 1) / ATM_TILE;
-  const int active = atm_active_splits(total_tiles, a.nsplit);
+  const int active = atm_active_splits(total_tiles, a.nsplit, a.wave);
   if (split >= active) return;
   const int lanes_total = active * ATM_WARPS;     // warps sharing the group
   const int my_first = split * ATM_WARPS + warp;  // tile t of this warp = my_first + t * lanes_total
@@ -328,80 +343,6 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
     return m;
   };
   Meta pre0 = load_meta(0), pre1 = load_meta(1);
-
-  // ---- stage Q (zero padded to 16 rows; LSHW: rows 4..7 = centred unit queries) ----
-  for (int idx = tid; idx < 16 * (C::ROWB / 16); idx += ATM_THREADS) {
-    const int r = idx / (C::ROWB / 16), c = idx - r * (C::ROWB / 16);
-    uint4 val = make_uint4(0u, 0u, 0u, 0u);
-    const int rq = (LSHW && r >= 4) ? r - 4 : r;
-    if (rq < a.R && (LSHW || r < a.R) && r < (LSHW ? 8 : 16)) {
-      const int gi = rq / a.q_block, qo = rq - gi * a.q_block;
-      const int qi = qb * a.q_block + qo;
-      if (qi < a.Sq) {
-        const int h = kvh * a.G + gi;
-        if (LSHW && r >= 4)
-          val = *reinterpret_cast<const uint4*>(a.qhat + ((b * a.Hq + h) * a.Sq + qi) * D + c * 8);
-        else
-          val = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.q) +
-                                                b * a.qs_b + (int64_t)h * a.qs_h + qi * a.qs_q + c * 8);
-      }
-    }
-    *reinterpret_cast<uint4*>(q_sm + r * C::RSTR + c * 16) = val;
-  }
-  __syncthreads();
-
-  // Q fragments.  Full: [ks][0..3] = (rows 0-7, k lo), (rows 8-15, k lo), (rows 0-7, k hi),
-  // (rows 8-15, k hi).  HALF: [ks][0..1] = (rows 0-7, k lo), (rows 0-7, k hi).
-  uint32_t qf[C::KSTEPS][HALF ? 2 : 4];
-  {
-    const uint32_t q_s = (uint32_t)__cvta_generic_to_shared(q_sm);
-    const int mi = lane >> 3, rr = lane & 7;
-#pragma unroll
-    for (int ks = 0; ks < C::KSTEPS; ++ks) {
-      if constexpr (HALF) {
-        const int c = 2 * ks + (mi & 1);  // lanes 0-7: k lo, lanes 8-15: k hi
-        atm_ldmatrix_x2(qf[ks][0], qf[ks][1], q_s + rr * C::RSTR + c * 16);
-      } else {
-        const int row = (mi & 1) * 8 + rr;
-        const int c = 2 * ks + (mi >> 1);
-        atm_ldmatrix_x4(qf[ks][0], qf[ks][1], qf[ks][HALF ? 0 : 2], qf[ks][HALF ? 1 : 3],
-                        q_s + row * C::RSTR + c * 16);
-      }
-    }
-  }
-
-  __syncthreads();  // every warp holds its Q fragments: the first ring is free for the pipeline
-
-  // rows this thread owns in the C fragment, and their bias rows
-  const int r0 = lane >> 2, r1 = r0 + 8;
-  const __nv_bfloat16* bias_row[2] = {nullptr, nullptr};
-  if (a.bias != nullptr) {
-    const __nv_bfloat16* bb = reinterpret_cast<const __nv_bfloat16*>(a.bias) + b * a.bias_s_b;
-#pragma unroll
-    for (int rs = 0; rs < NR; ++rs) {
-      const int r = rs ? r1 : r0;
-      const int gi = r / a.q_block, qo = r - gi * a.q_block;
-      const int qi = qb * a.q_block + qo;
-      if (r < a.R && qi < a.Sq) bias_row[rs] = bb + (kvh * a.G + gi) * a.bias_s_h + qi * a.bias_s_q;
-    }
-  }
-  float qmu0 = 0.f;  // qhat . mean of this thread's row
-  if constexpr (LSHW) {
-    if (r0 < a.R) {
-      const int gi = r0 / a.q_block, qo = r0 - gi * a.q_block;
-      const int qi = qb * a.q_block + qo;
-      if (qi < a.Sq) qmu0 = a.qmu[(b * a.Hq + kvh * a.G + gi) * a.Sq + qi];
-    }
-  }
-
-  float o[C::NT][2 * NR];
-#pragma unroll
-  for (int nt = 0; nt < C::NT; ++nt)
-#pragma unroll
-    for (int e = 0; e < 2 * NR; ++e) o[nt][e] = 0.f;
-  float m_run[NR], l_run[NR];
-#pragma unroll
-  for (int rs = 0; rs < NR; ++rs) { m_run[rs] = -INFINITY; l_run[rs] = 0.f; }
 
   // 16-byte asynchronous copies: CPR lanes cover one row, so a warp instruction
   // moves 32 / CPR whole rows; destination offsets are compile-time constants
@@ -472,6 +413,80 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
     if (s < my_tiles) issue(s);
     if constexpr (!TMA) asm volatile("cp.async.commit_group;\n" ::);
   }
+
+  // ---- stage Q while the first tiles are on their way (zero padded to 16 rows; LSHW: rows 4..7 = centred unit queries) ----
+  for (int idx = tid; idx < 16 * (C::ROWB / 16); idx += ATM_THREADS) {
+    const int r = idx / (C::ROWB / 16), c = idx - r * (C::ROWB / 16);
+    uint4 val = make_uint4(0u, 0u, 0u, 0u);
+    const int rq = (LSHW && r >= 4) ? r - 4 : r;
+    if (rq < a.R && (LSHW || r < a.R) && r < (LSHW ? 8 : 16)) {
+      const int gi = rq / a.q_block, qo = rq - gi * a.q_block;
+      const int qi = qb * a.q_block + qo;
+      if (qi < a.Sq) {
+        const int h = kvh * a.G + gi;
+        if (LSHW && r >= 4)
+          val = *reinterpret_cast<const uint4*>(a.qhat + ((b * a.Hq + h) * a.Sq + qi) * D + c * 8);
+        else
+          val = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.q) +
+                                                b * a.qs_b + (int64_t)h * a.qs_h + qi * a.qs_q + c * 8);
+      }
+    }
+    *reinterpret_cast<uint4*>(q_sm + r * C::RSTR + c * 16) = val;
+  }
+  __syncthreads();
+
+  // Q fragments.  Full: [ks][0..3] = (rows 0-7, k lo), (rows 8-15, k lo), (rows 0-7, k hi),
+  // (rows 8-15, k hi).  HALF: [ks][0..1] = (rows 0-7, k lo), (rows 0-7, k hi).
+  uint32_t qf[C::KSTEPS][HALF ? 2 : 4];
+  {
+    const uint32_t q_s = (uint32_t)__cvta_generic_to_shared(q_sm);
+    const int mi = lane >> 3, rr = lane & 7;
+#pragma unroll
+    for (int ks = 0; ks < C::KSTEPS; ++ks) {
+      if constexpr (HALF) {
+        const int c = 2 * ks + (mi & 1);  // lanes 0-7: k lo, lanes 8-15: k hi
+        atm_ldmatrix_x2(qf[ks][0], qf[ks][1], q_s + rr * C::RSTR + c * 16);
+      } else {
+        const int row = (mi & 1) * 8 + rr;
+        const int c = 2 * ks + (mi >> 1);
+        atm_ldmatrix_x4(qf[ks][0], qf[ks][1], qf[ks][HALF ? 0 : 2], qf[ks][HALF ? 1 : 3],
+                        q_s + row * C::RSTR + c * 16);
+      }
+    }
+  }
+
+  __syncthreads();  // every warp holds its Q fragments: the stage is free for the pipeline
+
+  // rows this thread owns in the C fragment, and their bias rows
+  const int r0 = lane >> 2, r1 = r0 + 8;
+  const __nv_bfloat16* bias_row[2] = {nullptr, nullptr};
+  if (a.bias != nullptr) {
+    const __nv_bfloat16* bb = reinterpret_cast<const __nv_bfloat16*>(a.bias) + b * a.bias_s_b;
+#pragma unroll
+    for (int rs = 0; rs < NR; ++rs) {
+      const int r = rs ? r1 : r0;
+      const int gi = r / a.q_block, qo = r - gi * a.q_block;
+      const int qi = qb * a.q_block + qo;
+      if (r < a.R && qi < a.Sq) bias_row[rs] = bb + (kvh * a.G + gi) * a.bias_s_h + qi * a.bias_s_q;
+    }
+  }
+  float qmu0 = 0.f;  // qhat . mean of this thread's row
+  if constexpr (LSHW) {
+    if (r0 < a.R) {
+      const int gi = r0 / a.q_block, qo = r0 - gi * a.q_block;
+      const int qi = qb * a.q_block + qo;
+      if (qi < a.Sq) qmu0 = a.qmu[(b * a.Hq + kvh * a.G + gi) * a.Sq + qi];
+    }
+  }
+
+  float o[C::NT][2 * NR];
+#pragma unroll
+  for (int nt = 0; nt < C::NT; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2 * NR; ++e) o[nt][e] = 0.f;
+  float m_run[NR], l_run[NR];
+#pragma unroll
+  for (int rs = 0; rs < NR; ++rs) { m_run[rs] = -INFINITY; l_run[rs] = 0.f; }
 
   bool alive = true;
   int t = 0;
@@ -642,57 +657,57 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
   } else {
     asm volatile("cp.async.wait_group 0;\n" ::);
   }
-  __syncthreads();
 
-  // ---- merge the warps of this CTA (ring reused as fp32 scratch) ----
+  // ---- merge the warps of this CTA: a warp scales its accumulator to the CTA's maximum and leaves
+  //      it in its ring ----
   // (LSHW: rows 4..7 of the tile carried no softmax state: their maximum is -inf and they
   // are beyond a.R, so nothing below reads them)
+  if ((lane & 3) == 0) {
+    ml_sm[warp][r0] = make_float2(m_run[0], l_run[0]);
+    if constexpr (!HALF) ml_sm[warp][r1] = make_float2(m_run[NR - 1], l_run[NR - 1]);
+  }
+  __syncthreads();
   constexpr int RS = C::RS;
   float* red_o = reinterpret_cast<float*>(ring);  // [16][RS]
-  float* red_ml = red_o + 16 * RS;                // [16][2]
 #pragma unroll
-  for (int nt = 0; nt < C::NT; ++nt) {
-    const int d = nt * 8 + 2 * (lane & 3);
-    *reinterpret_cast<float2*>(red_o + r0 * RS + d) = make_float2(o[nt][0], o[nt][1]);
-    if constexpr (!HALF)
-      *reinterpret_cast<float2*>(red_o + r1 * RS + d) =
-          make_float2(o[nt][2 * NR - 2], o[nt][2 * NR - 1]);
-  }
-  if ((lane & 3) == 0) {
-    red_ml[r0 * 2] = m_run[0];
-    red_ml[r0 * 2 + 1] = l_run[0];
-    if constexpr (!HALF) {
-      red_ml[r1 * 2] = m_run[NR - 1];
-      red_ml[r1 * 2 + 1] = l_run[NR - 1];
-    }
+  for (int rs = 0; rs < NR; ++rs) {
+    const int r = rs ? r1 : r0;
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < ATM_WARPS; ++w) M = fmaxf(M, ml_sm[w][r].x);
+    const float sc = (m_run[rs] == -INFINITY) ? 0.f : __expf(m_run[rs] - M);
+#pragma unroll
+    for (int nt = 0; nt < C::NT; ++nt)
+      *reinterpret_cast<float2*>(red_o + r * RS + nt * 8 + 2 * (lane & 3)) =
+          make_float2(o[nt][2 * rs] * sc, o[nt][2 * rs + 1] * sc);
   }
   __syncthreads();
   float* pout = a.partial + ((int64_t)g * a.nsplit + split) * a.R * (D + 2);
-  for (int idx = tid; idx < a.R * D; idx += ATM_THREADS) {
-    const int r = idx / D, d = idx - r * D;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < ATM_WARPS; ++w)
-      M = fmaxf(M, reinterpret_cast<const float*>(atm_smem + w * C::WARP_BYTES)[16 * RS + r * 2]);
-    float acc = 0.f, L = 0.f;
+  for (int idx = tid; idx < a.R * (D / 2); idx += ATM_THREADS) {
+    const int r = idx / (D / 2), d = (idx - r * (D / 2)) * 2;
+    float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < ATM_WARPS; ++w) {
-      const float* wo = reinterpret_cast<const float*>(atm_smem + w * C::WARP_BYTES);
-      const float mw = wo[16 * RS + r * 2];
-      if (mw != -INFINITY) {
-        const float sc = __expf(mw - M);
-        acc += wo[r * RS + d] * sc;
-        L += wo[16 * RS + r * 2 + 1] * sc;
-      }
+      const float2 x = *reinterpret_cast<const float2*>(
+          reinterpret_cast<const float*>(atm_smem + w * C::WARP_BYTES) + r * RS + d);
+      acc.x += x.x;
+      acc.y += x.y;
     }
-    pout[r * (D + 2) + d] = acc;
-    if (d == 0) {
-      pout[r * (D + 2) + D] = M;
-      pout[r * (D + 2) + D + 1] = L;
+    *reinterpret_cast<float2*>(pout + r * (D + 2) + d) = acc;
+  }
+  if (tid < a.R) {
+    float M = -INFINITY, L = 0.f;
+#pragma unroll
+    for (int w = 0; w < ATM_WARPS; ++w) M = fmaxf(M, ml_sm[w][tid].x);
+#pragma unroll
+    for (int w = 0; w < ATM_WARPS; ++w) {
+      const float2 ml = ml_sm[w][tid];
+      if (ml.x != -INFINITY) L += ml.y * __expf(ml.x - M);
     }
+    *reinterpret_cast<float2*>(pout + tid * (D + 2) + D) = make_float2(M, L);
   }
 
-  atm_finish_group<D, ATM_THREADS, __nv_bfloat16>(a, g, active, atm_smem, &is_last_sm, tickets, sinks, out, part_out);
+  atm_finish_group<D, ATM_THREADS, D / 64, __nv_bfloat16>(a, g, active, &is_last_sm, tickets, sinks, out, part_out);
 }
 
 // Row-gather probe: the copy half of the attention kernel alone.  Same grid, same dealing of
@@ -707,8 +722,8 @@ attention_gather_probe_kernel(AttnArgs a, unsigned int* __restrict__ sink) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* ring = atm_smem + warp * C::WARP_BYTES;
   const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
-  const int split = blockIdx.x;
-  const int64_t g = blockIdx.y;
+  const int split = a.group_major ? blockIdx.x : blockIdx.y;
+  const int64_t g = a.group_major ? blockIdx.y : blockIdx.x;
   const int64_t bk = g / a.nqb;
   const int kvh = (int)(bk % a.Hkv);
   const int64_t b = bk / a.Hkv;
@@ -717,7 +732,7 @@ attention_gather_probe_kernel(AttnArgs a, unsigned int* __restrict__ sink) {
   const int32_t* gcols = a.ucols + g * a.S;
   const int U = a.ucount[g];
   const int total_tiles = (U + ATM_TILE - 1) / ATM_TILE;
-  const int active = atm_active_splits(total_tiles, a.nsplit);
+  const int active = atm_active_splits(total_tiles, a.nsplit, a.wave);
   if (split >= active) return;
   const int lanes_total = active * ATM_WARPS;
   const int my_first = split * ATM_WARPS + warp;
@@ -842,15 +857,17 @@ static int launch_attention_mma(AttnArgs a, int B, int groups, int* tickets, int
                                 const float* sinks, void* out, float* part_out, bool lsh,
                                 cudaStream_t st) {
   static bool allowed[9][64] = {};
-  // shared memory that the last CTA of a group needs to merge the splits (atm_finish_group)
-  const size_t merge_bytes = (size_t)16 * a.nsplit * 4 + 128;
   static_assert(AtmCfg<D, false, 2>::RED_BYTES <= AtmCfg<D, false, 2>::WARP_BYTES &&
                 AtmCfg<D, true, 2>::RED_BYTES <= AtmCfg<D, true, 2>::WARP_BYTES,
                 "reduction scratch must fit the ring");
   if (lsh && a.R > 4)
     return sah_fail(SAH_ERR_UNSUPPORTED, "attention: in-place MagicPig weights need <= 4 mask rows "
                     "per KV group, got %d", a.R);
-  dim3 grid((unsigned)a.nsplit, (unsigned)groups);
+  // Where no list can be long enough for a second wave, the CTAs that have work come first; where
+  // lists are long the CTAs of a group run together, so that neighbouring rows are read together.
+  a.group_major = groups <= 65535 && (a.nsplit < ATM_FINE_SPLITS || a.nsplit <= a.wave ||
+                                      sah_ceil_div(a.S, ATM_TILE) >= (int64_t)a.nsplit * ATM_WARPS * ATM_ONE_WAVE_TILES);
+  const dim3 grid = a.group_major ? dim3((unsigned)a.nsplit, (unsigned)groups) : dim3((unsigned)groups, (unsigned)a.nsplit);
   AtmMaps maps;
   memset(&maps, 0, sizeof(maps));
   bool tma = false;
@@ -865,8 +882,6 @@ static int launch_attention_mma(AttnArgs a, int B, int groups, int* tickets, int
 #define ATM_LAUNCH(HALF, LSHW, TMA, NST, SLOT)                                                      \
   do {                                                                                              \
     const int smem = AtmCfg<D, TMA, NST>::SMEM;                                                     \
-    if (merge_bytes > (size_t)ATM_WARPS * AtmCfg<D, TMA, NST>::WARP_BYTES)                          \
-      return sah_fail(SAH_ERR_UNSUPPORTED, "attention: %d splits do not fit the merge scratch", a.nsplit); \
     e = sah_allow_smem(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, smem, allowed[SLOT]);  \
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "attention attr: %s", cudaGetErrorString(e)); \
     sah_launch_chain(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, grid, ATM_THREADS, smem, st, \

@@ -155,3 +155,28 @@ def test_bounded_wait_runs_out_and_reports_without_hanging():
         np.testing.assert_allclose(out.float().cpu().numpy(), ref, atol=TOL, rtol=TOL)
     finally:
         select_attention_kernel(prev)
+
+
+@pytest.mark.parametrize("selected", [1, 16, 33, 130, 545, 2100, 4800, 19000])
+@pytest.mark.parametrize("dtype,D", [("f32", 64), ("f32", 128), ("bf16", 64), ("bf16", 128)])
+def test_lists_from_one_tile_to_many_splits(dtype, D, selected):
+    """Eight KV groups whose lists hold from one entry to 1188 tiles: one CTA per group, a merge of up
+    to sixteen splits, of more, one wave of CTAs, two.  Against float64: bfloat16 rounds the
+    probabilities and the output (2^-9 each, relative); float32 sums of up to 19000 terms and
+    __expf with an argument below 16 (2^-21 of it) stay under 1e-5."""
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    gen = torch.Generator(device=DEV).manual_seed(selected)
+    S = 20000
+    q = torch.randn((1, 32, 1, D), generator=gen, device=DEV).to(dt)
+    k, v = (torch.randn((1, 8, S, D), generator=gen, device=DEV).to(dt) for _ in range(2))
+    dense = torch.zeros((1, 32, 1, S), dtype=dt, device=DEV)
+    columns = torch.randperm(S, generator=gen, device=DEV)[:selected]
+    dense[..., columns] = (torch.rand((1, 32, 1, selected), generator=gen, device=DEV) < 0.7).to(dt)
+    dense[..., columns[0]] = 1.0
+    out = native_masked_attention(q, k, v, None, None, D ** -0.5,
+                                  Mask.create_mask_from_dense_mask(dense.shape, dense, dt))
+    logits = torch.matmul(q.double(), k.repeat_interleave(4, 1).double().transpose(2, 3)) * D ** -0.5
+    p = torch.softmax(logits.masked_fill(dense == 0, -torch.inf), dim=-1)
+    ref = torch.matmul(p, v.repeat_interleave(4, 1).double()).transpose(1, 2)
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    assert err < (2 * 2.0 ** -9 if dtype == "bf16" else 1e-5), err
