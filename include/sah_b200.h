@@ -771,6 +771,50 @@ int sah_masked_attention_static(const uint32_t* bits, const void* q, const void*
                                 int64_t bias_s_b, int64_t bias_s_h, int64_t bias_s_q,
                                 const float* sinks, int sm_count, void* out, void* stream);
 
+/* ---------------------------------------------------------------------------
+ * A whole decode call over a mask of bands (sink, local window) and, with
+ * heavy > 0, the `heavy` largest q.k of the other columns of every row: the
+ * kernels of sah_qk_scores, sah_topk_select_bands, sah_attn_plan_bands or
+ * sah_attn_plan and sah_masked_attention, one after the other on `stream`.
+ * `bands` are those of sah_attn_plan_bands, in order.  `tickets` (int32
+ * [n_tickets], n_tickets > KV groups) is zero before the first call that uses
+ * it and is left zero; its first word is set when a bounded wait ran out.  Two
+ * calls that may overlap on the device need tickets and scratch of their own.
+ *
+ * sah_fixed_step_plan fills the layout of the scratch (`total` bytes, 256-byte
+ * aligned) from the extents and says SAH_ERR_UNSUPPORTED where the separate
+ * entry points are the faster or the only way: more than 32768 keys without a
+ * top-k, rows that sah_topk_select_fits spreads over the grid, too few
+ * tickets. */
+#define SAH_STEP_MAX_BANDS 6
+typedef struct {
+  const void *q, *k, *v;
+  int64_t q_stride[3], k_stride[3], v_stride[3]; /* batch, head, position */
+  int32_t dtype, B, Hq, Hkv, Sq, D;
+  int64_t S;
+  const void* bias; /* additive attention mask, NULL for none */
+  int64_t bias_stride[3];
+  const float* sinks; /* [Hq] sink logits, NULL for none */
+  float scaling;
+  int32_t n_bands;
+  int64_t bands[5 * SAH_STEP_MAX_BANDS];
+  int64_t heavy;
+  int32_t* tickets;
+  int64_t n_tickets;
+  int32_t sm_count;
+  void* scratch;
+  void* out; /* [B][Sq][Hq][D] */
+} sah_fixed_step;
+
+typedef struct {
+  sah_attn_sizes sizes;
+  int64_t words; /* of a bitmap row */
+  int64_t total, scores, bits, ucols, umemb, ucount, partial; /* bytes; offsets in the scratch */
+} sah_fixed_step_layout;
+
+int sah_fixed_step_plan(const sah_fixed_step* step, sah_fixed_step_layout* layout);
+int sah_fixed_step_run(const sah_fixed_step* step, const sah_fixed_step_layout* layout, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

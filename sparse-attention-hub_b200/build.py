@@ -1,4 +1,5 @@
-"""Build the sm_100a shared library `lib/libsah_b200.so` from `csrc/*.cu`.
+"""Build the sm_100a shared library `lib/libsah_b200.so` from `csrc/*.cu`, and the host module
+`lib/_sah_step.so` (CPython, against torch's headers) from `host/sah_step.cpp`.
 
     python sparse-attention-hub_b200/build.py [--force] [--verbose]
 
@@ -13,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -22,6 +24,8 @@ CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "libsah_b200.so"
 OBJ_DIR = PKG_DIR / "build"
+STEP_SRC = PKG_DIR / "host" / "sah_step.cpp"
+STEP_PATH = LIB_DIR / "_sah_step.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -53,8 +57,34 @@ def is_stale() -> bool:
     return (not LIB_PATH.exists()) or LIB_PATH.stat().st_mtime < _deps_mtime()
 
 
+def build_step(force: bool = False, verbose: bool = False) -> Path:
+    """Compile the host module; returns its path."""
+    newest = max(f.stat().st_mtime for f in (STEP_SRC, REPO_DIR / "include" / "sah_b200.h"))
+    if not force and STEP_PATH.exists() and STEP_PATH.stat().st_mtime >= newest:
+        return STEP_PATH
+    import torch
+    from torch.utils import cpp_extension
+
+    LIB_DIR.mkdir(exist_ok=True)
+    tmp = STEP_PATH.with_suffix(".so.tmp")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f"-I{REPO_DIR / 'include'}", f"-isystem{sysconfig.get_paths()['include']}",
+           *(f"-isystem{d}" for d in cpp_extension.include_paths()), str(STEP_SRC), "-o", str(tmp),
+           *(f"-L{d}" for d in cpp_extension.library_paths()), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on {STEP_SRC.name}")
+    os.replace(tmp, STEP_PATH)
+    return STEP_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every kernel file and link the shared library; returns its path."""
+    """Compile every kernel file and link the shared library, and build the host module; returns the
+    library's path."""
+    build_step(force, verbose)
     if not force and not is_stale():
         return LIB_PATH
     nvcc = _nvcc()

@@ -934,7 +934,7 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
                                  const sah_attn_sizes* sizes, const int32_t* ucols,
                                  const uint16_t* umemb, const float* uw, const int32_t* ucount,
                                  float* partial, void* out, float* part_out,
-                                 const AttnLsh* lsh, void* stream) {
+                                 const AttnLsh* lsh, void* stream, int* own_tickets = nullptr) {
   SAH_REQUIRE(q && k && v && sizes && ucols && umemb && ucount && partial && out,
               "masked_attention: null pointer");
   SAH_REQUIRE(B > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && Sq > 0 && S > 0,
@@ -974,10 +974,11 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_ATTENTION, (cudaStream_t)stream);
   int rc = SAH_OK;
+  // merge tickets of the groups and the error word (set when a bounded wait inside a kernel ran out)
+  int* tickets = own_tickets ? own_tickets + 1 : const_cast<int*>(ucount) + groups + (int64_t)groups * plan_chunks(S);
+  int* errflag = own_tickets ? own_tickets : tickets + groups;
   if (dtype == SAH_BF16) {
     // tensor-core path; the split merge is fused into the kernel (ticket per group)
-    int* tickets = const_cast<int*>(ucount) + groups + (int64_t)groups * plan_chunks(S);
-    int* errflag = tickets + groups;  // set when a bounded wait inside the kernel ran out
     // long lists: keys as the M dimension of tcgen05 tiles; otherwise the mma.sync kernel
     const int umma = aum_requested();
     if (D == 128 && (umma == 1 || (umma < 0 && aum_default(lsh != nullptr, S, groups)))) {
@@ -1005,9 +1006,8 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
   if (lsh != nullptr)
     return sah_fail(SAH_ERR_UNSUPPORTED, "masked_attention_lsh: bfloat16 only");
   // the split merge is fused into the kernel here too (ticket per group, as in bfloat16)
-  int* tickets32 = const_cast<int*>(ucount) + groups + (int64_t)groups * plan_chunks(S);
-  rc = (D == 128) ? launch_attention<float, 128>(a, groups, tickets32, sinks, out, part_out, st)
-                  : launch_attention<float, 64>(a, groups, tickets32, sinks, out, part_out, st);
+  rc = (D == 128) ? launch_attention<float, 128>(a, groups, tickets, sinks, out, part_out, st)
+                  : launch_attention<float, 64>(a, groups, tickets, sinks, out, part_out, st);
   if (rc != SAH_OK) return rc;
   g_last_attn_kernel = "masked_attention_kernel";
   SAH_LAUNCH_CHECK("masked_attention");
@@ -1432,4 +1432,69 @@ extern "C" int sah_masked_attention_static(
                               B, Hq, Hkv, Sq, S, D, scaling, bias, bias_s_b, bias_s_h, bias_s_q,
                               sinks, &sizes, ucols, umemb, nullptr, ucount, partial, out, nullptr,
                               stream);
+}
+
+// ---------------------------------------------------------------------------
+// A decode call over bands and an exact top-k in one entry (see the header).  The same kernels as
+// through the separate entry points, but for two bitmaps that nobody can ask for afterwards: the
+// bands are not written out.
+// ---------------------------------------------------------------------------
+static_assert(SAH_STEP_MAX_BANDS == SAH_MAX_BANDS, "one limit");
+
+extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layout* o) {
+  SAH_REQUIRE(s && o, "fixed_step_plan: null pointer");
+  SAH_REQUIRE(s->B > 0 && s->Hq > 0 && s->Hkv > 0 && s->Sq > 0 && s->S > 0 && s->D > 0 && s->heavy >= 0,
+              "fixed_step_plan: bad extents");
+  const int rc = sah_attn_query_sizes(s->B, s->Hq, s->Hkv, s->Sq, s->S, s->D, 0, s->sm_count, &o->sizes);
+  if (rc != SAH_OK) return rc;
+  const int64_t rows = (int64_t)s->B * s->Hq * s->Sq;
+  o->words = sah_ceil_div(sah_ceil_div(s->S, 32), 4) * 4;
+  if (o->sizes.groups >= s->n_tickets || (s->heavy == 0 && s->S > 32768) ||
+      (s->heavy > 0 && sah_topk_select_fits(s->dtype, rows, s->S, o->words) == 0))
+    return SAH_ERR_UNSUPPORTED;  // (no message: the caller has another way)
+  int64_t at = 0;
+  auto take = [&](int64_t bytes) {
+    const int64_t p = at;
+    at += sah_ceil_div(bytes, 256) * 256;
+    return p;
+  };
+  o->scores = take(s->heavy > 0 ? rows * s->S * (s->dtype == SAH_BF16 ? 2 : 4) : 0);
+  o->bits = take(s->heavy > 0 ? rows * o->words * 4 : 0);
+  o->ucols = take(o->sizes.ucols_bytes);
+  o->umemb = take(o->sizes.umemb_bytes);
+  o->ucount = take(o->sizes.ucount_bytes);
+  o->partial = take(o->sizes.partial_bytes);
+  o->total = at;
+  return SAH_OK;
+}
+
+extern "C" int sah_fixed_step_run(const sah_fixed_step* s, const sah_fixed_step_layout* o, void* stream) {
+  SAH_REQUIRE(s && o && s->scratch && s->tickets && s->out, "fixed_step: null pointer");
+  SAH_REQUIRE(o->sizes.groups < s->n_tickets, "fixed_step: too few tickets");
+  SAH_REQUIRE(((uintptr_t)s->scratch & 15) == 0, "fixed_step: scratch must be 16-byte aligned");
+  unsigned char* p = (unsigned char*)s->scratch;
+  int32_t *ucols = (int32_t*)(p + o->ucols), *ucount = (int32_t*)(p + o->ucount);
+  uint16_t* umemb = (uint16_t*)(p + o->umemb);
+  int rc;
+  if (s->heavy > 0) {
+    rc = sah_qk_scores(s->q, s->k, s->dtype, s->q_stride[0], s->q_stride[1], s->q_stride[2], s->k_stride[0], s->k_stride[1],
+                       s->k_stride[2], s->B, s->Hq, s->Hkv, s->Sq, s->S, s->D, s->bias, s->bias_stride[0],
+                       s->bias_stride[1], s->bias_stride[2], p + o->scores, stream);
+    if (rc != SAH_OK) return rc;
+    uint32_t* bits = (uint32_t*)(p + o->bits);
+    rc = sah_topk_select_bands(p + o->scores, s->dtype, (int64_t)s->B * s->Hq * s->Sq, s->Sq, s->S, o->words, 0, s->S,
+                               s->n_bands, s->bands, s->heavy, bits, stream);
+    if (rc != SAH_OK) return rc;
+    rc = sah_attn_plan(bits, nullptr, nullptr, nullptr, s->dtype, s->B, s->Hq, s->Hkv, s->Sq, s->S, o->words, &o->sizes,
+                       ucols, umemb, nullptr, ucount, stream);
+  } else {
+    rc = sah_attn_plan_bands(s->n_bands, s->bands, s->dtype, s->B, s->Hq, s->Hkv, s->Sq, s->S, &o->sizes, ucols, umemb,
+                             ucount, stream);
+  }
+  if (rc != SAH_OK) return rc;
+  return masked_attention_impl(s->q, s->k, s->v, s->dtype, s->q_stride[0], s->q_stride[1], s->q_stride[2], s->k_stride[0],
+                               s->k_stride[1], s->k_stride[2], s->v_stride[0], s->v_stride[1], s->v_stride[2], s->B, s->Hq,
+                               s->Hkv, s->Sq, s->S, s->D, s->scaling, s->bias, s->bias_stride[0], s->bias_stride[1],
+                               s->bias_stride[2], s->sinks, &o->sizes, ucols, umemb, nullptr, ucount,
+                               (float*)(p + o->partial), s->out, nullptr, nullptr, stream, s->tickets);
 }

@@ -32,7 +32,8 @@ SAH_BF16 = 1
 ACTIVATIONS = {"relu": 0, "silu": 1, "gelu": 2, "tanh": 3}
 
 _PKG_ROOT = Path(__file__).resolve().parent.parent
-LIB_PATH = Path(os.environ.get("SAH_B200_LIB", _PKG_ROOT / "lib" / "libsah_b200.so"))
+DEFAULT_LIB_DIR = _PKG_ROOT / "lib"
+LIB_PATH = Path(os.environ.get("SAH_B200_LIB", DEFAULT_LIB_DIR / "libsah_b200.so"))
 
 
 class NativeLibraryError(RuntimeError):
@@ -74,6 +75,8 @@ _SIGNATURES = {
     "sah_hash_encode": [_P, _I, _L, _L, _L, _I, _I, _I, _L, _L, _L, _I, POINTER(c_int),
                         POINTER(c_void_p), POINTER(c_void_p), _I, _P, _P, _P],
     "sah_hash_topk": [_P, _L, _P, _I, _P, _I, _L, _L, _L, _I, _I, _I, _L, _L, _P, _L, _P, _P],
+    "sah_fixed_step_plan": [_P, _P],
+    "sah_fixed_step_run": [_P, _P, _P],
     "sah_qk_scores": [_P, _P, _I, _L, _L, _L, _L, _L, _L, _I, _I, _I, _I, _L, _I, _P, _L, _L,
                       _L, _P, _P],
     "sah_topk_select": [_P, _I, _L, _L, _L, _L, _L, _P, _L, _P, _P],

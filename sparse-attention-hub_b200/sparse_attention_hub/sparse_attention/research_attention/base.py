@@ -18,6 +18,7 @@ from ..utils.mask_attention_utils import (
     get_masked_attention_output,
     get_true_attention_output,
 )
+from .fixed_step import fixed_step
 from .maskers.base import MaskerConfig, ResearchMasker
 from .maskers.sampling.base import SamplingMasker
 
@@ -77,10 +78,19 @@ class ResearchAttention(SparseAttention):
                 "sparse_meta_data must be provided in kwargs while calling custom_attention()"
             )
         sparse_meta_data: Dict[Any, Any] = kwargs.pop("sparse_meta_data")
+        logger = MicroMetricLogger()
+        if (not logger.enabled_metrics and not self.return_attention_weights and dropout == 0.0
+                and kwargs.get("sequence_shard") is None
+                and type(self).build_mask is ResearchAttention.build_mask and "build_mask" not in self.__dict__):
+            # nobody looks at the mask of this call: bands and an exact top-k need none
+            s_aux_raw = kwargs.get("s_aux")
+            out = fixed_step(self.maskers, queries, keys, values, attention_mask,
+                             s_aux_raw if isinstance(s_aux_raw, torch.Tensor) else None, scaling)
+            if out is not None:
+                return out, None
         mask = self.build_mask(queries, keys, values, attention_mask, scaling, dropout,
                                sparse_meta_data, **kwargs)
 
-        logger = MicroMetricLogger()
         if logger.is_metric_enabled("research_attention_density"):
             logger.log("research_attention_density", mask.get_density(),
                        metadata={"layer_idx": kwargs["layer_idx"]})

@@ -79,7 +79,8 @@ class DecodeStepGraph:
         # that the capture finds it, and keep it alive for as long as the graph may replay.
         from ..utils import mask_attention_utils
 
-        self._scratch = list(mask_attention_utils._workspace_cache.values())
+        self._scratch = [*mask_attention_utils._workspace_cache.values(),
+                         *mask_attention_utils._ticket_cache.values()]
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=side):
             self.out = call()

@@ -1,0 +1,109 @@
+"""Decode calls over bands and an exact top-k, through one native entry.
+
+The stacks of sink and local-window maskers, alone or followed by an oracle top-k, need no mask
+object between the maskers: the bands are numbers, and the top-k writes one bitmap that the
+attention plan reads.  `fixed_step` hands such a call to `host/sah_step.cpp`, which launches the
+kernels that the maskers and the attention step would (`sah_fixed_step_run`); the output is the same,
+bit for bit.  It returns None wherever the general path has to say or do something else: other
+maskers or subclasses of these, sizes that select every key, tensors that are not plain CUDA tensors
+of one dtype, rows whose selection is faster with a scratch buffer.
+"""
+
+from __future__ import annotations
+
+import ctypes
+import importlib.util
+import threading
+from typing import List, Optional
+
+import torch
+
+from ... import _native
+from ..utils import mask_attention_utils
+from .maskers.fixed.implementations.basic_fixed import LocalMasker, SinkMasker
+from .maskers.fixed.implementations.oracle_top_k import OracleTopK
+
+_MAX_BANDS = 6       # SAH_STEP_MAX_BANDS
+_N_TICKETS = 16384   # KV groups per call, and the error word
+
+_module = None
+
+
+def _step_module():
+    global _module
+    if _module is None:
+        path = _native.LIB_PATH.with_name("_sah_step.so")
+        if not path.exists():
+            path = _native.DEFAULT_LIB_DIR / "_sah_step.so"
+        if not path.exists():
+            raise _native.NativeLibraryError(f"{path} is missing: run sparse-attention-hub_b200/build.py")
+        spec = importlib.util.spec_from_file_location("_sah_step", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        lib = _native.load()
+        module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.sah_fixed_step_plan, lib.sah_fixed_step_run)))
+        _module = module
+    return _module
+
+
+def _tickets(device: torch.device, stream: int) -> torch.Tensor:
+    """Merge tickets (and the error word in front of them) of the calls of one stream and host thread:
+    zero between calls, so they are made once and not per call."""
+    pool = mask_attention_utils._ticket_cache
+    key = (device.index, stream, threading.get_ident())
+    found = pool.get(key)
+    if found is None:
+        if len(pool) > 16:
+            pool.clear()
+        found = pool[key] = torch.zeros(_N_TICKETS, dtype=torch.int32, device=device)
+    return found
+
+
+def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
+               attention_mask: Optional[torch.Tensor], sinks: Optional[torch.Tensor],
+               scaling: float) -> Optional[torch.Tensor]:
+    """`[B, Sq, Hq, D]`, or None when the call is not one that the native entry serves."""
+    if not maskers or type(queries) is not torch.Tensor or queries.dim() != 4 or not queries.is_cuda:
+        return None
+    if type(keys) is not torch.Tensor or keys.dim() != 4:
+        return None
+    Sq, S = queries.shape[2], keys.shape[2]
+    bands, heavy = (), 0
+    for masker in maskers:
+        kind = type(masker)
+        if heavy or len(bands) > 5 * (_MAX_BANDS - 2):
+            return None
+        if kind is SinkMasker:
+            size = masker._calculate_effective_sink_size(S)
+            if not 0 < size < S:
+                return None
+            bands += (0, 0, size, 0, 1)
+        elif kind is LocalMasker:
+            size = masker._calculate_effective_window_size(S)
+            if not 0 < size < S - Sq:
+                return None
+            bands += (S - Sq - size + 1, 1, S - Sq + 1, 1, 1)
+            if Sq > 1:
+                bands += (S - Sq + 1, 1, S, 0, 0)
+        elif kind is OracleTopK:
+            heavy = masker._calculate_effective_heavy_size(S)
+            if not 0 < heavy < S:
+                return None
+        else:
+            return None
+    device = queries.device
+    stream = _native.stream_of(device)
+    tickets = _tickets(device, stream)
+    done = _step_module().fixed_step(queries, keys, values, attention_mask, sinks, float(scaling), bands, heavy, tickets,
+                                     _native.sm_count(device), stream)
+    if done is None:
+        return None
+    if isinstance(done, int):
+        # a refused launch may leave tickets behind
+        mask_attention_utils._ticket_cache.pop((device.index, stream, threading.get_ident()), None)
+        _native.check(done, "sah_fixed_step_run")
+    out, scratch, ucols, umemb, ucount, groups, rows = done
+    B, Hq, _, D = queries.shape
+    mask_attention_utils._last_plan["step"] = (scratch, ucols, umemb, ucount, groups, rows, S,
+                                               (B, Hq, keys.shape[1], Sq, S, D, 0, _native.sm_count(device)))
+    return out

@@ -31,6 +31,9 @@ from .mask import Mask, NativeBits, words_per_row
 
 _workspace_cache: Dict[Tuple, Dict[str, torch.Tensor]] = {}
 
+# merge tickets of `fixed_step` calls by (device, stream, host thread); the first word is the error word
+_ticket_cache: Dict[Tuple, torch.Tensor] = {}
+
 
 def _bias_args(attention_mask: Optional[torch.Tensor], dtype: torch.dtype, n_keys: int):
     """(tensor kept alive, pointer, stride_b, stride_h, stride_q) of the additive bias."""
@@ -201,6 +204,7 @@ def native_masked_attention(
     _last_plan["ws"] = ws
     _last_plan["sizes"] = (sizes.groups, sizes.rows_per_group, S)
     _last_plan["attn_sizes"] = sizes
+    _last_plan["step"] = None
     if return_partials:
         return out, part
     return out
@@ -211,13 +215,29 @@ def native_masked_attention(
 # (float32 [groups * S * rows_per_group], union-list order; see last_union_list()).
 _weight_dump: Dict[str, Any] = {"request": None, "weights": None}
 
-_last_plan: Dict[str, Any] = {"ucount": None, "ws": None, "sizes": None}
+# "step": what a `fixed_step` call left of its work list (its scratch tensor and offsets), made into the
+# other entries only when somebody asks
+_last_plan: Dict[str, Any] = {"ucount": None, "ws": None, "sizes": None, "step": None}
+
+
+def _last() -> Dict[str, Any]:
+    if _last_plan["step"] is not None:
+        scratch, ucols, umemb, ucount, groups, rows, S, extents = _last_plan["step"]
+
+        def part(offset, count, dtype):
+            return scratch[offset:offset + count * dtype.itemsize].view(dtype)
+
+        ws = {"ucols": part(ucols, groups * S, torch.int32), "umemb": part(umemb, groups * S, torch.int16),
+              "ucount": part(ucount, groups, torch.int32)}
+        _last_plan.update(ucount=ws["ucount"], ws=ws, sizes=(groups, rows, S),
+                          attn_sizes=_native.attn_sizes(*extents), step=None)
+    return _last_plan
 
 
 def last_union_counts() -> Optional[torch.Tensor]:
     """int32 [groups]: distinct K/V rows the most recent attention call gathered per KV group
     (valid once the launching stream has run; used for bandwidth accounting)."""
-    return _last_plan["ucount"]
+    return _last()["ucount"]
 
 
 def attention_wait_errors() -> int:
@@ -228,6 +248,8 @@ def attention_wait_errors() -> int:
         groups = ws.get("groups")
         if groups is not None:
             n += int(ws["ucount"][ws["err_index"]].item() != 0)
+    for tickets in _ticket_cache.values():
+        n += int(tickets[0].item() != 0)
     return n
 
 
@@ -235,7 +257,7 @@ def last_union_list():
     """(ucols int32 [groups, S], umemb int16 [groups, S], ucount int32 [groups], rows per group)
     of the most recent attention call: the ascending union of the columns each KV group
     gathered, and which of the group's rows selected each."""
-    ws, (groups, R, S) = _last_plan["ws"], _last_plan["sizes"]
+    ws, (groups, R, S) = _last()["ws"], _last_plan["sizes"]
     return (ws["ucols"][: groups * S].view(groups, S), ws["umemb"][: groups * S].view(groups, S),
             ws["ucount"][:groups], R)
 
@@ -264,7 +286,7 @@ def gather_probe(keys: torch.Tensor, values: torch.Tensor, seq_len_queries: int 
     without its arithmetic.  Timed by the caller (profile slot "other"), it gives the ceiling
     that the gather of exactly those rows allows."""
     lib = _native.load()
-    ws, sizes = _last_plan["ws"], _last_plan["attn_sizes"]
+    ws, sizes = _last()["ws"], _last_plan["attn_sizes"]
     k, v = _rowmajor(keys), _rowmajor(values)
     B, Hkv, S, D = k.shape
     sink = ws.setdefault("probe_sink", torch.zeros(1, dtype=torch.int32, device=k.device))

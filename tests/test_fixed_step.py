@@ -1,0 +1,135 @@
+"""Calls over bands and an exact top-k through the single native entry against the general path (masker
+by masker, then the attention step) on the same tensors: the same kernels, so the same bits."""
+
+import pytest
+import torch
+
+import workloads
+from sparse_attention_hub.sparse_attention.research_attention import base
+from sparse_attention_hub.sparse_attention.research_attention import fixed_step as fs
+from sparse_attention_hub.sparse_attention.utils.mask_attention_utils import (
+    attention_wait_errors, get_masked_attention_output, last_union_counts)
+
+DEV = "cuda:0"
+SINK_LOCAL = [("sink", {"sink_size": 5}), ("local", {"window_size": 37})]
+TOPK = SINK_LOCAL + [("oracle_topk", {"heavy_size": 0.05})]
+
+
+def _inputs(dt, B, Hq, Hkv, Sq, S, D, layout="plain"):
+    gen = torch.Generator(device=DEV).manual_seed(S + Sq)
+    shape = {"plain": (B, Hkv, S, D), "cache": (B, Hkv, S + 77, D), "rows": (B, S, Hkv, D), "odd": (B, Hkv, S, D + 8)}[layout]
+    q = torch.randn((B, Sq, Hq, D), generator=gen, device=DEV).to(dt).transpose(1, 2)
+    kv = [torch.randn(shape, generator=gen, device=DEV).to(dt) for _ in range(2)]
+    if layout == "rows":
+        kv = [t.transpose(1, 2) for t in kv]
+    return q, kv[0][:, :, :S, :D], kv[1][:, :, :S, :D]
+
+
+def _both(ra, q, k, v, am=None, sinks=None):
+    out, weights = ra.custom_attention(None, q, k, v, am, 0.125, 0.0, sparse_meta_data={}, layer_idx=0, s_aux=sinks)
+    counts = last_union_counts().clone()
+    mask = ra.build_mask(q, k, v, am, 0.125, 0.0, {}, layer_idx=0)
+    want = get_masked_attention_output(None, q, k, v, am, sinks, 0.125, 0.0, mask)
+    assert weights is None
+    assert torch.equal(counts, last_union_counts())
+    return out, want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["plain", "cache", "rows", "odd"])
+@pytest.mark.parametrize("dtype,Sq,S,D,stack,served", [
+    ("f32", 1, 43, 64, "fixed", True), ("f32", 1, 42, 64, "fixed", True), ("f32", 1, 38, 64, "fixed", False),
+    ("bf16", 3, 131, 64, "fixed", True), ("bf16", 1, 32768, 128, "fixed", True), ("bf16", 2, 32769, 64, "fixed", False),
+    ("bf16", 1, 4097, 128, "topk", True), ("f32", 4, 1000, 64, "topk", True), ("bf16", 1, 90000, 64, "topk", False),
+    ("bf16", 24, 8191, 128, "topk", True), ("f32", 2, 40000, 64, "topk", True), ("bf16", 1, 19, 64, "topk only", False),
+    ("bf16", 2, 260, 64, "topk only", True)])
+def test_same_as_the_general_path(dtype, Sq, S, D, stack, served, layout, monkeypatch):
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    q, k, v = _inputs(dt, 2, 8, 2, Sq, S, D, layout)
+    stack = {"fixed": SINK_LOCAL, "topk": TOPK, "topk only": TOPK[2:]}[stack]
+    ra = workloads.research_attention(stack, dtype, DEV)
+    results = []
+
+    def noted(*args):
+        results.append(fs.fixed_step(*args))
+        return results[-1]
+
+    monkeypatch.setattr(base, "fixed_step", noted)
+    got, want = _both(ra, q, k, v)
+    assert (results[0] is not None) == served
+    assert torch.equal(got.nan_to_num(), want.nan_to_num())  # (5 % of 19 keys are none, and attention over none is NaN)
+    assert attention_wait_errors() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["one", "heads", "batches", "longer", "other type", "transposed"])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_masks_and_sink_logits(dtype, form):
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    B, Hq, Sq, S = 2, 8, 3, 700
+    q, k, v = _inputs(dt, B, Hq, 2, Sq, S, 64)
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    shape = {"heads": (1, Hq, Sq, S), "batches": (B, 1, Sq, S), "longer": (1, 1, Sq, S + 9), "transposed": (1, 1, S, Sq)}
+    am = torch.randn(shape.get(form, (1, 1, Sq, S)), generator=gen, device=DEV)
+    am = torch.where(am > 1.0, torch.finfo(dt).min, am).to(torch.float64 if form == "other type" else dt)
+    if form == "transposed":
+        am = am.transpose(2, 3)
+    sinks = torch.randn(Hq, generator=gen, device=DEV) if form in ("one", "heads") else None
+    for stack in (SINK_LOCAL, TOPK):
+        got, want = _both(workloads.research_attention(stack, dtype, DEV), q, k, v, am, sinks)
+        assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+def test_wrong_tensors_say_the_same():
+    ra = workloads.research_attention(TOPK, "f32", DEV)
+    q, k, v = _inputs(torch.float32, 1, 8, 2, 1, 300, 64)
+
+    def call(*args, am=None):
+        return ra.custom_attention(None, *args, am, 0.125, 0.0, sparse_meta_data={}, layer_idx=0)
+
+    with pytest.raises(ValueError, match="keys and values"):
+        call(q, k, v[:, :, :-1])
+    with pytest.raises(ValueError, match="covers"):
+        call(q, k, v, am=torch.zeros((1, 1, 1, 299), device=DEV))
+    with pytest.raises(ValueError, match="one dtype"):
+        call(q, k, v.bfloat16())
+    with pytest.raises(Exception, match="cpu"):
+        call(q.cpu(), k, v)
+    with pytest.raises(NotImplementedError, match="head dim"):
+        call(*(torch.randn((1, h, n, 32), device=DEV) for h, n in ((8, 1), (2, 300), (2, 300))))
+
+
+@pytest.mark.gpu
+def test_streams_and_capture():
+    """Two streams have tickets of their own; a captured call replays on new queries and keys."""
+    ra = workloads.research_attention(TOPK, "bf16", DEV)
+    q, k, v = _inputs(torch.bfloat16, 1, 8, 2, 1, 5000, 64)
+    q, k = q.contiguous(), k.contiguous()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call = lambda: ra.custom_attention(None, q, k, v, None, 0.125, 0.0, sparse_meta_data={}, layer_idx=0)[0]  # noqa: E731
+        warm = call()
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(warm, call())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = call()
+    q.copy_(torch.randn_like(q))
+    k.copy_(torch.randn_like(k))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, call())
+
+
+def test_other_stacks_keep_the_general_path():
+    """Nothing but plain sink, local and one final top-k masker is taken, whatever the tensors."""
+    class Cuda:  # stands in for a CUDA tensor: the maskers are looked at before anything else of it
+        pass
+
+    q = torch.zeros((1, 2, 1, 64))
+    assert fs.fixed_step([], q, q, q, None, None, 1.0) is None
+    assert fs.fixed_step([object()], q, q, q, None, None, 1.0) is None      # not on a CUDA device
+    assert fs.fixed_step([object()], Cuda(), q, q, None, None, 1.0) is None
