@@ -783,8 +783,8 @@ int sah_masked_attention_static(const uint32_t* bits, const void* q, const void*
  *
  * sah_fixed_step_plan fills the layout of the scratch (`total` bytes, 256-byte
  * aligned) from the extents and says SAH_ERR_UNSUPPORTED where the separate
- * entry points are the faster or the only way: more than 32768 keys without a
- * top-k, rows that sah_topk_select_fits spreads over the grid, too few
+ * entry points are the faster or the only way: several query positions over
+ * more than 32768 keys without a top-k, rows that sah_topk_select_fits spreads over the grid, too few
  * tickets. */
 #define SAH_STEP_MAX_BANDS 6
 typedef struct {
@@ -809,6 +809,7 @@ typedef struct {
 typedef struct {
   sah_attn_sizes sizes;
   int64_t words; /* of a bitmap row */
+  int32_t planned; /* 0: the attention kernel takes the bands themselves, there is no work list */
   int64_t total, scores, bits, ucols, umemb, ucount, partial; /* bytes; offsets in the scratch */
 } sah_fixed_step_layout;
 

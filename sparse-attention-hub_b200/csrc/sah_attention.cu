@@ -6,6 +6,7 @@
 //                          pipeline, weighted online softmax in fp32, every row
 //                          fetched once per group and shared by its query heads
 //   sah_attn_merge_parts   associative merge of sequence-sharded partials
+#include <algorithm>
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
@@ -541,6 +542,24 @@ __device__ __forceinline__ void at_cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
+// The union list of a mask that is bands alone, for one query position: the same columns for every row.
+// Entry u of the list is column u + shift[i] for the last i with start[i] <= u.  A decode call over a
+// sink and a window needs no plan then: the launch that wrote the list took 5.4 of 16.4 us (32 heads x
+// 4096 float32 keys, 10.2 us now), and no list of bands was found that is faster as a list (sink 128 and
+// windows of 256 to 7900 keys over 8 to 256 KV groups: 17.0 -> 8.0 us to 242 -> 179 us in bfloat16).
+#define ATTN_MAX_INTERVALS 8
+struct AttnIntervals {
+  int n, total;
+  int start[ATTN_MAX_INTERVALS], shift[ATTN_MAX_INTERVALS];
+};
+__device__ __forceinline__ int attn_interval_col(const AttnIntervals& iv, int u) {
+  int shift = iv.shift[0];
+#pragma unroll
+  for (int i = 1; i < ATTN_MAX_INTERVALS; ++i)
+    if (i < iv.n && u >= iv.start[i]) shift = iv.shift[i];
+  return u + shift;
+}
+
 struct AttnArgs {
   const void *q, *k, *v;
   int64_t qs_b, qs_h, qs_q, ks_b, ks_h, ks_s, vs_b, vs_h, vs_s;
@@ -564,6 +583,7 @@ struct AttnArgs {
   int k_rows_total, v_rows_total;
   int wave;            // CTAs per group that the device holds at once, two per SM
   int group_major;     // grid: 1 the splits of a group side by side, 0 the groups
+  AttnIntervals iv;    // instead of the list, where the kernel is instantiated for it
   int one_wave_tiles;  // tcgen05 kernel: tiles per CTA below which only half of the grid works
 };
 
@@ -588,7 +608,8 @@ static const char* g_last_attn_kernel = "none";
 #include "sah_attention_tc.cuh"
 #include "sah_attention_umma.cuh"
 
-template <typename T, int D, int NQUAD>
+// BANDS: the list is a.iv
+template <typename T, int D, int NQUAD, bool BANDS>
 __global__ void __launch_bounds__(AT_THREADS)
 masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __restrict__ sinks,
                         T* __restrict__ out, float* __restrict__ part_out) {
@@ -604,7 +625,7 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
   float* m_sm = p_sm + C::TILE * RP;                   // [RP]
   float* l_sm = m_sm + RP;                             // [RP]
   float* alpha_sm = l_sm + RP;                         // [RP]
-  int* cols_sm = reinterpret_cast<int*>(alpha_sm + RP);  // [STAGES][TILE]
+  int2* meta_sm = reinterpret_cast<int2*>(alpha_sm + RP);  // [STAGES][TILE] (column, membership)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int split = blockIdx.y;
@@ -622,7 +643,7 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
 
   // this CTA's slice of the group's union list: whole tiles, shared evenly by as many CTAs as there
   // are tiles, or as one wave of the device has for the group
-  const int U = a.ucount[g];
+  const int U = BANDS ? a.iv.total : a.ucount[g];
   const int total_tiles = (U + C::TILE - 1) / C::TILE;
   int active = total_tiles < a.nsplit ? total_tiles : a.nsplit;
   if (active > a.wave && total_tiles < a.nsplit * AT_ONE_WAVE_TILES) active = a.wave;
@@ -632,6 +653,23 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
   int end = (int)((int64_t)total_tiles * (split + 1) / active) * C::TILE;
   if (end > U) end = U;
   const int ntiles = (end - start + C::TILE - 1) / C::TILE;
+
+  // Column and membership of the tiles to issue are fetched two tiles early, a lane per entry.  (Loaded
+  // where they were needed, a dependent load per row of a tile and another in front of the softmax: 32
+  // heads x 16384 keys of which a head selects 968 15.8 us, 14.0 us so; 16 heads x 32768 16.4 -> 12.9 us.)
+  static_assert(C::TILE == 32, "a lane per entry of a tile");
+  struct Meta { int col; unsigned int memb; };
+  auto load_meta = [&](int t) {
+    Meta m;
+    m.col = -1; m.memb = 0u;
+    const int u = start + t * C::TILE + lane;
+    if (t < ntiles && u < end) {
+      m.col = BANDS ? attn_interval_col(a.iv, u) : gcols[u];
+      m.memb = BANDS ? ~0u : gmemb[u];
+    }
+    return m;
+  };
+  Meta pre0 = load_meta(0), pre1 = load_meta(1);
 
   // stage queries (fp32), reset softmax state
   for (int idx = tid; idx < RP * D; idx += AT_THREADS) {
@@ -666,12 +704,17 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
     const int st = t % AT_STAGES;
     unsigned char* kst = stage_base + st * C::STAGE_BYTES;
     unsigned char* vst = kst + C::TILE * C::ROWB;
-    const int t0 = start + t * C::TILE;
-    for (int idx = tid; idx < C::TILE * C::CPR; idx += AT_THREADS) {
-      const int i = idx / C::CPR, c = idx - i * C::CPR;
-      const int u = t0 + i;
-      if (u < end) {
-        const int64_t col = gcols[u];
+    const Meta cur = pre0;
+    pre0 = pre1;
+    pre1 = load_meta(t + 2);
+    if (warp == 0) meta_sm[st * C::TILE + lane] = make_int2(cur.col, (int)cur.memb);
+    constexpr int RPS = 32 / C::CPR;  // rows per warp and copy
+    const int c = lane % C::CPR;
+#pragma unroll
+    for (int n = 0; n < C::TILE; n += AT_THREADS / 32 * RPS) {
+      const int i = n + warp * RPS + lane / C::CPR;
+      const int64_t col = __shfl_sync(0xffffffffu, cur.col, i);
+      if (col >= 0) {
         const int slot = (c ^ (i & 7)) * 16;
         at_cp_async16(kst + i * C::ROWB + slot,
                       reinterpret_cast<const unsigned char*>(kbase + col * a.ks_s) + c * 16);
@@ -679,7 +722,6 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
                       reinterpret_cast<const unsigned char*>(vbase + col * a.vs_s) + c * 16);
       }
     }
-    if (tid < C::TILE) cols_sm[st * C::TILE + tid] = (t0 + tid < end) ? gcols[t0 + tid] : -1;
   };
 
 #pragma unroll
@@ -759,14 +801,15 @@ masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __re
         wv[kk] = 0.f;
         if (row_ok && i < nvalid) {
           const int u = t0 + i;
-          const unsigned int memb = gmemb[u];
+          const int2 meta = meta_sm[st * C::TILE + i];
+          const unsigned int memb = (unsigned int)meta.y;
           if ((memb >> r) & 1u) {
             float s = 0.f;
 #pragma unroll
             for (int pp = 0; pp < C::PARTS; ++pp) s += s_part[(pp * C::TILE + i) * RP + r];
             s *= a.scaling;
             if (a.bias != nullptr) {
-              const int64_t col = cols_sm[st * C::TILE + i];
+              const int64_t col = meta.x;
               s += sah_to_float<T>(reinterpret_cast<const T*>(
                   a.bias)[b * a.bias_s_b + h * a.bias_s_h + qi * a.bias_s_q + col]);
             }
@@ -890,24 +933,33 @@ static int launch_attention(const AttnArgs& a, int groups, int* tickets, const f
   size_t smem = (size_t)AT_STAGES * C::STAGE_BYTES +
                 sizeof(float) * ((size_t)RP * D + (size_t)C::PARTS * C::TILE * RP +
                                  (size_t)C::TILE * RP + 3 * RP) +
-                sizeof(int) * AT_STAGES * C::TILE;
+                sizeof(int2) * AT_STAGES * C::TILE;
   size_t red = sizeof(float) * 4 * RP * D;
   if (red > (size_t)AT_STAGES * C::STAGE_BYTES)
     return sah_fail(SAH_ERR_UNSUPPORTED, "attention: reduction buffer does not fit");
   dim3 grid((unsigned)groups, (unsigned)a.nsplit);
-#define SAH_AT_LAUNCH(NQ)                                                                        \
+#define SAH_AT_LAUNCH(NQ, BANDS)                                                                 \
   {                                                                                              \
-    cudaError_t e = cudaFuncSetAttribute(masked_attention_kernel<T, D, NQ>,                      \
+    cudaError_t e = cudaFuncSetAttribute(masked_attention_kernel<T, D, NQ, BANDS>,               \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "attention attr: %s", cudaGetErrorString(e)); \
-    sah_launch_chain(masked_attention_kernel<T, D, NQ>, grid, AT_THREADS, smem, st, a, tickets, sinks, \
+    sah_launch_chain(masked_attention_kernel<T, D, NQ, BANDS>, grid, AT_THREADS, smem, st, a, tickets, sinks, \
         (T*)out, part_out); \
   }
-  switch (nquad) {
-    case 1: SAH_AT_LAUNCH(1) break;
-    case 2: SAH_AT_LAUNCH(2) break;
-    case 3: SAH_AT_LAUNCH(3) break;
-    default: SAH_AT_LAUNCH(4) break;
+  if (a.iv.n > 0) {
+    switch (nquad) {
+      case 1: SAH_AT_LAUNCH(1, true) break;
+      case 2: SAH_AT_LAUNCH(2, true) break;
+      case 3: SAH_AT_LAUNCH(3, true) break;
+      default: SAH_AT_LAUNCH(4, true) break;
+    }
+  } else {
+    switch (nquad) {
+      case 1: SAH_AT_LAUNCH(1, false) break;
+      case 2: SAH_AT_LAUNCH(2, false) break;
+      case 3: SAH_AT_LAUNCH(3, false) break;
+      default: SAH_AT_LAUNCH(4, false) break;
+    }
   }
 #undef SAH_AT_LAUNCH
   return SAH_OK;
@@ -934,8 +986,9 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
                                  const sah_attn_sizes* sizes, const int32_t* ucols,
                                  const uint16_t* umemb, const float* uw, const int32_t* ucount,
                                  float* partial, void* out, float* part_out,
-                                 const AttnLsh* lsh, void* stream, int* own_tickets = nullptr) {
-  SAH_REQUIRE(q && k && v && sizes && ucols && umemb && ucount && partial && out,
+                                 const AttnLsh* lsh, void* stream, int* own_tickets = nullptr,
+                                 const AttnIntervals* iv = nullptr) {
+  SAH_REQUIRE(q && k && v && sizes && ((ucols && umemb && ucount) || (iv && own_tickets)) && partial && out,
               "masked_attention: null pointer");
   SAH_REQUIRE(B > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && Sq > 0 && S > 0,
               "masked_attention: bad extents");
@@ -968,6 +1021,7 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
   a.one_wave_tiles = a.group_major = 0;
   const int groups = sizes->groups;
   a.wave = attn_wave(groups);
+  a.iv = iv ? *iv : AttnIntervals();
   SAH_REQUIRE((int64_t)groups == (int64_t)B * Hkv * a.nqb && a.R == a.G * a.q_block &&
                   a.R <= AT_MAXR && a.nsplit >= 1,
               "masked_attention: sizes do not match the extents");
@@ -980,7 +1034,7 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
   if (dtype == SAH_BF16) {
     // tensor-core path; the split merge is fused into the kernel (ticket per group)
     // long lists: keys as the M dimension of tcgen05 tiles; otherwise the mma.sync kernel
-    const int umma = aum_requested();
+    const int umma = iv ? 0 : aum_requested();
     if (D == 128 && (umma == 1 || (umma < 0 && aum_default(lsh != nullptr, S, groups)))) {
       bool launched = false;
       rc = launch_attention_umma(a, B, groups, tickets, errflag, sinks, out, part_out, lsh != nullptr, st,
@@ -1439,6 +1493,38 @@ extern "C" int sah_masked_attention_static(
 // through the separate entry points, but for two bitmaps that nobody can ask for afterwards: the
 // bands are not written out.
 // ---------------------------------------------------------------------------
+// The columns that bands set for query position 0, as intervals of a list.
+static AttnIntervals step_intervals(const sah_fixed_step* s) {
+  AttnIntervals iv = {};
+  int64_t edge[2 * SAH_STEP_MAX_BANDS + 1];
+  int n = 0;
+  auto clip = [&](int64_t x) { return x < 0 ? 0 : x > s->S ? s->S : x; };
+  for (int i = 0; i < s->n_bands; ++i) {
+    edge[n++] = clip(s->bands[5 * i]);
+    edge[n++] = clip(s->bands[5 * i + 2]);
+  }
+  edge[n++] = 0;
+  std::sort(edge, edge + n);
+  int64_t open = -1;  // where the interval at hand began
+  for (int e = 0; e < n; ++e) {
+    const int64_t lo = edge[e], hi = e + 1 < n ? edge[e + 1] : s->S;
+    if (lo == hi) continue;
+    bool on = false;
+    for (int i = 0; i < s->n_bands; ++i)
+      if (s->bands[5 * i] <= lo && s->bands[5 * i + 2] >= hi) on = s->bands[5 * i + 4] != 0;
+    if (on && open < 0) open = lo;
+    if (open >= 0 && (!on || hi == s->S)) {
+      const int64_t end = on ? hi : lo;
+      iv.start[iv.n] = iv.total;
+      iv.shift[iv.n] = (int)(open - iv.total);
+      iv.total += (int)(end - open);
+      ++iv.n;
+      open = -1;
+    }
+  }
+  return iv;
+}
+
 static_assert(SAH_STEP_MAX_BANDS == SAH_MAX_BANDS, "one limit");
 
 extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layout* o) {
@@ -1449,7 +1535,13 @@ extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layou
   if (rc != SAH_OK) return rc;
   const int64_t rows = (int64_t)s->B * s->Hq * s->Sq;
   o->words = sah_ceil_div(sah_ceil_div(s->S, 32), 4) * 4;
-  if (o->sizes.groups >= s->n_tickets || (s->heavy == 0 && s->S > 32768) ||
+  SAH_REQUIRE(s->n_bands >= 0 && s->n_bands <= SAH_STEP_MAX_BANDS, "fixed_step_plan: 0..%d bands", SAH_STEP_MAX_BANDS);
+  o->planned = 1;
+  if (s->heavy == 0 && s->Sq == 1 && s->S < (1ll << 31)) {
+    const int64_t total = step_intervals(s).total;
+    o->planned = total == 0;
+  }
+  if (o->sizes.groups >= s->n_tickets || (s->heavy == 0 && o->planned && s->S > 32768) ||
       (s->heavy > 0 && sah_topk_select_fits(s->dtype, rows, s->S, o->words) == 0))
     return SAH_ERR_UNSUPPORTED;  // (no message: the caller has another way)
   int64_t at = 0;
@@ -1460,9 +1552,9 @@ extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layou
   };
   o->scores = take(s->heavy > 0 ? rows * s->S * (s->dtype == SAH_BF16 ? 2 : 4) : 0);
   o->bits = take(s->heavy > 0 ? rows * o->words * 4 : 0);
-  o->ucols = take(o->sizes.ucols_bytes);
-  o->umemb = take(o->sizes.umemb_bytes);
-  o->ucount = take(o->sizes.ucount_bytes);
+  o->ucols = take(o->planned ? o->sizes.ucols_bytes : 0);
+  o->umemb = take(o->planned ? o->sizes.umemb_bytes : 0);
+  o->ucount = take(o->planned ? o->sizes.ucount_bytes : 0);
   o->partial = take(o->sizes.partial_bytes);
   o->total = at;
   return SAH_OK;
@@ -1475,8 +1567,11 @@ extern "C" int sah_fixed_step_run(const sah_fixed_step* s, const sah_fixed_step_
   unsigned char* p = (unsigned char*)s->scratch;
   int32_t *ucols = (int32_t*)(p + o->ucols), *ucount = (int32_t*)(p + o->ucount);
   uint16_t* umemb = (uint16_t*)(p + o->umemb);
-  int rc;
-  if (s->heavy > 0) {
+  int rc = SAH_OK;
+  AttnIntervals iv;
+  if (!o->planned) {
+    iv = step_intervals(s);
+  } else if (s->heavy > 0) {
     rc = sah_qk_scores(s->q, s->k, s->dtype, s->q_stride[0], s->q_stride[1], s->q_stride[2], s->k_stride[0], s->k_stride[1],
                        s->k_stride[2], s->B, s->Hq, s->Hkv, s->Sq, s->S, s->D, s->bias, s->bias_stride[0],
                        s->bias_stride[1], s->bias_stride[2], p + o->scores, stream);
@@ -1496,5 +1591,6 @@ extern "C" int sah_fixed_step_run(const sah_fixed_step* s, const sah_fixed_step_
                                s->k_stride[1], s->k_stride[2], s->v_stride[0], s->v_stride[1], s->v_stride[2], s->B, s->Hq,
                                s->Hkv, s->Sq, s->S, s->D, s->scaling, s->bias, s->bias_stride[0], s->bias_stride[1],
                                s->bias_stride[2], s->sinks, &o->sizes, ucols, umemb, nullptr, ucount,
-                               (float*)(p + o->partial), s->out, nullptr, nullptr, stream, s->tickets);
+                               (float*)(p + o->partial), s->out, nullptr, nullptr, stream, s->tickets,
+                               o->planned ? nullptr : &iv);
 }

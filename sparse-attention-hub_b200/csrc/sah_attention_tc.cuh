@@ -267,7 +267,8 @@ __device__ __forceinline__ void atm_finish_group(const AttnArgs& a, int64_t g, i
 // NST: stages of the per-warp ring.  Three stages fit two CTAs (8 warps) per SM; two stages,
 // with the register count capped accordingly, fit three CTAs (12 warps): fewer tiles in flight
 // per warp, more warps to overlap one warp's arithmetic with the others' copies.
-template <int D, bool HALF, bool LSHW, bool TMA, int NST>
+// BANDS: the list is a.iv.
+template <int D, bool HALF, bool LSHW, bool TMA, int NST, bool BANDS>
 __global__ void __launch_bounds__(ATM_THREADS, NST == 2 ? 3 : 2)
 masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, int* __restrict__ tickets,
                             int* __restrict__ errflag, const float* __restrict__ sinks,
@@ -316,7 +317,7 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
   const float* ginv = LSHW ? a.uw + g * a.S : nullptr;  // 1 / (M * |transformed key|) per entry
 
   // ---- this warp's tiles ----
-  const int U = a.ucount[g];
+  const int U = BANDS ? a.iv.total : a.ucount[g];
   const int total_tiles = (U + ATM_TILE - 1) / ATM_TILE;
   const int active = atm_active_splits(total_tiles, a.nsplit, a.wave);
   if (split >= active) return;
@@ -335,8 +336,8 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
     if (t < my_tiles) {
       const int u = (my_first + t * lanes_total) * ATM_TILE + lane;
       if (lane < ATM_TILE && u < U) {
-        m.col = gcols[u];
-        m.memb = gmemb[u];
+        m.col = BANDS ? attn_interval_col(a.iv, u) : gcols[u];
+        m.memb = BANDS ? (1u << a.R) - 1u : gmemb[u];
         if constexpr (LSHW) m.inv = ginv[u];
       }
     }
@@ -856,7 +857,7 @@ template <int D>
 static int launch_attention_mma(AttnArgs a, int B, int groups, int* tickets, int* errflag,
                                 const float* sinks, void* out, float* part_out, bool lsh,
                                 cudaStream_t st) {
-  static bool allowed[9][64] = {};
+  static bool allowed[11][64] = {};
   static_assert(AtmCfg<D, false, 2>::RED_BYTES <= AtmCfg<D, false, 2>::WARP_BYTES &&
                 AtmCfg<D, true, 2>::RED_BYTES <= AtmCfg<D, true, 2>::WARP_BYTES,
                 "reduction scratch must fit the ring");
@@ -879,26 +880,29 @@ static int launch_attention_mma(AttnArgs a, int B, int groups, int* tickets, int
   }
   const bool two = atm_stages_requested() == 2;
   cudaError_t e = cudaSuccess;
-#define ATM_LAUNCH(HALF, LSHW, TMA, NST, SLOT)                                                      \
+#define ATM_LAUNCH(HALF, LSHW, TMA, NST, BANDS, SLOT)                                                      \
   do {                                                                                              \
     const int smem = AtmCfg<D, TMA, NST>::SMEM;                                                     \
-    e = sah_allow_smem(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, smem, allowed[SLOT]);  \
+    e = sah_allow_smem(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST, BANDS>, smem, allowed[SLOT]);  \
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "attention attr: %s", cudaGetErrorString(e)); \
-    sah_launch_chain(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST>, grid, ATM_THREADS, smem, st, \
+    sah_launch_chain(masked_attention_mma_kernel<D, HALF, LSHW, TMA, NST, BANDS>, grid, ATM_THREADS, smem, st, \
         a, maps, tickets, errflag, sinks, (__nv_bfloat16*)out, part_out);                           \
   } while (0)
-  if (lsh) {
-    if (tma && two) ATM_LAUNCH(true, true, true, 2, 5);
-    else if (tma) ATM_LAUNCH(true, true, true, 3, 3);
-    else if (two) ATM_LAUNCH(true, true, false, 2, 6);
-    else ATM_LAUNCH(true, true, false, 3, 2);
+  if (a.iv.n > 0) {
+    if (a.R <= 8) ATM_LAUNCH(true, false, false, 3, true, 9);
+    else ATM_LAUNCH(false, false, false, 3, true, 10);
+  } else if (lsh) {
+    if (tma && two) ATM_LAUNCH(true, true, true, 2, false, 5);
+    else if (tma) ATM_LAUNCH(true, true, true, 3, false, 3);
+    else if (two) ATM_LAUNCH(true, true, false, 2, false, 6);
+    else ATM_LAUNCH(true, true, false, 3, false, 2);
   } else if (a.R <= 8) {
-    if (tma && two) ATM_LAUNCH(true, false, true, 2, 7);
-    else if (tma) ATM_LAUNCH(true, false, true, 3, 4);
-    else if (two) ATM_LAUNCH(true, false, false, 2, 8);
-    else ATM_LAUNCH(true, false, false, 3, 0);
+    if (tma && two) ATM_LAUNCH(true, false, true, 2, false, 7);
+    else if (tma) ATM_LAUNCH(true, false, true, 3, false, 4);
+    else if (two) ATM_LAUNCH(true, false, false, 2, false, 8);
+    else ATM_LAUNCH(true, false, false, 3, false, 0);
   } else {
-    ATM_LAUNCH(false, false, false, 3, 1);
+    ATM_LAUNCH(false, false, false, 3, false, 1);
   }
 #undef ATM_LAUNCH
   return SAH_OK;

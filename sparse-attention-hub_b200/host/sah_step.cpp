@@ -47,7 +47,8 @@ bool rows_of(const at::Tensor& t, int64_t* strides) {
 
 // fixed_step(queries, keys, values, attention_mask or None, sinks or None, scaling, bands, heavy, tickets,
 //            sm_count, stream)
-// -> None, a non-zero status, or (out, scratch, offsets of ucols, umemb and ucount in it, groups, rows per group)
+// -> None, a non-zero status, or (out, scratch, offsets of ucols (-1: there is no list), umemb and ucount in it, groups,
+//     rows per group)
 PyObject* fixed_step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   if (nargs != 11 || plan_fn == nullptr) {
@@ -125,7 +126,7 @@ PyObject* fixed_step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (result == nullptr) return nullptr;
   PyTuple_SET_ITEM(result, 0, THPVariable_Wrap(std::move(out)));
   PyTuple_SET_ITEM(result, 1, THPVariable_Wrap(std::move(scratch)));
-  PyTuple_SET_ITEM(result, 2, PyLong_FromLongLong(layout.ucols));
+  PyTuple_SET_ITEM(result, 2, PyLong_FromLongLong(layout.planned ? layout.ucols : -1));
   PyTuple_SET_ITEM(result, 3, PyLong_FromLongLong(layout.umemb));
   PyTuple_SET_ITEM(result, 4, PyLong_FromLongLong(layout.ucount));
   PyTuple_SET_ITEM(result, 5, PyLong_FromLong(layout.sizes.groups));

@@ -104,6 +104,6 @@ def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values:
         _native.check(done, "sah_fixed_step_run")
     out, scratch, ucols, umemb, ucount, groups, rows = done
     B, Hq, _, D = queries.shape
-    mask_attention_utils._last_plan["step"] = (scratch, ucols, umemb, ucount, groups, rows, S,
+    mask_attention_utils._last_plan["step"] = (scratch, ucols, umemb, ucount, groups, rows, S, bands,
                                                (B, Hq, keys.shape[1], Sq, S, D, 0, _native.sm_count(device)))
     return out

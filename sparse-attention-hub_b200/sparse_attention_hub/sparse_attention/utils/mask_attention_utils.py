@@ -222,13 +222,24 @@ _last_plan: Dict[str, Any] = {"ucount": None, "ws": None, "sizes": None, "step":
 
 def _last() -> Dict[str, Any]:
     if _last_plan["step"] is not None:
-        scratch, ucols, umemb, ucount, groups, rows, S, extents = _last_plan["step"]
+        scratch, ucols, umemb, ucount, groups, rows, S, bands, extents = _last_plan["step"]
 
         def part(offset, count, dtype):
             return scratch[offset:offset + count * dtype.itemsize].view(dtype)
 
-        ws = {"ucols": part(ucols, groups * S, torch.int32), "umemb": part(umemb, groups * S, torch.int16),
-              "ucount": part(ucount, groups, torch.int32)}
+        if ucols >= 0:
+            ws = {"ucols": part(ucols, groups * S, torch.int32), "umemb": part(umemb, groups * S, torch.int16),
+                  "ucount": part(ucount, groups, torch.int32)}
+        else:  # the kernel went by the bands: the list it walked, the same for every group
+            on = torch.zeros(S, dtype=torch.bool, device=scratch.device)
+            for lo, _, hi, _, value in zip(*[iter(bands)] * 5):
+                on[max(lo, 0):max(hi, 0)] = bool(value)
+            columns = on.nonzero().flatten().to(torch.int32)
+            ws = {"ucols": torch.zeros((groups, S), dtype=torch.int32, device=scratch.device),
+                  "umemb": torch.full((groups * S,), (1 << rows) - 1, dtype=torch.int32, device=scratch.device).to(torch.int16),
+                  "ucount": torch.full((groups,), columns.numel(), dtype=torch.int32, device=scratch.device)}
+            ws["ucols"][:, :columns.numel()] = columns
+            ws["ucols"] = ws["ucols"].flatten()
         _last_plan.update(ucount=ws["ucount"], ws=ws, sizes=(groups, rows, S),
                           attn_sizes=_native.attn_sizes(*extents), step=None)
     return _last_plan

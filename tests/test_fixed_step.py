@@ -8,7 +8,7 @@ import workloads
 from sparse_attention_hub.sparse_attention.research_attention import base
 from sparse_attention_hub.sparse_attention.research_attention import fixed_step as fs
 from sparse_attention_hub.sparse_attention.utils.mask_attention_utils import (
-    attention_wait_errors, get_masked_attention_output, last_union_counts)
+    attention_wait_errors, get_masked_attention_output, last_union_list)
 
 DEV = "cuda:0"
 SINK_LOCAL = [("sink", {"sink_size": 5}), ("local", {"window_size": 37})]
@@ -27,11 +27,14 @@ def _inputs(dt, B, Hq, Hkv, Sq, S, D, layout="plain"):
 
 def _both(ra, q, k, v, am=None, sinks=None):
     out, weights = ra.custom_attention(None, q, k, v, am, 0.125, 0.0, sparse_meta_data={}, layer_idx=0, s_aux=sinks)
-    counts = last_union_counts().clone()
+    ucols, umemb, counts, _ = (t.clone() if isinstance(t, torch.Tensor) else t for t in last_union_list())
     mask = ra.build_mask(q, k, v, am, 0.125, 0.0, {}, layer_idx=0)
     want = get_masked_attention_output(None, q, k, v, am, sinks, 0.125, 0.0, mask)
     assert weights is None
-    assert torch.equal(counts, last_union_counts())
+    ucols_, umemb_, counts_, _ = last_union_list()
+    assert torch.equal(counts, counts_)
+    for g, n in enumerate(counts.tolist()):
+        assert torch.equal(ucols[g, :n], ucols_[g, :n]) and torch.equal(umemb[g, :n], umemb_[g, :n])
     return out, want
 
 
@@ -40,6 +43,7 @@ def _both(ra, q, k, v, am=None, sinks=None):
 @pytest.mark.parametrize("dtype,Sq,S,D,stack,served", [
     ("f32", 1, 43, 64, "fixed", True), ("f32", 1, 42, 64, "fixed", True), ("f32", 1, 38, 64, "fixed", False),
     ("bf16", 3, 131, 64, "fixed", True), ("bf16", 1, 32768, 128, "fixed", True), ("bf16", 2, 32769, 64, "fixed", False),
+    ("bf16", 1, 50001, 64, "fixed", True),
     ("bf16", 1, 4097, 128, "topk", True), ("f32", 4, 1000, 64, "topk", True), ("bf16", 1, 90000, 64, "topk", False),
     ("bf16", 24, 8191, 128, "topk", True), ("f32", 2, 40000, 64, "topk", True), ("bf16", 1, 19, 64, "topk only", False),
     ("bf16", 2, 260, 64, "topk only", True)])
@@ -57,7 +61,8 @@ def test_same_as_the_general_path(dtype, Sq, S, D, stack, served, layout, monkey
     monkeypatch.setattr(base, "fixed_step", noted)
     got, want = _both(ra, q, k, v)
     assert (results[0] is not None) == served
-    assert torch.equal(got.nan_to_num(), want.nan_to_num())  # (5 % of 19 keys are none, and attention over none is NaN)
+    got, want = got.nan_to_num(), want.nan_to_num()  # (5 % of 19 keys are none, and attention over none is NaN)
+    assert torch.equal(got, want)
     assert attention_wait_errors() == 0
 
 
@@ -98,6 +103,19 @@ def test_wrong_tensors_say_the_same():
         call(q.cpu(), k, v)
     with pytest.raises(NotImplementedError, match="head dim"):
         call(*(torch.randn((1, h, n, 32), device=DEV) for h, n in ((8, 1), (2, 300), (2, 300))))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Hq,Hkv", [(8, 8), (8, 1), (32, 2)])
+@pytest.mark.parametrize("maskers", [
+    [("sink", {"sink_size": 1})], [("local", {"window_size": 1})], [("local", {"window_size": 300}), ("sink", {"sink_size": 400})],
+    [("sink", {"sink_size": 3}), ("local", {"window_size": 9}), ("sink", {"sink_size": 64}), ("local", {"window_size": 640})]])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_lists_of_bands(dtype, maskers, Hq, Hkv):
+    """Bands that overlap, that come in another order, that are one column; up to sixteen rows per group."""
+    q, k, v = _inputs(torch.bfloat16 if dtype == "bf16" else torch.float32, 2, Hq, Hkv, 1, 701, 128)
+    got, want = _both(workloads.research_attention(maskers, dtype, DEV), q, k, v)
+    assert torch.equal(got, want)
 
 
 @pytest.mark.gpu
