@@ -10,11 +10,12 @@
 //         -|c|^2 / 2 split the same way,
 //   so that two tcgen05.mma (K = 16) give a_c = x . c - |c|^2 / 2 = (|x|^2 - distance) / 2 and the
 //   nearest centroid is the largest a_c.  One thread per key reads its row of a_c from tensor
-//   memory twice: first the maximum (three-operand maximum: half an instruction per value), then
-//   the sign of a_c - (max - E) shifted into a bit mask (an addition and a funnel shift per
-//   value).  One bit set: that is the answer.  Several: the fixed-order float32 distance
-//   (dimensions ascending, (x - c)^2 rounded, then added) of those, first minimum wins, as
-//   torch.argmin does.
+//   memory once, as a matrix of 16 columns, and keeps the largest value of every matrix row and of
+//   every matrix column: half an instruction per value each (three-operand maximum).  The overall
+//   maximum lies where a row's and a column's meet; a centroid within E of it shows in both.  One row
+//   and one column within E: that centroid is the answer.  Otherwise the fixed-order float32
+//   distance (dimensions ascending, (x - c)^2 rounded, then added) of all centroids where such rows
+//   and columns meet, first minimum wins, as torch.argmin does.
 //   E = 2^-16 (|x|^2 + max_c |c|^2).  A float32 sum of 27 exact products, in whatever order and
 //   even truncated, is within 27 * 2^-23 (|x||c| + |c|^2 / 2) <= 2^-18.2 (|x|^2 + |c|^2) of the
 //   exact one; the fixed-order distance is within 10 * 2^-24 * 2 (|x|^2 + |c|^2) <= 2^-19.6 (...)
@@ -22,32 +23,35 @@
 //   ordered the other way round therefore differ by less than 0.6 E in a_c: the fixed-order argmin
 //   is always among the candidates, and the codes equal pq_assign_kernel's bit for bit.
 //
-// Bound: the vector instructions of the epilogue, about 2.5 per (key, centroid), half of them on
-// the 16-lane ALU pipe; 8 KV heads x 65472 keys x 16 sub-vectors x 256 centroids are 2.1e9 pairs,
-// 0.18 ms at that rate; measured 0.45 ms.  The previous form (product and |c|^2 apart, E sixteen
-// times wider, a branch per centroid in the second pass) took 5.07 ms for it.
+// Bound: the vector instructions of the epilogue, 1.25 per (key, centroid) on the 16-lane ALU pipe.
+// 8 KV heads x 65472 keys x 16 sub-vectors x 256 centroids are 2.1e9 pairs, 0.15 ms at that rate;
+// measured 0.24 ms.  With the row read twice (maximum, then the sign of a_c - (max - E) shifted into
+// a bit mask, 2.5 instructions per pair) and the product issued by a thread of the epilogue behind
+// a barrier of its group it took 0.46 ms.  The product in halves of 128 columns, each handed back by
+// itself, takes 0.26 ms, two products under way 0.31 ms: what remains are instructions, not waits.
 //
-// One CTA of 256 threads per SM holding all of tensor memory: two groups of four warps, each with
-// an accumulator of 256 columns and an A tile of its own, so that one group's product and waits
-// hide behind the other's epilogue.  A CTA carries NS neighbouring sub-vectors (a key's 64
-// contiguous bytes for NS = 4: whole sectors, and one 4-byte store of codes) and a contiguous
-// share of the flattened (sub-vector block, key tile) space, cut evenly over the SMs; the B tiles
-// are rebuilt when the share crosses into another block.  The only mbarrier wait
-// (tcgen05.commit) is bounded; when it runs out the error word is set, and the threads walk
-// through their remaining tiles without working on them.
+// One CTA of 320 threads per SM holding all of tensor memory: two groups of four warps, each with
+// an accumulator of 256 columns and an A tile of its own, and a warp per group that issues its
+// products.  A group writes the A rows of its next product as soon as the present one is complete
+// and hands the accumulator back when its last columns are in registers, so that the next product
+// runs behind the rest of the epilogue and behind the other group's.  A CTA carries NS neighbouring
+// sub-vectors (a key's 64 contiguous bytes for NS = 4: whole sectors, and one 4-byte store of codes)
+// and a contiguous share of the flattened (sub-vector block, key tile) space, cut evenly over the
+// SMs; the B tiles are rebuilt when the share crosses into another block.  The mbarrier waits are
+// bounded; when one runs out the error word is set, and the threads walk through their remaining
+// tiles without working on them.
 #pragma once
 #include "sah_tcgen05.cuh"
 
 #define PTC_TILE 128
-#define PTC_THREADS 256
+#define PTC_THREADS 320  // two groups of four warps, and an issuing warp for each
 
 template <int NS>
 struct PtcCfg {
   static constexpr int A_OFF = 0;                                // two groups' [128 rows][128 B], first 64 B used
   static constexpr int B_OFF = 2 * PTC_TILE * 128;               // NS x [256 rows][128 B], first 64 B used
   static constexpr int CENT_OFF = B_OFF + NS * 256 * 128;        // NS x float32 [256][8]
-  static constexpr int CAND_OFF = CENT_OFF + NS * 256 * 8 * 4;   // candidate masks [8][threads]
-  static constexpr int MISC_OFF = CAND_OFF + 8 * PTC_THREADS * 4;  // max |c|^2 per sub-vector, mbarriers, slot, abort
+  static constexpr int MISC_OFF = CENT_OFF + NS * 256 * 8 * 4;   // max |c|^2 per sub-vector, mbarriers, slot, abort
   static constexpr int NEED = 1024 + MISC_OFF + 128;
   // never less than half of an SM's shared memory: one CTA per SM, it holds all of tensor memory
   static constexpr int SMEM = NEED > 120 * 1024 ? NEED : 120 * 1024;
@@ -90,20 +94,27 @@ __device__ __forceinline__ void ptc_split3(float v, __nv_bfloat16* h, __nv_bfloa
   *l = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(*m)));
 }
 
-__device__ __forceinline__ void ptc_max_block(const uint32_t* v, float* mx) {
+// 32 columns of an accumulator: two matrix rows of 16
+__device__ __forceinline__ void ptc_fold(const uint32_t* v, float* row, float* col) {
+  auto f = [&](int i) { return __uint_as_float(v[i]); };
 #pragma unroll
-  for (int i = 0; i < 32; i += 2)
-    mx[(i >> 1) & 3] = ptc_max3(mx[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+  for (int q = 0; q < 16; ++q) col[q] = ptc_max3(col[q], f(q), f(16 + q));
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int o = 16 * h;
+    float a = ptc_max3(f(o), f(o + 1), f(o + 2)), b = ptc_max3(f(o + 3), f(o + 4), f(o + 5));
+    a = ptc_max3(a, f(o + 6), f(o + 7)), b = ptc_max3(b, f(o + 8), f(o + 9));
+    a = ptc_max3(a, f(o + 10), f(o + 11)), b = ptc_max3(b, f(o + 12), f(o + 13));
+    row[h] = fmaxf(ptc_max3(a, f(o + 14), f(o + 15)), b);
+  }
 }
-// bit 31 - i: value i is not below thr (or is NaN); four short chains of shifts
-__device__ __forceinline__ uint32_t ptc_candidates(const uint32_t* v, float thr) {
-  uint32_t below[4] = {0u, 0u, 0u, 0u};
+// bit i: value i is not below thr (or one of the two is NaN)
+template <int N>
+__device__ __forceinline__ uint32_t ptc_near(const float* v, float thr) {
+  uint32_t m = 0u;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      below[q] = __funnelshift_l(__float_as_uint(__fsub_rn(__uint_as_float(v[q * 8 + i]), thr)), below[q], 1);
-  return ~((below[0] << 24) | (below[1] << 16) | (below[2] << 8) | below[3]);
+  for (int i = N - 1; i >= 0; --i) m = __funnelshift_l(__float_as_uint(__fsub_rn(v[i], thr)), m, 1);
+  return ~m & (N == 32 ? 0xffffffffu : (1u << (N & 31)) - 1u);
 }
 
 // NB: blocks of 32 accumulator columns (n_cent <= 32 NB; the columns past n_cent hold -inf)
@@ -120,16 +131,20 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
   unsigned char* sm = ptc_raw + (((raw_s + 1023u) & ~1023u) - raw_s);
   const uint32_t sm_s = (uint32_t)__cvta_generic_to_shared(sm);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wg = tid >> 7, keyl = tid & 127;  // group of four warps, key of its tile
+  const bool issuer = warp >= 8;
+  const int wg = issuer ? warp - 8 : warp >> 2, keyl = tid & 127;  // group of four warps, key of its tile
   float* cent_sm = reinterpret_cast<float*>(sm + C::CENT_OFF);
-  uint32_t* cand_sm = reinterpret_cast<uint32_t*>(sm + C::CAND_OFF);
   unsigned int* cmax_sm = reinterpret_cast<unsigned int*>(sm + C::MISC_OFF);  // [NS], float bits
-  const uint32_t bar = sm_s + C::MISC_OFF + 32 + wg * 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + C::MISC_OFF + 48);
-  volatile int* abort_sm = reinterpret_cast<volatile int*>(sm + C::MISC_OFF + 52);
+  const uint32_t full = sm_s + C::MISC_OFF + 32 + wg * 8;   // the group's product is complete
+  const uint32_t ready = sm_s + C::MISC_OFF + 48 + wg * 8;  // its A rows are written, its accumulator is read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + C::MISC_OFF + 64);
+  volatile int* abort_sm = reinterpret_cast<volatile int*>(sm + C::MISC_OFF + 68);
 
-  if (keyl == 0) atm_mbar_init(bar, 1);
   if (tid == 0) {
+    for (int g = 0; g < 2; ++g) {
+      atm_mbar_init(sm_s + C::MISC_OFF + 32 + g * 8, 1);
+      atm_mbar_init(sm_s + C::MISC_OFF + 48 + g * 8, 4);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     *abort_sm = 0;
   }
@@ -140,7 +155,7 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
   }
   unsigned char* arow = sm + C::A_OFF + wg * (PTC_TILE * 128) + keyl * 128;
-  {  // chunk 3 of an A row (the factors of -|c|^2 / 2) never changes
+  if (!issuer) {  // chunk 3 of an A row (the factors of -|c|^2 / 2) never changes
     const uint32_t one2 = 0x3f803f80u;
     *reinterpret_cast<uint4*>(arow + ((3 ^ (keyl & 7)) << 4)) = make_uint4(one2, 0x3f80u, 0u, 0u);
   }
@@ -191,101 +206,121 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
     const int64_t seg_end = (blk + 1) * n_tiles < it_end ? (blk + 1) * n_tiles : it_end;
-    uint4 raw[NS];
-    {
-      const int64_t j = key_begin + (it + wg - blk * n_tiles) * PTC_TILE + keyl;
-#pragma unroll
-      for (int s = 0; s < NS; ++s)
-        raw[s] = it + wg < seg_end && j < key_end ? *reinterpret_cast<const uint4*>(xb + j * xs_s + s * SD)
-                                                  : make_uint4(0u, 0u, 0u, 0u);
+    if (issuer) {
+      int left = it + wg < seg_end ? (int)((seg_end - it - wg + 1) >> 1) : 0;
+      for (; left > 0; --left) {
+#pragma unroll 1
+        for (int s = 0; s < NS; ++s) {
+          const bool ok = aum_wait_warp(ready, phase, abort_sm, errflag);
+          phase ^= 1u;
+          if (ok && lane == 0) {
+            aum_fence_after();
+            const uint32_t b_s = sm_s + C::B_OFF + s * (256 * 128);
+            aum_mma(tmem, aum_desc(a_s, 0, 1024, 2), aum_desc(b_s, 0, 1024, 2), idesc, 0u);
+            aum_mma(tmem, aum_desc(a_s + 32, 0, 1024, 2), aum_desc(b_s + 32, 0, 1024, 2), idesc, 1u);
+            aum_commit(full);
+          }
+          __syncwarp();
+        }
+      }
+      it = seg_end;
+      continue;
     }
-    for (int64_t t = it + wg; t < seg_end; t += 2) {
-      const int64_t j = key_begin + (t - blk * n_tiles) * PTC_TILE + keyl;
-      uint4 next[NS];
-      const int64_t jn = j + 2 * PTC_TILE;
-#pragma unroll
-      for (int s = 0; s < NS; ++s)
-        next[s] = t + 2 < seg_end && jn < key_end ? *reinterpret_cast<const uint4*>(xb + jn * xs_s + s * SD)
-                                                  : make_uint4(0u, 0u, 0u, 0u);
+    const int my_tiles = it + wg < seg_end ? (int)((seg_end - it - wg + 1) >> 1) : 0;
+    const int64_t j_first = key_begin + (it + wg - blk * n_tiles) * PTC_TILE + keyl;
+    const int64_t keys_left = key_end - j_first;
+    // tiles of this thread's share in which its key exists
+    const int have = keys_left <= 0 ? 0 : (int)min((int64_t)my_tiles, (keys_left + 2 * PTC_TILE - 1) / (2 * PTC_TILE));
+    const __nv_bfloat16* xp = xb + j_first * xs_s;   // its row in the tile that is fetched next
+    int ft = 0, fs = 0;
+    // the 16 bytes of its next sub-vector; all but the first of a key come out of L1
+    auto fetch = [&] {
+      const uint4 r = ft < have ? *reinterpret_cast<const uint4*>(xp + fs * SD) : make_uint4(0u, 0u, 0u, 0u);
+      if (++fs == NS) {
+        fs = 0;
+        ++ft;
+        xp += 2 * PTC_TILE * xs_s;
+      }
+      return r;
+    };
+    uint4 rw = fetch();  // the present product's
+    uint4 rn = fetch();  // the next one's
+    auto put_a = [&](const uint4& rw) {
+      *reinterpret_cast<uint4*>(arow + ((0 ^ (keyl & 7)) << 4)) = rw;
+      *reinterpret_cast<uint4*>(arow + ((1 ^ (keyl & 7)) << 4)) = rw;
+      *reinterpret_cast<uint4*>(arow + ((2 ^ (keyl & 7)) << 4)) = rw;
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    };
+    auto hand_over = [&] {
+      aum_fence_before();
+      __syncwarp();
+      if (lane == 0) aum_arrive(ready);
+    };
+    if (my_tiles > 0) {
+      put_a(rw);
+      hand_over();
+    }
+    uint8_t* dst = codes + (bk * cap + (j_first - init_offset)) * n_sub + sub0;
+#pragma unroll 1
+    for (int t = 0; t < my_tiles; ++t) {
       uint32_t packed = 0u;
 #pragma unroll 1
       for (int s = 0; s < NS; ++s) {
-        uint4 rw = raw[0];
-#pragma unroll
-        for (int q = 1; q < NS; ++q)
-          if (s == q) rw = raw[q];
-        *reinterpret_cast<uint4*>(arow + ((0 ^ (keyl & 7)) << 4)) = rw;
-        *reinterpret_cast<uint4*>(arow + ((1 ^ (keyl & 7)) << 4)) = rw;
-        *reinterpret_cast<uint4*>(arow + ((2 ^ (keyl & 7)) << 4)) = rw;
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        aum_fence_before();
-        // the group's A rows are written and its reads of the previous accumulator are done
-        asm volatile("bar.sync %0, 128;\n" ::"r"(1 + wg) : "memory");
-        if (keyl == 0 && !*abort_sm) {
-          aum_fence_after();
-          const uint32_t b_s = sm_s + C::B_OFF + s * (256 * 128);
-          aum_mma(tmem, aum_desc(a_s, 0, 1024, 2), aum_desc(b_s, 0, 1024, 2), idesc, 0u);
-          aum_mma(tmem, aum_desc(a_s + 32, 0, 1024, 2), aum_desc(b_s + 32, 0, 1024, 2), idesc, 1u);
-          aum_commit(bar);
-        }
-        float xv[SD];
-        sah_unpack8(rw, xv);
+        const bool more = s + 1 < NS || t + 1 < my_tiles;
+        const uint4 rnn = fetch();
         float x2 = 0.f;
+        {
+          float xv[SD];
+          sah_unpack8(rw, xv);
 #pragma unroll
-        for (int d = 0; d < SD; ++d) x2 = fmaf(xv[d], xv[d], x2);
+          for (int d = 0; d < SD; ++d) x2 = fmaf(xv[d], xv[d], x2);
+        }
         const float margin = 1.52587890625e-05f * (x2 + __uint_as_float(cmax_sm[s]));  // E
-        const bool ok = aum_wait_warp(bar, phase, abort_sm, errflag);
+        const bool ok = aum_wait_warp(full, phase, abort_sm, errflag);
         phase ^= 1u;
         if (!ok) continue;
         aum_fence_after();
         uint32_t va[32], vb[32];
-        // ---- the largest a_c; the loops stay rolled over pairs of blocks, which keeps the two
-        //      buffers the only long-lived values (unrolled, the kernel spilled) ----
-        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        float row[2 * NB], col[16];
         ptc_tmem_ld32(tmem_row, va);
-#pragma unroll 1
+        if (more) put_a(rn);  // the product has read the rows before
+#pragma unroll
+        for (int q = 0; q < 16; ++q) col[q] = -INFINITY;
+#pragma unroll
         for (int gq = 0; gq < NB; gq += 2) {
           ptc_tmem_wait(va);
           if (NB > 1) ptc_tmem_ld32(tmem_row + (gq + 1) * 32, vb);
-          ptc_max_block(va, mx);
+          else if (more) hand_over();
+          ptc_fold(va, row + 2 * gq, col);
           if (NB > 1) {
             ptc_tmem_wait(vb);
             if (gq + 2 < NB) ptc_tmem_ld32(tmem_row + (gq + 2) * 32, va);
-            ptc_max_block(vb, mx);
+            else if (more) hand_over();
+            ptc_fold(vb, row + 2 * gq + 2, col);
           }
         }
-        const float thr = __fsub_rn(fmaxf(ptc_max3(mx[0], mx[1], mx[2]), mx[3]), margin);
-        // ---- candidates: bit 31 - i of word gq is centroid 32 gq + i ----
-        int n_cand = 0, arg = 0;
-        ptc_tmem_ld32(tmem_row, va);
-#pragma unroll 1
-        for (int gq = 0; gq < NB; gq += 2) {
-          ptc_tmem_wait(va);
-          if (NB > 1) ptc_tmem_ld32(tmem_row + (gq + 1) * 32, vb);
-          uint32_t w = ptc_candidates(va, thr);
-          cand_sm[gq * PTC_THREADS + tid] = w;
-          n_cand += __popc(w);
-          if (w) arg = gq * 32 + __clz(w);
-          if (NB > 1) {
-            ptc_tmem_wait(vb);
-            if (gq + 2 < NB) ptc_tmem_ld32(tmem_row + (gq + 2) * 32, va);
-            w = ptc_candidates(vb, thr);
-            cand_sm[(gq + 1) * PTC_THREADS + tid] = w;
-            n_cand += __popc(w);
-            if (w) arg = gq * 32 + 32 + __clz(w);
-          }
-        }
-        if (n_cand != 1) {
+        float top = fmaxf(col[0], col[1]);
+#pragma unroll
+        for (int q = 2; q < 16; q += 2) top = ptc_max3(top, col[q], col[q + 1]);
+        const float thr = __fsub_rn(top, margin);
+        uint32_t rows = ptc_near<2 * NB>(row, thr);
+        const uint32_t cols = ptc_near<16>(col, thr);
+        int arg;
+        if (__popc(rows) == 1 && __popc(cols) == 1) {
+          arg = (__ffs(rows) - 1) * 16 + __ffs(cols) - 1;
+        } else {
           float best = INFINITY;
           arg = 0;
+          uint4 r = rw;  // unpacked anew: the channels are not to stay in registers through the fold
+          asm volatile("" : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w));
+          float xv[SD];
+          sah_unpack8(r, xv);
 #pragma unroll 1
-          for (int gq = 0; gq < NB; ++gq) {
-            uint32_t w = cand_sm[gq * PTC_THREADS + tid];
+          for (; rows; rows &= rows - 1) {  // ascending c: the first minimum wins
+            const int c0 = (__ffs(rows) - 1) * 16;
 #pragma unroll 1
-            while (w) {  // ascending c: the first minimum wins
-              const int i = __clz(w);
-              w &= ~(0x80000000u >> i);
-              const int c = gq * 32 + i;
+            for (uint32_t w = cols; w; w &= w - 1) {
+              const int c = c0 + __ffs(w) - 1;
               if (c < n_cent) {
                 const float dist = pq_dist(xv, cent_sm + (s * 256 + c) * SD, SD);
                 if (dist < best) { best = dist; arg = c; }
@@ -294,14 +329,14 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
           }
         }
         packed |= (uint32_t)arg << (8 * s);
+        rw = rn;
+        rn = rnn;
       }
-      if (j < key_end) {
-        uint8_t* dst = codes + (bk * cap + (j - init_offset)) * n_sub + sub0;
+      if (t < have) {
         if (NS == 4) *reinterpret_cast<uint32_t*>(dst) = packed;
         else *dst = (uint8_t)packed;
       }
-#pragma unroll
-      for (int s = 0; s < NS; ++s) raw[s] = next[s];
+      dst += (int64_t)(2 * PTC_TILE) * n_sub;
     }
     it = seg_end;
   }

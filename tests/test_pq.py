@@ -462,3 +462,38 @@ def test_gpu_assignment_of_keys_far_from_one(n_cent, scale):
                   "sah_pq_assign_tc")
     assert int(err.item()) == 0 and torch.equal(got, want)
     assert len(torch.unique(want)) > 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_cent", [16, 32, 64, 112, 256])
+def test_gpu_assignment_of_ties_and_non_finite_keys(n_cent):
+    """`sah_pq_assign_tc` where a key's row of the product holds several equal maxima (centroids given
+    twice, keys of zero) and where margins are infinite or NaN: the codes of `sah_pq_assign`."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, n_sub, n_keys = 1, 2, 8, 515
+    gen = torch.Generator(device=dev).manual_seed(n_cent)
+    keys = torch.randn((B, Hkv, n_keys, n_sub * 8), generator=gen, device=dev).to(torch.bfloat16)
+    keys[:, :, 3] = 0.0
+    keys[:, :, 130, 5] = float("nan")
+    keys[:, :, 257, 9] = float("inf")
+    keys[:, :, 514, 17] = -float("inf")
+    cent = torch.randn((B * Hkv * n_sub, n_cent, 8), generator=gen, device=dev)
+    cent[:, n_cent // 2:] = cent[:, :n_cent // 2].flip(1)
+    cent[1, n_cent // 3, 2] = float("inf")
+    cent[2, n_cent - 1, 2] = float("nan")
+    cent[3] = 0.0
+    st = _native.stream_of(torch.device(dev))
+    want = torch.full((B, Hkv, n_keys, n_sub), 255, dtype=torch.uint8, device=dev)
+    got = want.clone()
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    strides = (keys.stride(0), keys.stride(1), keys.stride(2))
+    _native.check(lib.sah_pq_assign(keys.data_ptr(), _native.SAH_BF16, *strides, B, Hkv, 0, n_keys, 0, n_sub, 8, n_cent,
+                                    cent.data_ptr(), want.data_ptr(), n_keys, 0, st), "sah_pq_assign")
+    _native.check(lib.sah_pq_assign_tc(keys.data_ptr(), *strides, B, Hkv, 0, n_keys, 0, n_sub, 8, n_cent,
+                                       cent.data_ptr(), got.data_ptr(), n_keys, err.data_ptr(), 148, st),
+                  "sah_pq_assign_tc")
+    assert int(err.item()) == 0 and torch.equal(got, want)
