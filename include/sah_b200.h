@@ -564,6 +564,18 @@ int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t 
                   const double* sums, const int* counts, const int64_t* reseed, float* centroids,
                   float* shift2, void* stream);
 
+/* All Lloyd iterations of kmeans_batched (pq_utils.py:220-423) over the keys [init_offset, init_offset + n_keys):
+ * assignment (sah_pq_assign_tc with use_tc != 0, for the shapes it takes; sah_pq_assign without), sums, new
+ * centres.  The comparison with the tolerance happens on the device; the kernels of the iterations that are
+ * left after it return at once.  reseed: n_iter device pointers (host array).  sums and counts are scratch of
+ * sah_pq_accumulate's sizes.  state: five words on the device; state[1] is the number of iterations that ran,
+ * state[2] is set when a bounded wait of the tensor-core kernel ran out (codes and centroids are then void).
+ * All operands stay untouched until the stream has passed the last launch. */
+int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                  int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int n_iter,
+                  const int64_t* const* reseed, float* centroids, uint8_t* codes, int64_t cap,
+                  double* sums, int* counts, int* state, int use_tc, int sm_count, void* stream);
+
 /* scores[row][init_offset + j] = sum over sub-vectors of lut[sub][code(j, sub)],
  * lut[sub][c] = q_sub . centroid (rounded to `dtype`), the sum taken in fp32 in
  * ascending sub-vector order and rounded once (_compute_pq_scores,

@@ -46,8 +46,9 @@ __global__ void __launch_bounds__(PQ_TILE)
 pq_assign_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
                  int64_t key_begin, int64_t key_end, int64_t init_offset, int n_sub, int sub_d,
                  int n_cent, const float* __restrict__ centroids, uint8_t* __restrict__ codes,
-                 int64_t cap) {
+                 int64_t cap, const int* __restrict__ done) {
   extern __shared__ float pq_cent_sm[];  // [n_cent][sub_d]
+  if (done && *done) return;
   const int sub = blockIdx.y;
   const int64_t bk = blockIdx.z;
   const int kvh = (int)(bk % Hkv);
@@ -80,10 +81,10 @@ __global__ void __launch_bounds__(256)
 pq_assign_few_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
                      int64_t key_begin, int n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent,
                      int64_t items, const float* __restrict__ centroids, uint8_t* __restrict__ codes,
-                     int64_t cap) {
+                     int64_t cap, const int* __restrict__ done) {
   const int lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // (group, key)
-  if (item >= items) return;
+  if (item >= items || (done && *done)) return;
   const int64_t grp = item / n_keys, j = key_begin + item % n_keys;
   const int sub = (int)(grp % n_sub);
   const int64_t bk = grp / n_sub;
@@ -123,11 +124,12 @@ pq_assign_few_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
   if (lane == 0) codes[(bk * cap + (j - init_offset)) * n_sub + sub] = (uint8_t)(arg < 256 ? arg : 0);
 }
 
-extern "C" int sah_pq_assign(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
-                             int B, int Hkv, int64_t key_begin, int64_t key_end,
-                             int64_t init_offset, int n_sub, int sub_d, int n_cent,
-                             const float* centroids, uint8_t* codes, int64_t cap, int dtype_math,
-                             void* stream) {
+// `done`, where the calls of this file take it: a word on the device that is not 0 once the clustering
+// has converged; the kernels of the iterations behind it return at once.
+static int pq_assign_run(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
+                         int B, int Hkv, int64_t key_begin, int64_t key_end, int64_t init_offset, int n_sub,
+                         int sub_d, int n_cent, const float* centroids, uint8_t* codes, int64_t cap, int dtype_math,
+                         const int* done, void* stream) {
   SAH_REQUIRE(x && centroids && codes, "pq_assign: null pointer");
   SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_cent > 0, "pq_assign: bad extents");
   SAH_REQUIRE(init_offset <= key_begin && key_begin <= key_end && key_end - init_offset <= cap,
@@ -144,11 +146,11 @@ extern "C" int sah_pq_assign(const void* x, int dtype, int64_t xs_b, int64_t xs_
       if (dtype_math)
         pq_assign_few_kernel<T, true><<<few, 256, 0, (cudaStream_t)stream>>>(
             (const T*)x, xs_b, xs_h, xs_s, Hkv, key_begin, n_keys, init_offset, n_sub, sub_d, n_cent, items,
-            centroids, codes, cap);
+            centroids, codes, cap, done);
       else
         pq_assign_few_kernel<T, false><<<few, 256, 0, (cudaStream_t)stream>>>(
             (const T*)x, xs_b, xs_h, xs_s, Hkv, key_begin, n_keys, init_offset, n_sub, sub_d, n_cent, items,
-            centroids, codes, cap);
+            centroids, codes, cap, done);
     });
     SAH_LAUNCH_CHECK("pq_assign_few");
     return SAH_OK;
@@ -160,23 +162,32 @@ extern "C" int sah_pq_assign(const void* x, int dtype, int64_t xs_b, int64_t xs_
     if (dtype_math)
       pq_assign_kernel<T, true><<<grid, PQ_TILE, smem, (cudaStream_t)stream>>>(
           (const T*)x, xs_b, xs_h, xs_s, Hkv, key_begin, key_end, init_offset, n_sub, sub_d, n_cent,
-          centroids, codes, cap);
+          centroids, codes, cap, done);
     else
       pq_assign_kernel<T, false><<<grid, PQ_TILE, smem, (cudaStream_t)stream>>>(
           (const T*)x, xs_b, xs_h, xs_s, Hkv, key_begin, key_end, init_offset, n_sub, sub_d, n_cent,
-          centroids, codes, cap);
+          centroids, codes, cap, done);
   });
   SAH_LAUNCH_CHECK("pq_assign");
   return SAH_OK;
 }
 
+extern "C" int sah_pq_assign(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
+                             int B, int Hkv, int64_t key_begin, int64_t key_end,
+                             int64_t init_offset, int n_sub, int sub_d, int n_cent,
+                             const float* centroids, uint8_t* codes, int64_t cap, int dtype_math,
+                             void* stream) {
+  return pq_assign_run(x, dtype, xs_b, xs_h, xs_s, B, Hkv, key_begin, key_end, init_offset, n_sub, sub_d, n_cent,
+                       centroids, codes, cap, dtype_math, nullptr, stream);
+}
+
 #include "sah_pq_tc.cuh"
 
 // The assignment step on the tensor cores; same codes as sah_pq_assign(dtype_math = 0).
-extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
-                                int64_t key_begin, int64_t key_end, int64_t init_offset, int n_sub,
-                                int sub_d, int n_cent, const float* centroids, uint8_t* codes, int64_t cap,
-                                int* errflag, int sm_count, void* stream) {
+static int pq_assign_tc_run(const void* x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                            int64_t key_begin, int64_t key_end, int64_t init_offset, int n_sub, int sub_d,
+                            int n_cent, const float* centroids, uint8_t* codes, int64_t cap, int* errflag,
+                            int sm_count, const int* done, void* stream) {
   SAH_REQUIRE(x && centroids && codes && errflag, "pq_assign_tc: null pointer");
   SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0, "pq_assign_tc: bad extents");
   SAH_REQUIRE(init_offset <= key_begin && key_begin <= key_end && key_end - init_offset <= cap,
@@ -206,7 +217,7 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
     if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_assign_tc attr: %s", cudaGetErrorString(e));         \
     pq_assign_tc_kernel<NS, NB><<<grid, PTC_THREADS, PtcCfg<NS>::SMEM, st>>>(                                    \
         reinterpret_cast<const __nv_bfloat16*>(x), xs_b, xs_h, xs_s, Hkv, key_begin, key_end, init_offset,       \
-        n_sub, n_cent, n_blocks, centroids, codes, cap, errflag);                                                \
+        n_sub, n_cent, n_blocks, centroids, codes, cap, errflag, done);                                                \
   } while (0)
 #define PTC_LAUNCH_NS(NS)                   \
   do {                                      \
@@ -221,6 +232,14 @@ extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64
 #undef PTC_LAUNCH
   SAH_LAUNCH_CHECK("pq_assign_tc");
   return SAH_OK;
+}
+
+extern "C" int sah_pq_assign_tc(const void* x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                                int64_t key_begin, int64_t key_end, int64_t init_offset, int n_sub,
+                                int sub_d, int n_cent, const float* centroids, uint8_t* codes, int64_t cap,
+                                int* errflag, int sm_count, void* stream) {
+  return pq_assign_tc_run(x, xs_b, xs_h, xs_s, B, Hkv, key_begin, key_end, init_offset, n_sub, sub_d, n_cent,
+                          centroids, codes, cap, errflag, sm_count, nullptr, stream);
 }
 
 // Cluster sums in fp64 (so that the summation order does not reach the fp32 result) and counts.
@@ -244,7 +263,8 @@ __global__ void __launch_bounds__(PQA_THREADS, 2)
 pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
                      int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int cblocks, int shares, int vec8,
                      const uint8_t* __restrict__ codes, int64_t cap, double* __restrict__ sums,
-                     int* __restrict__ counts) {
+                     int* __restrict__ counts, const int* __restrict__ done) {
+  if (done && *done) return;
   __shared__ int pos_sm[256];              // histogram, then the next free slot of every centroid
   __shared__ int start_sm[257];
   __shared__ int scan_sm[33];
@@ -351,10 +371,10 @@ pq_accumulate_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_
   }
 }
 
-extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
-                                 int B, int Hkv, int64_t n_keys, int64_t init_offset, int n_sub,
-                                 int sub_d, int n_cent, const uint8_t* codes, int64_t cap,
-                                 double* sums, int* counts, void* stream) {
+static int pq_accumulate_run(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                             int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent,
+                             const uint8_t* codes, int64_t cap, double* sums, int* counts, const int* done,
+                             void* stream) {
   SAH_REQUIRE(x && codes && sums && counts, "pq_accumulate: null pointer");
   SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_cent > 0 && n_keys >= 0,
               "pq_accumulate: bad extents");
@@ -375,22 +395,36 @@ extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t
   SAH_DISPATCH_DTYPE(dtype, T, {
     pq_accumulate_kernel<T><<<grid, PQA_THREADS, 0, (cudaStream_t)stream>>>(
         (const T*)x, xs_b, xs_h, xs_s, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, cblocks, shares, vec8, codes, cap,
-        sums, counts);
+        sums, counts, done);
   });
   SAH_LAUNCH_CHECK("pq_accumulate");
   return SAH_OK;
 }
 
+extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
+                                 int B, int Hkv, int64_t n_keys, int64_t init_offset, int n_sub,
+                                 int sub_d, int n_cent, const uint8_t* codes, int64_t cap,
+                                 double* sums, int* counts, void* stream) {
+  return pq_accumulate_run(x, dtype, xs_b, xs_h, xs_s, B, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, codes, cap,
+                           sums, counts, nullptr, stream);
+}
+
 // new centre = fp32(sum) / fp32(count); an empty cluster takes the key sub-vector at
 // reseed[group][cluster] (pq_utils.py:384-396); shift2[group] = (sum over clusters of
 // the centre's Euclidean move)^2, the quantity compared with the tolerance (:399-423).
+// With `state` (the words that sah_pq_kmeans keeps) the sums and counts are cleared for the next
+// iteration and the last block makes the comparison.
+struct PqState {
+  int done, iterations, err, open, ticket;
+};
 template <typename T>
 __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s,
                                  int Hkv, int64_t init_offset, int n_sub, int sub_d, int n_cent,
-                                 const double* __restrict__ sums, const int* __restrict__ counts,
+                                 double* __restrict__ sums, int* __restrict__ counts,
                                  const int64_t* __restrict__ reseed, float* __restrict__ centroids,
-                                 float* __restrict__ shift2) {
+                                 float* __restrict__ shift2, PqState* __restrict__ state) {
   __shared__ float scratch[33];
+  if (state && state->done) return;
   const int64_t grp = blockIdx.x;
   const int sub = (int)(grp % n_sub);
   const int64_t bk = grp / n_sub;
@@ -407,7 +441,7 @@ __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t 
     if (cnt <= 0) xr = x + b * xs_b + kvh * xs_h + (reseed[grp * n_cent + c] + init_offset) * xs_s + sub * sub_d;
     float d2 = 0.f;
     for (int c_lo = 0; c_lo < sub_d; c_lo += PQ_MAX_SUBD) {
-      const double* sp = sums + (grp * n_cent + c) * sub_d + c_lo;
+      double* sp = sums + (grp * n_cent + c) * sub_d + c_lo;
       float* cp = centroids + (grp * n_cent + c) * sub_d + c_lo;
       const int nch = sub_d - c_lo;
       double sv[PQ_MAX_SUBD];
@@ -424,13 +458,24 @@ __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t 
           const float t = __fsub_rn(nv, old[d]);
           d2 = __fadd_rn(d2, __fmul_rn(t, t));
           cp[d] = nv;
+          if (state) sp[d] = 0.0;
         }
     }
     move = sqrtf(d2);
+    if (state) counts[grp * n_cent + c] = 0;
   }
   float total;
   sah_block_excl_scan<float>(move, scratch, &total);
-  if (threadIdx.x == 0) shift2[grp] = total * total;
+  if (threadIdx.x != 0) return;
+  if (shift2) shift2[grp] = total * total;
+  if (!state) return;
+  if (!(total * total < 1e-4f)) atomicAdd(&state->open, 1);
+  __threadfence();
+  if (atomicAdd(&state->ticket, 1) == (int)gridDim.x - 1) {  // every block has read `done` by now
+    state->iterations += 1;
+    if (atomicExch(&state->open, 0) == 0) state->done = 1;
+    state->ticket = 0;
+  }
 }
 
 extern "C" int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s,
@@ -442,10 +487,44 @@ extern "C" int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_
   const int64_t groups = (int64_t)B * Hkv * n_sub;
   SAH_DISPATCH_DTYPE(dtype, T, {
     pq_update_kernel<T><<<(unsigned)groups, 256, 0, (cudaStream_t)stream>>>(
-        (const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub, sub_d, n_cent, sums, counts, reseed,
-        centroids, shift2);
+        (const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub, sub_d, n_cent, const_cast<double*>(sums),
+        const_cast<int*>(counts), reseed, centroids, shift2, nullptr);
   });
   SAH_LAUNCH_CHECK("pq_update");
+  return SAH_OK;
+}
+
+extern "C" int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                             int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int n_iter,
+                             const int64_t* const* reseed, float* centroids, uint8_t* codes, int64_t cap,
+                             double* sums, int* counts, int* state, int use_tc, int sm_count, void* stream) {
+  SAH_REQUIRE(x && reseed && centroids && codes && sums && counts && state, "pq_kmeans: null pointer");
+  SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_keys >= 0 && n_iter >= 0, "pq_kmeans: bad extents");
+  SAH_REQUIRE(n_cent > 0 && n_cent <= 256, "pq_kmeans: 1..256 centroids");
+  for (int it = 0; it < n_iter; ++it) SAH_REQUIRE(reseed[it], "pq_kmeans: null pointer");
+  const int64_t groups = (int64_t)B * Hkv * n_sub;
+  const cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t e = cudaMemsetAsync(sums, 0, (size_t)(groups * n_cent * sub_d) * sizeof(double), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, (size_t)(groups * n_cent) * sizeof(int), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(state, 0, sizeof(PqState), st);
+  if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_kmeans: %s", cudaGetErrorString(e));
+  PqState* ps = reinterpret_cast<PqState*>(state);
+  for (int it = 0; it < n_iter; ++it) {
+    int rc = use_tc ? pq_assign_tc_run(x, xs_b, xs_h, xs_s, B, Hkv, init_offset, init_offset + n_keys, init_offset,
+                                       n_sub, sub_d, n_cent, centroids, codes, cap, &ps->err, sm_count, &ps->done, stream)
+                    : pq_assign_run(x, dtype, xs_b, xs_h, xs_s, B, Hkv, init_offset, init_offset + n_keys, init_offset,
+                                    n_sub, sub_d, n_cent, centroids, codes, cap, 0, &ps->done, stream);
+    if (rc == SAH_OK)
+      rc = pq_accumulate_run(x, dtype, xs_b, xs_h, xs_s, B, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, codes, cap,
+                             sums, counts, &ps->done, stream);
+    if (rc != SAH_OK) return rc;
+    SAH_DISPATCH_DTYPE(dtype, T, {
+      pq_update_kernel<T><<<(unsigned)groups, 256, 0, st>>>((const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub,
+                                                            sub_d, n_cent, sums, counts, reseed[it], centroids, nullptr,
+                                                            ps);
+    });
+    SAH_LAUNCH_CHECK("pq_update");
+  }
   return SAH_OK;
 }
 

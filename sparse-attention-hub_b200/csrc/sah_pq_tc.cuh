@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(PTC_THREADS, 1)
 pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t xs_h, int64_t xs_s, int Hkv,
                     int64_t key_begin, int64_t key_end, int64_t init_offset, int n_sub, int n_cent,
                     int64_t n_blocks, const float* __restrict__ centroids, uint8_t* __restrict__ codes,
-                    int64_t cap, int* __restrict__ errflag) {
+                    int64_t cap, int* __restrict__ errflag, const int* __restrict__ done) {
+  if (done && *done) return;  // nothing allocated yet
   constexpr int SD = 8, NC = 32 * NB;
   using C = PtcCfg<NS>;
   extern __shared__ __align__(1024) unsigned char ptc_raw[];

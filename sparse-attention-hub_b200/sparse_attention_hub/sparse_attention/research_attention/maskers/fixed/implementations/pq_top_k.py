@@ -23,6 +23,7 @@ first `2**bits` entries of a random permutation per group unless
 """
 
 from dataclasses import dataclass
+import ctypes
 import os
 from typing import Any, Dict, Optional, Tuple, Union
 
@@ -235,17 +236,21 @@ class PQCache(TopKMasker):
         cap = codes.shape[2]
         sums = torch.empty((groups, n_cent, sub_d), dtype=torch.float64, device=dev)
         counts = torch.empty((groups, n_cent), dtype=torch.int32, device=dev)
-        shift2 = torch.empty(groups, dtype=torch.float32, device=dev)
         reseed_src = sparse_meta_data.get("pq_reseed_indices", {}).get(layer_idx)
-        own_pos = torch.arange(n_cent, device=dev, dtype=torch.long).repeat(groups, 1).contiguous()
         # the distance contraction of the assignment runs on the tensor cores when the shapes
         # allow (bfloat16 keys, 8 channels per sub-vector, 16..256 centroids in multiples of 16)
         use_tc = (os.environ.get("SAH_PQ_TC", "1") != "0" and k.dtype == torch.bfloat16 and sub_d == 8
                   and 16 <= n_cent <= 256 and n_cent % 16 == 0 and k.data_ptr() % 16 == 0
                   and all((k.stride(i) * 2) % 16 == 0 for i in range(3)))
-        tc_err = torch.zeros(1, dtype=torch.int32, device=dev)
         self.last_build_used_tensor_cores = use_tc
-        for it in range(self.kmeans_iter):
+        if shard is None:
+            self._lloyd(k, kargs, local_off, (B, Hkv, n_sub, sub_d, n_cent), reseed_src, centroids, codes, sums, counts,
+                        use_tc, lambda: self._gather_subvectors(k, init, local_off, None).reshape(centroids.shape))
+        else:
+            shift2 = torch.empty(groups, dtype=torch.float32, device=dev)
+            own_pos = torch.arange(n_cent, device=dev, dtype=torch.long).repeat(groups, 1).contiguous()
+            tc_err = torch.zeros(1, dtype=torch.int32, device=dev)
+        for it in range(self.kmeans_iter if shard is not None else 0):  # the ranks meet in every iteration
             if n_local > 0:
                 if use_tc:
                     _native.check(lib.sah_pq_assign_tc(k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), B, Hkv,
@@ -270,26 +275,18 @@ class PQCache(TopKMasker):
                 reseed = reseed_src[it].to(device=dev, dtype=torch.long).contiguous()
             else:
                 reseed = torch.randint(0, n_keys, (groups, n_cent), device=dev)
-                if shard is not None:
-                    reseed = shard.comm.all_reduce_sum_(reseed if shard.comm.rank == 0
-                                                        else torch.zeros_like(reseed))
-            if shard is None:
-                _native.check(lib.sah_pq_update(*kargs, B, Hkv, local_off, n_sub, sub_d, n_cent,
-                                                sums.data_ptr(), counts.data_ptr(), reseed.data_ptr(),
-                                                centroids.data_ptr(), shift2.data_ptr(), st),
-                              "sah_pq_update")
-            else:
-                # sums of bfloat16 / float32 key values in float64 and counts add up exactly over
-                # the ranks; the keys that re-seed empty clusters may live anywhere, so they are
-                # gathered into a [B, Hkv, n_cent, D] table that the update kernel reads instead
-                shard.comm.all_reduce_sum_(sums)
-                shard.comm.all_reduce_sum_(counts)
-                picked = self._gather_subvectors(k, reseed.reshape(B, Hkv, n_sub, n_cent), local_off, shard)
-                table = picked.permute(0, 1, 3, 2, 4).reshape(B, Hkv, n_cent, n_sub * sub_d).to(k.dtype).contiguous()
-                _native.check(lib.sah_pq_update(table.data_ptr(), _native.dtype_code(table.dtype), table.stride(0),
-                                                table.stride(1), table.stride(2), B, Hkv, 0, n_sub, sub_d,
-                                                n_cent, sums.data_ptr(), counts.data_ptr(), own_pos.data_ptr(),
-                                                centroids.data_ptr(), shift2.data_ptr(), st), "sah_pq_update")
+                reseed = shard.comm.all_reduce_sum_(reseed if shard.comm.rank == 0 else torch.zeros_like(reseed))
+            # sums of bfloat16 / float32 key values in float64 and counts add up exactly over
+            # the ranks; the keys that re-seed empty clusters may live anywhere, so they are
+            # gathered into a [B, Hkv, n_cent, D] table that the update kernel reads instead
+            shard.comm.all_reduce_sum_(sums)
+            shard.comm.all_reduce_sum_(counts)
+            picked = self._gather_subvectors(k, reseed.reshape(B, Hkv, n_sub, n_cent), local_off, shard)
+            table = picked.permute(0, 1, 3, 2, 4).reshape(B, Hkv, n_cent, n_sub * sub_d).to(k.dtype).contiguous()
+            _native.check(lib.sah_pq_update(table.data_ptr(), _native.dtype_code(table.dtype), table.stride(0),
+                                            table.stride(1), table.stride(2), B, Hkv, 0, n_sub, sub_d,
+                                            n_cent, sums.data_ptr(), counts.data_ptr(), own_pos.data_ptr(),
+                                            centroids.data_ptr(), shift2.data_ptr(), st), "sah_pq_update")
             if bool((shift2 < 1e-4).all().item()):  # the reference's convergence test (host sync)
                 break
         cent_t = centroids.to(keys.dtype).reshape(B, Hkv, n_sub, n_cent, sub_d).contiguous()
@@ -297,6 +294,48 @@ class PQCache(TopKMasker):
         sparse_meta_data["pq_centroids"][layer_idx] = cent_t
         sparse_meta_data["pq_codebook"][layer_idx] = packed
         return cent_t, packed
+
+    def _lloyd(self, k: torch.Tensor, kargs, local_off: int, geometry, reseed_src, centroids: torch.Tensor,
+               codes: torch.Tensor, sums: torch.Tensor, counts: torch.Tensor, use_tc: bool, first_centroids) -> None:
+        """The Lloyd iterations over one device's keys, launched together: the test for convergence is made
+        on the device, and the host waits once, at the end (with a wait for every iteration's test,
+        8 KV heads x 65472 keys and ten iterations took 0.9 ms longer)."""
+        if self.kmeans_iter <= 0:
+            return
+        lib = _native.load()
+        B, Hkv, n_sub, sub_d, n_cent = geometry
+        dev = k.device
+        n_keys = k.shape[2] - local_off
+        drawn_before = []  # the generator's state in front of every draw
+        reseed = []
+        for it in range(self.kmeans_iter):
+            if reseed_src is not None:
+                try:
+                    given = reseed_src[it]
+                except (IndexError, KeyError):  # as few as the clustering may need
+                    break
+                reseed.append(given.to(device=dev, dtype=torch.long).contiguous())
+            else:
+                drawn_before.append(torch.cuda.get_rng_state(dev))
+                reseed.append(torch.randint(0, n_keys, (B * Hkv * n_sub, n_cent), device=dev))
+        state = torch.empty(5, dtype=torch.int32, device=dev)
+        pointers = (ctypes.c_void_p * len(reseed))(*[r.data_ptr() for r in reseed])
+
+        def launch(tensor_cores: bool) -> list:
+            _native.check(lib.sah_pq_kmeans(*kargs, B, Hkv, n_keys, local_off, n_sub, sub_d, n_cent, len(reseed), pointers,
+                                            centroids.data_ptr(), codes.data_ptr(), codes.shape[2], sums.data_ptr(),
+                                            counts.data_ptr(), state.data_ptr(), int(tensor_cores),
+                                            _native.sm_count(dev), _native.stream_of(dev)), "sah_pq_kmeans")
+            return state.tolist()
+
+        done, ran, failed = launch(use_tc)[:3]
+        if failed:  # a bounded wait inside the tensor-core kernel ran out: fixed-order kernel, from the start
+            centroids.copy_(first_centroids())
+            done, ran, _ = launch(False)[:3]
+        if not done and len(reseed) < self.kmeans_iter:
+            reseed_src[len(reseed)]  # one more was needed: the error that the lookup raises
+        if ran < len(drawn_before):  # converged early: the draws behind it were not made
+            torch.cuda.set_rng_state(drawn_before[ran], dev)
 
     def _handle_incremental_keys(self, keys: torch.Tensor, layer_idx: int,
                                  sparse_meta_data: Dict[str, Any], local_off: Optional[int] = None):

@@ -497,3 +497,64 @@ def test_gpu_assignment_of_ties_and_non_finite_keys(n_cent):
                                        cent.data_ptr(), got.data_ptr(), n_keys, err.data_ptr(), 148, st),
                   "sah_pq_assign_tc")
     assert int(err.item()) == 0 and torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,n_keys,given,iters", [("bf16", 700, True, 6), ("bf16", 40, False, 8), ("f32", 300, False, 3),
+                                                      ("bf16", 40, True, 8)])
+def test_gpu_lloyd_iterations_launched_together(dtype, n_keys, given, iters):
+    """The clustering of a build equals its steps called one after the other with the host's test for
+    convergence between them (40 keys for 16 centres converge after a few iterations), and the
+    generator has made as many draws."""
+    import torch
+    from sparse_attention_hub import _native
+    from sparse_attention_hub.sparse_attention.research_attention.maskers.fixed import PQCache, PQCacheConfig
+
+    lib = _native.load()
+    dev = torch.device("cuda:0")
+    B, Hkv, n_sub, n_cent, off = 1, 2, 4, 16, 8
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    gen = torch.Generator(device=dev).manual_seed(n_keys)
+    keys = torch.randn((B, Hkv, n_keys + off, n_sub * 8), generator=gen, device=dev).to(dt)
+    groups, st = B * Hkv * n_sub, _native.stream_of(dev)
+    init = torch.rand((groups, n_keys), generator=gen, device=dev).topk(n_cent, dim=1).indices
+    draws = [torch.randint(0, n_keys, (groups, n_cent), generator=gen, device=dev) for _ in range(iters)]
+
+    torch.manual_seed(5)
+    rows = keys[:, :, off:].reshape(B * Hkv, n_keys, n_sub, 8).transpose(1, 2).reshape(groups, n_keys, 8).float()
+    cent = torch.gather(rows, 1, init[..., None].expand(-1, -1, 8)).contiguous()
+    codes = torch.zeros((B, Hkv, n_keys, n_sub), dtype=torch.uint8, device=dev)
+    args = (keys.data_ptr(), _native.dtype_code(dt), keys.stride(0), keys.stride(1), keys.stride(2), B, Hkv)
+    shift2 = torch.empty(groups, device=dev)
+    ran = 0
+    for it in range(iters):
+        _native.check(lib.sah_pq_assign(*args, off, off + n_keys, off, n_sub, 8, n_cent, cent.data_ptr(),
+                                        codes.data_ptr(), n_keys, 0, st), "sah_pq_assign")
+        sums = torch.zeros((groups, n_cent, 8), dtype=torch.float64, device=dev)
+        counts = torch.zeros((groups, n_cent), dtype=torch.int32, device=dev)
+        _native.check(lib.sah_pq_accumulate(*args, n_keys, off, n_sub, 8, n_cent, codes.data_ptr(), n_keys,
+                                            sums.data_ptr(), counts.data_ptr(), st), "sah_pq_accumulate")
+        reseed = draws[it] if given else torch.randint(0, n_keys, (groups, n_cent), device=dev)
+        _native.check(lib.sah_pq_update(*args, off, n_sub, 8, n_cent, sums.data_ptr(), counts.data_ptr(),
+                                        reseed.data_ptr(), cent.data_ptr(), shift2.data_ptr(), st), "sah_pq_update")
+        ran += 1
+        if bool((shift2 < 1e-4).all()):
+            break
+    generator = torch.cuda.get_rng_state(dev)
+    assert (ran < iters) == (n_keys == 40)
+
+    torch.manual_seed(5)
+    masker = PQCache(PQCacheConfig(heavy_size=8, pq_group_factor=n_sub, pq_bits=4, kmeans_iter=iters, init_offset=off,
+                                   metric="euclidean"))
+    meta = {"pq_init_indices": {0: init}}
+    if given:
+        meta["pq_reseed_indices"] = {0: draws[:ran]}  # no more than are needed
+    masker._initialize_pq_cache(meta, 0)
+    got_cent, got_codes = masker._perform_kmeans_clustering(keys, 0, meta)
+    assert torch.equal(got_codes.codes[:, :, :n_keys], codes)
+    assert torch.equal(got_cent.reshape(groups, n_cent, 8), cent.to(dt))
+    assert torch.equal(torch.cuda.get_rng_state(dev), generator)
+    if given:
+        meta["pq_reseed_indices"] = {0: draws[:ran - 1]}
+        with pytest.raises(IndexError):
+            masker._perform_kmeans_clustering(keys, 0, meta)
