@@ -671,6 +671,22 @@ int sah_masked_attention(const void* q, const void* k, const void* v, int dtype,
                          const uint16_t* umemb, const float* uw, const int32_t* ucount,
                          float* partial, void* out, float* part_out, void* stream);
 
+/* MagicPig attention of several query rows per KV head without a plan: all K and V rows are read once per
+ * block of 64 rows, and a (row, key) pair counts where match_bits or unit_bits ([rows][W]) has it, with the
+ * weights of sah_masked_attention_lsh.  bfloat16, head dim 128, rows 16-byte aligned.  n_parts: what
+ * sah_attn_stream_parts gave for these extents (lsh_k, lsh_l: bits per table and tables); it gives 0 where the
+ * gather kernels are the faster ones or a kernel has been chosen by sah_attn_select_kernel.  parts:
+ * scratch, float32 [n_parts][rows][D + 2].  *errflag is set when a bounded wait ran out. */
+int sah_attn_stream_parts(int B, int Hq, int Hkv, int Sq, int64_t S, int D, int lsh_k, int lsh_l, int sm_count);
+int sah_masked_attention_stream(const void* q, const void* k, const void* v, int64_t qs_b, int64_t qs_h, int64_t qs_q,
+                                int64_t ks_b, int64_t ks_h, int64_t ks_s, int64_t vs_b, int64_t vs_h, int64_t vs_s,
+                                int B, int Hq, int Hkv, int Sq, int64_t S, int D, float scaling, const void* bias,
+                                int64_t bias_s_b, int64_t bias_s_h, int64_t bias_s_q, const float* sinks,
+                                const uint32_t* match_bits, const uint32_t* unit_bits, int64_t W, const float* dens,
+                                int64_t dens_cap, const unsigned int* max_norm_bits, const void* qhat, const float* qmu,
+                                const uint16_t* weight_table, float* parts, int n_parts, void* out, int* errflag,
+                                void* stream);
+
 /* sah_masked_attention (bfloat16) over a union list made by sah_attn_plan_lsh, with the
  * MagicPig sampling weights computed where the key row already is: the weight of a
  * sampled key is 1 / (p + 1e-6) (Mask.apply_inv_mask_dense, utils/mask.py:718-740) with

@@ -7,6 +7,7 @@
 //                          fetched once per group and shared by its query heads
 //   sah_attn_merge_parts   associative merge of sequence-sharded partials
 #include <algorithm>
+#include <math.h>
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
@@ -607,6 +608,7 @@ static const char* g_last_attn_kernel = "none";
 
 #include "sah_attention_tc.cuh"
 #include "sah_attention_umma.cuh"
+#include "sah_attention_stream.cuh"
 
 // BANDS: the list is a.iv
 template <typename T, int D, int NQUAD, bool BANDS>
@@ -1248,6 +1250,70 @@ extern "C" int sah_attn_merge_parts(const float* parts, int n_parts, int B, int 
         n_parts, rows, Hq, Sq, D, sinks, (T*)out);
   });
   SAH_LAUNCH_CHECK("attn_merge_parts");
+  return SAH_OK;
+}
+
+// CTAs per KV head of the streaming kernel, 0 where the list of selected keys is the way to go.
+extern "C" int sah_attn_stream_parts(int B, int Hq, int Hkv, int Sq, int64_t S, int D, int lsh_k, int lsh_l,
+                                     int sm_count) {
+  if (B <= 0 || Hkv <= 0 || Hq <= 0 || Hq % Hkv != 0 || Sq <= 0 || S <= 0 || D != 128 || lsh_k <= 0 || lsh_l <= 0) return 0;
+  if (aum_requested() >= 0) return 0;  // a kernel has been chosen
+  const int rows = Hq / Hkv * Sq;
+  const int64_t blocks = sah_ceil_div((int64_t)rows, (int64_t)ast_rows(rows));
+  if ((int64_t)B * Hkv * blocks > 65535) return 0;
+  if (!ast_default(Hq / Hkv, Sq, lsh_k, lsh_l, blocks)) return 0;
+  return ast_splits((int64_t)B * Hkv, rows, S, sm_count > 0 ? sm_count : 148);
+}
+
+extern "C" int sah_masked_attention_stream(const void* q, const void* k, const void* v, int64_t qs_b, int64_t qs_h,
+                                           int64_t qs_q, int64_t ks_b, int64_t ks_h, int64_t ks_s, int64_t vs_b,
+                                           int64_t vs_h, int64_t vs_s, int B, int Hq, int Hkv, int Sq, int64_t S, int D,
+                                           float scaling, const void* bias, int64_t bias_s_b, int64_t bias_s_h,
+                                           int64_t bias_s_q, const float* sinks, const uint32_t* match_bits,
+                                           const uint32_t* unit_bits, int64_t W, const float* dens, int64_t dens_cap,
+                                           const unsigned int* max_norm_bits, const void* qhat, const float* qmu,
+                                           const uint16_t* weight_table, float* parts, int n_parts, void* out,
+                                           int* errflag, void* stream) {
+  SAH_REQUIRE(q && k && v && match_bits && dens && max_norm_bits && qhat && qmu && weight_table && parts && out && errflag,
+              "masked_attention_stream: null pointer");
+  SAH_REQUIRE(B > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && Sq > 0 && S > 0 && n_parts > 0,
+              "masked_attention_stream: bad extents");
+  SAH_REQUIRE(W * 32 >= S && dens_cap >= S, "masked_attention_stream: W or the key-constant stride too small");
+  if (D != 128) return sah_fail(SAH_ERR_UNSUPPORTED, "masked_attention_stream: head dim 128 (got %d)", D);
+  const int64_t strides = qs_b | qs_h | qs_q | ks_b | ks_h | ks_s | vs_b | vs_h | vs_s;
+  SAH_REQUIRE(strides % 8 == 0 && ((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)qhat) % 16 == 0,
+              "masked_attention_stream: query, K and V rows must be 16-byte aligned");
+  const int rows = Hq / Hkv * Sq, rp = ast_rows(rows);
+  const int64_t blocks = sah_ceil_div((int64_t)rows, (int64_t)rp);
+  SAH_REQUIRE((int64_t)B * Hkv * blocks <= 65535, "masked_attention_stream: too many blocks of rows");
+  AstArgs a;
+  a.q = (const __nv_bfloat16*)q; a.k = (const __nv_bfloat16*)k; a.v = (const __nv_bfloat16*)v;
+  a.qhat = (const __nv_bfloat16*)qhat; a.bias = (const __nv_bfloat16*)bias;
+  a.qs_b = qs_b; a.qs_h = qs_h; a.qs_q = qs_q;
+  a.ks_b = ks_b; a.ks_h = ks_h; a.ks_s = ks_s;
+  a.vs_b = vs_b; a.vs_h = vs_h; a.vs_s = vs_s;
+  a.bias_s_b = bias_s_b; a.bias_s_h = bias_s_h; a.bias_s_q = bias_s_q;
+  a.Hq = Hq; a.Hkv = Hkv; a.Sq = Sq; a.G = Hq / Hkv; a.blocks = (int)blocks;
+  const uint64_t at = (uintptr_t)bias | 2 * (uint64_t)(bias_s_b | bias_s_h | bias_s_q);
+  a.bias_bytes = at % 16 == 0 ? 16 : at % 8 == 0 ? 8 : at % 4 == 0 ? 4 : 2;
+  a.S = S; a.W = W; a.dens_cap = dens_cap; a.scaling = scaling;
+  a.match = match_bits; a.unit = unit_bits; a.dens = dens; a.qmu = qmu; a.max_bits = max_norm_bits;
+  a.wtable = weight_table; a.parts = parts; a.errflag = errflag;
+  const dim3 grid((unsigned)n_parts, (unsigned)(B * Hkv * blocks));
+  cudaStream_t st = (cudaStream_t)stream;
+  static bool allowed[2][64] = {};
+  const cudaError_t e = rp == 32 ? sah_allow_smem(masked_attention_stream_kernel<32>, AstCfg::SMEM, allowed[0])
+                                 : sah_allow_smem(masked_attention_stream_kernel<64>, AstCfg::SMEM, allowed[1]);
+  if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "masked_attention_stream attr: %s", cudaGetErrorString(e));
+  sah_prof_begin(SAH_PROF_ATTENTION, st);
+  if (rp == 32) sah_launch_chain(masked_attention_stream_kernel<32>, grid, AST_THREADS, AstCfg::SMEM, st, a);
+  else sah_launch_chain(masked_attention_stream_kernel<64>, grid, AST_THREADS, AstCfg::SMEM, st, a);
+  g_last_attn_kernel = "masked_attention_stream_kernel";
+  SAH_LAUNCH_CHECK("masked_attention_stream");
+  sah_launch_chain(attn_merge_parts_kernel<__nv_bfloat16>, (unsigned)((int64_t)B * Hq * Sq), D, 0, st,
+                   (const float*)parts, n_parts, (int64_t)B * Hq * Sq, Hq, Sq, D, sinks, (__nv_bfloat16*)out);
+  SAH_LAUNCH_CHECK("attn_merge_parts");
+  sah_prof_end(SAH_PROF_ATTENTION, st);
   return SAH_OK;
 }
 

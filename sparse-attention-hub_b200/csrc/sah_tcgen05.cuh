@@ -42,6 +42,15 @@ __device__ __forceinline__ void atm_cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
 
+// the same with `bytes` (16 or 0) of the source, zeros for the rest
+__device__ __forceinline__ void atm_cp_async16_zfill(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// one arrival (of those that the barrier was initialised for) once this thread's copies so far have landed
+__device__ __forceinline__ void atm_cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+
 // Shared-memory matrix descriptor of tcgen05.mma: start address, leading-dimension and stride
 // byte offsets (all in units of 16 bytes), the descriptor version of this architecture, and
 // the swizzle mode (0 none, 2 128-byte).
@@ -59,6 +68,14 @@ __device__ __forceinline__ uint64_t aum_desc(uint32_t saddr, uint32_t lbo, uint3
 __device__ __forceinline__ uint32_t aum_idesc(bool a_mn, bool b_mn, uint32_t n = 16u) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
          ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+// Descriptor of the operand `bytes` further on (the address is the lowest field, in units of 16 bytes).
+__device__ __forceinline__ uint64_t aum_desc_at(uint64_t desc, int bytes) { return desc + (uint64_t)(bytes >> 4); }
+// true in one lane of a converged warp
+__device__ __forceinline__ bool aum_elect() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0u;
 }
 __device__ __forceinline__ void aum_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {

@@ -104,6 +104,9 @@ _SIGNATURES = {
     "sah_masked_attention_lsh": [_P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _I, _I, _I, _L,
                                  _I, c_float, _P, _L, _L, _L, _P, POINTER(AttnSizes), _P, _P, _P, _P,
                                  _P, _P, _P, _P, _P, _P, _P, _P],
+    "sah_attn_stream_parts": [_I, _I, _I, _I, _L, _I, _I, _I, _I],  # returns a count
+    "sah_masked_attention_stream": [_P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _L, _L, _I, _I, _I, _I, _L, _I, c_float,
+                                    _P, _L, _L, _L, _P, _P, _P, _L, _P, _L, _P, _P, _P, _P, _P, _I, _P, _P, _P],
     "sah_mask_unit_data": [_P, _P, _P, _P, _I, _L, _L, _P, _P],
     "sah_mask_rowwise_scatter": [_P, _P, _I, _L, _L, _L, _P, _P, _P],
     "sah_mask_flat_add": [_P, _P, _I, _L, _L, _P, _P],

@@ -35,6 +35,40 @@ _workspace_cache: Dict[Tuple, Dict[str, torch.Tensor]] = {}
 _ticket_cache: Dict[Tuple, torch.Tensor] = {}
 
 
+def _error_word(device: torch.device, stream: int) -> torch.Tensor:
+    """Where the kernels that take no ticket scratch leave the error of a bounded wait, by stream and thread."""
+    key = (device.index, stream, threading.get_ident(), "error")
+    found = _ticket_cache.get(key)
+    if found is None:
+        if len(_ticket_cache) > 16:
+            _ticket_cache.clear()
+        found = _ticket_cache[key] = torch.zeros(1, dtype=torch.int32, device=device)
+    return found
+
+
+class _StreamedCall:
+    """What the union list of a call that streamed all keys is made from, should somebody ask for it."""
+
+    def __init__(self, payload, sizes, extents, stream) -> None:
+        self.match, self.unit = payload.match_bits, payload.unit_bits
+        self.dens, self.capacity, self.max_norm = payload.sig.dens, payload.sig.capacity, payload.sig.max_norm
+        self.sizes, self.extents, self.stream = sizes, extents, stream
+
+    def plan(self) -> Dict[str, Any]:
+        dev = self.match.device
+        S = self.extents[-1]
+        key = (dev.index, self.stream, threading.get_ident(), "streamed", *self.extents)
+        ws = _workspace(dev, self.sizes, key)
+        _native.check(
+            _native.load().sah_attn_plan_lsh(
+                self.match.data_ptr(), _native.ptr(self.unit), self.dens.data_ptr(), self.capacity,
+                self.max_norm.data_ptr(), *self.extents, self.match.shape[-1], ctypes.byref(self.sizes),
+                ws["ucols"].data_ptr(), ws["umemb"].data_ptr(), ws["uw"].data_ptr(), ws["ucount"].data_ptr(),
+                _native.stream_of(dev)), "sah_attn_plan_lsh")
+        return {"ucount": ws["ucount"][: self.sizes.groups], "ws": ws, "attn_sizes": self.sizes,
+                "sizes": (self.sizes.groups, self.sizes.rows_per_group, S)}
+
+
 def _bias_args(attention_mask: Optional[torch.Tensor], dtype: torch.dtype, n_keys: int):
     """(tensor kept alive, pointer, stride_b, stride_h, stride_q) of the additive bias."""
     if attention_mask is None:
@@ -130,6 +164,29 @@ def native_masked_attention(
         payload, has_data = None, int(nb.data is not None)  # materialises the weights
         nb.ensure_scan()
         sizes = _native.attn_sizes(B, Hq, Hkv, Sq, S, D, has_data, sms)
+    out = torch.empty((B, Sq, Hq, D), dtype=dtype, device=dev)
+    keep, bias_ptr, bsb, bsh, bsq = _bias_args(attention_mask, dtype, S)
+    sink_t = None
+    if sinks is not None:
+        if sinks.dim() != 1 or sinks.shape[0] != Hq:
+            raise ValueError(f"sinks must be 1D tensor of shape [H], got {tuple(sinks.shape)}")
+        sink_t = sinks.to(device=dev, dtype=torch.float32).contiguous()
+    strides = (*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
+    if payload is not None and not return_partials and _weight_dump["request"] is None:
+        n_parts = lib.sah_attn_stream_parts(B, Hq, Hkv, Sq, S, D, payload.masker.lsh_k, payload.masker.lsh_l, sms)
+        if n_parts > 0 and all(s % 8 == 0 for s in strides) and all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
+            sig = payload.sig
+            err = _error_word(dev, st)
+            parts = torch.empty((n_parts, B * Hq * Sq, D + 2), dtype=torch.float32, device=dev)
+            _native.check(
+                lib.sah_masked_attention_stream(
+                    q.data_ptr(), k.data_ptr(), v.data_ptr(), *strides, B, Hq, Hkv, Sq, S, D, float(scaling), bias_ptr,
+                    bsb, bsh, bsq, _native.ptr(sink_t), payload.match_bits.data_ptr(), _native.ptr(payload.unit_bits),
+                    payload.match_bits.shape[-1], sig.dens.data_ptr(), sig.capacity, sig.max_norm.data_ptr(),
+                    payload.qhat.data_ptr(), payload.qmu.data_ptr(), payload.weight_table.data_ptr(), parts.data_ptr(),
+                    n_parts, out.data_ptr(), err.data_ptr(), st), "sah_masked_attention_stream")
+            _last_plan["step"] = _StreamedCall(payload, sizes, (B, Hq, Hkv, Sq, S), st)
+            return out
     # scratch is reused across calls of one shape; calls that could overlap on the device
     # (another stream, another host thread) get their own
     key = (dev.index, st, threading.get_ident(), B, Hq, Hkv, Sq, S, D, has_data)
@@ -137,16 +194,8 @@ def native_masked_attention(
     if "groups" not in ws:  # where the kernel's error word sits behind the counters and tickets
         nchunks = (words_per_row(S) + 31) // 32
         ws["groups"], ws["err_index"] = sizes.groups, 2 * sizes.groups + sizes.groups * nchunks
-    keep, bias_ptr, bsb, bsh, bsq = _bias_args(attention_mask, dtype, S)
-    sink_t = None
-    if sinks is not None:
-        if sinks.dim() != 1 or sinks.shape[0] != Hq:
-            raise ValueError(f"sinks must be 1D tensor of shape [H], got {tuple(sinks.shape)}")
-        sink_t = sinks.to(device=dev, dtype=torch.float32).contiguous()
-    out = torch.empty((B, Sq, Hq, D), dtype=dtype, device=dev)
     rows = B * Hq * Sq
     part = torch.empty((rows, D + 2), dtype=torch.float32, device=dev) if return_partials else None
-    strides = (*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
     try:
         if payload is not None:
             sig = payload.sig
@@ -221,6 +270,8 @@ _last_plan: Dict[str, Any] = {"ucount": None, "ws": None, "sizes": None, "step":
 
 
 def _last() -> Dict[str, Any]:
+    if isinstance(_last_plan["step"], _StreamedCall):
+        _last_plan.update(_last_plan["step"].plan(), step=None)
     if _last_plan["step"] is not None:
         scratch, ucols, umemb, ucount, groups, rows, S, bands, extents = _last_plan["step"]
 

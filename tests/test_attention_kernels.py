@@ -180,3 +180,89 @@ def test_lists_from_one_tile_to_many_splits(dtype, D, selected):
     ref = torch.matmul(p, v.repeat_interleave(4, 1).double()).transpose(1, 2)
     err = ((out.double() - ref).norm() / ref.norm()).item()
     assert err < (2 * 2.0 ** -9 if dtype == "bf16" else 1e-5), err
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,S,bias,unit,sinks", [
+    (1, 8, 2, 4, 700, "causal", True, False),    # 16 rows, padded to a block of 32
+    (2, 8, 2, 9, 1025, "heads", True, True),     # 36 rows: a block of 64; an odd key count, one mask per head
+    (1, 4, 1, 16, 64, None, False, False),       # a single tile, nothing but matches
+    (1, 4, 1, 17, 63, "causal", True, False),    # 68 rows: two blocks, the second of four
+    (1, 4, 4, 33, 4099, "odd", True, False),     # one head per group: 33 rows; mask rows on any element
+    (1, 8, 4, 40, 321, "infinite", True, True),  # 80 rows, forbidden keys at -inf
+])
+def test_rows_of_several_positions_streamed(B, Hq, Hkv, Sq, S, bias, unit, sinks):
+    """MagicPig calls of several query positions read all keys once per block of rows: the outputs are
+    those of plain float32 attention under the mask's weights within four times what rounding to bfloat16
+    gives (1.7e-3 of the norm), the union list is the gather kernels', and so are the outputs."""
+    from sparse_attention_hub.sparse_attention.research_attention.maskers import fixed, sampling
+    from sparse_attention_hub.sparse_attention.utils import mask_attention_utils as mau
+
+    D, scaling = 128, 128 ** -0.5
+    gen = torch.Generator(device=DEV).manual_seed(S + Sq)
+    randn = lambda *s: torch.randn(s, generator=gen, device=DEV)  # noqa: E731
+    q, k, v = randn(B, Hq, Sq, D), randn(B, Hkv, S + 5, D), randn(B, Hkv, S + 5, D)
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    k, v = k[:, :, 2:S + 2], v[:, :, 2:S + 2]
+    am = None
+    if bias is not None:
+        ahead = torch.arange(S, device=DEV)[None] > torch.arange(Sq, device=DEV)[:, None] + max(S - Sq, 0)
+        low = -float("inf") if bias == "infinite" else torch.finfo(torch.bfloat16).min
+        heads = Hq if bias == "heads" else 1
+        am = torch.where(ahead, low, 0.0).expand(B, heads, Sq, S) + randn(B, heads, 1, S)
+        am = am.to(torch.bfloat16)
+        if bias == "odd":
+            am = torch.cat([am[..., :3], am], dim=-1)[..., 3:]
+    maskers = [fixed.SinkMasker(fixed.SinkMaskerConfig(sink_size=7)),
+               fixed.LocalMasker(fixed.LocalMaskerConfig(window_size=20))] if unit else []
+    maskers.append(sampling.MagicPig(sampling.MagicPigConfig(lsh_l=75, lsh_k=8, center=True)))
+    meta = {}
+
+    def mask():
+        m = Mask.create_empty_mask((B, Hq, Sq, S), torch.bfloat16, torch.device(DEV))
+        for masker in maskers:
+            m = masker.add_mask(keys=k, queries=q, values=v, attention_mask=am, scaling=scaling, dropout=0.0,
+                                sparse_meta_data=meta, previous_mask=m, layer_idx=0)
+        return m
+
+    sink = randn(Hq) if sinks else None
+    out = native_masked_attention(q, k, v, am, sink, scaling, mask())
+    assert mau.last_attention_kernel() == "masked_attention_stream_kernel"
+    streamed = [t.clone() if isinstance(t, torch.Tensor) else t for t in mau.last_union_list()]
+    prev = select_attention_kernel("mma")
+    try:
+        mau._weight_dump["request"] = True
+        gathered = native_masked_attention(q, k, v, am, sink, scaling, mask())
+        assert mau.last_attention_kernel() == "masked_attention_mma_kernel"
+        listed = mau.last_union_list()
+    finally:
+        mau._weight_dump["request"] = None
+        select_attention_kernel(prev)
+    assert attention_wait_errors() == 0
+    assert streamed[3] == listed[3] and torch.equal(streamed[2], listed[2])
+    for g, n in enumerate(listed[2].tolist()):
+        assert torch.equal(streamed[0][g, :n], listed[0][g, :n]) and torch.equal(streamed[1][g, :n], listed[1][g, :n])
+    # the weights that the gather kernel took, the attention in float64
+    kk, vv = (t.repeat_interleave(Hq // Hkv, dim=1).double() for t in (k, v))
+    logits = q.double() @ kk.transpose(2, 3) * scaling + (0.0 if am is None else am.double())
+    cols, memb, counts, R = listed
+    weights = mau._weight_dump["weights"].view(cols.shape[0], S, R).double()
+    inv = torch.zeros((B, Hq, Sq, S), dtype=torch.float64, device=DEV)
+    G = Hq // Hkv
+    q_block = R // G
+    for g, n in enumerate(counts.tolist()):
+        bk, qb = divmod(g, cols.shape[0] // (B * Hkv))
+        for r in range(R):
+            if qb * q_block + r % q_block < Sq:
+                on = (memb[g, :n].int() >> r) & 1
+                inv[bk // Hkv, bk % Hkv * G + r // q_block, qb * q_block + r % q_block, cols[g, :n].long()] = \
+                    weights[g, :n, r] * on
+    logits = logits.masked_fill(inv == 0.0, -float("inf"))
+    top = logits.amax(-1, keepdim=True).clamp(min=-1e30)
+    top = top if sink is None else torch.maximum(top, sink.double().view(1, -1, 1, 1))
+    w = torch.exp(logits - top) * inv
+    den = w.sum(-1, keepdim=True) + (0.0 if sink is None else torch.exp(sink.double().view(1, -1, 1, 1) - top))
+    want = (w @ vv / den).transpose(1, 2)
+    live = (inv.sum(-1) > 0).transpose(1, 2)[..., None]  # a row that selects nothing has no output
+    err = lambda a: (((a.double() - want) * live).nan_to_num().norm() / (want * live).nan_to_num().norm()).item()  # noqa: E731
+    assert err(out) < 6.8e-3 and err(gathered) < 6.8e-3
+    assert torch.equal(torch.isnan(out), torch.isnan(gathered))
