@@ -1037,7 +1037,7 @@ static int masked_attention_impl(const void* q, const void* k, const void* v, in
     // tensor-core path; the split merge is fused into the kernel (ticket per group)
     // long lists: keys as the M dimension of tcgen05 tiles; otherwise the mma.sync kernel
     const int umma = iv ? 0 : aum_requested();
-    if (D == 128 && (umma == 1 || (umma < 0 && aum_default(lsh != nullptr, S, groups)))) {
+    if (D == 128 && (umma == 1 || (umma < 0 && aum_default(lsh != nullptr, S, groups, a.R)))) {
       bool launched = false;
       rc = launch_attention_umma(a, B, groups, tickets, errflag, sinks, out, part_out, lsh != nullptr, st,
                                  &launched);

@@ -7,9 +7,8 @@
 //
 //   tile = 128 union entries.  Four producer warps gather their K rows and V rows with 16-byte
 //   asynchronous copies (16 lanes cover one 256-byte row, so every 32-byte sector that is
-//   fetched is used) into a three-stage ring (separate rings for K and V, with K slots freed as
-//   soon as S^T has completed, measured slower), in the 128-byte swizzled layout that the tensor
-//   core's shared-memory descriptors expect: two halves of [128 rows][128 B] per tile, 16-byte
+//   fetched is used) into rings of three K and three V tiles, in the 128-byte swizzled layout that
+//   the tensor core's shared-memory descriptors expect: two halves of [128 rows][128 B] per tile, 16-byte
 //   chunk c of row i at chunk slot c ^ (i % 8).  (Tensor-map gathers, tile::gather4, were
 //   measured first: one gather4 -- four 128-byte rows -- every ~64 cycles per SM, 2.2 TB/s over
 //   the device, below what the copies reach.)
@@ -23,14 +22,24 @@
 //   Two softmax groups of four warps take the even and the odd tiles of the CTA, each with its
 //   own S, P and O buffers and its own running maximum and denominator, so that the softmax of
 //   one tile overlaps the next tile's; the groups are merged in shared memory at the end.
-//   One elected thread issues all tcgen05.mma; completion is tracked with tcgen05.commit on
-//   mbarriers.  The running maximum is lazy: the accumulator is rescaled (tensor memory load,
+//   One warp issues all tcgen05.mma; completion is tracked with tcgen05.commit on mbarriers.
+//   S^T of a group's next tile is issued as soon as the group has the present one in registers, two
+//   tiles ahead of the second product: a group's chain is then its softmax alone.  K slots are free once S^T has completed, and the
+//   copies arrive on the barriers by themselves, so that the producers run ahead of both products.  The running maximum is lazy: the accumulator is rescaled (tensor memory load,
 //   multiply, store) only when a row's maximum grew by more than AUM_RESCALE_T, so that P stays
 //   below e^AUM_RESCALE_T; the final normalisation uses the same maximum, so the result is the
 //   softmax whatever the history of rescales.
 //
 // With LSHW the columns 4..7 of the Q tile hold the centred unit queries and the MagicPig weight
 // of a (row, key) pair is evaluated by the key's thread exactly as in the mma.sync kernel.
+//
+// Up to four rows P is multiplied in two parts, its bfloat16 rounding and the rounding of what that left, the
+// latter in columns 8 to 11, which N = 16 has anyway.
+//
+// Measured: 8 groups x 1M keys with MagicPig weights 597 us with S^T issued behind the second product of
+// the tile before, K and V freed together and a proxy fence of the producers behind every tile, 479 us this
+// way (458 us to gather the rows at the copy rate); 64 groups x 32768 keys of HashAttention 57.8 -> 52.5, a question
+// of 16 positions of PQCache over 65536 keys 121 -> 88 us.
 //
 // Every wait on an mbarrier is bounded (about a second of wall time) and watches a CTA-wide
 // abort word; a wait that runs out sets the abort word and the caller's error word, every role
@@ -57,8 +66,8 @@ struct AumCfg {
   static constexpr int Q_OFF = 2 * AUM_STAGES * KV_TILE;  // two halves of [16 rows][128 B]
   static constexpr int P_OFF = Q_OFF + 4096;              // two buffers of [128 keys][32 B]
   static constexpr int BAR_OFF = P_OFF + 2 * 4096;
-  // barriers: full[3] empty[3] s_full[2] s_free[2] p_full[2] p_free[2] max[2]
-  static constexpr int N_BARS = 2 * AUM_STAGES + 10;
+  // barriers: k_full k_free v_full v_free [3] each, s_full[2] s_free[2] p_full[2] p_free[2] max[2]
+  static constexpr int N_BARS = 4 * AUM_STAGES + 10;
   static constexpr int MISC_OFF = BAR_OFF + ((N_BARS * 8 + 15) & ~15);
   // misc: tmem slot, abort word, last flag, pad; then wmax [2][4][16], lred [2][4][16], group
   // maxima [2][16], qmu [16], bias offsets [16] (int64)
@@ -149,7 +158,8 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
   // barrier addresses
   const uint32_t bar0 = sm_s + C::BAR_OFF;
   constexpr int NST = AUM_STAGES;
-  const uint32_t full = bar0, empty = bar0 + NST * 8, s_full = bar0 + 2 * NST * 8, s_free = s_full + 16,
+  const uint32_t k_full = bar0, k_free = bar0 + NST * 8, v_full = bar0 + 2 * NST * 8, v_free = bar0 + 3 * NST * 8,
+                 s_full = bar0 + 4 * NST * 8, s_free = s_full + 16,
                  p_full = s_full + 32, p_free = s_full + 48, max_bar = s_full + 64;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + C::MISC_OFF);
   volatile int* abort_sm = reinterpret_cast<volatile int*>(sm + C::MISC_OFF + 4);
@@ -164,8 +174,10 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
   if (tid == 0) {
 #pragma unroll
     for (int i = 0; i < NST; ++i) {
-      atm_mbar_init(full + i * 8, AUM_PROD_WARPS);  // one arrival per producer warp
-      atm_mbar_init(empty + i * 8, 1);              // tcgen05.commit after the tile's second product
+      atm_mbar_init(k_full + i * 8, AUM_PROD_WARPS * 32);  // the copies of every producer thread
+      atm_mbar_init(v_full + i * 8, AUM_PROD_WARPS * 32);
+      atm_mbar_init(k_free + i * 8, 1);                    // tcgen05.commit after the tile's first product
+      atm_mbar_init(v_free + i * 8, 1);                    // ... after its second
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -178,6 +190,7 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     *abort_sm = 0;
   }
+  __syncthreads();  // the producers start on the barriers while the others prepare the queries
   if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::
                      "r"((uint32_t)__cvta_generic_to_shared(tmem_slot)),
@@ -186,7 +199,8 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
   }
   // ---- Q tile: rows = mask rows (LSHW: rows 4..7 = centred unit queries), zero padded to 16;
   //      two halves of [16 rows][128 B], 16-byte chunk c of a row at slot (c % 8) ^ (row % 8) ----
-  for (int idx = tid; idx < 16 * 16; idx += AUM_THREADS) {
+  if (warp < AUM_SOFT_WARPS) {  // 256 threads, one 16-byte chunk each
+    const int idx = tid;
     const int r = idx >> 4, c = idx & 15;
     uint4 val = make_uint4(0u, 0u, 0u, 0u);
     const int rq = (LSHW && r >= 4) ? r - 4 : r;
@@ -220,11 +234,14 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
     qmu_sm[r] = mu;
     boff_sm[r] = bo;
   }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // generic writes -> tensor-core reads
-  aum_fence_before();
-  __syncthreads();
-  aum_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  uint32_t tmem = 0;
+  if (warp < AUM_SOFT_WARPS || warp == MMA_WARP) {
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // generic writes -> tensor-core reads
+    aum_fence_before();
+    asm volatile("bar.sync 2, %0;\n" ::"n"((AUM_SOFT_WARPS + 1) * 32) : "memory");
+    aum_fence_after();
+    tmem = *tmem_slot;
+  }
   // tensor memory columns: S of group 0, S of group 1, O of group 0, O of group 1 (16 each)
 
   if (warp >= AUM_SOFT_WARPS && warp < MMA_WARP) {
@@ -240,8 +257,6 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
                                        reinterpret_cast<const __nv_bfloat16*>(a.v) + b * a.vs_b + kvh * a.vs_h) +
                                    my_chunk * 16;
     const int64_t ks_bytes = a.ks_s * 2, vs_bytes = a.vs_s * 2;
-    // destination of (row 2 * it + my_sub, chunk my_chunk) inside a K (or V) tile
-    const uint32_t half_off = (uint32_t)(my_chunk >> 3) * C::HALF_BYTES;
     auto load_col = [&](int t) {
       int col = -1;
       if (t < my_tiles) {
@@ -250,111 +265,93 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
       }
       return col;
     };
-    int col_next = load_col(0);
-    auto issue = [&](int t) {
-      const int st = t % NST;
-      const int col = col_next;
-      col_next = load_col(t + 1);
-      const uint32_t kt = C::K_RING + st * C::KV_TILE + half_off;
+    // (row 2 * it + my_sub, chunk my_chunk) of the warp's 32 rows; zeros past the end of the list, not
+    // stale bits, go into the tensor core
+    const uint32_t in = (uint32_t)(my_chunk >> 3) * C::HALF_BYTES + (uint32_t)(pw * 32 + my_sub) * 128;
+    auto copy = [&](uint32_t tile, const unsigned char* rows, int64_t row_bytes, int col) {
 #pragma unroll
       for (int it = 0; it < 16; ++it) {
-        const int rw = it * 2 + my_sub;  // row within the warp's 32
+        const int rw = it * 2 + my_sub;
         const int rc = __shfl_sync(0xffffffffu, col, rw);
-        const uint32_t off = kt + (uint32_t)(pw * 32 + rw) * 128 + ((uint32_t)((my_chunk & 7) ^ (rw & 7)) << 4);
-        if (rc >= 0) {
-          atm_cp_async16(sm_s + off, k_bytes + rc * ks_bytes);
-          atm_cp_async16(sm_s + off + (C::V_RING - C::K_RING), v_bytes + rc * vs_bytes);
-        } else {  // past the end of the list: zeros, not stale bits, go into the tensor core
-          *reinterpret_cast<uint4*>(sm + off) = make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(sm + off + (C::V_RING - C::K_RING)) = make_uint4(0u, 0u, 0u, 0u);
-        }
+        atm_cp_async16_zfill(tile + in + it * 256 + ((uint32_t)((my_chunk & 7) ^ (rw & 7)) << 4),
+                             rows + (rc < 0 ? 0 : rc) * row_bytes, rc < 0 ? 0u : 16u);
       }
     };
-    // issue() takes the tiles in order (it carries the prefetched columns along)
-#pragma unroll
-    for (int s0 = 0; s0 < NST - 1; ++s0) {
-      if (s0 < my_tiles) issue(s0);
-      asm volatile("cp.async.commit_group;\n" ::);
+    auto put_k = [&](int t, int col) {
+      const int st = t % NST;
+      if (t >= NST && !aum_wait_warp(k_free + st * 8, (uint32_t)((t / NST - 1) & 1), abort_sm, errflag)) return false;
+      copy(sm_s + C::K_RING + st * C::KV_TILE, k_bytes, ks_bytes, col);
+      atm_cp_async_arrive(k_full + st * 8);
+      return true;
+    };
+    int col = load_col(0), col_next = load_col(1);
+    bool okp = my_tiles <= 0 || put_k(0, col);
+    for (int t = 0; t < my_tiles && okp; ++t) {  // K one tile ahead of V
+      const int col_after = load_col(t + 2);
+      if (t + 1 < my_tiles) okp = put_k(t + 1, col_next);
+      if (!okp) break;
+      const int st = t % NST;
+      if (t >= NST) okp = aum_wait_warp(v_free + st * 8, (uint32_t)((t / NST - 1) & 1), abort_sm, errflag);
+      if (!okp) break;
+      copy(sm_s + C::V_RING + st * C::KV_TILE, v_bytes, vs_bytes, col);
+      atm_cp_async_arrive(v_full + st * 8);
+      col = col_next;
+      col_next = col_after;
     }
-    for (int t = 0; t < my_tiles; ++t) {
-      // tile t has landed (this thread's share): make it visible to the tensor core, signal
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(NST - 2));
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      __syncwarp();
-      if (lane == 0) aum_arrive(full + (t % NST) * 8);
-      // refill the stage that tile t - 1 used once its second product has completed
-      const int nx = t + NST - 1;
-      if (nx < my_tiles) {
-        bool okp = true;
-        if (nx >= NST) {
-          AUM_T0();
-          okp = aum_wait_warp(empty + (nx % NST) * 8, (uint32_t)(((nx / NST) - 1) & 1), abort_sm, errflag);
-          if (lane == 0 && pw == 0) AUM_T1(0);
-        }
-        if (!okp) break;
-        issue(nx);
-      }
-      asm volatile("cp.async.commit_group;\n" ::);
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
   } else if (warp == MMA_WARP) {
     // =========================== tensor-core issuer ===========================
-    if (lane == 0) {
-      const uint32_t idesc_qk = aum_idesc(false, false);
-      const uint32_t idesc_pv = aum_idesc(true, AUM_P_MN_MAJOR != 0);
-      const uint32_t q_s = sm_s + C::Q_OFF;
-      bool ok = true;
-      auto pv = [&](int t) {
-        const int st = t % NST, gg = t & 1, j = t >> 1;
-        {
-          AUM_T0();
-          const bool o2 = aum_wait(p_full + gg * 8, (uint32_t)(j & 1), abort_sm, errflag);
-          AUM_T1(5);
-          if (!o2) return false;
-        }
-        aum_fence_after();
-        const uint32_t v_s = sm_s + C::V_RING + st * C::KV_TILE;
-        const uint32_t p_s = sm_s + C::P_OFF + gg * 4096;
+    // The whole warp walks the tiles, so that the operands are known to be the same for all lanes, and one
+    // lane issues; descriptors differ by constants.
+    const uint32_t idesc_qk = aum_idesc(false, false);
+    const uint32_t idesc_pv = aum_idesc(true, AUM_P_MN_MAJOR != 0);
+    const uint64_t dq = aum_desc(sm_s + C::Q_OFF, 0, 1024, 2), dk = aum_desc(sm_s + C::K_RING, 0, 1024, 2),
+                   dv = aum_desc(sm_s + C::V_RING, C::HALF_BYTES, 1024, 2), dp = aum_p_desc(sm_s + C::P_OFF, 0);
+    bool ok = true;
+    auto qk = [&](int t) {
+      const int st = t % NST, gg = t & 1, j = t >> 1;
+      if (!aum_wait_warp(k_full + st * 8, (uint32_t)((t / NST) & 1), abort_sm, errflag)) return false;
+      if (j >= 1 && !aum_wait_warp(s_free + gg * 8, (uint32_t)((j - 1) & 1), abort_sm, errflag)) return false;
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the producers' copies -> tensor-core reads
+      aum_fence_after();
+      if (aum_elect()) {
+        const uint64_t kd = aum_desc_at(dk, st * C::KV_TILE);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
+        for (int ks = 0; ks < 8; ++ks)
+          // both K-major, 128-byte swizzle: 8-row groups 1 KB apart, 32 bytes per k-step
+          aum_mma(tmem + gg * 16, aum_desc_at(kd, (ks >> 2) * C::HALF_BYTES + (ks & 3) * 32),
+                  aum_desc_at(dq, (ks >> 2) * 2048 + (ks & 3) * 32), idesc_qk, ks > 0 ? 1u : 0u);
+        aum_commit(s_full + gg * 8);
+        aum_commit(k_free + st * 8);
+      }
+      __syncwarp();
+      return true;
+    };
+    auto pv = [&](int t) {
+      const int st = t % NST, gg = t & 1, j = t >> 1;
+      if (!aum_wait_warp(v_full + st * 8, (uint32_t)((t / NST) & 1), abort_sm, errflag)) return false;
+      if (!aum_wait_warp(p_full + gg * 8, (uint32_t)(j & 1), abort_sm, errflag)) return false;
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      aum_fence_after();
+      if (aum_elect()) {
+        const uint64_t vd = aum_desc_at(dv, st * C::KV_TILE), pd = aum_desc_at(dp, gg * 4096);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
           // A = V^T, MN-major: 64 dims contiguous per 128-byte row, 8 keys per 1 KB atom,
           // the second 64 dims one half further
-          const uint64_t ad = aum_desc(v_s + ks * 2048, C::HALF_BYTES, 1024, 2);
-          const uint64_t bd = aum_p_desc(p_s, ks);
-          aum_mma(tmem + 32 + gg * 16, ad, bd, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-        }
-        aum_commit(empty + st * 8);
+          aum_mma(tmem + 32 + gg * 16, aum_desc_at(vd, ks * 2048), aum_desc_at(pd, ks * 512), idesc_pv,
+                  (j > 0 || ks > 0) ? 1u : 0u);
+        aum_commit(v_free + st * 8);
         aum_commit(p_free + gg * 8);
-        return true;
-      };
-      for (int t = 0; t < my_tiles && ok; ++t) {
-        const int st = t % NST, gg = t & 1, j = t >> 1;
-        {
-          AUM_T0();
-          ok = aum_wait(full + st * 8, (uint32_t)((t / NST) & 1), abort_sm, errflag);
-          AUM_T1(6);
-        }
-        {
-          AUM_T0();
-          if (ok && j >= 1) ok = aum_wait(s_free + gg * 8, (uint32_t)((j - 1) & 1), abort_sm, errflag);
-          AUM_T1(7);
-        }
-        if (!ok) break;
-        aum_fence_after();
-        const uint32_t k_s = sm_s + C::K_RING + st * C::KV_TILE;
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          // both K-major, 128-byte swizzle: 8-row groups 1 KB apart, 32 bytes per k-step
-          const uint64_t ad = aum_desc(k_s + (ks >> 2) * C::HALF_BYTES + (ks & 3) * 32, 0, 1024, 2);
-          const uint64_t bd = aum_desc(q_s + (ks >> 2) * 2048 + (ks & 3) * 32, 0, 1024, 2);
-          aum_mma(tmem + gg * 16, ad, bd, idesc_qk, ks > 0 ? 1u : 0u);
-        }
-        aum_commit(s_full + gg * 8);
-        if (t >= 1) ok = pv(t - 1);
       }
-      if (ok && my_tiles > 0) pv(my_tiles - 1);
+      __syncwarp();
+      return true;
+    };
+    for (int t = 0; t < 2 && t < my_tiles && ok; ++t) ok = qk(t);
+    for (int t = 0; t < my_tiles && ok; ++t) {
+      if (t + 2 < my_tiles) ok = qk(t + 2);
+      ok = ok && pv(t);
     }
-    __syncwarp();
   } else {
     // =========================== softmax: one thread per key, two groups ===========================
     const int gg = warp >> 2;            // group: tiles gg, gg + 2, ...
@@ -481,6 +478,9 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
         l_thr[r] = l_thr[r] * alpha[r] + pr[r];
         l_thr[r + 1] = l_thr[r + 1] * alpha[r + 1] + pr[r + 1];
         pk[r >> 1] = atm_pack_bf16(pr[r], pr[r + 1]);
+        if constexpr (RMAX == 4)  // what rounding took away goes into columns 8 to 11, which are there anyway
+          pk[4 + (r >> 1)] = atm_pack_bf16(pr[r] - __uint_as_float(pk[r >> 1] << 16),
+                                           pr[r + 1] - __uint_as_float(pk[r >> 1] & 0xffff0000u));
       }
       // the group's P buffer is free, and its accumulator quiet, once the product of the group's
       // previous tile has completed
@@ -495,7 +495,10 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
         uint32_t orow[16];
         aum_tmem_ld16(tmem_o + lane_base, orow);
 #pragma unroll
-        for (int r = 0; r < RMAX; ++r) orow[r] = __float_as_uint(__uint_as_float(orow[r]) * alpha[r]);
+        for (int r = 0; r < RMAX; ++r) {
+          orow[r] = __float_as_uint(__uint_as_float(orow[r]) * alpha[r]);
+          if (RMAX == 4) orow[8 + r] = __float_as_uint(__uint_as_float(orow[8 + r]) * alpha[r]);
+        }
         aum_tmem_st16(tmem_o + lane_base, orow);
       }
       aum_store_p(sm + C::P_OFF + gg * 4096, key, pk);
@@ -520,6 +523,10 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
       if (ok) {
         aum_fence_after();
         aum_tmem_ld16(tmem_o + lane_base, orow);
+        if constexpr (RMAX == 4) {
+#pragma unroll
+          for (int r = 0; r < RMAX; ++r) orow[r] = __float_as_uint(__uint_as_float(orow[r]) + __uint_as_float(orow[8 + r]));
+        }
       }
     }
 #pragma unroll
@@ -581,24 +588,27 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
 }
 
 // Which problems take the tcgen05 kernel when neither the caller nor the environment says.
-// Measured on B200 (attention kernel, tcgen05 against mma.sync).  MagicPig weights in place,
-// 8 KV groups: 1M keys (~770 000 rows per group, two waves of CTAs) 639 us; with one wave of
-// CTAs (AUM_ONE_WAVE_TILES) 512K keys 332 against 366 us; 256K keys 177 against 189 us; 128K
-// keys 99 against 108 us; 64K keys 63 against 73 us (two waves from 512K down: 337, 185 and
-// 111 us -- a CTA's prologue, pipeline fill and merge are paid once per SM instead of twice).  64 KV groups with lists of a few
-// thousand rows (HashAttention and Quest at B = 8, S = 32768): 63 against 69 us and 56 against
-// 61 us.  In between -- 8 to 32 groups with lists of 10^4..10^5 rows -- the mma.sync kernel,
-// with two CTAs per SM and lower fixed costs, was ahead by 5-40 % (measured with two waves).
-// Few groups with short lists stay on the mma.sync kernel although this one is ahead there (one
-// query, 8 groups: 18 to 30 against 22 to 36 us for lists of 400 to 6000 rows), because it is less
-// exact: the maximum that P is taken against is shared by tiles of 128 entries and may lie up to
-// AUM_RESCALE_T below the true one, so a row's largest weights are rounded to bfloat16, while a warp
-// of the mma.sync kernel holds the largest of its 16 to 100 entries exactly (as 1).  Relative error
-// against float64 where one key of a hundred carries the weight (HashAttention, 8 groups, 4096 to
-// 97000 keys): 1.8e-3 to 2.3e-3 here, 1.7e-3 there; flat rows: 1.7e-3 in both.
-#define AUM_DEFAULT_MIN_KEYS (64 * 1024)
-static bool aum_default(bool lsh, int64_t S, int groups) {
-  return (lsh && S >= AUM_DEFAULT_MIN_KEYS) || (groups >= 64 && S <= 65536);
+// Measured on B200 (attention kernel, mma.sync against tcgen05, us; L2 flushed).
+//   MagicPig weights in place, one query position: 8 KV groups of 4 rows, 8192 keys 18.0 / 16.4, 32768
+//   37.7 / 29.4, 65500 61 / 49; 2 groups, 16384 keys 17.3 / 14.9; 8 groups of one row, 16384 keys
+//   17.8 / 14.8; 32 groups, 16384 keys 60 / 50.
+//   Up to four rows, lists: 8 groups, 16384 keys, union of 3600 14.2 / 13.4; 131072 keys, 10100 21.2 / 19.6;
+//   32768 keys, 25000 35.6 / 30.1; 32 groups, 65536 keys, weighted, 22600 84.5 / 78.1, 64000 208 / 176;
+//   64 groups, 32768 keys, 2550 35.0 / 27.3, 24900 166 / 142; 16 groups, 100000 keys, 97400 160 / 138.
+//   Fewer rows times keys leave short lists, where the other's fixed costs are lower: 8192 keys, 4 rows,
+//   union of 1530 10.7 / 11.8; 16384 keys, one row, 1630 10.3 / 11.1.  (Up to 32768 keys a mask may be bands
+//   alone, hundreds of columns, which this rule cannot see; it leaves those sizes to the other kernel.)
+//   More than four rows (no room for P's remainders, exactness below): 8 groups of 8, 65536 keys 36.2 / 38.5,
+//   32 groups of 8, 32768 keys 52 / 56; 64 groups with lists of a few thousand rows 69 / 63.
+// Up to four rows the error against float64 is below the other's, 1.6e-3 to 1.7e-3 against 1.8e-3 to 2.2e-3 of
+// the norm (what rounding the output leaves), because P is multiplied in two parts.  With more, P is rounded to
+// bfloat16 against a maximum that may lie up to AUM_RESCALE_T below the true one: 2.0e-3 to 2.3e-3.
+#define AUM_MIN_LSH_KEYS 8192
+#define AUM_MIN_KEYS 32768
+#define AUM_MIN_ROW_KEYS 65536
+static bool aum_default(bool lsh, int64_t S, int groups, int rows) {
+  if (rows <= 4 && (lsh ? S >= AUM_MIN_LSH_KEYS : S > AUM_MIN_KEYS && rows * S >= AUM_MIN_ROW_KEYS)) return true;
+  return groups >= 64 && S <= 65536;
 }
 
 // The kernel choice: a process-wide setting (sah_attn_select_kernel), else SAH_ATTN_UMMA in the
