@@ -18,7 +18,7 @@ from ..utils.mask_attention_utils import (
     get_masked_attention_output,
     get_true_attention_output,
 )
-from .fixed_step import fixed_step
+from .fixed_step import SERVED, fixed_step
 from .maskers.base import MaskerConfig, ResearchMasker
 from .maskers.sampling.base import SamplingMasker
 
@@ -79,7 +79,13 @@ class ResearchAttention(SparseAttention):
             )
         sparse_meta_data: Dict[Any, Any] = kwargs.pop("sparse_meta_data")
         logger = MicroMetricLogger()
-        if (not logger.enabled_metrics and not self.return_attention_weights and dropout == 0.0
+        for masker in self.maskers:  # all that other stacks pay for the native entry
+            if type(masker) not in SERVED:
+                native = False
+                break
+        else:
+            native = True
+        if (native and not logger.enabled_metrics and not self.return_attention_weights and dropout == 0.0
                 and kwargs.get("sequence_shard") is None
                 and type(self).build_mask is ResearchAttention.build_mask and "build_mask" not in self.__dict__):
             # nobody looks at the mask of this call: bands and an exact top-k need none
@@ -91,7 +97,7 @@ class ResearchAttention(SparseAttention):
         mask = self.build_mask(queries, keys, values, attention_mask, scaling, dropout,
                                sparse_meta_data, **kwargs)
 
-        if logger.is_metric_enabled("research_attention_density"):
+        if logger.enabled_metrics and logger.is_metric_enabled("research_attention_density"):
             logger.log("research_attention_density", mask.get_density(),
                        metadata={"layer_idx": kwargs["layer_idx"]})
 
@@ -107,7 +113,7 @@ class ResearchAttention(SparseAttention):
         else:
             attention_output, attention_weights = result, None
 
-        if logger.is_metric_enabled("research_attention_output_error"):
+        if logger.enabled_metrics and logger.is_metric_enabled("research_attention_output_error"):
             true_out, _ = get_true_attention_output(module, queries, keys, values, attention_mask,
                                                     scaling, dropout, **kwargs)
             error = torch.norm(true_out - attention_output) / torch.norm(true_out)

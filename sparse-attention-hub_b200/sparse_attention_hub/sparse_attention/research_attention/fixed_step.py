@@ -26,6 +26,9 @@ from .maskers.fixed.implementations.oracle_top_k import OracleTopK
 _MAX_BANDS = 6       # SAH_STEP_MAX_BANDS
 _N_TICKETS = 16384   # KV groups per call, and the error word
 
+#: the maskers that it serves, in some orders; their subclasses are not among them
+SERVED = frozenset((SinkMasker, LocalMasker, OracleTopK))
+
 _module = None
 
 

@@ -172,7 +172,7 @@ def native_masked_attention(
             raise ValueError(f"sinks must be 1D tensor of shape [H], got {tuple(sinks.shape)}")
         sink_t = sinks.to(device=dev, dtype=torch.float32).contiguous()
     strides = (*q.stride()[:3], *k.stride()[:3], *v.stride()[:3])
-    if payload is not None and not return_partials and _weight_dump["request"] is None:
+    if payload is not None and Sq > 1 and not return_partials and _weight_dump["request"] is None:
         n_parts = lib.sah_attn_stream_parts(B, Hq, Hkv, Sq, S, D, payload.masker.lsh_k, payload.masker.lsh_l, sms)
         if n_parts > 0 and all(s % 8 == 0 for s in strides) and all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
             sig = payload.sig
