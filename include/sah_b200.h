@@ -468,8 +468,8 @@ int sah_lsh_key_sign(const void* keys, int dtype, int64_t ks_b, int64_t ks_h, in
  * sah_lsh_key_sign_tc_ws_bytes) starts with two status words that the caller may read after the
  * stream has finished: [0] the number of 32-column groups that were redone -- a value above
  * (workspace_bytes - 16) / 16 means the list overflowed and the range must be redone with
- * sah_lsh_key_sign; [1] non-zero when a bounded wait inside the kernel ran out (the range must
- * be redone as well). */
+ * sah_lsh_key_sign; [1] non-zero when a bounded wait inside the kernel ran out, or when the list, whose
+ * end a long one leaves to a copy of the hyperplanes, overflowed (the range must be redone as well). */
 int64_t sah_lsh_key_sign_tc_ws_bytes(int B, int Hkv, int64_t n_keys);
 int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h, int64_t ks_s, int B, int Hkv,
                         int64_t s0, int64_t s1, int D, const void* mean, const float* norms,

@@ -414,9 +414,17 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
   cudaStream_t st = (cudaStream_t)stream;
   int* status = reinterpret_cast<int*>(workspace);
   LtcUncertain* list = reinterpret_cast<LtcUncertain*>(reinterpret_cast<unsigned char*>(workspace) + 16);
-  const int list_cap = (int)((workspace_bytes - 16) / (int64_t)sizeof(LtcUncertain) < (1ll << 30)
-                                 ? (workspace_bytes - 16) / (int64_t)sizeof(LtcUncertain)
-                                 : (1ll << 30));
+  int64_t entries = (workspace_bytes - 16) / (int64_t)sizeof(LtcUncertain);
+  if (entries > (1ll << 30)) entries = 1ll << 30;
+  // A long list leaves its end to the hyperplanes, one by one: a column of `proj` is a sector per
+  // channel (88 thousand entries 102 -> 51 us).  It holds a quarter of the keys and takes up to a sixth.
+  const int64_t plane_entries = (int64_t)L * 8 * LTC_PLANE * 2 / (int64_t)sizeof(LtcUncertain);
+  __nv_bfloat16* planes = nullptr;
+  if (entries >= 8 * plane_entries) {
+    entries -= plane_entries;
+    planes = reinterpret_cast<__nv_bfloat16*>(list + entries);
+  }
+  const int list_cap = (int)entries;
   cudaError_t e = cudaMemsetAsync(status, 0, 16, st);
   if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "lsh_key_sign_tc memset: %s", cudaGetErrorString(e));
   static bool allowed[2][64] = {};
@@ -438,12 +446,12 @@ extern "C" int sah_lsh_key_sign_tc(const void* keys, int64_t ks_b, int64_t ks_h,
   lsh_key_sign_tc_kernel<<<grid, LTC_THREADS, LtcCfg::SMEM, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(keys), ks_b, ks_h, ks_s, Hkv, BH, s0, s1,
       reinterpret_cast<const __nv_bfloat16*>(mean), norms, max_norm_bits, reinterpret_cast<const __nv_bfloat16*>(proj),
-      L, chunk_cols, cap, reinterpret_cast<uint8_t*>(codes), list, list_cap, status, status + 1);
+      L, chunk_cols, cap, reinterpret_cast<uint8_t*>(codes), list, list_cap, status, status + 1, planes);
   SAH_LAUNCH_CHECK("lsh_key_sign_tc");
   lsh_sign_recheck_kernel<<<(unsigned)(sm_count * 3), LTC_RC_WARPS * 32, LTC_RC_SMEM, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(keys), ks_b, ks_h, ks_s, Hkv, reinterpret_cast<const __nv_bfloat16*>(mean),
       norms, max_norm_bits, reinterpret_cast<const __nv_bfloat16*>(proj), L, cap, reinterpret_cast<uint8_t*>(codes),
-      list, list_cap, status);
+      list, list_cap, status, planes);
   SAH_LAUNCH_CHECK("lsh_sign_recheck");
   return SAH_OK;
 }

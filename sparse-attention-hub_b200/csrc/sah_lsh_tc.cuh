@@ -33,7 +33,9 @@
 // away at most, rounds to the same bfloat16 number; operands near the ends of the range take the
 // division (a division per channel, its slow path's branch and the load in front of it in series
 // were most of the 1495 us that the kernel took at that size; 629 us with one set of producers that
-// branched per row; now 531 us, and the recheck 507 -> 121 us).
+// branched per row; 546 us with two, which sent every row with a zero to the division -- a few in
+// every tile -- and with an epilogue that waited for each group's values in turn; 336 us now, pairs of
+// channels in one operation.  The recheck went from 507 over 121 to 51 us).
 //
 // Every mbarrier wait is bounded (sah_tcgen05.cuh); a wait that runs out sets the error word,
 // all roles leave their loops, tensor memory is freed.
@@ -47,6 +49,7 @@
 #define LTC_PROD 8       // producer warps, in two sets that take alternate tiles
 #define LTC_THREADS (32 * (LTC_EPI + LTC_PROD + 1))  // and 1 issuing warp
 #define LTC_QUEUE 64     // entries of a warp's queue of groups to redo
+#define LTC_PLANE 136    // channels of a hyperplane where they are stored one by one
 #define LTC_TAU_SCALE 3.0517578125e-05f  // 2^-15
 
 struct LtcCfg {
@@ -79,7 +82,17 @@ __device__ __forceinline__ void ltc_tmem_ld32(uint32_t taddr, uint32_t* r) {
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+// the values of a load may be read after this on the same registers
+__device__ __forceinline__ void ltc_tmem_wait(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                 "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
+                 "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
+                 "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
 }
 
 // smallest magnitude of three; NaN if there is one
@@ -87,6 +100,28 @@ __device__ __forceinline__ float ltc_minabs3(float a, float b, float c) {
   float d;
   asm("min.NaN.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(fabsf(b)), "f"(fabsf(c)));
   return d;
+}
+
+// pairs of floats in one operation, each half rounded as the scalar one is
+__device__ __forceinline__ unsigned long long ltc_bits(float2 v) {
+  unsigned long long u;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(u) : "f"(v.x), "f"(v.y));
+  return u;
+}
+__device__ __forceinline__ float2 ltc_pair(unsigned long long u) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(u));
+  return v;
+}
+__device__ __forceinline__ unsigned long long ltc_add2(unsigned long long a, unsigned long long b) {
+  unsigned long long c;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
+}
+__device__ __forceinline__ unsigned long long ltc_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long c;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
 }
 
 // Grid: (workers, column chunks of `chunk_cols`, a multiple of 32).  Worker w of a chunk takes the tiles w, w + workers, ... of the
@@ -97,7 +132,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
                        const float* __restrict__ norms, const unsigned int* __restrict__ max_bits,
                        const __nv_bfloat16* __restrict__ proj, int L, int chunk_cols, int64_t cap,
                        uint8_t* __restrict__ codes, LtcUncertain* __restrict__ list, int list_cap,
-                       int* __restrict__ list_count, int* __restrict__ errflag) {
+                       int* __restrict__ list_count, int* __restrict__ errflag, __nv_bfloat16* __restrict__ planes) {
   constexpr int D = 128;
   using C = LtcCfg;
   extern __shared__ __align__(1024) unsigned char ltc_raw[];
@@ -152,6 +187,9 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
     }
     *reinterpret_cast<uint4*>(sm + C::B_OFF + (c >> 3) * C::B_ATOM + n * 128 + (((c & 7) ^ (n & 7)) << 4)) =
         *reinterpret_cast<const uint4*>(v);
+    // the hyperplanes one by one for the kernel behind this one
+    if (planes != nullptr && blockIdx.x == 0 && n < ncols && c * 8 < LTC_PLANE)
+      *reinterpret_cast<uint4*>(planes + (int64_t)(col_base + n) * LTC_PLANE + c * 8) = *reinterpret_cast<const uint4*>(v);
   }
   // tau of every column: 2^-15 * 1.01 * |p|
   for (int n = tid; n < LTC_NCHUNK; n += LTC_THREADS) {
@@ -188,7 +226,8 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
     // the multiplication stands for the division only for a bfloat16 M well inside the range
     const bool divide = (__float_as_uint(M) & 0xffffu) != 0u || !(M >= 8.673617e-19f && M <= 1.152921504606847e18f);
     int64_t bh_cur = -1;
-    float m8[8];
+    unsigned long long neg_mean[4];
+    const unsigned long long rM2 = ltc_bits(make_float2(rM, rM));
     uint4 raw[16];
     auto fetch = [&](int t) {
       const int64_t flat = first + (int64_t)t * stride;
@@ -209,7 +248,12 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
       const int64_t key0 = s0 + (flat - bh * tiles_per_bh) * LTC_TILE;
       if (bh != bh_cur) {
         bh_cur = bh;
-        if (mean != nullptr) sah_unpack8(*reinterpret_cast<const uint4*>(mean + bh * D + my_chunk * 8), m8);
+        if (mean != nullptr) {
+          float m8[8];
+          sah_unpack8(*reinterpret_cast<const uint4*>(mean + bh * D + my_chunk * 8), m8);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) neg_mean[i] = ltc_bits(make_float2(-m8[2 * i], -m8[2 * i + 1]));
+        }
       }
       const float nk = key0 + pw * 32 + lane < s1 ? norms[bh * cap + key0 + pw * 32 + lane] : 0.f;
       if (t >= 2 && !aum_wait_warp(a_empty + buf * 8, (uint32_t)(((t >> 1) - 1) & 1), abort_sm, errflag)) break;
@@ -222,20 +266,28 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
       for (int it = 0; it < 16; ++it) {
         const int r = pw * 32 + it * 2 + my_sub;
         uint32_t w[4] = {raw[it].x, raw[it].y, raw[it].z, raw[it].w};
-        bool odd = divide;
+        float smallest = INFINITY;
+        float2 x[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xffff0000u);
+          x[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
           if (mean != nullptr) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(__fsub_rn(lo, m8[2 * i]), __fsub_rn(hi, m8[2 * i + 1]));
+            x[i] = ltc_pair(ltc_add2(ltc_bits(x[i]), neg_mean[i]));  // x - mean
+            const __nv_bfloat162 h = __floats2bfloat162_rn(x[i].x, x[i].y);
             const uint32_t u = *reinterpret_cast<const uint32_t*>(&h);
-            lo = __uint_as_float(u << 16);
-            hi = __uint_as_float(u & 0xffff0000u);
+            x[i] = make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
           }
-          // below 2^-60 the quotient might be denormal (or zero)
-          odd = odd || fabsf(lo) < 8.673617e-19f || fabsf(hi) < 8.673617e-19f;
-          const __nv_bfloat162 q = __floats2bfloat162_rn(__fmul_rn(lo, rM), __fmul_rn(hi, rM));
+          smallest = ltc_minabs3(smallest, x[i].x, x[i].y);
+          const float2 p = ltc_pair(ltc_mul2(ltc_bits(x[i]), rM2));
+          const __nv_bfloat162 q = __floats2bfloat162_rn(p.x, p.y);
           w[i] = *reinterpret_cast<const uint32_t*>(&q);
+        }
+        bool odd = divide;
+        if (!(smallest >= 8.673617e-19f)) {  // below 2^-60 the quotient might be denormal; zero stays zero
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            odd = odd || !(fabsf(x[i].x) >= 8.673617e-19f || x[i].x == 0.f) ||
+                  !(fabsf(x[i].y) >= 8.673617e-19f || x[i].y == 0.f);
         }
         const bool live = key0 + r < s1;
         if (odd && live) slow |= 1u << it;
@@ -304,6 +356,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
       __syncwarp();
       for (int i = lane; i < queued; i += 32)
         if (base + i < list_cap) list[base + i] = queue[i];
+      if (lane == 0 && base + queued > list_cap) atomicExch(errflag, 1);
       __syncwarp();
       queued = 0;
     };
@@ -325,9 +378,7 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
       if (!aum_wait_warp(d_full + buf * 8, (uint32_t)((t >> 1) & 1), abort_sm, errflag)) break;
       aum_fence_after();
       const int64_t row = bh * cap + s;
-      for (int gq = 0; gq < groups; ++gq) {
-        uint32_t acc[32];
-        ltc_tmem_ld32(tmem + lane_base + buf * LTC_NCHUNK + gq * 32, acc);
+      auto group = [&](int gq, const uint32_t* acc) {
         uint32_t neg[4] = {0u, 0u, 0u, 0u};
         float mn[4];
 #pragma unroll
@@ -375,6 +426,20 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
             __syncwarp();
           }
         }
+      };
+      // the next group's values are on their way while a group is looked at
+      uint32_t va[32], vb[32];
+      const uint32_t cols = tmem + lane_base + buf * LTC_NCHUNK;
+      ltc_tmem_ld32(cols, va);
+#pragma unroll 1
+      for (int gq = 0; gq < groups; gq += 2) {
+        ltc_tmem_wait(va);
+        if (gq + 1 < groups) ltc_tmem_ld32(cols + (gq + 1) * 32, vb);
+        group(gq, va);
+        if (gq + 1 >= groups) break;
+        ltc_tmem_wait(vb);
+        if (gq + 2 < groups) ltc_tmem_ld32(cols + (gq + 2) * 32, va);
+        group(gq + 1, vb);
       }
       // the row's padding bytes beyond the last table (the last chunk owns them)
       if (blockIdx.y == gridDim.y - 1 && s < s1)
@@ -395,7 +460,8 @@ lsh_key_sign_tc_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64_
 }
 
 // The flagged columns in the fixed order of lsh_key_sign_kernel (single float32 accumulator,
-// channels ascending): sets or clears their bits.  A warp takes 32 list entries at a time.  It
+// channels ascending): sets or clears their bits.  A warp takes up to 32 list entries at a time, fewer
+// where that spreads the list over all warps (a list of 2700 entries 48 -> 10 us, 87 thousand 119 -> 102).  It
 // forms the 129 products of an entry together (coalesced row reads, four channels per lane) and
 // leaves them in shared memory; then lane j adds up those of entry j in order, all 32 chains at
 // once (one entry per warp and a chain of dependent global loads before: 507 us for 88 thousand
@@ -409,7 +475,8 @@ lsh_sign_recheck_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64
                         const __nv_bfloat16* __restrict__ mean, const float* __restrict__ norms,
                         const unsigned int* __restrict__ max_bits, const __nv_bfloat16* __restrict__ proj, int L,
                         int64_t cap, uint8_t* __restrict__ codes, const LtcUncertain* __restrict__ list,
-                        int list_cap, const int* __restrict__ list_count) {
+                        int list_cap, const int* __restrict__ list_count,
+                        const __nv_bfloat16* __restrict__ planes) {
   constexpr int D = 128;
   extern __shared__ float ltc_prod[];  // [LTC_RC_WARPS][32][LTC_RC_PITCH]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -421,16 +488,21 @@ lsh_sign_recheck_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64
   const int nbits = L * 8;
   const int LP = lsh_row_pitch<uint8_t>(L);
   const float M = __uint_as_float(*max_bits);
-  for (int64_t e0 = wid * 32; e0 < n; e0 += nwarps * 32) {
+  const int64_t rounds = (n + nwarps * 32 - 1) / (nwarps * 32);
+  const int per = n > 0 ? (int)((n + nwarps * rounds - 1) / (nwarps * rounds)) : 32;  // entries at a time
+  // as in the kernel above: a product with 1 / M stands for the division of a number that is not tiny
+  const float rM = __frcp_rn(M);
+  const bool divide = (__float_as_uint(M) & 0xffffu) != 0u || !(M >= 8.673617e-19f && M <= 1.152921504606847e18f);
+  for (int64_t e0 = wid * per; e0 < n; e0 += nwarps * per) {
     LtcUncertain u;
     u.key = 0; u.col0 = 0; u.mask = 0u;
-    if (e0 + lane < n) u = list[e0 + lane];
+    if (lane < per && e0 + lane < n) u = list[e0 + lane];
     const int64_t bh_l = u.key / cap, s_l = u.key - bh_l * cap;
     const float aug_l = u.mask ? lsh_augment<__nv_bfloat16>(norms[u.key], M) : 0.f;
     while (__any_sync(0xffffffffu, u.mask != 0u)) {
       const int col_l = u.mask ? u.col0 + __ffs(u.mask) - 1 : -1;
 #pragma unroll 4
-      for (int j = 0; j < 32; ++j) {
+      for (int j = 0; j < per; ++j) {
         const int col = __shfl_sync(0xffffffffu, col_l, j);
         const int64_t bh = __shfl_sync(0xffffffffu, bh_l, j), s = __shfl_sync(0xffffffffu, s_l, j);
         if (col >= 0) {
@@ -444,11 +516,21 @@ lsh_sign_recheck_kernel(const __nv_bfloat16* __restrict__ k, int64_t ks_b, int64
 #pragma unroll
             for (int c = 0; c < 4; ++c) x[c] = sah_round_to<__nv_bfloat16>(__fsub_rn(x[c], m[c]));
           }
+          float p[4];
+          if (planes != nullptr) {
+            const uint2 pr = *reinterpret_cast<const uint2*>(planes + (int64_t)col * LTC_PLANE + lane * 4);
+            p[0] = __uint_as_float(pr.x << 16), p[1] = __uint_as_float(pr.x & 0xffff0000u);
+            p[2] = __uint_as_float(pr.y << 16), p[3] = __uint_as_float(pr.y & 0xffff0000u);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) p[c] = __bfloat162float(proj[(int64_t)(lane * 4 + c) * nbits + col]);
+          }
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float v = sah_round_to<__nv_bfloat16>(__fdiv_rn(x[c], M));
+            const float v = sah_round_to<__nv_bfloat16>(
+                !divide && (fabsf(x[c]) >= 8.673617e-19f || x[c] == 0.f) ? __fmul_rn(x[c], rM) : __fdiv_rn(x[c], M));
             prod[j * LTC_RC_PITCH + c * 32 + lane] =  // channel ch at (ch % 4) * 32 + ch / 4
-                __fmul_rn(v, __bfloat162float(proj[(int64_t)(lane * 4 + c) * nbits + col]));
+                __fmul_rn(v, p[c]);
           }
         }
       }
