@@ -20,7 +20,11 @@
 // the stream of K.  A thread therefore owns two keys where the head dimension is known, which
 // halves the query reads: 32 rows x 65536 keys x 4 sequences in bfloat16 (537 MB, 82 us at the
 // measured copy rate) 123 us with one key per thread, 113.7 us with two,
-// 110.3 us without the division of the row number that a single query does not need.
+// 110.3 us without the division of the row number that a single query does not need; half of what was
+// issued were addresses: 108.6 us with the copies' and the scores' addresses growing by constants (8 rows
+// per KV head, 4 x 32768 keys 102.7 -> 92.4 us; float32, 64 heads x 8000 keys x 2 34.8 -> 30.7 us).  A warp
+// with a ring of its own that copies ahead while it computes was slower at every size (134 to 155 us
+// with eight to four warps per SM: twelve are needed to keep the fma pipe fed).
 #define QK_THREADS 128
 
 // Two partial sums at once: sm_100 issues a pair of fp32 operations per instruction
@@ -90,28 +94,40 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
   unsigned char* k_sm = reinterpret_cast<unsigned char*>(q_sm + R * D);
   const int cpr = row_bytes / 16;
   const int64_t j0 = (int64_t)blockIdx.x * TILE;
+  const int nkeys = (int)(S - j0 < TILE ? S - j0 : TILE);
   {
-    const int nkeys = (int)(S - j0 < TILE ? S - j0 : TILE);
     const int64_t src_stride = ks_s * (int64_t)sizeof(T);
     const unsigned char* src = reinterpret_cast<const unsigned char*>(k + b * ks_b + kvh * ks_h) + j0 * src_stride;
     const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(k_sm);
-    for (int c = threadIdx.x; c < nkeys * cpr; c += QK_THREADS) {
-      const int row = c / cpr, col = c - row * cpr;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst0 + row * row_stride + col * 16),
-                   "l"(src + row * src_stride + col * 16));
+    if (DT != 0 && nkeys == TILE) {  // a thread stays in its column of chunks, its addresses grow by constants
+      constexpr int CPR = (DT ? DT : 8) * (int)sizeof(T) / 16, STEP = QK_THREADS / CPR;
+      src += (threadIdx.x / CPR) * src_stride + (threadIdx.x % CPR) * 16;
+      uint32_t dst = dst0 + (threadIdx.x / CPR) * row_stride + (threadIdx.x % CPR) * 16;
+#pragma unroll 16
+      for (int i = 0; i < TILE / STEP; ++i) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+        src += STEP * src_stride;
+        dst += STEP * row_stride;
+      }
+    } else {
+      for (int c = threadIdx.x; c < nkeys * cpr; c += QK_THREADS) {
+        const int row = c / cpr, col = c - row * cpr;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst0 + row * row_stride + col * 16),
+                     "l"(src + row * src_stride + col * 16));
+      }
     }
     asm volatile("cp.async.commit_group;\n" ::);
   }
   // Stage the group's queries as fp32: row r = g * Sq + qi.
   for (int idx = threadIdx.x; idx < R * D; idx += QK_THREADS) {
     int r = idx / D, d = idx - r * D;
-    int g = r / Sq, qi = r - g * Sq;
+    int g = Sq == 1 ? r : r / Sq, qi = r - g * Sq;
     q_sm[idx] = sah_to_float<T>(q[b * qs_b + (int64_t)(kvh * G + g) * qs_h + qi * qs_q + d]);
   }
   const int chunks = D / 8;
   asm volatile("cp.async.wait_group 0;\n" ::);
   __syncthreads();
-  if (j0 + threadIdx.x >= S) return;  // (the thread's other key lies further on)
+  if ((int)threadIdx.x >= nkeys) return;  // (the thread's other key lies further on)
   const unsigned char* kr = k_sm + threadIdx.x * row_stride;
   for (int r0 = 0; r0 < R; r0 += 4) {
     unsigned long long acc[KEYS][4][4];
@@ -146,21 +162,21 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
     for (int r = 0; r < 4; ++r) {
       if (FULL4 || r0 + r < R) {
         const int rr = r0 + r, g = Sq == 1 ? rr : rr / Sq, qi = rr - g * Sq, h = kvh * G + g;
-        const int64_t row = ((int64_t)b * Hq + h) * Sq + qi;
+        T* out = scores + (((int64_t)b * Hq + h) * Sq + qi) * S + j0;
 #pragma unroll
         for (int u = 0; u < KEYS; ++u) {
-          const int64_t j = j0 + u * QK_THREADS + threadIdx.x;
-          if (j >= S) continue;
+          const int i = u * QK_THREADS + threadIdx.x;
+          if (i >= nkeys) continue;
           const float2 p0 = qk_halves(acc[u][r][0]), p1 = qk_halves(acc[u][r][1]);
           const float2 p2 = qk_halves(acc[u][r][2]), p3 = qk_halves(acc[u][r][3]);
           float s = __fadd_rn(__fadd_rn(__fadd_rn(p0.x, p0.y), __fadd_rn(p1.x, p1.y)),
                               __fadd_rn(__fadd_rn(p2.x, p2.y), __fadd_rn(p3.x, p3.y)));
           s = sah_round_to<T>(s);
           if (bias != nullptr) {
-            float bv = sah_to_float<T>(bias[b * bias_s_b + h * bias_s_h + qi * bias_s_q + j]);
+            float bv = sah_to_float<T>(bias[b * bias_s_b + h * bias_s_h + qi * bias_s_q + j0 + i]);
             s = sah_round_to<T>(__fadd_rn(s, bv));
           }
-          scores[row * S + j] = sah_from_float<T>(s);
+          out[i] = sah_from_float<T>(s);
         }
       }
     }
