@@ -150,6 +150,12 @@ class PackedLSHSignatures:
         return new
 
 
+def _clear_padding(bits: torch.Tensor, n_cols: int) -> None:
+    """The words of a row's stride behind its last key, which the match does not write."""
+    if bits.shape[1] > (n_cols + 31) // 32:
+        bits[:, (n_cols + 31) // 32:].zero_()
+
+
 class DeferredLSHWeights:
     """What `sah_attn_plan_lsh` + `sah_masked_attention_lsh` need of one MagicPig call, and the
     way back to an ordinary bitmap + weight array (`materialise`)."""
@@ -172,6 +178,7 @@ class DeferredLSHWeights:
         the probability rounded as the reference rounds it (magic_pig.py:374-403, :581-593)."""
         B, Hq, Sq, S = self.shape
         rows = B * Hq * Sq
+        _clear_padding(self.match_bits, S)  # the plan and the attention kernels go by the key count
         this = NativeBits(self.match_bits, rows, S)
         self.masker._probabilities(this, self.keys, self.qunit, self.sig, self.mean, self.table,
                                    self.shape, self.G, self.previous_mask.dtype)
@@ -384,8 +391,6 @@ class MagicPig(SamplingMasker):
             lib.sah_lsh_match(sig.codes.data_ptr(), sig.capacity, qcodes.data_ptr(), B, Hq, Sq, G,
                               self.lsh_l, self.lsh_k, S, W, None, bits.data_ptr(), st),
             "sah_lsh_match")
-        if W * 32 > (S + 31) // 32 * 32:
-            bits[:, (S + 31) // 32:].zero_()  # padding words of the row stride
         table = _native_ops.lsh_prob_table(dev, self.lsh_k, self.lsh_l) if dtype == torch.bfloat16 else None
         shape = (B, Hq, Sq, S)
         if fused:
@@ -395,6 +400,7 @@ class MagicPig(SamplingMasker):
                                          _native_ops.lsh_weight_table(dev, self.lsh_k, self.lsh_l))
             return Mask._from_native(shape, previous_mask.dtype,
                                      NativeBits(None, rows, S, deferred=payload))
+        _clear_padding(bits, S)
         nb = NativeBits(bits, rows, S)
         self._probabilities(nb, k, qunit, sig, mean, table, shape, G, dtype)
         this_mask = Mask._from_native(shape, previous_mask.dtype, nb)
