@@ -26,6 +26,7 @@
 // with a ring of its own that copies ahead while it computes was slower at every size (134 to 155 us
 // with eight to four warps per SM: twelve are needed to keep the fma pipe fed).
 #define QK_THREADS 128
+#define QK_ROWS 16  // query rows of a CTA, at most
 
 // Two partial sums at once: sm_100 issues a pair of fp32 operations per instruction
 // (fma.rn.f32x2), each half rounding exactly as the scalar fma; used for bf16 inputs, whose
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(QK_THREADS, KEYS == 2 ? 3 : 5)
 qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b, int64_t qs_h,
                  int64_t qs_q, int64_t ks_b, int64_t ks_h, int64_t ks_s, int Hq, int Hkv, int Sq,
                  int64_t S, int D_rt, const T* __restrict__ bias, int64_t bias_s_b,
-                 int64_t bias_s_h, int64_t bias_s_q, T* __restrict__ scores) {
+                 int64_t bias_s_h, int64_t bias_s_q, int row_blocks, int RB, T* __restrict__ scores) {
   sah_pdl_entry();
   constexpr int TILE = QK_THREADS * KEYS;
   extern __shared__ __align__(16) float q_sm[];  // [R][D] queries, then the K tile
@@ -91,9 +92,11 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
   // bytes so that the per-thread row reads do not collide.
   const int row_bytes = D * (int)sizeof(T);
   const int row_stride = row_bytes + 16;
-  unsigned char* k_sm = reinterpret_cast<unsigned char*>(q_sm + R * D);
+  const int64_t tile = row_blocks == 1 ? blockIdx.x : blockIdx.x / row_blocks;
+  const int r_lo = ((int)blockIdx.x - (int)tile * row_blocks) * RB, r_hi = r_lo + RB < R ? r_lo + RB : R;  // this CTA's rows
+  unsigned char* k_sm = reinterpret_cast<unsigned char*>(q_sm + RB * D);
   const int cpr = row_bytes / 16;
-  const int64_t j0 = (int64_t)blockIdx.x * TILE;
+  const int64_t j0 = tile * TILE;
   const int nkeys = (int)(S - j0 < TILE ? S - j0 : TILE);
   {
     const int64_t src_stride = ks_s * (int64_t)sizeof(T);
@@ -119,8 +122,9 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
     asm volatile("cp.async.commit_group;\n" ::);
   }
   // Stage the group's queries as fp32: row r = g * Sq + qi.
-  for (int idx = threadIdx.x; idx < R * D; idx += QK_THREADS) {
+  for (int idx = threadIdx.x; idx < (r_hi - r_lo) * D; idx += QK_THREADS) {
     int r = idx / D, d = idx - r * D;
+    r += r_lo;
     int g = Sq == 1 ? r : r / Sq, qi = r - g * Sq;
     q_sm[idx] = sah_to_float<T>(q[b * qs_b + (int64_t)(kvh * G + g) * qs_h + qi * qs_q + d]);
   }
@@ -129,7 +133,7 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
   __syncthreads();
   if ((int)threadIdx.x >= nkeys) return;  // (the thread's other key lies further on)
   const unsigned char* kr = k_sm + threadIdx.x * row_stride;
-  for (int r0 = 0; r0 < R; r0 += 4) {
+  for (int r0 = r_lo; r0 < r_hi; r0 += 4) {
     unsigned long long acc[KEYS][4][4];
 #pragma unroll
     for (int u = 0; u < KEYS; ++u)
@@ -145,9 +149,9 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
         qk_load_pairs<T>(reinterpret_cast<const T*>(kr + u * QK_THREADS * row_stride) + t * 8, kp[u]);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        if (FULL4 || r0 + r < R) {
-          const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(q_sm + (r0 + r) * D + t * 8);
-          const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(q_sm + (r0 + r) * D + t * 8 + 4);
+        if (FULL4 || r0 + r < r_hi) {
+          const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(q_sm + (r0 - r_lo + r) * D + t * 8);
+          const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(q_sm + (r0 - r_lo + r) * D + t * 8 + 4);
 #pragma unroll
           for (int u = 0; u < KEYS; ++u) {
             qk_mac2<T>(acc[u][r][0], qa.x, kp[u][0]);
@@ -160,7 +164,7 @@ qk_scores_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t qs_b,
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      if (FULL4 || r0 + r < R) {
+      if (FULL4 || r0 + r < r_hi) {
         const int rr = r0 + r, g = Sq == 1 ? rr : rr / Sq, qi = rr - g * Sq, h = kvh * G + g;
         T* out = scores + (((int64_t)b * Hq + h) * Sq + qi) * S + j0;
 #pragma unroll
@@ -208,7 +212,14 @@ extern "C" int sah_qk_scores(const void* q, const void* k, int dtype, int64_t qs
   const bool two = dtype == SAH_BF16 && (D == 128 || D == 64) && R % 4 == 0 && pairs >= 4 * 148 &&
                    smem + (size_t)QK_THREADS * (D * elt + 16) <= 75 * 1024;
   if (two) smem += (size_t)QK_THREADS * (D * elt + 16);
-  const dim3 grid((unsigned)sah_ceil_div(S, (int64_t)QK_THREADS * (two ? 2 : 1)), (unsigned)Hkv, (unsigned)B);
+  // Rows of a question: a CTA takes QK_ROWS of them, so that five CTAs share an SM where the queries
+  // of all would leave room for one or two, and the waves are finer (96 rows per KV head, 8 x 8191 bfloat16 keys
+  // 108.6 us all at once, 90 by 48, 84 by 32, 79.9 by 16; 58 rows x 8576 keys 106 -> 65.5 us; float32, 36
+  // rows x 4096 keys 34.8 -> 32.8 us).
+  const int row_blocks = two ? 1 : (R + QK_ROWS - 1) / QK_ROWS;
+  const int RB = row_blocks == 1 ? R : ((R + row_blocks - 1) / row_blocks + 3) / 4 * 4;
+  smem -= (size_t)(R - RB) * D * sizeof(float);
+  const dim3 grid((unsigned)(sah_ceil_div(S, (int64_t)QK_THREADS * (two ? 2 : 1)) * row_blocks), (unsigned)Hkv, (unsigned)B);
   cudaStream_t st = (cudaStream_t)stream;
   sah_prof_begin(SAH_PROF_QK_SCORES, (cudaStream_t)stream);
 #define QK_LAUNCH(T, DT, F4, KEYS)                                                                  \
@@ -220,7 +231,7 @@ extern "C" int sah_qk_scores(const void* q, const void* k, int dtype, int64_t qs
     }                                                                                               \
     sah_launch_chain(qk_scores_kernel<T, DT, F4, KEYS>, grid, QK_THREADS, smem, st, \
         (const T*)q, (const T*)k, qs_b, qs_h, qs_q, ks_b, ks_h, ks_s, Hq, Hkv, Sq, S, D,            \
-        (const T*)bias, bias_s_b, bias_s_h, bias_s_q, (T*)scores);                                  \
+        (const T*)bias, bias_s_b, bias_s_h, bias_s_q, row_blocks, RB, (T*)scores);                  \
   } while (0)
   const bool full4 = (R % 4) == 0;
   SAH_DISPATCH_DTYPE(dtype, T, {

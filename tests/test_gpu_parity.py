@@ -634,3 +634,35 @@ def test_band_masks_without_a_bitmap(dtype, S, Sq, stack, monkeypatch):
         got = Mask._from_native((2, 4, Sq, S), dt, NativeBits(words, bits.rows, S)).get_dense_mask()
         assert torch.equal(got, fixed_dense)
         assert bool((words[:, (S + 31) // 32:] == 0).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,Hq,Hkv,Sq,S,D,bias", [
+    ("bf16", 8, 2, 5, 700, 128, True), ("bf16", 4, 1, 17, 129, 128, False), ("f32", 3, 1, 11, 257, 64, True),
+    ("bf16", 2, 2, 33, 40, 64, True), ("f32", 8, 1, 6, 128, 80, False), ("bf16", 8, 1, 2, 300, 128, True)])
+def test_scores_of_many_rows_equal_those_of_one_position(dtype, Hq, Hkv, Sq, S, D, bias):
+    """Rows per KV head that are cut into blocks (20, 68, 33, 33, 48 and 16 of them): the scores of every
+    position are those of a call for that position alone, bit for bit."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = torch.device("cuda:0")
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    gen = torch.Generator(device=dev).manual_seed(S + Sq)
+    q = torch.randn((2, Hq, Sq, D), generator=gen, device=dev).to(dt)
+    k = torch.randn((2, Hkv, S, D), generator=gen, device=dev).to(dt)
+    am = torch.randn((2, 1, Sq, S), generator=gen, device=dev).to(dt) if bias else None
+
+    def scores(lo, hi):
+        out = torch.full((2, Hq, hi - lo, S), float("nan"), dtype=dt, device=dev)
+        qs = q[:, :, lo:hi]
+        b = (None, 0, 0, 0) if am is None else (am[:, :, lo:hi].data_ptr(), am.stride(0), 0, am.stride(2))
+        _native.check(lib.sah_qk_scores(qs.data_ptr(), k.data_ptr(), _native.dtype_code(dt), *qs.stride()[:3],
+                                        *k.stride()[:3], 2, Hq, Hkv, hi - lo, S, D, *b, out.data_ptr(),
+                                        _native.stream_of(dev)), "sah_qk_scores")
+        return out
+
+    together = scores(0, Sq)
+    for i in range(Sq):
+        assert torch.equal(together[:, :, i:i + 1], scores(i, i + 1))
