@@ -69,10 +69,15 @@ struct AumCfg {
   // barriers: k_full k_free v_full v_free [3] each, s_full[2] s_free[2] p_full[2] p_free[2] max[2]
   static constexpr int N_BARS = 4 * AUM_STAGES + 10;
   static constexpr int MISC_OFF = BAR_OFF + ((N_BARS * 8 + 15) & ~15);
-  // misc: tmem slot, abort word, last flag, pad; then wmax [2][4][16], lred [2][4][16], group
-  // maxima [2][16], qmu [16], bias offsets [16] (int64)
+  // misc: tmem slot, abort word, last flag, pad; then wmax [WMAX_SLOTS][2][4][16], lred [2][4][16],
+  // group maxima [2][16], qmu [16], bias offsets [16] (int64)
   static constexpr int WMAX_OFF = MISC_OFF + 16;
-  static constexpr int LRED_OFF = WMAX_OFF + 2 * 4 * 16 * 4;
+  // Maxima of a group's tile j lie in slot j & 1: a warp that has read those of tile j may find the scores
+  // of tile j + 1 complete (every warp gave s_free(j) before it exchanged maxima) and leave its own while another
+  // still reads tile j's.  It gets no further: scores of tile j + 2 need the other warp's s_free(j + 1),
+  // which comes after that warp's reads of tile j.  So two slots are enough, and one is not.
+  static constexpr int WMAX_SLOTS = 2, WMAX_SLOT = 2 * 4 * 16;
+  static constexpr int LRED_OFF = WMAX_OFF + WMAX_SLOTS * WMAX_SLOT * 4;
   static constexpr int GMAX_OFF = LRED_OFF + 2 * 4 * 16 * 4;
   static constexpr int QMU_OFF = GMAX_OFF + 2 * 16 * 4;
   static constexpr int BOFF_OFF = QMU_OFF + 16 * 4;
@@ -429,10 +434,11 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
       }
       // tile maximum per row: warp reduction, then the group's four warps exchange through
       // shared memory
+      float* wmax_tile = wmax_sm + (j & (C::WMAX_SLOTS - 1)) * C::WMAX_SLOT + gg * 64;
 #pragma unroll
       for (int r = 0; r < RMAX; ++r) {
         const int mx = __reduce_max_sync(0xffffffffu, aum_ordered(sv[r]));
-        if (lane == 0) wmax_sm[(gg * 4 + wg) * 16 + r] = aum_unordered(mx);
+        if (lane == 0) wmax_tile[wg * 16 + r] = aum_unordered(mx);
       }
       __syncwarp();
       if (lane == 0) aum_arrive(max_bar + gg * 8);
@@ -459,7 +465,7 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
       bool rescale = false, moved = false;
 #pragma unroll
       for (int r = 0; r < RMAX; ++r) {
-        const float* wm = wmax_sm + gg * 64 + r;
+        const float* wm = wmax_tile + r;
         const float tm = fmaxf(fmaxf(wm[0], wm[16]), fmaxf(wm[32], wm[48]));
         alpha[r] = 1.f;
         if (tm > m_used[r] + AUM_RESCALE_T) {  // also the first finite maximum (-inf + T = -inf)

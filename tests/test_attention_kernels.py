@@ -131,6 +131,35 @@ def test_default_kernel_for_few_groups_is_as_exact_as_the_mma_kernel():
     assert error("auto") <= 1.02 * error("mma")
 
 
+@pytest.mark.parametrize("B,Hq,Hkv", [(64, 4, 1), (32, 8, 2), (64, 16, 1)])
+def test_maxima_that_grow_from_tile_to_tile(B, Hq, Hkv):
+    """Logits that grow by more than the rescale threshold with every tile of 128 keys, the largest in another
+    quarter of each tile, thirty tiles per CTA: every warp of the tcgen05 kernel has to go by the same maximum.  Against float64 (the
+    last tiles carry all the weight; bfloat16 rounds P and the output, 2^-9 each), and the same bits every time."""
+    S, D, scaling = 60 * 128, 128, 128 ** -0.5
+    gen = torch.Generator(device=DEV).manual_seed(Hq)
+    randn = lambda *s: torch.randn(s, generator=gen, device=DEV)  # noqa: E731
+    axis = torch.nn.functional.normalize(randn(B, Hkv, 1, D), dim=-1)
+    tile, quarter = torch.arange(S, device=DEV) // 128, torch.arange(S, device=DEV) % 128 // 32
+    height = tile * 12.0 - 6.0 * ((quarter - tile) % 4)
+    q = (D ** 0.5 * axis.repeat_interleave(Hq // Hkv, 1) + 0.1 * randn(B, Hq, 1, D)).bfloat16()
+    k = (height.view(1, 1, S, 1) * axis + 0.1 * randn(B, Hkv, S, D)).bfloat16()
+    v = randn(B, Hkv, S, D).bfloat16()
+    dense = (torch.rand((B, Hq, 1, S), generator=gen, device=DEV) < 0.9).bfloat16()
+    logits = torch.matmul(q.double(), k.repeat_interleave(Hq // Hkv, 1).double().transpose(2, 3)) * scaling
+    p = torch.softmax(logits.masked_fill(dense == 0, -float("inf")), dim=-1)
+    exact = torch.matmul(p, v.repeat_interleave(Hq // Hkv, 1).double()).transpose(1, 2)
+    prev = select_attention_kernel("umma")
+    try:
+        m = Mask.create_mask_from_dense_mask(tuple(dense.shape), dense, torch.bfloat16)
+        outs = [native_masked_attention(q, k, v, None, None, scaling, m) for _ in range(30)]
+    finally:
+        select_attention_kernel(prev)
+    assert attention_wait_errors() == 0
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    assert float((outs[0].double() - exact).norm() / exact.norm()) < 4 * 2.0 ** -9
+
+
 def test_bounded_wait_runs_out_and_reports_without_hanging():
     """Every mbarrier wait of the tcgen05 kernels is bounded.  `sah_wait_selftest` waits 2 ms for an
     arrival that never comes: the error word is set, the measured wait is about the limit, the
