@@ -341,15 +341,19 @@ masked_attention_stream_kernel(AstArgs a) {
     load_tile(gg);
     unsigned char* prow = sm + C::P_OFF + gg * 16384 + l * 128;
     float* tops = reinterpret_cast<float*>(sm + C::TOP_OFF) + gg * 256 + l;
+    // A warp that leaves the loop lets the other half's warp go at the exchange of maxima that it would have
+    // come to next.  That warp then gets to a bounded wait that the leaving one did not arrive for, and leaves
+    // there: for the next tile's scores if the wait for tile j's ran out (no s_free for j), for tile j's product if
+    // the wait for the one before did (no p_full for j; the scores of j + 1 may be there already).  Should both
+    // leave, the arrivals complete an exchange that nobody is at, or stay behind.
+    auto let_go = [&] { asm volatile("bar.arrive %0, 64;\n" ::"r"(1 + gg * 4 + wq) : "memory"); };
     bool ok = true;
     int j = 0;
     for (int t = gg; t < n_tiles; t += 2, ++j) {
       ok = aum_wait_warp(full + (t % NST) * 8, (uint32_t)((t / NST) & 1), abort_sm, a.errflag) &&  // the key constants
            aum_wait_warp(s_full + gg * 8, (uint32_t)(j & 1), abort_sm, a.errflag);
       if (!ok) {
-        // The other half's warp may have come past this wait: it is let go at the exchange below, and gets no
-        // further than its next wait, since the scores of a further tile need this warp's arrivals.
-        asm volatile("bar.arrive %0, 64;\n" ::"r"(1 + gg * 4 + wq) : "memory");
+        let_go();
         break;
       }
       aum_fence_after();
@@ -412,7 +416,10 @@ masked_attention_stream_kernel(AstArgs a) {
       l_run = l_run * alpha + sum;
       if (j >= 1) {
         ok = aum_wait_warp(p_free + gg * 8, (uint32_t)((j - 1) & 1), abort_sm, a.errflag);
-        if (!ok) break;
+        if (!ok) {
+          let_go();
+          break;
+        }
         if (__any_sync(0xffffffffu, grew)) {  // this half's dims of the accumulator
           aum_fence_after();
 #pragma unroll
