@@ -1310,9 +1310,9 @@ extern "C" int sah_masked_attention_stream(const void* q, const void* k, const v
   else sah_launch_chain(masked_attention_stream_kernel<64>, grid, AST_THREADS, AstCfg::SMEM, st, a);
   g_last_attn_kernel = "masked_attention_stream_kernel";
   SAH_LAUNCH_CHECK("masked_attention_stream");
-  sah_launch_chain(attn_merge_parts_kernel<__nv_bfloat16>, (unsigned)((int64_t)B * Hq * Sq), D, 0, st,
-                   (const float*)parts, n_parts, (int64_t)B * Hq * Sq, Hq, Sq, D, sinks, (__nv_bfloat16*)out);
-  SAH_LAUNCH_CHECK("attn_merge_parts");
+  sah_launch_chain(attn_stream_merge_kernel, (unsigned)((int64_t)B * Hq * Sq), D, 0, st, a, n_parts,
+                   (int64_t)B * Hq * Sq, sinks, (__nv_bfloat16*)out);
+  SAH_LAUNCH_CHECK("attn_stream_merge");
   sah_prof_end(SAH_PROF_ATTENTION, st);
   return SAH_OK;
 }

@@ -20,7 +20,7 @@
 //   it grows, so that a row's largest weight enters P as itself.  Everything else -- weights,
 //   roundings, who is a member -- is as in the gather kernels.
 //
-// Partials of the CTAs go to `parts` [nsplit][rows][D + 2]; attn_merge_parts_kernel adds them up.
+// Partials of the CTAs go to `parts` [nsplit][rows][D + 2]; attn_stream_merge_kernel adds them up.
 // Waits are bounded as in the gather kernel: one that runs out sets the abort word and the caller's
 // error word, and every role leaves its loop.
 //
@@ -503,6 +503,89 @@ masked_attention_stream_kernel(AstArgs a) {
     for (int c = 0; c < 256; c += RP) o += ob[(c + r) * C::OB_LD + d] * fac[c + r];
     a.parts[(split * all_rows + row_of(r)) * (D + 2) + d] = o;
   }
+}
+
+// Adds up the partials of a row, a thread per dim, and writes its output.
+//
+// The product takes every key's V row, with a probability of 0 where the row does not have the key, and
+// 0 times an infinity or a NaN is NaN.  A row whose sum is not finite is therefore added up anew from its own
+// keys alone, which is what the gather kernels read: M and L stand, they come from the scores of those keys.
+// Plain loads and float32 sums, about 1 ms for 64 rows of 8 KV heads x 65500 keys: nothing for speed, and nothing
+// that finite values pay for but a vote.
+__global__ void __launch_bounds__(128)
+attn_stream_merge_kernel(AstArgs a, int n_parts, int64_t rows, const float* __restrict__ sinks, __nv_bfloat16* __restrict__ out) {
+  sah_pdl_entry_early();
+  constexpr int D = 128;
+  __shared__ float part[4][D];
+  const int64_t row = blockIdx.x;
+  const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
+  const int qi = (int)(row % a.Sq), h = (int)(row / a.Sq % a.Hq);
+  const int64_t b = row / a.Sq / a.Hq, pstride = rows * (D + 2);
+  const float* pr = a.parts + row * (D + 2);
+  float M = -INFINITY, L = 0.f, o = 0.f;
+  for (int p = 0; p < n_parts; ++p) M = fmaxf(M, pr[p * pstride + D]);
+  for (int p = 0; p < n_parts; ++p) {
+    const float mp = pr[p * pstride + D];
+    if (mp != -INFINITY) {
+      const float f = expf(mp - M);
+      L += pr[p * pstride + D + 1] * f;
+      o += pr[p * pstride + d] * f;
+    }
+  }
+  if (__syncthreads_or(!(fabsf(o) < INFINITY))) {
+    const int kvh = h / a.G;
+    const int64_t bk = b * a.Hkv + kvh;
+    float q[4], qh[4], num[4] = {0.f, 0.f, 0.f, 0.f};
+    auto load4 = [&](const __nv_bfloat16* p, float* x) {
+      const uint2 v = *reinterpret_cast<const uint2*>(p + lane * 4);
+      x[0] = __uint_as_float(v.x << 16), x[1] = __uint_as_float(v.x & 0xffff0000u);
+      x[2] = __uint_as_float(v.y << 16), x[3] = __uint_as_float(v.y & 0xffff0000u);
+    };
+    load4(a.q + b * a.qs_b + (int64_t)h * a.qs_h + (int64_t)qi * a.qs_q, q);
+    load4(a.qhat + row * D, qh);
+    const __nv_bfloat16 *kb = a.k + b * a.ks_b + kvh * a.ks_h, *vb = a.v + b * a.vs_b + kvh * a.vs_h;
+    const __nv_bfloat16* brow = a.bias ? a.bias + b * a.bias_s_b + h * a.bias_s_h + qi * a.bias_s_q : nullptr;
+    const float mu = a.qmu[row], max_norm = __uint_as_float(*a.max_bits);
+    for (int64_t w = warp; w * 32 < a.S; w += 4) {
+      const uint32_t units = a.unit ? a.unit[row * a.W + w] : 0u;
+      uint32_t on = a.match[row * a.W + w] | units;
+      if (a.S - w * 32 < 32) on &= (1u << (a.S - w * 32)) - 1u;
+      for (; on; on &= on - 1) {
+        const int bit = __ffs(on) - 1;
+        const int64_t j = w * 32 + bit;
+        float k[4], v[4];
+        load4(kb + j * a.ks_s, k);
+        load4(vb + j * a.vs_s, v);
+        float s = q[0] * k[0] + q[1] * k[1] + q[2] * k[2] + q[3] * k[3];
+        float c = qh[0] * k[0] + qh[1] * k[1] + qh[2] * k[2] + qh[3] * k[3];
+#pragma unroll
+        for (int of = 16; of > 0; of >>= 1) {
+          s += __shfl_xor_sync(0xffffffffu, s, of);
+          c += __shfl_xor_sync(0xffffffffu, c, of);
+        }
+        const float weight = (units >> bit) & 1u ? 1.f
+                             : atm_lsh_weight(c, mu, __frcp_rn(__fmul_rn(max_norm, a.dens[bk * a.dens_cap + j])), a.wtable);
+        if (weight == 0.f) continue;
+        float x = s * a.scaling;
+        if (brow) x += __bfloat162float(brow[j]);
+        const float p = __expf(x - M) * weight;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) num[i] += p * v[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[warp][lane * 4 + i] = num[i];
+    __syncthreads();
+    o = part[0][d] + part[1][d] + part[2][d] + part[3][d];
+  }
+  float Mx = M, sink_term = 0.f;
+  if (sinks != nullptr) {
+    const float sk = sinks[h];
+    Mx = fmaxf(M, sk);
+    sink_term = expf(sk - Mx);
+  }
+  const float resc = (M == -INFINITY) ? 0.f : expf(M - Mx);
+  out[((b * a.Sq + qi) * a.Hq + h) * D + d] = __float2bfloat16_rn(o * resc / (L * resc + sink_term));
 }
 
 // Rows of a block and CTAs per (KV head, block): one CTA per SM, at least four tiles each.

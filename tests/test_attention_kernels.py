@@ -295,3 +295,47 @@ def test_rows_of_several_positions_streamed(B, Hq, Hkv, Sq, S, bias, unit, sinks
     err = lambda a: (((a.double() - want) * live).nan_to_num().norm() / (want * live).nan_to_num().norm()).item()  # noqa: E731
     assert err(out) < 6.8e-3 and err(gathered) < 6.8e-3
     assert torch.equal(torch.isnan(out), torch.isnan(gathered))
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_streamed_rows_go_by_their_own_keys(bad):
+    """An infinity or a NaN in V reaches the rows that select its key, in its dim, and no others, although
+    the streaming kernel reads every key for all rows: as with the kernels that gather a row's keys."""
+    from sparse_attention_hub.sparse_attention.research_attention.maskers import sampling
+    from sparse_attention_hub.sparse_attention.utils import mask_attention_utils as mau
+
+    B, Hq, Hkv, Sq, S, D, scaling = 2, 8, 2, 5, 1500, 128, 128 ** -0.5
+    gen = torch.Generator(device=DEV).manual_seed(11)
+    q, k, v = (torch.randn(s, generator=gen, device=DEV).bfloat16() for s in
+               ((B, Hq, Sq, D), (B, Hkv, S, D), (B, Hkv, S, D)))
+    am = torch.randn((B, 1, Sq, S), generator=gen, device=DEV).bfloat16()
+    masker = sampling.MagicPig(sampling.MagicPigConfig(lsh_l=75, lsh_k=8, center=True))
+    meta = {}
+
+    def mask():
+        return masker.add_mask(keys=k, queries=q, values=v, attention_mask=am, scaling=scaling, dropout=0.0,
+                               sparse_meta_data=meta, layer_idx=0,
+                               previous_mask=Mask.create_empty_mask((B, Hq, Sq, S), torch.bfloat16, torch.device(DEV)))
+
+    on = mask().get_dense_mask() != 0
+    clean = native_masked_attention(q, k, v, am, None, scaling, mask())
+    assert mau.last_attention_kernel() == "masked_attention_stream_kernel"
+    per_head = on.view(B, Hkv, Hq // Hkv * Sq, S).float().mean(2)  # share of a KV head's rows that have a key
+    hit = torch.zeros((B, Hq, Sq, D), dtype=torch.bool, device=DEV)
+    for b in range(B):
+        for h in range(Hkv):
+            few = torch.where(per_head[b, h] > 0, per_head[b, h], 2.0).argmin()
+            for dim, key in ((3, per_head[b, h].argmin()), (70, few), (127, per_head[b, h].argmax())):
+                v[b, h, key, dim] = bad
+                rows = on[b, h * Hq // Hkv:(h + 1) * Hq // Hkv, :, key]
+                hit[b, h * Hq // Hkv:(h + 1) * Hq // Hkv, :, dim] |= rows
+    assert float(per_head.amin()) == 0.0 and hit.any() and not hit[..., 3].all() and not hit[..., 70].all()
+    out = native_masked_attention(q, k, v, am, None, scaling, mask())
+    assert mau.last_attention_kernel() == "masked_attention_stream_kernel"
+    assert attention_wait_errors() == 0
+    hit = hit.transpose(1, 2)
+    assert torch.equal(~torch.isfinite(out), hit)
+    assert bool((torch.isnan(out) if bad != bad else out == bad)[hit].all())
+    # the same rows from finite values; rounding P and the output is 1.7e-3 of the norm
+    same, want = out.double()[~hit], clean.double()[~hit]
+    assert float((same - want).norm() / want.norm()) < 6.8e-3
