@@ -531,7 +531,12 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
         aum_tmem_ld16(tmem_o + lane_base, orow);
         if constexpr (RMAX == 4) {
 #pragma unroll
-          for (int r = 0; r < RMAX; ++r) orow[r] = __float_as_uint(__uint_as_float(orow[r]) + __uint_as_float(orow[8 + r]));
+          for (int r = 0; r < RMAX; ++r) {
+            // the remainders' share, unless a V is infinite: 0 or a negative remainder times it is NaN where
+            // the probability times it is what the sum should be
+            const float rest = __uint_as_float(orow[8 + r]);
+            if (fabsf(rest) < INFINITY) orow[r] = __float_as_uint(__uint_as_float(orow[r]) + rest);
+          }
         }
       }
     }

@@ -160,6 +160,26 @@ def test_maxima_that_grow_from_tile_to_tile(B, Hq, Hkv):
     assert float((outs[0].double() - exact).norm() / exact.norm()) < 4 * 2.0 ** -9
 
 
+@pytest.mark.parametrize("Hq,Hkv,S", [(8, 2, 900), (2, 2, 5000), (16, 2, 900)])
+def test_infinite_values_stay_infinite(kernel, Hq, Hkv, S):
+    """Every row selects the keys whose V is infinite in one dim each: that dim of the output is that infinity (NaN
+    where both signs meet), the others are those of finite values."""
+    gen = torch.Generator(device=DEV).manual_seed(S)
+    q, k, v = (torch.randn((1, h, n, 128), generator=gen, device=DEV).bfloat16() for h, n in ((Hq, 1), (Hkv, S), (Hkv, S)))
+    dense = (torch.rand((1, Hq, 1, S), generator=gen, device=DEV) < 0.4).bfloat16()
+    dense[..., [0, 17, 333, S - 1]] = 1.0
+    m = Mask.create_mask_from_dense_mask(tuple(dense.shape), dense, torch.bfloat16)
+    clean = native_masked_attention(q, k, v, None, None, 0.05, m)
+    inf = float("inf")
+    for key, dim, value in ((0, 5, inf), (17, 64, -inf), (333, 127, inf), (S - 1, 90, inf), (0, 90, -inf)):
+        v[:, :, key, dim] = value
+    out = native_masked_attention(q, k, v, None, None, 0.05, m)
+    want = clean.clone()
+    want[..., 5] = want[..., 127] = inf
+    want[..., 64], want[..., 90] = -inf, float("nan")
+    assert torch.equal(out.nan_to_num(nan=7.0), want.nan_to_num(nan=7.0))
+
+
 def test_bounded_wait_runs_out_and_reports_without_hanging():
     """Every mbarrier wait of the tcgen05 kernels is bounded.  `sah_wait_selftest` waits 2 ms for an
     arrival that never comes: the error word is set, the measured wait is about the limit, the
