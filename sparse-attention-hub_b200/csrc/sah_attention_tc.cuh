@@ -676,11 +676,14 @@ masked_attention_mma_kernel(AttnArgs a, const __grid_constant__ AtmMaps maps, in
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < ATM_WARPS; ++w) M = fmaxf(M, ml_sm[w][r].x);
-    const float sc = (m_run[rs] == -INFINITY) ? 0.f : __expf(m_run[rs] - M);
+    // A warp without an entry of the row adds nothing: not 0 times what its tiles' values, with probabilities of
+    // 0, have left in the accumulator (an infinity or a NaN there belongs to other rows).
+    const bool has = m_run[rs] != -INFINITY;
+    const float sc = has ? __expf(m_run[rs] - M) : 0.f;
 #pragma unroll
     for (int nt = 0; nt < C::NT; ++nt)
       *reinterpret_cast<float2*>(red_o + r * RS + nt * 8 + 2 * (lane & 3)) =
-          make_float2(o[nt][2 * rs] * sc, o[nt][2 * rs + 1] * sc);
+          make_float2(has ? o[nt][2 * rs] * sc : 0.f, has ? o[nt][2 * rs + 1] * sc : 0.f);
   }
   __syncthreads();
   float* pout = a.partial + ((int64_t)g * a.nsplit + split) * a.R * (D + 2);

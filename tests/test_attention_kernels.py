@@ -180,6 +180,25 @@ def test_infinite_values_stay_infinite(kernel, Hq, Hkv, S):
     assert torch.equal(out.nan_to_num(nan=7.0), want.nan_to_num(nan=7.0))
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_values_of_tiles_without_an_entry_stay_out(D):
+    """Four heads share a list of four tiles of sixteen keys, a warp of the mma.sync kernel each; a head selects the keys
+    of one tile.  A NaN in the first tile's V is the first head's alone."""
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v = (torch.randn((1, h, n, D), generator=gen, device=DEV).bfloat16() for h, n in ((4, 1), (1, 64), (1, 64)))
+    dense = torch.eye(4, device=DEV).repeat_interleave(16, 1).view(1, 4, 1, 64).bfloat16()
+    m = Mask.create_mask_from_dense_mask((1, 4, 1, 64), dense, torch.bfloat16)
+    prev = select_attention_kernel("mma")
+    try:
+        clean = native_masked_attention(q, k, v, None, None, D ** -0.5, m)
+        v[:, :, 3, 7], v[:, :, 9, 40] = float("nan"), float("inf")
+        out = native_masked_attention(q, k, v, None, None, D ** -0.5, m)
+    finally:
+        select_attention_kernel(prev)
+    clean[0, 0, 0, 7], clean[0, 0, 0, 40] = float("nan"), float("inf")
+    assert torch.equal(out.nan_to_num(nan=7.0), clean.nan_to_num(nan=7.0))
+
+
 def test_bounded_wait_runs_out_and_reports_without_hanging():
     """Every mbarrier wait of the tcgen05 kernels is bounded.  `sah_wait_selftest` waits 2 ms for an
     arrival that never comes: the error word is set, the measured wait is about the limit, the
