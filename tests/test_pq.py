@@ -277,6 +277,41 @@ def test_gpu_assignment_tile_edges_and_layouts(n_sub, n_cent, n_keys):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n_sub,n_cent", [(16, 256), (4, 128), (6, 64), (3, 32)])
+def test_gpu_assignment_with_many_near_ties(n_sub, n_cent):
+    """Stretches of a few distinct keys (centroids that are their copies, or nearly), of zeros and of keys far from
+    0 with little spread, between stretches of ordinary ones, all tiles in two CTAs.  The codes of `sah_pq_assign`."""
+    import torch
+    from sparse_attention_hub import _native
+
+    lib = _native.load()
+    dev = "cuda:0"
+    B, Hkv, off, n_keys = 1, 2, 3, 4300
+    gen = torch.Generator(device=dev).manual_seed(n_cent)
+    keys = torch.randn((B, Hkv, n_keys + off, n_sub * 8), generator=gen, device=dev).to(torch.bfloat16)
+    keys[:, :, 600:1900] = keys[:, :, torch.randint(0, 9, (1300,), generator=gen, device=dev)]
+    keys[:, :, 2500:3600] = keys[:, :, 2500:3600] * 0.5 + 64.0
+    keys[:, :, 3700:3900] = 0.0
+    groups = B * Hkv * n_sub
+    sub = keys.view(B * Hkv, n_keys + off, n_sub, 8).transpose(1, 2).reshape(groups, n_keys + off, 8).float()
+    pick = torch.randint(0, n_keys + off, (groups, n_cent), generator=gen, device=dev)
+    pick[:, ::3] = torch.randint(0, 9, (groups, (n_cent + 2) // 3), generator=gen, device=dev)
+    cent = torch.gather(sub, 1, pick[..., None].expand(-1, -1, 8)).contiguous()
+    cent[:, ::9] *= 1.0 + 2.0 ** -23
+    cap, st = n_keys + 2, _native.stream_of(torch.device(dev))
+    want = torch.full((B, Hkv, cap, n_sub), 255, dtype=torch.uint8, device=dev)
+    got = want.clone()
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    strides = (keys.stride(0), keys.stride(1), keys.stride(2))
+    _native.check(lib.sah_pq_assign(keys.data_ptr(), _native.SAH_BF16, *strides, B, Hkv, off, n_keys + off, off, n_sub, 8,
+                                    n_cent, cent.data_ptr(), want.data_ptr(), cap, 0, st), "sah_pq_assign")
+    _native.check(lib.sah_pq_assign_tc(keys.data_ptr(), *strides, B, Hkv, off, n_keys + off, off, n_sub, 8, n_cent,
+                                       cent.data_ptr(), got.data_ptr(), cap, err.data_ptr(), 2, st), "sah_pq_assign_tc")
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and torch.equal(got, want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype,n_sub,sub_d,n_keys,n_cent", [
     ("bf16", 16, 8, 1, 32), ("bf16", 16, 8, 4097, 32), ("bf16", 4, 9, 5000, 32), ("f32", 3, 16, 4096, 32),
     ("f32", 2, 5, 9000, 32), ("bf16", 16, 8, 4200, 256), ("f32", 2, 8, 4099, 129), ("bf16", 2, 8, 5001, 128),
