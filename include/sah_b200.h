@@ -564,12 +564,21 @@ int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t 
                   const double* sums, const int* counts, const int64_t* reseed, float* centroids,
                   float* shift2, void* stream);
 
-/* All Lloyd iterations of kmeans_batched (pq_utils.py:220-423) over the keys [init_offset, init_offset + n_keys):
- * assignment (sah_pq_assign_tc with use_tc != 0, for the shapes it takes; sah_pq_assign without), sums, new
- * centres.  The comparison with the tolerance happens on the device; the kernels of the iterations that are
- * left after it return at once.  reseed: n_iter device pointers (host array).  sums and counts are scratch of
- * sah_pq_accumulate's sizes.  state: five words on the device; state[1] is the number of iterations that ran,
- * state[2] is set when a bounded wait of the tensor-core kernel ran out (codes and centroids are then void).
+/* Lloyd iterations of kmeans_batched (pq_utils.py:220-423) over the keys [init_offset, init_offset + n_keys), in
+ * parts (`what`, in this order): BEGIN clears sums, counts and state; UPDATE ends an iteration (new centres, `reseed`
+ * for empty ones, the comparison with the tolerance); ASSIGN begins one (assignment -- sah_pq_assign_tc with
+ * use_tc != 0, for the shapes it takes; sah_pq_assign without -- and sums).  The comparison happens on the
+ * device: parts launched after the clustering has converged return at once, so the next ASSIGN can be launched
+ * before the host knows.  sums and counts are scratch of sah_pq_accumulate's sizes.  state: five words on the
+ * device; [0] is set once the clustering has converged, [1] is the number of iterations that ran, [2] is
+ * set when a bounded wait of the tensor-core kernel ran out (codes and centroids are then void). */
+enum { SAH_KMEANS_BEGIN = 1, SAH_KMEANS_UPDATE = 2, SAH_KMEANS_ASSIGN = 4 };
+int sah_pq_kmeans_step(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                       int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int what,
+                       const int64_t* reseed, float* centroids, uint8_t* codes, int64_t cap, double* sums, int* counts,
+                       int* state, int use_tc, int sm_count, void* stream);
+
+/* n_iter iterations launched together.  reseed: n_iter device pointers (host array).
  * All operands stay untouched until the stream has passed the last launch. */
 int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
                   int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int n_iter,

@@ -412,7 +412,7 @@ extern "C" int sah_pq_accumulate(const void* x, int dtype, int64_t xs_b, int64_t
 // new centre = fp32(sum) / fp32(count); an empty cluster takes the key sub-vector at
 // reseed[group][cluster] (pq_utils.py:384-396); shift2[group] = (sum over clusters of
 // the centre's Euclidean move)^2, the quantity compared with the tolerance (:399-423).
-// With `state` (the words that sah_pq_kmeans keeps) the sums and counts are cleared for the next
+// With `state` (the words that sah_pq_kmeans_step keeps) the sums and counts are cleared for the next
 // iteration and the last block makes the comparison.
 struct PqState {
   int done, iterations, err, open, ticket;
@@ -494,22 +494,31 @@ extern "C" int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_
   return SAH_OK;
 }
 
-extern "C" int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
-                             int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int n_iter,
-                             const int64_t* const* reseed, float* centroids, uint8_t* codes, int64_t cap,
-                             double* sums, int* counts, int* state, int use_tc, int sm_count, void* stream) {
-  SAH_REQUIRE(x && reseed && centroids && codes && sums && counts && state, "pq_kmeans: null pointer");
-  SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_keys >= 0 && n_iter >= 0, "pq_kmeans: bad extents");
+extern "C" int sah_pq_kmeans_step(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                                  int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int what,
+                                  const int64_t* reseed, float* centroids, uint8_t* codes, int64_t cap, double* sums,
+                                  int* counts, int* state, int use_tc, int sm_count, void* stream) {
+  SAH_REQUIRE(x && centroids && codes && sums && counts && state && (reseed || !(what & SAH_KMEANS_UPDATE)),
+              "pq_kmeans: null pointer");
+  SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_keys >= 0, "pq_kmeans: bad extents");
   SAH_REQUIRE(n_cent > 0 && n_cent <= 256, "pq_kmeans: 1..256 centroids");
-  for (int it = 0; it < n_iter; ++it) SAH_REQUIRE(reseed[it], "pq_kmeans: null pointer");
   const int64_t groups = (int64_t)B * Hkv * n_sub;
   const cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(sums, 0, (size_t)(groups * n_cent * sub_d) * sizeof(double), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, (size_t)(groups * n_cent) * sizeof(int), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(state, 0, sizeof(PqState), st);
-  if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_kmeans: %s", cudaGetErrorString(e));
   PqState* ps = reinterpret_cast<PqState*>(state);
-  for (int it = 0; it < n_iter; ++it) {
+  if (what & SAH_KMEANS_BEGIN) {
+    cudaError_t e = cudaMemsetAsync(sums, 0, (size_t)(groups * n_cent * sub_d) * sizeof(double), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, (size_t)(groups * n_cent) * sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(state, 0, sizeof(PqState), st);
+    if (e != cudaSuccess) return sah_fail(SAH_ERR_CUDA, "pq_kmeans: %s", cudaGetErrorString(e));
+  }
+  if (what & SAH_KMEANS_UPDATE) {
+    SAH_DISPATCH_DTYPE(dtype, T, {
+      pq_update_kernel<T><<<(unsigned)groups, 256, 0, st>>>((const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub,
+                                                            sub_d, n_cent, sums, counts, reseed, centroids, nullptr, ps);
+    });
+    SAH_LAUNCH_CHECK("pq_update");
+  }
+  if (what & SAH_KMEANS_ASSIGN) {
     int rc = use_tc ? pq_assign_tc_run(x, xs_b, xs_h, xs_s, B, Hkv, init_offset, init_offset + n_keys, init_offset,
                                        n_sub, sub_d, n_cent, centroids, codes, cap, &ps->err, sm_count, &ps->done, stream)
                     : pq_assign_run(x, dtype, xs_b, xs_h, xs_s, B, Hkv, init_offset, init_offset + n_keys, init_offset,
@@ -518,14 +527,23 @@ extern "C" int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_
       rc = pq_accumulate_run(x, dtype, xs_b, xs_h, xs_s, B, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent, codes, cap,
                              sums, counts, &ps->done, stream);
     if (rc != SAH_OK) return rc;
-    SAH_DISPATCH_DTYPE(dtype, T, {
-      pq_update_kernel<T><<<(unsigned)groups, 256, 0, st>>>((const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub,
-                                                            sub_d, n_cent, sums, counts, reseed[it], centroids, nullptr,
-                                                            ps);
-    });
-    SAH_LAUNCH_CHECK("pq_update");
   }
   return SAH_OK;
+}
+
+extern "C" int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
+                             int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int n_iter,
+                             const int64_t* const* reseed, float* centroids, uint8_t* codes, int64_t cap,
+                             double* sums, int* counts, int* state, int use_tc, int sm_count, void* stream) {
+  SAH_REQUIRE(reseed && n_iter >= 0, "pq_kmeans: no re-seeding indices");
+  for (int it = 0; it < n_iter; ++it) SAH_REQUIRE(reseed[it], "pq_kmeans: null pointer");
+  int rc = SAH_OK;
+  for (int it = 0; it <= n_iter && rc == SAH_OK; ++it)
+    rc = sah_pq_kmeans_step(x, dtype, xs_b, xs_h, xs_s, B, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent,
+                            (it == 0 ? SAH_KMEANS_BEGIN : SAH_KMEANS_UPDATE) | (it < n_iter ? SAH_KMEANS_ASSIGN : 0),
+                            it > 0 ? reseed[it - 1] : nullptr, centroids, codes, cap, sums, counts, state, use_tc, sm_count,
+                            stream);
+  return rc;
 }
 
 // ---------------------------------------------------------------------------

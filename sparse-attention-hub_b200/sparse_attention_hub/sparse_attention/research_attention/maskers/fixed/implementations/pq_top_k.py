@@ -23,7 +23,6 @@ first `2**bits` entries of a random permutation per group unless
 """
 
 from dataclasses import dataclass
-import ctypes
 import os
 from typing import Any, Dict, Optional, Tuple, Union
 
@@ -297,45 +296,51 @@ class PQCache(TopKMasker):
 
     def _lloyd(self, k: torch.Tensor, kargs, local_off: int, geometry, reseed_src, centroids: torch.Tensor,
                codes: torch.Tensor, sums: torch.Tensor, counts: torch.Tensor, use_tc: bool, first_centroids) -> None:
-        """The Lloyd iterations over one device's keys, launched together: the test for convergence is made
-        on the device, and the host waits once, at the end (with a wait for every iteration's test,
-        8 KV heads x 65472 keys and ten iterations took 0.9 ms longer)."""
-        if self.kmeans_iter <= 0:
-            return
+        """The Lloyd iterations over one device's keys.  The test for convergence is made on the device, and the next
+        iteration's assignment is launched before the host has its outcome (it returns at once if that was the
+        last): the host's wait passes behind it, every iteration draws what it uses when it is known to be
+        needed, and no more than one assignment is launched in vain.  (A wait without work behind it in every
+        iteration: 8 KV heads x 65472 keys and ten iterations took 0.9 ms longer.)"""
         lib = _native.load()
         B, Hkv, n_sub, sub_d, n_cent = geometry
         dev = k.device
         n_keys = k.shape[2] - local_off
-        drawn_before = []  # the generator's state in front of every draw
-        reseed = []
-        for it in range(self.kmeans_iter):
-            if reseed_src is not None:
-                try:
-                    given = reseed_src[it]
-                except (IndexError, KeyError):  # as few as the clustering may need
-                    break
-                reseed.append(given.to(device=dev, dtype=torch.long).contiguous())
-            else:
-                drawn_before.append(torch.cuda.get_rng_state(dev))
-                reseed.append(torch.randint(0, n_keys, (B * Hkv * n_sub, n_cent), device=dev))
         state = torch.empty(5, dtype=torch.int32, device=dev)
-        pointers = (ctypes.c_void_p * len(reseed))(*[r.data_ptr() for r in reseed])
+        seen = torch.empty(5, dtype=torch.int32, pin_memory=True)
+        reached = torch.cuda.Event()
+        drawn = []
 
-        def launch(tensor_cores: bool) -> list:
-            _native.check(lib.sah_pq_kmeans(*kargs, B, Hkv, n_keys, local_off, n_sub, sub_d, n_cent, len(reseed), pointers,
-                                            centroids.data_ptr(), codes.data_ptr(), codes.shape[2], sums.data_ptr(),
-                                            counts.data_ptr(), state.data_ptr(), int(tensor_cores),
-                                            _native.sm_count(dev), _native.stream_of(dev)), "sah_pq_kmeans")
-            return state.tolist()
+        def launch(what: int, reseed: Optional[torch.Tensor] = None) -> None:
+            _native.check(lib.sah_pq_kmeans_step(*kargs, B, Hkv, n_keys, local_off, n_sub, sub_d, n_cent, what,
+                                                 _native.ptr(reseed), centroids.data_ptr(), codes.data_ptr(),
+                                                 codes.shape[2], sums.data_ptr(), counts.data_ptr(), state.data_ptr(),
+                                                 int(use_tc), _native.sm_count(dev), _native.stream_of(dev)),
+                          "sah_pq_kmeans_step")
 
-        done, ran, failed = launch(use_tc)[:3]
-        if failed:  # a bounded wait inside the tensor-core kernel ran out: fixed-order kernel, from the start
-            centroids.copy_(first_centroids())
-            done, ran, _ = launch(False)[:3]
-        if not done and len(reseed) < self.kmeans_iter:
-            reseed_src[len(reseed)]  # one more was needed: the error that the lookup raises
-        if ran < len(drawn_before):  # converged early: the draws behind it were not made
-            torch.cuda.set_rng_state(drawn_before[ran], dev)
+        launch(_native.KMEANS_BEGIN | _native.KMEANS_ASSIGN)
+        it = 0
+        while it < self.kmeans_iter:
+            if it < len(drawn):
+                pass  # from the start again, below
+            elif reseed_src is not None:
+                drawn.append(reseed_src[it].to(device=dev, dtype=torch.long).contiguous())
+            else:
+                drawn.append(torch.randint(0, n_keys, (B * Hkv * n_sub, n_cent), device=dev))
+            launch(_native.KMEANS_UPDATE, drawn[it])
+            seen.copy_(state, non_blocking=True)
+            reached.record(torch.cuda.current_stream(dev))
+            it += 1
+            if it < self.kmeans_iter:
+                launch(_native.KMEANS_ASSIGN)
+            reached.synchronize()
+            done, _, failed = seen[:3].tolist()
+            if failed:  # a bounded wait inside the tensor-core kernel ran out: fixed-order kernel, from the start
+                use_tc = False
+                centroids.copy_(first_centroids())
+                launch(_native.KMEANS_BEGIN | _native.KMEANS_ASSIGN)
+                it = 0
+            elif done:
+                break
 
     def _handle_incremental_keys(self, keys: torch.Tensor, layer_idx: int,
                                  sparse_meta_data: Dict[str, Any], local_off: Optional[int] = None):

@@ -593,3 +593,37 @@ def test_gpu_lloyd_iterations_launched_together(dtype, n_keys, given, iters):
         meta["pq_reseed_indices"] = {0: draws[:ran - 1]}
         with pytest.raises(IndexError):
             masker._perform_kmeans_clustering(keys, 0, meta)
+
+
+@pytest.mark.gpu
+def test_gpu_clustering_goes_no_further_than_it_has_to(monkeypatch):
+    """Forty keys for sixteen centres: the clustering converges after a few of its hundred iterations.  No more
+    than one assignment is launched in vain, no index drawn in vain, and the generator is never set back (another
+    thread may have drawn from it meanwhile)."""
+    import torch
+    from sparse_attention_hub import _native
+    from sparse_attention_hub.sparse_attention.research_attention.maskers.fixed import PQCache, PQCacheConfig
+
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(1)
+    keys = torch.randn((1, 2, 48, 32), generator=gen, device=dev).bfloat16()
+    masker = PQCache(PQCacheConfig(heavy_size=8, pq_group_factor=4, pq_bits=4, kmeans_iter=100, init_offset=8,
+                                   metric="euclidean"))
+    init = torch.rand((8, 40), generator=gen, device=dev).topk(16, dim=1).indices
+    draw, draws = torch.randint, []
+
+    def counted(*args, **kwargs):
+        draws.append(draw(*args, **kwargs))
+        return draws[-1]
+
+    def refused(*args, **kwargs):
+        raise AssertionError("the generator was set back")
+
+    monkeypatch.setattr(torch, "randint", counted)
+    monkeypatch.setattr(torch.cuda, "set_rng_state", refused)
+    meta = {"pq_init_indices": {0: init}}
+    masker._initialize_pq_cache(meta, 0)
+    before = _native.launch_count()
+    masker._perform_kmeans_clustering(keys, 0, meta)
+    assert 1 <= len(draws) < 20
+    assert _native.launch_count() - before <= 3 * (len(draws) + 1)
