@@ -18,8 +18,8 @@
 //   and columns meet, first minimum wins, as torch.argmin does.
 //   Equal centroids (of equal keys, of channels that are 0) tie at every key, and their rows and columns meet nearly
 //   everywhere: only the lowest of them can be the answer, so the columns of the others are put below every
-//   centroid.  8 KV heads x 65472 keys, 16 of them distinct: 5.56 -> 1.52 ms; half of the sub-vectors 0: 6.3 -> 0.25 ms;
-//   all different 0.25 ms, of which finding that out is 5 us.
+//   centroid.  8 KV heads x 65472 keys, 16 of them distinct, 5.57 -> 0.25 ms, a fifth of the centroids one bit off
+//   5.46 -> 0.38 ms; half of the sub-vectors 0 6.3 -> 0.25 ms; all different 0.25 ms, of which finding that out is 7 us.
 //   E = 2^-16 (|x|^2 + max_c |c|^2).  A float32 sum of 27 exact products, in whatever order and
 //   even truncated, is within 27 * 2^-23 (|x||c| + |c|^2 / 2) <= 2^-18.2 (|x|^2 + |c|^2) of the
 //   exact one; the fixed-order distance is within 10 * 2^-24 * 2 (|x|^2 + |c|^2) <= 2^-19.6 (...)
@@ -50,6 +50,7 @@
 #define PTC_TILE 128
 #define PTC_SLOT_BITS 10
 #define PTC_SLOTS (1 << PTC_SLOT_BITS)  // where the lowest of equal centroids is noted
+#define PTC_SLOTS2 256                  // ... of those whose slot a lower one of another value has
 #define PTC_THREADS 320  // two groups of four warps, and an issuing warp for each
 
 template <int NS>
@@ -57,8 +58,8 @@ struct PtcCfg {
   static constexpr int A_OFF = 0;                                // two groups' [128 rows][128 B], first 64 B used
   static constexpr int B_OFF = 2 * PTC_TILE * 128;               // NS x [256 rows][128 B], first 64 B used
   static constexpr int CENT_OFF = B_OFF + NS * 256 * 128;        // NS x float32 [256][8]
-  static constexpr int FIRST_OFF = CENT_OFF + NS * 256 * 8 * 4;    // NS x lowest centroid of every slot
-  static constexpr int MISC_OFF = FIRST_OFF + NS * PTC_SLOTS * 4;  // max |c|^2 per sub-vector, mbarriers, slot, abort
+  static constexpr int FIRST_OFF = CENT_OFF + NS * 256 * 8 * 4;    // lowest centroids of the slots
+  static constexpr int MISC_OFF = FIRST_OFF + NS * (PTC_SLOTS + PTC_SLOTS2) * 4;  // max |c|^2 per sub-vector, mbarriers, slot, abort
   static constexpr int NEED = 1024 + MISC_OFF + 128;
   // never less than half of an SM's shared memory: one CTA per SM, it holds all of tensor memory
   static constexpr int SMEM = NEED > 120 * 1024 ? NEED : 120 * 1024;
@@ -101,14 +102,14 @@ __device__ __forceinline__ void ptc_split3(float v, __nv_bfloat16* h, __nv_bfloa
   *l = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(*m)));
 }
 
-// where a centroid of 8 floats is looked up, by its bits
-__device__ __forceinline__ int ptc_slot(const float* c) {
+// by which equal centroids of 8 floats are found (bits 22 to 31, then 7 to 14)
+__device__ __forceinline__ unsigned int ptc_hash(const float* c) {
   const uint4 a = reinterpret_cast<const uint4*>(c)[0], b = reinterpret_cast<const uint4*>(c)[1];
   const unsigned int v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   unsigned int h = 0u;
 #pragma unroll
-  for (int d = 0; d < 8; ++d) h = (h ^ v[d]) * 0x9e3779b1u;
-  return (int)(h >> (32 - PTC_SLOT_BITS));
+  for (int d = 0; d < 8; ++d) h = (__funnelshift_l(h, h, 13) ^ v[d]) * 0x9e3779b1u;
+  return h ^ (h >> 15);
 }
 
 // 32 columns of an accumulator: two matrix rows of 16
@@ -153,6 +154,7 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
   const int wg = issuer ? warp - 8 : warp >> 2, keyl = tid & 127;  // group of four warps, key of its tile
   float* cent_sm = reinterpret_cast<float*>(sm + C::CENT_OFF);
   unsigned int* first_sm = reinterpret_cast<unsigned int*>(sm + C::FIRST_OFF);
+  unsigned int* second_sm = first_sm + NS * PTC_SLOTS;
   unsigned int* cmax_sm = reinterpret_cast<unsigned int*>(sm + C::MISC_OFF);  // [NS], float bits
   const uint32_t full = sm_s + C::MISC_OFF + 32 + wg * 8;   // the group's product is complete
   const uint32_t ready = sm_s + C::MISC_OFF + 48 + wg * 8;  // its A rows are written, its accumulator is read
@@ -199,7 +201,7 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
     const __nv_bfloat16* xb = x + (bk / Hkv) * xs_b + (bk % Hkv) * xs_h + sub0 * SD;
     __syncthreads();  // both groups are done with the previous block
     if (tid < NS) cmax_sm[tid] = 0u;
-    for (int i = tid; i < NS * PTC_SLOTS; i += PTC_THREADS) first_sm[i] = 256u;
+    for (int i = tid; i < NS * (PTC_SLOTS + PTC_SLOTS2); i += PTC_THREADS) first_sm[i] = 256u;
     __syncthreads();
     for (int i = tid; i < NS * NC; i += PTC_THREADS) {
       const int s = i / NC, c = i - s * NC;
@@ -215,7 +217,7 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
       }
       if (c < n_cent) ptc_split3(-0.5f * n2, nn, nn + 1, nn + 2);
       else nn[0] = __float2bfloat16_rn(-INFINITY);  // below every centroid, however far out those lie
-      if (c < n_cent) atomicMin(first_sm + s * PTC_SLOTS + ptc_slot(cent_sm + (s * 256 + c) * SD), (unsigned int)c);
+      if (c < n_cent) atomicMin(first_sm + s * PTC_SLOTS + (ptc_hash(cent_sm + (s * 256 + c) * SD) >> (32 - PTC_SLOT_BITS)), (unsigned int)c);
       // a NaN or infinite norm makes the margin NaN or infinite: every centroid is then measured
       if (c < n_cent) atomicMax(cmax_sm + s, __float_as_uint(n2));
       unsigned char* row = sm + C::B_OFF + s * (256 * 128) + c * 128;
@@ -225,15 +227,33 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
       *reinterpret_cast<uint4*>(row + ((3 ^ (c & 7)) << 4)) = *reinterpret_cast<const uint4*>(nn);
     }
     __syncthreads();
-    for (int i = tid; i < NS * n_cent; i += PTC_THREADS) {  // copies of a lower centroid go below every centroid too
-      const int s = i / n_cent, c = i - s * n_cent, f = (int)first_sm[s * PTC_SLOTS + ptc_slot(cent_sm + (s * 256 + c) * SD)];
-      if (f >= c) continue;
+    // copies of a lower centroid go below every centroid too; the lowest of others that hold their slot are looked up
+    // a second time among those
+    auto copy_of = [&](int s, int c, int f) {
+      if (f >= c) return false;
       const uint4 *own = reinterpret_cast<const uint4*>(cent_sm + (s * 256 + c) * SD),
                   *other = reinterpret_cast<const uint4*>(cent_sm + (s * 256 + f) * SD);
       const uint4 a0 = own[0], a1 = own[1], b0 = other[0], b1 = other[1];
-      if (a0.x == b0.x && a0.y == b0.y && a0.z == b0.z && a0.w == b0.w && a1.x == b1.x && a1.y == b1.y && a1.z == b1.z &&
-          a1.w == b1.w)
-        *reinterpret_cast<uint4*>(sm + C::B_OFF + s * (256 * 128) + c * 128 + ((3 ^ (c & 7)) << 4)) = make_uint4(0xff80u, 0u, 0u, 0u);
+      if (a0.x != b0.x || a0.y != b0.y || a0.z != b0.z || a0.w != b0.w || a1.x != b1.x || a1.y != b1.y || a1.z != b1.z ||
+          a1.w != b1.w)
+        return false;
+      *reinterpret_cast<uint4*>(sm + C::B_OFF + s * (256 * 128) + c * 128 + ((3 ^ (c & 7)) << 4)) = make_uint4(0xff80u, 0u, 0u, 0u);
+      return true;
+    };
+    uint32_t again = 0u;
+    int m = 0;
+    for (int i = tid; i < NS * n_cent; i += PTC_THREADS, ++m) {
+      const int s = i / n_cent, c = i - s * n_cent;
+      const unsigned int bits = ptc_hash(cent_sm + (s * 256 + c) * SD);
+      const int f = (int)first_sm[s * PTC_SLOTS + (bits >> (32 - PTC_SLOT_BITS))];
+      if (f == c || copy_of(s, c, f)) continue;
+      again |= 1u << m;
+      atomicMin(second_sm + s * PTC_SLOTS2 + ((bits >> 7) & (PTC_SLOTS2 - 1)), (unsigned int)c);
+    }
+    __syncthreads();
+    for (; again; again &= again - 1) {
+      const int i = tid + (__ffs(again) - 1) * PTC_THREADS, s = i / n_cent, c = i - s * n_cent;
+      copy_of(s, c, (int)second_sm[s * PTC_SLOTS2 + ((ptc_hash(cent_sm + (s * 256 + c) * SD) >> 7) & (PTC_SLOTS2 - 1))]);
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
