@@ -850,6 +850,9 @@ typedef struct {
   int64_t total, scores, bits, ucols, umemb, ucount, partial; /* bytes; offsets in the scratch */
 } sah_fixed_step_layout;
 
+/* Identity of the capture that a stream is in, 0 for none. */
+int64_t sah_stream_capture(void* stream);
+
 int sah_fixed_step_plan(const sah_fixed_step* step, sah_fixed_step_layout* layout);
 int sah_fixed_step_run(const sah_fixed_step* step, const sah_fixed_step_layout* layout, void* stream);
 

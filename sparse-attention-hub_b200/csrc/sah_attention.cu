@@ -1593,6 +1593,16 @@ static AttnIntervals step_intervals(const sah_fixed_step* s) {
 
 static_assert(SAH_STEP_MAX_BANDS == SAH_MAX_BANDS, "one limit");
 
+extern "C" int64_t sah_stream_capture(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? (int64_t)id : 0;
+}
+
 extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layout* o) {
   SAH_REQUIRE(s && o, "fixed_step_plan: null pointer");
   SAH_REQUIRE(s->B > 0 && s->Hq > 0 && s->Hkv > 0 && s->Sq > 0 && s->S > 0 && s->D > 0 && s->heavy >= 0,

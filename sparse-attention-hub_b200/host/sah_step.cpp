@@ -23,19 +23,22 @@ namespace {
 
 int (*plan_fn)(const sah_fixed_step*, sah_fixed_step_layout*) = nullptr;
 int (*run_fn)(const sah_fixed_step*, const sah_fixed_step_layout*, void*) = nullptr;
+int64_t (*capture_fn)(void*) = nullptr;
 
-// bind(address of sah_fixed_step_plan, address of sah_fixed_step_run)
+// bind(addresses of sah_fixed_step_plan, sah_fixed_step_run and sah_stream_capture)
 PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-  if (nargs != 2) {
-    PyErr_SetString(PyExc_TypeError, "bind: two addresses expected");
+  if (nargs != 3) {
+    PyErr_SetString(PyExc_TypeError, "bind: three addresses expected");
     return nullptr;
   }
-  void* plan = PyLong_AsVoidPtr(args[0]);
-  if (plan == nullptr && PyErr_Occurred()) return nullptr;
-  void* run = PyLong_AsVoidPtr(args[1]);
-  if (run == nullptr && PyErr_Occurred()) return nullptr;
-  plan_fn = reinterpret_cast<decltype(plan_fn)>(plan);
-  run_fn = reinterpret_cast<decltype(run_fn)>(run);
+  void* address[3];
+  for (int i = 0; i < 3; ++i) {
+    address[i] = PyLong_AsVoidPtr(args[i]);
+    if (address[i] == nullptr && PyErr_Occurred()) return nullptr;
+  }
+  plan_fn = reinterpret_cast<decltype(plan_fn)>(address[0]);
+  run_fn = reinterpret_cast<decltype(run_fn)>(address[1]);
+  capture_fn = reinterpret_cast<decltype(capture_fn)>(address[2]);
   Py_RETURN_NONE;
 }
 
@@ -46,13 +49,13 @@ bool rows_of(const at::Tensor& t, int64_t* strides) {
 }
 
 // fixed_step(queries, keys, values, attention_mask or None, sinks or None, scaling, bands, heavy, tickets,
-//            sm_count, stream)
-// -> None, a non-zero status, or (out, scratch, offsets of ucols (-1: there is no list), umemb and ucount in it, groups,
+//            sm_count, stream, whether a capture may keep the tickets)
+// -> None, a non-zero status, (identity of the capture that the stream is in,) for tickets that it may not keep, or (out, scratch, offsets of ucols (-1: there is no list), umemb and ucount in it, groups,
 //     rows per group)
 PyObject* fixed_step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 11 || plan_fn == nullptr) {
-    PyErr_SetString(PyExc_TypeError, "fixed_step: eleven arguments expected, after bind()");
+  if (nargs != 12 || plan_fn == nullptr) {
+    PyErr_SetString(PyExc_TypeError, "fixed_step: twelve arguments expected, after bind()");
     return nullptr;
   }
   for (int i = 0; i < 3; ++i)
@@ -111,6 +114,10 @@ PyObject* fixed_step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   s.n_tickets = tickets.numel();
   sah_fixed_step_layout layout;
   if (plan_fn(&s, &layout) != SAH_OK) Py_RETURN_NONE;
+  if (args[11] != Py_True) {
+    const int64_t capture = capture_fn(stream);
+    if (capture != 0) return Py_BuildValue("(L)", (long long)capture);
+  }
   at::Tensor out, scratch;
   int status;
   {

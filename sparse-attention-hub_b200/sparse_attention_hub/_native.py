@@ -76,6 +76,7 @@ _SIGNATURES = {
     "sah_hash_encode": [_P, _I, _L, _L, _L, _I, _I, _I, _L, _L, _L, _I, POINTER(c_int),
                         POINTER(c_void_p), POINTER(c_void_p), _I, _P, _P, _P],
     "sah_hash_topk": [_P, _L, _P, _I, _P, _I, _L, _L, _L, _I, _I, _I, _L, _L, _P, _L, _P, _P],
+    "sah_stream_capture": [_P],  # returns int64
     "sah_fixed_step_plan": [_P, _P],
     "sah_fixed_step_run": [_P, _P, _P],
     "sah_qk_scores": [_P, _P, _I, _L, _L, _L, _L, _L, _L, _I, _I, _I, _I, _L, _I, _P, _L, _L,
@@ -187,6 +188,7 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.argtypes = argtypes
         fn.restype = c_int
+    lib.sah_stream_capture.restype = c_int64
     lib.sah_topk_select_ws_bytes.restype = c_int64
     lib.sah_attn_exchange_bytes.restype = c_int64
     lib.sah_lsh_key_sign_tc_ws_bytes.restype = c_int64

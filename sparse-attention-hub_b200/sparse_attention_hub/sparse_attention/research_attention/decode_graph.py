@@ -67,9 +67,12 @@ class DecodeStepGraph:
 
         # Warm up on a side stream: fills the workspaces, tables and signature caches
         # that must already exist when the capture starts.
+        from ..utils import mask_attention_utils
+
+        tickets = mask_attention_utils.TicketHolder()
         side = torch.cuda.Stream(device=queries.device)
         side.wait_stream(torch.cuda.current_stream(queries.device))
-        with torch.cuda.stream(side):
+        with torch.cuda.stream(side), tickets:
             for _ in range(max(1, warmup)):
                 call()
         torch.cuda.current_stream(queries.device).wait_stream(side)
@@ -77,12 +80,10 @@ class DecodeStepGraph:
 
         # The attention scratch is cached per (stream, shape): capture on the warm-up stream so
         # that the capture finds it, and keep it alive for as long as the graph may replay.
-        from ..utils import mask_attention_utils
-
         self._scratch = [*mask_attention_utils._workspace_cache.values(),
-                         *mask_attention_utils._ticket_cache.values()]
+                         *mask_attention_utils._error_words.values(), tickets]
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph, stream=side):
+        with torch.cuda.graph(self.graph, stream=side), tickets:
             self.out = call()
 
     def replay(self, queries: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -13,7 +13,6 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
-import threading
 from typing import List, Optional
 
 import torch
@@ -24,7 +23,6 @@ from .maskers.fixed.implementations.basic_fixed import LocalMasker, SinkMasker
 from .maskers.fixed.implementations.oracle_top_k import OracleTopK
 
 _MAX_BANDS = 6       # SAH_STEP_MAX_BANDS
-_N_TICKETS = 16384   # KV groups per call, and the error word
 
 #: the maskers that it serves, in some orders; their subclasses are not among them
 SERVED = frozenset((SinkMasker, LocalMasker, OracleTopK))
@@ -44,22 +42,10 @@ def _step_module():
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         lib = _native.load()
-        module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.sah_fixed_step_plan, lib.sah_fixed_step_run)))
+        module.bind(*(ctypes.cast(f, ctypes.c_void_p).value
+                      for f in (lib.sah_fixed_step_plan, lib.sah_fixed_step_run, lib.sah_stream_capture)))
         _module = module
     return _module
-
-
-def _tickets(device: torch.device, stream: int) -> torch.Tensor:
-    """Merge tickets (and the error word in front of them) of the calls of one stream and host thread:
-    zero between calls, so they are made once and not per call."""
-    pool = mask_attention_utils._ticket_cache
-    key = (device.index, stream, threading.get_ident())
-    found = pool.get(key)
-    if found is None:
-        if len(pool) > 16:
-            pool.clear()
-        found = pool[key] = torch.zeros(_N_TICKETS, dtype=torch.int32, device=device)
-    return found
 
 
 def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
@@ -96,14 +82,18 @@ def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values:
             return None
     device = queries.device
     stream = _native.stream_of(device)
-    tickets = _tickets(device, stream)
-    done = _step_module().fixed_step(queries, keys, values, attention_mask, sinks, float(scaling), bands, heavy, tickets,
-                                     _native.sm_count(device), stream)
+    tickets, captured = mask_attention_utils.merge_tickets(device, stream)
+    call = _step_module().fixed_step
+    done = call(queries, keys, values, attention_mask, sinks, float(scaling), bands, heavy, tickets,
+                _native.sm_count(device), stream, captured)
     if done is None:
         return None
+    if type(done) is tuple and len(done) == 1:  # nothing launched: the stream is being captured, with this identity
+        tickets = mask_attention_utils.graph_tickets(device, stream, done[0])
+        done = call(queries, keys, values, attention_mask, sinks, float(scaling), bands, heavy, tickets,
+                    _native.sm_count(device), stream, True)
     if isinstance(done, int):
-        # a refused launch may leave tickets behind
-        mask_attention_utils._ticket_cache.pop((device.index, stream, threading.get_ident()), None)
+        tickets.zero_()  # a refused launch may leave tickets behind
         _native.check(done, "sah_fixed_step_run")
     out, scratch, ucols, umemb, ucount, groups, rows = done
     B, Hq, _, D = queries.shape

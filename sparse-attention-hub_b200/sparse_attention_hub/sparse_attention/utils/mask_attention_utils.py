@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
+import weakref
 from typing import Any, Dict, Optional, Tuple, Union
 
 import torch
@@ -31,18 +32,67 @@ from .mask import Mask, NativeBits, words_per_row
 
 _workspace_cache: Dict[Tuple, Dict[str, torch.Tensor]] = {}
 
-# merge tickets of `fixed_step` calls by (device, stream, host thread); the first word is the error word
+_N_TICKETS = 16384  # KV groups of a `fixed_step` call, and the error word in front of them
+
+# Merge tickets of `fixed_step` calls; the first word is the error word.  Calls of one stream and host thread follow
+# one another and share theirs; what is captured gets tickets of its own, since graphs that were captured on
+# one stream may replay on several at once.  `_graph_tickets`: by capture, made (and zeroed) in it.
 _ticket_cache: Dict[Tuple, torch.Tensor] = {}
+_graph_tickets: Dict[Tuple, torch.Tensor] = {}
+_own_tickets = threading.local()                # .holder: TicketHolder of the calls of this thread, if it has one
+_ticket_holders: "weakref.WeakSet" = weakref.WeakSet()
+# where the kernels without tickets leave the error of a bounded wait: it is only ever set, so one word does
+_error_words: Dict[int, torch.Tensor] = {}
 
 
-def _error_word(device: torch.device, stream: int) -> torch.Tensor:
-    """Where the kernels that take no ticket scratch leave the error of a bounded wait, by stream and thread."""
-    key = (device.index, stream, threading.get_ident(), "error")
-    found = _ticket_cache.get(key)
+class TicketHolder:
+    """Tickets of one graph, made by the calls in front of its capture so that no replay has to zero them."""
+
+    def __init__(self) -> None:
+        self.tickets: Dict[Tuple, torch.Tensor] = {}
+        _ticket_holders.add(self)
+
+    def __enter__(self) -> "TicketHolder":
+        self._before = getattr(_own_tickets, "holder", None)
+        _own_tickets.holder = self
+        return self
+
+    def __exit__(self, *exc) -> None:
+        _own_tickets.holder = self._before
+
+
+def merge_tickets(device: torch.device, stream: int) -> Tuple[torch.Tensor, bool]:
+    """Zeros between calls, so they are made once and not per call; and whether a capture may keep them."""
+    holder = getattr(_own_tickets, "holder", None)
+    pool = _ticket_cache if holder is None else holder.tickets
+    key = (device.index, stream, threading.get_ident())
+    found = pool.get(key)
     if found is None:
-        if len(_ticket_cache) > 16:
-            _ticket_cache.clear()
-        found = _ticket_cache[key] = torch.zeros(1, dtype=torch.int32, device=device)
+        if torch.cuda.is_current_stream_capturing():
+            return graph_tickets(device, stream, _native.load().sah_stream_capture(stream)), True
+        if len(pool) > 16:
+            pool.clear()
+        found = pool[key] = torch.zeros(_N_TICKETS, dtype=torch.int32, device=device)
+    return found, holder is not None
+
+
+def graph_tickets(device: torch.device, stream: int, capture: int) -> torch.Tensor:
+    """Tickets of the graph that is being captured (one set per stream of it), zeroed by its replays."""
+    key = (device.index, stream, capture)
+    found = _graph_tickets.get(key)
+    if found is None:
+        if len(_graph_tickets) > 16:  # the memory stays the graphs'
+            _graph_tickets.clear()
+        found = _graph_tickets[key] = torch.zeros(_N_TICKETS, dtype=torch.int32, device=device)
+    return found
+
+
+def _error_word(device: torch.device) -> torch.Tensor:
+    found = _error_words.get(device.index)
+    if found is None:
+        found = torch.zeros(1, dtype=torch.int32, device=device)
+        if not torch.cuda.is_current_stream_capturing():
+            _error_words[device.index] = found
     return found
 
 
@@ -176,7 +226,7 @@ def native_masked_attention(
         n_parts = lib.sah_attn_stream_parts(B, Hq, Hkv, Sq, S, D, payload.masker.lsh_k, payload.masker.lsh_l, sms)
         if n_parts > 0 and all(s % 8 == 0 for s in strides) and all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
             sig = payload.sig
-            err = _error_word(dev, st)
+            err = _error_word(dev)
             parts = torch.empty((n_parts, B * Hq * Sq, D + 2), dtype=torch.float32, device=dev)
             _native.check(
                 lib.sah_masked_attention_stream(
@@ -310,7 +360,8 @@ def attention_wait_errors() -> int:
         groups = ws.get("groups")
         if groups is not None:
             n += int(ws["ucount"][ws["err_index"]].item() != 0)
-    for tickets in _ticket_cache.values():
+    for tickets in (*_ticket_cache.values(), *_graph_tickets.values(), *_error_words.values(),
+                    *(t for holder in _ticket_holders for t in holder.tickets.values())):
         n += int(tickets[0].item() != 0)
     return n
 

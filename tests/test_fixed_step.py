@@ -142,6 +142,45 @@ def test_streams_and_capture():
     assert torch.equal(out, call())
 
 
+@pytest.mark.gpu
+def test_graphs_have_tickets_of_their_own():
+    """Two graphs captured on one stream, the first never replayed before the second, with shapes of their own or
+    the same, and eager calls on that stream: nobody relies on another's tickets."""
+    from sparse_attention_hub.sparse_attention.research_attention.decode_graph import DecodeStepGraph
+    from sparse_attention_hub.sparse_attention.utils import mask_attention_utils as mau
+
+    ra = workloads.research_attention(TOPK, "bf16", DEV)
+    side = torch.cuda.Stream()
+    calls, graphs, outs = [], [], []
+    for S in (3000, 5000, 5000):
+        q, k, v = _inputs(torch.bfloat16, 1, 8, 2, 1, S, 64)
+        calls.append(lambda q=q, k=k, v=v: ra.custom_attention(None, q, k, v, None, 0.125, 0.0, sparse_meta_data={},
+                                                               layer_idx=0)[0])
+    want = [call() for call in calls]
+    torch.cuda.synchronize()
+    assert mau._ticket_cache
+    eager = {t.data_ptr() for t in mau._ticket_cache.values()}
+    for call in calls:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=side):
+            outs.append(call())
+    with torch.cuda.stream(side):
+        assert torch.equal(calls[1](), want[1])
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for g in reversed(range(3)):
+            outs[g].zero_()
+            graphs[g].replay()
+            assert torch.equal(outs[g], want[g])
+    own = [t.data_ptr() for t in mau._graph_tickets.values()][-3:]
+    assert len(set(own)) == 3 and not eager & set(own)
+    held = DecodeStepGraph(ra, q, k, v, None, 0.125, {})
+    held_tickets = held._scratch[-1].tickets
+    assert len(held_tickets) == 1 and not eager & {t.data_ptr() for t in held_tickets.values()}
+    assert torch.equal(held.replay(q), want[2])
+    assert attention_wait_errors() == 0
+
+
 def test_other_stacks_keep_the_general_path():
     """Nothing but plain sink, local and one final top-k masker is taken, whatever the tensors."""
     class Cuda:  # stands in for a CUDA tensor: the maskers are looked at before anything else of it
