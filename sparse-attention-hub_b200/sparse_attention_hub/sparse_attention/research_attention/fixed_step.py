@@ -13,12 +13,14 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+from functools import lru_cache
 from typing import List, Optional
 
 import torch
 
 from ... import _native
 from ..utils import mask_attention_utils
+from ..utils.mask import words_per_row
 from .maskers.fixed.implementations.basic_fixed import LocalMasker, SinkMasker
 from .maskers.fixed.implementations.oracle_top_k import OracleTopK
 
@@ -48,6 +50,12 @@ def _step_module():
     return _module
 
 
+@lru_cache(maxsize=1024)
+def _select_fits(dtype: torch.dtype, rows: int, S: int) -> int:
+    code = {torch.float32: _native.SAH_F32, torch.bfloat16: _native.SAH_BF16}.get(dtype)
+    return 0 if code is None else _native.load().sah_topk_select_fits(code, rows, S, words_per_row(S))
+
+
 def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
                attention_mask: Optional[torch.Tensor], sinks: Optional[torch.Tensor],
                scaling: float) -> Optional[torch.Tensor]:
@@ -57,6 +65,14 @@ def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values:
     if type(keys) is not torch.Tensor or keys.dim() != 4:
         return None
     Sq, S = queries.shape[2], keys.shape[2]
+    # what sah_fixed_step_plan refuses for its key count, without the way there (57 -> 64 us of a call of four
+    # positions over 40000 keys, 95 -> 102 us of one over 8 rows and a top-k, when the entry was tried first)
+    if S >= 32768:
+        if type(maskers[-1]) is OracleTopK:
+            if not _select_fits(queries.dtype, queries.shape[0] * queries.shape[1] * Sq, S):
+                return None
+        elif Sq > 1 and S > 32768:
+            return None
     bands, heavy = (), 0
     for masker in maskers:
         kind = type(masker)

@@ -143,6 +143,23 @@ def test_streams_and_capture():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("Hq,Sq,S,stack", [(8, 2, 32769, SINK_LOCAL), (8, 4, 70000, SINK_LOCAL), (8, 1, 40000, TOPK),
+                                           (2, 1, 131072, TOPK)])
+def test_key_counts_that_are_refused_are_not_tried(Hq, Sq, S, stack, monkeypatch):
+    """Nothing of the native entry is prepared for a call that it will not take, and what it would say is known."""
+    from sparse_attention_hub.sparse_attention.utils import mask_attention_utils as mau
+
+    q, k, v = _inputs(torch.bfloat16, 1, Hq, 2, Sq, S, 64)
+    maskers = workloads.research_attention(stack, "bf16", DEV).maskers
+    with monkeypatch.context() as m:
+        m.setattr(mau, "merge_tickets", None)
+        assert fs.fixed_step(maskers, q, k, v, None, None, 0.125) is None
+    monkeypatch.setattr(fs, "_select_fits", lambda *_: 1)
+    if stack is TOPK:
+        assert fs.fixed_step(maskers, q, k, v, None, None, 0.125) is None
+
+
+@pytest.mark.gpu
 def test_graphs_have_tickets_of_their_own():
     """Two graphs captured on one stream, the first never replayed before the second, with shapes of their own or
     the same, and eager calls on that stream: nobody relies on another's tickets."""
