@@ -18,7 +18,7 @@ from ..utils.mask_attention_utils import (
     get_masked_attention_output,
     get_true_attention_output,
 )
-from .fixed_step import SERVED, fixed_step
+from .fixed_step import SERVED, SERVED_ATTRIBUTES, fixed_step
 from .maskers.base import MaskerConfig, ResearchMasker
 from .maskers.sampling.base import SamplingMasker
 
@@ -80,14 +80,15 @@ class ResearchAttention(SparseAttention):
         sparse_meta_data: Dict[Any, Any] = kwargs.pop("sparse_meta_data")
         logger = MicroMetricLogger()
         for masker in self.maskers:  # all that other stacks pay for the native entry
-            if type(masker) not in SERVED:
-                native = False
+            kind = type(masker)
+            if kind not in SERVED or kind.add_mask is not SERVED[kind] or len(masker.__dict__) != SERVED_ATTRIBUTES:
+                native = False  # another masker, or one whose methods somebody has put another in place of
                 break
         else:
             native = True
         if (native and not logger.enabled_metrics and not self.return_attention_weights and dropout == 0.0
                 and kwargs.get("sequence_shard") is None
-                and type(self).build_mask is ResearchAttention.build_mask and "build_mask" not in self.__dict__):
+                and type(self).build_mask is _BUILD_MASK and "build_mask" not in self.__dict__):
             # nobody looks at the mask of this call: bands and an exact top-k need none
             s_aux_raw = kwargs.get("s_aux")
             out = fixed_step(self.maskers, queries, keys, values, attention_mask,
@@ -127,3 +128,6 @@ class ResearchAttention(SparseAttention):
             raise TypeError(f"Expected ResearchAttentionConfig, got {type(config)}")
         maskers = [ResearchMasker.create_masker_from_config(c) for c in config.masker_configs]
         return cls(config, maskers)
+
+
+_BUILD_MASK = ResearchAttention.build_mask

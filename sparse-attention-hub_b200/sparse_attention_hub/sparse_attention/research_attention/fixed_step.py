@@ -26,8 +26,10 @@ from .maskers.fixed.implementations.oracle_top_k import OracleTopK
 
 _MAX_BANDS = 6       # SAH_STEP_MAX_BANDS
 
-#: the maskers that it serves, in some orders; their subclasses are not among them
-SERVED = frozenset((SinkMasker, LocalMasker, OracleTopK))
+#: the maskers that it serves, in some orders, and their `add_mask`, which it does the work of; their subclasses
+#: are not among them
+SERVED = {kind: kind.add_mask for kind in (SinkMasker, LocalMasker, OracleTopK)}
+SERVED_ATTRIBUTES = 2  # of an instance: the configuration and the size; any other may stand in for a method
 
 _module = None
 

@@ -160,6 +160,30 @@ def test_key_counts_that_are_refused_are_not_tried(Hq, Sq, S, stack, monkeypatch
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("where", ["masker", "masker class", "score method", "attention", "attention class"])
+def test_methods_that_somebody_replaced_are_called(where, monkeypatch):
+    """A spy on a masker's or the attention's methods sees the call, on the instance and on the class."""
+    ra = workloads.research_attention(TOPK, "bf16", DEV)
+    q, k, v = _inputs(torch.bfloat16, 1, 8, 2, 1, 3000, 64)
+    owner, name = {"masker": (ra.maskers[1], "add_mask"), "masker class": (type(ra.maskers[0]), "add_mask"),
+                   "score method": (ra.maskers[2], "_compute_raw_attention_scores"), "attention": (ra, "build_mask"),
+                   "attention class": (type(ra), "build_mask")}[where]
+
+    def call():
+        return ra.custom_attention(None, q, k, v, None, 0.125, 0.0, sparse_meta_data={}, layer_idx=0)[0]
+
+    want, original, seen = call(), getattr(owner, name), []
+
+    def spy(*args, **kwargs):
+        seen.append(name)
+        return original(*args, **kwargs)
+
+    monkeypatch.setattr(owner, name, spy)
+    got = call()
+    assert seen == [name] and torch.equal(got, want)
+
+
+@pytest.mark.gpu
 def test_graphs_have_tickets_of_their_own():
     """Two graphs captured on one stream, the first never replayed before the second, with shapes of their own or
     the same, and eager calls on that stream: nobody relies on another's tickets."""
