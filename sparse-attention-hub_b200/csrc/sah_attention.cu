@@ -1616,6 +1616,10 @@ extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layou
   if (s->heavy == 0 && s->Sq == 1 && s->S < (1ll << 31)) {
     const int64_t total = step_intervals(s).total;
     o->planned = total == 0;
+    // the kernel without a list is the mma.sync kernel with three stages of copies: not where another was chosen
+    if (s->dtype == SAH_BF16 &&
+        ((s->D == 128 && aum_requested() == 1) || atm_tma_requested() || atm_stages_requested() == 2))
+      o->planned = 1;
   }
   if (o->sizes.groups >= s->n_tickets || (s->heavy == 0 && o->planned && s->S > 32768) ||
       (s->heavy > 0 && sah_topk_select_fits(s->dtype, rows, s->S, o->words) == 0))

@@ -184,6 +184,29 @@ def test_methods_that_somebody_replaced_are_called(where, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("D,S", [(128, 3000), (128, 40000), (64, 3000)])
+def test_a_chosen_kernel_is_taken_for_bands(D, S):
+    from sparse_attention_hub.sparse_attention.utils import mask_attention_utils as mau
+
+    ra = workloads.research_attention(SINK_LOCAL, "bf16", DEV)
+    q, k, v = _inputs(torch.bfloat16, 1, 8, 2, 1, S, D)
+    kernels = {}
+    for choice in ("auto", "mma", "umma"):
+        prev = mau.select_attention_kernel(choice)
+        try:
+            out = ra.custom_attention(None, q, k, v, None, 0.125, 0.0, sparse_meta_data={}, layer_idx=0)[0]
+            kernels[choice] = mau.last_attention_kernel()
+        finally:
+            mau.select_attention_kernel(prev)
+        if choice == "auto":
+            want = out
+        # rounding P and the output to bfloat16
+        assert float((out.double() - want.double()).norm() / want.double().norm()) < 4 * 2.0 ** -9
+    mma, umma = "masked_attention_mma_kernel", "masked_attention_umma_kernel"
+    assert kernels == {"auto": mma, "mma": mma, "umma": umma if D == 128 else mma}
+
+
+@pytest.mark.gpu
 def test_graphs_have_tickets_of_their_own():
     """Two graphs captured on one stream, the first never replayed before the second, with shapes of their own or
     the same, and eager calls on that stream: nobody relies on another's tickets."""
