@@ -818,7 +818,7 @@ int sah_masked_attention_static(const uint32_t* bits, const void* q, const void*
  * it and is left zero; its first word is set when a bounded wait ran out.  Two
  * calls that may overlap on the device need tickets and scratch of their own.
  *
- * sah_fixed_step_plan fills the layout of the scratch (`total` bytes, 256-byte
+ * sah_fixed_step_plan fills the layout of the scratch (256-byte
  * aligned) from the extents and says SAH_ERR_UNSUPPORTED where the separate
  * entry points are the faster or the only way: several query positions over
  * more than 32768 keys without a top-k, rows that sah_topk_select_fits spreads over the grid, too few
@@ -839,15 +839,17 @@ typedef struct {
   int32_t* tickets;
   int64_t n_tickets;
   int32_t sm_count;
-  void* scratch;
-  void* out; /* [B][Sq][Hq][D] */
+  void* scratch; /* `total` bytes: the work list and the partials */
+  void* scores;  /* `scores_total` bytes that nobody needs after the call: scores and their selection */
+  void* out;     /* [B][Sq][Hq][D] */
 } sah_fixed_step;
 
 typedef struct {
   sah_attn_sizes sizes;
   int64_t words; /* of a bitmap row */
   int32_t planned; /* 0: the attention kernel takes the bands themselves, there is no work list */
-  int64_t total, scores, bits, ucols, umemb, ucount, partial; /* bytes; offsets in the scratch */
+  int64_t total, ucols, umemb, ucount, partial; /* bytes; offsets in `scratch` */
+  int64_t scores_total, bits;                   /* ... in `scores`, which begins with them */
 } sah_fixed_step_layout;
 
 /* Identity of the capture that a stream is in, 0 for none. */

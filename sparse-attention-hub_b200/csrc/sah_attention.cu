@@ -1630,8 +1630,10 @@ extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layou
     at += sah_ceil_div(bytes, 256) * 256;
     return p;
   };
-  o->scores = take(s->heavy > 0 ? rows * s->S * (s->dtype == SAH_BF16 ? 2 : 4) : 0);
+  take(s->heavy > 0 ? rows * s->S * (s->dtype == SAH_BF16 ? 2 : 4) : 0);
   o->bits = take(s->heavy > 0 ? rows * o->words * 4 : 0);
+  o->scores_total = at;
+  at = 0;
   o->ucols = take(o->planned ? o->sizes.ucols_bytes : 0);
   o->umemb = take(o->planned ? o->sizes.umemb_bytes : 0);
   o->ucount = take(o->planned ? o->sizes.ucount_bytes : 0);
@@ -1641,9 +1643,9 @@ extern "C" int sah_fixed_step_plan(const sah_fixed_step* s, sah_fixed_step_layou
 }
 
 extern "C" int sah_fixed_step_run(const sah_fixed_step* s, const sah_fixed_step_layout* o, void* stream) {
-  SAH_REQUIRE(s && o && s->scratch && s->tickets && s->out, "fixed_step: null pointer");
+  SAH_REQUIRE(s && o && s->scratch && s->tickets && s->out && (s->scores || s->heavy == 0), "fixed_step: null pointer");
   SAH_REQUIRE(o->sizes.groups < s->n_tickets, "fixed_step: too few tickets");
-  SAH_REQUIRE(((uintptr_t)s->scratch & 15) == 0, "fixed_step: scratch must be 16-byte aligned");
+  SAH_REQUIRE((((uintptr_t)s->scratch | (uintptr_t)s->scores) & 15) == 0, "fixed_step: scratch must be 16-byte aligned");
   unsigned char* p = (unsigned char*)s->scratch;
   int32_t *ucols = (int32_t*)(p + o->ucols), *ucount = (int32_t*)(p + o->ucount);
   uint16_t* umemb = (uint16_t*)(p + o->umemb);
@@ -1654,10 +1656,10 @@ extern "C" int sah_fixed_step_run(const sah_fixed_step* s, const sah_fixed_step_
   } else if (s->heavy > 0) {
     rc = sah_qk_scores(s->q, s->k, s->dtype, s->q_stride[0], s->q_stride[1], s->q_stride[2], s->k_stride[0], s->k_stride[1],
                        s->k_stride[2], s->B, s->Hq, s->Hkv, s->Sq, s->S, s->D, s->bias, s->bias_stride[0],
-                       s->bias_stride[1], s->bias_stride[2], p + o->scores, stream);
+                       s->bias_stride[1], s->bias_stride[2], s->scores, stream);
     if (rc != SAH_OK) return rc;
-    uint32_t* bits = (uint32_t*)(p + o->bits);
-    rc = sah_topk_select_bands(p + o->scores, s->dtype, (int64_t)s->B * s->Hq * s->Sq, s->Sq, s->S, o->words, 0, s->S,
+    uint32_t* bits = (uint32_t*)((unsigned char*)s->scores + o->bits);
+    rc = sah_topk_select_bands(s->scores, s->dtype, (int64_t)s->B * s->Hq * s->Sq, s->Sq, s->S, o->words, 0, s->S,
                                s->n_bands, s->bands, s->heavy, bits, stream);
     if (rc != SAH_OK) return rc;
     rc = sah_attn_plan(bits, nullptr, nullptr, nullptr, s->dtype, s->B, s->Hq, s->Hkv, s->Sq, s->S, o->words, &o->sizes,

@@ -1,11 +1,11 @@
 // Host side of a decode call whose mask is bands (sink, local window) and, at most, an exact top-k
 // of q.k on top of them: tensors in, output out, in one call from Python.
 //
-// Such a call is two to four short kernels (16 us of a float32 call over 4096 keys), and the Python
+// Such a call is one to four short kernels (10 us of a float32 call over 4096 keys), and the Python
 // that checked the tensors, built Mask objects, allocated seven buffers and converted a hundred
-// arguments took longer than they did: 48 us; with this entry the call takes 16 us.  Here the tensors are looked at in C++, one scratch
-// tensor is allocated (with the output it is all that a call allocates, whatever the key count of
-// the call before), and the kernels are launched by sah_fixed_step_run.
+// arguments took longer than they did: 48 us; with this entry the call takes 10 us, as long as its kernel.  Here the
+// tensors are looked at in C++, one scratch tensor is allocated, with a top-k two (with the output all that a call
+// allocates, whatever the key count of the call before), and the kernels are launched by sah_fixed_step_run.
 //
 // fixed_step(...) returns None for tensors that this path does not serve; the caller then takes the
 // general path, which serves them or says what is wrong with them.
@@ -118,12 +118,16 @@ PyObject* fixed_step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int64_t capture = capture_fn(stream);
     if (capture != 0) return Py_BuildValue("(L)", (long long)capture);
   }
-  at::Tensor out, scratch;
+  at::Tensor out, scratch, scores;
   int status;
   {
     pybind11::gil_scoped_release no_gil;
     out = at::empty({s.B, s.Sq, s.Hq, s.D}, q.options().requires_grad(false));
     scratch = at::empty({layout.total}, q.options().dtype(at::kByte).requires_grad(false));
+    if (layout.scores_total > 0) {  // apart from the list, which outlives the call for those who ask about it
+      scores = at::empty({layout.scores_total}, q.options().dtype(at::kByte).requires_grad(false));
+      s.scores = scores.data_ptr();
+    }
     s.out = out.data_ptr();
     s.scratch = scratch.data_ptr();
     status = run_fn(&s, &layout, stream);

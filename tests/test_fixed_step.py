@@ -207,6 +207,21 @@ def test_a_chosen_kernel_is_taken_for_bands(D, S):
 
 
 @pytest.mark.gpu
+def test_scores_do_not_outlive_the_call():
+    """What is kept for last_union_list() is the list: 32 rows x 8000 scores (0.5 MB) and their bits are given back."""
+    ra = workloads.research_attention(TOPK, "bf16", DEV)
+    q, k, v = _inputs(torch.bfloat16, 2, 16, 1, 1, 8000, 64)
+    call = lambda: ra.custom_attention(None, q, k, v, None, 0.125, 0.0, sparse_meta_data={}, layer_idx=0)[0]  # noqa: E731
+    call()
+    torch.cuda.synchronize()
+    out = call()
+    kept = fs.mask_attention_utils._last_plan["step"][0]
+    sizes = fs._native.attn_sizes(2, 16, 1, 1, 8000, 64, 0, fs._native.sm_count(q.device))
+    assert kept.numel() < sizes.ucols_bytes + sizes.umemb_bytes + sizes.ucount_bytes + sizes.partial_bytes + 4 * 256
+    assert torch.equal(out, call())
+
+
+@pytest.mark.gpu
 def test_graphs_have_tickets_of_their_own():
     """Two graphs captured on one stream, the first never replayed before the second, with shapes of their own or
     the same, and eager calls on that stream: nobody relies on another's tickets."""
