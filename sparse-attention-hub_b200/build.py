@@ -16,6 +16,7 @@ import subprocess
 import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
+from importlib import metadata
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -26,6 +27,7 @@ LIB_PATH = LIB_DIR / "libsah_b200.so"
 OBJ_DIR = PKG_DIR / "build"
 STEP_SRC = PKG_DIR / "host" / "sah_step.cpp"
 STEP_PATH = LIB_DIR / "_sah_step.so"
+STEP_STAMP = OBJ_DIR / "_sah_step.made_for"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -57,10 +59,20 @@ def is_stale() -> bool:
     return (not LIB_PATH.exists()) or LIB_PATH.stat().st_mtime < _deps_mtime()
 
 
+def _step_made_for() -> str:
+    """What the host module's binary interface depends on besides its sources."""
+    return f"torch {metadata.version('torch')}, {sysconfig.get_config_var('SOABI')}"
+
+
+def step_is_stale() -> bool:
+    newest = max(f.stat().st_mtime for f in (STEP_SRC, REPO_DIR / "include" / "sah_b200.h"))
+    return (not STEP_PATH.exists() or STEP_PATH.stat().st_mtime < newest
+            or not STEP_STAMP.exists() or STEP_STAMP.read_text() != _step_made_for())
+
+
 def build_step(force: bool = False, verbose: bool = False) -> Path:
     """Compile the host module; returns its path."""
-    newest = max(f.stat().st_mtime for f in (STEP_SRC, REPO_DIR / "include" / "sah_b200.h"))
-    if not force and STEP_PATH.exists() and STEP_PATH.stat().st_mtime >= newest:
+    if not force and not step_is_stale():
         return STEP_PATH
     import torch
     from torch.utils import cpp_extension
@@ -78,6 +90,8 @@ def build_step(force: bool = False, verbose: bool = False) -> Path:
     if res.returncode != 0:
         raise RuntimeError(f"{cmd[0]} failed on {STEP_SRC.name}")
     os.replace(tmp, STEP_PATH)
+    OBJ_DIR.mkdir(exist_ok=True)
+    STEP_STAMP.write_text(_step_made_for())
     return STEP_PATH
 
 

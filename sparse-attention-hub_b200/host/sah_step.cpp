@@ -16,6 +16,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
+#include <torch/version.h>
 
 #include "sah_b200.h"
 
@@ -154,4 +155,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_sah_step", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__sah_step() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__sah_step() {
+  PyObject* m = PyModule_Create(&module);
+  // the torch that the tensors' layout was compiled for
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}

@@ -3,8 +3,9 @@
 The stacks of sink and local-window maskers, alone or followed by an oracle top-k, need no mask
 object between the maskers: the bands are numbers, and the top-k writes one bitmap that the
 attention plan reads.  `fixed_step` hands such a call to `host/sah_step.cpp`, which launches the
-kernels that the maskers and the attention step would (`sah_fixed_step_run`); the output is the same,
-bit for bit.  It returns None wherever the general path has to say or do something else: other
+kernels that the maskers and the attention step would (`sah_fixed_step_run`), for the same output (bit for bit,
+but for bands alone over more than 32768 bfloat16 keys: they need no list and take the mma.sync kernel, where the
+general path's list may take the tcgen05 one).  It returns None wherever the general path has to say or do something else: other
 maskers or subclasses of these, sizes that select every key, tensors that are not plain CUDA tensors
 of one dtype, rows whose selection is faster with a scratch buffer.
 """
@@ -13,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+import warnings
 from functools import lru_cache
 from typing import List, Optional
 
@@ -31,20 +33,30 @@ _MAX_BANDS = 6       # SAH_STEP_MAX_BANDS
 SERVED = {kind: kind.add_mask for kind in (SinkMasker, LocalMasker, OracleTopK)}
 SERVED_ATTRIBUTES = 2  # of an instance: the configuration and the size; any other may stand in for a method
 
-_module = None
+_module = None  # False: it cannot be loaded
 
 
 def _step_module():
+    """The native entry, or False (and a warning, once) where it is missing or made for another torch: the general
+    path then serves its calls."""
     global _module
     if _module is None:
         path = _native.LIB_PATH.with_name("_sah_step.so")
         if not path.exists():
             path = _native.DEFAULT_LIB_DIR / "_sah_step.so"
-        if not path.exists():
-            raise _native.NativeLibraryError(f"{path} is missing: run sparse-attention-hub_b200/build.py")
-        spec = importlib.util.spec_from_file_location("_sah_step", path)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
+        try:
+            if not path.exists():
+                raise ImportError(f"{path} is missing")
+            spec = importlib.util.spec_from_file_location("_sah_step", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            if module.torch_version != torch.__version__.split("+")[0]:
+                raise ImportError(f"{path} was made for torch {module.torch_version}")
+        except ImportError as error:
+            warnings.warn(f"decode calls take the slower general path: {error}; run "
+                          "sparse-attention-hub_b200/build.py", RuntimeWarning, stacklevel=2)
+            _module = False
+            return _module
         lib = _native.load()
         module.bind(*(ctypes.cast(f, ctypes.c_void_p).value
                       for f in (lib.sah_fixed_step_plan, lib.sah_fixed_step_run, lib.sah_stream_capture)))
@@ -98,10 +110,13 @@ def fixed_step(maskers: List, queries: torch.Tensor, keys: torch.Tensor, values:
                 return None
         else:
             return None
+    module = _step_module()
+    if module is False:
+        return None
     device = queries.device
     stream = _native.stream_of(device)
     tickets, captured = mask_attention_utils.merge_tickets(device, stream)
-    call = _step_module().fixed_step
+    call = module.fixed_step
     done = call(queries, keys, values, attention_mask, sinks, float(scaling), bands, heavy, tickets,
                 _native.sm_count(device), stream, captured)
     if done is None:

@@ -260,6 +260,43 @@ def test_graphs_have_tickets_of_their_own():
     assert attention_wait_errors() == 0
 
 
+def test_host_module_is_made_anew_for_another_torch(monkeypatch):
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("sah_b200_build", fs._native.DEFAULT_LIB_DIR.parent / "build.py")
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    build.build_step()
+    assert not build.step_is_stale()
+    monkeypatch.setattr(build.metadata, "version", lambda _: "1.0")
+    assert build.step_is_stale()
+
+
+@pytest.mark.parametrize("fault", ["missing", "not a module", "other torch"])
+def test_without_the_host_module_the_general_path_serves(fault, monkeypatch, tmp_path):
+    monkeypatch.setattr(fs, "_module", None)
+    if fault == "other torch":
+        monkeypatch.setattr(torch, "__version__", "1.0+cu0")
+    else:
+        monkeypatch.setattr(fs._native, "LIB_PATH", tmp_path / "libsah_b200.so")
+        monkeypatch.setattr(fs._native, "DEFAULT_LIB_DIR", tmp_path)
+        if fault == "not a module":
+            (tmp_path / "_sah_step.so").write_bytes(b"nothing")
+    with pytest.warns(RuntimeWarning, match="general path"):
+        assert fs._step_module() is False
+    assert fs._step_module() is False  # and no second warning
+
+
+@pytest.mark.gpu
+def test_calls_without_the_host_module(monkeypatch):
+    ra = workloads.research_attention(TOPK, "bf16", DEV)
+    q, k, v = _inputs(torch.bfloat16, 1, 8, 2, 1, 3000, 64)
+    call = lambda: ra.custom_attention(None, q, k, v, None, 0.125, 0.0, sparse_meta_data={}, layer_idx=0)[0]  # noqa: E731
+    want = call()
+    monkeypatch.setattr(fs, "_module", False)
+    assert torch.equal(call(), want)
+
+
 def test_other_stacks_keep_the_general_path():
     """Nothing but plain sink, local and one final top-k masker is taken, whatever the tensors."""
     class Cuda:  # stands in for a CUDA tensor: the maskers are looked at before anything else of it
