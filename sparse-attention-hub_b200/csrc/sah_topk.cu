@@ -3,6 +3,8 @@
 //                    (maskers/fixed/implementations/oracle_top_k.py:70-73)
 //   sah_topk_select  radix select over a [rows][S] score tensor
 //                    (maskers/fixed/base.py:74-85)
+#include <algorithm>
+
 #include "sah_common.cuh"
 #include "sah_select.cuh"
 
@@ -215,9 +217,21 @@ extern "C" int sah_qk_scores(const void* q, const void* k, int dtype, int64_t qs
   // Rows of a question: a CTA takes QK_ROWS of them, so that five CTAs share an SM where the queries
   // of all would leave room for one or two, and the waves are finer (96 rows per KV head, 8 x 8191 bfloat16 keys
   // 108.6 us all at once, 90 by 48, 84 by 32, 79.9 by 16; 58 rows x 8576 keys 106 -> 65.5 us; float32, 36
-  // rows x 4096 keys 34.8 -> 32.8 us).
-  const int row_blocks = two ? 1 : (R + QK_ROWS - 1) / QK_ROWS;
-  const int RB = row_blocks == 1 ? R : ((R + row_blocks - 1) / row_blocks + 3) / 4 * 4;
+  // rows x 4096 keys 34.8 -> 32.8 us).  Every block stages the keys anew and the last one has rows to spare, so all
+  // rows stay together where CTAs of all rows fill the chip as well: `fill` waves of them, `per_sm` on an SM.  They
+  // are split below a third of a wave, or below one from 32 rows on; and, as long as not more than a tenth
+  // of the blocks' rows is spare, where they leave an SM fewer CTAs than it takes to hide the loads (bfloat16) or
+  // to keep the fma pipe fed (float32).  Split at all of 820 sizes, 17, 18 and 33 rows were up to 10 % slower on long
+  // ranges (17 rows, 64 heads x 131072 keys: float32 3026 -> 3347 us, bfloat16 1836 -> 1980), float32 with 64 channels
+  // up to 6 % (24 rows 1657 -> 1745).
+  int row_blocks = two ? 1 : (R + QK_ROWS - 1) / QK_ROWS;
+  int RB = row_blocks == 1 ? R : ((R + row_blocks - 1) / row_blocks + 3) / 4 * 4;
+  if (row_blocks > 1) {
+    const int64_t per_sm = std::min<int64_t>(5, 227 * 1024 / (int64_t)(smem + 1024));
+    const double fill = (double)(sah_ceil_div(S, (int64_t)QK_THREADS) * Hkv * B) / (148.0 * (double)per_sm);
+    const bool few = per_sm <= (dtype == SAH_BF16 ? 4 : fill <= 3.0 ? 3 : 2);
+    if (!(fill <= 1.0 / 3.0 || (R >= 32 && fill <= 1.0) || (few && row_blocks * RB * 10 <= R * 11))) row_blocks = 1, RB = R;
+  }
   smem -= (size_t)(R - RB) * D * sizeof(float);
   const dim3 grid((unsigned)(sah_ceil_div(S, (int64_t)QK_THREADS * (two ? 2 : 1)) * row_blocks), (unsigned)Hkv, (unsigned)B);
   cudaStream_t st = (cudaStream_t)stream;

@@ -639,10 +639,11 @@ def test_band_masks_without_a_bitmap(dtype, S, Sq, stack, monkeypatch):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype,Hq,Hkv,Sq,S,D,bias", [
     ("bf16", 8, 2, 5, 700, 128, True), ("bf16", 4, 1, 17, 129, 128, False), ("f32", 3, 1, 11, 257, 64, True),
-    ("bf16", 2, 2, 33, 40, 64, True), ("f32", 8, 1, 6, 128, 80, False), ("bf16", 8, 1, 2, 300, 128, True)])
+    ("bf16", 2, 2, 33, 40, 64, True), ("f32", 8, 1, 6, 128, 80, False), ("bf16", 8, 1, 2, 300, 128, True),
+    ("bf16", 4, 1, 5, 40001, 128, True), ("f32", 1, 1, 17, 30001, 64, False), ("f32", 3, 1, 11, 70000, 128, False)])
 def test_scores_of_many_rows_equal_those_of_one_position(dtype, Hq, Hkv, Sq, S, D, bias):
-    """Rows per KV head that are cut into blocks (20, 68, 33, 33, 48 and 16 of them): the scores of every
-    position are those of a call for that position alone, bit for bit."""
+    """Rows per KV head that are cut into blocks (20, 68, 33, 33, 48 and 16 of them), that stay together on a grid of
+    more CTAs (20 and 17) and that are cut there too (33): the scores of every position are those of a call for that position alone, bit for bit."""
     import torch
     from sparse_attention_hub import _native
 
