@@ -610,9 +610,11 @@ static const char* g_last_attn_kernel = "none";
 #include "sah_attention_umma.cuh"
 #include "sah_attention_stream.cuh"
 
-// BANDS: the list is a.iv
+// BANDS: the list is a.iv.  CTAs per SM: as many as the rings leave room for.  (Left to itself the compiler gives the
+// merge at the end 168 registers, three CTAs with 64 channels where four fit: 33 positions of 32 heads x 20000 keys of
+// which half are selected 929 us, so 688; 24 positions 658 -> 483; one position of 16 sequences 492 -> 367.)
 template <typename T, int D, int NQUAD, bool BANDS>
-__global__ void __launch_bounds__(AT_THREADS)
+__global__ void __launch_bounds__(AT_THREADS, D == 64 ? 4 : 2)
 masked_attention_kernel(AttnArgs a, int* __restrict__ tickets, const float* __restrict__ sinks,
                         T* __restrict__ out, float* __restrict__ part_out) {
   sah_pdl_entry();
