@@ -49,6 +49,10 @@
 // split the merge next to nothing (8 tiles 13.2 us, 4 tiles 10.6, 2 tiles and 1 tile 9.1, 32 heads x 8191
 // keys, 90 tiles per group; 131072 keys, 560 tiles per group: 19.3, 16.1, 15.9, 15.9 us).
 #define ATM_MIN_TILES 2
+// Below this many tiles per warp of all CTAs many groups have one wave of them as well, once a list is long enough
+// for more than two: a second wave's merge of many rows costs more than it evens out (64 channels; 72 groups of 16
+// rows, lists of 700 keys 28.9 -> 25.0 us; 40 groups, 3500 keys 25.0 -> 21.0; 128 groups of one row, 700 keys 22.8 -> 21.0).
+#define ATM_SHARED_TILES 8
 #define ATM_ONE_WAVE_TILES 48  // below this many tiles per warp, one wave of CTAs instead of two
 #define ATM_FINE_SPLITS 16     // ... when the grid has at least this many CTAs per group
 
@@ -121,6 +125,7 @@ __device__ __forceinline__ int atm_active_splits(int total_tiles, int nsplit, in
   if (nsplit >= ATM_FINE_SPLITS && wave < nsplit && total_tiles < nsplit * ATM_WARPS * ATM_ONE_WAVE_TILES) active = wave;
   const int by_length = (total_tiles + ATM_WARPS * ATM_MIN_TILES - 1) / (ATM_WARPS * ATM_MIN_TILES);
   if (by_length < active) active = by_length;
+  if (active > wave && by_length > 2 * wave && total_tiles < nsplit * ATM_WARPS * ATM_SHARED_TILES) active = wave;
   return active < 1 ? 1 : active;
 }
 
