@@ -571,12 +571,13 @@ int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t 
  * device: parts launched after the clustering has converged return at once, so the next ASSIGN can be launched
  * before the host knows.  sums and counts are scratch of sah_pq_accumulate's sizes.  state: five words on the
  * device; [0] is set once the clustering has converged, [1] is the number of iterations that ran, [2] is
- * set when a bounded wait of the tensor-core kernel ran out (codes and centroids are then void). */
+ * set when a bounded wait of the tensor-core kernel ran out (codes and centroids are then void).  seen: NULL, or
+ * where an UPDATE leaves these three for the host (pinned memory; a copy in the stream would hold up the ASSIGN). */
 enum { SAH_KMEANS_BEGIN = 1, SAH_KMEANS_UPDATE = 2, SAH_KMEANS_ASSIGN = 4 };
 int sah_pq_kmeans_step(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
                        int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int what,
                        const int64_t* reseed, float* centroids, uint8_t* codes, int64_t cap, double* sums, int* counts,
-                       int* state, int use_tc, int sm_count, void* stream);
+                       int* state, int* seen, int use_tc, int sm_count, void* stream);
 
 /* n_iter iterations launched together.  reseed: n_iter device pointers (host array).
  * All operands stay untouched until the stream has passed the last launch. */

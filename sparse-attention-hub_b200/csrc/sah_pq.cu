@@ -422,7 +422,7 @@ __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t 
                                  int Hkv, int64_t init_offset, int n_sub, int sub_d, int n_cent,
                                  double* __restrict__ sums, int* __restrict__ counts,
                                  const int64_t* __restrict__ reseed, float* __restrict__ centroids,
-                                 float* __restrict__ shift2, PqState* __restrict__ state) {
+                                 float* __restrict__ shift2, PqState* __restrict__ state, int* __restrict__ seen) {
   __shared__ float scratch[33];
   if (state && state->done) return;
   const int64_t grp = blockIdx.x;
@@ -473,8 +473,15 @@ __global__ void pq_update_kernel(const T* __restrict__ x, int64_t xs_b, int64_t 
   __threadfence();
   if (atomicAdd(&state->ticket, 1) == (int)gridDim.x - 1) {  // every block has read `done` by now
     state->iterations += 1;
-    if (atomicExch(&state->open, 0) == 0) state->done = 1;
+    const int done = atomicExch(&state->open, 0) == 0;
+    state->done = done;
     state->ticket = 0;
+    if (seen) {
+      seen[0] = done;
+      seen[1] = state->iterations;
+      seen[2] = state->err;
+      __threadfence_system();
+    }
   }
 }
 
@@ -488,7 +495,7 @@ extern "C" int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_
   SAH_DISPATCH_DTYPE(dtype, T, {
     pq_update_kernel<T><<<(unsigned)groups, 256, 0, (cudaStream_t)stream>>>(
         (const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub, sub_d, n_cent, const_cast<double*>(sums),
-        const_cast<int*>(counts), reseed, centroids, shift2, nullptr);
+        const_cast<int*>(counts), reseed, centroids, shift2, nullptr, nullptr);
   });
   SAH_LAUNCH_CHECK("pq_update");
   return SAH_OK;
@@ -497,7 +504,7 @@ extern "C" int sah_pq_update(const void* x, int dtype, int64_t xs_b, int64_t xs_
 extern "C" int sah_pq_kmeans_step(const void* x, int dtype, int64_t xs_b, int64_t xs_h, int64_t xs_s, int B, int Hkv,
                                   int64_t n_keys, int64_t init_offset, int n_sub, int sub_d, int n_cent, int what,
                                   const int64_t* reseed, float* centroids, uint8_t* codes, int64_t cap, double* sums,
-                                  int* counts, int* state, int use_tc, int sm_count, void* stream) {
+                                  int* counts, int* state, int* seen, int use_tc, int sm_count, void* stream) {
   SAH_REQUIRE(x && centroids && codes && sums && counts && state && (reseed || !(what & SAH_KMEANS_UPDATE)),
               "pq_kmeans: null pointer");
   SAH_REQUIRE(B > 0 && Hkv > 0 && n_sub > 0 && sub_d > 0 && n_keys >= 0, "pq_kmeans: bad extents");
@@ -514,7 +521,8 @@ extern "C" int sah_pq_kmeans_step(const void* x, int dtype, int64_t xs_b, int64_
   if (what & SAH_KMEANS_UPDATE) {
     SAH_DISPATCH_DTYPE(dtype, T, {
       pq_update_kernel<T><<<(unsigned)groups, 256, 0, st>>>((const T*)x, xs_b, xs_h, xs_s, Hkv, init_offset, n_sub,
-                                                            sub_d, n_cent, sums, counts, reseed, centroids, nullptr, ps);
+                                                            sub_d, n_cent, sums, counts, reseed, centroids, nullptr, ps,
+                                                            seen);
     });
     SAH_LAUNCH_CHECK("pq_update");
   }
@@ -541,8 +549,8 @@ extern "C" int sah_pq_kmeans(const void* x, int dtype, int64_t xs_b, int64_t xs_
   for (int it = 0; it <= n_iter && rc == SAH_OK; ++it)
     rc = sah_pq_kmeans_step(x, dtype, xs_b, xs_h, xs_s, B, Hkv, n_keys, init_offset, n_sub, sub_d, n_cent,
                             (it == 0 ? SAH_KMEANS_BEGIN : SAH_KMEANS_UPDATE) | (it < n_iter ? SAH_KMEANS_ASSIGN : 0),
-                            it > 0 ? reseed[it - 1] : nullptr, centroids, codes, cap, sums, counts, state, use_tc, sm_count,
-                            stream);
+                            it > 0 ? reseed[it - 1] : nullptr, centroids, codes, cap, sums, counts, state, nullptr, use_tc,
+                            sm_count, stream);
   return rc;
 }
 

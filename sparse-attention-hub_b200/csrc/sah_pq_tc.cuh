@@ -108,8 +108,8 @@ __device__ __forceinline__ unsigned int ptc_hash(const float* c) {
   const unsigned int v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   unsigned int h = 0u;
 #pragma unroll
-  for (int d = 0; d < 8; ++d) h = (__funnelshift_l(h, h, 13) ^ v[d]) * 0x9e3779b1u;
-  return h ^ (h >> 15);
+  for (int d = 0; d < 8; ++d) h += v[d] * (0x9e3779b1u + 0x3c6ef372u * d);  // odd factors, terms that do not wait for one another
+  return (h ^ (h >> 16)) * 0x85ebca6bu;
 }
 
 // 32 columns of an accumulator: two matrix rows of 16
@@ -242,8 +242,9 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
     };
     uint32_t again = 0u;
     int m = 0;
-    for (int i = tid; i < NS * n_cent; i += PTC_THREADS, ++m) {
-      const int s = i / n_cent, c = i - s * n_cent;
+    for (int i = tid; i < NS * NC; i += PTC_THREADS, ++m) {
+      const int s = i / NC, c = i - s * NC;
+      if (c >= n_cent) continue;
       const unsigned int bits = ptc_hash(cent_sm + (s * 256 + c) * SD);
       const int f = (int)first_sm[s * PTC_SLOTS + (bits >> (32 - PTC_SLOT_BITS))];
       if (f == c || copy_of(s, c, f)) continue;
@@ -252,7 +253,7 @@ pq_assign_tc_kernel(const __nv_bfloat16* __restrict__ x, int64_t xs_b, int64_t x
     }
     __syncthreads();
     for (; again; again &= again - 1) {
-      const int i = tid + (__ffs(again) - 1) * PTC_THREADS, s = i / n_cent, c = i - s * n_cent;
+      const int i = tid + (__ffs(again) - 1) * PTC_THREADS, s = i / NC, c = i - s * NC;
       copy_of(s, c, (int)second_sm[s * PTC_SLOTS2 + ((ptc_hash(cent_sm + (s * 256 + c) * SD) >> 7) & (PTC_SLOTS2 - 1))]);
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");

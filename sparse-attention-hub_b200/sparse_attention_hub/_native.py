@@ -148,7 +148,8 @@ _SIGNATURES = {
     "sah_pq_assign": [_P, _I, _L, _L, _L, _I, _I, _L, _L, _L, _I, _I, _I, _P, _P, _L, _I, _P],
     "sah_pq_accumulate": [_P, _I, _L, _L, _L, _I, _I, _L, _L, _I, _I, _I, _P, _L, _P, _P, _P],
     "sah_pq_update": [_P, _I, _L, _L, _L, _I, _I, _L, _I, _I, _I, _P, _P, _P, _P, _P, _P],
-    "sah_pq_kmeans_step": [_P, _I, _L, _L, _L, _I, _I, _L, _L, _I, _I, _I, _I, _P, _P, _P, _L, _P, _P, _P, _I, _I, _P],
+    "sah_pq_kmeans_step": [_P, _I, _L, _L, _L, _I, _I, _L, _L, _I, _I, _I, _I, _P, _P, _P, _L, _P, _P, _P, _P, _I, _I,
+                           _P],
     "sah_pq_kmeans": [_P, _I, _L, _L, _L, _I, _I, _L, _L, _I, _I, _I, _I, POINTER(c_void_p), _P, _P, _L, _P, _P, _P,
                       _I, _I, _P],
     "sah_pq_scores_ws_bytes": [_I, _I, _I, _I, _I, _I],  # returns int64

@@ -306,7 +306,7 @@ class PQCache(TopKMasker):
         dev = k.device
         n_keys = k.shape[2] - local_off
         state = torch.empty(5, dtype=torch.int32, device=dev)
-        seen = torch.empty(5, dtype=torch.int32, pin_memory=True)
+        seen = torch.empty(3, dtype=torch.int32, pin_memory=True)
         reached = torch.cuda.Event()
         drawn = []
 
@@ -314,7 +314,7 @@ class PQCache(TopKMasker):
             _native.check(lib.sah_pq_kmeans_step(*kargs, B, Hkv, n_keys, local_off, n_sub, sub_d, n_cent, what,
                                                  _native.ptr(reseed), centroids.data_ptr(), codes.data_ptr(),
                                                  codes.shape[2], sums.data_ptr(), counts.data_ptr(), state.data_ptr(),
-                                                 int(use_tc), _native.sm_count(dev), _native.stream_of(dev)),
+                                                 seen.data_ptr(), int(use_tc), _native.sm_count(dev), _native.stream_of(dev)),
                           "sah_pq_kmeans_step")
 
         launch(_native.KMEANS_BEGIN | _native.KMEANS_ASSIGN)
@@ -327,13 +327,12 @@ class PQCache(TopKMasker):
             else:
                 drawn.append(torch.randint(0, n_keys, (B * Hkv * n_sub, n_cent), device=dev))
             launch(_native.KMEANS_UPDATE, drawn[it])
-            seen.copy_(state, non_blocking=True)
             reached.record(torch.cuda.current_stream(dev))
             it += 1
             if it < self.kmeans_iter:
                 launch(_native.KMEANS_ASSIGN)
             reached.synchronize()
-            done, _, failed = seen[:3].tolist()
+            done, _, failed = seen.tolist()
             if failed:  # a bounded wait inside the tensor-core kernel ran out: fixed-order kernel, from the start
                 use_tc = False
                 centroids.copy_(first_centroids())
