@@ -686,7 +686,8 @@ int sah_masked_attention(const void* q, const void* k, const void* v, int dtype,
  * weights of sah_masked_attention_lsh.  bfloat16, head dim 128, rows 16-byte aligned.  n_parts: what
  * sah_attn_stream_parts gave for these extents (lsh_k, lsh_l: bits per table and tables); it gives 0 where the
  * gather kernels are the faster ones or a kernel has been chosen by sah_attn_select_kernel.  parts:
- * scratch, float32 [n_parts][rows][D + 2].  *errflag is set when a bounded wait ran out. */
+ * scratch, float32 [n_parts][rows][D + 2].  *errflag is set when a bounded wait ran out.  A row's output goes by
+ * the V rows of its own keys, also where others hold infinities or NaN. */
 int sah_attn_stream_parts(int B, int Hq, int Hkv, int Sq, int64_t S, int D, int lsh_k, int lsh_l, int sm_count);
 int sah_masked_attention_stream(const void* q, const void* k, const void* v, int64_t qs_b, int64_t qs_h, int64_t qs_q,
                                 int64_t ks_b, int64_t ks_h, int64_t ks_s, int64_t vs_b, int64_t vs_h, int64_t vs_s,

@@ -607,8 +607,9 @@ masked_attention_umma_kernel(AttnArgs a, int* __restrict__ tickets, int* __restr
 //   32768 keys, 25000 35.6 / 30.1; 32 groups, 65536 keys, weighted, 22600 84.5 / 78.1, 64000 208 / 176;
 //   64 groups, 32768 keys, 2550 35.0 / 27.3, 24900 166 / 142; 16 groups, 100000 keys, 97400 160 / 138.
 //   Fewer rows times keys leave short lists, where the other's fixed costs are lower: 8192 keys, 4 rows,
-//   union of 1530 10.7 / 11.8; 16384 keys, one row, 1630 10.3 / 11.1.  (Up to 32768 keys a mask may be bands
-//   alone, hundreds of columns, which this rule cannot see; it leaves those sizes to the other kernel.)
+//   union of 1530 10.7 / 11.8; 16384 keys, one row, 1630 10.3 / 11.1.  (Up to 32768 keys a list may be that
+//   of bands alone, hundreds of columns -- of several query positions, or where the call is not one of the native
+//   decode entry --, which this rule cannot see; it leaves those sizes to the other kernel.)
 //   More than four rows (no room for P's remainders, exactness below): 8 groups of 8, 65536 keys 36.2 / 38.5,
 //   32 groups of 8, 32768 keys 52 / 56; 64 groups with lists of a few thousand rows 69 / 63.
 // Up to four rows the error against float64 is below the other's, 1.6e-3 to 1.7e-3 against 1.8e-3 to 2.2e-3 of
