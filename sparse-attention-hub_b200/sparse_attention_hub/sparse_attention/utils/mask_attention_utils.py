@@ -92,12 +92,14 @@ def _error_word(device: torch.device) -> torch.Tensor:
     if found is None:
         found = torch.zeros(1, dtype=torch.int32, device=device)
         if not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(device).synchronize()  # once: other streams' kernels may set it from here on
             _error_words[device.index] = found
     return found
 
 
 class _StreamedCall:
-    """What the union list of a call that streamed all keys is made from, should somebody ask for it."""
+    """What the union list of a call that streamed all keys is made from, should somebody ask for it: the call's
+    bitmaps and the keys' constants, kept until the next call."""
 
     def __init__(self, payload, sizes, extents, stream) -> None:
         self.match, self.unit = payload.match_bits, payload.unit_bits
