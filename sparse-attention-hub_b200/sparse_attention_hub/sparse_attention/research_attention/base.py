@@ -79,13 +79,14 @@ class ResearchAttention(SparseAttention):
             )
         sparse_meta_data: Dict[Any, Any] = kwargs.pop("sparse_meta_data")
         logger = MicroMetricLogger()
-        for masker in self.maskers:  # all that other stacks pay for the native entry
-            kind = type(masker)
-            if kind not in SERVED or kind.add_mask is not SERVED[kind] or len(masker.__dict__) != SERVED_ATTRIBUTES:
-                native = False  # another masker, or one whose methods somebody has put another in place of
-                break
-        else:
-            native = True
+        # all that other stacks pay for the native entry: they mostly end with the masker that it does not serve
+        native = bool(self.maskers) and type(self.maskers[-1]) in SERVED
+        if native:
+            for masker in self.maskers:
+                kind = type(masker)
+                if kind not in SERVED or kind.add_mask is not SERVED[kind] or len(masker.__dict__) != SERVED_ATTRIBUTES:
+                    native = False  # another masker, or one whose methods somebody has put another in place of
+                    break
         if (native and not logger.enabled_metrics and not self.return_attention_weights and dropout == 0.0
                 and kwargs.get("sequence_shard") is None
                 and type(self).build_mask is _BUILD_MASK and "build_mask" not in self.__dict__):
